@@ -515,6 +515,63 @@ KFB_API int kfb_gemm_bf16(const void* a, const void* b, void* d, const float* bi
                   long long ldb, long long ldd, long long batch_stride_a, long long batch_stride_b,
                   long long batch_stride_d, int out_dtype, void* stream);
 
+/*
+ * Whole transformer stacks of the diffusion network in one call (the kernels of the single operators above, issued from native
+ * code; nothing is allocated, no synchronisation).
+ *
+ * kfb_conditioning: the projections of the conditioning s that all blocks share.  w_gs [gs_cols, c_s]: every AdaLN's gate and
+ *   shift matrix in block order, its LayerNorm scale folded into the columns, b_gs [gs_cols] fp32; w_og [og_cols, c_s] and b_og:
+ *   every block's output-gate projection.  bf16, or bf16 triple splits [cols, 6 c_s] in the fp32-accurate mode.
+ * kfb_token_stack_fwd: CachedGlobalTransformerStack.forward (src/kfold/model/layers/folding/diffusion_transformer.py:260-413).
+ *   a, out (groups, samples, l, c) of act_dtype (bf16 or fp32; fp32 when `precise`); s (groups, s_samples, l, c_s), s_samples 1 or
+ *   samples; pair_bias: block i's plane of (group g, head h) starts at i * bias_block_stride + (g * heads + h) * bias_head_stride,
+ *   rows bias_ld elements apart, bf16 (fp32 when `precise`); mask (groups, l) bytes; gs_cols = 4 c n_blocks with the columns
+ *   [attention gate | shift | transition gate | shift] per block, og_cols = 2 c n_blocks.  out may be a.
+ * kfb_atom_stack_fwd: LocalTransformerStack.forward (diffusion_transformer.py:419-512), bf16 compute, head dim <= 32.
+ *   a, out (groups, samples, l, c); s (groups, l, c_s) shared by the samples; window_bias bf16 [n_blocks][heads][bias_windows][32][128];
+ *   `bias_share` consecutive samples use the same window biases, `mask_share` the same row of mask; gs_cols = 6 c n_blocks with
+ *   [query gate | shift | key gate | shift | transition gate | shift] per block, og_cols = 2 c n_blocks.
+ */
+typedef struct {
+  const void* w_gs;
+  const float* b_gs;
+  const void* w_og;
+  const float* b_og;
+  long long gs_cols, og_cols;
+  int c_s;
+  float eps;
+} kfb_conditioning;
+typedef struct {
+  const void* w_proj;
+  const float* proj_bias;
+  const void* w_out;
+  const float* out_bias;
+  const void* w_swiglu;
+  const void* w_tout;
+} kfb_token_block;
+typedef struct {
+  const void* w_q;
+  const float* q_bias;
+  const void* w_kv;
+  const void* w_out;
+  const float* out_bias;
+  const void* w_swiglu;
+  const void* w_tout;
+} kfb_atom_block;
+KFB_API size_t kfb_token_stack_workspace_bytes(int groups, int samples, int s_samples, int l, int c, int c_s, int heads, int hidden,
+                                               long long gs_cols, long long og_cols, int precise);
+KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, const kfb_conditioning* cond, const void* a, void* out,
+                                int act_dtype, const void* s, int s_dtype, const void* pair_bias, long long bias_block_stride,
+                                long long bias_head_stride, long long bias_ld, const unsigned char* mask, void* workspace,
+                                size_t workspace_bytes, int groups, int samples, int s_samples, int l, int c, int heads, int hidden,
+                                float eps, int precise, void* stream);
+KFB_API size_t kfb_atom_stack_workspace_bytes(int groups, int samples, int l, int c, int c_s, int heads, int hidden, long long gs_cols,
+                                              long long og_cols);
+KFB_API int kfb_atom_stack_fwd(const kfb_atom_block* blocks, int n_blocks, const kfb_conditioning* cond, const void* a, void* out,
+                               int act_dtype, const void* s, int s_dtype, const void* window_bias, long long bias_windows,
+                               const unsigned char* mask, int mask_share, int bias_share, void* workspace, size_t workspace_bytes,
+                               int groups, int samples, int l, int c, int heads, int hidden, float eps, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

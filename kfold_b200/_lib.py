@@ -23,6 +23,20 @@ class KfbError(RuntimeError):
     pass
 
 
+class Conditioning(ctypes.Structure):
+    """kfb_conditioning: the stacked projections of the conditioning that all blocks of a stack share."""
+    _fields_ = [("w_gs", c_void_p), ("b_gs", c_void_p), ("w_og", c_void_p), ("b_og", c_void_p), ("gs_cols", c_ll), ("og_cols", c_ll),
+                ("c_s", c_int), ("eps", c_float)]
+
+
+class TokenBlock(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("w_proj", "proj_bias", "w_out", "out_bias", "w_swiglu", "w_tout")]
+
+
+class AtomBlock(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("w_q", "q_bias", "w_kv", "w_out", "out_bias", "w_swiglu", "w_tout")]
+
+
 # name -> argtypes; every function returns int except where noted
 _SIGNATURES = {
     "kfb_version": [],
@@ -87,6 +101,10 @@ _SIGNATURES = {
                            c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "kfb_rigid_align": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_int, c_int, c_void_p],
     "kfb_center_coords": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
+    "kfb_token_stack_fwd": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_ll, c_ll, c_ll, c_void_p,
+                            c_void_p, ctypes.c_size_t] + [c_int] * 7 + [c_float, c_int, c_void_p],
+    "kfb_atom_stack_fwd": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_ll, c_void_p, c_int, c_int,
+                           c_void_p, ctypes.c_size_t] + [c_int] * 6 + [c_float, c_void_p],
     "kfb_transition_fwd_static": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int,
                                   c_float, c_int, c_void_p],
 }
@@ -110,6 +128,8 @@ _SIZE_FUNCS = {
     "kfb_apb_cross_workspace_bytes_precise": [c_int, c_int, c_int, c_int],
     "kfb_trimul_workspace_bytes": [c_int, c_int, c_int],
     "kfb_parcae_workspace_bytes": [c_ll, c_int],
+    "kfb_token_stack_workspace_bytes": [c_int] * 8 + [c_ll, c_ll, c_int],
+    "kfb_atom_stack_workspace_bytes": [c_int] * 7 + [c_ll, c_ll],
 }
 
 
@@ -146,11 +166,21 @@ def check(status: int) -> None:
 
 
 def ptr(t: torch.Tensor | None):
-    return None if t is None else c_void_p(t.data_ptr())
+    """Address for a ``void*`` parameter (ctypes converts plain integers; building a c_void_p here only costs time)."""
+    return None if t is None else t.data_ptr()
+
+
+def ref(struct: ctypes.Structure):
+    return ctypes.addressof(struct)
+
+
+def raw_stream(index: int | None = None) -> int:
+    """cudaStream_t of the current stream, without the Stream object torch.cuda.current_stream() builds around it."""
+    return torch._C._cuda_getCurrentRawStream(torch.cuda.current_device() if index is None else index)
 
 
 def stream_ptr():
-    return c_void_p(torch.cuda.current_stream().cuda_stream)
+    return raw_stream()
 
 
 class on_device:

@@ -678,7 +678,7 @@ static int launch_cfg(cudaStream_t stream, const AttnParams& p) {
       KFB_TRY(make_tmap(&tb, p.bias, 2, 3, dims, str, box, 128));
     } else {
       const uint64_t dims[3] = {(uint64_t)p.lk, (uint64_t)p.lq, (uint64_t)bias_batches * p.heads};
-      const uint64_t str[2] = {(uint64_t)p.ldb * 2, (uint64_t)p.lq * p.ldb * 2};
+      const uint64_t str[2] = {(uint64_t)p.ldb * 2, (uint64_t)(p.bias_hs > 0 ? p.bias_hs : p.lq * p.ldb) * 2};
       const uint32_t box[3] = {64, kBQ, 1};
       KFB_TRY(make_tmap(&tb, p.bias, 2, 3, dims, str, box, 128));
     }
@@ -697,7 +697,7 @@ int launch_attention(cudaStream_t stream, const AttnParams& p_in) {
   p.trace = g_attention_trace;
   KFB_CHECK_ARG(p.batch > 0 && p.heads > 0 && p.lq > 0 && p.lk > 0, "attention: empty problem");
   KFB_CHECK_ARG(p.d % 8 == 0 && p.d <= p.dpad, "attention: head dim %d must be a multiple of 8 and <= %d", p.d, p.dpad);
-  KFB_CHECK_ARG(p.ldq % 8 == 0 && p.ldk % 8 == 0 && p.ldv % 8 == 0 && p.ldb % 8 == 0 && p.ldo % 8 == 0,
+  KFB_CHECK_ARG(p.ldq % 8 == 0 && p.ldk % 8 == 0 && p.ldv % 8 == 0 && p.ldb % 8 == 0 && p.ldo % 8 == 0 && p.bias_hs % 8 == 0,
                 "attention: leading dimensions must be multiples of 8 elements");
   KFB_CHECK_ARG(p.bias_div >= 1 && p.bias_mod >= 0 && p.mask_lo_extent >= 1, "attention: bad divisors");
   KFB_CHECK_ARG(p.bias_head_major == 0 || p.bias_head_major >= cdiv(p.batch, p.bias_div) * (p.bias_mod > 0 ? p.bias_mod : 1),

@@ -40,7 +40,8 @@ struct AttnParams {
   // bias : [bias_batches][heads][lq][ldb] bf16 ; batch entry b uses bias batch b / bias_div, or, with bias_mod > 0,
   // (b / bias_div) * bias_mod + b % bias_mod: batch entries ordered (group, sample, window) with bias_mod windows and
   // bias_div = samples * windows, one bias per (group, window) that every sample of the group reuses
-  const void* bias; long long ldb; int bias_div; int bias_mod;
+  // (bias_hs: elements between the planes of consecutive heads; 0 = lq * ldb)
+  const void* bias; long long ldb; long long bias_hs; int bias_div; int bias_mod;
   // 0: bias stored [bias_batches][heads][lq][ldb]; n > 0: stored [heads][n bias batches][lq][ldb] (head-major, as one
   // projection of all heads of several layers at once writes it)
   int bias_head_major;
@@ -71,7 +72,7 @@ struct AttnFp32Params {
   long long ld;                // row stride of q and g
   long long ld_kv;             // row stride of k and v (0: same as ld)
   int q_col0, k_col0, v_col0, g_col0;
-  const float* bias; long long ldb; int bias_div; int bias_mod; int bias_head_major;  // as in AttnParams
+  const float* bias; long long ldb; long long bias_hs; int bias_div; int bias_mod; int bias_head_major;  // as in AttnParams
   const unsigned char* mask; long long m_hi, m_lo, m_k; int mask_lo_extent;
   __nv_bfloat16* out6;
   const char* tag;

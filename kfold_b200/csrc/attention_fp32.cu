@@ -37,7 +37,7 @@ __global__ void __launch_bounds__(kFq) attention_fp32_kernel(const AttnFp32Param
   const int bias_b = p.bias_mod > 0 ? (b / p.bias_div) * p.bias_mod + b % p.bias_mod : b / p.bias_div;
   const long long bias_z = p.bias_head_major > 0 ? static_cast<long long>(h) * p.bias_head_major + bias_b
                                                  : static_cast<long long>(bias_b) * p.heads + h;
-  const float* bias_base = p.bias + bias_z * static_cast<long long>(p.lq) * p.ldb;
+  const float* bias_base = p.bias + bias_z * (p.bias_hs > 0 ? p.bias_hs : p.lq * p.ldb);
   const long long ld_kv = p.ld_kv > 0 ? p.ld_kv : p.ld;
 
   for (int k0 = 0; k0 < p.lk; k0 += kFk) {

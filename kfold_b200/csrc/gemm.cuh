@@ -35,6 +35,7 @@ struct EpiSeg {
   int out_fp32;     // 0: bf16 output, 1: fp32 output
   int vec;          // 1: s_col == 1 and every row start is 16-byte aligned -> vector stores
   int tma_slot;     // >= 0: channel-major bf16 segment stored through shared memory with TMA store map `tma_slot`
+  int n_pad;        // rows may be written up to this position along n (their allocated pitch), 0: up to n_extent
   int split;        // precise mode: 0 plain store; 1 / 2: the value is split into three bf16 parts x0+x1+x2 and stored
                     // six times, s_part elements apart, as [x0 x0 x1 x1 x0 x2] (1) or [x0 x1 x0 x1 x2 x0] (2)
   long long s_part;
@@ -643,9 +644,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           const int n0 = nb * kBM + c;
           if (lane_ok) {
             __nv_bfloat16* d = drow + n0;
-            if (n0 + 32 <= p.n_extent && (reinterpret_cast<uintptr_t>(d) & 31) == 0) {
+            const int n_lim = sg.n_pad > 0 ? sg.n_pad : p.n_extent;
+            if (n0 + 32 <= n_lim && (reinterpret_cast<uintptr_t>(d) & 31) == 0) {
               st_global_v8(d, w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7]);
               st_global_v8(d + 16, w[8], w[9], w[10], w[11], w[12], w[13], w[14], w[15]);
+            } else if ((n_lim & 7) == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                if (n0 + 8 * i < n_lim)
+                  *reinterpret_cast<uint4*>(d + 8 * i) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
             } else {
 #pragma unroll
               for (int i = 0; i < 32; ++i)

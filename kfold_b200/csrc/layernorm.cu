@@ -225,6 +225,28 @@ int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w
   return KFB_ERR_INVALID_ARGUMENT;
 }
 
+// fp32 -> bf16 conversion, eight elements per thread (HBM-bound; the conditioning rows of a stack: one small launch).
+__global__ void __launch_bounds__(256) to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
+  const long long i = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * 8;
+  if (i + 8 <= n) {
+    const float4 a = *reinterpret_cast<const float4*>(x + i), b = *reinterpret_cast<const float4*>(x + i + 4);
+    const __nv_bfloat162 p[4] = {__floats2bfloat162_rn(a.x, a.y), __floats2bfloat162_rn(a.z, a.w), __floats2bfloat162_rn(b.x, b.y),
+                                 __floats2bfloat162_rn(b.z, b.w)};
+    *reinterpret_cast<uint4*>(y + i) = *reinterpret_cast<const uint4*>(p);
+  } else {
+    for (long long k = i; k < n; ++k) y[k] = __float2bfloat16_rn(x[k]);
+  }
+}
+
+int launch_to_bf16(cudaStream_t stream, const float* x, __nv_bfloat16* y, long long n) {
+  if (n <= 0) return KFB_OK;
+  KFB_CHECK_ARG(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0, "to_bf16: pointers must be 16-byte aligned");
+  LaunchScope scope(stream, "to_bf16");
+  to_bf16_kernel<<<static_cast<unsigned>((n + 2047) / 2048), 256, 0, stream>>>(x, y, n);
+  KFB_CUDA(cudaGetLastError());
+  return KFB_OK;
+}
+
 // ------------------------------------------------------------------------------------------------
 // fp32-accurate mode: LayerNorm (or a plain copy) of fp32 rows, written as the bf16 triple split.
 // ------------------------------------------------------------------------------------------------

@@ -15,6 +15,9 @@ struct RowPerm {
 int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w, const float* b, long long rows, int c,
                      long long xs, long long ys, float eps, int in_dtype, int out_dtype, RowPerm perm = RowPerm());
 
+// fp32 -> bf16 (round to nearest), n elements.
+int launch_to_bf16(cudaStream_t stream, const float* x, __nv_bfloat16* y, long long n);
+
 // Row-wise LayerNorm of fp32 rows written as the bf16 triple split [x0 x0 x1 x1 x0 x2] (six blocks of c columns,
 // row stride 6c): the A operand of the fp32-accurate GEMMs.  With w == b == nullptr and `normalise` == 0 it only
 // splits (used for operands that are not normalised).

@@ -44,7 +44,7 @@ size_t carve_apb(ApbWs& w, void* base, int batch, int l, int c, int heads) {
   const size_t rows = static_cast<size_t>(batch) * l;
   const int hdp = heads * dpad_of(c / heads);
   w.qkg = cv.take<__nv_bfloat16>(rows * 3 * hdp);
-  w.vt = cv.take<__nv_bfloat16>(rows * hdp);
+  w.vt = cv.take<__nv_bfloat16>(static_cast<size_t>(batch) * pitch16(l) * hdp);
   w.og = cv.take<__nv_bfloat16>(rows * c);
   return cv.off;
 }
@@ -534,23 +534,14 @@ KFB_API size_t kfb_apb_workspace_bytes(int batch, int l, int c, int heads) {
   return carve_apb(w, nullptr, batch, l, c, heads);
 }
 
-KFB_API int kfb_apb_fwd(const void* x, const void* pair_bias, const unsigned char* mask, const void* w_proj_packed,
-                        const float* proj_bias, const void* w_out, const float* out_bias, const void* out_gate,
-                        int gate_share, long long gate_ld, void* out, const void* resid, void* workspace,
-                        size_t workspace_bytes, int batch, int l, int c, int heads, int bias_div, int out_dtype, void* stream_) {
-  KFB_CHECK_ARG(x && pair_bias && mask && w_proj_packed && w_out && out && workspace, "apb: null pointer");
-  KFB_CHECK_ARG(is_dtype(out_dtype), "apb: bad dtype %d", out_dtype);
-  KFB_CHECK_ARG(batch >= 1 && l >= 8 && l % 8 == 0, "apb: L=%d must be a positive multiple of 8 (pad in the caller)", l);
-  KFB_CHECK_ARG(heads >= 1 && c % heads == 0 && c % 8 == 0, "apb: c=%d heads=%d", c, heads);
-  KFB_CHECK_ARG(bias_div >= 1 && batch % bias_div == 0, "apb: batch %d not a multiple of bias_div %d", batch, bias_div);
-  if (out_gate != nullptr)
-    KFB_CHECK_ARG(gate_share >= 1 && batch % gate_share == 0, "apb: batch %d not a multiple of gate_share %d", batch, gate_share);
-  else
-    gate_share = 1;
-  if (gate_ld <= 0) gate_ld = c;
-  KFB_CHECK_ARG(gate_ld >= c, "apb: gate row stride %lld below c=%d", gate_ld, c);
-  KFB_CHECK_ARG(out_gate == nullptr || out_dtype == KFB_FP32_PRECISE || (gate_ld % 8 == 0 && (reinterpret_cast<uintptr_t>(out_gate) & 15) == 0),
-                "apb: bf16 gate rows must start on 16-byte boundaries (pointer and row stride %lld)", gate_ld);
+}  // extern "C"
+
+namespace kfb {
+int apb_run(cudaStream_t stream, const ApbArgs& r) {
+  const int batch = r.batch, l = r.l, c = r.c, heads = r.heads, out_dtype = r.out_dtype, gate_share = r.gate_share;
+  const long long gate_ld = r.gate_ld;
+  void* workspace = r.workspace;
+  const size_t workspace_bytes = r.workspace_bytes;
   const int d = c / heads;
   KFB_CHECK_ARG(d % 8 == 0 && d >= 16 && d <= 64, "apb: head dim %d not in {16, 24, ..., 64}", d);
   if (out_dtype == KFB_FP32_PRECISE) {
@@ -559,10 +550,13 @@ KFB_API int kfb_apb_fwd(const void* x, const void* pair_bias, const unsigned cha
     const size_t need_p = carve_apb_precise(wp, workspace, batch, l, c);
     KFB_CHECK_ARG(workspace_bytes >= need_p, "apb: workspace %zu < %zu bytes", workspace_bytes, need_p);
     KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "apb: workspace must be 256-byte aligned");
-    cudaStream_t stream = as_stream(stream_);
     const long long rows = static_cast<long long>(batch) * l;
     const long long c6 = 6ll * c;
-    KFB_TRY(launch_layernorm_split(stream, static_cast<const float*>(x), wp.x6, nullptr, nullptr, rows, c, c, 0.f, 0));
+    const void* x6 = r.x;
+    if (!r.x_is_split) {
+      KFB_TRY(launch_layernorm_split(stream, static_cast<const float*>(r.x), wp.x6, nullptr, nullptr, rows, c, c, 0.f, 0));
+      x6 = wp.x6;
+    }
     {
       GemmParams p = {};
       p.n_extent = static_cast<int>(rows);
@@ -573,9 +567,9 @@ KFB_API int kfb_apb_fwd(const void* x, const void* pair_bias, const unsigned cha
       p.precise = 1;
       p.nseg = 1;
       p.seg[0] = row_major_seg(wp.qkgv, 4 * c, 4 * c, 0, 0, 1);
-      p.col_bias = proj_bias;
-      GemmOperandA a = {wp.x6, c6, 0, 0};
-      GemmOperandB b = {w_proj_packed, c6, 0};
+      p.col_bias = r.proj_bias;
+      GemmOperandA a = {x6, c6, 0, 0};
+      GemmOperandB b = {r.w_proj, c6, 0};
       KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "apb_proj_precise"));
     }
     {
@@ -588,9 +582,9 @@ KFB_API int kfb_apb_fwd(const void* x, const void* pair_bias, const unsigned cha
       p.q = p.k = p.v = p.g = wp.qkgv;
       p.ld = 4 * c;
       p.q_col0 = 0; p.k_col0 = c; p.g_col0 = 2 * c; p.v_col0 = 3 * c;
-      p.bias = static_cast<const float*>(pair_bias); p.ldb = l; p.bias_div = bias_div;
-      p.mask = mask;
-      p.mask_lo_extent = 1;
+      p.bias = static_cast<const float*>(r.pair_bias); p.ldb = r.ldb; p.bias_hs = r.bias_hs; p.bias_div = r.bias_div;
+      p.mask = r.mask;
+      p.mask_lo_extent = r.mask_share;
       p.m_hi = l;
       p.m_lo = 0;
       p.m_k = 1;
@@ -607,26 +601,25 @@ KFB_API int kfb_apb_fwd(const void* x, const void* pair_bias, const unsigned cha
     p.precise = 1;
     p.nseg = 1;
     const long long lc = static_cast<long long>(l) * c;
-    p.seg[0] = row_major_seg(out, c, c, lc, lc * gate_share, 1);
-    p.col_bias = out_bias;
-    p.resid = resid;
-    if (out_gate != nullptr) {
-      p.gate = static_cast<const __nv_bfloat16*>(out_gate);  // fp32 logits in this mode
+    p.seg[0] = row_major_seg(r.out, c, c, lc, lc * gate_share, 1);
+    p.col_bias = r.out_bias;
+    p.resid = r.resid;
+    if (r.out_gate != nullptr) {
+      p.gate = static_cast<const __nv_bfloat16*>(r.out_gate);  // fp32 logits in this mode
       p.g_col = 1;
       p.g_n = gate_ld;
       p.g_o = 0;
       p.g_b = l * gate_ld;
     }
     GemmOperandA a = {wp.og6, c6, l * c6, l * c6 * gate_share};
-    GemmOperandB b = {w_out, c6, 0};
+    GemmOperandB b = {r.w_out, c6, 0};
     return launch_gemm_bf16(stream, a, b, p, 0, "apb_out_proj_precise");
   }
-  const int dp = dpad_of(d), hdp = heads * dp;
+  const int dp = dpad_of(d), hdp = heads * dp, lv = pitch16(l);
   ApbWs w;
   const size_t need = carve_apb(w, workspace, batch, l, c, heads);
   KFB_CHECK_ARG(workspace_bytes >= need, "apb: workspace %zu < %zu bytes", workspace_bytes, need);
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "apb: workspace must be 256-byte aligned");
-  cudaStream_t stream = as_stream(stream_);
   {
     GemmParams p = {};
     p.n_extent = l;
@@ -641,12 +634,13 @@ KFB_API int kfb_apb_fwd(const void* x, const void* pair_bias, const unsigned cha
     sv.col_begin = 3 * hdp;
     sv.ncols = hdp;
     sv.dst = w.vt;
-    sv.s_col = l;
+    sv.s_col = lv;
     sv.s_n = 1;
-    sv.s_o = static_cast<long long>(hdp) * l;
-    p.col_bias = proj_bias;
-    GemmOperandA a = {x, c, static_cast<long long>(l) * c, 0};
-    GemmOperandB b = {w_proj_packed, c, 0};
+    sv.n_pad = lv;
+    sv.s_o = static_cast<long long>(hdp) * lv;
+    p.col_bias = r.proj_bias;
+    GemmOperandA a = {r.x, c, static_cast<long long>(l) * c, 0};
+    GemmOperandB b = {r.w_proj, c, 0};
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "apb_proj"));
   }
   {
@@ -660,10 +654,10 @@ KFB_API int kfb_apb_fwd(const void* x, const void* pair_bias, const unsigned cha
     p.q = w.qkg; p.ldq = 3 * hdp; p.q_col0 = 0;
     p.k = w.qkg; p.ldk = 3 * hdp; p.k_col0 = hdp;
     p.g = w.qkg; p.ldg = 3 * hdp; p.g_col0 = 2 * hdp;
-    p.vt = w.vt; p.ldv = l;
-    p.bias = pair_bias; p.ldb = l; p.bias_div = bias_div;
-    p.mask = mask;
-    p.mask_lo_extent = 1;
+    p.vt = w.vt; p.ldv = lv;
+    p.bias = r.pair_bias; p.ldb = r.ldb; p.bias_hs = r.bias_hs; p.bias_div = r.bias_div;
+    p.mask = r.mask;
+    p.mask_lo_extent = r.mask_share;
     p.m_hi = l;
     p.m_lo = 0;
     p.m_k = 1;
@@ -681,21 +675,54 @@ KFB_API int kfb_apb_fwd(const void* x, const void* pair_bias, const unsigned cha
     p.k_extent = c;
     p.nseg = 1;
     const long long lc = static_cast<long long>(l) * c;
-    p.seg[0] = row_major_seg(out, c, c, lc, lc * gate_share, out_dtype == KFB_FP32);
-    p.col_bias = out_bias;
-    p.resid = resid;
-    if (out_gate != nullptr) {
-      p.gate = static_cast<const __nv_bfloat16*>(out_gate);
+    p.seg[0] = row_major_seg(r.out, c, c, lc, lc * gate_share, out_dtype == KFB_FP32);
+    p.col_bias = r.out_bias;
+    p.resid = r.resid;
+    if (r.out_gate != nullptr) {
+      p.gate = static_cast<const __nv_bfloat16*>(r.out_gate);
       p.g_col = 1;
       p.g_n = gate_ld;
       p.g_o = 0;
       p.g_b = l * gate_ld;
     }
     GemmOperandA a = {w.og, c, lc, lc * gate_share};
-    GemmOperandB b = {w_out, c, 0};
+    GemmOperandB b = {r.w_out, c, 0};
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "apb_out_proj"));
   }
   return KFB_OK;
+}
+}  // namespace kfb
+
+extern "C" {
+
+KFB_API int kfb_apb_fwd(const void* x, const void* pair_bias, const unsigned char* mask, const void* w_proj_packed,
+                        const float* proj_bias, const void* w_out, const float* out_bias, const void* out_gate,
+                        int gate_share, long long gate_ld, void* out, const void* resid, void* workspace,
+                        size_t workspace_bytes, int batch, int l, int c, int heads, int bias_div, int out_dtype, void* stream_) {
+  KFB_CHECK_ARG(x && pair_bias && mask && w_proj_packed && w_out && out && workspace, "apb: null pointer");
+  KFB_CHECK_ARG(is_dtype(out_dtype), "apb: bad dtype %d", out_dtype);
+  KFB_CHECK_ARG(batch >= 1 && l >= 8 && l % 8 == 0, "apb: L=%d must be a positive multiple of 8 (pad in the caller)", l);
+  KFB_CHECK_ARG(heads >= 1 && c % heads == 0 && c % 8 == 0, "apb: c=%d heads=%d", c, heads);
+  KFB_CHECK_ARG(bias_div >= 1 && batch % bias_div == 0, "apb: batch %d not a multiple of bias_div %d", batch, bias_div);
+  if (out_gate != nullptr)
+    KFB_CHECK_ARG(gate_share >= 1 && batch % gate_share == 0, "apb: batch %d not a multiple of gate_share %d", batch, gate_share);
+  else
+    gate_share = 1;
+  if (gate_ld <= 0) gate_ld = c;
+  KFB_CHECK_ARG(gate_ld >= c, "apb: gate row stride %lld below c=%d", gate_ld, c);
+  KFB_CHECK_ARG(out_gate == nullptr || out_dtype == KFB_FP32_PRECISE || (gate_ld % 8 == 0 && (reinterpret_cast<uintptr_t>(out_gate) & 15) == 0),
+                "apb: bf16 gate rows must start on 16-byte boundaries (pointer and row stride %lld)", gate_ld);
+  ApbArgs r;
+  r.x = x;
+  r.pair_bias = pair_bias; r.ldb = l; r.bias_div = bias_div;
+  r.mask = mask;
+  r.w_proj = w_proj_packed; r.proj_bias = proj_bias;
+  r.w_out = w_out; r.out_bias = out_bias;
+  r.out_gate = out_gate; r.gate_share = gate_share; r.gate_ld = gate_ld;
+  r.out = out; r.resid = resid;
+  r.workspace = workspace; r.workspace_bytes = workspace_bytes;
+  r.batch = batch; r.l = l; r.c = c; r.heads = heads; r.out_dtype = out_dtype;
+  return apb_run(as_stream(stream_), r);
 }
 
 KFB_API size_t kfb_apb_cross_workspace_bytes(int batch, int lq, int lk, int c, int heads) {

@@ -84,11 +84,13 @@ KFB_API size_t kfb_cond_transition_workspace_bytes(long long rows, int hidden) {
   return align_up(static_cast<size_t>(rows) * hidden * sizeof(__nv_bfloat16), 256);
 }
 
+}  // extern "C"
+
 // out = sigmoid(gate[s(r)]) * (silu(u_a) * u_b) W_out^T  (+ resid),  [u_a, u_b] = x W_swiglu^T,  x already AdaLN-normalised
-KFB_API int kfb_cond_transition_fwd(const void* x_normed, const void* w_swiglu_packed, const void* w_out,
-                                    const void* out_gate, long long gate_ld, void* out, const void* resid, void* workspace,
-                                    size_t workspace_bytes, long long rows, int c, int hidden, int samples, int l, int dtype,
-                                    void* stream_) {
+namespace kfb {
+int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_split, const void* w_swiglu_packed, const void* w_out,
+                        const void* out_gate, long long gate_ld, void* out, const void* resid, void* workspace,
+                        size_t workspace_bytes, long long rows, int c, int hidden, int samples, int l, int dtype) {
   KFB_CHECK_ARG(x_normed && w_swiglu_packed && w_out && out_gate && out && workspace, "cond_transition: null pointer");
   if (gate_ld <= 0) gate_ld = c;
   KFB_CHECK_ARG(gate_ld >= c, "cond_transition: gate row stride %lld below c=%d", gate_ld, c);
@@ -99,7 +101,6 @@ KFB_API int kfb_cond_transition_fwd(const void* x_normed, const void* w_swiglu_p
                 "cond_transition: rows %lld samples %d l %d", rows, samples, l);
   KFB_CHECK_ARG(c % 8 == 0 && hidden % 128 == 0, "cond_transition: c=%d (multiple of 8), hidden=%d (multiple of 128)", c, hidden);
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "cond_transition: workspace must be 256-byte aligned");
-  cudaStream_t stream = as_stream(stream_);
   if (dtype == KFB_FP32_PRECISE) {
     // x_normed, out_gate (logits), out and resid are fp32; the weights are bf16 triple splits
     KFB_CHECK_ARG(workspace_bytes >= kfb_cond_transition_workspace_bytes_precise(rows, c, hidden),
@@ -107,7 +108,11 @@ KFB_API int kfb_cond_transition_fwd(const void* x_normed, const void* w_swiglu_p
     Carver cv(workspace);
     __nv_bfloat16* x6 = cv.take<__nv_bfloat16>(static_cast<size_t>(rows) * 6 * c);
     __nv_bfloat16* h6 = cv.take<__nv_bfloat16>(static_cast<size_t>(rows) * 6 * hidden);
-    KFB_TRY(launch_layernorm_split(stream, static_cast<const float*>(x_normed), x6, nullptr, nullptr, rows, c, c, 0.f, 0));
+    const void* xs = x_normed;
+    if (!x_is_split) {
+      KFB_TRY(launch_layernorm_split(stream, static_cast<const float*>(x_normed), x6, nullptr, nullptr, rows, c, c, 0.f, 0));
+      xs = x6;
+    }
     {
       GemmParams p = {};
       p.n_extent = static_cast<int>(rows);
@@ -122,7 +127,7 @@ KFB_API int kfb_cond_transition_fwd(const void* x_normed, const void* w_swiglu_p
       p.seg[0].vec = 0;
       p.seg[0].split = 1;
       p.seg[0].s_part = hidden;
-      GemmOperandA a = {x6, 6ll * c, 0, 0};
+      GemmOperandA a = {xs, 6ll * c, 0, 0};
       GemmOperandB b = {w_swiglu_packed, 6ll * c, 0};
       KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "cond_transition_swiglu_precise"));
     }
@@ -185,6 +190,17 @@ KFB_API int kfb_cond_transition_fwd(const void* x_normed, const void* w_swiglu_p
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "cond_transition_out"));
   }
   return KFB_OK;
+}
+}  // namespace kfb
+
+extern "C" {
+
+KFB_API int kfb_cond_transition_fwd(const void* x_normed, const void* w_swiglu_packed, const void* w_out,
+                                    const void* out_gate, long long gate_ld, void* out, const void* resid, void* workspace,
+                                    size_t workspace_bytes, long long rows, int c, int hidden, int samples, int l, int dtype,
+                                    void* stream_) {
+  return cond_transition_run(as_stream(stream_), x_normed, 0, w_swiglu_packed, w_out, out_gate, gate_ld, out, resid, workspace,
+                             workspace_bytes, rows, c, hidden, samples, l, dtype);
 }
 
 KFB_API int kfb_window_bias_fwd(const void* z, const float* ln_w, const float* ln_b, const void* w, void* bias_out,

@@ -40,4 +40,31 @@ inline EpiSeg row_major_seg(void* dst, int ncols, long long ld, long long s_o, l
   return s;
 }
 
+// Pitch of rows of l positions that TMA maps read or the epilogues store channel-major: whole 32-byte sectors.
+inline int pitch16(int l) { return (l + 15) / 16 * 16; }
+
+// Gated pair-bias self-attention on normalised rows (kfb_apb_fwd and the stacks; see include/kfold_b200.h).
+struct ApbArgs {
+  const void* x = nullptr;            // bf16 (batch, l, c); precise: fp32, or its triple split when x_is_split
+  int x_is_split = 0;
+  const void* pair_bias = nullptr;    // [batch / bias_div][heads][l][ldb], head planes bias_hs elements apart (0: l * ldb)
+  long long ldb = 0, bias_hs = 0;
+  int bias_div = 1;
+  const unsigned char* mask = nullptr;  // [batch / mask_share][l]
+  int mask_share = 1;
+  const void* w_proj = nullptr; const float* proj_bias = nullptr;
+  const void* w_out = nullptr; const float* out_bias = nullptr;
+  const void* out_gate = nullptr; int gate_share = 1; long long gate_ld = 0;
+  void* out = nullptr; const void* resid = nullptr;
+  void* workspace = nullptr; size_t workspace_bytes = 0;
+  int batch = 0, l = 0, c = 0, heads = 0, out_dtype = 0;
+};
+int apb_run(cudaStream_t stream, const ApbArgs& r);
+
+// Conditioned transition on AdaLN-normalised rows (kfb_cond_transition_fwd and the stacks).  x_is_split: precise mode, x is
+// already the triple split.
+int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_split, const void* w_swiglu, const void* w_out,
+                        const void* out_gate, long long gate_ld, void* out, const void* resid, void* workspace,
+                        size_t workspace_bytes, long long rows, int c, int hidden, int samples, int l, int dtype);
+
 }  // namespace kfb

@@ -16,7 +16,7 @@ _workspaces: dict = {}
 
 
 def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
-    key = (device.index, torch.cuda.current_stream(device).cuda_stream)
+    key = (device.index, L.raw_stream(device.index))
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
         ws = None
@@ -317,6 +317,53 @@ def attention_pair_bias(x: torch.Tensor, pair_bias: torch.Tensor, mask: torch.Te
                                 gate_share, gate_ld, L.ptr(out), L.ptr(res), L.ptr(ws), ws.numel(), batch, lp, c, heads, bias_div,
                                 L.KFB_FP32_PRECISE if precise else L.dtype_code(out.dtype), L.stream_ptr()))
     return out[:, :l].reshape(*lead, l, c).to(want)
+
+
+def token_stack(a: torch.Tensor, s: torch.Tensor, pair_bias: torch.Tensor, mask: torch.Tensor, plan, groups: int, samples: int,
+                s_samples: int, heads: int, hidden: int, precise: bool, eps: float = 1e-5) -> torch.Tensor:
+    """The blocks of CachedGlobalTransformerStack in one native call (model/layers/folding/diffusion_transformer.py:260-413).
+    a (groups * samples, L, c) flattened; s (groups * s_samples, L, c_s); pair_bias (blocks, groups, ..., H, L, L) in the compute
+    dtype with rows at a pitch of eights; mask (groups, L); `plan`: the stack's packed weights."""
+    _require_cuda(a, s, pair_bias, mask)
+    l, c = a.shape[-2:]
+    ac = (a.float() if precise else a).contiguous()
+    sc = (s.float() if precise or s.dtype not in (torch.bfloat16, torch.float32) else s).contiguous()
+    mk = mask.to(torch.bool).contiguous()
+    out = torch.empty_like(ac)
+    st = pair_bias.stride()
+    lib = L.lib()
+    with L.on_device(a.device):
+        need = lib.kfb_token_stack_workspace_bytes(groups, samples, s_samples, l, c, plan.c_s, heads, hidden, plan.gs_cols, plan.og_cols,
+                                                   precise)
+        ws = _workspace(a.device, need)
+        L.check(lib.kfb_token_stack_fwd(plan.blocks, len(plan.blocks), L.ref(plan.cond), L.ptr(ac), L.ptr(out), L.dtype_code(ac.dtype),
+                                        L.ptr(sc), L.dtype_code(sc.dtype), L.ptr(pair_bias), st[0], st[-3], st[-2], L.ptr(mk), L.ptr(ws),
+                                        ws.numel(), groups, samples, s_samples, l, c, heads, hidden, eps, precise, L.stream_ptr()))
+    return out.to(a.dtype) if precise else out
+
+
+def atom_stack(a: torch.Tensor, s: torch.Tensor, window_biases: torch.Tensor, mask: torch.Tensor, plan, groups: int, bias_share: int,
+               heads: int, hidden: int, eps: float = 1e-5) -> torch.Tensor:
+    """The blocks of LocalTransformerStack in one native call (diffusion_transformer.py:419-512), bfloat16 compute, head dim <= 32:
+    a (groups * samples, L, c) flattened, s (groups, L, c_s), window_biases (blocks * H, windows, 32, 128) bf16, mask (batch //
+    mask share, L)."""
+    _require_cuda(a, s, window_biases, mask)
+    l, c = a.shape[-2:]
+    batch = a.numel() // (l * c)
+    ac = a.contiguous()
+    sc = (s if s.dtype in (torch.bfloat16, torch.float32) else s.float()).contiguous()
+    mk = mask.to(torch.bool).contiguous()
+    out = torch.empty_like(ac)
+    nbb = window_biases.numel() // (len(plan.blocks) * heads * 4096)
+    samples = batch // groups
+    lib = L.lib()
+    with L.on_device(a.device):
+        need = lib.kfb_atom_stack_workspace_bytes(groups, samples, l, c, plan.c_s, heads, hidden, plan.gs_cols, plan.og_cols)
+        ws = _workspace(a.device, need)
+        L.check(lib.kfb_atom_stack_fwd(plan.blocks, len(plan.blocks), L.ref(plan.cond), L.ptr(ac), L.ptr(out), L.dtype_code(ac.dtype),
+                                       L.ptr(sc), L.dtype_code(sc.dtype), L.ptr(window_biases), nbb, L.ptr(mk), batch // mk.shape[0],
+                                       bias_share, L.ptr(ws), ws.numel(), groups, samples, l, c, heads, hidden, eps, L.stream_ptr()))
+    return out
 
 
 def window_bias(z: torch.Tensor, ln_w: torch.Tensor | None, ln_b: torch.Tensor | None, w: torch.Tensor,

@@ -32,15 +32,22 @@ class GraphedCall:
         self._inputs = [t.clone() for t in example_inputs]
         dev = example_inputs[0].device
         with torch.cuda.device(dev), torch.no_grad():
-            side = torch.cuda.Stream()
-            side.wait_stream(torch.cuda.current_stream())
+            # Warm-up and capture on one side stream.  torch.cuda.graph() would collect Python garbage and return the
+            # allocator's cached blocks to the driver first; with a model of a few hundred parameters in memory that is
+            # 0.1 s and more, and every later allocation pays for it again, so the capture is begun and ended directly.
+            current, side = torch.cuda.current_stream(), torch.cuda.Stream()
+            side.wait_stream(current)
             with torch.cuda.stream(side):          # warm-up outside the capture: weight packing, workspace allocation
                 for _ in range(max(warmup, 1)):
                     fn(*self._inputs)
-            torch.cuda.current_stream().wait_stream(side)
-            self._graph = torch.cuda.CUDAGraph()
-            with torch.cuda.graph(self._graph):
-                self._output = fn(*self._inputs)
+                side.synchronize()
+                self._graph = torch.cuda.CUDAGraph()
+                self._graph.capture_begin()
+                try:
+                    self._output = fn(*self._inputs)
+                finally:
+                    self._graph.capture_end()
+            current.wait_stream(side)
 
     def __call__(self, *inputs: torch.Tensor):
         if len(inputs) != len(self._inputs):

@@ -25,7 +25,9 @@ import torch
 from torch import nn
 
 from . import functional as F
+from . import _lib as L
 from . import packing
+from .plans import ParamState
 
 __all__ = [
     "LayerNorm", "LinearNoBias", "Linear",
@@ -117,14 +119,14 @@ class _PackedMixin:
 
     _pack_cache = None
     _pack_key = None
+    _pack_state = None
 
     def _packed(self, device: torch.device, dtype: torch.dtype, pack_fn):
-        key = (device.type, device.index, dtype) + tuple(
-            v for p in self.parameters() for v in (p.data_ptr(), None if torch.is_inference(p) else p._version))
-        if self._pack_cache is None or self._pack_key != key:
+        key = (device, dtype)
+        if self._pack_cache is None or self._pack_key != key or not self._pack_state.current():
             sd = {k: v for k, v in self.state_dict().items()}
             self._pack_cache = pack_fn(sd, device)
-            self._pack_key = key
+            self._pack_key, self._pack_state = key, ParamState(self)
         return self._pack_cache
 
 
@@ -281,27 +283,32 @@ class _ConditioningBank:
     gates Linear(s).  All of them depend on s alone, so the stack normalises s once (the per-AdaLN scale is folded into
     that AdaLN's weight columns), multiplies once by all stacked AdaLN matrices and once by all stacked gate matrices,
     and every block reads its columns of the two wide tables in place (the kernels take a row stride).
-    bfloat16 compute only: folding the scale moves a bf16 rounding, which the float32-accurate path must not do."""
+    In the float32-accurate mode the scale is folded in float32 before the matrices are split."""
 
     def __init__(self):
         self._key = None
         self._packed = None
+
+    @staticmethod
+    def pack(adalns, gates, device, precise: bool = False):
+        """(w_gs, b_gs, w_og, b_og): the stacked matrices in bf16 (or as bf16 triple splits) and their float32 biases."""
+        f = lambda t: t.detach().to(device, torch.float32)
+        w1, b1 = [], []
+        for m in adalns:
+            gamma = f(m.layernorm_s.weight)[None, :]
+            w1 += [f(m.linear_g.weight) * gamma, f(m.linear_bias.weight) * gamma]
+            b1 += [f(m.linear_g.bias), torch.zeros_like(m.linear_g.bias, dtype=torch.float32, device=device)]
+        w2 = [f(g.weight) for g in gates]
+        b2 = [f(g.bias) for g in gates]
+        fix = packing.split3_weights if precise else (lambda t: t.to(torch.bfloat16).contiguous())
+        return fix(torch.cat(w1)), torch.cat(b1).contiguous(), fix(torch.cat(w2)), torch.cat(b2).contiguous()
 
     def _pack(self, adalns, gates, device):
         params = [p for m in adalns for p in (m.layernorm_s.weight, m.linear_g.weight, m.linear_g.bias, m.linear_bias.weight)]
         params += [p for g in gates for p in (g.weight, g.bias)]
         key = (device,) + tuple(v for p in params for v in (p.data_ptr(), None if torch.is_inference(p) else p._version))
         if self._key != key:
-            w1, b1 = [], []
-            for m in adalns:
-                gamma = m.layernorm_s.weight.detach().float()[None, :]
-                w1 += [m.linear_g.weight.detach().float() * gamma, m.linear_bias.weight.detach().float() * gamma]
-                b1 += [m.linear_g.bias.detach().float(), torch.zeros_like(m.linear_g.bias, dtype=torch.float32)]
-            w2 = [g.weight.detach().float() for g in gates]
-            b2 = [g.bias.detach().float() for g in gates]
-            bf = torch.bfloat16
-            self._packed = (torch.cat(w1).to(device, bf).contiguous(), torch.cat(b1).to(device).contiguous(),
-                            torch.cat(w2).to(device, bf).contiguous(), torch.cat(b2).to(device).contiguous())
+            self._packed = self.pack(adalns, gates, device)
             self._key = key
         return self._packed
 
@@ -321,6 +328,28 @@ class _ConditioningBank:
             og.append(t2[..., off: off + g.weight.shape[0]])
             off += g.weight.shape[0]
         return gs, og
+
+
+class _StackPlan:
+    """The packed weights of a whole stack as the structs the native stack calls take; `state` tells when they are stale."""
+
+    def __init__(self, root: nn.Module, blocks: list, block_type, adalns: list, gates: list, device, precise: bool):
+        self.key, self.state = (device, precise), ParamState(root)
+        self.keep = []                               # the packed tensors behind the pointers
+        self.blocks = (block_type * len(blocks))()
+        for dst, fields in zip(self.blocks, blocks):
+            for name, t in fields.items():
+                setattr(dst, name, L.ptr(t))
+                self.keep.append(t)
+        w_gs, b_gs, w_og, b_og = _ConditioningBank.pack(adalns, gates, device, precise)
+        self.keep += [w_gs, b_gs, w_og, b_og]
+        self.c_s = adalns[0].channel_s
+        self.gs_cols, self.og_cols = w_gs.shape[0], w_og.shape[0]
+        self.cond = L.Conditioning(L.ptr(w_gs), L.ptr(b_gs), L.ptr(w_og), L.ptr(b_og), self.gs_cols, self.og_cols, self.c_s,
+                                   adalns[0].layernorm_s.eps)
+
+    def fits(self, device, precise: bool) -> bool:
+        return self.key == (device, precise) and self.state.current()
 
 
 class SelfAttentionPairBias(nn.Module, _PackedMixin):
@@ -412,10 +441,15 @@ class ConditionedTransitionBlock(nn.Module, _PackedMixin):
     def __init__(self, channel_a: int, channel_s: int, expansion_factor: int = 2):
         super().__init__()
         model_dim = int(channel_a * expansion_factor)
+        self.hidden = model_dim
         self.adaln = AdaLN(channel_a, channel_s)
         self.swiglu = _SwiGLU(channel_a, model_dim)
         self.linear_g = Linear(channel_s, channel_a)
         self.linear_out = LinearNoBias(model_dim, channel_a)
+
+    def _packed_transition(self, device, precise: bool):
+        return self._packed(device, torch.float32 if precise else torch.bfloat16,
+                            lambda sd, dev: packing.pack_cond_transition(sd, dev, precise=precise))
 
     @torch.compiler.disable
     def forward(self, a: torch.Tensor, s: torch.Tensor, residual: bool = False, precise: bool | None = None,
@@ -425,8 +459,7 @@ class ConditionedTransitionBlock(nn.Module, _PackedMixin):
         _check_inference(a)
         if precise is None:
             precise = _is_precise(compute_dtype(a), "ConditionedTransitionBlock")
-        pk = self._packed(a.device, torch.float32 if precise else torch.bfloat16,
-                          lambda sd, dev: packing.pack_cond_transition(sd, dev, precise=precise))
+        pk = self._packed_transition(a.device, precise)
         with torch.autocast(a.device.type, enabled=False):
             share = _sample_share(a, s)
             if precise:
@@ -545,19 +578,35 @@ class CachedGlobalTransformerStack(nn.Module):
         self._bias_cache = None
         self._bias_key = None
         self._bias_src = None
-        self._bank = _ConditioningBank()
+        self._plan = None
 
     def _prepared_bias(self, pair_bias: torch.Tensor, precise: bool = False):
-        key = _tensor_key(pair_bias) + (precise,)
+        """(*, N, H, L, L) with the N blocks in front, in the compute dtype, rows at a pitch of a multiple of eight elements
+        (what the attention kernel's tensor maps take).  A bias that already lies so is used in place."""
+        key = _tensor_key(pair_bias) + (pair_bias.stride(), precise)
         if self._bias_key != key:
-            # (*, N, H, L, L) -> N tensors (*, H, L, L), contiguous: bf16 for the tensor-core kernel, float32 for the
-            # fp32-accurate one
-            pb = pair_bias.movedim(-4, 0).to(torch.float32 if precise else torch.bfloat16).contiguous()
+            pb, dt = pair_bias.movedim(-4, 0), torch.float32 if precise else torch.bfloat16
+            l = pb.shape[-1]
+            if pb.dtype != dt or not _bias_in_place(pb):
+                padded = pb.new_zeros(*pb.shape[:-1], (l + 7) // 8 * 8, dtype=dt)
+                padded[..., :l] = pb
+                pb = padded[..., :l]
             self._bias_cache, self._bias_key = pb, key
             # the conversion may have copied: keep the source alive, so that its address cannot be handed to the bias of
             # the next complex (same shape, version 0) while this entry is still in the cache
             self._bias_src = pair_bias
         return self._bias_cache
+
+    def _plan_for(self, device, precise: bool) -> "_StackPlan":
+        if self._plan is None or not self._plan.fits(device, precise):
+            blocks = []
+            for b in self.blocks:
+                pa, pt = b.attention._apb_packed(device, precise), b.transition._packed_transition(device, precise)
+                blocks.append({"w_proj": pa["w_proj"], "proj_bias": pa["proj_bias"], "w_out": pa["w_out"], "out_bias": pa["out_bias"],
+                               "w_swiglu": pt["w_swiglu"], "w_tout": pt["w_out"]})
+            self._plan = _StackPlan(self, blocks, L.TokenBlock, [m for b in self.blocks for m in (b.attention.adaln_a, b.transition.adaln)],
+                                    [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)], device, precise)
+        return self._plan
 
     def reset_caches(self) -> None:
         """Forget the converted pair bias (call once per complex when the bias tensor is overwritten in place under
@@ -569,16 +618,54 @@ class CachedGlobalTransformerStack(nn.Module):
         _check_inference(a)
         precise = _is_precise(compute_dtype(a), "CachedGlobalTransformerStack")
         pb = self._prepared_bias(pair_bias, precise)
-        conds = [None] * len(self.blocks)
-        if not precise:
-            # the conditioning projections of all blocks: one LayerNorm of s and two GEMMs
-            with torch.autocast(a.device.type, enabled=False):
-                gs, og = self._bank.tables(s, [m for b in self.blocks for m in (b.attention.adaln_a, b.transition.adaln)],
-                                           [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)])
-            conds = [((gs[2 * i], og[2 * i]), (gs[2 * i + 1], og[2 * i + 1])) for i in range(len(self.blocks))]
+        lead = tuple(a.shape[:-2])
+        # (groups, samples): the samples share bias, mask and usually the conditioning
+        groups, samples = _group_samples(lead, tuple(pb.shape[1:-3]), tuple(mask.shape[:-1]))
+        s_lead = tuple(s.shape[:-2])
+        s_samples = 1 if samples == 1 or _leading(s_lead) == groups else samples
+        with torch.autocast(a.device.type, enabled=False):
+            if groups and _leading(s_lead) == groups * s_samples and self.blocks[0].attention.use_single_conditioning:
+                return F.token_stack(a, s, pb, mask, self._plan_for(a.device, precise), groups, samples, s_samples,
+                                     self.blocks[0].attention.num_heads, self.blocks[0].transition.hidden, precise)
+        # biases, masks or conditionings shared in some other pattern: one block at a time
         for i, blk in enumerate(self.blocks):
-            a = blk(a, s, pb[i], mask, cond=conds[i])
+            a = blk(a, s, pb[i], mask)
         return a
+
+
+def _leading(lead: tuple) -> int:
+    n = 1
+    for d in lead:
+        n *= d
+    return n
+
+
+def _bias_in_place(pb: torch.Tensor) -> bool:
+    """Whether a bias (N, ..., H, L, L) is addressed by one block stride, one head-plane stride and a row pitch of eights."""
+    st, sh = pb.stride(), pb.shape
+    if st[-1] != 1 or st[-2] % 8 or st[-3] % 8 or st[0] % 8 or pb.data_ptr() % 16:
+        return False
+    plane = st[-3]
+    span = plane * sh[-3]
+    for d in range(pb.dim() - 4, 0, -1):
+        if sh[d] != 1:
+            if st[d] != span:
+                return False
+            span *= sh[d]
+    return plane >= st[-2] * sh[-2]
+
+
+def _group_samples(lead: tuple, bias_lead: tuple, mask_lead: tuple):
+    """(groups, samples) of a batch with leading dims `lead` whose bias and mask are shared by the trailing (sample) dims, or
+    (0, 0) for another pattern.  Leading 1s may be missing from the bias' and the mask's dims."""
+    fill = lambda t: (1,) * (len(lead) - len(t)) + t
+    bias_lead, mask_lead = fill(bias_lead), fill(mask_lead)
+    k = len(lead)
+    while k > 0 and bias_lead[k - 1] == 1 and mask_lead[k - 1] == 1:
+        k -= 1
+    if bias_lead[:k] != lead[:k] or mask_lead[:k] != lead[:k]:
+        return 0, 0
+    return _leading(lead[:k]), _leading(lead[k:])
 
 
 # --------------------------------------------------------------------------------------------
@@ -772,6 +859,7 @@ class LocalTransformerStack(nn.Module):
         self._bias_all = None
         self._bias_all_key = None
         self._bias_all_src = None
+        self._plan = None
         self._bank = _ConditioningBank()
 
     def _stacked_bias_weights(self, device, dt):
@@ -796,6 +884,18 @@ class LocalTransformerStack(nn.Module):
             self._bias_all_key = key
             self._bias_all_src = z          # keeps z's storage alive so that its address cannot be reused
         return self._bias_all
+
+    def _plan_for(self, device) -> _StackPlan:
+        if self._plan is None or not self._plan.fits(device, False):
+            blocks = []
+            for b in self.blocks:
+                pa, pt = b.attention._cross_packed(device), b.transition._packed_transition(device, False)
+                blocks.append({"w_q": pa["w_q"], "q_bias": pa["q_bias"], "w_kv": pa["w_kv"], "w_out": pa["w_out"], "out_bias": pa["out_bias"],
+                               "w_swiglu": pt["w_swiglu"], "w_tout": pt["w_out"]})
+            self._plan = _StackPlan(self, blocks, L.AtomBlock,
+                                    [m for b in self.blocks for m in (b.attention.adaln_a_q, b.attention.adaln_a_k, b.transition.adaln)],
+                                    [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)], device, False)
+        return self._plan
 
     def reset_caches(self) -> None:
         """Forget the window biases (see CachedGlobalTransformerStack.reset_caches)."""
@@ -826,6 +926,13 @@ class LocalTransformerStack(nn.Module):
                     batch *= dd
                 bias_share = _index_share(lead, tuple(z.shape[:-4]))
                 mask2 = mask.to(torch.bool).reshape(-1, length)
+                # conditioning shared by the samples, window biases and mask shared inside each group: one native call
+                groups = _leading(tuple(s.shape[:-2]))
+                if (self.blocks[0].attention.use_single_conditioning and batch % groups == 0
+                        and _index_share(lead, tuple(s.shape[:-2])) == batch // groups
+                        and (batch // groups) % bias_share == 0 and (batch // groups) % (batch // mask2.shape[0]) == 0):
+                    return F.atom_stack(a, s, bias_all, mask2, self._plan_for(a.device), groups, bias_share, h,
+                                        self.blocks[0].transition.hidden)
                 bias_all = bias_all.reshape(len(self.blocks), h, -1, WINDOW_Q, WINDOW_K)
             else:
                 to_qk = build_atom_to_qk_fn(length, a.device)

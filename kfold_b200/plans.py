@@ -1,0 +1,47 @@
+"""What a module keeps between calls: its packed weights, and a cheap way to see whether they are still those of its parameters.
+
+A forward call has to notice a parameter that was replaced, moved or changed in place (``load_state_dict``, ``.to(device)``, an
+optimiser step), but walking ``module.parameters()`` of a 24-block stack costs more host time than launching its kernels does.
+`ParamState` remembers where the parameters live (the modules' own dictionaries) and reads their addresses and versions from
+there: about 0.15 us per parameter.
+"""
+from __future__ import annotations
+
+__all__ = ["ParamState"]
+
+
+def _version(p):
+    try:
+        return p._version
+    except RuntimeError:      # inference tensors carry no version counter
+        return None
+
+
+class ParamState:
+    """Addresses and in-place versions of every parameter below `modules`, as they were when this was made."""
+
+    __slots__ = ("_slots", "_children", "_seen")
+
+    def __init__(self, *modules):
+        self._slots, self._children = [], []
+        for root in modules:
+            for m in root.modules():
+                self._slots += [(m._parameters, name) for name, p in m._parameters.items() if p is not None]
+                self._children += [(m._modules, name, child) for name, child in m._modules.items()]
+        self._seen = self._read()
+
+    def _read(self):
+        ps = [d.get(name) for d, name in self._slots]
+        try:
+            return [(p.data_ptr(), p._version) for p in ps]
+        except RuntimeError:
+            return [(p.data_ptr(), _version(p)) for p in ps]
+        except AttributeError:      # a parameter was removed
+            return None
+
+    def current(self) -> bool:
+        """Whether nothing changed since."""
+        for d, name, child in self._children:
+            if d.get(name) is not child:
+                return False
+        return self._read() == self._seen
