@@ -27,6 +27,7 @@ template <typename TX, typename TO>
 __global__ void __launch_bounds__(256) tokens_to_atoms_kernel(const TX* __restrict__ x, const long long* __restrict__ index,
                                                               const TO* __restrict__ addend, TO* __restrict__ out, long long rows,
                                                               int n_atom, int n_token, int d, int index_div) {
+  grid_dependency_enter();
   const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -56,6 +57,7 @@ template <typename TQ>
 __global__ void __launch_bounds__(256) coord_embed_kernel(const TQ* __restrict__ q, const float* __restrict__ r,
                                                           const float* __restrict__ w, const unsigned char* __restrict__ mask,
                                                           float* __restrict__ out, long long rows, int c, int kc, int samples, int l) {
+  grid_dependency_enter();
   const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -77,6 +79,7 @@ __global__ void __launch_bounds__(256) ln_project_kernel(const T* __restrict__ x
                                                          const float* __restrict__ ln_b, const float* __restrict__ w,
                                                          const unsigned char* __restrict__ mask, float* __restrict__ out,
                                                          long long rows, int c, int n_out, float eps, int samples, int l) {
+  grid_dependency_enter();
   const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -114,11 +117,13 @@ __global__ void __launch_bounds__(256) ln_project_kernel(const T* __restrict__ x
 // then scans only that range; it still tests every atom in it, so unsorted indices stay correct, and for the usual
 // sorted atom order the range is just the token's own atoms.
 __global__ void __launch_bounds__(256) token_range_init_kernel(int2* __restrict__ range, long long n) {
+  grid_dependency_enter();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) range[i] = make_int2(0x7fffffff, -1);
 }
 __global__ void __launch_bounds__(256) token_range_kernel(const long long* __restrict__ index, const unsigned char* __restrict__ mask,
                                                           int2* __restrict__ range, long long total, int n_atom, int n_token) {
+  grid_dependency_enter();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= total) return;
   const long long t = index[i];
@@ -138,6 +143,7 @@ __global__ void __launch_bounds__(256) atoms_to_tokens_kernel(const T* __restric
                                                               const unsigned char* __restrict__ mask, T* __restrict__ out,
                                                               long long rows, int n_atom, int n_token, int d, int index_div,
                                                               int relu, const int2* __restrict__ range) {
+  grid_dependency_enter();
   const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
   const int lane = threadIdx.x & 31;
@@ -206,16 +212,17 @@ KFB_API int kfb_tokens_to_atoms(const void* x, const long long* token_index, con
   LaunchScope scope(stream, "tokens_to_atoms");
   using bf = __nv_bfloat16;
   if (x_dtype == KFB_BF16 && out_dtype == KFB_BF16)
-    tokens_to_atoms_kernel<bf, bf><<<blocks, 256, 0, stream>>>(static_cast<const bf*>(x), token_index, static_cast<const bf*>(addend),
-                                                               static_cast<bf*>(out), rows, n_atom, n_token, d, index_div);
+    KFB_TRY(launch_kernel(stream, tokens_to_atoms_kernel<bf, bf>, blocks, 256, 0, static_cast<const bf*>(x), token_index,
+        static_cast<const bf*>(addend),
+                                                               static_cast<bf*>(out), rows, n_atom, n_token, d, index_div));
   else if (x_dtype == KFB_BF16)
-    tokens_to_atoms_kernel<bf, float><<<blocks, 256, 0, stream>>>(static_cast<const bf*>(x), token_index,
+    KFB_TRY(launch_kernel(stream, tokens_to_atoms_kernel<bf, float>, blocks, 256, 0, static_cast<const bf*>(x), token_index,
                                                                   static_cast<const float*>(addend), static_cast<float*>(out), rows,
-                                                                  n_atom, n_token, d, index_div);
+                                                                  n_atom, n_token, d, index_div));
   else
-    tokens_to_atoms_kernel<float, float><<<blocks, 256, 0, stream>>>(static_cast<const float*>(x), token_index,
+    KFB_TRY(launch_kernel(stream, tokens_to_atoms_kernel<float, float>, blocks, 256, 0, static_cast<const float*>(x), token_index,
                                                                      static_cast<const float*>(addend), static_cast<float*>(out),
-                                                                     rows, n_atom, n_token, d, index_div);
+                                                                     rows, n_atom, n_token, d, index_div));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -242,19 +249,23 @@ KFB_API int kfb_atoms_to_tokens(const void* x, const long long* token_index, con
     range = static_cast<int2*>(workspace);
     const long long nr = static_cast<long long>(batch / index_div) * n_token, na = static_cast<long long>(batch / index_div) * n_atom;
     LaunchScope scope_r(stream, "atoms_to_tokens_ranges");
-    token_range_init_kernel<<<static_cast<unsigned>((nr + 255) / 256), 256, 0, stream>>>(range, nr);
-    token_range_kernel<<<static_cast<unsigned>((na + 255) / 256), 256, 0, stream>>>(token_index, mask, range, na, n_atom, n_token);
+    KFB_TRY(launch_kernel(stream, token_range_init_kernel, static_cast<unsigned>((nr + 255) / 256), 256, 0, range, nr));
+    KFB_TRY(launch_kernel(stream, token_range_kernel, static_cast<unsigned>((na + 255) / 256), 256, 0, token_index, mask,
+        range, na, n_atom, n_token));
     KFB_CUDA(cudaGetLastError());
   }
   LaunchScope scope(stream, "atoms_to_tokens");
   if (dtype == KFB_BF16)
-    atoms_to_tokens_kernel<__nv_bfloat16, 8><<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), token_index, mask,
-                                                                          static_cast<__nv_bfloat16*>(out), rows, n_atom, n_token, d,
-                                                                          index_div, relu, range);
+    KFB_TRY(launch_kernel(stream, atoms_to_tokens_kernel<__nv_bfloat16, 8>, blocks, 256, 0,
+        static_cast<const __nv_bfloat16*>(x), token_index, mask,
+                                                                          static_cast<__nv_bfloat16*>(out), rows, n_atom,
+                                                                          n_token, d,
+                                                                          index_div, relu, range));
   else
-    atoms_to_tokens_kernel<float, 8><<<blocks, 256, 0, stream>>>(static_cast<const float*>(x), token_index, mask,
-                                                                  static_cast<float*>(out), rows, n_atom, n_token, d, index_div, relu,
-                                                                  range);
+    KFB_TRY(launch_kernel(stream, atoms_to_tokens_kernel<float, 8>, blocks, 256, 0, static_cast<const float*>(x), token_index, mask,
+                                                                  static_cast<float*>(out), rows, n_atom, n_token, d,
+                                                                  index_div, relu,
+                                                                  range));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -270,10 +281,12 @@ KFB_API int kfb_coord_embed(const void* q, const float* r, const float* w, const
   const unsigned blocks = static_cast<unsigned>((rows + 7) / 8);
   LaunchScope scope(stream, "coord_embed");
   if (q_dtype == KFB_BF16)
-    coord_embed_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(q), r, w, mask, out, rows, c, kc,
-                                                                   samples, l);
+    KFB_TRY(launch_kernel(stream, coord_embed_kernel<__nv_bfloat16>, blocks, 256, 0, static_cast<const __nv_bfloat16*>(q), r,
+        w, mask, out, rows, c, kc,
+                                                                   samples, l));
   else
-    coord_embed_kernel<float><<<blocks, 256, 0, stream>>>(static_cast<const float*>(q), r, w, mask, out, rows, c, kc, samples, l);
+    KFB_TRY(launch_kernel(stream, coord_embed_kernel<float>, blocks, 256, 0, static_cast<const float*>(q), r, w, mask, out,
+        rows, c, kc, samples, l));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -290,11 +303,13 @@ KFB_API int kfb_ln_project(const void* x, const float* ln_w, const float* ln_b, 
   const unsigned blocks = static_cast<unsigned>((rows + 7) / 8);
   LaunchScope scope(stream, "ln_project");
   if (dtype == KFB_BF16)
-    ln_project_kernel<__nv_bfloat16><<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(x), ln_w, ln_b, w, mask, out, rows,
-                                                                  c, n_out, eps, samples, l);
+    KFB_TRY(launch_kernel(stream, ln_project_kernel<__nv_bfloat16>, blocks, 256, 0, static_cast<const __nv_bfloat16*>(x),
+        ln_w, ln_b, w, mask, out, rows,
+                                                                  c, n_out, eps, samples, l));
   else
-    ln_project_kernel<float><<<blocks, 256, 0, stream>>>(static_cast<const float*>(x), ln_w, ln_b, w, mask, out, rows, c, n_out, eps,
-                                                         samples, l);
+    KFB_TRY(launch_kernel(stream, ln_project_kernel<float>, blocks, 256, 0, static_cast<const float*>(x), ln_w, ln_b, w,
+        mask, out, rows, c, n_out, eps,
+                                                         samples, l));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }

@@ -107,15 +107,6 @@ attention_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   int nhalf = WIN ? 4 : 2 * ((p.lk + kBKV - 1) / kBKV);
   uint32_t* s_last = tmem_slot + 1;                   // [warps]: last valid key + 1 seen by each warp
   constexpr bool kTrim = !WIN && R == 1;
-  if (kTrim) {
-    const int b_hi = b0 / p.mask_lo_extent, b_lo = b0 - b_hi * p.mask_lo_extent;
-    const unsigned char* mrow = p.mask + static_cast<long long>(b_hi) * p.m_hi + static_cast<long long>(b_lo) * p.m_lo;
-    int last = 0;
-    for (int k = threadIdx.x; k < p.lk; k += blockDim.x)
-      if (mrow[static_cast<long long>(k) * p.m_k]) last = k + 1;
-    last = __reduce_max_sync(0xffffffffu, last);
-    if (lane == 0) s_last[warp] = static_cast<uint32_t>(last);
-  }
   long long* trace = (p.trace != nullptr && blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) ? p.trace : nullptr;
 #ifdef KFB_DEBUG_TRACE
 #ifdef KFB_DEBUG_TRACE
@@ -169,6 +160,16 @@ attention_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     for (int u = 0; u < R * 3; ++u)
       *reinterpret_cast<uint4*>(s_maskrow + u * Cfg::kSmallBytes + off + 128) = make_uint4(0, 0, 0, 0);
     ptx::fence_proxy_async_smem();
+  }
+  grid_dependency_enter();   // from here on global memory is read
+  if (kTrim) {
+    const int b_hi = b0 / p.mask_lo_extent, b_lo = b0 - b_hi * p.mask_lo_extent;
+    const unsigned char* mrow = p.mask + static_cast<long long>(b_hi) * p.m_hi + static_cast<long long>(b_lo) * p.m_lo;
+    int last = 0;
+    for (int k = threadIdx.x; k < p.lk; k += blockDim.x)
+      if (mrow[static_cast<long long>(k) * p.m_k]) last = k + 1;
+    last = __reduce_max_sync(0xffffffffu, last);
+    if (lane == 0) s_last[warp] = static_cast<uint32_t>(last);
   }
   // The mask bytes of the first two key tiles (the operands of S(0) .. S(3)) are fetched before the block-wide barrier by
   // the threads that will store them: their latency runs under the tensor-memory allocation and the barrier.
@@ -686,9 +687,8 @@ static int launch_cfg(cudaStream_t stream, const AttnParams& p) {
   dim3 grid(cdiv(p.lq, kBQ), p.heads, p.batch / R);
   {
     LaunchScope scope(stream, p.tag ? p.tag : "attention");
-    attention_bias_kernel<DPAD, R, WIN><<<grid, Cfg::kThreads, Cfg::kSmemBytes, stream>>>(tq, tk, tv, tb, p);
+    KFB_TRY(launch_kernel(stream, attention_bias_kernel<DPAD, R, WIN>, grid, Cfg::kThreads, Cfg::kSmemBytes, tq, tk, tv, tb, p));
   }
-  KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
 

@@ -15,6 +15,7 @@ static constexpr int kFk = 32;   // keys per tile
 
 template <int D>
 __global__ void __launch_bounds__(kFq) attention_fp32_kernel(const AttnFp32Params p) {
+  grid_dependency_enter();
   __shared__ float s_k[kFk][D + 1];
   __shared__ float s_v[kFk][D + 1];
   __shared__ float s_bias[kFq][kFk + 1];
@@ -114,11 +115,11 @@ int launch_attention_fp32(cudaStream_t stream, const AttnFp32Params& p) {
   dim3 grid(cdiv(p.lq, kFq), p.heads, p.batch);
   LaunchScope scope(stream, p.tag ? p.tag : "attention_fp32");
   switch (p.d) {
-    case 16: attention_fp32_kernel<16><<<grid, kFq, 0, stream>>>(p); break;
-    case 24: attention_fp32_kernel<24><<<grid, kFq, 0, stream>>>(p); break;
-    case 32: attention_fp32_kernel<32><<<grid, kFq, 0, stream>>>(p); break;
-    case 48: attention_fp32_kernel<48><<<grid, kFq, 0, stream>>>(p); break;
-    case 64: attention_fp32_kernel<64><<<grid, kFq, 0, stream>>>(p); break;
+    case 16: KFB_TRY(launch_kernel(stream, attention_fp32_kernel<16>, grid, kFq, 0, p)); break;
+    case 24: KFB_TRY(launch_kernel(stream, attention_fp32_kernel<24>, grid, kFq, 0, p)); break;
+    case 32: KFB_TRY(launch_kernel(stream, attention_fp32_kernel<32>, grid, kFq, 0, p)); break;
+    case 48: KFB_TRY(launch_kernel(stream, attention_fp32_kernel<48>, grid, kFq, 0, p)); break;
+    case 64: KFB_TRY(launch_kernel(stream, attention_fp32_kernel<64>, grid, kFq, 0, p)); break;
     default:
       set_error("attention_fp32: head dim %d not supported (16, 24, 32, 48, 64)", p.d);
       return KFB_ERR_UNSUPPORTED;

@@ -11,6 +11,7 @@ namespace {
 // reduced exactly by cospif (cos(pi x) with x = 2 t w + b / pi), so large |t w| loses nothing to range reduction.
 __global__ void __launch_bounds__(256) fourier_embed_kernel(const float* __restrict__ t, const float* __restrict__ w,
                                                             const float* __restrict__ b, float* __restrict__ out, int rows, int dim) {
+  grid_dependency_enter();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * dim) return;
   const int row = idx / dim, j = idx - row * dim;
@@ -21,6 +22,7 @@ __global__ void __launch_bounds__(256) fourier_embed_kernel(const float* __restr
 // out[g][n][l][:] = s[g][l][:] + f[g][n][:]   (token conditioning plus the per-sample noise embedding), fp32
 __global__ void __launch_bounds__(256) broadcast_add_kernel(const float* __restrict__ s, const float* __restrict__ f,
                                                             float* __restrict__ out, long long total, int samples, int l, int c) {
+  grid_dependency_enter();
   const long long idx = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   if (idx >= total) return;
   const int col = static_cast<int>(idx % c);
@@ -45,7 +47,7 @@ KFB_API int kfb_fourier_embed(const float* t, const float* w, const float* b, fl
   KFB_CHECK_ARG(rows >= 1 && dim >= 1 && static_cast<long long>(rows) * dim < (1ll << 31), "fourier_embed: rows %d dim %d", rows, dim);
   cudaStream_t stream = as_stream(stream_);
   LaunchScope scope(stream, "fourier_embed");
-  fourier_embed_kernel<<<cdiv(rows * dim, 256), 256, 0, stream>>>(t, w, b, out, rows, dim);
+  KFB_TRY(launch_kernel(stream, fourier_embed_kernel, cdiv(rows * dim, 256), 256, 0, t, w, b, out, rows, dim));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -59,7 +61,8 @@ KFB_API int kfb_broadcast_add(const float* s, const float* f, float* out, int gr
   cudaStream_t stream = as_stream(stream_);
   const long long total = static_cast<long long>(groups) * samples * l * c;
   LaunchScope scope(stream, "broadcast_add");
-  broadcast_add_kernel<<<static_cast<unsigned>((total / 4 + 255) / 256), 256, 0, stream>>>(s, f, out, total, samples, l, c);
+  KFB_TRY(launch_kernel(stream, broadcast_add_kernel, static_cast<unsigned>((total / 4 + 255) / 256), 256, 0, s, f, out,
+      total, samples, l, c));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }

@@ -37,9 +37,9 @@ static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUte
   }
   {
     LaunchScope scope(stream, tag);
-    gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP><<<grid, kGemmThreads, Cfg::kSmemBytes, stream>>>(ta, tb, tout[0], tout[1], q);
+    KFB_TRY(launch_kernel(stream, gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP>, grid, kGemmThreads, Cfg::kSmemBytes, ta, tb, tout[0],
+                          tout[1], q));
   }
-  KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
 

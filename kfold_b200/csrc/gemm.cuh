@@ -21,6 +21,7 @@
 #pragma once
 #include <cuda_bf16.h>
 
+#include "common.cuh"
 #include "ptx.cuh"
 
 namespace kfb {
@@ -82,6 +83,8 @@ struct GemmParams {
   const __nv_bfloat16* gate;      // optional: seg 0 value *= sigmoid(gate[...]), addressed with seg 0 strides
                                   // (points at float logits when `precise`)
   long long g_col, g_n, g_o, g_b;
+  int b_static;                   // B is a weight matrix that the stream finished writing before the previous launch: its first
+                                  // tiles are fetched while that launch still drains
   int stages;                     // depth of the operand ring (launcher)
   int aux;                        // 1: gate / residual tiles are prefetched into shared memory by TMA (launcher)
   int aux_gate, aux_resid;        // which of the two the prefetch covers
@@ -345,6 +348,21 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
+  // Everything above ran under the tail of the launch before this one (programmatic launch).  The producer also fetches the
+  // weight half of the first tile's stages before it waits: for the few-row GEMMs of the samplers, whose time is the latency of
+  // one tile, that takes the weights' trip from HBM off the critical path.
+  int b_ahead = 0;
+  if (warp == 0 && lane == 0 && p.b_static && !p.k_inner) {
+    const int n_tile = static_cast<int>(blockIdx.x) % p.num_n_tiles;
+    const int b_col_hi = (n_tile * BN) / p.b_col_inner;
+    b_ahead = num_k < kStages ? num_k : kStages;
+    for (int kb = 0; kb < b_ahead; ++kb) {
+      ptx::mbar_expect_tx(&full_bar[kb], Cfg::kStageBytes);
+      ptx::tma_load_4d(s_b + kb * Cfg::kBStage, &tm_b, &full_bar[kb], kb * kBK, n_tile * BN - b_col_hi * p.b_col_inner, b_col_hi, 0);
+    }
+  }
+  grid_dependency_wait();
+
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
     if (lane == 0) {
@@ -359,6 +377,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         const int o = rest % p.o_extent;
         const int b = rest / p.o_extent;
         const int bb = p.b_batched ? b : 0;
+        // the next kernel's blocks may take this SM over as soon as this CTA is on its last tile
+        if (tile + static_cast<int>(gridDim.x) >= total_tiles) grid_dependency_launch();
         const int b_col_hi = (n_tile * BN) / p.b_col_inner;
         const int b_col_lo = n_tile * BN - b_col_hi * p.b_col_inner;
         if (AUX) {
@@ -378,8 +398,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           }
         }
         for (int kb = 0; kb < num_k; ++kb) {
-          if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1, 101)) { ok = false; break; }
-          ptx::mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
+          const bool b_done = b_ahead > 0;      // this stage's weights are already on their way
+          if (b_done) {
+            --b_ahead;
+          } else {
+            if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1, 101)) { ok = false; break; }
+            ptx::mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
+          }
           if (p.a_mn_major) {
             // two boxes of [64 k][64 rows]: 128-byte rows of consecutive rows (positions), one per k index
             ptx::tma_load_4d(s_a + stage * Cfg::kAStage, &tm_a, &full_bar[stage], nb * kBM, kb * kBK, o, b);
@@ -393,7 +418,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             continue;
           } else
           ptx::tma_load_4d(s_a + stage * Cfg::kAStage, &tm_a, &full_bar[stage], kb * kBK, nb * kBM, o, b);
-          ptx::tma_load_4d(s_b + stage * Cfg::kBStage, &tm_b, &full_bar[stage], kb * kBK, b_col_lo, b_col_hi, bb);
+          if (!b_done)
+            ptx::tma_load_4d(s_b + stage * Cfg::kBStage, &tm_b, &full_bar[stage], kb * kBK, b_col_lo, b_col_hi, bb);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
         KFB_GSTAMP(4 + (tile / gridDim.x) * 4 + 3);

@@ -40,6 +40,7 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* __restric
                                                              const float* __restrict__ w, const float* __restrict__ b,
                                                              long long rows, int c, long long xs, long long ys, float eps,
                                                              RowPerm perm) {
+  grid_dependency_enter();
   const int lane = threadIdx.x & 31;
   const long long warps_per_grid = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   for (long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows;
@@ -100,6 +101,7 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* __restric
 __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                                                   const float* __restrict__ w, const float* __restrict__ b,
                                                                   long long rows, float eps) {
+  grid_dependency_enter();
   const int lane = threadIdx.x & 31;
   const int sub = lane & 15;                 // 16-byte chunk of the row
   const int half = lane >> 4;                // which of the warp's two rows
@@ -167,15 +169,15 @@ static int launch_rows(cudaStream_t stream, const void* x, void* y, const float*
   LaunchScope scope(stream, "layernorm_rows");
   if (perm.rows) {
     if constexpr (std::is_same<TO, __nv_bfloat16>::value) {   // the exchange order is only ever written in bf16
-      layernorm_rows_kernel<TI, TO, G, true><<<static_cast<unsigned>(blocks), warps * 32, 0, stream>>>(
-          static_cast<const TI*>(x), static_cast<TO*>(y), w, b, rows, c, xs, ys, eps, perm);
+      KFB_TRY(launch_kernel(stream, layernorm_rows_kernel<TI, TO, G, true>, static_cast<unsigned>(blocks), warps * 32, 0,
+          static_cast<const TI*>(x), static_cast<TO*>(y), w, b, rows, c, xs, ys, eps, perm));
     } else {
       set_error("layernorm: the exchange order is written in bf16 only");
       return KFB_ERR_UNSUPPORTED;
     }
   } else {
-    layernorm_rows_kernel<TI, TO, G, false><<<static_cast<unsigned>(blocks), warps * 32, 0, stream>>>(
-        static_cast<const TI*>(x), static_cast<TO*>(y), w, b, rows, c, xs, ys, eps, perm);
+    KFB_TRY(launch_kernel(stream, layernorm_rows_kernel<TI, TO, G, false>, static_cast<unsigned>(blocks), warps * 32, 0,
+        static_cast<const TI*>(x), static_cast<TO*>(y), w, b, rows, c, xs, ys, eps, perm));
   }
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
@@ -208,8 +210,8 @@ int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w
     const long long cap = static_cast<long long>(sm_count()) * 16;
     if (blocks > cap) blocks = cap;
     LaunchScope scope(stream, "layernorm_rows");
-    layernorm_c128_bf16_kernel<<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), w, b, rows, eps);
+    KFB_TRY(launch_kernel(stream, layernorm_c128_bf16_kernel, static_cast<unsigned>(blocks), 256, 0,
+        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), w, b, rows, eps));
     KFB_CUDA(cudaGetLastError());
     return KFB_OK;
   }
@@ -227,6 +229,7 @@ int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w
 
 // fp32 -> bf16 conversion, eight elements per thread (HBM-bound; the conditioning rows of a stack: one small launch).
 __global__ void __launch_bounds__(256) to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
+  grid_dependency_enter();
   const long long i = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * 8;
   if (i + 8 <= n) {
     const float4 a = *reinterpret_cast<const float4*>(x + i), b = *reinterpret_cast<const float4*>(x + i + 4);
@@ -242,7 +245,7 @@ int launch_to_bf16(cudaStream_t stream, const float* x, __nv_bfloat16* y, long l
   if (n <= 0) return KFB_OK;
   KFB_CHECK_ARG(((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0, "to_bf16: pointers must be 16-byte aligned");
   LaunchScope scope(stream, "to_bf16");
-  to_bf16_kernel<<<static_cast<unsigned>((n + 2047) / 2048), 256, 0, stream>>>(x, y, n);
+  KFB_TRY(launch_kernel(stream, to_bf16_kernel, static_cast<unsigned>((n + 2047) / 2048), 256, 0, x, y, n));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -261,6 +264,7 @@ __device__ __forceinline__ void split3_store(__nv_bfloat16* y6, int c, int ch, f
 __global__ void __launch_bounds__(256) layernorm_split_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y6,
                                                               const float* __restrict__ w, const float* __restrict__ b,
                                                               long long rows, int c, long long xs, float eps, int normalise) {
+  grid_dependency_enter();
   const int lane = threadIdx.x & 31;
   const long long warps_per_grid = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   for (long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows;
@@ -297,7 +301,8 @@ int launch_layernorm_split(cudaStream_t stream, const float* x, __nv_bfloat16* y
   const long long cap = static_cast<long long>(sm_count()) * 16;
   if (blocks > cap) blocks = cap;
   LaunchScope scope(stream, "layernorm_split");
-  layernorm_split_kernel<<<static_cast<unsigned>(blocks), warps * 32, 0, stream>>>(x, y6, w, b, rows, c, xs, eps, normalise);
+  KFB_TRY(launch_kernel(stream, layernorm_split_kernel, static_cast<unsigned>(blocks), warps * 32, 0, x, y6, w, b, rows, c,
+      xs, eps, normalise));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -307,6 +312,7 @@ __global__ void __launch_bounds__(128) layernorm_cm_split_kernel(const float* __
                                                                  const float* __restrict__ w, const float* __restrict__ b,
                                                                  long long npos, int c, long long chan_stride,
                                                                  long long batch_stride, float eps, int blocks_per_batch) {
+  grid_dependency_enter();
   extern __shared__ __align__(16) unsigned char slab_raw_f[];
   float* slab = reinterpret_cast<float*>(slab_raw_f);  // [c][128]
   const int batch = blockIdx.x / blocks_per_batch;
@@ -345,6 +351,7 @@ template <typename TI, typename TO, typename TG, int G>
 __global__ void __launch_bounds__(256) adaln_rows_kernel(const TI* __restrict__ a, TO* __restrict__ y,
                                                          const TG* __restrict__ gv, long long gv_ld, long long rows, int c,
                                                          int samples, int l, float eps) {
+  grid_dependency_enter();
   const int lane = threadIdx.x & 31;
   const long long warps_per_grid = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   for (long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows;
@@ -411,6 +418,7 @@ template <typename TI, int CH, int LANES>
 __global__ void __launch_bounds__(256) adaln_vec_kernel(const TI* __restrict__ a, __nv_bfloat16* __restrict__ y,
                                                         const __nv_bfloat16* __restrict__ gv, long long gv_ld, long long rows,
                                                         int samples, int l, float eps) {
+  grid_dependency_enter();
   constexpr int c = 8 * LANES * CH;
   constexpr int kRowsPerWarp = 32 / LANES;
   const int lane = threadIdx.x & 31;
@@ -483,9 +491,9 @@ static int launch_adaln_vec(cudaStream_t stream, const void* a, void* y, const v
   const long long cap = static_cast<long long>(sm_count()) * 16;
   if (blocks > cap) blocks = cap;
   LaunchScope scope(stream, "adaln_rows");
-  adaln_vec_kernel<TI, CH, LANES><<<static_cast<unsigned>(blocks), 256, 0, stream>>>(
+  KFB_TRY(launch_kernel(stream, adaln_vec_kernel<TI, CH, LANES>, static_cast<unsigned>(blocks), 256, 0,
       static_cast<const TI*>(a), static_cast<__nv_bfloat16*>(y), static_cast<const __nv_bfloat16*>(gv), gv_ld, rows,
-      samples, l, eps);
+      samples, l, eps));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -501,8 +509,8 @@ static int adaln_dispatch(cudaStream_t stream, const void* a, void* y, const voi
   const int g = cdiv(c, 64);
   LaunchScope scope(stream, "adaln_rows");
 #define KFB_ADALN(GG)                                                                                          \
-  adaln_rows_kernel<TI, TO, TG, GG><<<static_cast<unsigned>(blocks), warps * 32, 0, stream>>>(                  \
-      static_cast<const TI*>(a), static_cast<TO*>(y), gv, gv_ld, rows, c, samples, l, eps)
+  KFB_TRY(launch_kernel(stream, adaln_rows_kernel<TI, TO, TG, GG>, static_cast<unsigned>(blocks), warps * 32, 0, \
+      static_cast<const TI*>(a), static_cast<TO*>(y), gv, gv_ld, rows, c, samples, l, eps))
   if (g <= 2) KFB_ADALN(2);
   else if (g <= 6) KFB_ADALN(6);
   else if (g <= 12) KFB_ADALN(12);
@@ -571,6 +579,7 @@ __global__ void __launch_bounds__(kCmPos) layernorm_cm_kernel(const TI* __restri
                                                               const float* __restrict__ w, const float* __restrict__ b,
                                                               long long npos, int c, long long chan_stride,
                                                               long long batch_stride, float eps, int blocks_per_batch) {
+  grid_dependency_enter();
   extern __shared__ __align__(16) unsigned char slab_raw[];
   __nv_bfloat16* slab = reinterpret_cast<__nv_bfloat16*>(slab_raw);  // [c][128]
   const int batch = blockIdx.x / blocks_per_batch;
@@ -646,6 +655,7 @@ __global__ void __launch_bounds__(kCmPos) layernorm_cm_kernel(const TI* __restri
 // (mean, rstd) over the channels of every position of a channel-major tensor t[c][npos]; two positions per thread
 __global__ void __launch_bounds__(256) cm_stats_kernel(const __nv_bfloat16* __restrict__ t, float2* __restrict__ stats,
                                                        long long npos, int c, long long chan_stride, float eps) {
+  grid_dependency_enter();
   const long long p2 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 2;
   if (p2 >= npos) return;
   const bool pair = p2 + 1 < npos;
@@ -683,6 +693,7 @@ __global__ void __launch_bounds__(256) cm_stats_kernel(const __nv_bfloat16* __re
 // tensor, and twice the bytes in flight per thread.  npos and the channel stride multiples of 4, t 8-byte aligned.
 __global__ void __launch_bounds__(128) cm_stats4_kernel(const __nv_bfloat16* __restrict__ t, float2* __restrict__ stats,
                                                         long long npos, int c, long long chan_stride, float eps) {
+  grid_dependency_enter();
   const long long p4 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   if (p4 >= npos) return;
   float s[4] = {0.f, 0.f, 0.f, 0.f}, q[4] = {0.f, 0.f, 0.f, 0.f}, x0[4];
@@ -727,12 +738,14 @@ int launch_cm_stats(cudaStream_t stream, const __nv_bfloat16* t, float2* stats, 
   if (npos % 4 == 0 && chan_stride % 4 == 0 && (reinterpret_cast<uintptr_t>(t) & 7) == 0 &&
       (reinterpret_cast<uintptr_t>(stats) & 15) == 0) {
     const long long threads4 = npos / 4;
-    cm_stats4_kernel<<<static_cast<unsigned>((threads4 + 127) / 128), 128, 0, stream>>>(t, stats, npos, c, chan_stride, eps);
+    KFB_TRY(launch_kernel(stream, cm_stats4_kernel, static_cast<unsigned>((threads4 + 127) / 128), 128, 0, t, stats, npos, c,
+        chan_stride, eps));
     KFB_CUDA(cudaGetLastError());
     return KFB_OK;
   }
   const long long threads = npos / 2;
-  cm_stats_kernel<<<static_cast<unsigned>((threads + 255) / 256), 256, 0, stream>>>(t, stats, npos, c, chan_stride, eps);
+  KFB_TRY(launch_kernel(stream, cm_stats_kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, t, stats, npos, c,
+      chan_stride, eps));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -741,6 +754,7 @@ int launch_cm_stats(cudaStream_t stream, const __nv_bfloat16* t, float2* stats, 
 __global__ void __launch_bounds__(128) ln_fold_weights_kernel(const __nv_bfloat16* __restrict__ w, const float* __restrict__ gamma,
                                                               const float* __restrict__ beta, __nv_bfloat16* __restrict__ wf,
                                                               float* __restrict__ s1, float* __restrict__ s0, int k) {
+  grid_dependency_enter();
   const int n = blockIdx.x;
   float a1 = 0.f, a0 = 0.f;
   for (int i = threadIdx.x; i < k; i += blockDim.x) {
@@ -765,7 +779,7 @@ int launch_ln_fold_weights(cudaStream_t stream, const __nv_bfloat16* w, const fl
                            float* s1, float* s0, int n, int k) {
   KFB_CHECK_ARG(n > 0 && k > 0, "ln_fold_weights: n %d k %d", n, k);
   LaunchScope scope(stream, "layernorm_fold_weights");
-  ln_fold_weights_kernel<<<n, 128, 0, stream>>>(w, gamma, beta, wf, s1, s0, k);
+  KFB_TRY(launch_kernel(stream, ln_fold_weights_kernel, n, 128, 0, w, gamma, beta, wf, s1, s0, k));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -784,6 +798,7 @@ template <int C, typename T>
 __global__ void __launch_bounds__(256) window_bias_kernel(const T* __restrict__ x, const float* __restrict__ ln_w,
                                                           const float* __restrict__ ln_b, const T* __restrict__ w,
                                                           T* __restrict__ y, long long npos, int nh, float eps, int normalise) {
+  grid_dependency_enter();
   extern __shared__ float s_w[];  // [nh][C] fp32, then gamma[C], beta[C]
   float* s_g = s_w + nh * C;
   float* s_b = s_g + C;
@@ -832,13 +847,13 @@ static int launch_window_bias_c(cudaStream_t stream, const void* x, const float*
   const unsigned blocks = static_cast<unsigned>((npos + 255) / 256);
   LaunchScope scope(stream, "window_bias");
   if (dtype == KFB_BF16)
-    window_bias_kernel<C, __nv_bfloat16><<<blocks, 256, smem, stream>>>(
+    KFB_TRY(launch_kernel(stream, window_bias_kernel<C, __nv_bfloat16>, blocks, 256, smem,
         static_cast<const __nv_bfloat16*>(x), ln_w, ln_b, static_cast<const __nv_bfloat16*>(w), static_cast<__nv_bfloat16*>(y),
-        npos, nh, eps, normalise);
+        npos, nh, eps, normalise));
   else
-    window_bias_kernel<C, float><<<blocks, 256, smem, stream>>>(static_cast<const float*>(x), ln_w, ln_b,
+    KFB_TRY(launch_kernel(stream, window_bias_kernel<C, float>, blocks, 256, smem, static_cast<const float*>(x), ln_w, ln_b,
                                                                 static_cast<const float*>(w), static_cast<float*>(y), npos, nh, eps,
-                                                                normalise);
+                                                                normalise));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -871,8 +886,9 @@ int launch_layernorm_cm(cudaStream_t stream, const void* t, __nv_bfloat16* y, co
     if (smem > 48 * 1024)
       KFB_CUDA(cudaFuncSetAttribute(layernorm_cm_split_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
     LaunchScope scope(stream, "layernorm_cm_split");
-    layernorm_cm_split_kernel<<<bpb * batch, 128, smem, stream>>>(static_cast<const float*>(t), y, w, b, npos, c, chan_stride,
-                                                                 batch_stride, eps, bpb);
+    KFB_TRY(launch_kernel(stream, layernorm_cm_split_kernel, bpb * batch, 128, smem, static_cast<const float*>(t), y, w, b,
+        npos, c, chan_stride,
+                                                                 batch_stride, eps, bpb));
     KFB_CUDA(cudaGetLastError());
     return KFB_OK;
   }
@@ -884,13 +900,15 @@ int launch_layernorm_cm(cudaStream_t stream, const void* t, __nv_bfloat16* y, co
   if (in_dtype == KFB_BF16) {
     if (smem > 48 * 1024)
       KFB_CUDA(cudaFuncSetAttribute(layernorm_cm_kernel<__nv_bfloat16>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    layernorm_cm_kernel<__nv_bfloat16><<<bpb * batch, kCmPos, smem, stream>>>(static_cast<const __nv_bfloat16*>(t), y, w, b, npos,
-                                                                           c, chan_stride, batch_stride, eps, bpb);
+    KFB_TRY(launch_kernel(stream, layernorm_cm_kernel<__nv_bfloat16>, bpb * batch, kCmPos, smem,
+        static_cast<const __nv_bfloat16*>(t), y, w, b, npos,
+                                                                           c, chan_stride, batch_stride, eps, bpb));
   } else {
     if (smem > 48 * 1024)
       KFB_CUDA(cudaFuncSetAttribute(layernorm_cm_kernel<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem));
-    layernorm_cm_kernel<float><<<bpb * batch, kCmPos, smem, stream>>>(static_cast<const float*>(t), y, w, b, npos, c, chan_stride,
-                                                                   batch_stride, eps, bpb);
+    KFB_TRY(launch_kernel(stream, layernorm_cm_kernel<float>, bpb * batch, kCmPos, smem, static_cast<const float*>(t), y, w,
+        b, npos, c, chan_stride,
+                                                                   batch_stride, eps, bpb));
   }
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;

@@ -125,6 +125,7 @@ int triatt_precise(cudaStream_t stream, int ending, const void* x, const unsigne
     const long long c6 = 6ll * c;
     GemmOperandA a = {w.xn6, ending ? n * c6 : c6, ending ? c6 : n * c6, nn * c6};
     GemmOperandB b = {w_proj6, c6, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "triatt_proj_precise"));
   }
   {
@@ -162,6 +163,7 @@ int triatt_precise(cudaStream_t stream, int ending, const void* x, const unsigne
     const long long c6 = 6ll * c;
     GemmOperandA a = {w.og6, c6, n * c6, nn * c6};
     GemmOperandB b = {w_out6, c6, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "triatt_out_proj_precise"));
   }
   return KFB_OK;
@@ -261,6 +263,7 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
     sb.s_b = static_cast<long long>(heads) * nn;
     GemmOperandA a = {w.xn, ending ? static_cast<long long>(n) * c : c, ending ? c : static_cast<long long>(n) * c, nn * c};
     GemmOperandB b = {w_proj_packed, c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "triatt_proj"));
   }
   {
@@ -299,6 +302,7 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
     p.resid = resid;
     GemmOperandA a = {w.og, c, static_cast<long long>(n) * c, nn * c};
     GemmOperandB b = {w_out, c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "triatt_out_proj"));
   }
   return KFB_OK;
@@ -439,6 +443,7 @@ KFB_API int kfb_triatt_finish(const void* qkg, const void* vt, const void* bias_
     p.seg[0] = row_major_seg(out, c, c, static_cast<long long>(rows) * rows * c, static_cast<long long>(rows) * c, 0);
     a = {og_scratch, c, static_cast<long long>(rows) * c, static_cast<long long>(n) * c};
   }
+  p.b_static = 1;
   return launch_gemm_bf16(stream, a, b, p, 0, "triatt_out_proj");
 }
 
@@ -472,6 +477,7 @@ static int pair_bias_impl(const void* z, const float* ln_w, const float* ln_b, c
   s.s_b = static_cast<long long>(heads) * rn;
   GemmOperandA a = {zn, c, static_cast<long long>(n) * c, rn * c};
   GemmOperandB b = {w, c, 0};
+  p.b_static = 1;
   return launch_gemm_bf16(stream, a, b, p, 0, "pair_bias_proj");
 }
 
@@ -510,6 +516,7 @@ KFB_API int kfb_pair_bias_fwd(const void* z, const float* ln_w, const float* ln_
     const long long c6 = 6ll * c;
     GemmOperandA a = {zn6, c6, n * c6, nn * c6};
     GemmOperandB b = {w, c6, 0};
+    p.b_static = 1;
     return launch_gemm_bf16(stream, a, b, p, 0, "pair_bias_proj_precise");
   }
   KFB_CHECK_ARG(workspace_bytes >= kfb_pair_bias_workspace_bytes(batch, n, c), "pair_bias: workspace too small");
@@ -570,6 +577,7 @@ int apb_run(cudaStream_t stream, const ApbArgs& r) {
       p.col_bias = r.proj_bias;
       GemmOperandA a = {x6, c6, 0, 0};
       GemmOperandB b = {r.w_proj, c6, 0};
+      p.b_static = !r.x_is_split || r.w_static;
       KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "apb_proj_precise"));
     }
     {
@@ -613,6 +621,7 @@ int apb_run(cudaStream_t stream, const ApbArgs& r) {
     }
     GemmOperandA a = {wp.og6, c6, l * c6, l * c6 * gate_share};
     GemmOperandB b = {r.w_out, c6, 0};
+    p.b_static = 1;
     return launch_gemm_bf16(stream, a, b, p, 0, "apb_out_proj_precise");
   }
   const int dp = dpad_of(d), hdp = heads * dp, lv = pitch16(l);
@@ -641,6 +650,7 @@ int apb_run(cudaStream_t stream, const ApbArgs& r) {
     p.col_bias = r.proj_bias;
     GemmOperandA a = {r.x, c, static_cast<long long>(l) * c, 0};
     GemmOperandB b = {r.w_proj, c, 0};
+    p.b_static = r.w_static;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "apb_proj"));
   }
   {
@@ -687,6 +697,7 @@ int apb_run(cudaStream_t stream, const ApbArgs& r) {
     }
     GemmOperandA a = {w.og, c, lc, lc * gate_share};
     GemmOperandB b = {r.w_out, c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "apb_out_proj"));
   }
   return KFB_OK;
@@ -825,6 +836,7 @@ KFB_API int kfb_apb_cross_fwd(const void* x_q, const void* x_k, const void* pair
     }
     GemmOperandA a = {wp.og6, c6, gate_rows * c6, 0};
     GemmOperandB b = {w_out, c6, 0};
+    p.b_static = 1;
     return launch_gemm_bf16(stream, a, b, p, 0, "apb_cross_out_proj_precise");
   }
   const int dp = dpad_of(d), hdp = heads * dp;
@@ -866,6 +878,7 @@ KFB_API int kfb_apb_cross_fwd(const void* x_q, const void* x_k, const void* pair
     sv.s_o = static_cast<long long>(hdp) * lk;
     GemmOperandA a = {x_k, c, static_cast<long long>(lk) * c, 0};
     GemmOperandB b = {w_kv_packed, c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "apb_cross_kv_proj"));
   }
   {
@@ -910,6 +923,7 @@ KFB_API int kfb_apb_cross_fwd(const void* x_q, const void* x_k, const void* pair
     }
     GemmOperandA a = {w.og, c, gate_rows * c, 0};
     GemmOperandB b = {w_out, c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "apb_cross_out_proj"));
   }
   return KFB_OK;
@@ -983,6 +997,7 @@ KFB_API int kfb_apb_window_fwd(const void* x_q, const void* x_k, const void* pai
     sv.s_o = static_cast<long long>(hdp) * l;
     GemmOperandA a = {x_k, c, static_cast<long long>(l) * c, 0};
     GemmOperandB b = {w_kv_packed, c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "apb_window_kv_proj"));
   }
   {
@@ -1028,6 +1043,7 @@ KFB_API int kfb_apb_window_fwd(const void* x_q, const void* x_k, const void* pai
     }
     GemmOperandA a = {w.og, c, gate_rows * c, 0};
     GemmOperandB b = {w_out, c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "apb_window_out_proj"));
   }
   return KFB_OK;

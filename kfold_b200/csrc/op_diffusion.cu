@@ -45,6 +45,7 @@ KFB_API int kfb_linear_fp32(const void* x, const void* w6, const float* bias, vo
   p.col_bias = bias;
   GemmOperandA a = {x6, 6ll * k, 0, 0};
   GemmOperandB b = {w6, 6ll * k, 0};
+  p.b_static = 1;
   return launch_gemm_bf16(stream, a, b, p, 0, "linear_fp32");
 }
 
@@ -73,6 +74,7 @@ KFB_API int kfb_ln_linear_fp32(const void* x, const float* ln_w, const float* ln
   p.resid = resid;
   GemmOperandA a = {x6, 6ll * k, 0, 0};
   GemmOperandB b = {w6, 6ll * k, 0};
+  p.b_static = 1;
   return launch_gemm_bf16(stream, a, b, p, 0, "ln_linear_fp32");
 }
 
@@ -88,7 +90,7 @@ KFB_API size_t kfb_cond_transition_workspace_bytes(long long rows, int hidden) {
 
 // out = sigmoid(gate[s(r)]) * (silu(u_a) * u_b) W_out^T  (+ resid),  [u_a, u_b] = x W_swiglu^T,  x already AdaLN-normalised
 namespace kfb {
-int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_split, const void* w_swiglu_packed, const void* w_out,
+int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_split, int w_static, const void* w_swiglu_packed, const void* w_out,
                         const void* out_gate, long long gate_ld, void* out, const void* resid, void* workspace,
                         size_t workspace_bytes, long long rows, int c, int hidden, int samples, int l, int dtype) {
   KFB_CHECK_ARG(x_normed && w_swiglu_packed && w_out && out_gate && out && workspace, "cond_transition: null pointer");
@@ -129,6 +131,7 @@ int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_spli
       p.seg[0].s_part = hidden;
       GemmOperandA a = {xs, 6ll * c, 0, 0};
       GemmOperandB b = {w_swiglu_packed, 6ll * c, 0};
+      p.b_static = !x_is_split || w_static;
       KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "cond_transition_swiglu_precise"));
     }
     const int groups = static_cast<int>(rows / (static_cast<long long>(samples) * l));
@@ -150,6 +153,7 @@ int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_spli
     p.g_b = l * gate_ld;
     GemmOperandA a = {h6, 6ll * hidden, lh6, lh6 * samples};
     GemmOperandB b = {w_out, 6ll * hidden, 0};
+    p.b_static = 1;
     return launch_gemm_bf16(stream, a, b, p, 0, "cond_transition_out_precise");
   }
   KFB_CHECK_ARG(workspace_bytes >= kfb_cond_transition_workspace_bytes(rows, hidden), "cond_transition: workspace too small");
@@ -166,6 +170,7 @@ int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_spli
     p.seg[0] = row_major_seg(h, hidden, hidden, 0, 0, 0);
     GemmOperandA a = {x_normed, c, 0, 0};
     GemmOperandB b = {w_swiglu_packed, c, 0};
+    p.b_static = w_static;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 256, "cond_transition_swiglu"));
   }
   {
@@ -187,6 +192,7 @@ int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_spli
     p.g_b = l * gate_ld;
     GemmOperandA a = {h, hidden, lh, lh * samples};
     GemmOperandB b = {w_out, hidden, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "cond_transition_out"));
   }
   return KFB_OK;
@@ -199,7 +205,7 @@ KFB_API int kfb_cond_transition_fwd(const void* x_normed, const void* w_swiglu_p
                                     const void* out_gate, long long gate_ld, void* out, const void* resid, void* workspace,
                                     size_t workspace_bytes, long long rows, int c, int hidden, int samples, int l, int dtype,
                                     void* stream_) {
-  return cond_transition_run(as_stream(stream_), x_normed, 0, w_swiglu_packed, w_out, out_gate, gate_ld, out, resid, workspace,
+  return cond_transition_run(as_stream(stream_), x_normed, 0, 0, w_swiglu_packed, w_out, out_gate, gate_ld, out, resid, workspace,
                              workspace_bytes, rows, c, hidden, samples, l, dtype);
 }
 

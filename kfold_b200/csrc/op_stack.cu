@@ -35,6 +35,7 @@ int table_gemm(cudaStream_t stream, const void* x, const void* w, const float* b
   p.nseg = 1;
   p.seg[0] = row_major_seg(dst, static_cast<int>(n), n, 0, 0, precise);
   p.col_bias = bias;
+  p.b_static = 1;
   GemmOperandA a = {x, static_cast<long long>(p.k_extent), 0, 0};
   GemmOperandB b = {w, static_cast<long long>(p.k_extent), 0};
   return launch_gemm_bf16(stream, a, b, p, 0, tag);
@@ -133,6 +134,7 @@ KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, con
                          precise ? KFB_FP32 : KFB_BF16, t.gs_cols));
     ApbArgs r;
     r.x = an;
+    r.w_static = 1;
     r.pair_bias = static_cast<const uint8_t*>(pair_bias) + bias_block_stride * i * bias_e;
     r.ldb = bias_ld; r.bias_hs = bias_head_stride; r.bias_div = samples;
     r.mask = mask; r.mask_share = samples;
@@ -145,7 +147,7 @@ KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, con
     cur = out;                                      // from here on the stream is updated in place
     KFB_TRY(launch_adaln(stream, cur, an, column(t.gs, 4ll * c * i + 2ll * c, precise), rows, c, share, l, eps, ada_dtype,
                          precise ? KFB_FP32 : KFB_BF16, t.gs_cols));
-    KFB_TRY(cond_transition_run(stream, an, 0, w.w_swiglu, w.w_tout, column(t.og, 2ll * c * i + c, precise), t.og_cols, out, cur, op_ws,
+    KFB_TRY(cond_transition_run(stream, an, 0, 1, w.w_swiglu, w.w_tout, column(t.og, 2ll * c * i + c, precise), t.og_cols, out, cur, op_ws,
                                 op_bytes, rows, c, hidden, share, l, op_dtype));
   }
   return KFB_OK;
@@ -202,7 +204,7 @@ KFB_API int kfb_atom_stack_fwd(const kfb_atom_block* blocks, int n_blocks, const
     }
     cur = out;
     KFB_TRY(launch_adaln(stream, cur, xq, column(t.gs, g0 + 4ll * c, 0), rows, c, samples, l, eps, act_dtype, KFB_BF16, t.gs_cols));
-    KFB_TRY(cond_transition_run(stream, xq, 0, w.w_swiglu, w.w_tout, column(t.og, 2ll * c * i + c, 0), t.og_cols, out, cur, op_ws, op_bytes,
+    KFB_TRY(cond_transition_run(stream, xq, 0, 1, w.w_swiglu, w.w_tout, column(t.og, 2ll * c * i + c, 0), t.og_cols, out, cur, op_ws, op_bytes,
                                 rows, c, hidden, samples, l, act_dtype));
   }
   return KFB_OK;

@@ -53,6 +53,7 @@ static int transition_precise(cudaStream_t stream, const void* x, const float* l
     p.seg[0].s_part = hidden;
     GemmOperandA a = {xn6, 6ll * c, 0, 0};
     GemmOperandB b = {w_swiglu6, 6ll * c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "transition_swiglu_precise"));
   }
   {
@@ -68,6 +69,7 @@ static int transition_precise(cudaStream_t stream, const void* x, const float* l
     p.resid = resid;
     GemmOperandA a = {h6, 6ll * hidden, 0, 0};
     GemmOperandB b = {w_out6, 6ll * hidden, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "transition_out_precise"));
   }
   return KFB_OK;
@@ -104,6 +106,7 @@ KFB_API int kfb_transition_fwd(const void* x, const float* ln_w, const float* ln
     p.seg[0] = row_major_seg(w.h, hidden, hidden, 0, 0, 0);
     GemmOperandA a = {w.xn, c, 0, 0};
     GemmOperandB b = {w_swiglu_packed, c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 256, "transition_swiglu"));
   }
   {
@@ -118,6 +121,7 @@ KFB_API int kfb_transition_fwd(const void* x, const float* ln_w, const float* ln
     p.resid = resid;
     GemmOperandA a = {w.h, hidden, 0, 0};
     GemmOperandB b = {w_out, hidden, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "transition_out"));
   }
   return KFB_OK;

@@ -81,6 +81,7 @@ int project(cudaStream_t stream, int transposed_walk, const void* x, const unsig
     GemmOperandA a = {xn, transposed_walk ? static_cast<long long>(n) * c : c,
                       transposed_walk ? c : static_cast<long long>(n) * c, rn * c};
     GemmOperandB b = {static_cast<const __nv_bfloat16*>(w_in_packed) + static_cast<long long>(part) * (4 * c / parts) * c, c, 0};
+    p.b_static = x != nullptr;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 256, "trimul_in_proj"));
   }
   if (w_gout != nullptr) {
@@ -94,6 +95,7 @@ int project(cudaStream_t stream, int transposed_walk, const void* x, const unsig
     p.seg[0] = row_major_seg(gl, c, c, 0, 0, 0);
     GemmOperandA a = {xn, c, 0, 0};
     GemmOperandB b = {w_gout, c, 0};
+    p.b_static = x != nullptr || w_in_packed != nullptr;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "trimul_gate_proj"));
   }
   return KFB_OK;
@@ -156,6 +158,7 @@ int finish(cudaStream_t stream, const __nv_bfloat16* a, const __nv_bfloat16* b, 
     GemmOperandA oa = {t, 1, 0, 0};
     oa.s_k = pos;
     GemmOperandB ob = {wf, c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, oa, ob, p, 0, "trimul_out_proj"));
     return KFB_OK;
   }
@@ -175,6 +178,7 @@ int finish(cudaStream_t stream, const __nv_bfloat16* a, const __nv_bfloat16* b, 
     p.resid = resid;
     GemmOperandA oa = {tn, c, 0, 0};
     GemmOperandB ob = {w_pout, c, 0};
+    p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, oa, ob, p, 0, "trimul_out_proj"));
   }
   return KFB_OK;

@@ -47,6 +47,7 @@ inline int pitch16(int l) { return (l + 15) / 16 * 16; }
 struct ApbArgs {
   const void* x = nullptr;            // bf16 (batch, l, c); precise: fp32, or its triple split when x_is_split
   int x_is_split = 0;
+  int w_static = 0;                   // a launch of this library lies between the last write of the weights and this call
   const void* pair_bias = nullptr;    // [batch / bias_div][heads][l][ldb], head planes bias_hs elements apart (0: l * ldb)
   long long ldb = 0, bias_hs = 0;
   int bias_div = 1;
@@ -62,8 +63,8 @@ struct ApbArgs {
 int apb_run(cudaStream_t stream, const ApbArgs& r);
 
 // Conditioned transition on AdaLN-normalised rows (kfb_cond_transition_fwd and the stacks).  x_is_split: precise mode, x is
-// already the triple split.
-int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_split, const void* w_swiglu, const void* w_out,
+// already the triple split; w_static as in ApbArgs.
+int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_split, int w_static, const void* w_swiglu, const void* w_out,
                         const void* out_gate, long long gate_ld, void* out, const void* resid, void* workspace,
                         size_t workspace_bytes, long long rows, int c, int hidden, int samples, int l, int dtype);
 

@@ -8,7 +8,21 @@ every temporary of the Python layer comes from torch's caching allocator, which 
 """
 from __future__ import annotations
 
+import threading
+
 import torch
+
+_local = threading.local()
+
+
+def _capture_stream(device: torch.device) -> torch.cuda.Stream:
+    """This thread's side stream for warm-up and capture on `device`.  One stream for all captures: memory the allocator has
+    cached for it, and the workspace the operators keep per stream, serve the next capture instead of being allocated anew."""
+    streams = _local.__dict__.setdefault("streams", {})
+    index = torch.cuda.current_device() if device.index is None else device.index
+    if index not in streams:
+        streams[index] = torch.cuda.Stream(index)
+    return streams[index]
 
 
 class GraphedCall:
@@ -35,7 +49,7 @@ class GraphedCall:
             # Warm-up and capture on one side stream.  torch.cuda.graph() would collect Python garbage and return the
             # allocator's cached blocks to the driver first; with a model of a few hundred parameters in memory that is
             # 0.1 s and more, and every later allocation pays for it again, so the capture is begun and ended directly.
-            current, side = torch.cuda.current_stream(), torch.cuda.Stream()
+            current, side = torch.cuda.current_stream(), _capture_stream(dev)
             side.wait_stream(current)
             with torch.cuda.stream(side):          # warm-up outside the capture: weight packing, workspace allocation
                 for _ in range(max(warmup, 1)):

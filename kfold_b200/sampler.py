@@ -324,7 +324,7 @@ class KFoldECSI:
                     def net(r6_, cn_):
                         with torch.autocast("cuda", enabled=autocast_state[0], dtype=autocast_state[1]):
                             return network(r6_, cn_)
-                    graphed = GraphedCall(net, r6, cn)
+                    graphed = GraphedCall(net, r6, cn, warmup=1)
                 r_update = graphed(r6, cn)
             else:
                 r_update = network(r6, cn)
