@@ -572,6 +572,51 @@ KFB_API int kfb_atom_stack_fwd(const kfb_atom_block* blocks, int n_blocks, const
                                const unsigned char* mask, int mask_share, int bias_share, void* workspace, size_t workspace_bytes,
                                int groups, int samples, int l, int c, int heads, int hidden, float eps, void* stream);
 
+/*
+ * A whole block of the pair stacks in one call: triangle multiplication out and in, optionally triangle attention starting and
+ * ending, transition, and optionally the single track (pair bias from LayerNorm(z), pair-bias attention, transition), every
+ * residual fused.  TriangularBlock.forward (src/kfold/model/modules/tri_stack.py:119-151), PairformerBlock.forward
+ * (apo_module.py:107-172), ConfidencePairSingleBlock.forward (confidence_head.py:125-175).
+ *   Weights as in the single operators' entry points (same packings).  z, z_out (batch, n, n, c) of z_dtype, s, s_out (batch, n,
+ *   c_s) of s_dtype; z_out may be z, s_out may be s; pair_mask (batch, n, n) and mask (batch, n) bytes.  Any n >= 24, or a
+ *   multiple of 8 (which the fp32-accurate mode, both dtypes KFB_FP32_PRECISE, always needs).
+ *   has_attention / has_single say which parts are present.
+ */
+typedef struct {
+  const float *ln_in_w, *ln_in_b;
+  const void *w_in, *w_gout;
+  const float *ln_out_w, *ln_out_b;
+  const void* w_pout;
+} kfb_trimul_weights;
+typedef struct {
+  const float *ln_w, *ln_b;
+  const void *w_proj, *w_out;
+} kfb_triatt_weights;
+typedef struct {
+  const float *ln_w, *ln_b;
+  const void *w_swiglu, *w_out;
+} kfb_transition_weights;
+typedef struct {
+  kfb_trimul_weights mul_out, mul_in;
+  kfb_triatt_weights att_start, att_end;
+  kfb_transition_weights trans_z;
+  const float *ln_z_w, *ln_z_b;
+  const void* w_bias;
+  const float *ln_s_w, *ln_s_b;
+  const void* w_proj;
+  const float* proj_bias;
+  const void* w_out;
+  const float* out_bias;
+  kfb_transition_weights trans_s;
+  int has_attention, has_single;
+  int c, c_s, tri_heads, heads, hidden_z, hidden_s;
+  float eps;
+} kfb_pair_block;
+KFB_API size_t kfb_pair_block_workspace_bytes(const kfb_pair_block* blk, int batch, int n, int precise);
+KFB_API int kfb_pair_block_fwd(const kfb_pair_block* blk, const void* z, void* z_out, int z_dtype, const void* s, void* s_out, int s_dtype,
+                               const unsigned char* pair_mask, const unsigned char* mask, void* workspace, size_t workspace_bytes,
+                               int batch, int n, void* stream);
+
 #ifdef __cplusplus
 }
 #endif

@@ -37,6 +37,27 @@ class AtomBlock(ctypes.Structure):
     _fields_ = [(n, c_void_p) for n in ("w_q", "q_bias", "w_kv", "w_out", "out_bias", "w_swiglu", "w_tout")]
 
 
+class TrimulWeights(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("ln_in_w", "ln_in_b", "w_in", "w_gout", "ln_out_w", "ln_out_b", "w_pout")]
+
+
+class TriattWeights(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("ln_w", "ln_b", "w_proj", "w_out")]
+
+
+class TransitionWeights(ctypes.Structure):
+    _fields_ = [(n, c_void_p) for n in ("ln_w", "ln_b", "w_swiglu", "w_out")]
+
+
+class PairBlock(ctypes.Structure):
+    _fields_ = ([("mul_out", TrimulWeights), ("mul_in", TrimulWeights), ("att_start", TriattWeights), ("att_end", TriattWeights),
+                 ("trans_z", TransitionWeights)]
+                + [(n, c_void_p) for n in ("ln_z_w", "ln_z_b", "w_bias", "ln_s_w", "ln_s_b", "w_proj", "proj_bias", "w_out", "out_bias")]
+                + [("trans_s", TransitionWeights)]
+                + [(n, c_int) for n in ("has_attention", "has_single", "c", "c_s", "tri_heads", "heads", "hidden_z", "hidden_s")]
+                + [("eps", c_float)])
+
+
 # name -> argtypes; every function returns int except where noted
 _SIGNATURES = {
     "kfb_version": [],
@@ -103,6 +124,8 @@ _SIGNATURES = {
     "kfb_center_coords": [c_void_p, c_void_p, c_void_p, c_int, c_int, c_int, c_void_p],
     "kfb_token_stack_fwd": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_ll, c_ll, c_ll, c_void_p,
                             c_void_p, ctypes.c_size_t] + [c_int] * 7 + [c_float, c_int, c_void_p],
+    "kfb_pair_block_fwd": [c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_int, c_void_p, c_void_p, c_void_p, ctypes.c_size_t,
+                           c_int, c_int, c_void_p],
     "kfb_atom_stack_fwd": [c_void_p, c_int, c_void_p, c_void_p, c_void_p, c_int, c_void_p, c_int, c_void_p, c_ll, c_void_p, c_int, c_int,
                            c_void_p, ctypes.c_size_t] + [c_int] * 6 + [c_float, c_void_p],
     "kfb_transition_fwd_static": [c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_void_p, c_ll, c_int, c_int,
@@ -128,6 +151,7 @@ _SIZE_FUNCS = {
     "kfb_apb_cross_workspace_bytes_precise": [c_int, c_int, c_int, c_int],
     "kfb_trimul_workspace_bytes": [c_int, c_int, c_int],
     "kfb_parcae_workspace_bytes": [c_ll, c_int],
+    "kfb_pair_block_workspace_bytes": [c_void_p, c_int, c_int, c_int],
     "kfb_token_stack_workspace_bytes": [c_int] * 8 + [c_ll, c_ll, c_int],
     "kfb_atom_stack_workspace_bytes": [c_int] * 7 + [c_ll, c_ll],
 }

@@ -15,7 +15,7 @@ from torch import nn
 
 from . import functional as F
 from .modules import (LayerNorm, LinearNoBias, SelfAttentionPairBias, Transition, TriangularBlock, _check_inference, _is_precise,
-                      _ProjectionCache, compute_dtype)
+                      _PairBlockPlan, _ProjectionCache, compute_dtype)
 
 __all__ = ["ConfidencePairSingleBlock", "ConfidencePairSingleStack", "ConfidenceHead"]
 
@@ -32,13 +32,20 @@ class ConfidencePairSingleBlock(nn.Module):
         self.attention = SelfAttentionPairBias(channel_s, num_heads, None, "confidence")
         self.transition = Transition(channel_s, expansion_factor=4)
         self._proj = _ProjectionCache()
+        self._plan = None
 
     @torch.compiler.disable
     def forward(self, z: torch.Tensor, s: torch.Tensor, pair_mask: torch.Tensor, mask: torch.Tensor):
         _check_inference(z)
-        z = self.pair_block(z, pair_mask)
         cd = compute_dtype(z)
         precise = _is_precise(cd, "ConfidencePairSingleBlock")
+        if cd == compute_dtype(s) and z.dim() == 4 and F.takes_any_n(z.shape[1], precise):      # one native call
+            if self._plan is None or not self._plan.fits(z.device, cd, precise):
+                pb = self.pair_block
+                self._plan = _PairBlockPlan(self, z.device, cd, precise, pb.tri_mul_out, pb.tri_mul_in, pb.transition_z, None,
+                                            (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
+            return F.pair_block(z, pair_mask, self._plan, s, mask, precise)
+        z = self.pair_block(z, pair_mask)
         ln = self.layernorm_z
         with torch.autocast(z.device.type, enabled=False):
             zz = z if z.dtype == cd else z.to(cd)

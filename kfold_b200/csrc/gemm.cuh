@@ -65,6 +65,7 @@ struct GemmParams {
   int k_inner;                    // launcher: != 0: both operands store K in pieces of k_inner elements (a multiple of the K
                                   // tile) that lie `s_k_hi` apart: K index = (k / k_inner, k % k_inner), five-dimensional maps
   const float2* row_stats;        // optional LayerNorm fold: out = rstd[row] * (acc - mean[row] * col_s1[col]) + col_s0[col]
+  int stats_pitch;                //   rows of consecutive o lie stats_pitch entries apart (0: n_extent)
   const float* col_s1;            //   (mean, rstd) per flat row; col_s1 = sum_k W'[col][k], col_s0 = sum_k beta[k] W[col][k]
   const float* col_s0;            //   with W' = gamma * W the matrix actually multiplied (applied before gate / residual)
   int swap_col_begin;             // launcher (BN = 128, plain epilogue): tiles whose first column is >= this hold channel-major
@@ -223,6 +224,15 @@ __device__ __forceinline__ void epi_store_chunk(const EpiSeg& sg, long long row_
         for (int i = 0; i < 4; ++i) d4[i] = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
       }
     }
+    return;
+  }
+  if (sg.vec && (nvalid & 7) == 0 && !sg.out_fp32) {   // the ragged last chunk of a row: whole 16-byte pieces
+    __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(sg.dst) + row_off + col_local;
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      if (8 * i < nvalid)
+        *reinterpret_cast<uint4*>(d + 8 * i) = make_uint4(pack_bf16x2(v[8 * i], v[8 * i + 1]), pack_bf16x2(v[8 * i + 2], v[8 * i + 3]),
+                                                          pack_bf16x2(v[8 * i + 4], v[8 * i + 5]), pack_bf16x2(v[8 * i + 6], v[8 * i + 7]));
     return;
   }
   // scalar path: per column; coalesced across the warp's lanes when s_n == 1 (channel-major output)
@@ -947,7 +957,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         }
         if (p.row_stats != nullptr && si == 0) {
           // folded LayerNorm of the A rows: acc was computed on the raw rows with gamma folded into the weights
-          const float2 st = row_ok ? p.row_stats[(static_cast<long long>(b) * p.o_extent + o) * p.n_extent + n] : make_float2(0.f, 1.f);
+          const float2 st = row_ok ? p.row_stats[(static_cast<long long>(b) * p.o_extent + o) * (p.stats_pitch > 0 ? p.stats_pitch : p.n_extent) + n] : make_float2(0.f, 1.f);
           const float4* s1 = reinterpret_cast<const float4*>(p.col_s1 + out_col);
           const float4* s0 = reinterpret_cast<const float4*>(p.col_s0 + out_col);
 #pragma unroll

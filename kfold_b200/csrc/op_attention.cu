@@ -29,9 +29,10 @@ size_t carve_triatt(TriattWs& w, void* base, int batch, int n, int c, int heads)
   const size_t pos = static_cast<size_t>(batch) * n * n;
   const int hdp = heads * dpad_of(c / heads);
   w.xn = cv.take<__nv_bfloat16>(pos * c);
+  const size_t pos_p = static_cast<size_t>(batch) * n * pitch16(n);
   w.qkg = cv.take<__nv_bfloat16>(pos * 3 * hdp);
-  w.vt = cv.take<__nv_bfloat16>(pos * hdp);
-  w.bias = cv.take<__nv_bfloat16>(pos * heads);
+  w.vt = cv.take<__nv_bfloat16>(pos_p * hdp);
+  w.bias = cv.take<__nv_bfloat16>(pos_p * heads);
   w.og = cv.take<__nv_bfloat16>(pos * c);
   return cv.off;
 }
@@ -210,7 +211,7 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
                            size_t workspace_bytes, int batch, int n, int c, int heads, float eps, int dtype, void* stream_) {
   KFB_CHECK_ARG(x && mask && w_proj_packed && w_out && out && workspace, "triatt: null pointer");
   KFB_CHECK_ARG(is_dtype(dtype), "triatt: bad dtype %d", dtype);
-  KFB_CHECK_ARG(batch >= 1 && n >= 8 && n % 8 == 0, "triatt: N=%d must be a positive multiple of 8 (pad in the caller)", n);
+  KFB_CHECK_ARG(batch >= 1 && n >= 1, "triatt: batch %d N=%d", batch, n);
   KFB_CHECK_ARG(heads >= 1 && c % heads == 0 && c % 8 == 0, "triatt: C=%d heads=%d", c, heads);
   const int d = c / heads;
   KFB_CHECK_ARG(d % 8 == 0 && d >= 16 && d <= 64, "triatt: head dim %d not in {16, 24, ..., 64}", d);
@@ -231,6 +232,7 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
   cudaStream_t stream = as_stream(stream_);
   const long long nn = static_cast<long long>(n) * n;
   const long long pos = nn * batch;
+  const int np = pitch16(n);     // row pitch of V^T and the bias planes; everything else has the caller's n
 
   KFB_TRY(launch_layernorm(stream, x, w.xn, ln_w, ln_b, pos, c, c, c, eps, dtype, KFB_BF16));
   // projection: rows walked as (b, o, n); for the ending node (o, n) = (second, first) pair index
@@ -248,19 +250,21 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
     sv.col_begin = 3 * hdp;
     sv.ncols = hdp;
     sv.dst = w.vt;
-    sv.s_col = n;
+    sv.s_col = np;
     sv.s_n = 1;
-    sv.s_o = static_cast<long long>(hdp) * n;
-    sv.s_b = static_cast<long long>(hdp) * nn;
+    sv.n_pad = np;
+    sv.s_o = static_cast<long long>(hdp) * np;
+    sv.s_b = static_cast<long long>(hdp) * np * n;
     EpiSeg& sb = p.seg[2];
     sb = {};
     sb.col_begin = 4 * hdp;
     sb.ncols = heads;
     sb.dst = w.bias;
-    sb.s_col = nn;
+    sb.s_col = static_cast<long long>(np) * n;
     sb.s_n = 1;
-    sb.s_o = n;
-    sb.s_b = static_cast<long long>(heads) * nn;
+    sb.n_pad = np;
+    sb.s_o = np;
+    sb.s_b = static_cast<long long>(heads) * np * n;
     GemmOperandA a = {w.xn, ending ? static_cast<long long>(n) * c : c, ending ? c : static_cast<long long>(n) * c, nn * c};
     GemmOperandB b = {w_proj_packed, c, 0};
     p.b_static = 1;
@@ -277,8 +281,8 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
     p.q = w.qkg; p.ldq = 3 * hdp; p.q_col0 = 0;
     p.k = w.qkg; p.ldk = 3 * hdp; p.k_col0 = hdp;
     p.g = w.qkg; p.ldg = 3 * hdp; p.g_col0 = 2 * hdp;
-    p.vt = w.vt; p.ldv = n;
-    p.bias = w.bias; p.ldb = n; p.bias_div = n;
+    p.vt = w.vt; p.ldv = np;
+    p.bias = w.bias; p.ldb = np; p.bias_div = n;
     p.mask = mask;
     p.mask_lo_extent = n;
     p.m_hi = nn;
@@ -451,12 +455,15 @@ KFB_API size_t kfb_pair_bias_workspace_bytes(int batch, int n, int c) {
   return align_up(static_cast<size_t>(batch) * n * n * c * sizeof(__nv_bfloat16), 256);
 }
 
+}  // extern "C"
+namespace kfb {
 // bias[b][h][i][j] = sum_c LN(z)[b][i][j][c] * W[h][c], stored bf16 head-major; with `transposed` the
 // last two indices are swapped (bias_out[b][h][j][i]).  z is (batch, rows, n, c): square on one GPU,
 // a row shard (rows < n) otherwise.
-static int pair_bias_impl(const void* z, const float* ln_w, const float* ln_b, const void* w, void* bias_out,
+int pair_bias_run(const void* z, const float* ln_w, const float* ln_b, const void* w, void* bias_out,
                           void* workspace, int batch, int rows, int n, int c, int heads, int transposed, float eps,
-                          int dtype, cudaStream_t stream) {
+                          int dtype, cudaStream_t stream, int pitch) {
+  if (pitch == 0) pitch = n;     // row pitch of the bias planes (untransposed)
   const long long rn = static_cast<long long>(rows) * n;
   __nv_bfloat16* zn = static_cast<__nv_bfloat16*>(workspace);
   KFB_TRY(launch_layernorm(stream, z, zn, ln_w, ln_b, rn * batch, c, c, c, eps, dtype, KFB_BF16));
@@ -471,15 +478,17 @@ static int pair_bias_impl(const void* z, const float* ln_w, const float* ln_b, c
   s.col_begin = 0;
   s.ncols = heads;
   s.dst = bias_out;
-  s.s_col = rn;
+  s.s_col = static_cast<long long>(rows) * pitch;
   s.s_n = transposed ? rows : 1;
-  s.s_o = transposed ? 1 : n;
-  s.s_b = static_cast<long long>(heads) * rn;
+  s.s_o = transposed ? 1 : pitch;
+  s.s_b = s.s_col * heads;
   GemmOperandA a = {zn, c, static_cast<long long>(n) * c, rn * c};
   GemmOperandB b = {w, c, 0};
   p.b_static = 1;
   return launch_gemm_bf16(stream, a, b, p, 0, "pair_bias_proj");
 }
+}  // namespace kfb
+extern "C" {
 
 KFB_API int kfb_pair_bias_fwd(const void* z, const float* ln_w, const float* ln_b, const void* w, void* bias_out,
                               void* workspace, size_t workspace_bytes, int batch, int n, int c, int heads, int transposed,
@@ -520,7 +529,7 @@ KFB_API int kfb_pair_bias_fwd(const void* z, const float* ln_w, const float* ln_
     return launch_gemm_bf16(stream, a, b, p, 0, "pair_bias_proj_precise");
   }
   KFB_CHECK_ARG(workspace_bytes >= kfb_pair_bias_workspace_bytes(batch, n, c), "pair_bias: workspace too small");
-  return pair_bias_impl(z, ln_w, ln_b, w, bias_out, workspace, batch, n, n, c, heads, transposed, eps, dtype, as_stream(stream_));
+  return pair_bias_run(z, ln_w, ln_b, w, bias_out, workspace, batch, n, n, c, heads, transposed, eps, dtype, as_stream(stream_), 0);
 }
 
 // Row-shard form: z (rows, n, c) -> bias_out bf16 [heads][rows][n].  workspace: rows*n*c bf16.
@@ -533,7 +542,7 @@ KFB_API int kfb_pair_bias_rows_fwd(const void* z, const float* ln_w, const float
                 "pair_bias_rows: rows %d n %d c %d heads %d", rows, n, c, heads);
   KFB_CHECK_ARG(workspace_bytes >= static_cast<size_t>(rows) * n * c * sizeof(__nv_bfloat16), "pair_bias_rows: workspace too small");
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "pair_bias_rows: workspace must be 256-byte aligned");
-  return pair_bias_impl(z, ln_w, ln_b, w, bias_out, workspace, 1, rows, n, c, heads, 0, eps, dtype, as_stream(stream_));
+  return pair_bias_run(z, ln_w, ln_b, w, bias_out, workspace, 1, rows, n, c, heads, 0, eps, dtype, as_stream(stream_), 0);
 }
 
 KFB_API size_t kfb_apb_workspace_bytes(int batch, int l, int c, int heads) {

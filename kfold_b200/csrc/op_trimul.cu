@@ -24,16 +24,20 @@ using namespace kfb;
 
 namespace {
 
+// Row pitch of the channel-major tensors: whole 16-byte units, which the tensor maps ask for.  Positions between n and the
+// pitch are never read: the maps' extents end at n.
+inline int pitch8(int n) { return (n + 7) / 8 * 8; }
+
 struct TrimulWs {
   __nv_bfloat16 *xn, *ab, *gl, *t;
 };
 size_t carve(TrimulWs& w, void* base, int batch, int n, int c) {
   Carver cv(base);
-  const size_t pos = static_cast<size_t>(batch) * n * n;
-  w.xn = cv.take<__nv_bfloat16>(pos * c);  // also reused as tn
-  w.ab = cv.take<__nv_bfloat16>(pos * 2 * c);
+  const size_t pos = static_cast<size_t>(batch) * n * n, pos_p = static_cast<size_t>(batch) * n * pitch8(n);
+  w.xn = cv.take<__nv_bfloat16>(pos_p * c);  // also reused as tn
+  w.ab = cv.take<__nv_bfloat16>(pos_p * 2 * c);
   w.gl = cv.take<__nv_bfloat16>(pos * c);
-  w.t = cv.take<__nv_bfloat16>(pos * c);
+  w.t = cv.take<__nv_bfloat16>(pos_p * c);
   return cv.off;
 }
 
@@ -69,10 +73,10 @@ int project(cudaStream_t stream, int transposed_walk, const void* x, const unsig
     s.out_fp32 = 0;
     s.vec = 0;
     s.dst = ab;
-    s.s_col = pos;
     s.s_n = 1;
-    s.s_o = p.n_extent;
-    s.s_b = rn;
+    s.s_o = rows == n ? pitch8(n) : p.n_extent;   // (shards keep the exchange layout)
+    s.s_b = s.s_o * p.o_extent;
+    s.s_col = s.s_b * batch;
     p.rowmask = mask;
     p.mask_segs = 1;
     p.m_b = rn;
@@ -101,12 +105,15 @@ int project(cudaStream_t stream, int transposed_walk, const void* x, const unsig
   return KFB_OK;
 }
 
-// steps 4-6.  a: [c][batch][rows][n]; b: pieces of [c][batch][b_piece_rows][n], `b_piece_stride` elements apart.
+// steps 4-6.  a: [c][batch][rows][np]; b: pieces of [c][batch][b_piece_rows][np], `b_piece_stride` elements apart; np = n rounded
+// up to the row pitch.  A ragged n costs nothing but tiles that end early: no padded copy of x, out or the mask is made.
 int finish(cudaStream_t stream, const __nv_bfloat16* a, const __nv_bfloat16* b, int b_piece_rows, long long b_piece_stride,
            const __nv_bfloat16* gl, const float* ln_out_w, const float* ln_out_b, const void* w_pout, __nv_bfloat16* t,
            __nv_bfloat16* tn, void* out, const void* resid, int batch, int rows, int n, int c, float eps, int dtype) {
   const long long rn = static_cast<long long>(rows) * n;
   const long long pos = rn * batch;
+  const int np = pitch8(n);
+  const long long rnp = static_cast<long long>(rows) * np, posp = rnp * batch;
   if (a != nullptr) {
     // t[ch*B+b][i][j] = sum_k A[i][k] B[j][k]
     GemmParams p = {};
@@ -117,9 +124,9 @@ int finish(cudaStream_t stream, const __nv_bfloat16* a, const __nv_bfloat16* b, 
     p.k_extent = n;
     p.b_batched = 1;
     p.nseg = 1;
-    p.seg[0] = row_major_seg(t, n, n, 0, rn, 0);
-    GemmOperandA oa = {a, n, 0, rn};
-    GemmOperandB ob = {b, n, static_cast<long long>(b_piece_rows) * n};
+    p.seg[0] = row_major_seg(t, np, np, 0, rnp, 0);
+    GemmOperandA oa = {a, np, 0, rnp};
+    GemmOperandB ob = {b, np, static_cast<long long>(b_piece_rows) * np};
     int force_bn = 0;
     if (b_piece_rows != n) {
       ob.col_inner = b_piece_rows;
@@ -130,8 +137,7 @@ int finish(cudaStream_t stream, const __nv_bfloat16* a, const __nv_bfloat16* b, 
   }
   // LayerNorm_out folded into the output projection: the GEMM reads t as it lies (channel-major, read MN-major), the
   // epilogue applies the per-position statistics.  The scratch buffer tn holds the folded weights and the statistics.
-  const bool fold = (c % kBK == 0) && (pos % 8 == 0) &&
-                    pos * static_cast<long long>(c) * 2 >= static_cast<long long>(c) * c * 2 + 256 + 2ll * c * 4 + 256 + pos * 8;
+  const bool fold = (c % kBK == 0) && posp * static_cast<long long>(c) * 2 >= static_cast<long long>(c) * c * 2 + 256 + 2ll * c * 4 + 256 + posp * 8;
   if (fold) {
     uint8_t* base = reinterpret_cast<uint8_t*>(tn);
     __nv_bfloat16* wf = reinterpret_cast<__nv_bfloat16*>(base);
@@ -139,29 +145,36 @@ int finish(cudaStream_t stream, const __nv_bfloat16* a, const __nv_bfloat16* b, 
     float* s0 = s1 + c;
     float2* stats = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(s1) + align_up(static_cast<size_t>(2) * c * 4, 256));
     KFB_TRY(launch_ln_fold_weights(stream, static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, wf, s1, s0, c, c));
-    KFB_TRY(launch_cm_stats(stream, t, stats, pos, c, pos, eps));
+    KFB_TRY(launch_cm_stats(stream, t, stats, posp, c, posp, eps));
+    // flat rows when there is no pitch, row by row otherwise (t's rows are np apart, out's n)
+    const bool flat = np == n;
     GemmParams p = {};
-    p.n_extent = static_cast<int>(pos);
-    p.o_extent = 1;
-    p.batch = 1;
+    p.n_extent = flat ? static_cast<int>(pos) : n;
+    p.o_extent = flat ? 1 : rows;
+    p.batch = flat ? 1 : batch;
     p.n_cols = c;
     p.k_extent = c;
     p.nseg = 1;
-    p.seg[0] = row_major_seg(out, c, c, 0, 0, dtype == KFB_FP32);
+    const long long oc = flat ? 0 : static_cast<long long>(n) * c, bc = flat ? 0 : rn * c;
+    p.seg[0] = row_major_seg(out, c, c, oc, bc, dtype == KFB_FP32);
     p.gate = gl;
     p.g_col = 1;
     p.g_n = c;
+    p.g_o = oc;
+    p.g_b = bc;
+    p.stats_pitch = flat ? 0 : np;
     p.resid = resid;
     p.row_stats = stats;
     p.col_s1 = s1;
     p.col_s0 = s0;
-    GemmOperandA oa = {t, 1, 0, 0};
-    oa.s_k = pos;
+    GemmOperandA oa = {t, 1, flat ? 0 : np, flat ? 0 : rnp};
+    oa.s_k = posp;
     GemmOperandB ob = {wf, c, 0};
     p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, oa, ob, p, 0, "trimul_out_proj"));
     return KFB_OK;
   }
+  KFB_CHECK_ARG(np == n, "trimul: N=%d too small for C=%d (pad to a multiple of 8)", n, c);
   KFB_TRY(launch_layernorm_cm(stream, t, tn, ln_out_w, ln_out_b, batch, rn, c, pos, rn, eps, KFB_BF16));
   {
     GemmParams p = {};
@@ -315,7 +328,9 @@ KFB_API int kfb_trimul_fwd(int incoming, const void* x, const unsigned char* mas
                            int batch, int n, int c, float eps, int dtype, void* stream_) {
   KFB_CHECK_ARG(x && mask && w_in_packed && w_gout && w_pout && out && workspace, "trimul: null pointer");
   KFB_CHECK_ARG(is_dtype(dtype), "trimul: bad dtype %d", dtype);
-  KFB_TRY(check_shape("trimul", batch, n, n, c));
+  // any N on the bf16 path (except tensors too small for the folded LayerNorm's scratch), multiples of 8 otherwise
+  const bool ragged_ok = dtype != KFB_FP32_PRECISE && n >= 24;
+  KFB_TRY(check_shape("trimul", batch, ragged_ok ? pitch8(n) : n, ragged_ok ? pitch8(n) : n, c));
   if (dtype == KFB_FP32_PRECISE) {
     KFB_CHECK_ARG(c <= 256, "trimul: the fp32-accurate mode supports at most 256 channels");
     TrimulWsPrecise wp;
@@ -330,9 +345,8 @@ KFB_API int kfb_trimul_fwd(int incoming, const void* x, const unsigned char* mas
   KFB_CHECK_ARG(workspace_bytes >= need, "trimul: workspace %zu < %zu bytes", workspace_bytes, need);
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "trimul: workspace must be 256-byte aligned");
   cudaStream_t stream = as_stream(stream_);
-  const long long pos = static_cast<long long>(batch) * n * n;
   KFB_TRY(project(stream, incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, w.xn, w.ab, w.gl, batch, n, n, c, eps, dtype));
-  return finish(stream, w.ab, w.ab + static_cast<long long>(c) * pos, n, 0, w.gl, ln_out_w, ln_out_b, w_pout, w.t, w.xn, out,
+  return finish(stream, w.ab, w.ab + static_cast<long long>(c) * batch * n * pitch8(n), n, 0, w.gl, ln_out_w, ln_out_b, w_pout, w.t, w.xn, out,
                 resid, batch, n, n, c, eps, dtype);
 }
 

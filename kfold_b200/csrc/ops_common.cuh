@@ -62,6 +62,10 @@ struct ApbArgs {
 };
 int apb_run(cudaStream_t stream, const ApbArgs& r);
 
+// bf16 pair bias (kfb_pair_bias_fwd) with bias rows `pitch` elements apart (0: n).
+int pair_bias_run(const void* z, const float* ln_w, const float* ln_b, const void* w, void* bias_out, void* workspace, int batch,
+                  int rows, int n, int c, int heads, int transposed, float eps, int dtype, cudaStream_t stream, int pitch);
+
 // Conditioned transition on AdaLN-normalised rows (kfb_cond_transition_fwd and the stacks).  x_is_split: precise mode, x is
 // already the triple split; w_static as in ApbArgs.
 int cond_transition_run(cudaStream_t stream, const void* x_normed, int x_is_split, int w_static, const void* w_swiglu, const void* w_out,

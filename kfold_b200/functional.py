@@ -55,8 +55,16 @@ def _require_cuda(*ts: torch.Tensor) -> None:
             raise RuntimeError("kfold_b200 kernels require CUDA tensors (there is no CPU path)")
 
 
-def _pad_pair(x: torch.Tensor, mask: torch.Tensor, mult: int = 8):
+def takes_any_n(n: int, precise: bool) -> bool:
+    """Whether the pair operators take this token count as it is: the bfloat16 kernels any count from 24 on, the float32-accurate
+    ones multiples of eight."""
+    return n % 8 == 0 or (n >= 24 and not precise)
+
+
+def _pad_pair(x: torch.Tensor, mask: torch.Tensor, precise: bool = True, mult: int = 8):
     n = x.shape[-2]
+    if takes_any_n(n, precise):
+        return x, mask, n
     npad = (n + mult - 1) // mult * mult
     if npad == n:
         return x, mask, n
@@ -98,12 +106,12 @@ def triangle_multiplication(x: torch.Tensor, mask: torch.Tensor, packed: dict, d
     c = x.shape[-1]
     if c != packed["c"]:
         raise ValueError(f"triangle_multiplication: channel mismatch {c} vs {packed['c']}")
-    xp, mp, n = _pad_pair(x.contiguous(), mask.to(torch.bool).contiguous())
+    precise = bool(packed.get("precise"))
+    xp, mp, n = _pad_pair(x.contiguous(), mask.to(torch.bool).contiguous(), precise)
     b, npad = xp.shape[0], xp.shape[1]
     mp8 = mp.view(torch.uint8)
     out = torch.empty_like(xp)
     lib = L.lib()
-    precise = bool(packed.get("precise"))
     if precise and xp.dtype != torch.float32:
         raise ValueError("the fp32-accurate mode takes float32 tensors")
     with L.on_device(x.device):
@@ -131,11 +139,11 @@ def triangle_attention(x: torch.Tensor, mask: torch.Tensor | None, packed: dict,
     c, heads = x.shape[-1], packed["heads"]
     if c != packed["c"]:
         raise ValueError(f"triangle_attention: channel mismatch {c} vs {packed['c']}")
-    xp, mp, n = _pad_pair(x.contiguous(), mask.to(torch.bool).contiguous())
+    precise = bool(packed.get("precise"))
+    xp, mp, n = _pad_pair(x.contiguous(), mask.to(torch.bool).contiguous(), precise)
     b, npad = xp.shape[0], xp.shape[1]
     out = torch.empty_like(xp)
     lib = L.lib()
-    precise = bool(packed.get("precise"))
     if precise and xp.dtype != torch.float32:
         raise ValueError("the fp32-accurate mode takes float32 tensors")
     with L.on_device(x.device):
@@ -317,6 +325,33 @@ def attention_pair_bias(x: torch.Tensor, pair_bias: torch.Tensor, mask: torch.Te
                                 gate_share, gate_ld, L.ptr(out), L.ptr(res), L.ptr(ws), ws.numel(), batch, lp, c, heads, bias_div,
                                 L.KFB_FP32_PRECISE if precise else L.dtype_code(out.dtype), L.stream_ptr()))
     return out[:, :l].reshape(*lead, l, c).to(want)
+
+
+def pair_block(z: torch.Tensor, pair_mask: torch.Tensor, plan, s: torch.Tensor | None = None, mask: torch.Tensor | None = None,
+               precise: bool = False):
+    """A block of the pair stacks in one native call: z (B, N, N, c), pair_mask (B, N, N) -> z, or (z, s) with the single track
+    s (B, N, c_s), mask (B, N).  `plan`: the block's packed weights (modules._PairBlockPlan)."""
+    _require_cuda(z, pair_mask, s, mask)
+    if z.dim() != 4 or z.shape[1] != z.shape[2] or pair_mask.shape != z.shape[:-1] or z.shape[-1] != plan.struct.c:
+        raise ValueError(f"pair_block: z {tuple(z.shape)} / pair_mask {tuple(pair_mask.shape)}")
+    b, n = z.shape[:2]
+    zc = (z.float() if precise else z).contiguous()
+    pm = pair_mask.to(torch.bool).contiguous()
+    z_out = torch.empty_like(zc)
+    sc = s_out = mk = None
+    code = lambda t: L.KFB_FP32_PRECISE if precise else L.dtype_code(t.dtype)
+    if s is not None:
+        if s.shape[:-1] != z.shape[:2] or mask.shape != z.shape[:2] or s.shape[-1] != plan.struct.c_s:
+            raise ValueError(f"pair_block: s {tuple(s.shape)} / mask {tuple(mask.shape)}")
+        sc, mk = (s.float() if precise else s).contiguous(), mask.to(torch.bool).contiguous()
+        s_out = torch.empty_like(sc)
+    lib = L.lib()
+    with L.on_device(z.device):
+        ws = _workspace(z.device, lib.kfb_pair_block_workspace_bytes(plan.ref, b, n, precise))
+        L.check(lib.kfb_pair_block_fwd(plan.ref, L.ptr(zc), L.ptr(z_out), code(zc), L.ptr(sc), L.ptr(s_out), 0 if sc is None else code(sc),
+                                       L.ptr(pm), L.ptr(mk), L.ptr(ws), ws.numel(), b, n, L.stream_ptr()))
+    z_out = z_out if z_out.dtype == z.dtype else z_out.to(z.dtype)
+    return z_out if s is None else (z_out, s_out if s_out.dtype == s.dtype else s_out.to(s.dtype))
 
 
 def token_stack(a: torch.Tensor, s: torch.Tensor, pair_bias: torch.Tensor, mask: torch.Tensor, plan, groups: int, samples: int,

@@ -1170,6 +1170,52 @@ class DiffusionStack(nn.Module):
 # --------------------------------------------------------------------------------------------
 # blocks
 # --------------------------------------------------------------------------------------------
+class _PairBlockPlan:
+    """The packed weights of a block of the pair stacks as the struct kfb_pair_block_fwd takes; `state` tells when they are stale."""
+
+    def __init__(self, root: nn.Module, device, dtype, precise: bool, mul_out, mul_in, trans_z, attention=None, single=None):
+        """`attention`: (starting, ending) or None; `single`: (layernorm_z, linear_pair_bias, attention, transition) or None."""
+        self.key, self.state = (device, dtype, precise), ParamState(root)
+        self.keep = []
+
+        def put(dst, packed: dict, **names):
+            for field, key in names.items():
+                t = packed[key]
+                self.keep.append(t)
+                setattr(dst, field, L.ptr(t))
+
+        k = self.struct = L.PairBlock()
+        for dst, mod in ((k.mul_out, mul_out), (k.mul_in, mul_in)):
+            pk = mod._packed(device, dtype, lambda sd, dev: packing.pack_trimul(sd, dev, precise=precise))
+            put(dst, pk, **{n: n for n in ("ln_in_w", "ln_in_b", "w_in", "w_gout", "ln_out_w", "ln_out_b", "w_pout")})
+        k.c, k.eps = pk["c"], mul_out.layernorm_in.eps
+        for dst, mod in zip((k.att_start, k.att_end), attention or ()):
+            pk = mod._packed(device, dtype, lambda sd, dev: packing.pack_triatt(sd, mod.no_heads, dev, precise=precise))
+            put(dst, pk, ln_w="ln_w", ln_b="ln_b", w_proj="w_proj", w_out="w_out")
+            k.has_attention, k.tri_heads = 1, mod.no_heads
+
+        def transition(dst, mod):
+            pk = mod._packed(device, dtype, lambda sd, dev: packing.pack_transition(sd, dev, precise=precise))
+            put(dst, pk, ln_w="ln_w", ln_b="ln_b", w_swiglu="w_swiglu", w_out="w_out")
+            return pk["hidden"]
+
+        k.hidden_z = transition(k.trans_z, trans_z)
+        if single is not None:
+            ln_z, lin, att, trans_s = single
+            f32 = lambda t: None if t is None else t.detach().to(device, torch.float32).contiguous()
+            w = lin.weight
+            small = {"zw": f32(ln_z.weight), "zb": f32(ln_z.bias), "sw": f32(att.layernorm_a.weight), "sb": f32(att.layernorm_a.bias),
+                     "wb": packing.split3_weights(w).to(device) if precise else w.detach().to(device, torch.bfloat16).contiguous()}
+            put(k, small, ln_z_w="zw", ln_z_b="zb", ln_s_w="sw", ln_s_b="sb", w_bias="wb")
+            put(k, att._apb_packed(device, precise), w_proj="w_proj", proj_bias="proj_bias", w_out="w_out", out_bias="out_bias")
+            k.has_single, k.c_s, k.heads = 1, att.channel_a, att.num_heads
+            k.hidden_s = transition(k.trans_s, trans_s)
+        self.ref = L.ref(k)
+
+    def fits(self, device, dtype, precise: bool) -> bool:
+        return self.key == (device, dtype, precise) and self.state.current()
+
+
 class TriangularBlock(nn.Module):
     """K-Fold trunk block: tri-mult out, tri-mult in, transition, residual adds fused into the kernels."""
 
@@ -1179,8 +1225,16 @@ class TriangularBlock(nn.Module):
         self.tri_mul_out = TriangleMultiplicationOutgoing(channel_z)
         self.tri_mul_in = TriangleMultiplicationIncoming(channel_z)
         self.transition_z = Transition(channel_z, expansion_factor=4)
+        self._plan = None
 
     def forward(self, z: torch.Tensor, pair_mask: torch.Tensor) -> torch.Tensor:
+        _check_inference(z)
+        cd = compute_dtype(z)
+        precise = _is_precise(cd, "TriangularBlock")
+        if z.dim() == 4 and F.takes_any_n(z.shape[1], precise):      # one native call
+            if self._plan is None or not self._plan.fits(z.device, cd, precise):
+                self._plan = _PairBlockPlan(self, z.device, cd, precise, self.tri_mul_out, self.tri_mul_in, self.transition_z)
+            return F.pair_block(z, pair_mask, self._plan, precise=precise)
         z = self.tri_mul_out(z, pair_mask, residual=True)
         z = self.tri_mul_in(z, pair_mask, residual=True)
         return self.transition_z(z, residual=True)
@@ -1206,6 +1260,7 @@ class PairformerBlock(nn.Module):
         self.transition = Transition(channel_s, expansion_factor=4)
         self._bias_w = None
         self._bias_key = None
+        self._plan = None
 
     def _pair_bias(self, z: torch.Tensor) -> torch.Tensor:
         p = self.linear_pair_bias.weight
@@ -1228,6 +1283,14 @@ class PairformerBlock(nn.Module):
     def forward(self, z: torch.Tensor, s: torch.Tensor, pair_mask: torch.Tensor, mask: torch.Tensor):
         """z (B,N,N,c_z), s (B,N,c_s), pair_mask (B,N,N), mask (B,N) -> (z, s)."""
         _check_inference(z)
+        cd = compute_dtype(z)
+        precise = _is_precise(cd, "PairformerBlock")
+        if cd == compute_dtype(s) and z.dim() == 4 and F.takes_any_n(z.shape[1], precise):      # one native call
+            if self._plan is None or not self._plan.fits(z.device, cd, precise):
+                self._plan = _PairBlockPlan(self, z.device, cd, precise, self.tri_mul_out, self.tri_mul_in, self.transition_z,
+                                            (self.tri_att_start, self.tri_att_end),
+                                            (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
+            return F.pair_block(z, pair_mask, self._plan, s, mask, precise)
         z = self.tri_mul_out(z, pair_mask, residual=True)
         z = self.tri_mul_in(z, pair_mask, residual=True)
         z = self.tri_att_start(z, pair_mask, residual=True)

@@ -1,0 +1,81 @@
+"""The native block and stack calls at the sizes where their kernels change form: ragged token counts around the row pitches and
+the GEMM tiles, several complexes and samples per call, in bfloat16 and float32, against the oracle."""
+import pytest
+import torch
+
+from helpers import err_stats
+from oracle import pairformer_oracle as O
+from test_gpu_parity import PRECISE_MAX_TOL, PRECISE_RMS_TOL, _check, _oracle_on
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.fixture(scope="module")
+def dev():
+    return torch.device("cuda:0")
+
+
+@pytest.fixture(autouse=True)
+def _no_grad_and_status():
+    from kfold_b200 import _lib as L
+    with torch.no_grad():
+        yield
+    assert L.device_status() == 0
+
+
+def _compare(out, ref, precise, what):
+    if precise:
+        mx, r = err_stats(out, ref)
+        assert mx < PRECISE_MAX_TOL and r < PRECISE_RMS_TOL, f"{what}: {mx:.3e} {r:.3e}"
+    else:
+        _check(*err_stats(out, ref), what)
+
+
+@pytest.mark.parametrize("n,batch,precise", [(8, 1, False), (24, 1, False), (25, 2, False), (63, 1, False), (129, 2, False), (257, 1, False),
+                                             (40, 2, True)])
+def test_pair_block_ragged(dev, n, batch, precise):
+    from kfold_b200 import modules as M
+    import synth
+    dt = torch.float32 if precise else torch.bfloat16
+    z, pm, m = synth.pair_inputs(n, n, 128, batch, valid=n - n // 10)
+    s = synth.single_inputs(n, n, 384, batch)
+    z, s = z.to(dt), s.to(dt)
+    w = synth.pairformer_block_weights(n, 128, 384)
+    blk = M.PairformerBlock(128, 384).to(dev)
+    blk.load_state_dict(w, strict=True)
+    zo, so = blk(z.to(dev), s.to(dev), pm.to(dev), m.to(dev))
+    assert zo.dtype == dt and so.dtype == dt
+
+    def run(z_, s_, pm_, m_, w_):
+        zr, sr = O.pairformer_block(z_, s_, pm_, m_, w_, row_chunk=32)
+        return torch.cat([zr.reshape(-1), sr.reshape(-1)])
+
+    ref = _oracle_on(dev, run, z.float(), s.float(), pm, m, w)
+    _compare(zo.float().cpu(), ref[: zo.numel()].view(zo.shape), precise, f"block N={n} z")
+    _compare(so.float().cpu(), ref[zo.numel():].view(so.shape), precise, f"block N={n} s")
+
+
+@pytest.mark.parametrize("l,groups,samples,own_s,precise", [(9, 1, 1, False, False), (37, 2, 3, False, False), (130, 1, 2, True, False),
+                                                            (33, 2, 2, True, True), (45, 1, 3, False, True)])
+def test_token_stack_ragged(dev, l, groups, samples, own_s, precise):
+    """Two blocks (c = 256, 8 heads x 32): shared and per-sample conditioning, bias given as an unpadded and as a pitched tensor."""
+    from kfold_b200 import modules as M
+    import synth
+    rng, blocks, c, heads = synth._Rng(l), 2, 256, 8
+    w = {}
+    for i in range(blocks):
+        w.update(synth._prefixed(f"blocks.{i}.attention", synth.apb_weights(rng, c, 384)))
+        w.update(synth._prefixed(f"blocks.{i}.transition", synth.conditioned_transition_weights(rng, c, 384)))
+    a = rng.normal(groups, samples, l, c)
+    s = rng.normal(groups, samples if own_s else 1, l, 384)
+    bias = rng.normal(groups, 1, blocks, heads, l, l)
+    mask = synth.token_mask(l, valid=l - l // 8).view(1, 1, l).expand(groups, 1, l).contiguous()
+    stack = M.CachedGlobalTransformerStack(c, 384, heads, blocks).to(dev)
+    stack.load_state_dict(w, strict=True)
+    ref = _oracle_on(dev, O.global_transformer_stack, a, s, bias, mask, w, heads, blocks)
+    pitched = torch.zeros(groups, 1, blocks, heads, l, (l + 15) // 16 * 16)
+    pitched[..., :l] = bias
+    for given in (bias.to(dev), pitched.to(dev)[..., :l]):
+        with torch.autocast("cuda", dtype=torch.bfloat16, enabled=not precise):
+            out = stack(a.to(dev), s.to(dev), given, mask.to(dev))
+        _compare(out.float().cpu(), ref, precise, f"token stack L={l}")
