@@ -49,6 +49,10 @@ static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorM
   using Cfg = GemmCfg<BN>;
   if (p.aux && Cfg::stages_for(Cfg::kAuxBytes) < 2) p.aux = 0;  // no room (BN = 256): fall back to direct loads
   p.stages = Cfg::stages_for(p.aux ? Cfg::kAuxBytes : Cfg::kStagingBytes);
+  if constexpr (BN == 32) {
+    KFB_CHECK_ARG(!p.precise && !p.glu && !p.aux, "32-column tiles exist for the plain kernel only");
+    return launch_variant<32, false, false, false>(stream, ta, tb, tout, p, tag);
+  } else {
   if constexpr (BN <= 128) {
     if (p.precise) {
       p.k_main_blocks = (p.k_extent / 6) / kBK;
@@ -71,6 +75,27 @@ static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorM
     if (p.aux) return launch_variant<BN, false, true, false>(stream, ta, tb, tout, p, tag);
   }
   return launch_variant<BN, false, false, false>(stream, ta, tb, tout, p, tag);
+  }
+}
+
+// Narrower tiles for GEMMs of few rows: with the default width a sampler step's projections of 96 tokens fill 6 to 32 of the 148
+// SMs, and a tile's time is the trip of its operands through one SM.  Modelled time of a width: waves x (K blocks x bytes of a
+// stage / 64 B per cycle + epilogue); it is only taken where the default leaves SMs idle, so that large GEMMs keep their tiles.
+// (The GLU kernels pair value and gate columns inside 128-channel blocks: 64 columns are their narrowest tile.)
+static int narrow_tile(const GemmParams& p, int bn) {
+  const long long sms = sm_count();
+  if (static_cast<long long>(p.num_m_tiles) * cdiv(p.n_cols, bn) >= sms) return bn;
+  const int num_k = cdiv(p.k_extent, kBK);
+  const int lo = p.glu ? 64 : 32;
+  double best = 1e30;
+  int pick = bn;
+  for (int w = bn; w >= lo; w /= 2) {
+    const long long tiles = static_cast<long long>(p.num_m_tiles) * cdiv(p.n_cols, w);
+    const double waves = static_cast<double>((tiles + sms - 1) / sms);
+    const double t = waves * (num_k * (16384.0 + 128.0 * w) / 64.0 + 600.0 + 12.0 * w);
+    if (t < best) { best = t; pick = w; }
+  }
+  return pick;
 }
 
 static long long* g_trace_buf = nullptr;
@@ -84,13 +109,16 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
                      const char* tag) {
   KFB_CHECK_ARG(p.n_extent > 0 && p.o_extent > 0 && p.batch > 0 && p.n_cols > 0 && p.k_extent > 0, "empty GEMM");
   KFB_CHECK_ARG(p.nseg >= 1 && p.nseg <= 3, "GEMM needs 1..3 output segments");
+  p.n_blocks = cdiv(p.n_extent, kBM);
+  p.num_m_tiles = p.n_blocks * p.o_extent * p.batch;
   int bn = force_bn;
   if (bn == 0) bn = p.n_cols >= 256 ? 256 : (p.n_cols > 64 ? 128 : 64);
+  if (!p.precise && a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0 && p.glu != GLU_SIGMOID) bn = narrow_tile(p, bn);
   if (p.precise && bn > 128) bn = 128;  // the fp32-accurate variant keeps four accumulators in tensor memory
   // One row-major float32 segment with a gate and / or a residual (the output projections of the sampler's float32 activation
   // stream): 128-column tiles whose epilogue moves gate, residual and output through per-warp shared-memory tiles.
   p.xpose = 0;
-  if (!p.precise && !p.glu && force_bn == 0 && bn >= 128 && p.nseg == 1 && a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0 &&
+  if (!p.precise && !p.glu && force_bn == 0 && p.nseg == 1 && a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0 &&
       (p.gate != nullptr || p.resid != nullptr) && p.resid_scale == nullptr) {
     const EpiSeg& sg = p.seg[0];
     const bool seg_ok = sg.out_fp32 && sg.vec && sg.s_col == 1 && sg.col_begin == 0 && !sg.split && sg.ncols % 32 == 0 &&
@@ -101,16 +129,14 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
                           p.g_b % 8 == 0);
     if (seg_ok && gate_ok) {
       p.xpose = 1;
-      bn = 128;
+      if (bn > 128) bn = 128;
     }
   }
-  KFB_CHECK_ARG(bn == 64 || bn == 128 || bn == 256, "unsupported BN %d", bn);
+  KFB_CHECK_ARG(bn == 32 || bn == 64 || bn == 128 || bn == 256, "unsupported BN %d", bn);
   if (p.precise) KFB_CHECK_ARG(p.k_extent % 6 == 0, "precise GEMM: K=%d is not six equal parts", p.k_extent);
   if (p.glu) KFB_CHECK_ARG(p.n_cols % bn == 0, "GLU GEMM needs n_cols (%d) to be a multiple of the N tile (%d)", p.n_cols, bn);
   for (int i = 0; i < p.nseg; ++i) KFB_CHECK_ARG(p.seg[i].col_begin % 32 == 0, "segment start must be a multiple of 32");
   p.trace = (g_trace_buf != nullptr && strcmp(g_trace_tag, tag) == 0) ? g_trace_buf : nullptr;
-  p.n_blocks = cdiv(p.n_extent, kBM);
-  p.num_m_tiles = p.n_blocks * p.o_extent * p.batch;
   p.num_n_tiles = cdiv(p.n_cols, bn);
 
   CUtensorMap ta, tb;
@@ -154,7 +180,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
     const uint64_t dims[4] = {(uint64_t)p.k_extent, (uint64_t)inner, (uint64_t)(p.n_cols / inner),
                               (uint64_t)(p.b_batched ? p.batch : 1)};
     const uint64_t str[3] = {(uint64_t)b.s_col * 2, (uint64_t)b.s_col_hi * 2, (uint64_t)b.s_b * 2};
-    const uint32_t box[4] = {kBK, (uint32_t)bn, 1, 1};
+    const uint32_t box[4] = {kBK, (uint32_t)(p.glu && !p.precise && bn < 256 ? bn / 2 : bn), 1, 1};
     KFB_TRY(make_tmap(&tb, b.ptr, 2, 4, dims, str, box, 128));
     }
   }
@@ -262,6 +288,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
     }
   }
   switch (bn) {
+    case 32: return launch_bn<32>(stream, ta, tb, tout, p, tag);
     case 64: return launch_bn<64>(stream, ta, tb, tout, p, tag);
     case 128: return launch_bn<128>(stream, ta, tb, tout, p, tag);
     default: return launch_bn<256>(stream, ta, tb, tout, p, tag);

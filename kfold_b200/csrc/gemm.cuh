@@ -56,7 +56,7 @@ struct GemmParams {
   int swap_staged;                // launcher: the swapped GLU tile leaves through shared memory and TMA stores (map tm_out0)
   int rm_seg, rm_slot;            // launcher: segment whose full tiles leave through shared memory and a TMA store (row-major
                                   // bf16; BN = 128 plain kernel), and the output map it uses; rm_seg < 0: none
-  int xpose;                      // launcher (BN = 128 plain kernel, one row-major float32 segment with gate / residual):
+  int xpose;                      // launcher (plain kernel, BN <= 128, one row-major float32 segment with gate / residual):
                                   // every warp moves its 32 x 32 chunk of gate, residual and output through a private
                                   // shared-memory tile, so that global memory sees whole 128-byte rows
   int glu;                        // GluMode; with GLU a BN tile holds BN/2 values then BN/2 gates
@@ -110,7 +110,8 @@ struct GemmCfg {
   // output tiles (two 64-column boxes of [128 rows][128 bytes] each) on their way to a TMA store
   static constexpr int kSlabBytes = (kEpiWarps / 4) * 2 * 32 * kBM * 2;
   static constexpr int kRowTileBytes = kBM * 128 * 2;
-  static constexpr int kStagingBytes = (BN == 128) ? 2 * kRowTileBytes : kSlabBytes;
+  static constexpr int kXposeBytes = kEpiWarps * 6144;     // per-warp tiles of the float32 gate / residual route
+  static constexpr int kStagingBytes = (BN == 128) ? 2 * kRowTileBytes : (BN < 128 ? kXposeBytes : kSlabBytes);
   // the GLU kernel at BN = 256 writes 128 output columns per tile: the same two row-major tile buffers
   static constexpr int kGluStagingBytes = (BN == 256) ? 2 * kRowTileBytes : kStagingBytes;
   // swapped-orientation GLU kernel (BN = 256): the tile's position mask (1 KB, two accumulators) and two whole
@@ -300,6 +301,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   constexpr int ACC_COLS = PRECISE ? 2 * BN : BN;  // precise: main accumulator, then the correction accumulator
   static_assert(!PRECISE || BN <= 128, "the fp32-accurate variant needs four accumulators of BN columns");
   static_assert(!SWAP || (BN == 256 && GLU && !AUX && !PRECISE), "the swapped orientation exists for the BN = 256 GLU tile");
+  constexpr bool kSplitGlu = GLU && !PRECISE && BN < 256;
+  constexpr bool kXpose = BN <= 128 && !GLU && !AUX && !PRECISE;
   constexpr bool kPlain128 = (BN == 128 && !GLU && !AUX && !PRECISE);  // the variant that may swap single tiles
 
   extern __shared__ uint8_t smem_raw[];
@@ -362,13 +365,23 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   // weight half of the first tile's stages before it waits: for the few-row GEMMs of the samplers, whose time is the latency of
   // one tile, that takes the weights' trip from HBM off the critical path.
   int b_ahead = 0;
+  // GLU tiles narrower than the packing's blocks (128 value rows, then the 128 gate rows of the same channels): two boxes
+  auto load_glu_b = [&](int stage, int n_tile, int kb) {
+    const int v0 = n_tile * (BN / 2);
+    const int row = (v0 / 128) * 256 + (v0 % 128);
+    ptx::tma_load_4d(s_b + stage * Cfg::kBStage, &tm_b, &full_bar[stage], kb * kBK, row, 0, 0);
+    ptx::tma_load_4d(s_b + stage * Cfg::kBStage + Cfg::kBStage / 2, &tm_b, &full_bar[stage], kb * kBK, row + 128, 0, 0);
+  };
   if (warp == 0 && lane == 0 && p.b_static && !p.k_inner) {
     const int n_tile = static_cast<int>(blockIdx.x) % p.num_n_tiles;
     const int b_col_hi = (n_tile * BN) / p.b_col_inner;
     b_ahead = num_k < kStages ? num_k : kStages;
     for (int kb = 0; kb < b_ahead; ++kb) {
       ptx::mbar_expect_tx(&full_bar[kb], Cfg::kStageBytes);
-      ptx::tma_load_4d(s_b + kb * Cfg::kBStage, &tm_b, &full_bar[kb], kb * kBK, n_tile * BN - b_col_hi * p.b_col_inner, b_col_hi, 0);
+      if constexpr (kSplitGlu)
+        load_glu_b(kb, n_tile, kb);
+      else
+        ptx::tma_load_4d(s_b + kb * Cfg::kBStage, &tm_b, &full_bar[kb], kb * kBK, n_tile * BN - b_col_hi * p.b_col_inner, b_col_hi, 0);
     }
   }
   grid_dependency_wait();
@@ -428,7 +441,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             continue;
           } else
           ptx::tma_load_4d(s_a + stage * Cfg::kAStage, &tm_a, &full_bar[stage], kb * kBK, nb * kBM, o, b);
-          if (!b_done)
+          if constexpr (kSplitGlu) {
+            if (!b_done) load_glu_b(stage, n_tile, kb);
+          } else if (!b_done)
             ptx::tma_load_4d(s_b + stage * Cfg::kBStage, &tm_b, &full_bar[stage], kb * kBK, b_col_lo, b_col_hi, bb);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
@@ -514,6 +529,34 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                          static_cast<long long>(n) * p.m_n));
       return raw;
     };
+    // Float32 route (GemmParams::xpose): this warp's shared-memory tile, and the lane-contiguous asynchronous copies that bring
+    // the gate logits (32 rows x 64 bytes) and the residual (32 rows x 128 bytes) of one 32-column chunk into it.
+    uint8_t* xp_res = s_stage_out + (warp - 2) * 6144;
+    uint8_t* xp_gate = xp_res + 4096;
+    int xp_nb = 0, xp_o = 0, xp_b = 0;
+    auto xp_fetch = [&](int out_col) {
+      const EpiSeg& s0 = p.seg[0];
+      const int n_first = xp_nb * kBM + quad * 32;
+      if (p.resid != nullptr) {
+        const float* rbase = reinterpret_cast<const float*>(p.resid) + static_cast<long long>(xp_b) * s0.s_b +
+                             static_cast<long long>(xp_o) * s0.s_o + out_col;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int rr = i * 4 + (lane >> 3), pc = lane & 7;
+          if (n_first + rr < p.n_extent)
+            ptx::cp_async_16(xp_res + rr * 128 + ((pc ^ (rr & 7)) << 4), rbase + static_cast<long long>(n_first + rr) * s0.s_n + pc * 4);
+        }
+      }
+      if (p.gate != nullptr) {
+        const __nv_bfloat16* gbase = p.gate + static_cast<long long>(xp_b) * p.g_b + static_cast<long long>(xp_o) * p.g_o + out_col;
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const int rr = i * 8 + (lane >> 2), pc = lane & 3;
+          if (n_first + rr < p.n_extent)
+            ptx::cp_async_16(xp_gate + rr * 64 + ((pc ^ ((rr >> 1) & 3)) << 4), gbase + static_cast<long long>(n_first + rr) * p.g_n + pc * 8);
+        }
+      }
+    };
     TileIdx tile_cur = tile_decompose(static_cast<int>(blockIdx.x), p);
     uint32_t mask_next = load_mask(blockIdx.x, tile_cur);
     for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++tile_iter, tile_advance(tile_cur, p)) {
@@ -528,6 +571,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       }
       const uint32_t acc = tile_iter & 1;
       const uint32_t acc_phase = (tile_iter >> 1) & 1;
+      if constexpr (kXpose) {
+        const int out_col = n_tile * BN + chunk_phase * 32;
+        xp_nb = nb; xp_o = o; xp_b = b;
+        if (p.xpose && chunk_phase * 32 < BN && out_col + 32 <= p.seg[0].ncols) xp_fetch(out_col);
+      }
       if (!ptx::mbar_wait(&tmem_full[acc], acc_phase, 104)) { ok = false; break; }
       if (threadIdx.x == 64) KFB_GSTAMP(4 + tile_iter * 4 + 0);
       ptx::tc_fence_after_sync();
@@ -859,37 +907,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         // tile with lane-contiguous asynchronous copies, issued here so that they fly under the tensor-memory load, and
         // writes the result back the same way.  Only warp-level synchronisation is involved.
         bool xp = false;
-        uint8_t* xp_res = nullptr;
-        uint8_t* xp_gate = nullptr;
-        if constexpr (BN == 128 && !GLU && !AUX && !PRECISE) {
+        if constexpr (kXpose) {
           xp = p.xpose != 0 && out_col + 32 <= p.seg[0].ncols;   // uniform across the warp
-          if (xp) {
-            const EpiSeg& s0 = p.seg[0];
-            xp_res = s_stage_out + (warp - 2) * 6144;
-            xp_gate = xp_res + 4096;
-            const int n_first = nb * kBM + quad * 32;
-            if (p.resid != nullptr) {
-              const float* rbase = reinterpret_cast<const float*>(p.resid) + static_cast<long long>(b) * s0.s_b +
-                                   static_cast<long long>(o) * s0.s_o + out_col;
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                const int rr = i * 4 + (lane >> 3), pc = lane & 7;
-                if (n_first + rr < p.n_extent)
-                  ptx::cp_async_16(xp_res + rr * 128 + ((pc ^ (rr & 7)) << 4),
-                                   rbase + static_cast<long long>(n_first + rr) * s0.s_n + pc * 4);
-              }
-            }
-            if (p.gate != nullptr) {
-              const __nv_bfloat16* gbase = p.gate + static_cast<long long>(b) * p.g_b + static_cast<long long>(o) * p.g_o + out_col;
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                const int rr = i * 8 + (lane >> 2), pc = lane & 3;
-                if (n_first + rr < p.n_extent)
-                  ptx::cp_async_16(xp_gate + rr * 64 + ((pc ^ ((rr >> 1) & 3)) << 4),
-                                   gbase + static_cast<long long>(n_first + rr) * p.g_n + pc * 8);
-              }
-            }
-          }
+          if (xp && c != chunk_phase * 32) xp_fetch(out_col);     // (the first chunk's copies went out before the accumulator was ready)
         }
         float v[32];
         if (GLU && !PRECISE) {
@@ -1008,7 +1028,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         }
         const long long row_off = static_cast<long long>(b) * sg.s_b + static_cast<long long>(o) * sg.s_o +
                                   static_cast<long long>(n) * sg.s_n;
-        if constexpr (BN == 128 && !GLU && !AUX && !PRECISE) {
+        if constexpr (kXpose) {
           if (xp) {
             const int rl = lane;   // this thread's row within the warp's 32
             ptx::cp_async_wait_all();
