@@ -361,6 +361,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
+  TileIdx first_tile = tile_decompose(static_cast<int>(blockIdx.x), p);   // (its divisions run before the wait, too)
+
   // Everything above ran under the tail of the launch before this one (programmatic launch).  The producer also fetches the
   // weight half of the first tile's stages before it waits: for the few-row GEMMs of the samplers, whose time is the latency of
   // one tile, that takes the weights' trip from HBM off the critical path.
@@ -372,8 +374,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     ptx::tma_load_4d(s_b + stage * Cfg::kBStage, &tm_b, &full_bar[stage], kb * kBK, row, 0, 0);
     ptx::tma_load_4d(s_b + stage * Cfg::kBStage + Cfg::kBStage / 2, &tm_b, &full_bar[stage], kb * kBK, row + 128, 0, 0);
   };
-  if (warp == 0 && lane == 0 && p.b_static && !p.k_inner) {
-    const int n_tile = static_cast<int>(blockIdx.x) % p.num_n_tiles;
+  if (warp == 0 && p.b_static && !p.k_inner && ptx::elect_one()) {
+    const int n_tile = first_tile.n_tile;
     const int b_col_hi = (n_tile * BN) / p.b_col_inner;
     b_ahead = num_k < kStages ? num_k : kStages;
     for (int kb = 0; kb < b_ahead; ++kb) {
@@ -388,17 +390,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
-    if (lane == 0) {
+    if (ptx::elect_one()) {   // (elect.sync, not lane == 0: the compiler then knows one thread runs this, see ptx.cuh)
       int stage = 0;
       uint32_t phase = 0;  // ring position, advanced without divisions (the ring depth is a run-time value)
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x) {
-        const int m_tile = tile / p.num_n_tiles;
-        const int n_tile = tile - m_tile * p.num_n_tiles;
-        const int nb = m_tile % p.n_blocks;
-        const int rest = m_tile / p.n_blocks;
-        const int o = rest % p.o_extent;
-        const int b = rest / p.o_extent;
+      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, tile_advance(first_tile, p)) {
+        const int n_tile = first_tile.n_tile, nb = first_tile.nb, o = first_tile.o, b = first_tile.b;
         const int bb = p.b_batched ? b : 0;
         // the next kernel's blocks may take this SM over as soon as this CTA is on its last tile
         if (tile + static_cast<int>(gridDim.x) >= total_tiles) grid_dependency_launch();
@@ -452,7 +449,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (lane == 0) {
+    if (ptx::elect_one()) {
       constexpr uint32_t idesc = ptx::make_idesc(kBM, BN, /*bf16*/ 1);
       uint32_t tile_iter = 0;
       int stage = 0;
@@ -557,7 +554,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         }
       }
     };
-    TileIdx tile_cur = tile_decompose(static_cast<int>(blockIdx.x), p);
+    TileIdx tile_cur = first_tile;
     uint32_t mask_next = load_mask(blockIdx.x, tile_cur);
     for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++tile_iter, tile_advance(tile_cur, p)) {
       const int n_tile = tile_cur.n_tile, nb = tile_cur.nb, o = tile_cur.o, b = tile_cur.b;

@@ -37,6 +37,9 @@ __device__ __forceinline__ uint32_t lane_id() {
   asm volatile("mov.u32 %0, %laneid;" : "=r"(l));
   return l;
 }
+// One lane of a converged warp.  Guarding single-thread TMA / tcgen05 issue with this rather than with `lane == 0` lets the compiler
+// keep the instructions' uniform-register operands uniform: a K block's issue (wait, four MMAs, commit) takes 364 cycles instead of
+// 561, a producer step 350 instead of 600 (clock stamps, 128 x 32 tiles).
 __device__ __forceinline__ bool elect_one() {
   uint32_t pred;
   asm volatile(
