@@ -37,8 +37,8 @@ static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUte
   }
   {
     LaunchScope scope(stream, tag);
-    KFB_TRY(launch_kernel(stream, gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP>, grid, kGemmThreads, Cfg::kSmemBytes, ta, tb, tout[0],
-                          tout[1], q));
+    KFB_TRY(launch_kernel(stream, gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP>, grid,
+                          AUX ? kAuxThreads : kGemmThreads, Cfg::kSmemBytes, ta, tb, tout[0], tout[1], tout[2], q));
   }
   return KFB_OK;
 }
@@ -47,8 +47,7 @@ template <int BN>
 static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* tout,
                      GemmParams p, const char* tag) {
   using Cfg = GemmCfg<BN>;
-  if (p.aux && Cfg::stages_for(Cfg::kAuxBytes) < 2) p.aux = 0;  // no room (BN = 256): fall back to direct loads
-  p.stages = Cfg::stages_for(p.aux ? Cfg::kAuxBytes : Cfg::kStagingBytes);
+  p.stages = Cfg::stages_for(p.aux ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes : Cfg::kStagingBytes);
   if constexpr (BN == 32) {
     KFB_CHECK_ARG(!p.precise && !p.glu && !p.aux, "32-column tiles exist for the plain kernel only");
     return launch_variant<32, false, false, false>(stream, ta, tb, tout, p, tag);
@@ -71,7 +70,7 @@ static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorM
     p.stages = Cfg::stages_for(Cfg::kGluStagingBytes);
     return launch_variant<BN, true, false, false>(stream, ta, tb, tout, p, tag);
   }
-  if constexpr (BN <= 128) {
+  if constexpr (BN >= 64) {
     if (p.aux) return launch_variant<BN, false, true, false>(stream, ta, tb, tout, p, tag);
   }
   return launch_variant<BN, false, false, false>(stream, ta, tb, tout, p, tag);
@@ -132,6 +131,31 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
       if (bn > 128) bn = 128;
     }
   }
+  // Gate / residual prefetch and staged output: one row-major bf16 segment of whole 32-column chunks, aligned strides.  Two buffers
+  // of 128-column tiles (each set is loaded while the one before is in the epilogue); with a long K and the residual only, one
+  // buffer of 256-column tiles: its load hides behind the K loop, and A is read once.
+  p.aux = p.aux_gate = p.aux_resid = 0;
+  p.aux_bufs = 2;
+  if (!p.precise && !p.xpose && !p.glu && p.nseg == 1 && p.seg[0].vec && !p.seg[0].out_fp32 && p.seg[0].s_col == 1 &&
+      p.seg[0].col_begin == 0 && p.seg[0].ncols == p.n_cols && (p.gate != nullptr || p.resid != nullptr) && bn >= 64 && p.n_cols % 32 == 0) {
+    const EpiSeg& sg = p.seg[0];
+    const bool ok_o = (reinterpret_cast<uintptr_t>(sg.dst) & 15) == 0 && sg.s_n % 8 == 0 && sg.s_o % 8 == 0 && (sg.s_o != 0 || p.o_extent == 1) &&
+                      sg.s_b % 8 == 0 && (sg.s_b != 0 || p.batch == 1);
+    const bool ok_g = p.gate == nullptr || (p.g_col == 1 && (reinterpret_cast<uintptr_t>(p.gate) & 15) == 0 && p.g_n % 8 == 0 && p.g_n != 0 &&
+                                            p.g_o % 8 == 0 && (p.g_o != 0 || p.o_extent == 1) && p.g_b % 8 == 0 && (p.g_b != 0 || p.batch == 1));
+    const bool ok_r = p.resid == nullptr || (reinterpret_cast<uintptr_t>(p.resid) & 15) == 0;
+    if (ok_o && ok_g && ok_r) {
+      p.aux = 1;
+      p.aux_gate = p.gate != nullptr;
+      p.aux_resid = p.resid != nullptr;
+      if (bn == 256) {
+        if (p.k_extent >= 512 && p.aux_gate + p.aux_resid == 1)
+          p.aux_bufs = 1;
+        else
+          bn = 128;
+      }
+    }
+  }
   KFB_CHECK_ARG(bn == 32 || bn == 64 || bn == 128 || bn == 256, "unsupported BN %d", bn);
   if (p.precise) KFB_CHECK_ARG(p.k_extent % 6 == 0, "precise GEMM: K=%d is not six equal parts", p.k_extent);
   if (p.glu) KFB_CHECK_ARG(p.n_cols % bn == 0, "GLU GEMM needs n_cols (%d) to be a multiple of the N tile (%d)", p.n_cols, bn);
@@ -185,9 +209,8 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
     }
   }
   // channel-major bf16 segments that satisfy the TMA alignment rules are stored through shared memory
-  CUtensorMap tout[2];
-  tout[0] = ta;  // placeholders (never dereferenced unless a segment selects them)
-  tout[1] = ta;
+  CUtensorMap tout[3];
+  tout[0] = tout[1] = tout[2] = ta;  // placeholders (never dereferenced unless a segment selects them)
   int next_slot = 0;
   // a sigmoid-GLU GEMM whose only output is channel-major bf16 is computed in the swapped orientation
   p.swap = (p.glu == GLU_SIGMOID && bn == 256 && p.nseg == 1 && !p.precise && p.seg[0].s_n == 1 && p.seg[0].s_col != 1 &&
@@ -235,35 +258,16 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
       sg.tma_slot = next_slot++;
     }
   }
-  // gate / residual prefetch: only without staged segments, bf16 tensors, full 32-column chunks, aligned strides
-  p.aux = 0;
-  p.aux_gate = 0;
-  p.aux_resid = 0;
-  if (!p.precise && !p.xpose && next_slot == 0 && p.nseg == 1 && p.seg[0].vec && (p.gate != nullptr || p.resid != nullptr) &&
-      bn >= 64 && p.n_cols % 32 == 0 && !p.glu) {
+  if (p.aux) {
+    KFB_CHECK_ARG(next_slot == 0, "GEMM: gate / residual prefetch beside a staged segment");
     const EpiSeg& sg = p.seg[0];
-    bool ok_g = true, ok_r = true;
-    if (p.gate != nullptr)
-      ok_g = p.g_col == 1 && (reinterpret_cast<uintptr_t>(p.gate) & 15) == 0 && p.g_n % 8 == 0 && p.g_n != 0 &&
-             p.g_o % 8 == 0 && (p.g_o != 0 || p.o_extent == 1) && p.g_b % 8 == 0 && (p.g_b != 0 || p.batch == 1);
-    if (p.resid != nullptr)
-      ok_r = !sg.out_fp32 && (reinterpret_cast<uintptr_t>(p.resid) & 15) == 0 && sg.s_n % 8 == 0 && sg.s_o % 8 == 0 &&
-             (sg.s_o != 0 || p.o_extent == 1) && sg.s_b % 8 == 0 && (sg.s_b != 0 || p.batch == 1);
-    if (ok_g && ok_r) {
-      const uint32_t box[4] = {64, kBM, 1, 1};
-      const uint64_t dims[4] = {(uint64_t)p.n_cols, (uint64_t)p.n_extent, (uint64_t)p.o_extent, (uint64_t)p.batch};
-      if (p.gate != nullptr) {
-        const uint64_t str[3] = {(uint64_t)p.g_n * 2, (uint64_t)p.g_o * 2, (uint64_t)p.g_b * 2};
-        KFB_TRY(make_tmap(&tout[0], p.gate, 2, 4, dims, str, box, 128));
-        p.aux_gate = 1;
-      }
-      if (p.resid != nullptr) {
-        const uint64_t str[3] = {(uint64_t)sg.s_n * 2, (uint64_t)sg.s_o * 2, (uint64_t)sg.s_b * 2};
-        KFB_TRY(make_tmap(&tout[1], p.resid, 2, 4, dims, str, box, 128));
-        p.aux_resid = 1;
-      }
-      p.aux = 1;
-    }
+    const uint32_t box[4] = {64, kBM, 1, 1};
+    const uint64_t dims[4] = {(uint64_t)p.n_cols, (uint64_t)p.n_extent, (uint64_t)p.o_extent, (uint64_t)p.batch};
+    const uint64_t ostr[3] = {(uint64_t)sg.s_n * 2, (uint64_t)sg.s_o * 2, (uint64_t)sg.s_b * 2};
+    const uint64_t gstr[3] = {(uint64_t)p.g_n * 2, (uint64_t)p.g_o * 2, (uint64_t)p.g_b * 2};
+    if (p.aux_gate) KFB_TRY(make_tmap(&tout[0], p.gate, 2, 4, dims, gstr, box, 128));
+    if (p.aux_resid) KFB_TRY(make_tmap(&tout[1], p.resid, 2, 4, dims, ostr, box, 128));
+    KFB_TRY(make_tmap(&tout[2], sg.dst, 2, 4, dims, ostr, box, 128));
   }
   // full tiles of one row-major bf16 segment of the plain BN = 128 kernel leave through shared memory and a TMA store
   p.rm_seg = -1;

@@ -87,8 +87,10 @@ struct GemmParams {
   int b_static;                   // B is a weight matrix that the stream finished writing before the previous launch: its first
                                   // tiles are fetched while that launch still drains
   int stages;                     // depth of the operand ring (launcher)
-  int aux;                        // 1: gate / residual tiles are prefetched into shared memory by TMA (launcher)
+  int aux;                        // 1: gate / residual tiles are prefetched into shared memory by TMA, the output tile is built in
+                                  // place of one of them and leaves by TMA (launcher; bf16 output)
   int aux_gate, aux_resid;        // which of the two the prefetch covers
+  int aux_bufs;                   // 1 or 2 sets of those tiles
   long long* trace;               // debugging aid: CTA 0 stores clock64() stamps per tile here when non-null
   const void* resid;              // optional: seg 0 value += resid[...] (same dtype and strides as seg 0 dst)
   const float* resid_scale;       // optional, per output column: seg 0 value += resid_scale[col] * resid[...] instead
@@ -99,6 +101,7 @@ static constexpr int kBM = 128;
 static constexpr int kBK = 64;   // bf16 elements = 128 bytes = one swizzle span
 static constexpr int kEpiWarps = 8;  // two warps per TMEM lane quadrant, each taking every other 32-column chunk
 static constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
+static constexpr int kAuxThreads = kGemmThreads + 32;  // the AUX variant's last warp hands finished tiles to the copy engine
 
 template <int BN>
 struct GemmCfg {
@@ -119,10 +122,9 @@ struct GemmCfg {
   static constexpr int kSwapStagingBytes = 1024 + 2 * kRowTileBytes;
   static constexpr int kBarrierBytes = 512;
   static constexpr int kSmemBytes = 232448 - 1024;        // everything an SM offers one CTA
-  // after the operand ring comes EITHER the channel-major staging slabs OR two buffers of prefetched
-  // gate + residual tiles (128 rows x BN columns bf16 each); the launcher picks the ring depth accordingly
+  // after the operand ring comes EITHER the channel-major staging slabs OR one or two buffers of prefetched
+  // gate and / or residual tiles (128 rows x BN columns bf16 each); the launcher picks the ring depth accordingly
   static constexpr int kAuxTileBytes = kBM * BN * 2;
-  static constexpr int kAuxBytes = 2 * 2 * kAuxTileBytes;
   static constexpr int stages_for(int extra_bytes) {
     const int fit = (kSmemBytes - 1024 - extra_bytes - kBarrierBytes) / kStageBytes;
     return fit < kMaxStages ? fit : kMaxStages;
@@ -290,11 +292,11 @@ __device__ __forceinline__ void tile_advance(TileIdx& t, const GemmParams& p) {
 //         tile are the M operands of two N=128 MMAs and the 128 positions are the N operand.  A thread then holds
 //         consecutive positions of ONE channel and writes them with 32-byte stores: no transpose through shared memory.
 template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false>
-__global__ void __launch_bounds__(kGemmThreads, 1)
+__global__ void __launch_bounds__(AUX ? kAuxThreads : kGemmThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                  const __grid_constant__ CUtensorMap tm_out0, const __grid_constant__ CUtensorMap tm_out1,
-                 const GemmParams p) {
-  // tm_out0 / tm_out1: TMA-store maps of channel-major segments, or (p.aux) the gate / residual load maps
+                 const __grid_constant__ CUtensorMap tm_out2, const GemmParams p) {
+  // tm_out0 / tm_out1: TMA-store maps of channel-major segments, or (p.aux) the gate / residual load maps and, tm_out2, the output
   using Cfg = GemmCfg<BN>;
   const int kStages = p.stages;
   constexpr int OUT_BN_GLU = BN / 2;
@@ -310,15 +312,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   uint8_t* s_a = smem;
   uint8_t* s_b = smem + kStages * Cfg::kAStage;
   uint8_t* s_stage_out = smem + kStages * Cfg::kStageBytes;  // [group of 4 epilogue warps][2][32 channels][128 rows] bf16 ...
-  uint8_t* s_aux = s_stage_out;                               // ... or [2 buffers][gate, resid][2 halves? BN/64][128 x 64] bf16
+  uint8_t* s_aux = s_stage_out;                               // ... or [buffers][gate, resid][BN / 64][128 x 64] bf16
   uint64_t* bars = reinterpret_cast<uint64_t*>(
-      s_stage_out + (AUX ? Cfg::kAuxBytes : (SWAP ? Cfg::kSwapStagingBytes : (GLU ? Cfg::kGluStagingBytes : Cfg::kStagingBytes))));
+      s_stage_out + (AUX ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes : (SWAP ? Cfg::kSwapStagingBytes : (GLU ? Cfg::kGluStagingBytes : Cfg::kStagingBytes))));
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + Cfg::kMaxStages;
   uint64_t* tmem_full = bars + 2 * Cfg::kMaxStages;
   uint64_t* tmem_empty = tmem_full + 2;
   uint64_t* aux_full = tmem_empty + 2;   // [2]
-  uint64_t* aux_empty = aux_full + 2;    // [2], one arrival per epilogue warp
+  uint64_t* aux_empty = aux_full + 2;    // [2]: the output tile has left, one arrival by the store warp
   uint64_t* cm_bar = aux_empty + 2;      // [2 groups][slab free, slab written], 128 arrivals each
   uint64_t* rm_bar = cm_bar + 4;         // [2 staging buffers]: row-major tile written, one arrival per epilogue thread
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rm_bar + 2);
@@ -346,7 +348,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       ptx::mbar_init(&tmem_full[a], 1);
       ptx::mbar_init(&tmem_empty[a], 32 * kEpiWarps);
       ptx::mbar_init(&aux_full[a], 1);
-      ptx::mbar_init(&aux_empty[a], kEpiWarps);
+      ptx::mbar_init(&aux_empty[a], 1);
     }
     for (int a = 0; a < 4; ++a) ptx::mbar_init(&cm_bar[a], 128);
     for (int a = 0; a < 2; ++a) ptx::mbar_init(&rm_bar[a], 32 * kEpiWarps);
@@ -393,6 +395,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     if (ptx::elect_one()) {   // (elect.sync, not lane == 0: the compiler then knows one thread runs this, see ptx.cuh)
       int stage = 0;
       uint32_t phase = 0;  // ring position, advanced without divisions (the ring depth is a run-time value)
+      int aux_buf = 0;
+      uint32_t aux_par = 0;
       bool ok = true;
       for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, tile_advance(first_tile, p)) {
         const int n_tile = first_tile.n_tile, nb = first_tile.nb, o = first_tile.o, b = first_tile.b;
@@ -401,23 +405,25 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         if (tile + static_cast<int>(gridDim.x) >= total_tiles) grid_dependency_launch();
         const int b_col_hi = (n_tile * BN) / p.b_col_inner;
         const int b_col_lo = n_tile * BN - b_col_hi * p.b_col_inner;
-        if (AUX) {
-          // gate / residual tiles of this output tile, one tile ahead of the epilogue
-          const uint32_t ti = (tile - blockIdx.x) / gridDim.x;
-          const int ab = ti & 1;
-          if (!ptx::mbar_wait(&aux_empty[ab], ((ti >> 1) & 1) ^ 1, 106)) { ok = false; break; }
-          uint8_t* dst = s_aux + ab * (2 * Cfg::kAuxTileBytes);
-          ptx::mbar_expect_tx(&aux_full[ab], (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes);
+        // AUX: the gate / residual tiles of this output tile go out as soon as their buffer is free; operand tiles never wait for it
+        bool aux_due = AUX;
+        auto load_aux = [&]() {
+          const int set_bytes = (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes;
+          uint8_t* dst = s_aux + aux_buf * set_bytes;
+          uint8_t* dst_r = dst + p.aux_gate * Cfg::kAuxTileBytes;
+          ptx::mbar_expect_tx(&aux_full[aux_buf], set_bytes);
 #pragma unroll
           for (int hcol = 0; hcol < BN / 64; ++hcol) {
             if (p.aux_gate)
-              ptx::tma_load_4d(dst + hcol * (kBM * 128), &tm_out0, &aux_full[ab], n_tile * BN + hcol * 64, nb * kBM, o, b);
+              ptx::tma_load_4d(dst + hcol * (kBM * 128), &tm_out0, &aux_full[aux_buf], n_tile * BN + hcol * 64, nb * kBM, o, b);
             if (p.aux_resid)
-              ptx::tma_load_4d(dst + Cfg::kAuxTileBytes + hcol * (kBM * 128), &tm_out1, &aux_full[ab], n_tile * BN + hcol * 64,
-                               nb * kBM, o, b);
+              ptx::tma_load_4d(dst_r + hcol * (kBM * 128), &tm_out1, &aux_full[aux_buf], n_tile * BN + hcol * 64, nb * kBM, o, b);
           }
-        }
+          if (++aux_buf == p.aux_bufs) { aux_buf = 0; aux_par ^= 1u; }
+          aux_due = false;
+        };
         for (int kb = 0; kb < num_k; ++kb) {
+          if (AUX && aux_due && ptx::mbar_test(&aux_empty[aux_buf], aux_par ^ 1)) load_aux();
           const bool b_done = b_ahead > 0;      // this stage's weights are already on their way
           if (b_done) {
             --b_ahead;
@@ -443,6 +449,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           } else if (!b_done)
             ptx::tma_load_4d(s_b + stage * Cfg::kBStage, &tm_b, &full_bar[stage], kb * kBK, b_col_lo, b_col_hi, bb);
           if (++stage == kStages) { stage = 0; phase ^= 1; }
+        }
+        if (AUX && ok && aux_due) {
+          if (!ptx::mbar_wait(&aux_empty[aux_buf], aux_par ^ 1, 106)) { ok = false; break; }
+          load_aux();
         }
         KFB_GSTAMP(4 + (tile / gridDim.x) * 4 + 3);
       }
@@ -504,6 +514,27 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         KFB_GSTAMP(4 + tile_iter * 4 + 2);
       }
     }
+  } else if (AUX && warp == kGemmThreads / 32) {
+    // ------------------------------------------------------------ store warp of the AUX variant: finished tiles leave, their
+    // buffer goes back to the producer.  (A warp of its own: the epilogue warps never wait for a store.)
+    if (ptx::elect_one()) {
+      int buf = 0;
+      uint32_t par = 0;
+      TileIdx t = first_tile;
+      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, tile_advance(t, p)) {
+        if (!ptx::mbar_wait(&rm_bar[buf], par, 113)) break;
+        const uint8_t* src = s_aux + buf * ((p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes) + (p.aux_resid ? p.aux_gate * Cfg::kAuxTileBytes : 0);
+#pragma unroll
+        for (int hcol = 0; hcol < BN / 64; ++hcol)
+          if (t.n_tile * BN + hcol * 64 < p.n_cols)
+            ptx::tma_store_4d(&tm_out2, src + hcol * (kBM * 128), t.n_tile * BN + hcol * 64, t.nb * kBM, t.o, t.b);
+        ptx::tma_store_commit();
+        ptx::tma_store_wait_read();
+        ptx::mbar_arrive(&aux_empty[buf]);
+        if (++buf == p.aux_bufs) { buf = 0; par ^= 1u; }
+      }
+      ptx::tma_store_wait_all();
+    }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..9)
     const int quad = warp & 3;  // TMEM lane quadrant this warp may read
@@ -512,6 +543,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     uint32_t rm_use = 0;  // row-major tiles sent through the staging buffers so far (the same count in every epilogue thread)
     const int r = quad * 32 + lane;
     uint32_t tile_iter = 0;
+    int aux_buf = 0;        // AUX: buffer of gate / residual tiles of this tile, and its phase
+    uint32_t aux_par = 0;
     bool ok = true;
     // the row-mask byte of a tile is fetched one tile ahead, so that its latency never shows in the epilogue: the load is
     // issued here as it stands (volatile asm: the compiler may not sink it to its use) and only its raw byte is kept; the
@@ -568,6 +601,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       }
       const uint32_t acc = tile_iter & 1;
       const uint32_t acc_phase = (tile_iter >> 1) & 1;
+      float2 stats = make_float2(0.f, 1.f);     // this row's (mean, rstd), on its way while the tensor core works
+      if constexpr (AUX) {
+        if (p.row_stats != nullptr && row_ok)
+          stats = p.row_stats[(static_cast<long long>(b) * p.o_extent + o) * (p.stats_pitch > 0 ? p.stats_pitch : p.n_extent) + n];
+      }
       if constexpr (kXpose) {
         const int out_col = n_tile * BN + chunk_phase * 32;
         xp_nb = nb; xp_o = o; xp_b = b;
@@ -576,8 +614,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       if (!ptx::mbar_wait(&tmem_full[acc], acc_phase, 104)) { ok = false; break; }
       if (threadIdx.x == 64) KFB_GSTAMP(4 + tile_iter * 4 + 0);
       ptx::tc_fence_after_sync();
-      const uint8_t* aux_tile = s_aux + (tile_iter & 1) * (2 * Cfg::kAuxTileBytes);
-      if (AUX && !ptx::mbar_wait(&aux_full[tile_iter & 1], (tile_iter >> 1) & 1, 107)) { ok = false; break; }
+      if (AUX && !ptx::mbar_wait(&aux_full[aux_buf], aux_par, 107)) { ok = false; break; }
       const uint32_t t_row = tmem_base + acc * ACC_COLS + (static_cast<uint32_t>(quad * 32) << 16);
 
       constexpr int out_bn = GLU ? OUT_BN_GLU : BN;
@@ -841,6 +878,97 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           tile_done = true;
         }
       }
+      // AUX: gate logits and residual lie in the tiles the producer prefetched (128-byte rows, the copy engine's 16-byte swizzle);
+      // a thread owns its row of them, so it builds the output row in place of the residual (or gate) row and the store warp
+      // sends the whole tile.  Writing the rows from the registers instead cost 25 000 cycles per 128 x 256 tile with both
+      // operands read the same way, 8 000 per 128 x 128 tile with prefetched operands (one memory request per 32-byte sector).
+      // The columns go by as pieces of 16, the tensor-memory load of the next piece issued before the arithmetic of the current.
+      if constexpr (AUX) {
+        uint8_t* gate_row = s_aux + aux_buf * ((p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes) + r * 128;
+        uint8_t* res_row = gate_row + p.aux_gate * Cfg::kAuxTileBytes;
+        uint8_t* out_row = p.aux_resid ? res_row : gate_row;
+        const bool masked = (p.mask_segs & 1) != 0;
+        constexpr int kPieces = BN / 32;
+        auto piece_col = [&](int i) { return chunk_phase * 32 + (i >> 1) * 64 + (i & 1) * 16; };
+        uint32_t va[16], vb[16];
+        ptx::tmem_ld_32x32b_x16(t_row + piece_col(0), va);
+        auto finish_piece = [&](int c, const uint32_t (&vv)[16]) {
+          const int out_col = out_col_tile + c;
+          if (out_col >= p.n_cols) return;      // (n_cols is a multiple of 32)
+          float v[16];
+#pragma unroll
+          for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(vv[i]);
+          if (p.col_bias != nullptr) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] += __ldg(p.col_bias + out_col + i);
+          }
+          if (p.row_stats != nullptr) {   // folded LayerNorm of the A rows (see GemmParams)
+            const float4* s1 = reinterpret_cast<const float4*>(p.col_s1 + out_col);
+            const float4* s0 = reinterpret_cast<const float4*>(p.col_s0 + out_col);
+#pragma unroll
+            for (int q = 0; q < 4; ++q) {
+              const float4 a1 = __ldg(s1 + q), a0 = __ldg(s0 + q);
+              v[4 * q] = fmaf(stats.y, fmaf(-stats.x, a1.x, v[4 * q]), a0.x);
+              v[4 * q + 1] = fmaf(stats.y, fmaf(-stats.x, a1.y, v[4 * q + 1]), a0.y);
+              v[4 * q + 2] = fmaf(stats.y, fmaf(-stats.x, a1.z, v[4 * q + 2]), a0.z);
+              v[4 * q + 3] = fmaf(stats.y, fmaf(-stats.x, a1.w, v[4 * q + 3]), a0.w);
+            }
+          }
+          if (masked) {
+#pragma unroll
+            for (int i = 0; i < 16; ++i) v[i] *= mask_v;
+          }
+          const int half = (c >> 6) * (kBM * 128);
+          const int piece = (c & 63) >> 3;
+#pragma unroll
+          for (int h = 0; h < 2; ++h) {
+            const int off = half + (((piece + h) ^ (r & 7)) << 4);
+            if (p.aux_gate) {
+              const uint4 u = *reinterpret_cast<const uint4*>(gate_row + off);
+              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                v[h * 8 + j * 2] *= sigmoidf_fast(__uint_as_float(w[j] << 16));
+                v[h * 8 + j * 2 + 1] *= sigmoidf_fast(__uint_as_float(w[j] & 0xffff0000u));
+              }
+            }
+            if (p.aux_resid) {
+              const uint4 u = *reinterpret_cast<const uint4*>(res_row + off);
+              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
+              if (p.resid_scale != nullptr) {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  v[h * 8 + j * 2] = fmaf(__uint_as_float(w[j] << 16), __ldg(p.resid_scale + out_col + h * 8 + j * 2), v[h * 8 + j * 2]);
+                  v[h * 8 + j * 2 + 1] =
+                      fmaf(__uint_as_float(w[j] & 0xffff0000u), __ldg(p.resid_scale + out_col + h * 8 + j * 2 + 1), v[h * 8 + j * 2 + 1]);
+                }
+              } else {
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                  v[h * 8 + j * 2] += __uint_as_float(w[j] << 16);
+                  v[h * 8 + j * 2 + 1] += __uint_as_float(w[j] & 0xffff0000u);
+                }
+              }
+            }
+            *reinterpret_cast<uint4*>(out_row + off) =
+                make_uint4(pack_bf16x2(v[h * 8], v[h * 8 + 1]), pack_bf16x2(v[h * 8 + 2], v[h * 8 + 3]),
+                           pack_bf16x2(v[h * 8 + 4], v[h * 8 + 5]), pack_bf16x2(v[h * 8 + 6], v[h * 8 + 7]));
+          }
+        };
+#pragma unroll
+        for (int i = 0; i < kPieces; i += 2) {
+          ptx::tmem_ld_wait();
+          ptx::tmem_ld_32x32b_x16(t_row + piece_col(i + 1), vb);
+          finish_piece(piece_col(i), va);
+          ptx::tmem_ld_wait();
+          if (i + 2 < kPieces) ptx::tmem_ld_32x32b_x16(t_row + piece_col(i + 2), va);
+          finish_piece(piece_col(i + 1), vb);
+        }
+        ptx::fence_proxy_async_smem();
+        ptx::mbar_arrive(&rm_bar[aux_buf]);
+        if (++aux_buf == p.aux_bufs) { aux_buf = 0; aux_par ^= 1u; }
+        tile_done = true;
+      }
       // the GLU kernel's 128 output columns per tile take the same staged route when they lie in the staged segment
       bool glu_staged = false;
       if constexpr (GLU && !AUX && !PRECISE && BN == 256) {
@@ -1074,47 +1202,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             continue;
           }
         }
-        if (AUX && si == 0) {
-          // gate logits and residual come from the tiles the producer prefetched (128-byte swizzled rows)
-          const uint8_t* rowp = aux_tile + (c >> 6) * (kBM * 128) + r * 128;
-          const int cbase = ((c >> 5) & 1) * 4;
-          if (p.aux_gate) {
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const uint4 u = *reinterpret_cast<const uint4*>(rowp + (((cbase + q) ^ (r & 7)) << 4));
-              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-#pragma unroll
-              for (int j = 0; j < 4; ++j) {
-                v[q * 8 + j * 2] *= sigmoidf_fast(__uint_as_float(w[j] << 16));
-                v[q * 8 + j * 2 + 1] *= sigmoidf_fast(__uint_as_float(w[j] & 0xffff0000u));
-              }
-            }
-          }
-          if (p.aux_resid) {
-            const uint8_t* rrow = rowp + Cfg::kAuxTileBytes;
-#pragma unroll
-            for (int q = 0; q < 4; ++q) {
-              const uint4 u = *reinterpret_cast<const uint4*>(rrow + (((cbase + q) ^ (r & 7)) << 4));
-              const uint32_t w[4] = {u.x, u.y, u.z, u.w};
-              if (p.resid_scale != nullptr) {
-                const float4 s0 = __ldg(reinterpret_cast<const float4*>(p.resid_scale + out_col + q * 8));
-                const float4 s1 = __ldg(reinterpret_cast<const float4*>(p.resid_scale + out_col + q * 8 + 4));
-                const float sc[8] = {s0.x, s0.y, s0.z, s0.w, s1.x, s1.y, s1.z, s1.w};
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  v[q * 8 + j * 2] = fmaf(__uint_as_float(w[j] << 16), sc[j * 2], v[q * 8 + j * 2]);
-                  v[q * 8 + j * 2 + 1] = fmaf(__uint_as_float(w[j] & 0xffff0000u), sc[j * 2 + 1], v[q * 8 + j * 2 + 1]);
-                }
-              } else {
-#pragma unroll
-                for (int j = 0; j < 4; ++j) {
-                  v[q * 8 + j * 2] += __uint_as_float(w[j] << 16);
-                  v[q * 8 + j * 2 + 1] += __uint_as_float(w[j] & 0xffff0000u);
-                }
-              }
-            }
-          }
-        } else if (!AUX && si == 0 && row_ok) {
+        if (!AUX && si == 0 && row_ok) {
           if (PRECISE && p.gate != nullptr) {
             const float* g = reinterpret_cast<const float*>(p.gate) + static_cast<long long>(b) * p.g_b +
                              static_cast<long long>(o) * p.g_o + static_cast<long long>(n) * p.g_n +
@@ -1226,10 +1314,6 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       }
       }
       if (!ok) break;
-      if (AUX) {
-        __syncwarp();
-        if (lane == 0) ptx::mbar_arrive(&aux_empty[tile_iter & 1]);
-      }
       ptx::tc_fence_before_sync();
       ptx::mbar_arrive(&tmem_empty[acc]);
       if (threadIdx.x == 64) KFB_GSTAMP(4 + tile_iter * 4 + 1);
