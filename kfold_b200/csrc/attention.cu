@@ -708,6 +708,7 @@ int launch_attention(cudaStream_t stream, const AttnParams& p_in) {
                   "attention: window mode needs head dim <= 32, Lq == Lk a multiple of 32 and bias_mod == Lq / 32 windows");
     return launch_cfg<32, 1, true>(stream, p);
   }
+  if (p.row_info != nullptr) return launch_attention_rows(stream, p);
   // head dim <= 32: one row group per CTA, two CTAs resident per SM -- they interleave their softmax and tensor-core
   // phases better than two row groups inside one CTA did (measured 6 % faster at N=768); the bias tile both read stays
   // in L2

@@ -36,6 +36,7 @@ struct EpiSeg {
   int out_fp32;     // 0: bf16 output, 1: fp32 output
   int vec;          // 1: s_col == 1 and every row start is 16-byte aligned -> vector stores
   int tma_slot;     // >= 0: channel-major bf16 segment stored through shared memory with TMA store map `tma_slot`
+  float scale;      // bf16 segments of the plain kernel: factor on the values, before col_bias (0: none)
   int n_pad;        // rows may be written up to this position along n (their allocated pitch), 0: up to n_extent
   int split;        // precise mode: 0 plain store; 1 / 2: the value is split into three bf16 parts x0+x1+x2 and stored
                     // six times, s_part elements apart, as [x0 x0 x1 x1 x0 x2] (1) or [x0 x1 x0 x1 x2 x0] (2)
@@ -747,6 +748,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         const EpiSeg& sg = p.seg[si];
         const int ch_local = out_col_tile + r - sg.col_begin;
         const bool lane_ok = ch_local < sg.ncols;
+        const float scale_v = sg.scale != 0.f ? sg.scale : 1.f;
         const float bias_v = (p.col_bias != nullptr && lane_ok) ? p.col_bias[out_col_tile + r] : 0.0f;
         __nv_bfloat16* drow = reinterpret_cast<__nv_bfloat16*>(sg.dst) + static_cast<long long>(lane_ok ? ch_local : 0) * sg.s_col +
                               static_cast<long long>(b) * sg.s_b + static_cast<long long>(o) * sg.s_o;
@@ -758,7 +760,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           uint32_t w[16];
 #pragma unroll
           for (int i = 0; i < 32; i += 2)
-            w[i >> 1] = pack_bf16x2(__uint_as_float(raw[i]) + bias_v, __uint_as_float(raw[i + 1]) + bias_v);
+            w[i >> 1] = pack_bf16x2(fmaf(__uint_as_float(raw[i]), scale_v, bias_v), fmaf(__uint_as_float(raw[i + 1]), scale_v, bias_v));
           const int n0 = nb * kBM + c;
           if (lane_ok) {
             __nv_bfloat16* d = drow + n0;
@@ -1096,6 +1098,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         const EpiSeg& sg = p.seg[si];
         const int col_local = out_col - sg.col_begin;
         if (col_local >= sg.ncols) continue;  // uniform across the warp
+        if (!GLU && !AUX && !PRECISE && sg.scale != 0.f) {
+#pragma unroll
+          for (int i = 0; i < 32; ++i) v[i] *= sg.scale;
+        }
         if (p.col_bias != nullptr) {
 #pragma unroll
           for (int i = 0; i < 32; ++i) v[i] += (col_local + i < sg.ncols) ? p.col_bias[out_col + i] : 0.0f;

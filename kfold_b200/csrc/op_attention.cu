@@ -23,6 +23,7 @@ inline int dpad_of(int d) { return d <= 32 ? 32 : 64; }
 
 struct TriattWs {
   __nv_bfloat16 *xn, *qkg, *vt, *bias, *og;
+  int2* rows;
 };
 size_t carve_triatt(TriattWs& w, void* base, int batch, int n, int c, int heads) {
   Carver cv(base);
@@ -34,6 +35,7 @@ size_t carve_triatt(TriattWs& w, void* base, int batch, int n, int c, int heads)
   w.vt = cv.take<__nv_bfloat16>(pos_p * hdp);
   w.bias = cv.take<__nv_bfloat16>(pos_p * heads);
   w.og = cv.take<__nv_bfloat16>(pos * c);
+  w.rows = cv.take<int2>(static_cast<size_t>(batch) * n);
   return cv.off;
 }
 
@@ -225,6 +227,7 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
                           heads, eps);
   }
   const int dp = dpad_of(d), hdp = heads * dp;
+  const bool rows_kernel = dp == 32 && n >= 2;   // see attention_rows.cu
   TriattWs w;
   const size_t need = carve_triatt(w, workspace, batch, n, c, heads);
   KFB_CHECK_ARG(workspace_bytes >= need, "triatt: workspace %zu < %zu bytes", workspace_bytes, need);
@@ -259,6 +262,7 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
     sb = {};
     sb.col_begin = 4 * hdp;
     sb.ncols = heads;
+    if (rows_kernel) sb.scale = 1.4426950408889634f;   // its bias is in log2 units, as q is
     sb.dst = w.bias;
     sb.s_col = static_cast<long long>(np) * n;
     sb.s_n = 1;
@@ -288,6 +292,7 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
     p.m_hi = nn;
     p.m_lo = ending ? 1 : n;
     p.m_k = ending ? n : 1;
+    if (rows_kernel) p.row_info = w.rows;
     p.out = w.og; p.ldo = c;
     p.tag = "triatt_attention";
     KFB_TRY(launch_attention(stream, p));

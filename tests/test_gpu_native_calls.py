@@ -79,3 +79,28 @@ def test_token_stack_ragged(dev, l, groups, samples, own_s, precise):
         with torch.autocast("cuda", dtype=torch.bfloat16, enabled=not precise):
             out = stack(a.to(dev), s.to(dev), given, mask.to(dev))
         _compare(out.float().cpu(), ref, precise, f"token stack L={l}")
+
+
+@pytest.mark.parametrize("starting", [True, False])
+@pytest.mark.parametrize("n,batch,c,heads", [(2, 2, 128, 4), (33, 1, 128, 8), (65, 2, 96, 4), (130, 1, 128, 4), (257, 1, 128, 4)])
+def test_triatt_rows_masks_and_stabiliser(dev, n, batch, c, heads, starting):
+    """Pair rows around the tile and row-group sizes, with rows whose first 32 or 64 keys, scattered keys or all keys are masked, and
+    heads whose logits all lie far above or below zero (a constant bias, which softmax ignores): every way the stabiliser moves."""
+    from kfold_b200 import functional as F
+    from kfold_b200 import packing
+    import synth
+    z, pm, _ = synth.pair_inputs(n, n, c, batch)
+    g = torch.Generator().manual_seed(n)
+    holes = torch.rand(pm.shape, generator=g) < 0.2
+    rows = torch.arange(n) % 5
+    keys = torch.arange(n)
+    off = ((rows[:, None] == 1) & (keys < 32)) | ((rows[:, None] == 2) & (keys < 64)) | ((rows[:, None] == 3) & holes) | (rows[:, None] == 4)
+    pm = pm & ~(off if starting else off.transpose(-1, -2))
+    w = synth.triatt_weights(synth._Rng(n), c, heads)
+    w["layer_norm.weight"][0], w["layer_norm.bias"][0] = 0.0, 1.0
+    w["linear.weight"] *= (torch.arange(heads) % 2 == 0).float()[:, None]
+    w["linear.weight"][1::2, 0] = torch.tensor([256.0, -256.0]).repeat(heads)[: heads // 2]
+    zb = z.bfloat16()
+    out = F.triangle_attention(zb.to(dev), pm.to(dev), packing.pack_triatt(w, heads, dev), starting).float().cpu()
+    ref = _oracle_on(dev, O.triangle_attention, zb.float(), pm, w, heads, starting)
+    _check(*err_stats(out, ref), f"triatt N={n} starting={starting}")
