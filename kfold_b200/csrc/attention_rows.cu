@@ -638,12 +638,12 @@ static int launch_rows(cudaStream_t stream, const AttnParams& a) {
 }
 
 int launch_attention_rows(cudaStream_t stream, const AttnParams& a) {
-  // A CTA of three row groups takes 4/3 of the time of two for 3/2 of the work (more warps to fill each other's waits; one
+  // A CTA of three row groups takes 5/4 of the time of two (N = 1024) for 3/2 of the work (more warps to fill each other's waits; one
   // more group would leave a single S buffer each, which measured slower); two leave fewer SMs idle in the last wave of few items.
   auto waves = [&](int r) {
     return cdiv(static_cast<long long>(cdiv(a.lq, kQ)) * a.heads * cdiv(a.bias_div, r) * cdiv(a.batch, a.bias_div), (long long)sm_count());
   };
-  return waves(3) * 4 <= waves(2) * 3 ? launch_rows<3>(stream, a) : launch_rows<2>(stream, a);
+  return waves(3) * 5 <= waves(2) * 4 ? launch_rows<3>(stream, a) : launch_rows<2>(stream, a);
 }
 
 }  // namespace kfb
