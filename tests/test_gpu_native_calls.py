@@ -104,3 +104,19 @@ def test_triatt_rows_masks_and_stabiliser(dev, n, batch, c, heads, starting):
     out = F.triangle_attention(zb.to(dev), pm.to(dev), packing.pack_triatt(w, heads, dev), starting).float().cpu()
     ref = _oracle_on(dev, O.triangle_attention, zb.float(), pm, w, heads, starting)
     _check(*err_stats(out, ref), f"triatt N={n} starting={starting}")
+
+
+@pytest.mark.parametrize("n,batch,c,heads", [(8, 1, 128, 8), (40, 2, 96, 4), (72, 1, 128, 4), (72, 2, 128, 2)])
+def test_triatt_fp32_key_split(dev, n, batch, c, heads):
+    """float32 attention at key counts that leave some of a block's eight warps without keys, with one and two query rows per lane,
+    masked keys and rows without any key."""
+    from kfold_b200 import functional as F
+    from kfold_b200 import packing
+    import synth
+    z, pm, _ = synth.pair_inputs(n, n, c, batch)
+    pm = pm & ((torch.arange(n) % 3 != 1) | (torch.arange(n)[:, None] % 2 == 0)) & (torch.arange(n)[:, None] != 5)
+    w = synth.triatt_weights(synth._Rng(n), c, heads)
+    out = F.triangle_attention(z.to(dev), pm.to(dev), packing.pack_triatt(w, heads, dev, precise=True), True).cpu()
+    ref = _oracle_on(dev, O.triangle_attention, z, pm, w, heads, True)
+    mx, r = err_stats(out, ref)
+    assert mx < PRECISE_MAX_TOL and r < PRECISE_RMS_TOL, f"{mx:.3e} {r:.3e}"
