@@ -2,7 +2,7 @@
 //
 // CUDA cores, float32 throughout, an online softmax (the L x L x H logits are never stored).  Same semantics as attention.cu:
 // additive pair bias, masked keys get -1e9 (finite, as the reference does), optional sigmoid gate, and the result is written as the
-// bf16 triple split [o0 o0 o1 o1 o0 o2] that the fp32-accurate output projection consumes.
+// bf16 triple split (an A operand's row, see part_a) that the fp32-accurate output projection consumes.
 //
 // A block takes 32 or 64 queries of one head and splits the keys over its eight warps, eight keys at a time; a lane owns one or two
 // query rows, and the warps' (maximum, sum, accumulator) are merged at the end.  The single-track problems (a few hundred queries,
@@ -11,6 +11,7 @@
 // warp; K and V are read as broadcast 16-byte pieces, which bounds the loop (one load feeds four multiply-adds per query row: two
 // rows per lane where there are enough blocks without it).
 #include "attention.cuh"
+#include "gemm.cuh"  // part_a
 #include "ptx.cuh"
 
 #include <mutex>
@@ -219,7 +220,9 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
     const float r1 = o - __bfloat162float(x0);
     const __nv_bfloat16 x1 = __float2bfloat16_rn(r1);
     const __nv_bfloat16 x2 = __float2bfloat16_rn(r1 - __bfloat162float(x1));
-    o6[col] = x0; o6[hd + col] = x0; o6[2 * hd + col] = x1; o6[3 * hd + col] = x1; o6[4 * hd + col] = x0; o6[5 * hd + col] = x2;
+    o6[part_a(0) * hd + col] = x0;
+    o6[part_a(1) * hd + col] = x1;
+    o6[part_a(2) * hd + col] = x2;
   }
 }
 

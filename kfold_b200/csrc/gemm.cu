@@ -54,8 +54,6 @@ static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorM
   } else {
   if constexpr (BN <= 128) {
     if (p.precise) {
-      p.k_main_blocks = (p.k_extent / 6) / kBK;
-      if (p.k_main_blocks == 0) p.k_main_blocks = 1;  // short K: the first block mixes parts, harmless
       if (p.glu) return launch_variant<BN, true, false, true>(stream, ta, tb, tout, p, tag);
       return launch_variant<BN, false, false, true>(stream, ta, tb, tout, p, tag);
     }
@@ -84,8 +82,8 @@ static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorM
 static int narrow_tile(const GemmParams& p, int bn) {
   const long long sms = sm_count();
   if (static_cast<long long>(p.num_m_tiles) * cdiv(p.n_cols, bn) >= sms) return bn;
-  const int num_k = cdiv(p.k_extent, kBK);
-  const int lo = p.glu ? 64 : 32;
+  const int num_k = p.precise ? 3 * cdiv(p.k_extent / 6, kBK) : cdiv(p.k_extent, kBK);
+  const int lo = p.glu || p.precise ? 64 : 32;
   double best = 1e30;
   int pick = bn;
   for (int w = bn; w >= lo; w /= 2) {
@@ -112,8 +110,8 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
   p.num_m_tiles = p.n_blocks * p.o_extent * p.batch;
   int bn = force_bn;
   if (bn == 0) bn = p.n_cols >= 256 ? 256 : (p.n_cols > 64 ? 128 : 64);
-  if (!p.precise && a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0 && p.glu != GLU_SIGMOID) bn = narrow_tile(p, bn);
   if (p.precise && bn > 128) bn = 128;  // the fp32-accurate variant keeps four accumulators in tensor memory
+  if (a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0 && (p.precise ? !p.glu : p.glu != GLU_SIGMOID)) bn = narrow_tile(p, bn);
   // One row-major float32 segment with a gate and / or a residual (the output projections of the sampler's float32 activation
   // stream): 128-column tiles whose epilogue moves gate, residual and output through per-warp shared-memory tiles.
   p.xpose = 0;
@@ -157,7 +155,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
     }
   }
   KFB_CHECK_ARG(bn == 32 || bn == 64 || bn == 128 || bn == 256, "unsupported BN %d", bn);
-  if (p.precise) KFB_CHECK_ARG(p.k_extent % 6 == 0, "precise GEMM: K=%d is not six equal parts", p.k_extent);
+  if (p.precise) KFB_CHECK_ARG(p.k_extent % 48 == 0, "precise GEMM: K=%d is not six equal parts of whole 16-byte pieces", p.k_extent);
   if (p.glu) KFB_CHECK_ARG(p.n_cols % bn == 0, "GLU GEMM needs n_cols (%d) to be a multiple of the N tile (%d)", p.n_cols, bn);
   for (int i = 0; i < p.nseg; ++i) KFB_CHECK_ARG(p.seg[i].col_begin % 32 == 0, "segment start must be a multiple of 32");
   p.trace = (g_trace_buf != nullptr && strcmp(g_trace_tag, tag) == 0) ? g_trace_buf : nullptr;
@@ -167,7 +165,15 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
   p.a_mn_major = a.s_k != 0 ? 1 : 0;
   p.k_inner = a.k_inner;
   KFB_CHECK_ARG(a.k_inner == b.k_inner, "split K: both operands must be split alike (%d, %d)", a.k_inner, b.k_inner);
-  if (p.k_inner) {
+  if (p.precise) {
+    // the parts are a dimension of their own: a K block never runs into the next part, whatever K is
+    const int k = p.k_extent / 6;
+    KFB_CHECK_ARG(!p.a_mn_major && !p.k_inner, "precise GEMM: plain K-major operands only");
+    const uint64_t dims[5] = {(uint64_t)k, (uint64_t)p.n_extent, (uint64_t)p.o_extent, 6, (uint64_t)p.batch};
+    const uint64_t str[4] = {(uint64_t)a.s_n * 2, (uint64_t)a.s_o * 2, (uint64_t)k * 2, (uint64_t)a.s_b * 2};
+    const uint32_t box[5] = {kBK, kBM, 1, 1, 1};
+    KFB_TRY(make_tmap(&ta, a.ptr, 2, 5, dims, str, box, 128));
+  } else if (p.k_inner) {
     KFB_CHECK_ARG(!p.a_mn_major && !p.precise && p.k_inner % kBK == 0 && p.k_extent % p.k_inner == 0,
                   "split K: pieces of %d elements (multiple of %d) in K=%d, plain bf16 GEMM", p.k_inner, kBK, p.k_extent);
     const uint64_t dims[5] = {(uint64_t)p.k_inner, (uint64_t)p.n_extent, (uint64_t)p.o_extent, (uint64_t)(p.k_extent / p.k_inner),
@@ -194,7 +200,13 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
       KFB_CHECK_ARG(p.n_cols % inner == 0 && inner % bn == 0, "split B operand: %d columns in pieces of %d, tile %d", p.n_cols,
                     inner, bn);
     p.b_col_inner = inner;
-    if (p.k_inner) {
+    if (p.precise) {
+      const int k = p.k_extent / 6;
+      const uint64_t dims[5] = {(uint64_t)k, (uint64_t)inner, (uint64_t)(p.n_cols / inner), 6, (uint64_t)(p.b_batched ? p.batch : 1)};
+      const uint64_t str[4] = {(uint64_t)b.s_col * 2, (uint64_t)b.s_col_hi * 2, (uint64_t)k * 2, (uint64_t)b.s_b * 2};
+      const uint32_t box[5] = {kBK, (uint32_t)bn, 1, 1, 1};
+      KFB_TRY(make_tmap(&tb, b.ptr, 2, 5, dims, str, box, 128));
+    } else if (p.k_inner) {
       const uint64_t dims[5] = {(uint64_t)p.k_inner, (uint64_t)inner, (uint64_t)(p.n_cols / inner),
                                 (uint64_t)(p.k_extent / p.k_inner), (uint64_t)(p.b_batched ? p.batch : 1)};
       const uint64_t str[4] = {(uint64_t)b.s_col * 2, (uint64_t)b.s_col_hi * 2, (uint64_t)b.s_k_hi * 2, (uint64_t)b.s_b * 2};
@@ -204,7 +216,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
     const uint64_t dims[4] = {(uint64_t)p.k_extent, (uint64_t)inner, (uint64_t)(p.n_cols / inner),
                               (uint64_t)(p.b_batched ? p.batch : 1)};
     const uint64_t str[3] = {(uint64_t)b.s_col * 2, (uint64_t)b.s_col_hi * 2, (uint64_t)b.s_b * 2};
-    const uint32_t box[4] = {kBK, (uint32_t)(p.glu && !p.precise && bn < 256 ? bn / 2 : bn), 1, 1};
+    const uint32_t box[4] = {kBK, (uint32_t)(p.glu && bn < 256 ? bn / 2 : bn), 1, 1};
     KFB_TRY(make_tmap(&tb, b.ptr, 2, 4, dims, str, box, 128));
     }
   }

@@ -38,8 +38,8 @@ struct EpiSeg {
   int tma_slot;     // >= 0: channel-major bf16 segment stored through shared memory with TMA store map `tma_slot`
   float scale;      // bf16 segments of the plain kernel: factor on the values, before col_bias (0: none)
   int n_pad;        // rows may be written up to this position along n (their allocated pitch), 0: up to n_extent
-  int split;        // precise mode: 0 plain store; 1 / 2: the value is split into three bf16 parts x0+x1+x2 and stored
-                    // six times, s_part elements apart, as [x0 x0 x1 x1 x0 x2] (1) or [x0 x1 x0 x1 x2 x0] (2)
+  int split;        // precise mode: 0 plain store; 1 / 2: the value is split into three bf16 parts x0+x1+x2, stored in an A
+                    // (1) or B (2) operand's places of them (see part_a), s_part elements apart
   long long s_part;
   void* dst;
   long long s_col, s_n, s_o, s_b;
@@ -78,10 +78,6 @@ struct GemmParams {
   int mask_segs;                  // bit i: apply rowmask to segment i
   const float* col_bias;          // optional, per output column, added before everything else
   int precise;                    // fp32-accurate mode: exact sigmoid, fp32 gate logits, split stores
-  int k_main_blocks;              // precise: the first k_main_blocks k-blocks (the x0*w0 products) accumulate in their own
-                                  // TMEM accumulator, the five correction blocks in a second one; the epilogue adds the
-                                  // two in fp32.  The tensor core truncates on every accumulation step, relative to the
-                                  // accumulator's magnitude: keeping the small corrections apart keeps their error small
   const __nv_bfloat16* gate;      // optional: seg 0 value *= sigmoid(gate[...]), addressed with seg 0 strides
                                   // (points at float logits when `precise`)
   long long g_col, g_n, g_o, g_b;
@@ -166,23 +162,48 @@ __device__ __forceinline__ void split3(float x, __nv_bfloat16& x0, __nv_bfloat16
   x2 = __float2bfloat16_rn(r1 - __bfloat162float(x1));
 }
 
-// Split store of 32 values of one row: six copies, s_part elements apart (see EpiSeg::split).
+// The places of the parts in an operand's row of six times K elements: an A row is [x0 . x1 . . x2], a B row [w0 w1 . . w2 .] (the
+// remaining places hold copies of the parts in packed weights and nothing in activations; no kernel reads them).
+__host__ __device__ constexpr int part_a(int i) { return i == 0 ? 0 : (i == 1 ? 2 : 5); }
+__host__ __device__ constexpr int part_b(int i) { return i == 0 ? 0 : (i == 1 ? 1 : 4); }
+
+// Split store of 32 values of one row (see EpiSeg::split).
 __device__ __forceinline__ void epi_store_split(const EpiSeg& sg, long long row_off, int col_local, const float (&v)[32],
                                                 bool row_ok) {
   if (!row_ok) return;
   const int nvalid = min(32, sg.ncols - col_local);
   __nv_bfloat16* d = reinterpret_cast<__nv_bfloat16*>(sg.dst) + row_off + static_cast<long long>(col_local) * sg.s_col;
+  const long long at1 = (sg.split == 1 ? part_a(1) : part_b(1)) * sg.s_part, at2 = (sg.split == 1 ? part_a(2) : part_b(2)) * sg.s_part;
+  if (nvalid == 32 && sg.s_col == 1 && (sg.s_part & 7) == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
+    // a row-major row: 16-byte pieces (two-byte stores of 32 rows touch 32 sectors each; together with the halved operand traffic
+    // the gated projections of 25 600 rows of 128 channels went from 272 to 55 us)
+#pragma unroll
+    for (int i = 0; i < 32; i += 8) {
+      uint32_t w[3][4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        __nv_bfloat16 x[2][3];
+        split3(v[i + 2 * j], x[0][0], x[0][1], x[0][2]);
+        split3(v[i + 2 * j + 1], x[1][0], x[1][1], x[1][2]);
+#pragma unroll
+        for (int q = 0; q < 3; ++q)
+          w[q][j] = static_cast<uint32_t>(__bfloat16_as_ushort(x[0][q])) | (static_cast<uint32_t>(__bfloat16_as_ushort(x[1][q])) << 16);
+      }
+      *reinterpret_cast<uint4*>(d + i) = make_uint4(w[0][0], w[0][1], w[0][2], w[0][3]);
+      *reinterpret_cast<uint4*>(d + at1 + i) = make_uint4(w[1][0], w[1][1], w[1][2], w[1][3]);
+      *reinterpret_cast<uint4*>(d + at2 + i) = make_uint4(w[2][0], w[2][1], w[2][2], w[2][3]);
+    }
+    return;
+  }
 #pragma unroll 4
   for (int i = 0; i < 32; ++i) {
     if (i >= nvalid) break;
     __nv_bfloat16 x0, x1, x2;
     split3(v[i], x0, x1, x2);
     __nv_bfloat16* e = d + static_cast<long long>(i) * sg.s_col;
-    if (sg.split == 1) {
-      e[0] = x0; e[sg.s_part] = x0; e[2 * sg.s_part] = x1; e[3 * sg.s_part] = x1; e[4 * sg.s_part] = x0; e[5 * sg.s_part] = x2;
-    } else {
-      e[0] = x0; e[sg.s_part] = x1; e[2 * sg.s_part] = x0; e[3 * sg.s_part] = x1; e[4 * sg.s_part] = x2; e[5 * sg.s_part] = x0;
-    }
+    e[0] = x0;
+    e[at1] = x1;
+    e[at2] = x2;
   }
 }
 
@@ -286,7 +307,7 @@ __device__ __forceinline__ void tile_advance(TileIdx& t, const GemmParams& p) {
 // GLU and AUX are compile-time so that each variant carries only its own epilogue code (and registers):
 //   GLU  the tile holds values and gates (p.glu says which activation);
 //   AUX  gate logits / residual come from shared-memory tiles prefetched by the producer.
-//   PRECISE  fp32-accurate mode (operands are bf16 triple splits concatenated along K, see split3): exact
+//   PRECISE  fp32-accurate mode (operands are bf16 triple splits, see split3 and part_a): exact
 //            sigmoid, fp32 gate logits, split stores.
 //   SWAP  channel-major GLU output (the triangle-multiplication operands): the tensor core computes the TRANSPOSED tile,
 //         D[channel][position] = W[channel][:] . X[position][:], i.e. the 128 value rows and the 128 gate rows of the weight
@@ -328,7 +349,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
-  const int num_k = (p.k_extent + kBK - 1) / kBK;
+  // K blocks; PRECISE: ring stages, three for a K block: (x0, w0), (x1, w1), (x2, w2)
+  const int num_k = PRECISE ? 3 * ((p.k_extent / 6 + kBK - 1) / kBK) : (p.k_extent + kBK - 1) / kBK;
   const int total_tiles = p.num_m_tiles * p.num_n_tiles;
   long long* trace = (p.trace != nullptr && blockIdx.x == 0) ? p.trace : nullptr;
 #ifdef KFB_DEBUG_TRACE
@@ -385,6 +407,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       ptx::mbar_expect_tx(&full_bar[kb], Cfg::kStageBytes);
       if constexpr (kSplitGlu)
         load_glu_b(kb, n_tile, kb);
+      else if constexpr (PRECISE)
+        ptx::tma_load_5d(s_b + kb * Cfg::kBStage, &tm_b, &full_bar[kb], kb / 3 * kBK, n_tile * BN - b_col_hi * p.b_col_inner, b_col_hi,
+                         part_b(kb % 3), 0);
       else
         ptx::tma_load_4d(s_b + kb * Cfg::kBStage, &tm_b, &full_bar[kb], kb * kBK, n_tile * BN - b_col_hi * p.b_col_inner, b_col_hi, 0);
     }
@@ -423,6 +448,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           if (++aux_buf == p.aux_bufs) { aux_buf = 0; aux_par ^= 1u; }
           aux_due = false;
         };
+        int kb_main = 0, part = 0;     // PRECISE: K block and operand part of a stage
         for (int kb = 0; kb < num_k; ++kb) {
           if (AUX && aux_due && ptx::mbar_test(&aux_empty[aux_buf], aux_par ^ 1)) load_aux();
           const bool b_done = b_ahead > 0;      // this stage's weights are already on their way
@@ -431,6 +457,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           } else {
             if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1, 101)) { ok = false; break; }
             ptx::mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
+          }
+          if constexpr (PRECISE) {
+            ptx::tma_load_5d(s_a + stage * Cfg::kAStage, &tm_a, &full_bar[stage], kb_main * kBK, nb * kBM, o, part_a(part), b);
+            if (!b_done)
+              ptx::tma_load_5d(s_b + stage * Cfg::kBStage, &tm_b, &full_bar[stage], kb_main * kBK, b_col_lo, b_col_hi, part_b(part), bb);
+            if (++part == 3) { part = 0; ++kb_main; }
+            if (++stage == kStages) { stage = 0; phase ^= 1; }
+            continue;
           }
           if (p.a_mn_major) {
             // two boxes of [64 k][64 rows]: 128-byte rows of consecutive rows (positions), one per k index
@@ -473,15 +507,50 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         if (!ptx::mbar_wait(&tmem_empty[acc], acc_phase ^ 1, 102)) { ok = false; break; }
         ptx::tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
+        if constexpr (PRECISE) {
+          // Six products of a K block from three pairs of parts, each pair loaded once: 96 KB through the SM's port (64 B per cycle)
+          // under 1 536 cycles of tensor work, where operands concatenated six times along K took 192 KB.
+          for (int kb = 0; kb < num_k; kb += 3) {
+            uint64_t a_desc[3], b_desc[3];
+            int stages[3];
+            auto product = [&](uint64_t ad, uint64_t bd, uint32_t d, bool first) {
+#pragma unroll
+              for (int k = 0; k < kBK / 16; ++k) ptx::mma_f16_ss(d, ad + k * 2, bd + k * 2, idesc, (first && k == 0) ? 0u : 1u);
+            };
+#pragma unroll
+            for (int i = 0; i < 3; ++i) {
+              if (!ptx::mbar_wait(&full_bar[stage], phase, 103)) { ok = false; break; }
+              ptx::tc_fence_after_sync();
+              stages[i] = stage;
+              a_desc[i] = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_a + stage * Cfg::kAStage));
+              b_desc[i] = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_b + stage * Cfg::kBStage));
+              if (++stage == kStages) { stage = 0; phase ^= 1; }
+              // x0 w0 has its own accumulator, the five small products a second one; the epilogue adds the two in fp32.  The
+              // tensor core truncates on every accumulation step, relative to the accumulator's magnitude: kept apart, the small
+              // ones keep their small error.
+              if (i == 0) {
+                product(a_desc[0], b_desc[0], d_tmem, kb == 0);
+              } else {
+                product(a_desc[0], b_desc[i], d_tmem + BN, kb == 0 && i == 1);
+                product(a_desc[i], b_desc[0], d_tmem + BN, false);
+                if (i == 1) product(a_desc[1], b_desc[1], d_tmem + BN, false);
+              }
+            }
+            if (!ok) break;
+#pragma unroll
+            for (int i = 0; i < 3; ++i) ptx::tc_commit(&empty_bar[stages[i]]);
+          }
+          if (ok) ptx::tc_commit(&tmem_full[acc]);
+          continue;
+        }
         for (int kb = 0; kb < num_k; ++kb) {
           if (!ptx::mbar_wait(&full_bar[stage], phase, 103)) { ok = false; break; }
           ptx::tc_fence_after_sync();
           // one descriptor per stage; inside the 128-byte swizzle span only the address field advances
           const uint64_t a_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_a + stage * Cfg::kAStage));
           const uint64_t b_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_b + stage * Cfg::kBStage));
-          const bool corr = PRECISE && kb >= p.k_main_blocks;
-          const uint32_t d_acc = corr ? d_tmem + BN : d_tmem;
-          const bool first = corr ? (kb == p.k_main_blocks) : (kb == 0);
+          const uint32_t d_acc = d_tmem;
+          const bool first = kb == 0;
           if constexpr (SWAP) {
             // value rows (first 128 rows of the weight stage) -> columns 0..127, gate rows -> columns 128..255
             constexpr uint32_t idesc_sw = ptx::make_idesc(kBM, 128, /*bf16*/ 1);

@@ -3,6 +3,8 @@
 // variance of the centred values, which is what torch's layer_norm computes).
 #include "layernorm.cuh"
 
+#include "gemm.cuh"  // part_a
+
 #include <type_traits>
 
 namespace kfb {
@@ -258,7 +260,9 @@ __device__ __forceinline__ void split3_store(__nv_bfloat16* y6, int c, int ch, f
   const float r1 = v - __bfloat162float(x0);
   const __nv_bfloat16 x1 = __float2bfloat16_rn(r1);
   const __nv_bfloat16 x2 = __float2bfloat16_rn(r1 - __bfloat162float(x1));
-  y6[ch] = x0; y6[c + ch] = x0; y6[2 * c + ch] = x1; y6[3 * c + ch] = x1; y6[4 * c + ch] = x0; y6[5 * c + ch] = x2;
+  y6[part_a(0) * c + ch] = x0;
+  y6[part_a(1) * c + ch] = x1;
+  y6[part_a(2) * c + ch] = x2;
 }
 
 __global__ void __launch_bounds__(256) layernorm_split_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y6,
