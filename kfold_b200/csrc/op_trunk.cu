@@ -8,6 +8,8 @@
 // and of the confidence head (model/modules/confidence_head.py:306-470):
 //   kfb_pair_outer_add       z + Linear_1(s)[j] + Linear_2(s)[i]       the single representation added along both token axes
 //   kfb_distogram_embed_add  z + Linear(one_hot(distance bin))         the predicted structure's distogram, embedded
+#include <type_traits>
+
 #include "ops_common.cuh"
 
 using namespace kfb;
@@ -160,21 +162,47 @@ __global__ void __launch_bounds__(256) pair_outer_add_kernel(const T* __restrict
 
 // out[b, i, j, :] = z[b, i, j, :] + w_t[bin(|x_i - x_j|), :], bin = number of boundaries below the distance: the one-hot
 // distogram of the predicted structure embedded and added to the pair tensor.  x fp32 (b, n, 3); w_t (bins, c).
-template <typename T>
+// A warp takes 32 positions: a lane finds the bin of one, then the lanes walk the 32 rows in pieces of VEC channels (16 bytes; 1 where
+// rows are not whole pieces).  HBM-bound; with a block per position, 64 comparisons on every thread and 2-byte accesses,
+// 400 x 400 positions of 128 channels took 450 us.
+template <typename T, int VEC>
 __global__ void __launch_bounds__(256) distogram_embed_add_kernel(const T* __restrict__ z, const float* __restrict__ x,
                                                                   const float* __restrict__ boundaries, int n_bound,
-                                                                  const T* __restrict__ w_t, T* __restrict__ out, int n, int c) {
-  const long long pos = blockIdx.x;                     // (b * n + i) * n + j
+                                                                  const T* __restrict__ w_t, T* __restrict__ out, int n, int c,
+                                                                  long long total) {
+  const int lane = threadIdx.x & 31;
+  const long long pos0 = (static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5)) * 32;   // (b * n + i) * n + j
+  if (pos0 >= total) return;
+  const long long pos = pos0 + lane < total ? pos0 + lane : total - 1;
   const long long bi = pos / n;
   const int j = static_cast<int>(pos - bi * n);
-  const long long b = bi / n;
   const float* xi = x + bi * 3;
-  const float* xj = x + (b * n + j) * 3;
+  const float* xj = x + (bi / n * n + j) * 3;
   const float dx = xi[0] - xj[0], dy = xi[1] - xj[1], dz = xi[2] - xj[2];
   const float d = sqrtf(dx * dx + dy * dy + dz * dz);
   int bin = 0;
   for (int k = 0; k < n_bound; ++k) bin += d > boundaries[k] ? 1 : 0;
-  for (int ch = threadIdx.x; ch < c; ch += 256) stf(out + pos * c + ch, ldf(z + pos * c + ch) + ldf(w_t + static_cast<long long>(bin) * c + ch));
+  const int pieces = c / VEC;
+  const T* zr = z + pos0 * c;
+  T* yr = out + pos0 * c;
+#pragma unroll 4
+  for (int e = lane; e < 32 * pieces; e += 32) {
+    const int p = e / pieces, ch = (e - p * pieces) * VEC;
+    const T* wr = w_t + static_cast<long long>(__shfl_sync(0xffffffffu, bin, p)) * c + ch;
+    if (pos0 + p >= total) continue;
+    const long long off = static_cast<long long>(p) * c + ch;
+    if constexpr (VEC == 1) {
+      stf(yr + off, ldf(zr + off) + ldf(wr));
+    } else {
+      uint4 zv = *reinterpret_cast<const uint4*>(zr + off);
+      const uint4 wv = __ldg(reinterpret_cast<const uint4*>(wr));
+      T* ze = reinterpret_cast<T*>(&zv);
+      const T* we = reinterpret_cast<const T*>(&wv);
+#pragma unroll
+      for (int i = 0; i < VEC; ++i) stf(ze + i, ldf(ze + i) + ldf(we + i));
+      *reinterpret_cast<uint4*>(yr + off) = zv;
+    }
+  }
 }
 
 }  // namespace
@@ -209,15 +237,24 @@ KFB_API int kfb_distogram_embed_add(const void* z, const float* x, const float* 
                 "distogram_embed_add: batch %d n %d c %d boundaries %d", batch, n, c, n_boundaries);
   KFB_CHECK_ARG(dtype == KFB_BF16 || dtype == KFB_FP32, "distogram_embed_add: dtype %d", dtype);
   cudaStream_t stream = as_stream(stream_);
-  const unsigned blocks = static_cast<unsigned>(static_cast<long long>(batch) * n * n);
+  const long long total = static_cast<long long>(batch) * n * n;
+  const unsigned blocks = static_cast<unsigned>((total + 255) / 256);
+  const bool whole = (static_cast<long long>(c) * (dtype == KFB_BF16 ? 2 : 4)) % 16 == 0 &&
+                     ((reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(w_t) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
+  auto launch = [&](auto kernel, auto* t) {
+    using T = std::remove_pointer_t<decltype(t)>;
+    kernel<<<blocks, 256, 0, stream>>>(static_cast<const T*>(z), x, boundaries, n_boundaries, static_cast<const T*>(w_t),
+                                       static_cast<T*>(out), n, c, total);
+  };
   {
     LaunchScope scope(stream, "distogram_embed_add");
-    if (dtype == KFB_BF16)
-      distogram_embed_add_kernel<<<blocks, 256, 0, stream>>>(static_cast<const __nv_bfloat16*>(z), x, boundaries, n_boundaries,
-                                                             static_cast<const __nv_bfloat16*>(w_t), static_cast<__nv_bfloat16*>(out), n, c);
-    else
-      distogram_embed_add_kernel<<<blocks, 256, 0, stream>>>(static_cast<const float*>(z), x, boundaries, n_boundaries,
-                                                             static_cast<const float*>(w_t), static_cast<float*>(out), n, c);
+    if (dtype == KFB_BF16) {
+      using T = __nv_bfloat16;
+      whole ? launch(distogram_embed_add_kernel<T, 8>, static_cast<T*>(out)) : launch(distogram_embed_add_kernel<T, 1>, static_cast<T*>(out));
+    } else {
+      whole ? launch(distogram_embed_add_kernel<float, 4>, static_cast<float*>(out))
+            : launch(distogram_embed_add_kernel<float, 1>, static_cast<float*>(out));
+    }
   }
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
