@@ -97,16 +97,19 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* __restric
   }
 }
 
-// The pair track's shape: 128 bf16 channels, contiguous rows.  A row is 256 bytes = 16 lanes x 16 bytes, so a warp takes two
-// rows per step and two steps per iteration: four rows (1 KB) in flight per warp, 16-byte loads and stores, the statistics
-// reduced over the 16 lanes of a row.  Same arithmetic as layernorm_rows_kernel (two passes, fp32).
-__global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
+// The pair tracks' shapes: 128 or 256 bf16 channels, contiguous rows.  A row is LANES x 16 bytes, LANES 16 or 32, so a warp takes
+// 32 / LANES rows per step and STEPS steps per iteration: 1 or 2 KB in flight per warp, 16-byte loads and stores, the statistics
+// reduced over the lanes of a row.  Same arithmetic as layernorm_rows_kernel (two passes, fp32), whose 4-byte accesses took 150 us
+// for 768 x 768 rows of 256 channels (92 at the memory's rate).
+template <int LANES, int STEPS>
+__global__ void __launch_bounds__(256) layernorm_vec_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                                                   const float* __restrict__ w, const float* __restrict__ b,
                                                                   long long rows, float eps) {
+  constexpr int C = LANES * 8, kRows = 32 / LANES;
   grid_dependency_enter();
   const int lane = threadIdx.x & 31;
-  const int sub = lane & 15;                 // 16-byte chunk of the row
-  const int half = lane >> 4;                // which of the warp's two rows
+  const int sub = lane % LANES;              // 16-byte chunk of the row
+  const int half = lane / LANES;             // which of the step's rows
   float g[8], o[8];
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
@@ -115,17 +118,17 @@ __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfl
   }
   const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   const long long warp_id = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
-  for (long long base = warp_id * 4; base < rows; base += warps * 4) {
-    uint4 raw[2];
-    bool live[2];
+  for (long long base = warp_id * (kRows * STEPS); base < rows; base += warps * (kRows * STEPS)) {
+    uint4 raw[STEPS];
+    bool live[STEPS];
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
-      const long long row = base + s * 2 + half;
+    for (int s = 0; s < STEPS; ++s) {
+      const long long row = base + s * kRows + half;
       live[s] = row < rows;
-      raw[s] = live[s] ? *reinterpret_cast<const uint4*>(x + row * 128 + sub * 8) : make_uint4(0, 0, 0, 0);
+      raw[s] = live[s] ? *reinterpret_cast<const uint4*>(x + row * C + sub * 8) : make_uint4(0, 0, 0, 0);
     }
 #pragma unroll
-    for (int s = 0; s < 2; ++s) {
+    for (int s = 0; s < STEPS; ++s) {
       const uint32_t wv[4] = {raw[s].x, raw[s].y, raw[s].z, raw[s].w};
       float v[8];
       float sum = 0.f;
@@ -136,8 +139,8 @@ __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfl
         sum += v[2 * i] + v[2 * i + 1];
       }
 #pragma unroll
-      for (int m = 8; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
-      const float mean = sum * (1.0f / 128.0f);
+      for (int m = LANES / 2; m > 0; m >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, m);
+      const float mean = sum * (1.0f / C);
       float sq = 0.f;
 #pragma unroll
       for (int i = 0; i < 8; ++i) {
@@ -145,8 +148,8 @@ __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfl
         sq = fmaf(v[i], v[i], sq);
       }
 #pragma unroll
-      for (int m = 8; m > 0; m >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, m);
-      const float rstd = rsqrtf(sq * (1.0f / 128.0f) + eps);
+      for (int m = LANES / 2; m > 0; m >>= 1) sq += __shfl_xor_sync(0xffffffffu, sq, m);
+      const float rstd = rsqrtf(sq * (1.0f / C) + eps);
       uint4 out;
       uint32_t* ov = reinterpret_cast<uint32_t*>(&out);
 #pragma unroll
@@ -155,8 +158,8 @@ __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfl
                                                         fmaf(v[2 * i + 1] * rstd, g[2 * i + 1], o[2 * i + 1]));
         ov[i] = *reinterpret_cast<const uint32_t*>(&pr);
       }
-      const long long row = base + s * 2 + half;
-      if (live[s]) *reinterpret_cast<uint4*>(y + row * 128 + sub * 8) = out;
+      const long long row = base + s * kRows + half;
+      if (live[s]) *reinterpret_cast<uint4*>(y + row * C + sub * 8) = out;
     }
   }
 }
@@ -206,14 +209,14 @@ int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w
                 "layernorm: exchange order needs a (%d, %d) shard, got %lld rows", perm.rows, perm.n, rows);
   KFB_CHECK_ARG(xs % 2 == 0 && ys % 2 == 0, "layernorm: row strides must be even");
   if (rows == 0) return KFB_OK;
-  if (in_dtype == KFB_BF16 && out_dtype == KFB_BF16 && c == 128 && xs == 128 && ys == 128 && perm.rows == 0 &&
+  if (in_dtype == KFB_BF16 && out_dtype == KFB_BF16 && (c == 128 || c == 256) && xs == c && ys == c && perm.rows == 0 &&
       ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(y)) & 15) == 0) {
     long long blocks = (rows + 31) / 32;      // 8 warps x 4 rows per iteration
     const long long cap = static_cast<long long>(sm_count()) * 16;
     if (blocks > cap) blocks = cap;
     LaunchScope scope(stream, "layernorm_rows");
-    KFB_TRY(launch_kernel(stream, layernorm_c128_bf16_kernel, static_cast<unsigned>(blocks), 256, 0,
-        static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), w, b, rows, eps));
+    KFB_TRY(launch_kernel(stream, c == 128 ? layernorm_vec_bf16_kernel<16, 2> : layernorm_vec_bf16_kernel<32, 4>, static_cast<unsigned>(blocks),
+                          256, 0, static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), w, b, rows, eps));
     KFB_CUDA(cudaGetLastError());
     return KFB_OK;
   }
@@ -355,7 +358,8 @@ __global__ void __launch_bounds__(256) layernorm_cm_split_kernel(const float* __
 // ------------------------------------------------------------------------------------------------
 // Adaptive LayerNorm (AdaLN): one warp per row, same register layout as layernorm_rows_kernel.
 // ------------------------------------------------------------------------------------------------
-template <typename TI, typename TO, typename TG, int G>
+// SPLIT: the result as a bf16 triple split (an A operand's row of six times c, see part_a) for the fp32-accurate projections.
+template <typename TI, typename TO, typename TG, int G, bool SPLIT>
 __global__ void __launch_bounds__(256) adaln_rows_kernel(const TI* __restrict__ a, TO* __restrict__ y,
                                                          const TG* __restrict__ gv, long long gv_ld, long long rows, int c,
                                                          int samples, int l, float eps) {
@@ -390,13 +394,22 @@ __global__ void __launch_bounds__(256) adaln_rows_kernel(const TI* __restrict__ 
       }
     }
     const float rstd = rsqrtf(warp_sum(q) / static_cast<float>(c) + eps);
-    TO* yr = y + row * c;
+    TO* yr = y + row * (SPLIT ? 6 * c : c);
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       const int ch = (lane + 32 * g) * 2;
       if (ch < c) {
         const float s0 = 1.f / (1.f + __expf(-gate[g].x)), s1 = 1.f / (1.f + __expf(-gate[g].y));
-        store2<TO>(yr + ch, s0 * (v[g].x * rstd) + shift[g].x, s1 * (v[g].y * rstd) + shift[g].y);
+        const float r0 = s0 * (v[g].x * rstd) + shift[g].x, r1 = s1 * (v[g].y * rstd) + shift[g].y;
+        if constexpr (SPLIT) {
+          __nv_bfloat16 x[2][3];
+          split3(r0, x[0][0], x[0][1], x[0][2]);
+          split3(r1, x[1][0], x[1][1], x[1][2]);
+#pragma unroll
+          for (int q = 0; q < 3; ++q) *reinterpret_cast<__nv_bfloat162*>(yr + part_a(q) * c + ch) = __halves2bfloat162(x[0][q], x[1][q]);
+        } else {
+          store2<TO>(yr + ch, r0, r1);
+        }
       }
     }
   }
@@ -506,7 +519,7 @@ static int launch_adaln_vec(cudaStream_t stream, const void* a, void* y, const v
   return KFB_OK;
 }
 
-template <typename TI, typename TO, typename TG>
+template <typename TI, typename TO, typename TG, bool SPLIT = false>
 static int adaln_dispatch(cudaStream_t stream, const void* a, void* y, const void* gv_, long long gv_ld, long long rows, int c,
                           int samples, int l, float eps) {
   const TG* gv = static_cast<const TG*>(gv_);
@@ -517,7 +530,7 @@ static int adaln_dispatch(cudaStream_t stream, const void* a, void* y, const voi
   const int g = cdiv(c, 64);
   LaunchScope scope(stream, "adaln_rows");
 #define KFB_ADALN(GG)                                                                                          \
-  KFB_TRY(launch_kernel(stream, adaln_rows_kernel<TI, TO, TG, GG>, static_cast<unsigned>(blocks), warps * 32, 0, \
+  KFB_TRY(launch_kernel(stream, adaln_rows_kernel<TI, TO, TG, GG, SPLIT>, static_cast<unsigned>(blocks), warps * 32, 0, \
       static_cast<const TI*>(a), static_cast<TO*>(y), gv, gv_ld, rows, c, samples, l, eps))
   if (g <= 2) KFB_ADALN(2);
   else if (g <= 6) KFB_ADALN(6);
@@ -560,6 +573,8 @@ int launch_adaln(cudaStream_t stream, const void* a, void* y, const void* gv, lo
     return adaln_dispatch<__nv_bfloat16, __nv_bfloat16, __nv_bfloat16>(stream, a, y, gv, gv_ld, rows, c, samples, l, eps);
   if (in_dtype == KFB_FP32 && out_dtype == KFB_BF16)
     return adaln_dispatch<float, __nv_bfloat16, __nv_bfloat16>(stream, a, y, gv, gv_ld, rows, c, samples, l, eps);
+  if (in_dtype == KFB_FP32_PRECISE && out_dtype == KFB_FP32_PRECISE)  // fp32 in, triple split out: no pass of its own for the split
+    return adaln_dispatch<float, __nv_bfloat16, float, true>(stream, a, y, gv, gv_ld, rows, c, samples, l, eps);
   if (in_dtype == KFB_FP32_PRECISE && out_dtype == KFB_FP32)  // everything fp32, gate / shift rows included
     return adaln_dispatch<float, float, float>(stream, a, y, gv, gv_ld, rows, c, samples, l, eps);
   set_error("adaln: unsupported dtype combination");

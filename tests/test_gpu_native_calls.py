@@ -120,3 +120,16 @@ def test_triatt_fp32_key_split(dev, n, batch, c, heads):
     ref = _oracle_on(dev, O.triangle_attention, z, pm, w, heads, True)
     mx, r = err_stats(out, ref)
     assert mx < PRECISE_MAX_TOL and r < PRECISE_RMS_TOL, f"{mx:.3e} {r:.3e}"
+
+
+@pytest.mark.parametrize("rows", [1, 3, 33, 5000])
+@pytest.mark.parametrize("c", [128, 256])
+def test_layernorm_bf16_rows(dev, c, rows):
+    """The 16-byte LayerNorm at row counts that leave part of a warp's rows empty and that make warps loop."""
+    from kfold_b200 import functional as F
+    g = torch.Generator().manual_seed(rows)
+    x = (torch.randn(rows, c, generator=g) * 3 + 1).bfloat16()
+    w, b = torch.rand(c, generator=g) + 0.5, torch.randn(c, generator=g)
+    out = F.layer_norm(x.to(dev), w.to(dev), b.to(dev), 1e-5).float().cpu()
+    ref = torch.nn.functional.layer_norm(x.float(), (c,), w, b, 1e-5)
+    _check(*err_stats(out, ref), f"layernorm {rows} x {c}")
