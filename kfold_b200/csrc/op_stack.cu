@@ -92,7 +92,7 @@ KFB_API size_t kfb_token_stack_workspace_bytes(int groups, int samples, int s_sa
   const long long rows = static_cast<long long>(groups) * samples * l;
   const size_t a = attn_ws(groups * samples, l, c, heads, precise), t = trans_ws(rows, c, hidden, precise);
   return tables_bytes(static_cast<long long>(groups) * s_samples * l, c_s, gs_cols, og_cols, precise) +
-         align_up(static_cast<size_t>(rows) * c * (precise ? 4 : 2), 256) + align_up(a > t ? a : t, 256);
+         align_up(static_cast<size_t>(rows) * c * (precise ? 12 : 2), 256) + align_up(a > t ? a : t, 256);
 }
 
 KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, const kfb_conditioning* cond, const void* a, void* out,
@@ -121,7 +121,7 @@ KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, con
   Carver cv(workspace);
   Tables t;
   KFB_TRY(build_tables(stream, cv, t, *cond, s, s_dtype, static_cast<long long>(groups) * s_samples * l, precise));
-  void* an = cv.take<uint8_t>(static_cast<size_t>(rows) * c * (precise ? 4 : 2));
+  void* an = cv.take<uint8_t>(static_cast<size_t>(rows) * c * (precise ? 12 : 2));   // fp32-accurate: triple-split rows
   const size_t ab = attn_ws(batch, l, c, heads, precise), tb = trans_ws(rows, c, hidden, precise);
   const size_t op_bytes = ab > tb ? ab : tb;
   void* op_ws = cv.take<uint8_t>(op_bytes);
@@ -131,9 +131,10 @@ KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, con
   for (int i = 0; i < n_blocks; ++i) {
     const kfb_token_block& w = blocks[i];
     KFB_TRY(launch_adaln(stream, cur, an, column(t.gs, 4ll * c * i, precise), rows, c, share, l, eps, ada_dtype,
-                         precise ? KFB_FP32 : KFB_BF16, t.gs_cols));
+                         precise ? KFB_FP32_PRECISE : KFB_BF16, t.gs_cols));
     ApbArgs r;
     r.x = an;
+    r.x_is_split = precise;
     r.w_static = 1;
     r.pair_bias = static_cast<const uint8_t*>(pair_bias) + bias_block_stride * i * bias_e;
     r.ldb = bias_ld; r.bias_hs = bias_head_stride; r.bias_div = samples;
@@ -146,8 +147,8 @@ KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, con
     KFB_TRY(apb_run(stream, r));
     cur = out;                                      // from here on the stream is updated in place
     KFB_TRY(launch_adaln(stream, cur, an, column(t.gs, 4ll * c * i + 2ll * c, precise), rows, c, share, l, eps, ada_dtype,
-                         precise ? KFB_FP32 : KFB_BF16, t.gs_cols));
-    KFB_TRY(cond_transition_run(stream, an, 0, 1, w.w_swiglu, w.w_tout, column(t.og, 2ll * c * i + c, precise), t.og_cols, out, cur, op_ws,
+                         precise ? KFB_FP32_PRECISE : KFB_BF16, t.gs_cols));
+    KFB_TRY(cond_transition_run(stream, an, precise, 1, w.w_swiglu, w.w_tout, column(t.og, 2ll * c * i + c, precise), t.og_cols, out, cur, op_ws,
                                 op_bytes, rows, c, hidden, share, l, op_dtype));
   }
   return KFB_OK;
