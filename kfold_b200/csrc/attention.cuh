@@ -55,10 +55,11 @@ struct AttnParams {
   const unsigned char* mask; long long m_hi, m_lo, m_k; int mask_lo_extent;
   // optional gate logits, addressed like q
   const void* g; long long ldg; int g_col0;
-  // non-null: the kernel for pair rows (attention_rows.cu), with this scratch of one entry per batch entry.  It takes head
-  // dims up to 32, a mask, one bias for every bias_div >= 2 consecutive entries (bias_mod = win = 0, batch a multiple of
-  // bias_div), and the bias in log2 units.
+  // non-null: the kernel for entries that share a bias (attention_rows.cu), with this scratch of one entry per batch entry.  It
+  // takes a mask, one bias for every bias_div >= 2 consecutive entries (bias_mod = win = 0, batch a multiple of bias_div), and,
+  // with dpad 32, the bias in log2 units.
   int2* row_info;
+  int row_info_ready;   // 1: the scratch already holds what launch_attention_mask_rows writes for these masks
   // output bf16: row (b, q) at out + (b*lq + q)*ldo, head h at column h*d
   void* out; long long ldo;
   long long* trace;  // debugging aid: when non-null, CTA (0,0,0) stores clock64() stamps of its pipeline events here
@@ -66,6 +67,7 @@ struct AttnParams {
 };
 
 int launch_attention(cudaStream_t stream, const AttnParams& p);
+int launch_attention_mask_rows(cudaStream_t stream, const AttnParams& p);
 int launch_attention_rows(cudaStream_t stream, const AttnParams& p);   // (chosen by launch_attention)
 
 // fp32-accurate mode: q, g and k, v are columns of fp32 row-major buffers (row = batch * L + position, `ld` / `ld_kv`

@@ -36,29 +36,32 @@
 namespace kfb {
 namespace {
 
-constexpr int kD = 32;             // padded head dim
 constexpr int kQ = 128;            // queries per row group
 constexpr int kT = 64;             // keys per tile
-constexpr int kQBytes = kQ * kD * 2;
-constexpr int kKBytes = kT * kD * 2;
-constexpr int kVBytes = kD * kT * 2;
 constexpr int kBiasBytes = kQ * kT * 2;
 constexpr int kMaskBytes = kT * 32;            // a 64 x 16 bf16 K-major operand without swizzle
 constexpr int kE0Bytes = kQ * 32;
-constexpr int kEyeBytes = (48 + 16 + 48) * 32; // a 16 x 16 identity between 48 zero rows on either side: the four K steps of a 64 x 64 identity
+constexpr int kEyeBytes = (48 + 16 + 48) * 32; // a 16 x 16 identity (times a factor) between 48 zero rows on either side: the four K
+                                               // steps of a 64 x 64 one
 
-template <int R>
+// R row groups, padded head dim D (32 or 64)
+template <int R, int D>
 struct RowsCfg {
   static constexpr int kSoftWarps = 4 * R;
   static constexpr int kThreads = 32 * (kSoftWarps + 2 + R);
-  static constexpr int kStages = R == 3 ? 4 : 5;      // ring of tiles: bias, and K, V^T of all row groups
+  static constexpr int kQBytes = kQ * D * 2, kKBytes = kT * D * 2, kVBytes = D * kT * 2;
+  static constexpr int kStages = D == 64 ? 3 : (R == 3 ? 4 : 5);      // ring of tiles: bias, and K, V^T of all row groups
   static constexpr int kStageBytes = kBiasBytes + R * (kKBytes + kVBytes);
-  static constexpr int kMaskSlots = R == 3 ? 1 : 2;   // mask operands per group (shared memory has no room for more)
-  static constexpr int kTmemCols = 512;               // 160 per group are used: S 2 x 64, O 32
-  static constexpr int kSmem = kStages * kStageBytes + 2 * R * kQBytes + R * kMaskSlots * kMaskBytes + kE0Bytes + kEyeBytes + R * 32 * 4 + 1024 /*alignment*/ +
-                               512 /*barriers*/;
+  static constexpr int kMaskSlots = R == 3 || D == 64 ? 1 : 2;   // mask operands per group (shared memory has no room for more)
+  static constexpr int kTmemCols = 512;               // 128 + D per group are used: S 2 x 64, O D
+  // identities: the bias of D = 32 (triangle attention) comes in log2 units; the other callers' does not, and log2(e) is applied
+  // as two bf16 factors, high and low part (relative error 4e-6, below the bias' own bf16 rounding)
+  static constexpr int kEyes = D == 64 ? 2 : 1;
+  static constexpr int kSmem = kStages * kStageBytes + 2 * R * kQBytes + R * kMaskSlots * kMaskBytes + kE0Bytes + kEyes * kEyeBytes +
+                               R * D * 4 + 1024 /*alignment*/ + 512 /*barriers*/;
   static_assert(kSmem <= 227 * 1024, "shared memory");
 };
+constexpr float kLog2e = 1.4426950408889634f;
 constexpr float kMasked = -1e9f * 1.4426950408889634f;   // a masked key: the reference's finite -1e9, in log2 units
 constexpr float kAbsent = -1e30f;                         // keys beyond lk
 constexpr float kHighSum = 1.2676506e30f;                 // 2^100: a tile's row sum above this moves the stabiliser
@@ -115,11 +118,12 @@ __device__ __forceinline__ Item<R> load_item(const RowsParams& p, int item) {
   return it;
 }
 
-template <int R>
-__global__ void __launch_bounds__(RowsCfg<R>::kThreads, 1)
+template <int R, int kD>
+__global__ void __launch_bounds__(RowsCfg<R, kD>::kThreads, 1)
 attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_constant__ CUtensorMap tm_k,
                       const __grid_constant__ CUtensorMap tm_v, const __grid_constant__ CUtensorMap tm_b, const RowsParams p) {
-  using Cfg = RowsCfg<R>;
+  using Cfg = RowsCfg<R, kD>;
+  constexpr int kQBytes = Cfg::kQBytes, kKBytes = Cfg::kKBytes, kVBytes = Cfg::kVBytes, kEyes = Cfg::kEyes;
   constexpr int kStages = Cfg::kStages, kStageBytes = Cfg::kStageBytes, kMaskSlots = Cfg::kMaskSlots;
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -128,8 +132,8 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   uint8_t* s_mask = s_q + 2 * R * kQBytes;                   // [R][slots]
   uint8_t* s_e0 = s_mask + R * kMaskSlots * kMaskBytes;
   uint8_t* s_eye = s_e0 + kE0Bytes;
-  float* s_mean = reinterpret_cast<float*>(s_eye + kEyeBytes); // [R][32]
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_mean + R * 32);
+  float* s_mean = reinterpret_cast<float*>(s_eye + kEyes * kEyeBytes); // [R][D]
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_mean + R * kD);
   uint64_t* stage_full = bars;                    // [stages]
   uint64_t* stage_empty = stage_full + kStages;   // [stages]: a commit per group
   uint64_t* q_full = stage_empty + kStages;       // [2]
@@ -182,12 +186,17 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     *reinterpret_cast<uint4*>(s_e0 + operand_row(r) + 128) = make_uint4(0, 0, 0, 0);
     if (r < 112) {
 #pragma unroll
-      for (int h = 0; h < 2; ++h) {
-        const int one = r - 48 - h * 8;   // column of the row's one within this half of the K step
-        uint32_t w[4];
+      for (int e = 0; e < kEyes; ++e) {
+        const float hi = __bfloat162float(__float2bfloat16_rn(kLog2e));
+        const uint32_t one = __bfloat16_as_ushort(__float2bfloat16_rn(kEyes == 1 ? 1.f : (e == 0 ? hi : kLog2e - hi)));
 #pragma unroll
-        for (int i = 0; i < 4; ++i) w[i] = (one >> 1) == i ? ((one & 1) ? 0x3F800000u : 0x3F80u) : 0u;
-        *reinterpret_cast<uint4*>(s_eye + operand_row(r) + h * 128) = make_uint4(w[0], w[1], w[2], w[3]);
+        for (int h = 0; h < 2; ++h) {
+          const int at = r - 48 - h * 8;   // column of the row's factor within this half of the K step
+          uint32_t w[4];
+#pragma unroll
+          for (int i = 0; i < 4; ++i) w[i] = (at >> 1) == i ? ((at & 1) ? one << 16 : one) : 0u;
+          *reinterpret_cast<uint4*>(s_eye + e * kEyeBytes + operand_row(r) + h * 128) = make_uint4(w[0], w[1], w[2], w[3]);
+        }
       }
     }
     if (r < kT) {
@@ -242,11 +251,11 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const uint64_t e0_desc = noswizzle_desc(ptx::smem_u32(s_e0));
       const uint64_t eye_desc = noswizzle_desc(ptx::smem_u32(s_eye));
       const uint64_t bias_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_stage));
-      const uint64_t q_desc = ptx::make_kmajor_desc<64>(ptx::smem_u32(s_q + g * kQBytes));
-      const uint64_t k_desc = ptx::make_kmajor_desc<64>(ptx::smem_u32(s_stage + kv_off));
+      const uint64_t q_desc = ptx::make_kmajor_desc<kD * 2>(ptx::smem_u32(s_q + g * kQBytes));
+      const uint64_t k_desc = ptx::make_kmajor_desc<kD * 2>(ptx::smem_u32(s_stage + kv_off));
       const uint64_t v_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_stage + kv_off + kKBytes));
       const uint64_t m_desc = noswizzle_desc(ptx::smem_u32(s_mask + g * kMaskSlots * kMaskBytes));
-      const uint32_t tmem_g = tmem_base + g * 160, tmem_o = tmem_g + 128;
+      const uint32_t tmem_g = tmem_base + g * (128 + kD), tmem_o = tmem_g + 128;
       auto first_masked = [&](const Item<R>& it) {
         int f = it.first[0];
 #pragma unroll
@@ -278,8 +287,12 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 #pragma unroll
         for (int c = 0; c < 4; ++c)   // bias x identity: exact products, added in float32 like the rest
           ptx::mma_f16_ss(d, bd + c * 2, eye_desc + (48 - 16 * c) * 2, idesc_s, c > 0 ? 1u : 0u);
-        ptx::mma_f16_ss(d, qd, kd, idesc_s, 1u);
-        ptx::mma_f16_ss(d, qd + 2, kd + 2, idesc_s, 1u);
+        if constexpr (kEyes == 2) {
+#pragma unroll
+          for (int c = 0; c < 4; ++c) ptx::mma_f16_ss(d, bd + c * 2, eye_desc + (kEyeBytes >> 4) + (48 - 16 * c) * 2, idesc_s, 1u);
+        }
+#pragma unroll
+        for (int c = 0; c < kD / 16; ++c) ptx::mma_f16_ss(d, qd + c * 2, kd + c * 2, idesc_s, 1u);
         if (masked) {
           ptx::mma_f16_ss(d, e0_desc, m_desc + m_slot * (kMaskBytes >> 4), idesc_s, 1u);
           ptx::tc_commit(&m_empty[g * kMaskSlots + m_slot]);
@@ -363,7 +376,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     // ---------------------------------------------------------------- softmax and output of row group g
     const int g = warp >> 2, quad = warp & 3;
     const int r = quad * 32 + lane;
-    const uint32_t tmem_g = tmem_base + g * 160 + (static_cast<uint32_t>(quad * 32) << 16);
+    const uint32_t tmem_g = tmem_base + g * (128 + kD) + (static_cast<uint32_t>(quad * 32) << 16);
     const uint32_t tmem_o = tmem_g + 128;
     bool ok = true;
     uint32_t n = 0;                   // tiles so far
@@ -405,7 +418,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           if (!__all_sync(0xffffffffu, ptx::mbar_wait(&pv_done[g * 2 + ((n - 1) & 1)], ((n - 1) >> 1) & 1, 310))) ok = false;
           ptx::tc_fence_after_sync();
 #pragma unroll 1
-          for (int c = 0; c < 2; ++c) {
+          for (int c = 0; c < kD / 16; ++c) {
             uint32_t o16[16];
             ptx::tmem_ld_32x32b_x16(tmem_o + c * 16, o16);
             ptx::tmem_ld_wait();
@@ -460,22 +473,22 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       const int b = it.b0 + min(g, it.rows - 1);
       const long long row = static_cast<long long>(b) * a.lq + (q < a.lq ? q : 0);
       const __nv_bfloat16* gp = a.g != nullptr ? reinterpret_cast<const __nv_bfloat16*>(a.g) + row * a.ldg + a.g_col0 + it.h * kD : nullptr;
-      uint4 gate[4];
+      uint4 gate[kD / 8];
       if (gp != nullptr) {
 #pragma unroll
-        for (int i = 0; i < 4; ++i) gate[i] = *reinterpret_cast<const uint4*>(gp + i * 8);
+        for (int i = 0; i < kD / 8; ++i) gate[i] = *reinterpret_cast<const uint4*>(gp + i * 8);
       }
       float scale = 1.0f;
       if (it.tiles == 0) {
         // no valid key in any row (padding): every logit is the same finite -1e9 in the reference's float32 arithmetic, the result
         // the mean of V over all keys
         const __nv_bfloat16* vrows = reinterpret_cast<const __nv_bfloat16*>(a.vt) + (static_cast<long long>(b) * a.heads + it.h) * kD * a.ldv;
-        for (int dd = quad * 8; dd < quad * 8 + 8; ++dd) {
+        for (int dd = quad * (kD / 4); dd < (quad + 1) * (kD / 4); ++dd) {
           float acc = 0.f;
           for (int key = lane; key < a.lk; key += 32) acc += __bfloat162float(vrows[static_cast<long long>(dd) * a.ldv + key]);
 #pragma unroll
           for (int o = 16; o > 0; o >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, o);
-          if (lane == 0) s_mean[g * 32 + dd] = acc / static_cast<float>(a.lk);
+          if (lane == 0) s_mean[g * kD + dd] = acc / static_cast<float>(a.lk);
         }
         asm volatile("bar.sync %0, 128;" ::"r"(1 + g) : "memory");
       } else {
@@ -486,11 +499,11 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       }
       __nv_bfloat16* o = reinterpret_cast<__nv_bfloat16*>(a.out) + row * a.ldo + it.h * a.d;
 #pragma unroll
-      for (int half = 0; half < 2; ++half) {
+      for (int half = 0; half < kD / 16; ++half) {
         float v[16];
         if (it.tiles == 0) {
 #pragma unroll
-          for (int i = 0; i < 16; ++i) v[i] = s_mean[g * 32 + half * 16 + i];
+          for (int i = 0; i < 16; ++i) v[i] = s_mean[g * kD + half * 16 + i];
         } else {
           ptx::tmem_ld_32x32b_x16(tmem_o + half * 16, reinterpret_cast<uint32_t(&)[16]>(v));
           ptx::tmem_ld_wait();
@@ -581,15 +594,20 @@ __global__ void __launch_bounds__(256) mask_rows_kernel(const AttnParams a, int2
 
 }  // namespace
 
-template <int R>
+int launch_attention_mask_rows(cudaStream_t stream, const AttnParams& a) {
+  LaunchScope scope(stream, "attention_mask_rows");
+  return launch_kernel(stream, mask_rows_kernel, cdiv(a.batch, 32), 256, 0, a, a.row_info);
+}
+
+template <int R, int kD>
 static int launch_rows(cudaStream_t stream, const AttnParams& a) {
-  using Cfg = RowsCfg<R>;
+  using Cfg = RowsCfg<R, kD>;
   static std::once_flag once[64];
   int dev = 0;
   KFB_CUDA(cudaGetDevice(&dev));
   cudaError_t attr_err = cudaSuccess;
   std::call_once(once[dev & 63], [&] {
-    attr_err = cudaFuncSetAttribute(attention_rows_kernel<R>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+    attr_err = cudaFuncSetAttribute(attention_rows_kernel<R, kD>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
   });
   KFB_CUDA(attr_err);
   CUtensorMap tq, tk, tv, tb;
@@ -597,13 +615,13 @@ static int launch_rows(cudaStream_t stream, const AttnParams& a) {
     const uint64_t dims[3] = {(uint64_t)a.ldq, (uint64_t)a.lq, (uint64_t)a.batch};
     const uint64_t str[2] = {(uint64_t)a.ldq * 2, (uint64_t)a.lq * a.ldq * 2};
     const uint32_t box[3] = {kD, kQ, 1};
-    KFB_TRY(make_tmap(&tq, a.q, 2, 3, dims, str, box, 64));
+    KFB_TRY(make_tmap(&tq, a.q, 2, 3, dims, str, box, kD * 2));
   }
   {
     const uint64_t dims[3] = {(uint64_t)a.ldk, (uint64_t)a.lk, (uint64_t)a.batch};
     const uint64_t str[2] = {(uint64_t)a.ldk * 2, (uint64_t)a.lk * a.ldk * 2};
     const uint32_t box[3] = {kD, kT, 1};
-    KFB_TRY(make_tmap(&tk, a.k, 2, 3, dims, str, box, 64));
+    KFB_TRY(make_tmap(&tk, a.k, 2, 3, dims, str, box, kD * 2));
   }
   {
     const uint64_t dims[3] = {(uint64_t)a.lk, (uint64_t)a.heads * kD, (uint64_t)a.batch};
@@ -625,25 +643,23 @@ static int launch_rows(cudaStream_t stream, const AttnParams& a) {
   p.sets_per_bias = cdiv(a.bias_div, R);
   p.q_blocks = cdiv(a.lq, kQ);
   p.items = p.q_blocks * a.heads * p.sets_per_bias * groups;
-  {
-    LaunchScope scope(stream, "attention_mask_rows");
-    KFB_TRY(launch_kernel(stream, mask_rows_kernel, cdiv(a.batch, 32), 256, 0, a, a.row_info));
-  }
+  if (!a.row_info_ready) KFB_TRY(launch_attention_mask_rows(stream, a));
   {
     LaunchScope scope(stream, a.tag ? a.tag : "attention_rows");
-    KFB_TRY(launch_kernel(stream, attention_rows_kernel<R>, p.items < sm_count() ? p.items : sm_count(), Cfg::kThreads, Cfg::kSmem, tq, tk,
+    KFB_TRY(launch_kernel(stream, attention_rows_kernel<R, kD>, p.items < sm_count() ? p.items : sm_count(), Cfg::kThreads, Cfg::kSmem, tq, tk,
                           tv, tb, p));
   }
   return KFB_OK;
 }
 
 int launch_attention_rows(cudaStream_t stream, const AttnParams& a) {
+  if (a.dpad == 64) return launch_rows<2, 64>(stream, a);   // (shared memory has room for two groups)
   // A CTA of three row groups takes 5/4 of the time of two (N = 1024) for 3/2 of the work (more warps to fill each other's waits; one
   // more group would leave a single S buffer each, which measured slower); two leave fewer SMs idle in the last wave of few items.
   auto waves = [&](int r) {
     return cdiv(static_cast<long long>(cdiv(a.lq, kQ)) * a.heads * cdiv(a.bias_div, r) * cdiv(a.batch, a.bias_div), (long long)sm_count());
   };
-  return waves(3) * 5 <= waves(2) * 4 ? launch_rows<3>(stream, a) : launch_rows<2>(stream, a);
+  return waves(3) * 5 <= waves(2) * 4 ? launch_rows<3, 32>(stream, a) : launch_rows<2, 32>(stream, a);
 }
 
 }  // namespace kfb

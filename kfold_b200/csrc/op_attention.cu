@@ -686,6 +686,8 @@ int apb_run(cudaStream_t stream, const ApbArgs& r) {
     p.m_lo = 0;
     p.m_k = 1;
     p.out = w.og; p.ldo = c;
+    p.row_info = r.rows;
+    p.row_info_ready = 1;
     p.tag = "apb_attention";
     KFB_TRY(launch_attention(stream, p));
   }

@@ -5,6 +5,7 @@
 // Both stacks start with the conditioning tables: every AdaLN's gate / shift rows and every output gate of every block depend
 // on the conditioning s alone, so one LayerNorm of s and two GEMMs (each AdaLN's scale folded into its weight columns) produce
 // two wide tables, and the blocks read their columns in place.
+#include "attention.cuh"
 #include "ops_common.cuh"
 
 using namespace kfb;
@@ -79,6 +80,12 @@ int check_cond(const char* what, const kfb_conditioning* cond, const void* s, in
 size_t attn_ws(int batch, int l, int c, int heads, int precise) {
   return precise ? kfb_apb_workspace_bytes_precise(batch, l, c) : kfb_apb_workspace_bytes(batch, l, c, heads);
 }
+// Samples of one complex share their pair bias: with head dims of 33 to 64 their attention goes through the kernel that adds a bias
+// tile to two batch entries at once (attention_rows.cu), where the other kernel's CTAs (one for 128 queries of a head and sample)
+// are more than one wave: 768 tokens x 5 samples, 16 heads of 48, 54 -> 38 us; 256 x 3, one wave, 10 -> 12 us.
+bool attn_shares_bias(int precise, int batch, int samples, int l, int heads, int d) {
+  return !precise && samples >= 2 && d > 32 && static_cast<long long>(cdiv(l, 128)) * heads * batch > sm_count();
+}
 size_t trans_ws(long long rows, int c, int hidden, int precise) {
   return precise ? kfb_cond_transition_workspace_bytes_precise(rows, c, hidden) : kfb_cond_transition_workspace_bytes(rows, hidden);
 }
@@ -92,7 +99,8 @@ KFB_API size_t kfb_token_stack_workspace_bytes(int groups, int samples, int s_sa
   const long long rows = static_cast<long long>(groups) * samples * l;
   const size_t a = attn_ws(groups * samples, l, c, heads, precise), t = trans_ws(rows, c, hidden, precise);
   return tables_bytes(static_cast<long long>(groups) * s_samples * l, c_s, gs_cols, og_cols, precise) +
-         align_up(static_cast<size_t>(rows) * c * (precise ? 12 : 2), 256) + align_up(a > t ? a : t, 256);
+         align_up(static_cast<size_t>(rows) * c * (precise ? 12 : 2), 256) + align_up(sizeof(int2) * groups * samples, 256) +
+         align_up(a > t ? a : t, 256);
 }
 
 KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, const kfb_conditioning* cond, const void* a, void* out,
@@ -122,6 +130,20 @@ KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, con
   Tables t;
   KFB_TRY(build_tables(stream, cv, t, *cond, s, s_dtype, static_cast<long long>(groups) * s_samples * l, precise));
   void* an = cv.take<uint8_t>(static_cast<size_t>(rows) * c * (precise ? 12 : 2));   // fp32-accurate: triple-split rows
+  int2* mask_rows = cv.take<int2>(batch);
+  if (!attn_shares_bias(precise, batch, samples, l, heads, c / heads)) {
+    mask_rows = nullptr;
+  } else {
+    AttnParams m = {};
+    m.batch = batch;
+    m.lk = l;
+    m.mask = mask;
+    m.mask_lo_extent = samples;
+    m.m_hi = l;
+    m.m_k = 1;
+    m.row_info = mask_rows;
+    KFB_TRY(launch_attention_mask_rows(stream, m));   // once for all blocks
+  }
   const size_t ab = attn_ws(batch, l, c, heads, precise), tb = trans_ws(rows, c, hidden, precise);
   const size_t op_bytes = ab > tb ? ab : tb;
   void* op_ws = cv.take<uint8_t>(op_bytes);
@@ -138,7 +160,7 @@ KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, con
     r.w_static = 1;
     r.pair_bias = static_cast<const uint8_t*>(pair_bias) + bias_block_stride * i * bias_e;
     r.ldb = bias_ld; r.bias_hs = bias_head_stride; r.bias_div = samples;
-    r.mask = mask; r.mask_share = samples;
+    r.mask = mask; r.mask_share = samples; r.rows = mask_rows;
     r.w_proj = w.w_proj; r.proj_bias = w.proj_bias; r.w_out = w.w_out; r.out_bias = w.out_bias;
     r.out_gate = column(t.og, 2ll * c * i, precise); r.gate_share = share; r.gate_ld = t.og_cols;
     r.out = out; r.resid = cur;

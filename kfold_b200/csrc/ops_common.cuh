@@ -53,6 +53,7 @@ struct ApbArgs {
   int bias_div = 1;
   const unsigned char* mask = nullptr;  // [batch / mask_share][l]
   int mask_share = 1;
+  int2* rows = nullptr;               // launch_attention_mask_rows' result for the mask: the attention kernel for shared biases
   const void* w_proj = nullptr; const float* proj_bias = nullptr;
   const void* w_out = nullptr; const float* out_bias = nullptr;
   const void* out_gate = nullptr; int gate_share = 1; long long gate_ld = 0;

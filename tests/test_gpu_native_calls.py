@@ -81,6 +81,30 @@ def test_token_stack_ragged(dev, l, groups, samples, own_s, precise):
         _compare(out.float().cpu(), ref, precise, f"token stack L={l}")
 
 
+@pytest.mark.parametrize("l,groups,samples,c,heads", [(65, 4, 3, 768, 16), (130, 2, 5, 768, 16), (257, 1, 4, 768, 16), (200, 3, 4, 512, 8)])
+def test_token_stack_shared_bias(dev, l, groups, samples, c, heads):
+    """Head dims 48 and 64, enough samples per complex for the attention that adds one bias tile to several of them: odd sample
+    counts, ragged tokens, scattered masks, heads whose bias lies far above and below zero."""
+    from kfold_b200 import modules as M
+    import synth
+    rng = synth._Rng(l)
+    w = synth._prefixed("blocks.0.attention", synth.apb_weights(rng, c, 384))
+    w.update(synth._prefixed("blocks.0.transition", synth.conditioned_transition_weights(rng, c, 384)))
+    a, s = rng.normal(groups, samples, l, c), rng.normal(groups, 1, l, 384)
+    bias = rng.normal(groups, 1, 1, heads, l, l).bfloat16().float()
+    bias[:, :, :, 1] = 256.0
+    bias[:, :, :, 2] = -256.0
+    mask = synth.token_mask(l, valid=l - l // 8).view(1, 1, l).expand(groups, 1, l).clone()
+    mask[0, 0, :33] = False
+    mask[-1, 0, 5::7] = False
+    stack = M.CachedGlobalTransformerStack(c, 384, heads, 1).to(dev)
+    stack.load_state_dict(w, strict=True)
+    ref = _oracle_on(dev, O.global_transformer_stack, a, s, bias, mask, w, heads, 1)
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        out = stack(a.to(dev), s.to(dev), bias.to(dev), mask.to(dev))
+    _compare(out.float().cpu(), ref, False, f"token stack L={l}")
+
+
 @pytest.mark.parametrize("starting", [True, False])
 @pytest.mark.parametrize("n,batch,c,heads", [(25, 2, 128, 4), (33, 1, 128, 8), (65, 2, 96, 4), (130, 1, 128, 4), (257, 1, 128, 4)])
 def test_triatt_rows_masks_and_stabiliser(dev, n, batch, c, heads, starting):
