@@ -157,3 +157,18 @@ def test_layernorm_bf16_rows(dev, c, rows):
     out = F.layer_norm(x.to(dev), w.to(dev), b.to(dev), 1e-5).float().cpu()
     ref = torch.nn.functional.layer_norm(x.float(), (c,), w, b, 1e-5)
     _check(*err_stats(out, ref), f"layernorm {rows} x {c}")
+
+
+@pytest.mark.parametrize("d", [6, 130, 132, 768])
+def test_atoms_to_tokens_widths(dev, d):
+    """The masked mean at widths that end inside a warp's channels and that are not whole vectors, with tokens of 0 to 40 atoms."""
+    from kfold_b200 import functional as F
+    g = torch.Generator().manual_seed(d)
+    index = torch.cat([torch.zeros(40, dtype=torch.long), torch.randint(2, 30, (160,), generator=g)]).sort().values.view(1, 200)
+    mask = torch.rand(1, 200, generator=g) < 0.8
+    x = torch.randn(1, 3, 200, d, generator=g)
+    out = F.aggregate_atoms_to_tokens(x.to(dev), index.to(dev), mask.to(dev), 31).cpu()
+    for t in range(31):
+        rows = x[:, :, (index[0] == t) & mask[0]]
+        ref = rows.mean(2) if rows.shape[2] else torch.zeros(1, 3, d)
+        assert torch.allclose(out[:, :, t], ref, atol=1e-5), t
