@@ -353,7 +353,9 @@ KFB_API int kfb_linear_fp32(const void* x, const void* w6, const float* bias, vo
                             size_t workspace_bytes, long long rows, int n, int k, void* stream);
 /* out = LayerNorm(x) W^T (+ bias) (+ resid) at fp32 accuracy (kfb_linear_fp32 with the LayerNorm and the residual fused):
  * `a + linear_s_to_a(layernorm_s(s))` of DiffusionStack.step (src/kfold/model/layers/folding/diffusion.py:568).
- * x, resid, out fp32; ln_w / ln_b fp32 [k] or NULL; normalise == 0 skips the LayerNorm; workspace as kfb_linear_fp32. */
+ * x, resid, out fp32; ln_w / ln_b fp32 [k] or NULL; normalise == 0 skips the LayerNorm; workspace as kfb_linear_fp32.
+ * normalise == KFB_NORMALISE_BF16_ROWS: with the LayerNorm, x bf16 (the heads of a bf16 stack: no float32 copy of x is made). */
+#define KFB_NORMALISE_BF16_ROWS 0x101
 KFB_API int kfb_ln_linear_fp32(const void* x, const float* ln_w, const float* ln_b, const void* w6, const float* bias,
                                const void* resid, void* out, void* workspace, size_t workspace_bytes, long long rows, int n, int k,
                                float eps, int normalise, void* stream);

@@ -103,7 +103,7 @@ class ConfidenceHead(nn.Module):
     def _head(self, seq: nn.Sequential, x: torch.Tensor) -> torch.Tensor:
         """float32 LayerNorm + Linear (the heads run with autocast off, :461-468)."""
         ln, lin = seq[0], seq[1]
-        return F.ln_linear_fp32(x.float(), ln.weight, ln.bias, self._proj.get(lin, x.device, True), None, eps=ln.eps)
+        return F.ln_linear_fp32(x, ln.weight, ln.bias, self._proj.get(lin, x.device, True), None, eps=ln.eps)
 
     @torch.compiler.disable
     def prepare(self, s_inputs: torch.Tensor, s_lm: torch.Tensor, z: torch.Tensor):

@@ -19,6 +19,13 @@ template <>
 __device__ __forceinline__ float2 load2<__nv_bfloat16>(const __nv_bfloat16* p) {
   return __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(p));
 }
+__device__ __forceinline__ float load1(const float* p) { return *p; }
+__device__ __forceinline__ float load1(const __nv_bfloat16* p) { return __bfloat162float(*p); }
+__device__ __forceinline__ float4 load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+__device__ __forceinline__ float4 load4(const __nv_bfloat16* p) {
+  const uint2 u = *reinterpret_cast<const uint2*>(p);
+  return make_float4(__uint_as_float(u.x << 16), __uint_as_float(u.x & 0xffff0000u), __uint_as_float(u.y << 16), __uint_as_float(u.y & 0xffff0000u));
+}
 template <typename T>
 __device__ __forceinline__ void store2(T* p, float a, float b);
 template <>
@@ -268,7 +275,70 @@ __device__ __forceinline__ void split3_store(__nv_bfloat16* y6, int c, int ch, f
   y6[part_a(2) * c + ch] = x2;
 }
 
-__global__ void __launch_bounds__(256) layernorm_split_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y6,
+// One warp per row, G pieces of 128 channels held in registers: four channels of a lane per load and per part's store.
+// HBM-bound; 25 600 rows of 128 float32 channels 13 -> 6 us against the form below, which reads a row three times, channel by
+// channel, and remains for rows that are not whole aligned pieces of four.
+template <typename TI, int G>
+__global__ void __launch_bounds__(256) layernorm_split_vec_kernel(const TI* __restrict__ x, __nv_bfloat16* __restrict__ y6,
+                                                                  const float* __restrict__ w, const float* __restrict__ b,
+                                                                  long long rows, int c, long long xs, float eps, int normalise) {
+  grid_dependency_enter();
+  const int lane = threadIdx.x & 31;
+  const long long warps_per_grid = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  for (long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows;
+       row += warps_per_grid) {
+    const TI* xr = x + row * xs;
+    float v[G][4];
+    float s = 0.f;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int ch = (lane + 32 * g) * 4;
+      v[g][0] = v[g][1] = v[g][2] = v[g][3] = 0.f;
+      if (ch < c) {
+        const float4 f = load4(xr + ch);
+        v[g][0] = f.x; v[g][1] = f.y; v[g][2] = f.z; v[g][3] = f.w;
+      }
+      s += (v[g][0] + v[g][1]) + (v[g][2] + v[g][3]);
+    }
+    float mean = 0.f, rstd = 1.f;
+    if (normalise) {
+      mean = warp_sum(s) / static_cast<float>(c);
+      float q = 0.f;
+#pragma unroll
+      for (int g = 0; g < G; ++g)
+        if ((lane + 32 * g) * 4 < c) {
+#pragma unroll
+          for (int i = 0; i < 4; ++i) q += (v[g][i] - mean) * (v[g][i] - mean);
+        }
+      rstd = 1.0f / sqrtf(warp_sum(q) / static_cast<float>(c) + eps);
+    }
+    __nv_bfloat16* yr = y6 + row * 6 * c;
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int ch = (lane + 32 * g) * 4;
+      if (ch >= c) continue;
+      uint16_t parts[3][4];
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        float o = (v[g][i] - mean) * rstd;
+        if (w != nullptr) o *= w[ch + i];
+        if (b != nullptr) o += b[ch + i];
+        __nv_bfloat16 x0, x1, x2;
+        split3(o, x0, x1, x2);
+        parts[0][i] = __bfloat16_as_ushort(x0);
+        parts[1][i] = __bfloat16_as_ushort(x1);
+        parts[2][i] = __bfloat16_as_ushort(x2);
+      }
+#pragma unroll
+      for (int q = 0; q < 3; ++q)
+        *reinterpret_cast<uint2*>(yr + part_a(q) * c + ch) =
+            make_uint2(parts[q][0] | (static_cast<uint32_t>(parts[q][1]) << 16), parts[q][2] | (static_cast<uint32_t>(parts[q][3]) << 16));
+    }
+  }
+}
+
+template <typename TI>
+__global__ void __launch_bounds__(256) layernorm_split_kernel(const TI* __restrict__ x, __nv_bfloat16* __restrict__ y6,
                                                               const float* __restrict__ w, const float* __restrict__ b,
                                                               long long rows, int c, long long xs, float eps, int normalise) {
   grid_dependency_enter();
@@ -276,22 +346,22 @@ __global__ void __launch_bounds__(256) layernorm_split_kernel(const float* __res
   const long long warps_per_grid = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
   for (long long row = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5); row < rows;
        row += warps_per_grid) {
-    const float* xr = x + row * xs;
+    const TI* xr = x + row * xs;
     float mean = 0.f, rstd = 1.f;
     if (normalise) {
       float s = 0.f;
-      for (int ch = lane; ch < c; ch += 32) s += xr[ch];
+      for (int ch = lane; ch < c; ch += 32) s += load1(xr + ch);
       mean = warp_sum(s) / static_cast<float>(c);
       float q = 0.f;
       for (int ch = lane; ch < c; ch += 32) {
-        const float d = xr[ch] - mean;
+        const float d = load1(xr + ch) - mean;
         q += d * d;
       }
       rstd = 1.0f / sqrtf(warp_sum(q) / static_cast<float>(c) + eps);
     }
     __nv_bfloat16* yr = y6 + row * 6 * c;
     for (int ch = lane; ch < c; ch += 32) {
-      float v = (xr[ch] - mean) * rstd;
+      float v = (load1(xr + ch) - mean) * rstd;
       if (w != nullptr) v *= w[ch];
       if (b != nullptr) v += b[ch];
       split3_store(yr, c, ch, v);
@@ -299,8 +369,9 @@ __global__ void __launch_bounds__(256) layernorm_split_kernel(const float* __res
   }
 }
 
-int launch_layernorm_split(cudaStream_t stream, const float* x, __nv_bfloat16* y6, const float* w, const float* b, long long rows,
-                           int c, long long xs, float eps, int normalise) {
+template <typename TI>
+static int launch_split(cudaStream_t stream, const TI* x, __nv_bfloat16* y6, const float* w, const float* b, long long rows, int c,
+                        long long xs, float eps, int normalise) {
   KFB_CHECK_ARG(rows >= 0 && c > 0, "layernorm_split: rows %lld, channels %d", rows, c);
   if (rows == 0) return KFB_OK;
   const int warps = 8;
@@ -308,10 +379,24 @@ int launch_layernorm_split(cudaStream_t stream, const float* x, __nv_bfloat16* y
   const long long cap = static_cast<long long>(sm_count()) * 16;
   if (blocks > cap) blocks = cap;
   LaunchScope scope(stream, "layernorm_split");
-  KFB_TRY(launch_kernel(stream, layernorm_split_kernel, static_cast<unsigned>(blocks), warps * 32, 0, x, y6, w, b, rows, c,
-      xs, eps, normalise));
-  KFB_CUDA(cudaGetLastError());
-  return KFB_OK;
+  auto launch = [&](auto kernel) {
+    return launch_kernel(stream, kernel, static_cast<unsigned>(blocks), warps * 32, 0, x, y6, w, b, rows, c, xs, eps, normalise);
+  };
+  if (c % 4 != 0 || c > 1024 || xs % 4 != 0 || (reinterpret_cast<uintptr_t>(x) & 15) != 0 || (reinterpret_cast<uintptr_t>(y6) & 7) != 0)
+    return launch(layernorm_split_kernel<TI>);
+  if (c <= 128) return launch(layernorm_split_vec_kernel<TI, 1>);
+  if (c <= 256) return launch(layernorm_split_vec_kernel<TI, 2>);
+  if (c <= 512) return launch(layernorm_split_vec_kernel<TI, 4>);
+  return launch(layernorm_split_vec_kernel<TI, 8>);
+}
+
+int launch_layernorm_split(cudaStream_t stream, const float* x, __nv_bfloat16* y6, const float* w, const float* b, long long rows,
+                           int c, long long xs, float eps, int normalise) {
+  return launch_split(stream, x, y6, w, b, rows, c, xs, eps, normalise);
+}
+int launch_layernorm_split(cudaStream_t stream, const __nv_bfloat16* x, __nv_bfloat16* y6, const float* w, const float* b, long long rows,
+                           int c, long long xs, float eps, int normalise) {
+  return launch_split(stream, x, y6, w, b, rows, c, xs, eps, normalise);
 }
 
 // Channel-major fp32 in, position-major triple split out (fp32-accurate mode).  A block turns 32 positions around through shared

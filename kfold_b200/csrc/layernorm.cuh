@@ -23,6 +23,8 @@ int launch_to_bf16(cudaStream_t stream, const float* x, __nv_bfloat16* y, long l
 // splits (used for operands that are not normalised).
 int launch_layernorm_split(cudaStream_t stream, const float* x, __nv_bfloat16* y6, const float* w, const float* b, long long rows,
                            int c, long long xs, float eps, int normalise);
+int launch_layernorm_split(cudaStream_t stream, const __nv_bfloat16* x, __nv_bfloat16* y6, const float* w, const float* b, long long rows,
+                           int c, long long xs, float eps, int normalise);
 
 // LayerNorm over channels of a CHANNEL-major tensor t[batch][c][pos] (pos contiguous, channel stride
 // `chan_stride`, batch stride `batch_stride`), written POSITION-major y[batch*npos + pos][c] in bf16.

@@ -59,8 +59,13 @@ KFB_API int kfb_ln_linear_fp32(const void* x, const float* ln_w, const float* ln
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "ln_linear_fp32: workspace must be 256-byte aligned");
   cudaStream_t stream = as_stream(stream_);
   __nv_bfloat16* x6 = static_cast<__nv_bfloat16*>(workspace);
-  KFB_TRY(launch_layernorm_split(stream, static_cast<const float*>(x), x6, normalise ? ln_w : nullptr, normalise ? ln_b : nullptr, rows,
-                                 k, k, eps, normalise ? 1 : 0));
+  const int norm = normalise != 0;
+  if (normalise == KFB_NORMALISE_BF16_ROWS)
+    KFB_TRY(launch_layernorm_split(stream, static_cast<const __nv_bfloat16*>(x), x6, norm ? ln_w : nullptr, norm ? ln_b : nullptr, rows, k, k,
+                                   eps, norm));
+  else
+    KFB_TRY(launch_layernorm_split(stream, static_cast<const float*>(x), x6, norm ? ln_w : nullptr, norm ? ln_b : nullptr, rows, k, k, eps,
+                                   norm));
   GemmParams p = {};
   p.n_extent = static_cast<int>(rows);
   p.o_extent = 1;

@@ -192,13 +192,14 @@ def linear_fp32(x: torch.Tensor, w6: torch.Tensor, bias: torch.Tensor | None = N
 
 def ln_linear_fp32(x: torch.Tensor, ln_w: torch.Tensor | None, ln_b: torch.Tensor | None, w6: torch.Tensor,
                    bias: torch.Tensor | None = None, resid: torch.Tensor | None = None, eps: float = 1e-5) -> torch.Tensor:
-    """resid + LayerNorm(x) w^T (+ bias) at float32 accuracy (model/layers/folding/diffusion.py:568): x (..., k) float32,
-    w6 (n, 6k) the bf16 triple split of w; float32 result."""
+    """resid + LayerNorm(x) w^T (+ bias) at float32 accuracy (model/layers/folding/diffusion.py:568): x (..., k) float32
+    or bfloat16, w6 (n, 6k) the bf16 triple split of w; float32 result."""
     _require_cuda(x, w6)
     k = x.shape[-1]
     if w6.shape[1] != 6 * k:
         raise ValueError(f"ln_linear_fp32: weight {tuple(w6.shape)} is not the triple split of a (n, {k}) matrix")
-    x2 = x.reshape(-1, k).float().contiguous()
+    bf = x.dtype == torch.bfloat16        # read as it is: the LayerNorm starts from the same float32 values
+    x2 = (x if bf else x.float()).reshape(-1, k).contiguous()
     n = w6.shape[0]
     out = torch.empty(x2.shape[0], n, dtype=torch.float32, device=x.device)
     res = None if resid is None else resid.expand(*x.shape[:-1], n).reshape(-1, n).float().contiguous()
@@ -208,7 +209,7 @@ def ln_linear_fp32(x: torch.Tensor, ln_w: torch.Tensor | None, ln_b: torch.Tenso
     with L.on_device(x.device):
         ws = _workspace(x.device, lib.kfb_linear_fp32_workspace_bytes(x2.shape[0], k))
         L.check(lib.kfb_ln_linear_fp32(L.ptr(x2), L.ptr(lw), L.ptr(lb), L.ptr(w6), L.ptr(bias), L.ptr(res), L.ptr(out), L.ptr(ws),
-                                       ws.numel(), x2.shape[0], n, k, eps, 1, L.stream_ptr()))
+                                       ws.numel(), x2.shape[0], n, k, eps, L.KFB_NORMALISE_BF16_ROWS if bf else 1, L.stream_ptr()))
     return out.view(*x.shape[:-1], n)
 
 

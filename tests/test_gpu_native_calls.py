@@ -172,3 +172,19 @@ def test_atoms_to_tokens_widths(dev, d):
         rows = x[:, :, (index[0] == t) & mask[0]]
         ref = rows.mean(2) if rows.shape[2] else torch.zeros(1, 3, d)
         assert torch.allclose(out[:, :, t], ref, atol=1e-5), t
+
+
+@pytest.mark.parametrize("bf16", [False, True])
+@pytest.mark.parametrize("rows,k", [(1, 8), (37, 128), (300, 264), (65, 520), (40, 1032)])
+def test_ln_linear_fp32_rows(dev, rows, k, bf16):
+    """The split LayerNorm at the edges of its register forms (up to 128, 256, 512, 1024 channels, above) from both row types."""
+    from kfold_b200 import functional as F
+    from kfold_b200 import packing
+    g = torch.Generator().manual_seed(k)
+    x = torch.randn(rows, k, generator=g) * 2 + 0.5
+    x = x.bfloat16() if bf16 else x
+    lw, lb, w = torch.rand(k, generator=g) + 0.5, torch.randn(k, generator=g), torch.randn(64, k, generator=g) / k ** 0.5
+    out = F.ln_linear_fp32(x.to(dev), lw.to(dev), lb.to(dev), packing.split3_weights(w).to(dev)).cpu()
+    ref = (torch.nn.functional.layer_norm(x.double(), (k,), lw.double(), lb.double(), 1e-5) @ w.double().T).float()
+    mx, r = err_stats(out, ref)
+    assert mx < PRECISE_MAX_TOL and r < PRECISE_RMS_TOL, f"{mx:.3e} {r:.3e}"
