@@ -4,8 +4,8 @@
 // additive pair bias, masked keys get -1e9 (finite, as the reference does), optional sigmoid gate, and the result is written as the
 // bf16 triple split (an A operand's row, see part_a) that the fp32-accurate output projection consumes.
 //
-// A block takes 32 or 64 queries of one head and splits the keys over its eight warps, eight keys at a time; a lane owns one or two
-// query rows, and the warps' (maximum, sum, accumulator) are merged at the end.  The single-track problems (a few hundred queries,
+// A block takes 32 or 64 queries of one head and splits the keys over its eight or four warps, eight keys at a time; a lane owns one
+// or two query rows, and the warps' (maximum, sum, accumulator) are merged at the end.  The single-track problems (a few hundred queries,
 // one batch entry, 16 heads) have too few rows to fill the chip with one thread per row and all keys each: 301 queries x 16 heads x 48
 // took 250 us that way.  A warp stages its own keys in a two-slot ring with cp.async, so nothing but the merge waits for another
 // warp; K and V are read as broadcast 16-byte pieces, which bounds the loop (one load feeds four multiply-adds per query row: two
@@ -19,14 +19,13 @@
 namespace kfb {
 namespace {
 
-constexpr int kWarps = 8;
 constexpr int kKeys = 8;    // keys per warp and step
 
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ptx::smem_u32(smem)), "l"(gmem) : "memory");
 }
 
-template <int D, int QPT>
+template <int D, int QPT, int kWarps>
 struct F32Cfg {
   static constexpr int kQ = 32 * QPT;
   static constexpr int kRing = kWarps * 2 * 2 * kKeys * D;             // floats: [warp][slot][K | V][key][D]
@@ -36,9 +35,9 @@ struct F32Cfg {
   static constexpr int kSmem = (kMain + kBias + 2 * kWarps * kQ) * 4;
 };
 
-template <int D, int QPT>
+template <int D, int QPT, int kWarps>
 __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnFp32Params p) {
-  using Cfg = F32Cfg<D, QPT>;
+  using Cfg = F32Cfg<D, QPT, kWarps>;
   constexpr int kQ = Cfg::kQ;
   grid_dependency_enter();
   extern __shared__ __align__(16) float smem[];
@@ -226,20 +225,20 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
   }
 }
 
-template <int D, int QPT>
+template <int D, int QPT, int kWarps>
 int launch(cudaStream_t stream, const AttnFp32Params& p) {
-  using Cfg = F32Cfg<D, QPT>;
+  using Cfg = F32Cfg<D, QPT, kWarps>;
   static std::once_flag once[64];
   int dev = 0;
   KFB_CUDA(cudaGetDevice(&dev));
   cudaError_t attr_err = cudaSuccess;
   std::call_once(once[dev & 63], [&] {
-    attr_err = cudaFuncSetAttribute(attention_fp32_kernel<D, QPT>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+    attr_err = cudaFuncSetAttribute(attention_fp32_kernel<D, QPT, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
   });
   KFB_CUDA(attr_err);
   LaunchScope scope(stream, p.tag ? p.tag : "attention_fp32");
   const dim3 grid(cdiv(p.lq, Cfg::kQ), p.heads, p.batch);
-  KFB_TRY(launch_kernel(stream, attention_fp32_kernel<D, QPT>, grid, kWarps * 32, Cfg::kSmem, p));
+  KFB_TRY(launch_kernel(stream, attention_fp32_kernel<D, QPT, kWarps>, grid, kWarps * 32, Cfg::kSmem, p));
   return KFB_OK;
 }
 
@@ -248,14 +247,15 @@ int launch(cudaStream_t stream, const AttnFp32Params& p) {
 int launch_attention_fp32(cudaStream_t stream, const AttnFp32Params& p) {
   KFB_CHECK_ARG(p.batch > 0 && p.heads > 0 && p.lq > 0 && p.lk > 0, "attention_fp32: empty problem");
   KFB_CHECK_ARG(p.batch <= 65535 && p.heads <= 65535, "attention_fp32: batch %d / heads %d exceed the grid limits", p.batch, p.heads);
-  // two query rows per lane: half the shared-memory reads per row, but half the blocks (and registers for head dims up to 32 only)
+  // two query rows per lane: half the shared-memory reads per row, but half the blocks (and registers for head dims up to 32 only);
+  // with that many blocks four warps share the keys, which halves what is merged (160 x 160 rows: 180 us with eight)
   const bool two = p.lq > 32 && static_cast<long long>(cdiv(p.lq, 64)) * p.heads * p.batch >= 2ll * sm_count();
   switch (p.d) {
-    case 16: return two ? launch<16, 2>(stream, p) : launch<16, 1>(stream, p);
-    case 24: return two ? launch<24, 2>(stream, p) : launch<24, 1>(stream, p);
-    case 32: return two ? launch<32, 2>(stream, p) : launch<32, 1>(stream, p);
-    case 48: return launch<48, 1>(stream, p);
-    case 64: return launch<64, 1>(stream, p);
+    case 16: return two ? launch<16, 2, 4>(stream, p) : launch<16, 1, 8>(stream, p);
+    case 24: return two ? launch<24, 2, 4>(stream, p) : launch<24, 1, 8>(stream, p);
+    case 32: return two ? launch<32, 2, 4>(stream, p) : launch<32, 1, 8>(stream, p);
+    case 48: return launch<48, 1, 8>(stream, p);
+    case 64: return launch<64, 1, 8>(stream, p);
     default:
       set_error("attention_fp32: head dim %d not supported (16, 24, 32, 48, 64)", p.d);
       return KFB_ERR_UNSUPPORTED;
