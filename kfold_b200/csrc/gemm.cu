@@ -49,7 +49,8 @@ static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorM
   using Cfg = GemmCfg<BN>;
   p.stages = Cfg::stages_for(p.aux ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes : Cfg::kStagingBytes);
   if constexpr (BN == 32) {
-    KFB_CHECK_ARG(!p.precise && !p.glu && !p.aux, "32-column tiles exist for the plain kernel only");
+    KFB_CHECK_ARG(!p.glu && !p.aux, "32-column tiles exist for the plain kernels only");
+    if (p.precise) return launch_variant<32, false, false, true>(stream, ta, tb, tout, p, tag);
     return launch_variant<32, false, false, false>(stream, ta, tb, tout, p, tag);
   } else {
   if constexpr (BN <= 128) {
@@ -83,7 +84,7 @@ static int narrow_tile(const GemmParams& p, int bn) {
   const long long sms = sm_count();
   if (static_cast<long long>(p.num_m_tiles) * cdiv(p.n_cols, bn) >= sms) return bn;
   const int num_k = p.precise ? 3 * cdiv(p.k_extent / 6, kBK) : cdiv(p.k_extent, kBK);
-  const int lo = p.glu || p.precise ? 64 : 32;
+  const int lo = p.glu ? 64 : 32;
   double best = 1e30;
   int pick = bn;
   for (int w = bn; w >= lo; w /= 2) {

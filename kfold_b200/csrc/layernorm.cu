@@ -104,15 +104,13 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* __restric
   }
 }
 
-// The pair tracks' shapes: 128 or 256 bf16 channels, contiguous rows.  A row is LANES x 16 bytes, LANES 16 or 32, so a warp takes
-// 32 / LANES rows per step and STEPS steps per iteration: 1 or 2 KB in flight per warp, 16-byte loads and stores, the statistics
-// reduced over the lanes of a row.  Same arithmetic as layernorm_rows_kernel (two passes, fp32), whose 4-byte accesses took 150 us
-// for 768 x 768 rows of 256 channels (92 at the memory's rate).
-template <int LANES, int STEPS>
-__global__ void __launch_bounds__(256) layernorm_vec_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
+// The pair track's shape: 128 bf16 channels, contiguous rows.  A row is 256 bytes = 16 lanes x 16 bytes, so a warp takes two
+// rows per step and two steps per iteration: four rows (1 KB) in flight per warp, 16-byte loads and stores, the statistics
+// reduced over the 16 lanes of a row.  Same arithmetic as layernorm_rows_kernel (two passes, fp32).
+__global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                                                   const float* __restrict__ w, const float* __restrict__ b,
                                                                   long long rows, float eps) {
-  constexpr int C = LANES * 8, kRows = 32 / LANES;
+  constexpr int LANES = 16, STEPS = 2, C = LANES * 8, kRows = 32 / LANES;
   grid_dependency_enter();
   const int lane = threadIdx.x & 31;
   const int sub = lane % LANES;              // 16-byte chunk of the row
@@ -171,6 +169,62 @@ __global__ void __launch_bounds__(256) layernorm_vec_bf16_kernel(const __nv_bflo
   }
 }
 
+// 256 bf16 channels, contiguous rows: layernorm_rows_kernel's lane layout, expressions and bits, with the weights kept in registers
+// and four rows in flight per warp.  That kernel, one row at a time with the weights fetched for each, took 150 us for 768 x 768
+// rows; this one 130 (92 at the memory's rate; 16-byte accesses gave 96, but another order of summation: a last-bit difference that
+// four blocks of bf16 rounding turn into 0.8 % of the result).
+constexpr int kC256Rows = 4;
+__global__ void __launch_bounds__(256) layernorm_c256_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
+                                                                  const float* __restrict__ w, const float* __restrict__ b,
+                                                                  long long rows, float eps) {
+  constexpr int G = 4, C = 256;
+  grid_dependency_enter();
+  const int lane = threadIdx.x & 31;
+  float2 ww[G], bb[G];
+#pragma unroll
+  for (int g = 0; g < G; ++g) {
+    ww[g] = w != nullptr ? *reinterpret_cast<const float2*>(w + (lane + 32 * g) * 2) : make_float2(1.f, 1.f);
+    bb[g] = b != nullptr ? *reinterpret_cast<const float2*>(b + (lane + 32 * g) * 2) : make_float2(0.f, 0.f);
+  }
+  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  const long long warp_id = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  for (long long base = warp_id * kC256Rows; base < rows; base += warps * kC256Rows) {
+    float2 v[kC256Rows][G];
+#pragma unroll
+    for (int r = 0; r < kC256Rows; ++r) {
+      const __nv_bfloat16* xr = x + (base + r < rows ? base + r : rows - 1) * C;
+#pragma unroll
+      for (int g = 0; g < G; ++g) v[r][g] = load2<__nv_bfloat16>(xr + (lane + 32 * g) * 2);
+    }
+#pragma unroll
+    for (int r = 0; r < kC256Rows; ++r) {
+      float s = 0.f;
+#pragma unroll
+      for (int g = 0; g < G; ++g) s += v[r][g].x + v[r][g].y;
+      const float mean = warp_sum(s) / static_cast<float>(C);
+      float q = 0.f;
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        v[r][g].x -= mean;
+        v[r][g].y -= mean;
+        q += v[r][g].x * v[r][g].x + v[r][g].y * v[r][g].y;
+      }
+      const float rstd = rsqrtf(warp_sum(q) / static_cast<float>(C) + eps);
+      if (base + r >= rows) break;
+      __nv_bfloat16* yr = y + (base + r) * C;
+#pragma unroll
+      for (int g = 0; g < G; ++g) {
+        float a0 = v[r][g].x * rstd, a1 = v[r][g].y * rstd;
+        a0 *= ww[g].x;
+        a1 *= ww[g].y;
+        a0 += bb[g].x;
+        a1 += bb[g].y;
+        store2<__nv_bfloat16>(yr + (lane + 32 * g) * 2, a0, a1);
+      }
+    }
+  }
+}
+
 template <typename TI, typename TO, int G>
 static int launch_rows(cudaStream_t stream, const void* x, void* y, const float* w, const float* b, long long rows, int c,
                        long long xs, long long ys, float eps, RowPerm perm) {
@@ -222,7 +276,7 @@ int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w
     const long long cap = static_cast<long long>(sm_count()) * 16;
     if (blocks > cap) blocks = cap;
     LaunchScope scope(stream, "layernorm_rows");
-    KFB_TRY(launch_kernel(stream, c == 128 ? layernorm_vec_bf16_kernel<16, 2> : layernorm_vec_bf16_kernel<32, 4>, static_cast<unsigned>(blocks),
+    KFB_TRY(launch_kernel(stream, c == 128 ? layernorm_c128_bf16_kernel : layernorm_c256_bf16_kernel, static_cast<unsigned>(blocks),
                           256, 0, static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), w, b, rows, eps));
     KFB_CUDA(cudaGetLastError());
     return KFB_OK;

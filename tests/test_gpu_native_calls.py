@@ -157,6 +157,10 @@ def test_layernorm_bf16_rows(dev, c, rows):
     out = F.layer_norm(x.to(dev), w.to(dev), b.to(dev), 1e-5).float().cpu()
     ref = torch.nn.functional.layer_norm(x.float(), (c,), w, b, 1e-5)
     _check(*err_stats(out, ref), f"layernorm {rows} x {c}")
+    if c == 256:    # same bits as the general kernel, which takes rows that are not contiguous
+        wide = torch.zeros(rows, c + 8, dtype=torch.bfloat16)
+        wide[:, :c] = x
+        assert torch.equal(out, F.layer_norm(wide.to(dev)[:, :c], w.to(dev), b.to(dev), 1e-5).float().cpu())
 
 
 @pytest.mark.parametrize("d", [6, 130, 132, 768])
