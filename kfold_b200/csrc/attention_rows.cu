@@ -1,5 +1,5 @@
-// Triangle attention over pair rows, head dim <= 32 (see attention.cuh for the operator): a persistent kernel whose time is the
-// softmax warps'.
+// Attention of batch entries that share their bias (see attention.cuh for the operator): triangle attention over pair rows, head dim
+// <= 32, and the token transformer's samples, head dim <= 64.  A persistent kernel whose time is the softmax warps'.
 //
 // What bounds it.  A 128 x 64 tile of logits is 8 192 exponentials, 512 cycles of the SM's MUFU.  The kernel of attention.cu (two
 // CTAs per SM, eight softmax warps each, a thread per row and 32 keys) took 1 100 cycles per tile plus 9 000 per CTA of fill and
