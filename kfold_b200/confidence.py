@@ -16,6 +16,7 @@ from torch import nn
 from . import functional as F
 from .modules import (LayerNorm, LinearNoBias, SelfAttentionPairBias, Transition, TriangularBlock, _check_inference, _is_precise,
                       _PairBlockPlan, _ProjectionCache, compute_dtype)
+from .plans import handed_out
 
 __all__ = ["ConfidencePairSingleBlock", "ConfidencePairSingleStack", "ConfidenceHead"]
 
@@ -44,7 +45,7 @@ class ConfidencePairSingleBlock(nn.Module):
                 pb = self.pair_block
                 self._plan = _PairBlockPlan(self, z.device, cd, precise, pb.tri_mul_out, pb.tri_mul_in, pb.transition_z, None,
                                             (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
-            return F.pair_block(z, pair_mask, self._plan, s, mask, precise)
+            return F.pair_block(z, pair_mask, handed_out(self._plan), s, mask, precise)
         z = self.pair_block(z, pair_mask)
         ln = self.layernorm_z
         with torch.autocast(z.device.type, enabled=False):
@@ -131,7 +132,7 @@ class ConfidenceHead(nn.Module):
         if self._dgram_w.get("key") != key:
             self._dgram_w = {"key": key, "w": w.detach().t().to(z.device, z.dtype).contiguous()}
         with torch.autocast(z.device.type, enabled=False):
-            z = F.distogram_embed_add(z, x, self.boundaries, self._dgram_w["w"])
+            z = F.distogram_embed_add(z, x, self.boundaries, handed_out(self._dgram_w["w"]))
         pair_mask = mask[..., :, None] & mask[..., None, :]
         z, s = self.stack(z, s.clone(), pair_mask, mask)
         with torch.autocast(z.device.type, enabled=False):

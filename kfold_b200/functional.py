@@ -11,6 +11,7 @@ from __future__ import annotations
 import torch
 
 from . import _lib as L
+from .plans import handed_out
 
 _workspaces: dict = {}
 
@@ -23,7 +24,15 @@ def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
         _workspaces.pop(key, None)
         ws = torch.empty(int(nbytes * 1.05) + 4096, dtype=torch.uint8, device=device)
         _workspaces[key] = ws
-    return ws
+    return handed_out(ws)
+
+
+def withdraw_workspaces(tensors) -> None:
+    """Take `tensors` out of the workspaces that later calls are given: their holder uses them alone from now on."""
+    held = {id(t) for t in tensors}
+    for key, ws in list(_workspaces.items()):
+        if id(ws) in held:
+            _workspaces.pop(key, None)
 
 
 def release_workspaces() -> None:

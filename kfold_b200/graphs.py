@@ -12,12 +12,15 @@ import threading
 
 import torch
 
+from . import functional as F
+from .plans import HandedOut
+
 _local = threading.local()
 
 
 def _capture_stream(device: torch.device) -> torch.cuda.Stream:
     """This thread's side stream for warm-up and capture on `device`.  One stream for all captures: memory the allocator has
-    cached for it, and the workspace the operators keep per stream, serve the next capture instead of being allocated anew."""
+    cached for it, that of a workspace whose graph is gone included, serves the next capture instead of being allocated anew."""
     streams = _local.__dict__.setdefault("streams", {})
     index = torch.cuda.current_device() if device.index is None else device.index
     if index not in streams:
@@ -37,12 +40,18 @@ class GraphedCall:
     transformers) in caches that already hold their result when the capture runs, so those kernels are NOT part of the
     graph: the pair tensor ``z``, the window pair tensor ``p`` and ``pair_bias`` must be closed over by ``fn``, never passed
     as inputs that later calls replace -- a replay would keep using the bias of the captured tensors.  For a new complex
-    build a new GraphedCall.
+    build a new GraphedCall; the earlier one stays valid.
+
+    A graph holds addresses, so a GraphedCall owns what lies at them for as long as it lives: ``fn`` and what it closes over, its
+    workspaces (from then on no other call is given them) and everything that the modules called keep between calls -- packed
+    weights, the converted pair bias, the window biases -- even after a module has replaced it.  What a *parameter* points to is
+    not held: weights must not be replaced while the graph is in use.
     """
 
     def __init__(self, fn, *example_inputs: torch.Tensor, warmup: int = 2):
         if not example_inputs or not all(t.is_cuda for t in example_inputs):
             raise ValueError("GraphedCall needs CUDA tensors as example inputs")
+        self._fn = fn
         self._inputs = [t.clone() for t in example_inputs]
         dev = example_inputs[0].device
         with torch.cuda.device(dev), torch.no_grad():
@@ -58,10 +67,13 @@ class GraphedCall:
                 self._graph = torch.cuda.CUDAGraph()
                 self._graph.capture_begin()
                 try:
-                    self._output = fn(*self._inputs)
+                    with HandedOut() as used:
+                        self._output = fn(*self._inputs)
                 finally:
                     self._graph.capture_end()
             current.wait_stream(side)
+        self._kept, self._streams = used.tensors(), set()
+        F.withdraw_workspaces(self._kept)
 
     def __call__(self, *inputs: torch.Tensor):
         if len(inputs) != len(self._inputs):
@@ -71,5 +83,12 @@ class GraphedCall:
                 raise ValueError(f"input {tuple(src.shape)} {src.dtype} does not match the captured {tuple(dst.shape)} {dst.dtype}")
             if dst.data_ptr() != src.data_ptr():
                 dst.copy_(src, non_blocking=True)
+        stream = torch.cuda.current_stream(self._inputs[0].device)
+        if stream.cuda_stream not in self._streams:
+            # the kernels of a replay use this memory on a stream that it was not allocated on: it goes back to its own only
+            # when the replays that are under way at that time have ended
+            for t in self._kept + self._inputs:
+                t.record_stream(stream)
+            self._streams.add(stream.cuda_stream)
         self._graph.replay()
         return self._output

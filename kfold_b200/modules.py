@@ -27,7 +27,7 @@ from torch import nn
 from . import functional as F
 from . import _lib as L
 from . import packing
-from .plans import ParamState
+from .plans import ParamState, handed_out
 
 __all__ = [
     "LayerNorm", "LinearNoBias", "Linear",
@@ -127,7 +127,7 @@ class _PackedMixin:
             sd = {k: v for k, v in self.state_dict().items()}
             self._pack_cache = pack_fn(sd, device)
             self._pack_key, self._pack_state = key, ParamState(self)
-        return self._pack_cache
+        return handed_out(self._pack_cache)
 
 
 # --------------------------------------------------------------------------------------------
@@ -310,7 +310,7 @@ class _ConditioningBank:
         if self._key != key:
             self._packed = self.pack(adalns, gates, device)
             self._key = key
-        return self._packed
+        return handed_out(self._packed)
 
     def tables(self, s: torch.Tensor, adalns, gates):
         """-> (gate_shift, out_gate): lists of views, one per AdaLN (..., L, 2 c_a) and one per gate (..., L, c_a)."""
@@ -393,7 +393,7 @@ class SelfAttentionPairBias(nn.Module, _PackedMixin):
             wd = packing.split3_weights(w).to(device) if precise else w.detach().to(device, torch.bfloat16).contiguous()
             self._ada_w = (wd, b.detach().to(device, torch.float32).contiguous())
             self._ada_key = key
-        return self._ada_w
+        return handed_out(self._ada_w)
 
     @torch.compiler.disable
     def forward(self, a: torch.Tensor, s: torch.Tensor | None, pair_bias: torch.Tensor, mask: torch.Tensor,
@@ -544,7 +544,7 @@ def _token_pair_bias(z: torch.Tensor, layernorm_z, linear_z_to_bias, blocks: int
         zz = z.float() if precise else z.to(torch.bfloat16)
         if lp != l:
             zz = torch.nn.functional.pad(zz, (0, 0, 0, lp - l, 0, lp - l))
-        out = F.pair_bias(zz, layernorm_z.weight.detach().float(), None, cache["w"], layernorm_z.eps)      # (B, blocks*H, L, L)
+        out = F.pair_bias(zz, layernorm_z.weight.detach().float(), None, handed_out(cache["w"]), layernorm_z.eps)      # (B, blocks*H, L, L)
     out = out.view(b, blocks, heads, lp, lp)
     return out if lp == l else out[..., :l, :l]
 
@@ -595,7 +595,7 @@ class CachedGlobalTransformerStack(nn.Module):
             # the conversion may have copied: keep the source alive, so that its address cannot be handed to the bias of
             # the next complex (same shape, version 0) while this entry is still in the cache
             self._bias_src = pair_bias
-        return self._bias_cache
+        return handed_out(self._bias_cache)
 
     def _plan_for(self, device, precise: bool) -> "_StackPlan":
         if self._plan is None or not self._plan.fits(device, precise):
@@ -606,7 +606,7 @@ class CachedGlobalTransformerStack(nn.Module):
                                "w_swiglu": pt["w_swiglu"], "w_tout": pt["w_out"]})
             self._plan = _StackPlan(self, blocks, L.TokenBlock, [m for b in self.blocks for m in (b.attention.adaln_a, b.transition.adaln)],
                                     [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)], device, precise)
-        return self._plan
+        return handed_out(self._plan)
 
     def reset_caches(self) -> None:
         """Forget the converted pair bias (call once per complex when the bias tensor is overwritten in place under
@@ -868,7 +868,7 @@ class LocalTransformerStack(nn.Module):
         if self._bias_w_key != key:
             self._bias_w = torch.cat([w.detach() for w in ws], dim=0).to(device, dt).contiguous()
             self._bias_w_key = key
-        return self._bias_w
+        return handed_out(self._bias_w)
 
     def _window_biases(self, z: torch.Tensor, dt) -> torch.Tensor:
         """LayerNorm(z) projected to the heads of every block, head-major.  The window pair tensor does not change between
@@ -883,7 +883,7 @@ class LocalTransformerStack(nn.Module):
                                            None if ln.bias is None else ln.bias.detach().float(), w, ln.eps)
             self._bias_all_key = key
             self._bias_all_src = z          # keeps z's storage alive so that its address cannot be reused
-        return self._bias_all
+        return handed_out(self._bias_all)
 
     def _plan_for(self, device) -> _StackPlan:
         if self._plan is None or not self._plan.fits(device, False):
@@ -895,7 +895,7 @@ class LocalTransformerStack(nn.Module):
             self._plan = _StackPlan(self, blocks, L.AtomBlock,
                                     [m for b in self.blocks for m in (b.attention.adaln_a_q, b.attention.adaln_a_k, b.transition.adaln)],
                                     [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)], device, False)
-        return self._plan
+        return handed_out(self._plan)
 
     def reset_caches(self) -> None:
         """Forget the window biases (see CachedGlobalTransformerStack.reset_caches)."""
@@ -991,7 +991,7 @@ class _ProjectionCache:
             wd = packing.split3_weights(w).to(device) if precise else w.detach().to(device, torch.bfloat16).contiguous()
             hit = (key, wd)
             self._c[id(lin)] = hit
-        return hit[1]
+        return handed_out(hit[1])
 
 
 def _project(x: torch.Tensor, w: torch.Tensor, precise: bool) -> torch.Tensor:
@@ -1234,7 +1234,7 @@ class TriangularBlock(nn.Module):
         if z.dim() == 4 and F.takes_any_n(z.shape[1], precise):      # one native call
             if self._plan is None or not self._plan.fits(z.device, cd, precise):
                 self._plan = _PairBlockPlan(self, z.device, cd, precise, self.tri_mul_out, self.tri_mul_in, self.transition_z)
-            return F.pair_block(z, pair_mask, self._plan, precise=precise)
+            return F.pair_block(z, pair_mask, handed_out(self._plan), precise=precise)
         z = self.tri_mul_out(z, pair_mask, residual=True)
         z = self.tri_mul_in(z, pair_mask, residual=True)
         return self.transition_z(z, residual=True)
@@ -1269,6 +1269,7 @@ class PairformerBlock(nn.Module):
         if self._bias_key != key:
             self._bias_w = packing.split3_weights(p).to(z.device) if precise else p.detach().to(z.device, torch.bfloat16).contiguous()
             self._bias_key = key
+        handed_out(self._bias_w)
         n = z.shape[1]
         if n % 8 != 0:  # rare: pad the pair tensor so that bias rows stay 16-byte aligned
             npad = (n + 7) // 8 * 8
@@ -1290,7 +1291,7 @@ class PairformerBlock(nn.Module):
                 self._plan = _PairBlockPlan(self, z.device, cd, precise, self.tri_mul_out, self.tri_mul_in, self.transition_z,
                                             (self.tri_att_start, self.tri_att_end),
                                             (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
-            return F.pair_block(z, pair_mask, self._plan, s, mask, precise)
+            return F.pair_block(z, pair_mask, handed_out(self._plan), s, mask, precise)
         z = self.tri_mul_out(z, pair_mask, residual=True)
         z = self.tri_mul_in(z, pair_mask, residual=True)
         z = self.tri_att_start(z, pair_mask, residual=True)

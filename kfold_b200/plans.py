@@ -7,7 +7,55 @@ there: about 0.15 us per parameter.
 """
 from __future__ import annotations
 
-__all__ = ["ParamState"]
+import threading
+
+import torch
+
+__all__ = ["ParamState", "handed_out", "HandedOut"]
+
+_recording = threading.local()
+
+
+def handed_out(kept):
+    """Every place that keeps device memory between calls (workspaces, packed weights, what is derived from the tensors of one
+    complex) passes what it gives to a call through here, so that a CUDA graph can hold what its kernels point to."""
+    seen = getattr(_recording, "seen", None)
+    if seen is not None:
+        seen[id(kept)] = kept
+    return kept
+
+
+class HandedOut:
+    """``with HandedOut() as h:`` collects in `h.kept` everything that calls of this thread were handed meanwhile."""
+
+    def __init__(self):
+        self.kept = {}
+
+    def __enter__(self):
+        self._outer = getattr(_recording, "seen", None)
+        _recording.seen = self.kept
+        return self
+
+    def __exit__(self, *exc):
+        _recording.seen = self._outer
+        if self._outer is not None:
+            self._outer.update(self.kept)
+        return False
+
+    def tensors(self) -> list:
+        """The tensors among it: themselves, the values of a dict or a sequence, the `keep` list of a plan."""
+        out, todo = {}, list(self.kept.values())
+        while todo:
+            t = todo.pop()
+            if isinstance(t, torch.Tensor):
+                out[id(t)] = t
+            elif isinstance(t, dict):
+                todo += t.values()
+            elif isinstance(t, (list, tuple)):
+                todo += t
+            else:
+                todo += getattr(t, "keep", ())
+        return list(out.values())
 
 
 def _version(p):

@@ -19,6 +19,7 @@ from torch import nn
 from . import functional as F
 from . import packing
 from .modules import LayerNorm, Linear, LinearNoBias, Transition, _check_inference, _is_precise, compute_dtype
+from .plans import handed_out
 
 __all__ = ["ParcaeRecurrence", "LMToPair", "PairConditioning"]
 
@@ -54,7 +55,7 @@ class ParcaeRecurrence(nn.Module):
             # the reference casts both to the autocast dtype before use (model.py:505)
             self._dyn = (a.to(torch.bfloat16).float().to(device).contiguous(), b.to(device, torch.bfloat16).contiguous())
             self._dyn_key = key
-        return self._dyn
+        return handed_out(self._dyn)
 
     @torch.compiler.disable
     def forward(self, z: torch.Tensor, u: torch.Tensor) -> torch.Tensor:
@@ -88,7 +89,7 @@ class LMToPair(nn.Module):
             self._w = [(m.weight.detach().to(device, torch.bfloat16).contiguous(), m.bias.detach().to(device, torch.float32).contiguous())
                        for m in lins]
             self._w_key = key
-        return self._w
+        return handed_out(self._w)
 
     @torch.compiler.disable
     def forward(self, s_lm: torch.Tensor) -> torch.Tensor:
@@ -130,7 +131,7 @@ class PairConditioning(nn.Module):
             wp = tF.pad(w.detach().float(), (0, k_pad - w.shape[1]))          # zero columns for the padded features
             self._w = packing.split3_weights(wp).to(device)
             self._w_key = key
-        return self._w
+        return handed_out(self._w)
 
     @torch.compiler.disable
     def forward(self, rel_pos, z: torch.Tensor) -> torch.Tensor:
