@@ -51,6 +51,7 @@ class LayerNorm(nn.Module):
         self.weight = nn.Parameter(torch.ones(normalized_shape)) if create_scale else None
         self.bias = nn.Parameter(torch.zeros(normalized_shape)) if create_offset else None
 
+    @torch.compiler.disable
     def forward(self, x: torch.Tensor) -> torch.Tensor:
         _check_inference(x)
         return F.layer_norm(x, self.weight, self.bias, self.eps)
@@ -528,6 +529,7 @@ class TokenPairBias(nn.Module):
         return _token_pair_bias(z, self.layernorm_z, self.linear_z_to_bias, self.blocks, self.heads, self._cache)
 
 
+@torch.compiler.disable
 def _token_pair_bias(z: torch.Tensor, layernorm_z, linear_z_to_bias, blocks: int, heads: int, cache: dict) -> torch.Tensor:
     """LayerNorm(z) projected to blocks x heads values per pair, laid out (B, Nblock, H, L, L)
     (model/layers/folding/diffusion.py:411-416); `cache` keeps the device copy of the projection weight."""
@@ -1227,6 +1229,7 @@ class TriangularBlock(nn.Module):
         self.transition_z = Transition(channel_z, expansion_factor=4)
         self._plan = None
 
+    @torch.compiler.disable
     def forward(self, z: torch.Tensor, pair_mask: torch.Tensor) -> torch.Tensor:
         _check_inference(z)
         cd = compute_dtype(z)
