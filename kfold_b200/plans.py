@@ -8,6 +8,7 @@ there: about 0.15 us per parameter.
 from __future__ import annotations
 
 import threading
+from itertools import chain
 
 import torch
 
@@ -65,31 +66,28 @@ def _version(p):
         return None
 
 
+def _values(dicts):
+    return chain.from_iterable(map(dict.values, dicts))
+
+
 class ParamState:
     """Addresses and in-place versions of every parameter below `modules`, as they were when this was made."""
 
-    __slots__ = ("_slots", "_children", "_seen")
+    __slots__ = ("_parameters", "_modules", "_empty", "_children", "_seen")
 
     def __init__(self, *modules):
-        self._slots, self._children = [], []
-        for root in modules:
-            for m in root.modules():
-                self._slots += [(m._parameters, name) for name, p in m._parameters.items() if p is not None]
-                self._children += [(m._modules, name, child) for name, child in m._modules.items()]
-        self._seen = self._read()
+        # the dictionaries themselves: a parameter or a submodule that is added where there was none shows in them too
+        dicts = [(m._parameters, m._modules) for root in modules for m in root.modules()]
+        self._parameters, self._modules = [p for p, _ in dicts if p], [c for _, c in dicts if c]
+        self._empty = [d for pair in dicts for d in pair if not d]
+        self._children, self._seen = list(_values(self._modules)), self._read()
 
     def _read(self):
-        ps = [d.get(name) for d, name in self._slots]
         try:
-            return [(p.data_ptr(), p._version) for p in ps]
+            return [(p.data_ptr(), p._version) for p in _values(self._parameters) if p is not None]
         except RuntimeError:
-            return [(p.data_ptr(), _version(p)) for p in ps]
-        except AttributeError:      # a parameter was removed
-            return None
+            return [(p.data_ptr(), _version(p)) for p in _values(self._parameters) if p is not None]
 
     def current(self) -> bool:
         """Whether nothing changed since."""
-        for d, name, child in self._children:
-            if d.get(name) is not child:
-                return False
-        return self._read() == self._seen
+        return not any(self._empty) and list(_values(self._modules)) == self._children and self._read() == self._seen
