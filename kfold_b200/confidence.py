@@ -14,14 +14,15 @@ import torch
 from torch import nn
 
 from . import functional as F
-from .modules import (LayerNorm, LinearNoBias, SelfAttentionPairBias, Transition, TriangularBlock, _check_inference, _is_precise,
-                      _PairBlockPlan, _ProjectionCache, compute_dtype)
-from .plans import handed_out
+from .modules import (LayerNorm, LinearNoBias, SelfAttentionPairBias, Transition, TriangleMultiplicationIncoming,
+                      TriangleMultiplicationOutgoing, TriangularBlock, _check_inference, _is_precise, _PairBlockPlan, _ProjectionCache,
+                      compute_dtype)
+from .plans import NativeCall, StandsFor, handed_out
 
 __all__ = ["ConfidencePairSingleBlock", "ConfidencePairSingleStack", "ConfidenceHead"]
 
 
-class ConfidencePairSingleBlock(nn.Module):
+class ConfidencePairSingleBlock(nn.Module, NativeCall):
     """model/modules/confidence_head.py:125-175."""
 
     def __init__(self, channel_s: int, channel_z: int, num_heads: int, dropout: float = 0.25, kernel_backend: str = "b200"):
@@ -33,19 +34,26 @@ class ConfidencePairSingleBlock(nn.Module):
         self.attention = SelfAttentionPairBias(channel_s, num_heads, None, "confidence")
         self.transition = Transition(channel_s, expansion_factor=4)
         self._proj = _ProjectionCache()
-        self._plan = None
+
+    def _stands_for(self) -> StandsFor:
+        pair = (TriangularBlock, {"tri_mul_out": TriangleMultiplicationOutgoing, "tri_mul_in": TriangleMultiplicationIncoming,
+                                  "transition_z": Transition})
+        return StandsFor((self.pair_block, pair), (self.attention, SelfAttentionPairBias), (self.transition, Transition))
+
+    def _make_plan(self, device, dtype, precise: bool) -> _PairBlockPlan:
+        pb = self.pair_block
+        return _PairBlockPlan(self, device, dtype, precise, pb.tri_mul_out, pb.tri_mul_in, pb.transition_z, None,
+                              (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
 
     @torch.compiler.disable
     def forward(self, z: torch.Tensor, s: torch.Tensor, pair_mask: torch.Tensor, mask: torch.Tensor):
         _check_inference(z)
         cd = compute_dtype(z)
         precise = _is_precise(cd, "ConfidencePairSingleBlock")
-        if cd == compute_dtype(s) and z.dim() == 4 and F.takes_any_n(z.shape[1], precise):      # one native call
-            if self._plan is None or not self._plan.fits(z.device, cd, precise):
-                pb = self.pair_block
-                self._plan = _PairBlockPlan(self, z.device, cd, precise, pb.tri_mul_out, pb.tri_mul_in, pb.transition_z, None,
-                                            (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
-            return F.pair_block(z, pair_mask, handed_out(self._plan), s, mask, precise)
+        one_call = cd == compute_dtype(s) and z.dim() == 4 and F.takes_any_n(z.shape[1], precise)
+        plan = self._plan_for(z.device, cd, precise) if one_call else None
+        if plan is not None:      # one native call
+            return F.pair_block(z, pair_mask, plan, s, mask, precise)
         z = self.pair_block(z, pair_mask)
         ln = self.layernorm_z
         with torch.autocast(z.device.type, enabled=False):

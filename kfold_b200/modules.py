@@ -27,7 +27,7 @@ from torch import nn
 from . import functional as F
 from . import _lib as L
 from . import packing
-from .plans import ParamState, handed_out
+from .plans import NativeCall, ParamState, StandsFor, handed_out
 
 __all__ = [
     "LayerNorm", "LinearNoBias", "Linear",
@@ -567,7 +567,12 @@ class CachedGlobalTransformerBlock(nn.Module):
         return self.transition(a, s, residual=True, cond=None if cond is None else cond[1])
 
 
-class CachedGlobalTransformerStack(nn.Module):
+# the submodules that the native stack calls stand for (plans.StandsFor)
+_COND_TRANSITION = (ConditionedTransitionBlock, {"adaln": AdaLN})
+_TOKEN_BLOCK = (CachedGlobalTransformerBlock, {"attention": (SelfAttentionPairBias, {"adaln_a": AdaLN}), "transition": _COND_TRANSITION})
+
+
+class CachedGlobalTransformerStack(nn.Module, NativeCall):
     """model/layers/folding/diffusion_transformer.py:260-339.  pair_bias (*, Nblock, H, L, L), as produced by
     DiffusionStack.get_pair_bias; it is converted to bf16 once per tensor and reused across sampler steps."""
 
@@ -580,7 +585,6 @@ class CachedGlobalTransformerStack(nn.Module):
         self._bias_cache = None
         self._bias_key = None
         self._bias_src = None
-        self._plan = None
 
     def _prepared_bias(self, pair_bias: torch.Tensor, precise: bool = False):
         """(*, N, H, L, L) with the N blocks in front, in the compute dtype, rows at a pitch of a multiple of eight elements
@@ -599,16 +603,17 @@ class CachedGlobalTransformerStack(nn.Module):
             self._bias_src = pair_bias
         return handed_out(self._bias_cache)
 
-    def _plan_for(self, device, precise: bool) -> "_StackPlan":
-        if self._plan is None or not self._plan.fits(device, precise):
-            blocks = []
-            for b in self.blocks:
-                pa, pt = b.attention._apb_packed(device, precise), b.transition._packed_transition(device, precise)
-                blocks.append({"w_proj": pa["w_proj"], "proj_bias": pa["proj_bias"], "w_out": pa["w_out"], "out_bias": pa["out_bias"],
-                               "w_swiglu": pt["w_swiglu"], "w_tout": pt["w_out"]})
-            self._plan = _StackPlan(self, blocks, L.TokenBlock, [m for b in self.blocks for m in (b.attention.adaln_a, b.transition.adaln)],
-                                    [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)], device, precise)
-        return handed_out(self._plan)
+    def _stands_for(self) -> StandsFor:
+        return StandsFor(*[(b, _TOKEN_BLOCK) for b in self.blocks])
+
+    def _make_plan(self, device, precise: bool) -> "_StackPlan":
+        blocks = []
+        for b in self.blocks:
+            pa, pt = b.attention._apb_packed(device, precise), b.transition._packed_transition(device, precise)
+            blocks.append({"w_proj": pa["w_proj"], "proj_bias": pa["proj_bias"], "w_out": pa["w_out"], "out_bias": pa["out_bias"],
+                           "w_swiglu": pt["w_swiglu"], "w_tout": pt["w_out"]})
+        return _StackPlan(self, blocks, L.TokenBlock, [m for b in self.blocks for m in (b.attention.adaln_a, b.transition.adaln)],
+                          [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)], device, precise)
 
     def reset_caches(self) -> None:
         """Forget the converted pair bias (call once per complex when the bias tensor is overwritten in place under
@@ -626,10 +631,11 @@ class CachedGlobalTransformerStack(nn.Module):
         s_lead = tuple(s.shape[:-2])
         s_samples = 1 if samples == 1 or _leading(s_lead) == groups else samples
         with torch.autocast(a.device.type, enabled=False):
-            if groups and _leading(s_lead) == groups * s_samples and self.blocks[0].attention.use_single_conditioning:
-                return F.token_stack(a, s, pb, mask, self._plan_for(a.device, precise), groups, samples, s_samples,
-                                     self.blocks[0].attention.num_heads, self.blocks[0].transition.hidden, precise)
-        # biases, masks or conditionings shared in some other pattern: one block at a time
+            plan = self._plan_for(a.device, precise) if groups and _leading(s_lead) == groups * s_samples else None
+            if plan is not None:
+                return F.token_stack(a, s, pb, mask, plan, groups, samples, s_samples, self.blocks[0].attention.num_heads,
+                                     self.blocks[0].transition.hidden, precise)
+        # biases, masks or conditionings shared in some other pattern, submodules that have to be called: one block at a time
         for i, blk in enumerate(self.blocks):
             a = blk(a, s, pb[i], mask)
         return a
@@ -842,7 +848,11 @@ class LocalTransformerBlock(nn.Module):
         return out.view(shape)
 
 
-class LocalTransformerStack(nn.Module):
+_ATOM_BLOCK = (LocalTransformerBlock, {"attention": (CrossAttentionPairBias, {"adaln_a_q": AdaLN, "adaln_a_k": AdaLN}),
+                                       "transition": _COND_TRANSITION})
+
+
+class LocalTransformerStack(nn.Module, NativeCall):
     """model/layers/folding/diffusion_transformer.py:419-512.  The whole stack works on the un-windowed atoms: the
     prologues, the projections, the output gate and the transition are row-wise, and under bfloat16 compute (head dim
     <= 32) the attention kernel walks the windows itself; the float32 path gathers the key side into windows.  The pair
@@ -861,7 +871,6 @@ class LocalTransformerStack(nn.Module):
         self._bias_all = None
         self._bias_all_key = None
         self._bias_all_src = None
-        self._plan = None
         self._bank = _ConditioningBank()
 
     def _stacked_bias_weights(self, device, dt):
@@ -887,17 +896,18 @@ class LocalTransformerStack(nn.Module):
             self._bias_all_src = z          # keeps z's storage alive so that its address cannot be reused
         return handed_out(self._bias_all)
 
-    def _plan_for(self, device) -> _StackPlan:
-        if self._plan is None or not self._plan.fits(device, False):
-            blocks = []
-            for b in self.blocks:
-                pa, pt = b.attention._cross_packed(device), b.transition._packed_transition(device, False)
-                blocks.append({"w_q": pa["w_q"], "q_bias": pa["q_bias"], "w_kv": pa["w_kv"], "w_out": pa["w_out"], "out_bias": pa["out_bias"],
-                               "w_swiglu": pt["w_swiglu"], "w_tout": pt["w_out"]})
-            self._plan = _StackPlan(self, blocks, L.AtomBlock,
-                                    [m for b in self.blocks for m in (b.attention.adaln_a_q, b.attention.adaln_a_k, b.transition.adaln)],
-                                    [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)], device, False)
-        return handed_out(self._plan)
+    def _stands_for(self) -> StandsFor:
+        return StandsFor(*[(b, _ATOM_BLOCK) for b in self.blocks])
+
+    def _make_plan(self, device, precise: bool) -> _StackPlan:
+        blocks = []
+        for b in self.blocks:
+            pa, pt = b.attention._cross_packed(device, precise), b.transition._packed_transition(device, precise)
+            blocks.append({"w_q": pa["w_q"], "q_bias": pa["q_bias"], "w_kv": pa["w_kv"], "w_out": pa["w_out"], "out_bias": pa["out_bias"],
+                           "w_swiglu": pt["w_swiglu"], "w_tout": pt["w_out"]})
+        return _StackPlan(self, blocks, L.AtomBlock,
+                          [m for b in self.blocks for m in (b.attention.adaln_a_q, b.attention.adaln_a_k, b.transition.adaln)],
+                          [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)], device, precise)
 
     def reset_caches(self) -> None:
         """Forget the window biases (see CachedGlobalTransformerStack.reset_caches)."""
@@ -930,11 +940,11 @@ class LocalTransformerStack(nn.Module):
                 mask2 = mask.to(torch.bool).reshape(-1, length)
                 # conditioning shared by the samples, window biases and mask shared inside each group: one native call
                 groups = _leading(tuple(s.shape[:-2]))
-                if (self.blocks[0].attention.use_single_conditioning and batch % groups == 0
-                        and _index_share(lead, tuple(s.shape[:-2])) == batch // groups
+                if (batch % groups == 0 and _index_share(lead, tuple(s.shape[:-2])) == batch // groups
                         and (batch // groups) % bias_share == 0 and (batch // groups) % (batch // mask2.shape[0]) == 0):
-                    return F.atom_stack(a, s, bias_all, mask2, self._plan_for(a.device), groups, bias_share, h,
-                                        self.blocks[0].transition.hidden)
+                    plan = self._plan_for(a.device, False)
+                    if plan is not None:
+                        return F.atom_stack(a, s, bias_all, mask2, plan, groups, bias_share, h, self.blocks[0].transition.hidden)
                 bias_all = bias_all.reshape(len(self.blocks), h, -1, WINDOW_Q, WINDOW_K)
             else:
                 to_qk = build_atom_to_qk_fn(length, a.device)
@@ -1218,7 +1228,7 @@ class _PairBlockPlan:
         return self.key == (device, dtype, precise) and self.state.current()
 
 
-class TriangularBlock(nn.Module):
+class TriangularBlock(nn.Module, NativeCall):
     """K-Fold trunk block: tri-mult out, tri-mult in, transition, residual adds fused into the kernels."""
 
     def __init__(self, channel_z: int = 256, dropout: float = 0.25, kernel_backend: str = "b200"):
@@ -1227,23 +1237,28 @@ class TriangularBlock(nn.Module):
         self.tri_mul_out = TriangleMultiplicationOutgoing(channel_z)
         self.tri_mul_in = TriangleMultiplicationIncoming(channel_z)
         self.transition_z = Transition(channel_z, expansion_factor=4)
-        self._plan = None
+
+    def _stands_for(self) -> StandsFor:
+        return StandsFor((self.tri_mul_out, TriangleMultiplicationOutgoing), (self.tri_mul_in, TriangleMultiplicationIncoming),
+                         (self.transition_z, Transition))
+
+    def _make_plan(self, device, dtype, precise: bool) -> _PairBlockPlan:
+        return _PairBlockPlan(self, device, dtype, precise, self.tri_mul_out, self.tri_mul_in, self.transition_z)
 
     @torch.compiler.disable
     def forward(self, z: torch.Tensor, pair_mask: torch.Tensor) -> torch.Tensor:
         _check_inference(z)
         cd = compute_dtype(z)
         precise = _is_precise(cd, "TriangularBlock")
-        if z.dim() == 4 and F.takes_any_n(z.shape[1], precise):      # one native call
-            if self._plan is None or not self._plan.fits(z.device, cd, precise):
-                self._plan = _PairBlockPlan(self, z.device, cd, precise, self.tri_mul_out, self.tri_mul_in, self.transition_z)
-            return F.pair_block(z, pair_mask, handed_out(self._plan), precise=precise)
+        plan = self._plan_for(z.device, cd, precise) if z.dim() == 4 and F.takes_any_n(z.shape[1], precise) else None
+        if plan is not None:      # one native call
+            return F.pair_block(z, pair_mask, plan, precise=precise)
         z = self.tri_mul_out(z, pair_mask, residual=True)
         z = self.tri_mul_in(z, pair_mask, residual=True)
         return self.transition_z(z, residual=True)
 
 
-class PairformerBlock(nn.Module):
+class PairformerBlock(nn.Module, NativeCall):
     """AF3-shaped Pairformer block assembled from the reference's modules: the pair track in the order of
     ``PairformerBlock.forward`` (tri-mult out/in, tri-att start/end, transition x4) and the single track of
     ``ConfidencePairSingleBlock.forward`` (pair bias from LN(z), single attention with pair bias, transition x4)."""
@@ -1263,7 +1278,16 @@ class PairformerBlock(nn.Module):
         self.transition = Transition(channel_s, expansion_factor=4)
         self._bias_w = None
         self._bias_key = None
-        self._plan = None
+
+    def _stands_for(self) -> StandsFor:
+        return StandsFor((self.tri_mul_out, TriangleMultiplicationOutgoing), (self.tri_mul_in, TriangleMultiplicationIncoming),
+                         (self.tri_att_start, TriangleAttentionStartingNode), (self.tri_att_end, TriangleAttentionEndingNode),
+                         (self.transition_z, Transition), (self.attention, SelfAttentionPairBias), (self.transition, Transition))
+
+    def _make_plan(self, device, dtype, precise: bool) -> _PairBlockPlan:
+        return _PairBlockPlan(self, device, dtype, precise, self.tri_mul_out, self.tri_mul_in, self.transition_z,
+                              (self.tri_att_start, self.tri_att_end),
+                              (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
 
     def _pair_bias(self, z: torch.Tensor) -> torch.Tensor:
         p = self.linear_pair_bias.weight
@@ -1289,12 +1313,10 @@ class PairformerBlock(nn.Module):
         _check_inference(z)
         cd = compute_dtype(z)
         precise = _is_precise(cd, "PairformerBlock")
-        if cd == compute_dtype(s) and z.dim() == 4 and F.takes_any_n(z.shape[1], precise):      # one native call
-            if self._plan is None or not self._plan.fits(z.device, cd, precise):
-                self._plan = _PairBlockPlan(self, z.device, cd, precise, self.tri_mul_out, self.tri_mul_in, self.transition_z,
-                                            (self.tri_att_start, self.tri_att_end),
-                                            (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
-            return F.pair_block(z, pair_mask, handed_out(self._plan), s, mask, precise)
+        one_call = cd == compute_dtype(s) and z.dim() == 4 and F.takes_any_n(z.shape[1], precise)
+        plan = self._plan_for(z.device, cd, precise) if one_call else None
+        if plan is not None:      # one native call
+            return F.pair_block(z, pair_mask, plan, s, mask, precise)
         z = self.tri_mul_out(z, pair_mask, residual=True)
         z = self.tri_mul_in(z, pair_mask, residual=True)
         z = self.tri_att_start(z, pair_mask, residual=True)

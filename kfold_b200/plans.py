@@ -11,8 +11,9 @@ import threading
 from itertools import chain
 
 import torch
+from torch.nn.modules import module as _nn_module
 
-__all__ = ["ParamState", "handed_out", "HandedOut"]
+__all__ = ["ParamState", "StandsFor", "NativeCall", "handed_out", "HandedOut"]
 
 _recording = threading.local()
 
@@ -57,6 +58,60 @@ class HandedOut:
             else:
                 todo += getattr(t, "keep", ())
         return list(out.values())
+
+
+class StandsFor:
+    """The submodules whose `forward` a native call of the whole block or stack stands for.
+
+    The native call reads their weights and never calls them.  That is the same thing only while they are what the framework
+    made them: of exactly that class, without a `forward` of their own and without forward hooks, which would not fire.
+    Given as `module, class` or `module, (class, {child: ...})` pairs, children being looked at below a plain module only."""
+
+    __slots__ = ("_submodules", "_classes")
+
+    def __init__(self, *pairs):
+        self._submodules, self._classes, todo = [], [], list(pairs)
+        while todo:
+            m, cls = todo.pop()
+            children = {}
+            if isinstance(cls, tuple):
+                cls, children = cls
+            self._submodules.append(m)
+            self._classes.append(cls)
+            if type(m) is cls:
+                todo += [(m._modules.get(name), sub) for name, sub in children.items()]
+
+    def plain(self) -> bool:
+        """Whether every submodule is of the expected class itself."""
+        return list(map(type, self._submodules)) == self._classes and not any(["forward" in m.__dict__ for m in self._submodules])
+
+    def holds(self) -> bool:
+        """Whether the native call may be made: plain submodules, and nobody listens to them."""
+        if _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks or list(map(type, self._submodules)) != self._classes:
+            return False
+        for d in map(vars, self._submodules):
+            if d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d:
+                return False
+        return True
+
+
+class NativeCall:
+    """Mixin of a block or stack that runs as one native call: `_plan_for(*key)` gives the plan of that call, or None where the
+    submodules have to be called one by one.  The class provides `_stands_for()` and `_make_plan(*key)`; a plan has
+    `fits(*key)`."""
+
+    _plan = None
+
+    def _plan_for(self, *key):
+        plan = self._plan
+        if plan is None or not plan.fits(*key):
+            stands = self._stands_for()
+            if not stands.holds():
+                self._plan = None
+                return None
+            plan = self._plan = self._make_plan(*key)
+            plan.stands = stands      # the submodules are still these for as long as the plan fits
+        return handed_out(plan) if plan.stands.holds() else None
 
 
 def _version(p):

@@ -192,3 +192,46 @@ def test_ln_linear_fp32_rows(dev, rows, k, bf16):
     ref = (torch.nn.functional.layer_norm(x.double(), (k,), lw.double(), lb.double(), 1e-5) @ w.double().T).float()
     mx, r = err_stats(out, ref)
     assert mx < PRECISE_MAX_TOL and r < PRECISE_RMS_TOL, f"{mx:.3e} {r:.3e}"
+
+
+def _hooked_cases(dev):
+    """(module, its call, a submodule that the module calls)"""
+    from kfold_b200 import modules as M
+    from kfold_b200.confidence import ConfidencePairSingleBlock
+    g = torch.Generator(device=dev).manual_seed(11)
+    rnd = lambda *shape, dt=torch.bfloat16: torch.randn(shape, generator=g, device=dev, dtype=dt)
+    n = 41
+    z, s = rnd(1, n, n, 128), rnd(1, n, 384)
+    m = torch.ones(1, n, dtype=torch.bool, device=dev)
+    pm = torch.ones(1, n, n, dtype=torch.bool, device=dev)
+    a, c, bias = rnd(1, 2, n, 256, dt=torch.float32), rnd(1, 1, n, 384, dt=torch.float32), rnd(1, 1, 2, 8, n, n)
+    q, qc, p = rnd(1, 2, 64, 128, dt=torch.float32), rnd(1, 1, 64, 128, dt=torch.float32), rnd(1, 1, 2, 32, 128, 16, dt=torch.float32)
+    am = torch.ones(1, 1, 64, dtype=torch.bool, device=dev)
+    with torch.device(dev):
+        tri, blk, conf = M.TriangularBlock(128), M.PairformerBlock(128, 384), ConfidencePairSingleBlock(384, 128, 16)
+        tok, atm = M.CachedGlobalTransformerStack(256, 384, 8, 2), M.LocalTransformerStack(128, 128, 16, 4, 2)
+    return {"triangular": (tri, lambda: tri(z, pm), tri.tri_mul_in), "pairformer": (blk, lambda: blk(z, s, pm, m), blk.attention),
+            "confidence": (conf, lambda: conf(z, s, pm, m), conf.pair_block.transition_z),
+            "token": (tok, lambda: tok(a, c, bias, m.unsqueeze(1)), tok.blocks[1].transition),
+            "atom": (atm, lambda: atm(q, qc, p, am), atm.blocks[0].transition)}
+
+
+@pytest.mark.parametrize("which", ["triangular", "pairformer", "confidence", "token", "atom"])
+def test_hooks_of_submodules_fire(dev, which):
+    """A forward hook on a submodule sees that submodule's output, and what it returns is used; the submodules called one by one
+    give what the native call gives, to the rounding of the bf16 results that lie between them."""
+    mod, call, sub = _hooked_cases(dev)[which]
+    flat = lambda o: torch.cat([t.float().reshape(-1) for t in (o if isinstance(o, tuple) else (o,))])
+    with torch.autocast("cuda", dtype=torch.bfloat16):
+        one = flat(call())
+        seen = []
+        handle = sub.register_forward_hook(lambda m, args, out: seen.append(out.shape))
+        hooked = flat(call())
+        assert len(seen) == 1
+        handle.remove()
+        handle = sub.register_forward_hook(lambda m, args, out: out * 0)
+        changed = flat(call())
+        handle.remove()
+        again = flat(call())
+    _check(*err_stats(hooked, one), f"{which}: one by one against one call")
+    assert torch.equal(again, one) and not torch.allclose(changed, one, rtol=0.1, atol=0.1)

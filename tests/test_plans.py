@@ -44,3 +44,57 @@ def test_every_change_of_the_weights_is_noticed(change):
     change(m)
     assert not state.current()
     assert ParamState(m).current()
+
+
+# ------------------------------------------------------------------------------------------------ when the one native call is made
+DEV = torch.device("cpu")
+
+
+def _owners():
+    from kfold_b200.confidence import ConfidencePairSingleBlock
+    pair = (DEV, torch.bfloat16, False)
+    return {
+        "TriangularBlock": (M.TriangularBlock(64), pair, ["tri_mul_out", "tri_mul_in", "transition_z"]),
+        "PairformerBlock": (M.PairformerBlock(64, 64, 2, 2), pair,
+                            ["tri_mul_out", "tri_att_start", "tri_att_end", "transition_z", "attention", "transition"]),
+        "ConfidencePairSingleBlock": (ConfidencePairSingleBlock(64, 64, 2), pair,
+                                      ["pair_block", "pair_block.tri_mul_in", "pair_block.transition_z", "attention", "transition"]),
+        "CachedGlobalTransformerStack": (M.CachedGlobalTransformerStack(64, 32, 2, 2), (DEV, False),
+                                         ["blocks.1", "blocks.0.attention", "blocks.1.transition", "blocks.1.attention.adaln_a"]),
+        "LocalTransformerStack": (M.LocalTransformerStack(64, 64, 16, 2, 2), (DEV, False), ["blocks.0.transition", "blocks.1.attention"]),
+    }
+
+
+PATHS = [(name, path) for name, (_, _, paths) in _owners().items() for path in paths]
+
+
+@pytest.mark.parametrize("name,path", PATHS)
+def test_submodules_that_are_hooked_or_replaced_are_called(name, path):
+    """The native call of a block or stack is made only while its submodules are what it stands for."""
+    owner, key, _ = _owners()[name]
+    sub = owner.get_submodule(path)
+    parent, _, leaf = path.rpartition(".")
+    parent = owner.get_submodule(parent)
+    with torch.no_grad():
+        plan = owner._plan_for(*key)
+        assert plan is not None and owner._plan_for(*key) is plan
+        for register in (sub.register_forward_hook, sub.register_forward_pre_hook):
+            handle = register(lambda *a: None)
+            assert owner._plan_for(*key) is None
+            handle.remove()
+            assert owner._plan_for(*key) is plan
+        everywhere = nn.modules.module.register_module_forward_hook(lambda *a: None)
+        assert owner._plan_for(*key) is None
+        everywhere.remove()
+        sub.forward = lambda *a, **k: a[0]
+        assert owner._plan_for(*key) is None
+        del sub.forward
+        assert owner._plan_for(*key) is plan
+        patched = type("Patched", (type(sub),), {"forward": lambda self, x, *a, **k: x})
+        subclassed = patched.__new__(patched)
+        subclassed.__dict__.update(sub.__dict__)      # the same parameters under another forward
+        for new in (subclassed, nn.Identity()):
+            setattr(parent, leaf, new)
+            assert owner._plan_for(*key) is None
+        setattr(parent, leaf, sub)
+        assert owner._plan_for(*key) is not None
