@@ -38,12 +38,16 @@ class ConfidencePairSingleBlock(nn.Module, NativeCall):
     def _stands_for(self) -> StandsFor:
         pair = (TriangularBlock, {"tri_mul_out": TriangleMultiplicationOutgoing, "tri_mul_in": TriangleMultiplicationIncoming,
                                   "transition_z": Transition})
-        return StandsFor((self.pair_block, pair), (self.attention, SelfAttentionPairBias), (self.transition, Transition))
+        return StandsFor((self.pair_block, pair), (self.attention, SelfAttentionPairBias), (self.transition, Transition),
+                         norms=lambda: _PairBlockPlan.norms(*self._parts()))
+
+    def _parts(self) -> tuple:
+        pb = self.pair_block
+        return (pb.tri_mul_out, pb.tri_mul_in, pb.transition_z, (),
+                (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
 
     def _make_plan(self, device, dtype, precise: bool) -> _PairBlockPlan:
-        pb = self.pair_block
-        return _PairBlockPlan(self, device, dtype, precise, pb.tri_mul_out, pb.tri_mul_in, pb.transition_z, None,
-                              (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
+        return _PairBlockPlan(self, device, dtype, precise, *self._parts())
 
     @torch.compiler.disable
     def forward(self, z: torch.Tensor, s: torch.Tensor, pair_mask: torch.Tensor, mask: torch.Tensor):

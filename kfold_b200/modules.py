@@ -346,8 +346,10 @@ class _StackPlan:
         self.keep += [w_gs, b_gs, w_og, b_og]
         self.c_s = adalns[0].channel_s
         self.gs_cols, self.og_cols = w_gs.shape[0], w_og.shape[0]
-        self.cond = L.Conditioning(L.ptr(w_gs), L.ptr(b_gs), L.ptr(w_og), L.ptr(b_og), self.gs_cols, self.og_cols, self.c_s,
-                                   adalns[0].layernorm_s.eps)
+        self.cond = L.Conditioning(L.ptr(w_gs), L.ptr(b_gs), L.ptr(w_og), L.ptr(b_og), self.gs_cols, self.og_cols, self.c_s)
+
+    def set_eps(self, eps: float) -> None:
+        self.cond.eps = eps
 
     def fits(self, device, precise: bool) -> bool:
         return self.key == (device, precise) and self.state.current()
@@ -604,7 +606,13 @@ class CachedGlobalTransformerStack(nn.Module, NativeCall):
         return handed_out(self._bias_cache)
 
     def _stands_for(self) -> StandsFor:
-        return StandsFor(*[(b, _TOKEN_BLOCK) for b in self.blocks])
+        return StandsFor(*[(b, _TOKEN_BLOCK) for b in self.blocks], norms=lambda: [m.layernorm_s for m in self._adalns()])
+
+    def _adalns(self) -> list:
+        return [m for b in self.blocks for m in (b.attention.adaln_a, b.transition.adaln)]
+
+    def _gates(self) -> list:
+        return [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)]
 
     def _make_plan(self, device, precise: bool) -> "_StackPlan":
         blocks = []
@@ -612,8 +620,7 @@ class CachedGlobalTransformerStack(nn.Module, NativeCall):
             pa, pt = b.attention._apb_packed(device, precise), b.transition._packed_transition(device, precise)
             blocks.append({"w_proj": pa["w_proj"], "proj_bias": pa["proj_bias"], "w_out": pa["w_out"], "out_bias": pa["out_bias"],
                            "w_swiglu": pt["w_swiglu"], "w_tout": pt["w_out"]})
-        return _StackPlan(self, blocks, L.TokenBlock, [m for b in self.blocks for m in (b.attention.adaln_a, b.transition.adaln)],
-                          [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)], device, precise)
+        return _StackPlan(self, blocks, L.TokenBlock, self._adalns(), self._gates(), device, precise)
 
     def reset_caches(self) -> None:
         """Forget the converted pair bias (call once per complex when the bias tensor is overwritten in place under
@@ -897,7 +904,13 @@ class LocalTransformerStack(nn.Module, NativeCall):
         return handed_out(self._bias_all)
 
     def _stands_for(self) -> StandsFor:
-        return StandsFor(*[(b, _ATOM_BLOCK) for b in self.blocks])
+        return StandsFor(*[(b, _ATOM_BLOCK) for b in self.blocks], norms=lambda: [m.layernorm_s for m in self._adalns()])
+
+    def _adalns(self) -> list:
+        return [m for b in self.blocks for m in (b.attention.adaln_a_q, b.attention.adaln_a_k, b.transition.adaln)]
+
+    def _gates(self) -> list:
+        return [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)]
 
     def _make_plan(self, device, precise: bool) -> _StackPlan:
         blocks = []
@@ -905,9 +918,7 @@ class LocalTransformerStack(nn.Module, NativeCall):
             pa, pt = b.attention._cross_packed(device, precise), b.transition._packed_transition(device, precise)
             blocks.append({"w_q": pa["w_q"], "q_bias": pa["q_bias"], "w_kv": pa["w_kv"], "w_out": pa["w_out"], "out_bias": pa["out_bias"],
                            "w_swiglu": pt["w_swiglu"], "w_tout": pt["w_out"]})
-        return _StackPlan(self, blocks, L.AtomBlock,
-                          [m for b in self.blocks for m in (b.attention.adaln_a_q, b.attention.adaln_a_k, b.transition.adaln)],
-                          [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)], device, precise)
+        return _StackPlan(self, blocks, L.AtomBlock, self._adalns(), self._gates(), device, precise)
 
     def reset_caches(self) -> None:
         """Forget the window biases (see CachedGlobalTransformerStack.reset_caches)."""
@@ -957,11 +968,10 @@ class LocalTransformerStack(nn.Module, NativeCall):
                 bias_all = bias_all.reshape(len(self.blocks), h, -1, WINDOW_Q, WINDOW_K)
                 batch = mask_k.shape[0]
             conds = [None] * len(self.blocks)
-            if not precise and all(b.attention.use_single_conditioning for b in self.blocks):
+            if (not precise and all(b.attention.use_single_conditioning for b in self.blocks)
+                    and len({m.layernorm_s.eps for m in self._adalns()}) == 1):
                 # the conditioning projections of all blocks: one LayerNorm of s and two GEMMs
-                gs, og = self._bank.tables(
-                    s, [m for b in self.blocks for m in (b.attention.adaln_a_q, b.attention.adaln_a_k, b.transition.adaln)],
-                    [g for b in self.blocks for g in (b.attention.linear_ada_out, b.transition.linear_g)])
+                gs, og = self._bank.tables(s, self._adalns(), self._gates())
                 conds = [((gs[3 * i], gs[3 * i + 1], og[2 * i]), (gs[3 * i + 2], og[2 * i + 1])) for i in range(len(self.blocks))]
             for i, blk in enumerate(self.blocks):
                 att = blk.attention
@@ -1185,8 +1195,8 @@ class DiffusionStack(nn.Module):
 class _PairBlockPlan:
     """The packed weights of a block of the pair stacks as the struct kfb_pair_block_fwd takes; `state` tells when they are stale."""
 
-    def __init__(self, root: nn.Module, device, dtype, precise: bool, mul_out, mul_in, trans_z, attention=None, single=None):
-        """`attention`: (starting, ending) or None; `single`: (layernorm_z, linear_pair_bias, attention, transition) or None."""
+    def __init__(self, root: nn.Module, device, dtype, precise: bool, mul_out, mul_in, trans_z, attention=(), single=None):
+        """`attention`: (starting, ending) or (); `single`: (layernorm_z, linear_pair_bias, attention, transition) or None."""
         self.key, self.state = (device, dtype, precise), ParamState(root)
         self.keep = []
 
@@ -1200,8 +1210,8 @@ class _PairBlockPlan:
         for dst, mod in ((k.mul_out, mul_out), (k.mul_in, mul_in)):
             pk = mod._packed(device, dtype, lambda sd, dev: packing.pack_trimul(sd, dev, precise=precise))
             put(dst, pk, **{n: n for n in ("ln_in_w", "ln_in_b", "w_in", "w_gout", "ln_out_w", "ln_out_b", "w_pout")})
-        k.c, k.eps = pk["c"], mul_out.layernorm_in.eps
-        for dst, mod in zip((k.att_start, k.att_end), attention or ()):
+        k.c = pk["c"]
+        for dst, mod in zip((k.att_start, k.att_end), attention):
             pk = mod._packed(device, dtype, lambda sd, dev: packing.pack_triatt(sd, mod.no_heads, dev, precise=precise))
             put(dst, pk, ln_w="ln_w", ln_b="ln_b", w_proj="w_proj", w_out="w_out")
             k.has_attention, k.tri_heads = 1, mod.no_heads
@@ -1224,6 +1234,18 @@ class _PairBlockPlan:
             k.hidden_s = transition(k.trans_s, trans_s)
         self.ref = L.ref(k)
 
+    def set_eps(self, eps: float) -> None:
+        self.struct.eps = eps
+
+    @staticmethod
+    def norms(mul_out, mul_in, trans_z, attention=(), single=None) -> list:
+        """The LayerNorms of such a block, arguments as above."""
+        out = [mul_out.layernorm_in, mul_in.layernorm_in, trans_z.layernorm] + [a.layer_norm for a in attention]
+        if single is not None:
+            ln_z, _, att, trans_s = single
+            out += [ln_z, att.layernorm_a, trans_s.layernorm]
+        return out
+
     def fits(self, device, dtype, precise: bool) -> bool:
         return self.key == (device, dtype, precise) and self.state.current()
 
@@ -1240,10 +1262,13 @@ class TriangularBlock(nn.Module, NativeCall):
 
     def _stands_for(self) -> StandsFor:
         return StandsFor((self.tri_mul_out, TriangleMultiplicationOutgoing), (self.tri_mul_in, TriangleMultiplicationIncoming),
-                         (self.transition_z, Transition))
+                         (self.transition_z, Transition), norms=lambda: _PairBlockPlan.norms(*self._parts()))
+
+    def _parts(self) -> tuple:
+        return self.tri_mul_out, self.tri_mul_in, self.transition_z
 
     def _make_plan(self, device, dtype, precise: bool) -> _PairBlockPlan:
-        return _PairBlockPlan(self, device, dtype, precise, self.tri_mul_out, self.tri_mul_in, self.transition_z)
+        return _PairBlockPlan(self, device, dtype, precise, *self._parts())
 
     @torch.compiler.disable
     def forward(self, z: torch.Tensor, pair_mask: torch.Tensor) -> torch.Tensor:
@@ -1282,12 +1307,15 @@ class PairformerBlock(nn.Module, NativeCall):
     def _stands_for(self) -> StandsFor:
         return StandsFor((self.tri_mul_out, TriangleMultiplicationOutgoing), (self.tri_mul_in, TriangleMultiplicationIncoming),
                          (self.tri_att_start, TriangleAttentionStartingNode), (self.tri_att_end, TriangleAttentionEndingNode),
-                         (self.transition_z, Transition), (self.attention, SelfAttentionPairBias), (self.transition, Transition))
+                         (self.transition_z, Transition), (self.attention, SelfAttentionPairBias), (self.transition, Transition),
+                         norms=lambda: _PairBlockPlan.norms(*self._parts()))
+
+    def _parts(self) -> tuple:
+        return (self.tri_mul_out, self.tri_mul_in, self.transition_z, (self.tri_att_start, self.tri_att_end),
+                (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
 
     def _make_plan(self, device, dtype, precise: bool) -> _PairBlockPlan:
-        return _PairBlockPlan(self, device, dtype, precise, self.tri_mul_out, self.tri_mul_in, self.transition_z,
-                              (self.tri_att_start, self.tri_att_end),
-                              (self.layernorm_z, self.linear_pair_bias, self.attention, self.transition))
+        return _PairBlockPlan(self, device, dtype, precise, *self._parts())
 
     def _pair_bias(self, z: torch.Tensor) -> torch.Tensor:
         p = self.linear_pair_bias.weight

@@ -65,11 +65,12 @@ class StandsFor:
 
     The native call reads their weights and never calls them.  That is the same thing only while they are what the framework
     made them: of exactly that class, without a `forward` of their own and without forward hooks, which would not fire.
-    Given as `module, class` or `module, (class, {child: ...})` pairs, children being looked at below a plain module only."""
+    Given as `module, class` or `module, (class, {child: ...})` pairs, children being looked at below a plain module only.
+    `norms()`, asked when all are plain, lists the LayerNorms for which the call has one epsilon: they have to agree on it."""
 
-    __slots__ = ("_submodules", "_classes")
+    __slots__ = ("_submodules", "_classes", "_norms")
 
-    def __init__(self, *pairs):
+    def __init__(self, *pairs, norms):
         self._submodules, self._classes, todo = [], [], list(pairs)
         while todo:
             m, cls = todo.pop()
@@ -80,25 +81,31 @@ class StandsFor:
             self._classes.append(cls)
             if type(m) is cls:
                 todo += [(m._modules.get(name), sub) for name, sub in children.items()]
+        self._norms = norms() if self.plain() else []
 
     def plain(self) -> bool:
         """Whether every submodule is of the expected class itself."""
         return list(map(type, self._submodules)) == self._classes and not any(["forward" in m.__dict__ for m in self._submodules])
 
+    def eps(self):
+        """The epsilon of the LayerNorms, None where they differ."""
+        seen = {n.eps for n in self._norms}
+        return seen.pop() if len(seen) == 1 else None
+
     def holds(self) -> bool:
-        """Whether the native call may be made: plain submodules, and nobody listens to them."""
+        """Whether the native call may be made: plain submodules, nobody listens to them, one epsilon."""
         if _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks or list(map(type, self._submodules)) != self._classes:
             return False
         for d in map(vars, self._submodules):
             if d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d:
                 return False
-        return True
+        return self.eps() is not None
 
 
 class NativeCall:
     """Mixin of a block or stack that runs as one native call: `_plan_for(*key)` gives the plan of that call, or None where the
     submodules have to be called one by one.  The class provides `_stands_for()` and `_make_plan(*key)`; a plan has
-    `fits(*key)`."""
+    `fits(*key)` and `set_eps(eps)`, for an epsilon is no parameter and may be changed between calls."""
 
     _plan = None
 
@@ -111,7 +118,10 @@ class NativeCall:
                 return None
             plan = self._plan = self._make_plan(*key)
             plan.stands = stands      # the submodules are still these for as long as the plan fits
-        return handed_out(plan) if plan.stands.holds() else None
+        elif not plan.stands.holds():
+            return None
+        plan.set_eps(plan.stands.eps())
+        return handed_out(plan)
 
 
 def _version(p):

@@ -98,3 +98,30 @@ def test_submodules_that_are_hooked_or_replaced_are_called(name, path):
             assert owner._plan_for(*key) is None
         setattr(parent, leaf, sub)
         assert owner._plan_for(*key) is not None
+
+
+NORMS = {"TriangularBlock": ["tri_mul_out.layernorm_in", "tri_mul_in.layernorm_in", "transition_z.layernorm"],
+         "PairformerBlock": ["tri_mul_out.layernorm_in", "tri_mul_in.layernorm_in", "tri_att_start.layer_norm", "tri_att_end.layer_norm",
+                             "transition_z.layernorm", "layernorm_z", "attention.layernorm_a", "transition.layernorm"],
+         "ConfidencePairSingleBlock": ["pair_block.tri_mul_out.layernorm_in", "pair_block.tri_mul_in.layernorm_in",
+                                       "pair_block.transition_z.layernorm", "layernorm_z", "attention.layernorm_a", "transition.layernorm"],
+         "CachedGlobalTransformerStack": [f"blocks.{i}.{m}.layernorm_s" for i in range(2) for m in ("attention.adaln_a", "transition.adaln")],
+         "LocalTransformerStack": [f"blocks.{i}.{m}.layernorm_s" for i in range(2)
+                                   for m in ("attention.adaln_a_q", "attention.adaln_a_k", "transition.adaln")]}
+
+
+@pytest.mark.parametrize("name", sorted(NORMS))
+def test_one_epsilon_per_native_call(name):
+    """A native call has one epsilon for all its LayerNorms: it is made where they agree, with the value they have at the time."""
+    owner, key, _ = _owners()[name]
+    eps = lambda plan: (plan.struct if hasattr(plan, "struct") else plan.cond).eps
+    with torch.no_grad():
+        assert eps(owner._plan_for(*key)) == pytest.approx(1e-5)
+        for path in NORMS[name]:
+            norm = owner.get_submodule(path)
+            norm.eps = 1e-3
+            assert owner._plan_for(*key) is None, f"{path}: another epsilon than the others'"
+            norm.eps = 1e-5
+        for path in NORMS[name]:
+            owner.get_submodule(path).eps = 1e-3
+        assert eps(owner._plan_for(*key)) == pytest.approx(1e-3)
