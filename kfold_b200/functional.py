@@ -228,6 +228,8 @@ def adaln(a: torch.Tensor, gate_shift: torch.Tensor, samples: int, eps: float = 
     _require_cuda(a, gate_shift)
     c, l = a.shape[-1], a.shape[-2]
     a2 = a.reshape(-1, c).contiguous()
+    if gate_shift.shape[-1] != 2 * c or gate_shift.numel() // (2 * c) * samples != a2.shape[0]:
+        raise ValueError(f"adaln: gate / shift {tuple(gate_shift.shape)} for rows {tuple(a.shape)} of which {samples} entries share")
     precise = gate_shift.dtype == torch.float32     # float32 gate / shift rows: everything stays float32
     if precise:
         a2 = a2.float()
@@ -247,6 +249,9 @@ def conditioned_transition(x_normed: torch.Tensor, packed: dict, out_gate: torch
     c, hidden, l = packed["c"], packed["hidden"], x_normed.shape[-2]
     x2 = x_normed.reshape(-1, c).contiguous()
     rows = x2.shape[0]
+    if x_normed.shape[-1] != c or out_gate.shape[-1] != c or out_gate.numel() // c * samples != rows:
+        raise ValueError(f"conditioned_transition: gate {tuple(out_gate.shape)} for rows {tuple(x_normed.shape)} of which {samples} "
+                         "entries share")
     precise = bool(packed.get("precise"))
     want = out_dtype or (resid.dtype if resid is not None else x_normed.dtype)
     out = torch.empty(rows, c, dtype=torch.float32 if precise else want, device=x2.device)
@@ -311,6 +316,8 @@ def attention_pair_bias(x: torch.Tensor, pair_bias: torch.Tensor, mask: torch.Te
         mb = torch.nn.functional.pad(mb, (0, lp - l))
     gate, gate_ld = None, 0
     if out_gate is not None:
+        if out_gate.shape[-1] != c or out_gate.numel() // c * gate_share != batch * l:
+            raise ValueError(f"attention_pair_bias: gate {tuple(out_gate.shape)} for rows {tuple(x.shape)} of which {gate_share} entries share")
         if lp != l:
             gate = torch.nn.functional.pad(out_gate.reshape(-1, l, c).to(act), (0, 0, 0, lp - l)).contiguous()
         else:

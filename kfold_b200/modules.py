@@ -264,17 +264,21 @@ class AdaLN(nn.Module, _PackedMixin):
         _check_inference(a)
         precise = _is_precise(compute_dtype(a), "AdaLN")
         with torch.autocast(a.device.type, enabled=False):
-            samples = _sample_share(a, s)
+            s, samples = _shared_conditioning(a, s)
             return F.adaln(a, self.gate_shift(s, precise), samples)
 
 
-def _sample_share(a: torch.Tensor, s: torch.Tensor) -> int:
-    """How many consecutive samples of `a` share one conditioning row of `s` (its sample dim is 1 or equal)."""
-    if a.dim() < 3 or s.dim() != a.dim():
-        return 1
-    if s.shape[-3] == 1 and a.shape[-3] != 1:
-        return int(a.shape[-3])
-    return 1
+def _shared_conditioning(a: torch.Tensor, s: torch.Tensor):
+    """(s, share): `share` consecutive entries of `a` (*, L, c_a), leading dims flattened, use one entry of `s` (*, L, c_s), whose
+    leading dims may be 1 or missing where a's are not.  Dims of size one other than the trailing ones are expanded."""
+    if s.shape[-2] == a.shape[-2] and s.numel() // s.shape[-1] == a.numel() // a.shape[-1]:      # row for row
+        return s, 1
+    if s.shape[-2] == 1 and a.shape[-2] != 1:
+        s = s.expand(*s.shape[:-2], a.shape[-2], s.shape[-1])
+    if s.shape[-2] != a.shape[-2] or s.dim() > a.dim():
+        raise ValueError(f"conditioning {tuple(s.shape)} does not match activations {tuple(a.shape)}")
+    share = F._index_sharing(tuple(a.shape[:-2]), tuple(s.shape[:-2]))
+    return (s.expand(*a.shape[:-1], s.shape[-1]), 1) if share is None else (s, share)
 
 
 class _ConditioningBank:
@@ -409,13 +413,13 @@ class SelfAttentionPairBias(nn.Module, _PackedMixin):
         pk = self._apb_packed(a.device, precise)
         with torch.autocast(a.device.type, enabled=False):
             if cond is not None and not precise and self.use_single_conditioning:
-                share = _sample_share(a, s)
+                s, share = _shared_conditioning(a, s)
                 an = F.adaln(a, cond[0], share)
                 return F.attention_pair_bias(an, pair_bias, mask, pk, out_dtype=a.dtype, out_gate=cond[1], gate_share=share,
                                              resid=a if residual else None)
             if precise and self.use_single_conditioning:
                 assert s is not None
-                share = _sample_share(a, s)
+                s, share = _shared_conditioning(a, s)
                 an = F.adaln(a.float(), self.adaln_a.gate_shift(s, True), share)
                 w6, b_ada = self._ada_out(a.device, True)
                 gate = F.linear_fp32(s.float(), w6, b_ada)
@@ -427,7 +431,7 @@ class SelfAttentionPairBias(nn.Module, _PackedMixin):
                 return F.attention_pair_bias(an, pair_bias, mask, pk, out_dtype=a.dtype, resid=a if residual else None)
             if self.use_single_conditioning:
                 assert s is not None
-                share = _sample_share(a, s)
+                s, share = _shared_conditioning(a, s)
                 an = F.adaln(a, self.adaln_a.gate_shift(s), share)
                 w_ada, b_ada = self._ada_out(a.device)
                 gate = F.linear(s, w_ada, b_ada)
@@ -464,7 +468,7 @@ class ConditionedTransitionBlock(nn.Module, _PackedMixin):
             precise = _is_precise(compute_dtype(a), "ConditionedTransitionBlock")
         pk = self._packed_transition(a.device, precise)
         with torch.autocast(a.device.type, enabled=False):
-            share = _sample_share(a, s)
+            s, share = _shared_conditioning(a, s)
             if precise:
                 an = F.adaln(a.float(), self.adaln.gate_shift(s, True), share)
                 gate = F.linear_fp32(s.float(), pk["w_g"], pk["b_g"])
@@ -635,10 +639,10 @@ class CachedGlobalTransformerStack(nn.Module, NativeCall):
         lead = tuple(a.shape[:-2])
         # (groups, samples): the samples share bias, mask and usually the conditioning
         groups, samples = _group_samples(lead, tuple(pb.shape[1:-3]), tuple(mask.shape[:-1]))
-        s_lead = tuple(s.shape[:-2])
-        s_samples = 1 if samples == 1 or _leading(s_lead) == groups else samples
+        s, share = _shared_conditioning(a, s)
+        s_samples = samples // share if share in (1, samples) else 0       # conditioning entries of a group
         with torch.autocast(a.device.type, enabled=False):
-            plan = self._plan_for(a.device, precise) if groups and _leading(s_lead) == groups * s_samples else None
+            plan = self._plan_for(a.device, precise) if groups and s_samples else None
             if plan is not None:
                 return F.token_stack(a, s, pb, mask, plan, groups, samples, s_samples, self.blocks[0].attention.num_heads,
                                      self.blocks[0].transition.hidden, precise)
@@ -780,7 +784,7 @@ class CrossAttentionPairBias(nn.Module, _PackedMixin):
         gate/shift rows, key gate/shift rows, output gate logits) from a stack's conditioning tables."""
         if self.use_single_conditioning:
             assert s is not None
-            share = _sample_share(a, s)
+            s, share = _shared_conditioning(a, s)
             if cond is not None and not precise:
                 return F.adaln(a, cond[0], share), F.adaln(a, cond[1], share), cond[2]
             af = a.float() if precise else a
@@ -809,10 +813,11 @@ class CrossAttentionPairBias(nn.Module, _PackedMixin):
             flat = lambda t: None if t is None else t.flatten(-3, -2)
             if self.use_single_conditioning:
                 assert s_q is not None and s_k is not None
-                aqf, akf, sqf, skf = flat(a_q), flat(a_k), flat(s_q), flat(s_k)
+                aqf, akf = flat(a_q), flat(a_k)
+                (sqf, share_q), (skf, share_k) = _shared_conditioning(aqf, flat(s_q)), _shared_conditioning(akf, flat(s_k))
                 cast = (lambda t: t.float()) if precise else (lambda t: t)
-                xq = F.adaln(cast(aqf), self.adaln_a_q.gate_shift(sqf, precise), _sample_share(aqf, sqf)).view(a_q.shape)
-                xk = F.adaln(cast(akf), self.adaln_a_k.gate_shift(skf, precise), _sample_share(akf, skf)).view(a_k.shape)
+                xq = F.adaln(cast(aqf), self.adaln_a_q.gate_shift(sqf, precise), share_q).view(a_q.shape)
+                xk = F.adaln(cast(akf), self.adaln_a_k.gate_shift(skf, precise), share_k).view(a_k.shape)
             else:
                 assert s_q is None and s_k is None
                 dt = torch.float32 if precise else torch.bfloat16
@@ -937,6 +942,7 @@ class LocalTransformerStack(nn.Module, NativeCall):
             raise ValueError("Length must be divisible by 32")
         windows = length // WINDOW_Q
         h = self.num_heads
+        s, _ = _shared_conditioning(a, s)
         with torch.autocast(a.device.type, enabled=False):
             bias_all = self._window_biases(z, dt)                                        # (blocks*H, *z_lead, W, 32, 128)
             z_lead = tuple(z.shape[:-3])                                                 # includes the window dim
