@@ -591,16 +591,18 @@ class CachedGlobalTransformerStack(nn.Module, NativeCall):
         self._bias_cache = None
         self._bias_key = None
         self._bias_src = None
+        self._bank = _ConditioningBank()
 
-    def _prepared_bias(self, pair_bias: torch.Tensor, precise: bool = False):
-        """(*, N, H, L, L) with the N blocks in front, in the compute dtype, rows at a pitch of a multiple of eight elements
-        (what the attention kernel's tensor maps take).  A bias that already lies so is used in place."""
-        key = _tensor_key(pair_bias) + (pair_bias.stride(), precise)
+    def _prepared_bias(self, pair_bias: torch.Tensor, precise: bool = False, per_block: bool = False):
+        """(*, N, H, L, L) with the N blocks in front, in the compute dtype.  For the stack's call the rows lie at a pitch of a
+        multiple of eight elements (what the attention kernel's tensor maps take); `per_block`, for blocks called one by one, each
+        block's bias is contiguous.  A bias that already lies so is used in place."""
+        key = _tensor_key(pair_bias) + (pair_bias.stride(), precise, per_block)
         if self._bias_key != key:
             pb, dt = pair_bias.movedim(-4, 0), torch.float32 if precise else torch.bfloat16
             l = pb.shape[-1]
-            if pb.dtype != dt or not _bias_in_place(pb):
-                padded = pb.new_zeros(*pb.shape[:-1], (l + 7) // 8 * 8, dtype=dt)
+            if pb.dtype != dt or not (pb[0].is_contiguous() if per_block else _bias_in_place(pb)):
+                padded = pb.new_zeros(*pb.shape[:-1], l if per_block else (l + 7) // 8 * 8, dtype=dt)
                 padded[..., :l] = pb
                 pb = padded[..., :l]
             self._bias_cache, self._bias_key = pb, key
@@ -635,20 +637,26 @@ class CachedGlobalTransformerStack(nn.Module, NativeCall):
     def forward(self, a: torch.Tensor, s: torch.Tensor, pair_bias: torch.Tensor, mask: torch.Tensor) -> torch.Tensor:
         _check_inference(a)
         precise = _is_precise(compute_dtype(a), "CachedGlobalTransformerStack")
-        pb = self._prepared_bias(pair_bias, precise)
         lead = tuple(a.shape[:-2])
         # (groups, samples): the samples share bias, mask and usually the conditioning
-        groups, samples = _group_samples(lead, tuple(pb.shape[1:-3]), tuple(mask.shape[:-1]))
+        groups, samples = _group_samples(lead, tuple(pair_bias.shape[:-4]), tuple(mask.shape[:-1]))
         s, share = _shared_conditioning(a, s)
         s_samples = samples // share if share in (1, samples) else 0       # conditioning entries of a group
+        conds = [()] * len(self.blocks)
         with torch.autocast(a.device.type, enabled=False):
             plan = self._plan_for(a.device, precise) if groups and s_samples else None
             if plan is not None:
-                return F.token_stack(a, s, pb, mask, plan, groups, samples, s_samples, self.blocks[0].attention.num_heads,
-                                     self.blocks[0].transition.hidden, precise)
-        # biases, masks or conditionings shared in some other pattern, submodules that have to be called: one block at a time
+                return F.token_stack(a, s, self._prepared_bias(pair_bias, precise), mask, plan, groups, samples, s_samples,
+                                     self.blocks[0].attention.num_heads, self.blocks[0].transition.hidden, precise)
+            # biases, masks or conditionings shared in some other pattern, or submodules that have to be called: one block at a
+            # time, under bfloat16 compute with the conditioning projections of all blocks from one LayerNorm of s and two GEMMs
+            stands = self._stands_for()
+            if not precise and stands.plain() and stands.eps() is not None:
+                gs, og = self._bank.tables(s, self._adalns(), self._gates())
+                conds = [(((gs[2 * i], og[2 * i]), (gs[2 * i + 1], og[2 * i + 1])),) for i in range(len(self.blocks))]
+            pb = self._prepared_bias(pair_bias, precise, per_block=True)
         for i, blk in enumerate(self.blocks):
-            a = blk(a, s, pb[i], mask)
+            a = blk(a, s, pb[i], mask, *conds[i])
         return a
 
 

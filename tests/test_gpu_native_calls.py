@@ -235,3 +235,46 @@ def test_hooks_of_submodules_fire(dev, which):
         again = flat(call())
     _check(*err_stats(hooked, one), f"{which}: one by one against one call")
     assert torch.equal(again, one) and not torch.allclose(changed, one, rtol=0.1, atol=0.1)
+
+
+def _token_weights(rng, blocks, c):
+    import synth
+    w = {}
+    for i in range(blocks):
+        w.update(synth._prefixed(f"blocks.{i}.attention", synth.apb_weights(rng, c, 384)))
+        w.update(synth._prefixed(f"blocks.{i}.transition", synth.conditioned_transition_weights(rng, c, 384)))
+    return w
+
+
+@pytest.mark.parametrize("l", [33, 40])
+@pytest.mark.parametrize("pattern", ["mask per sample", "conditioning of all complexes"])
+def test_token_stack_other_sharing_patterns(dev, l, pattern):
+    """What the one native call does not take runs block by block: against the oracle, with the bias given at a wider pitch than
+    its own, and with no more launches a block than its own seven (the conditioning is projected once for all blocks)."""
+    from kfold_b200 import _lib as L
+    from kfold_b200 import modules as M
+    import synth
+    groups, samples, c, heads = 2, 2, 256, 8
+    rng = synth._Rng(l)
+    a, bias = rng.normal(groups, samples, l, c), rng.normal(groups, 1, 3, heads, l, l)
+    s = rng.normal(groups, 1, l, 384) if pattern == "mask per sample" else rng.normal(1, 1, l, 384)
+    mask = synth.token_mask(l, valid=l - 4).view(1, 1, l).repeat(groups, samples if pattern == "mask per sample" else 1, 1)
+    if pattern == "mask per sample":
+        mask[1, 1, : l // 2] = False
+    pitched = torch.zeros(groups, 1, 3, heads, l, (l + 15) // 16 * 16 + 8)
+    pitched[..., :l] = bias
+    pitched = pitched.to(dev)[..., :l]
+    launches = []
+    for blocks in (2, 3):
+        w = _token_weights(synth._Rng(7), blocks, c)
+        stack = M.CachedGlobalTransformerStack(c, 384, heads, blocks).to(dev)
+        stack.load_state_dict(w, strict=True)
+        args = (a.to(dev), s.to(dev), pitched[:, :, :blocks], mask.to(dev))
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            stack(*args)
+            before = L.launch_count()
+            out = stack(*args)
+            launches.append(L.launch_count() - before)
+        ref = _oracle_on(dev, O.global_transformer_stack, a, s.expand(groups, 1, l, 384), bias[:, :, :blocks], mask, w, heads, blocks)
+        _compare(out.float().cpu(), ref, False, f"token stack L={l}, {pattern}")
+    assert launches[1] - launches[0] <= 7, launches

@@ -125,3 +125,14 @@ def test_one_epsilon_per_native_call(name):
         for path in NORMS[name]:
             owner.get_submodule(path).eps = 1e-3
         assert eps(owner._plan_for(*key)) == pytest.approx(1e-3)
+
+
+@pytest.mark.parametrize("l,pitch", [(16, 16), (16, 24), (20, 24), (20, 20)])
+def test_a_bias_for_blocks_called_one_by_one_is_converted_once(l, pitch):
+    """Each block's bias is contiguous, so that no block copies it again, and it is kept for the next call."""
+    stack = M.CachedGlobalTransformerStack(64, 32, 2, 3)
+    bias = torch.randn(2, 1, 3, 2, l, pitch)[..., :l]
+    pb = stack._prepared_bias(bias, per_block=True)
+    assert all(pb[i].is_contiguous() for i in range(3)) and stack._prepared_bias(bias, per_block=True) is pb
+    assert torch.equal(pb.float(), bias.movedim(-4, 0).bfloat16().float())
+    assert stack._prepared_bias(bias).stride(-2) % 8 == 0      # the stack's own form
