@@ -340,6 +340,7 @@ class _StackPlan:
 
     def __init__(self, root: nn.Module, blocks: list, block_type, adalns: list, gates: list, device, precise: bool):
         self.key, self.state = (device, precise), ParamState(root)
+        self.heads, self.hidden = root.blocks[0].attention.num_heads, root.blocks[0].transition.hidden
         self.keep = []                               # the packed tensors behind the pointers
         self.blocks = (block_type * len(blocks))()
         for dst, fields in zip(self.blocks, blocks):
@@ -643,13 +644,13 @@ class CachedGlobalTransformerStack(nn.Module, NativeCall):
         s, share = _shared_conditioning(a, s)
         s_samples = samples // share if share in (1, samples) else 0       # conditioning entries of a group
         conds = [()] * len(self.blocks)
+        plan = self._plan_for(a.device, precise) if groups and s_samples else None
+        if plan is not None:
+            return F.token_stack(a, s, self._prepared_bias(pair_bias, precise), mask, plan, groups, samples, s_samples, plan.heads,
+                                 plan.hidden, precise)
+        # biases, masks or conditionings shared in some other pattern, or submodules that have to be called: one block at a time,
+        # under bfloat16 compute with the conditioning projections of all blocks from one LayerNorm of s and two GEMMs
         with torch.autocast(a.device.type, enabled=False):
-            plan = self._plan_for(a.device, precise) if groups and s_samples else None
-            if plan is not None:
-                return F.token_stack(a, s, self._prepared_bias(pair_bias, precise), mask, plan, groups, samples, s_samples,
-                                     self.blocks[0].attention.num_heads, self.blocks[0].transition.hidden, precise)
-            # biases, masks or conditionings shared in some other pattern, or submodules that have to be called: one block at a
-            # time, under bfloat16 compute with the conditioning projections of all blocks from one LayerNorm of s and two GEMMs
             stands = self._stands_for()
             if not precise and stands.plain() and stands.eps() is not None:
                 gs, og = self._bank.tables(s, self._adalns(), self._gates())
@@ -969,7 +970,7 @@ class LocalTransformerStack(nn.Module, NativeCall):
                         and (batch // groups) % bias_share == 0 and (batch // groups) % (batch // mask2.shape[0]) == 0):
                     plan = self._plan_for(a.device, False)
                     if plan is not None:
-                        return F.atom_stack(a, s, bias_all, mask2, plan, groups, bias_share, h, self.blocks[0].transition.hidden)
+                        return F.atom_stack(a, s, bias_all, mask2, plan, groups, bias_share, h, plan.hidden)
                 bias_all = bias_all.reshape(len(self.blocks), h, -1, WINDOW_Q, WINDOW_K)
             else:
                 to_qk = build_atom_to_qk_fn(length, a.device)

@@ -68,10 +68,10 @@ class StandsFor:
     Given as `module, class` or `module, (class, {child: ...})` pairs, children being looked at below a plain module only.
     `norms()`, asked when all are plain, lists the LayerNorms for which the call has one epsilon: they have to agree on it."""
 
-    __slots__ = ("_submodules", "_classes", "_norms")
+    __slots__ = ("_submodules", "_classes", "_called", "_norms")
 
     def __init__(self, *pairs, norms):
-        self._submodules, self._classes, todo = [], [], list(pairs)
+        self._submodules, self._classes, self._called, todo = [], [], [], list(pairs)
         while todo:
             m, cls = todo.pop()
             children = {}
@@ -80,26 +80,26 @@ class StandsFor:
             self._submodules.append(m)
             self._classes.append(cls)
             if type(m) is cls:
+                self._called.append(m.__dict__)
                 todo += [(m._modules.get(name), sub) for name, sub in children.items()]
         self._norms = norms() if self.plain() else []
 
     def plain(self) -> bool:
         """Whether every submodule is of the expected class itself."""
-        return list(map(type, self._submodules)) == self._classes and not any(["forward" in m.__dict__ for m in self._submodules])
+        return list(map(type, self._submodules)) == self._classes and not any(["forward" in d for d in self._called])
 
     def eps(self):
         """The epsilon of the LayerNorms, None where they differ."""
         seen = {n.eps for n in self._norms}
         return seen.pop() if len(seen) == 1 else None
 
-    def holds(self) -> bool:
-        """Whether the native call may be made: plain submodules, nobody listens to them, one epsilon."""
+    def holds(self):
+        """The epsilon of the native call if it may be made -- plain submodules, nobody listens to them, one epsilon -- else None."""
         if _nn_module._global_forward_hooks or _nn_module._global_forward_pre_hooks or list(map(type, self._submodules)) != self._classes:
-            return False
-        for d in map(vars, self._submodules):
-            if d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d:
-                return False
-        return self.eps() is not None
+            return None
+        if any([d["_forward_hooks"] or d["_forward_pre_hooks"] or "forward" in d for d in self._called]):
+            return None
+        return self.eps()
 
 
 class NativeCall:
@@ -113,14 +113,15 @@ class NativeCall:
         plan = self._plan
         if plan is None or not plan.fits(*key):
             stands = self._stands_for()
-            if not stands.holds():
-                self._plan = None
-                return None
-            plan = self._plan = self._make_plan(*key)
-            plan.stands = stands      # the submodules are still these for as long as the plan fits
-        elif not plan.stands.holds():
+            eps = stands.holds()
+            plan = self._plan = None if eps is None else self._make_plan(*key)
+            if plan is not None:
+                plan.stands = stands      # the submodules are still these for as long as the plan fits
+        else:
+            eps = plan.stands.holds()
+        if eps is None:
             return None
-        plan.set_eps(plan.stands.eps())
+        plan.set_eps(eps)
         return handed_out(plan)
 
 
@@ -131,8 +132,7 @@ def _version(p):
         return None
 
 
-def _values(dicts):
-    return chain.from_iterable(map(dict.values, dicts))
+_data_ptr = torch.Tensor.data_ptr
 
 
 class ParamState:
@@ -141,18 +141,19 @@ class ParamState:
     __slots__ = ("_parameters", "_modules", "_empty", "_children", "_seen")
 
     def __init__(self, *modules):
-        # the dictionaries themselves: a parameter or a submodule that is added where there was none shows in them too
+        # views of the modules' own dictionaries: a parameter or a submodule that is added where there was none shows in them too
         dicts = [(m._parameters, m._modules) for root in modules for m in root.modules()]
-        self._parameters, self._modules = [p for p, _ in dicts if p], [c for _, c in dicts if c]
+        self._parameters, self._modules = [p.values() for p, _ in dicts if p], [c.values() for _, c in dicts if c]
         self._empty = [d for pair in dicts for d in pair if not d]
-        self._children, self._seen = list(_values(self._modules)), self._read()
+        self._children, self._seen = list(chain.from_iterable(self._modules)), self._read()
 
     def _read(self):
+        ps = [p for p in chain.from_iterable(self._parameters) if p is not None]
         try:
-            return [(p.data_ptr(), p._version) for p in _values(self._parameters) if p is not None]
+            return list(map(_data_ptr, ps)), [p._version for p in ps]
         except RuntimeError:
-            return [(p.data_ptr(), _version(p)) for p in _values(self._parameters) if p is not None]
+            return list(map(_data_ptr, ps)), [_version(p) for p in ps]
 
     def current(self) -> bool:
         """Whether nothing changed since."""
-        return not any(self._empty) and list(_values(self._modules)) == self._children and self._read() == self._seen
+        return self._read() == self._seen and not any(self._empty) and list(chain.from_iterable(self._modules)) == self._children
