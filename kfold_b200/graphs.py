@@ -8,6 +8,7 @@ every temporary of the Python layer comes from torch's caching allocator, which 
 """
 from __future__ import annotations
 
+import gc
 import threading
 
 import torch
@@ -26,6 +27,21 @@ def _capture_stream(device: torch.device) -> torch.cuda.Stream:
     if index not in streams:
         streams[index] = torch.cuda.Stream(index)
     return streams[index]
+
+
+def _capture(fn, inputs):
+    graph = torch.cuda.CUDAGraph()
+    graph.capture_begin()
+    try:
+        output = fn(*inputs)
+    except BaseException:
+        try:
+            graph.capture_end()
+        except RuntimeError:      # the capture had become invalid: the error that made it so is the one to report
+            pass
+        raise
+    graph.capture_end()
+    return graph, output
 
 
 class GraphedCall:
@@ -57,20 +73,23 @@ class GraphedCall:
         with torch.cuda.device(dev), torch.no_grad():
             # Warm-up and capture on one side stream.  torch.cuda.graph() would collect Python garbage and return the
             # allocator's cached blocks to the driver first; with a model of a few hundred parameters in memory that is
-            # 0.1 s and more, and every later allocation pays for it again, so the capture is begun and ended directly.
+            # 0.1 s and more, and every later allocation pays for it again, so the capture is begun and ended directly, and
+            # only one that finds no memory is tried again after that.
             current, side = torch.cuda.current_stream(), _capture_stream(dev)
             side.wait_stream(current)
             with torch.cuda.stream(side):          # warm-up outside the capture: weight packing, workspace allocation
                 for _ in range(max(warmup, 1)):
                     fn(*self._inputs)
                 side.synchronize()
-                self._graph = torch.cuda.CUDAGraph()
-                self._graph.capture_begin()
-                try:
-                    with HandedOut() as used:
-                        self._output = fn(*self._inputs)
-                finally:
-                    self._graph.capture_end()
+                with HandedOut() as used:
+                    try:
+                        self._graph, self._output = _capture(fn, self._inputs)
+                    except torch.OutOfMemoryError:
+                        # the allocator returns no cached block to the driver while a capture is under way: what the calls
+                        # before have left in its cache may be the memory that is missing
+                        gc.collect()
+                        torch.cuda.empty_cache()
+                        self._graph, self._output = _capture(fn, self._inputs)
             current.wait_stream(side)
         self._kept, self._streams = used.tensors(), set()
         F.withdraw_workspaces(self._kept)

@@ -132,6 +132,49 @@ def test_modules_record_what_they_hand_out():
     assert prepared.data_ptr() in kept and w.data_ptr() in kept and pk["w_proj"].data_ptr() in kept
 
 
+def test_a_capture_without_memory_is_tried_again(fake_cuda, monkeypatch):
+    """An allocation that fails under capture: the failed capture is ended, the cache emptied outside of it, the call captured
+    once more; a second failure, and any other error, is the caller's."""
+    from kfold_b200.graphs import GraphedCall
+    events = []
+
+    class Graph:
+        def __init__(self):
+            self.n = sum(e[0] == "begin" for e in events)
+
+        def capture_begin(self):
+            events.append(("begin", self.n))
+
+        def capture_end(self):
+            events.append(("end", self.n))
+            if self.n == bad_end:
+                raise RuntimeError("capture invalidated")
+
+    monkeypatch.setattr(torch.cuda, "CUDAGraph", Graph)
+    monkeypatch.setattr(torch.cuda, "empty_cache", lambda: events.append(("empty",)))
+
+    def failing(times, error):
+        def fn(x):
+            if events and events[-1][0] == "begin" and sum(e[0] == "begin" for e in events) <= times:
+                raise error
+            return x
+        return fn
+
+    for bad_end in (None, 0):
+        events.clear()
+        g = GraphedCall(failing(1, torch.OutOfMemoryError("no memory")), _Input())
+        assert events == [("begin", 0), ("end", 0), ("empty",), ("begin", 1), ("end", 1)] and g._graph.n == 1
+    bad_end = None
+    events.clear()
+    with pytest.raises(torch.OutOfMemoryError):
+        GraphedCall(failing(2, torch.OutOfMemoryError("no memory")), _Input())
+    assert events[-1] == ("end", 1)
+    events.clear()
+    with pytest.raises(ValueError):
+        GraphedCall(failing(1, ValueError("the call's own")), _Input())
+    assert events == [("begin", 0), ("end", 0)]
+
+
 # ------------------------------------------------------------------------------------------------ replays, on a GPU
 def _token_call(dev, l, seed):
     from kfold_b200 import modules as M
@@ -203,4 +246,32 @@ def test_one_network_two_complexes_both_graphs_live():
             out = graphed(a, s)
             assert torch.equal(out, ref), err_stats(out, ref)
         del junk
+    assert L.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_a_capture_beside_a_full_cache():
+    """A capture that needs the memory which the allocator has cached, under a limit that the allocator itself enforces."""
+    from kfold_b200 import _lib as L
+    from kfold_b200.graphs import GraphedCall
+    dev = torch.device("cuda:0")
+    big = 1 << 30
+    gc.collect()
+    torch.cuda.empty_cache()
+    total = torch.cuda.get_device_properties(dev).total_memory
+    x = torch.randn(1 << 20, device=dev)
+
+    def fn(t):
+        scratch = torch.empty(big, dtype=torch.uint8, device=dev)      # freed to the capture stream's cache by the warm-up
+        del scratch
+        return t * 2
+
+    with torch.no_grad():
+        try:
+            torch.cuda.set_per_process_memory_fraction((torch.cuda.memory_reserved(dev) + 1.5 * big) / total, dev)
+            graphed = GraphedCall(fn, x)
+        finally:
+            torch.cuda.set_per_process_memory_fraction(1.0, dev)
+        assert torch.equal(graphed(x), x * 2)
+        torch.cuda.synchronize()
     assert L.device_status() == 0
