@@ -169,6 +169,8 @@ def linear(x: torch.Tensor, w: torch.Tensor, bias: torch.Tensor | None = None, o
     """y = x w^T (+ bias) on the tensor-core GEMM.  x (..., k) bf16, w (n, k) bf16, bias fp32 (n,) or None."""
     _require_cuda(x, w)
     k = x.shape[-1]
+    if w.shape[1] != k:
+        raise ValueError(f"linear: x {tuple(x.shape)} for a weight {tuple(w.shape)}")
     x2 = x.reshape(-1, k)
     if x2.dtype != torch.bfloat16:
         x2 = x2.to(torch.bfloat16)
@@ -378,6 +380,10 @@ def token_stack(a: torch.Tensor, s: torch.Tensor, pair_bias: torch.Tensor, mask:
     dtype with rows at a pitch of eights; mask (groups, L); `plan`: the stack's packed weights."""
     _require_cuda(a, s, pair_bias, mask)
     l, c = a.shape[-2:]
+    if (c != plan.c or s.shape[-1] != plan.c_s or a.numel() != groups * samples * l * c or s.numel() != groups * s_samples * l * plan.c_s
+            or pair_bias.shape[0] < len(plan.blocks) or pair_bias.shape[-3:] != (heads, l, l) or mask.numel() != groups * l):
+        raise ValueError(f"token_stack: a {tuple(a.shape)}, s {tuple(s.shape)}, pair bias {tuple(pair_bias.shape)}, mask {tuple(mask.shape)} "
+                         f"for {len(plan.blocks)} blocks of {heads} heads, {plan.c} and {plan.c_s} channels")
     ac = (a.float() if precise else a).contiguous()
     sc = (s.float() if precise or s.dtype not in (torch.bfloat16, torch.float32) else s).contiguous()
     mk = mask.to(torch.bool).contiguous()
@@ -402,6 +408,10 @@ def atom_stack(a: torch.Tensor, s: torch.Tensor, window_biases: torch.Tensor, ma
     _require_cuda(a, s, window_biases, mask)
     l, c = a.shape[-2:]
     batch = a.numel() // (l * c)
+    if (c != plan.c or s.shape[-1] != plan.c_s or s.numel() != groups * l * plan.c_s or mask.shape[-1] != l
+            or window_biases.shape[-2:] != (32, 128) or window_biases.numel() != len(plan.blocks) * heads * (batch // bias_share) * l * 128):
+        raise ValueError(f"atom_stack: a {tuple(a.shape)}, s {tuple(s.shape)}, window biases {tuple(window_biases.shape)}, mask "
+                         f"{tuple(mask.shape)} for {len(plan.blocks)} blocks of {heads} heads, {plan.c} and {plan.c_s} channels")
     ac = a.contiguous()
     sc = (s if s.dtype in (torch.bfloat16, torch.float32) else s.float()).contiguous()
     mk = mask.to(torch.bool).contiguous()
@@ -428,6 +438,8 @@ def window_bias(z: torch.Tensor, ln_w: torch.Tensor | None, ln_b: torch.Tensor |
     c = z.shape[-1]
     if z.dtype not in (torch.bfloat16, torch.float32) or w.dtype != z.dtype:
         raise TypeError("window_bias: z and w must both be bfloat16 or both float32")
+    if w.shape[1] != c:
+        raise ValueError(f"window_bias: z {tuple(z.shape)} for a weight {tuple(w.shape)}")
     z2 = z.reshape(-1, c).contiguous()
     nh = w.shape[0]
     out = torch.empty((nh,) + tuple(z.shape[:-1]), dtype=z.dtype, device=z.device)

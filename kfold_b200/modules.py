@@ -340,7 +340,7 @@ class _StackPlan:
 
     def __init__(self, root: nn.Module, blocks: list, block_type, adalns: list, gates: list, device, precise: bool):
         self.key, self.state = (device, precise), ParamState(root)
-        self.heads, self.hidden = root.blocks[0].attention.num_heads, root.blocks[0].transition.hidden
+        self.heads, self.hidden, self.c = root.blocks[0].attention.num_heads, root.blocks[0].transition.hidden, adalns[0].channel_a
         self.keep = []                               # the packed tensors behind the pointers
         self.blocks = (block_type * len(blocks))()
         for dst, fields in zip(self.blocks, blocks):
@@ -639,6 +639,8 @@ class CachedGlobalTransformerStack(nn.Module, NativeCall):
         _check_inference(a)
         precise = _is_precise(compute_dtype(a), "CachedGlobalTransformerStack")
         lead = tuple(a.shape[:-2])
+        if mask.shape[-1] != a.shape[-2]:
+            mask = mask.expand(*mask.shape[:-1], a.shape[-2])
         # (groups, samples): the samples share bias, mask and usually the conditioning
         groups, samples = _group_samples(lead, tuple(pair_bias.shape[:-4]), tuple(mask.shape[:-1]))
         s, share = _shared_conditioning(a, s)
@@ -950,6 +952,8 @@ class LocalTransformerStack(nn.Module, NativeCall):
         if length % WINDOW_Q != 0:
             raise ValueError("Length must be divisible by 32")
         windows = length // WINDOW_Q
+        if z.shape[-4] not in (1, windows) or z.shape[-3:-1] != (WINDOW_Q, WINDOW_K) or mask.shape[-1] != length:
+            raise ValueError(f"LocalTransformerStack: a {tuple(a.shape)}, z {tuple(z.shape)}, mask {tuple(mask.shape)}")
         h = self.num_heads
         s, _ = _shared_conditioning(a, s)
         with torch.autocast(a.device.type, enabled=False):

@@ -1,4 +1,4 @@
-"""Which conditioning row a kernel is told to read for which entry, without a GPU: a kernel has no way of knowing how many rows its
+"""What the native calls are told about their tensors.  Which conditioning row a kernel is told to read for which entry, without a GPU: a kernel has no way of knowing how many rows its
 tables have, so the host must not ask it to share fewer than there are."""
 import itertools
 
@@ -73,3 +73,59 @@ def test_token_stack_conditioning_entries(monkeypatch, no_gpu_needed, s_lead, ex
         stack(torch.zeros(2, 3, 8, 64, dtype=torch.bfloat16), torch.zeros(*s_lead, 8, CS), torch.zeros(2, 1, 1, 2, 8, 8),
               torch.ones(2, 1, 8, dtype=torch.bool))
     assert calls == [None if expected is None else (2, 3, expected, 2 * expected)]
+
+
+# ------------------------------------------------------------------------------------------------ shapes of the stacks' native calls
+def _token_args():
+    return {"a": torch.zeros(2, 3, 8, 64, dtype=torch.bfloat16), "s": torch.zeros(2, 1, 8, CS), "pair_bias": torch.zeros(2, 1, 2, 2, 8, 8),
+            "mask": torch.ones(2, 1, 8, dtype=torch.bool)}
+
+
+def _atom_args():
+    return {"a": torch.zeros(2, 3, 64, 64, dtype=torch.bfloat16), "s": torch.zeros(2, 1, 64, 64), "z": torch.zeros(2, 1, 2, 32, 128, 16),
+            "mask": torch.ones(2, 1, 64, dtype=torch.bool)}
+
+
+def _cut(t, dim, by):
+    return t.narrow(dim, 0, t.shape[dim] - by) if by > 0 else torch.cat([t, t.narrow(dim, 0, -by)], dim)
+
+
+@pytest.mark.parametrize("which,arg,dim,by", [
+    ("token", "a", -1, 8), ("token", "s", -1, 1), ("token", "s", -1, -2), ("token", "pair_bias", -1, 1), ("token", "pair_bias", -1, -4),
+    ("token", "pair_bias", -2, 2), ("token", "pair_bias", -3, 1), ("token", "pair_bias", -4, 1), ("token", "mask", -1, 1),
+    ("token", "mask", -1, -3), ("token", "s", -2, 1), ("atom", "a", -1, 8), ("atom", "s", -1, 8), ("atom", "s", -2, 4), ("atom", "z", -4, -1),
+    ("atom", "z", -2, 8), ("atom", "z", -3, 1), ("atom", "z", -1, 4), ("atom", "mask", -1, 32), ("atom", "mask", -1, -64)])
+def test_a_wrong_extent_is_refused(monkeypatch, no_gpu_needed, which, arg, dim, by):
+    """One argument shorter or longer than the others say, along one dim: the kernels address by the extents they are told."""
+    monkeypatch.setattr(M, "_check_inference", lambda x: None)
+    if which == "token":
+        stack, args = M.CachedGlobalTransformerStack(64, CS, 2, 2), _token_args()
+    else:
+        stack, args = M.LocalTransformerStack(64, 64, 16, 2, 2), _atom_args()
+        if arg != "z" or dim == -4:      # the window biases are another call's concern
+            monkeypatch.setattr(M.F, "window_bias", lambda z, lw, lb, w, eps: torch.zeros(w.shape[0], *z.shape[:-1]))
+    args[arg] = _cut(args[arg], dim, by)
+    with torch.no_grad(), torch.autocast("cpu", dtype=torch.bfloat16), pytest.raises((ValueError, RuntimeError, IndexError)):
+        stack(**args)
+
+
+@pytest.mark.parametrize("which", ["token", "atom"])
+def test_right_extents_reach_the_native_call(monkeypatch, no_gpu_needed, which):
+    monkeypatch.setattr(M, "_check_inference", lambda x: None)
+    stack, args = ((M.CachedGlobalTransformerStack(64, CS, 2, 2), _token_args()) if which == "token"
+                   else (M.LocalTransformerStack(64, 64, 16, 2, 2), _atom_args()))
+    monkeypatch.setattr(M.F, "window_bias", lambda z, lw, lb, w, eps: torch.zeros(w.shape[0], *z.shape[:-1]))
+    with torch.no_grad(), torch.autocast("cpu", dtype=torch.bfloat16):
+        with pytest.raises(AssertionError, match="the native library was called"):
+            stack(**args)
+        if which == "token":      # a mask of one value per complex is spread over its tokens
+            args["mask"] = torch.ones(2, 1, 1, dtype=torch.bool)
+            with pytest.raises(AssertionError, match="the native library was called"):
+                stack(**args)
+
+
+def test_projections_of_other_widths_are_refused(no_gpu_needed):
+    with pytest.raises(ValueError):
+        F.linear(torch.zeros(4, 16), torch.zeros(8, 24))
+    with pytest.raises(ValueError):
+        F.window_bias(torch.zeros(2, 32, 128, 16), None, None, torch.zeros(4, 8))
