@@ -54,7 +54,7 @@ class ConfidencePairSingleBlock(nn.Module, NativeCall):
         _check_inference(z)
         cd = compute_dtype(z)
         precise = _is_precise(cd, "ConfidencePairSingleBlock")
-        one_call = cd == compute_dtype(s) and z.dim() == 4 and F.takes_any_n(z.shape[1], precise)
+        one_call = cd == compute_dtype(s) and F.pair_block_takes(precise, z, pair_mask, s, mask)
         plan = self._plan_for(z.device, cd, precise) if one_call else None
         if plan is not None:      # one native call
             return F.pair_block(z, pair_mask, plan, s, mask, precise)

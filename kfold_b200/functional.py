@@ -346,6 +346,14 @@ def attention_pair_bias(x: torch.Tensor, pair_bias: torch.Tensor, mask: torch.Te
     return out[:, :l].reshape(*lead, l, c).to(want)
 
 
+def pair_block_takes(precise: bool, z: torch.Tensor, pair_mask: torch.Tensor, s: torch.Tensor | None = None,
+                     mask: torch.Tensor | None = None) -> bool:
+    """Whether the one native call of a block takes tensors of these shapes.  The operators one by one take more: a mask that
+    the complexes share, a single track with a sample dim, token counts that have to be padded; and refuse the rest."""
+    return (z.dim() == 4 and z.shape[1] == z.shape[2] and pair_mask.shape == z.shape[:-1] and takes_any_n(z.shape[1], precise)
+            and (s is None or (s.shape[:-1] == z.shape[:2] and mask.shape == z.shape[:2])))
+
+
 def pair_block(z: torch.Tensor, pair_mask: torch.Tensor, plan, s: torch.Tensor | None = None, mask: torch.Tensor | None = None,
                precise: bool = False):
     """A block of the pair stacks in one native call: z (B, N, N, c), pair_mask (B, N, N) -> z, or (z, s) with the single track

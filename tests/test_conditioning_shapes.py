@@ -129,3 +129,26 @@ def test_projections_of_other_widths_are_refused(no_gpu_needed):
         F.linear(torch.zeros(4, 16), torch.zeros(8, 24))
     with pytest.raises(ValueError):
         F.window_bias(torch.zeros(2, 32, 128, 16), None, None, torch.zeros(4, 8))
+
+
+@pytest.mark.parametrize("cls", ["PairformerBlock", "ConfidencePairSingleBlock"])
+@pytest.mark.parametrize("b,s_lead,mask_lead,one", [(2, (2,), (2,), True), (2, (2,), (1,), False), (2, (2,), (), False), (1, (1, 3), (1, 1), False)])
+def test_blocks_take_what_their_operators_take(monkeypatch, no_gpu_needed, cls, b, s_lead, mask_lead, one):
+    """A mask shared by the complexes and a single track with a sample dim go operator by operator, as they did before a block
+    was one call; their shapes are the operators' to judge."""
+    from kfold_b200 import confidence
+    n, calls = 32, []
+    for mod in (M, confidence):
+        monkeypatch.setattr(mod, "_check_inference", lambda x: None)
+    monkeypatch.setattr(M.F, "pair_block", lambda z, pm, plan, s=None, mask=None, precise=False: calls.append("block") or ((z, s) if s is not None else z))
+    monkeypatch.setattr(M.F, "pair_bias", lambda z, *a: torch.zeros(z.shape[0], 2, n, n))
+    for name in ("_TriangleMultiplication", "_TriangleAttention", "Transition"):
+        monkeypatch.setattr(getattr(M, name), "forward", lambda self, x, *a, **k: calls.append(type(self).__name__) or x)
+    monkeypatch.setattr(M.SelfAttentionPairBias, "forward", lambda self, a, s, pb, mask, residual=False: calls.append((tuple(a.shape), tuple(mask.shape))) or a)
+    blk = M.PairformerBlock(64, 64, 2, 2) if cls == "PairformerBlock" else confidence.ConfidencePairSingleBlock(64, 64, 2)
+    z, s = torch.zeros(b, n, n, 64, dtype=torch.bfloat16), torch.zeros(*s_lead, n, 64, dtype=torch.bfloat16)
+    mask = torch.ones(*mask_lead, n, dtype=torch.bool)
+    with torch.no_grad():
+        zo, so = blk(z, s, torch.ones(b, n, n, dtype=torch.bool), mask)
+    assert zo.shape == z.shape and so.shape == s.shape
+    assert (calls == ["block"]) is one and (one or (tuple(s.shape), tuple(mask.shape)) in calls)

@@ -278,3 +278,17 @@ def test_token_stack_other_sharing_patterns(dev, l, pattern):
         ref = _oracle_on(dev, O.global_transformer_stack, a, s.expand(groups, 1, l, 384), bias[:, :, :blocks], mask, w, heads, blocks)
         _compare(out.float().cpu(), ref, False, f"token stack L={l}, {pattern}")
     assert launches[1] - launches[0] <= 7, launches
+
+
+def test_a_block_with_a_mask_shared_by_its_complexes(dev):
+    """(1, N) for two complexes: operator by operator, to the rounding of the bf16 results between them what the one call gives."""
+    from kfold_b200 import modules as M
+    g = torch.Generator(device=dev).manual_seed(3)
+    n = 41
+    z, s = (torch.randn(*shape, generator=g, device=dev).bfloat16() for shape in ((2, n, n, 128), (2, n, 384)))
+    m = (torch.arange(n, device=dev) < n - 5).unsqueeze(0)
+    pm = (m[:, :, None] & m[:, None, :]).expand(2, n, n)
+    with torch.device(dev):
+        blk = M.PairformerBlock(128, 384)
+    for got, ref in zip(blk(z, s, pm, m), blk(z, s, pm, m.expand(2, n))):
+        _check(*err_stats(got.float(), ref.float()), "shared mask")
