@@ -14,9 +14,15 @@ from . import _lib as L
 from .plans import handed_out
 
 _workspaces: dict = {}
+# A stack's workspace holds the conditioning tables of all its blocks, which grow with samples x tokens x blocks (4.5 GB for 5 x
+# 2048 tokens in float32 with a conditioning per sample).  Above this size it is given back after the call.
+MOST_KEPT_BYTES = 1 << 30
 
 
-def _workspace(device: torch.device, nbytes: int) -> torch.Tensor:
+def _workspace(device: torch.device, nbytes: int, most_kept: int | None = None) -> torch.Tensor:
+    """At least `nbytes` of scratch for a call on the current stream, kept for the next call on it unless more than `most_kept`."""
+    if most_kept is not None and nbytes > most_kept:
+        return torch.empty(nbytes, dtype=torch.uint8, device=device)
     key = (device.index, L.raw_stream(device.index))
     ws = _workspaces.get(key)
     if ws is None or ws.numel() < nbytes:
@@ -401,7 +407,7 @@ def token_stack(a: torch.Tensor, s: torch.Tensor, pair_bias: torch.Tensor, mask:
     with L.on_device(a.device):
         need = lib.kfb_token_stack_workspace_bytes(groups, samples, s_samples, l, c, plan.c_s, heads, hidden, plan.gs_cols, plan.og_cols,
                                                    precise)
-        ws = _workspace(a.device, need)
+        ws = _workspace(a.device, need, MOST_KEPT_BYTES)
         L.check(lib.kfb_token_stack_fwd(plan.blocks, len(plan.blocks), L.ref(plan.cond), L.ptr(ac), L.ptr(out), L.dtype_code(ac.dtype),
                                         L.ptr(sc), L.dtype_code(sc.dtype), L.ptr(pair_bias), st[0], st[-3], st[-2], L.ptr(mk), L.ptr(ws),
                                         ws.numel(), groups, samples, s_samples, l, c, heads, hidden, eps, precise, L.stream_ptr()))
@@ -429,7 +435,7 @@ def atom_stack(a: torch.Tensor, s: torch.Tensor, window_biases: torch.Tensor, ma
     lib = L.lib()
     with L.on_device(a.device):
         need = lib.kfb_atom_stack_workspace_bytes(groups, samples, l, c, plan.c_s, heads, hidden, plan.gs_cols, plan.og_cols)
-        ws = _workspace(a.device, need)
+        ws = _workspace(a.device, need, MOST_KEPT_BYTES)
         L.check(lib.kfb_atom_stack_fwd(plan.blocks, len(plan.blocks), L.ref(plan.cond), L.ptr(ac), L.ptr(out), L.dtype_code(ac.dtype),
                                        L.ptr(sc), L.dtype_code(sc.dtype), L.ptr(window_biases), nbb, L.ptr(mk), batch // mk.shape[0],
                                        bias_share, L.ptr(ws), ws.numel(), groups, samples, l, c, heads, hidden, eps, L.stream_ptr()))

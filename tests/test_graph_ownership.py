@@ -77,6 +77,34 @@ def test_two_live_graphs_own_their_workspaces(fake_cuda):
     del b, c
 
 
+def test_a_large_stack_workspace_is_given_back(fake_cuda, monkeypatch):
+    """The workspace of a stack call above the bound lives as long as the call; a smaller one, and an operator's, is kept."""
+    from kfold_b200 import functional as F, modules as M
+    sizes = {}
+
+    class Lib:
+        kfb_token_stack_workspace_bytes = kfb_atom_stack_workspace_bytes = lambda self, *a: sizes["need"]
+        kfb_token_stack_fwd = kfb_atom_stack_fwd = lambda self, *a: 0
+
+    monkeypatch.setattr(F.L, "lib", lambda: Lib())
+    monkeypatch.setattr(F.L, "stream_ptr", lambda: 7)
+    monkeypatch.setattr(F, "_require_cuda", lambda *t: None)
+    monkeypatch.setattr(M, "_check_inference", lambda x: None)
+    monkeypatch.setattr(M.F, "window_bias", lambda z, lw, lb, w, eps: torch.zeros(w.shape[0], *z.shape[:-1]))
+    monkeypatch.setattr(F, "MOST_KEPT_BYTES", 1 << 20)
+    token, atom = M.CachedGlobalTransformerStack(64, 8, 2, 1), M.LocalTransformerStack(64, 64, 16, 2, 1)
+    for stack, args in ((token, (torch.zeros(1, 8, 64), torch.zeros(1, 8, 8), torch.zeros(1, 1, 2, 8, 8), torch.ones(1, 8).bool())),
+                        (atom, (torch.zeros(1, 64, 64), torch.zeros(1, 64, 64), torch.zeros(1, 2, 32, 128, 16), torch.ones(1, 64).bool()))):
+        F.release_workspaces()
+        for need, kept in ((1 << 16, True), (1 << 22, False)):
+            sizes["need"] = need
+            before = dict(F._workspaces)
+            with torch.no_grad(), torch.autocast("cpu", dtype=torch.bfloat16):
+                stack(*args)
+            assert any(ws.numel() >= need for ws in F._workspaces.values()) is kept
+            assert kept or F._workspaces == before
+
+
 def test_a_graph_holds_what_modules_replace(fake_cuda):
     """Packed weights, converted biases and plans that the captured call was handed, and what the function closes over."""
     from kfold_b200.graphs import GraphedCall
@@ -214,6 +242,26 @@ def test_graphs_of_growing_complexes_stay_valid():
         for _ in range(2):
             for graphed, a, s, ref in built:
                 assert torch.equal(graphed(a, s), ref)
+        del junk
+    assert L.device_status() == 0
+
+
+@pytest.mark.gpu
+def test_a_stack_with_a_workspace_of_its_own(monkeypatch):
+    """Eager and captured, with nothing kept for the stack: the same result to the bit, and no workspace left behind."""
+    from kfold_b200 import _lib as L, functional as F
+    from kfold_b200.graphs import GraphedCall
+    dev = torch.device("cuda:0")
+    with torch.no_grad():
+        fn, a, s = _token_call(dev, 77, 9)
+        ref = fn(a, s).clone()
+        monkeypatch.setattr(F, "MOST_KEPT_BYTES", 0)
+        F.release_workspaces()
+        assert torch.equal(fn(a, s), ref) and not F._workspaces
+        graphed = GraphedCall(fn, a, s)
+        junk = [torch.full((1 << 18,), float("nan"), device=dev) for _ in range(32)]
+        for _ in range(2):
+            assert torch.equal(graphed(a, s), ref)
         del junk
     assert L.device_status() == 0
 
