@@ -49,14 +49,6 @@ struct AttCfg {
                                     256 /*barriers*/;
 };
 
-// K-major operand without swizzle: 8 x 8 core matrices (8 rows of 16 bytes); the two K halves of a K=16
-// slice are 128 bytes apart (leading byte offset), groups of 8 rows 256 bytes apart (stride byte offset).
-__device__ __forceinline__ uint64_t make_noswizzle_desc(uint32_t smem_addr) {
-  return static_cast<uint64_t>((smem_addr & 0x3ffff) >> 4) | (static_cast<uint64_t>(128 >> 4) << 16) |
-         (static_cast<uint64_t>(256 >> 4) << 32) | (1ull << 46);
-}
-__device__ __forceinline__ uint32_t small_operand_row_offset(int r) { return (r >> 3) * 256 + (r & 7) * 16; }
-
 // Pipeline.  A CTA owns 128 queries of R pair rows ("row groups", they share the bias tile).  Keys go by in half
 // tiles of 64 (t = 0, 1, ...).  Each row group has two softmax streams of four warps: stream c owns 32 of the 64
 // key columns of every half tile and keeps its own stabiliser, row sum and output accumulator O[g][c] (in tensor
@@ -150,7 +142,7 @@ attention_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   // constant operand e0 (128 x 16, first column ones) and the zero halves of the mask-row operands
   if (warp >= 4 && warp < 8) {
     const int r = (warp - 4) * 32 + lane;
-    const uint32_t off = small_operand_row_offset(r);
+    const uint32_t off = ptx::noswizzle_row_offset(r);
     // e0: a one in column 0; window mode: a one in column r / 32, the window of query row r (four windows per block)
     const int e_col = WIN ? (r >> 5) : 0;
     *reinterpret_cast<uint4*>(s_e0 + off) = make_uint4(e_col == 0 ? 0x3F80u : (e_col == 1 ? 0x3F800000u : 0u),
@@ -299,11 +291,11 @@ attention_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       constexpr uint32_t idesc_s = ptx::make_idesc(kBQ, 64, 1);
       constexpr uint32_t idesc_o = ptx::make_idesc(kBQ, DPAD, 1);
       // operand descriptors are built once; inside the loop only their 16-byte-unit address field advances
-      const uint64_t e0_desc = make_noswizzle_desc(ptx::smem_u32(s_e0));
+      const uint64_t e0_desc = ptx::make_noswizzle_desc(ptx::smem_u32(s_e0));
       const uint64_t q_desc = ptx::make_kmajor_desc<Cfg::kSpan>(ptx::smem_u32(s_q + g * Cfg::kQBytes));
       const uint64_t k_desc0 = ptx::make_kmajor_desc<Cfg::kSpan>(ptx::smem_u32(s_k + g * kStages * Cfg::kKBytes));
       const uint64_t v_desc0 = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_v + g * kStages * Cfg::kVBytes));
-      const uint64_t m_desc0 = make_noswizzle_desc(ptx::smem_u32(s_maskrow + g * 3 * Cfg::kSmallBytes));
+      const uint64_t m_desc0 = ptx::make_noswizzle_desc(ptx::smem_u32(s_maskrow + g * 3 * Cfg::kSmallBytes));
       const uint32_t tmem_s0 = tmem_base_u + g * 192;
       const uint32_t tmem_o0 = tmem_base_u + Cfg::kTmemO + g * 2 * DPAD;
       bool ok = true;
@@ -374,7 +366,7 @@ attention_bias_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     const uint32_t tmem_o = tmem_base + Cfg::kTmemO + (g * 2 + u) * DPAD + lane_base;
     const int b_hi = b / p.mask_lo_extent, b_lo = b - b_hi * p.mask_lo_extent;
     const unsigned char* mrow = p.mask + static_cast<long long>(b_hi) * p.m_hi + static_cast<long long>(b_lo) * p.m_lo;
-    uint8_t* my_maskrow = s_maskrow + g * 3 * Cfg::kSmallBytes + small_operand_row_offset(r);
+    uint8_t* my_maskrow = s_maskrow + g * 3 * Cfg::kSmallBytes + ptx::noswizzle_row_offset(r);
     const uint8_t* my_bias = s_bias + r * 128;
     const int swz = r & 7;
 

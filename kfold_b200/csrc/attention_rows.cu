@@ -74,12 +74,6 @@ struct RowsParams {
   int q_blocks, items;
 };
 
-__device__ __forceinline__ uint64_t noswizzle_desc(uint32_t smem_addr) {
-  return static_cast<uint64_t>((smem_addr & 0x3ffff) >> 4) | (static_cast<uint64_t>(128 >> 4) << 16) |
-         (static_cast<uint64_t>(256 >> 4) << 32) | (1ull << 46);
-}
-__device__ __forceinline__ uint32_t operand_row(int r) { return (r >> 3) * 256 + (r & 7) * 16; }
-
 __device__ __forceinline__ float ex2(float x) {
   float y;
   asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(y) : "f"(x));
@@ -182,8 +176,8 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   }
   if (warp < 4) {   // constant operands: e0 (ones in column 0), the identity; the zero halves of the mask operands
     const int r = warp * 32 + lane;
-    *reinterpret_cast<uint4*>(s_e0 + operand_row(r)) = make_uint4(0x3F80u, 0, 0, 0);
-    *reinterpret_cast<uint4*>(s_e0 + operand_row(r) + 128) = make_uint4(0, 0, 0, 0);
+    *reinterpret_cast<uint4*>(s_e0 + ptx::noswizzle_row_offset(r)) = make_uint4(0x3F80u, 0, 0, 0);
+    *reinterpret_cast<uint4*>(s_e0 + ptx::noswizzle_row_offset(r) + 128) = make_uint4(0, 0, 0, 0);
     if (r < 112) {
 #pragma unroll
       for (int e = 0; e < kEyes; ++e) {
@@ -195,13 +189,13 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           uint32_t w[4];
 #pragma unroll
           for (int i = 0; i < 4; ++i) w[i] = (at >> 1) == i ? ((at & 1) ? one << 16 : one) : 0u;
-          *reinterpret_cast<uint4*>(s_eye + e * kEyeBytes + operand_row(r) + h * 128) = make_uint4(w[0], w[1], w[2], w[3]);
+          *reinterpret_cast<uint4*>(s_eye + e * kEyeBytes + ptx::noswizzle_row_offset(r) + h * 128) = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
     }
     if (r < kT) {
 #pragma unroll
-      for (int u = 0; u < kMaskSlots * R; ++u) *reinterpret_cast<uint4*>(s_mask + u * kMaskBytes + operand_row(r) + 128) = make_uint4(0, 0, 0, 0);
+      for (int u = 0; u < kMaskSlots * R; ++u) *reinterpret_cast<uint4*>(s_mask + u * kMaskBytes + ptx::noswizzle_row_offset(r) + 128) = make_uint4(0, 0, 0, 0);
     }
     ptx::fence_proxy_async_smem();
   }
@@ -248,13 +242,13 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       constexpr uint32_t idesc_s = ptx::make_idesc(kQ, kT, 1);
       constexpr uint32_t idesc_o = ptx::make_idesc(kQ, kD, 1);
       const uint32_t kv_off = kBiasBytes + g * (kKBytes + kVBytes);
-      const uint64_t e0_desc = noswizzle_desc(ptx::smem_u32(s_e0));
-      const uint64_t eye_desc = noswizzle_desc(ptx::smem_u32(s_eye));
+      const uint64_t e0_desc = ptx::make_noswizzle_desc(ptx::smem_u32(s_e0));
+      const uint64_t eye_desc = ptx::make_noswizzle_desc(ptx::smem_u32(s_eye));
       const uint64_t bias_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_stage));
       const uint64_t q_desc = ptx::make_kmajor_desc<kD * 2>(ptx::smem_u32(s_q + g * kQBytes));
       const uint64_t k_desc = ptx::make_kmajor_desc<kD * 2>(ptx::smem_u32(s_stage + kv_off));
       const uint64_t v_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_stage + kv_off + kKBytes));
-      const uint64_t m_desc = noswizzle_desc(ptx::smem_u32(s_mask + g * kMaskSlots * kMaskBytes));
+      const uint64_t m_desc = ptx::make_noswizzle_desc(ptx::smem_u32(s_mask + g * kMaskSlots * kMaskBytes));
       const uint32_t tmem_g = tmem_base + g * (128 + kD), tmem_o = tmem_g + 128;
       auto first_masked = [&](const Item<R>& it) {
         int f = it.first[0];
@@ -364,7 +358,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
           if (!ok) continue;
           uint8_t* dst = s_mask + (g * kMaskSlots + slot) * kMaskBytes;
 #pragma unroll
-          for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(dst + operand_row(lane + 32 * i)) = make_uint4(v[i], 0, 0, 0);
+          for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(dst + ptx::noswizzle_row_offset(lane + 32 * i)) = make_uint4(v[i], 0, 0, 0);
           ptx::fence_proxy_async_smem();
           __syncwarp();
           if (lane == 0) ptx::mbar_arrive(&m_full[g * kMaskSlots + slot]);

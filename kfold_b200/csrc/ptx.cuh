@@ -301,6 +301,14 @@ __device__ __forceinline__ uint64_t make_kmajor_desc(uint32_t smem_addr) {
   return static_cast<uint64_t>((smem_addr & 0x3ffff) >> 4) | (1ull << 16) | (sbo << 32) | (1ull << 46) |
          (layout << 61);
 }
+// K-major operand without swizzle: 8 x 8 core matrices (8 rows of 16 bytes); the two K halves of a K=16
+// slice are 128 bytes apart (leading byte offset), groups of 8 rows 256 bytes apart (stride byte offset).
+__device__ __forceinline__ uint64_t make_noswizzle_desc(uint32_t smem_addr) {
+  return static_cast<uint64_t>((smem_addr & 0x3ffff) >> 4) | (static_cast<uint64_t>(128 >> 4) << 16) |
+         (static_cast<uint64_t>(256 >> 4) << 32) | (1ull << 46);
+}
+// Byte offset of row r of such an operand (its first eight K values; the other eight are 128 bytes on).
+__device__ __forceinline__ uint32_t noswizzle_row_offset(int r) { return (r >> 3) * 256 + (r & 7) * 16; }
 // Instruction descriptor for kind::f16 / kind::tf32 with fp32 accumulation, both operands K-major.
 //   [4,6) D format 1 = f32   [7,10) A format   [10,13) B format (0 f16, 1 bf16, 2 tf32)
 //   [17,23) N >> 3           [24,29) M >> 4
