@@ -86,7 +86,8 @@ KFB_API int kfb_profile_report(char* buf, size_t cap);
  * Replaces TriangleMultiplicationOutgoing.forward / TriangleMultiplicationIncoming.forward
  * (src/kfold/model/primitives/triangle_multiplication.py:179-229 and :263-313) and the Triton
  * entry point `forward(x, cached, direction, mask, eps)` called at :138-144.
- *   x, out : (batch, n, n, c) contiguous, `dtype`; n a multiple of 8, c a multiple of 64.
+ *   x, out : (batch, n, n, c) contiguous, `dtype`; c a multiple of 64; any n from 24 on, below that and with KFB_FP32_PRECISE a
+ *            multiple of 8.
  *   mask   : (batch, n, n) bytes, non-zero = valid.
  *   w_in_packed : bf16 [4c, c], linear_p_in / linear_g_in interleaved in blocks of 128 rows
  *                 (value rows of 128 channels, then their gate rows), BOTH multiplied by 0.5 (exact in bf16): the
@@ -353,8 +354,14 @@ KFB_API int kfb_linear_fp32(const void* x, const void* w6, const float* bias, vo
                             size_t workspace_bytes, long long rows, int n, int k, void* stream);
 /* out = LayerNorm(x) W^T (+ bias) (+ resid) at fp32 accuracy (kfb_linear_fp32 with the LayerNorm and the residual fused):
  * `a + linear_s_to_a(layernorm_s(s))` of DiffusionStack.step (src/kfold/model/layers/folding/diffusion.py:568).
- * x, resid, out fp32; ln_w / ln_b fp32 [k] or NULL; normalise == 0 skips the LayerNorm; workspace as kfb_linear_fp32.
- * normalise == KFB_NORMALISE_BF16_ROWS: with the LayerNorm, x bf16 (the heads of a bf16 stack: no float32 copy of x is made). */
+ * resid, out fp32; ln_w / ln_b fp32 [k] or NULL; workspace as kfb_linear_fp32.  `normalise` says what x holds and what is done
+ * with it, not only whether:
+ *   KFB_NORMALISE_NONE       x fp32, projected as it is (resid and bias still apply);
+ *   KFB_NORMALISE_FP32_ROWS  x fp32, LayerNorm first (so does any other non-zero value);
+ *   KFB_NORMALISE_BF16_ROWS  x bf16, LayerNorm first, from the same values as fp32 (the heads of a bf16 stack: no float32 copy
+ *                            of x is made). */
+#define KFB_NORMALISE_NONE 0
+#define KFB_NORMALISE_FP32_ROWS 1
 #define KFB_NORMALISE_BF16_ROWS 0x101
 KFB_API int kfb_ln_linear_fp32(const void* x, const float* ln_w, const float* ln_b, const void* w6, const float* bias,
                                const void* resid, void* out, void* workspace, size_t workspace_bytes, long long rows, int n, int k,

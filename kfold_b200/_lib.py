@@ -14,7 +14,7 @@ _PKG = os.path.dirname(os.path.abspath(__file__))
 LIB_PATH = os.path.join(_PKG, "_C", "libkfold_b200.so")
 
 KFB_BF16, KFB_FP32, KFB_FP32_PRECISE = 0, 1, 2
-KFB_NORMALISE_BF16_ROWS = 0x101   # kfb_ln_linear_fp32: LayerNorm of bf16 rows
+KFB_NORMALISE_FP32_ROWS, KFB_NORMALISE_BF16_ROWS = 1, 0x101   # kfb_ln_linear_fp32: what the normalised rows are
 _lib = None
 
 c_void_p, c_int, c_ll, c_float = ctypes.c_void_p, ctypes.c_int, ctypes.c_longlong, ctypes.c_float

@@ -84,7 +84,9 @@ inline int launch_kernel(cudaStream_t stream, void (*kernel)(KArgs...), dim3 gri
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
 __device__ __forceinline__ void grid_dependency_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
 // The start of every kernel that has nothing to do before its inputs: wait, then let the next kernel's blocks in -- at once when
-// the grid is small (its time is latency, which the overlap hides), otherwise as this grid's blocks exit.
+// the grid is small (its time is latency, which the overlap hides), otherwise as this grid's blocks exit.  The line is two blocks
+// for each of a B200's 148 multiprocessors, a constant where the host's rules ask sm_count(): reading %nsmid here cost 0.1 us a
+// launch (64-token pair block 178.8 -> 182.6 us), and where a part has fewer only the time of grids near the line moves.
 static constexpr unsigned kEarlyGrid = 2 * 148;
 __device__ __forceinline__ void grid_dependency_enter() {
   grid_dependency_wait();

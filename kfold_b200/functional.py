@@ -226,7 +226,7 @@ def ln_linear_fp32(x: torch.Tensor, ln_w: torch.Tensor | None, ln_b: torch.Tenso
     with L.on_device(x.device):
         ws = _workspace(x.device, lib.kfb_linear_fp32_workspace_bytes(x2.shape[0], k))
         L.check(lib.kfb_ln_linear_fp32(L.ptr(x2), L.ptr(lw), L.ptr(lb), L.ptr(w6), L.ptr(bias), L.ptr(res), L.ptr(out), L.ptr(ws),
-                                       ws.numel(), x2.shape[0], n, k, eps, L.KFB_NORMALISE_BF16_ROWS if bf else 1, L.stream_ptr()))
+                                       ws.numel(), x2.shape[0], n, k, eps, L.KFB_NORMALISE_BF16_ROWS if bf else L.KFB_NORMALISE_FP32_ROWS, L.stream_ptr()))
     return out.view(*x.shape[:-1], n)
 
 
