@@ -22,7 +22,7 @@ from .plans import NativeCall, StandsFor, handed_out
 __all__ = ["ConfidencePairSingleBlock", "ConfidencePairSingleStack", "ConfidenceHead"]
 
 
-class ConfidencePairSingleBlock(nn.Module, NativeCall):
+class ConfidencePairSingleBlock(NativeCall, nn.Module):
     """model/modules/confidence_head.py:125-175."""
 
     def __init__(self, channel_s: int, channel_z: int, num_heads: int, dropout: float = 0.25, kernel_backend: str = "b200"):

@@ -27,7 +27,7 @@ from torch import nn
 from . import functional as F
 from . import _lib as L
 from . import packing
-from .plans import NativeCall, ParamState, StandsFor, handed_out
+from .plans import NativeCall, ParamState, StandsFor, Unshared, handed_out
 
 __all__ = [
     "LayerNorm", "LinearNoBias", "Linear",
@@ -114,13 +114,14 @@ def _tensor_key(t: torch.Tensor) -> tuple:
     return (t.data_ptr(), tuple(t.shape), t.dtype, None if torch.is_inference(t) else t._version)
 
 
-class _PackedMixin:
+class _PackedMixin(Unshared):
     """Packs the module's weights once and re-packs when any parameter changes
     (same cache key as model/primitives/triangle_multiplication.py:73-91)."""
 
     _pack_cache = None
     _pack_key = None
     _pack_state = None
+    _unshared = ("_pack_cache", "_pack_key", "_pack_state")
 
     def _packed(self, device: torch.device, dtype: torch.dtype, pack_fn):
         key = (device, dtype)
@@ -134,7 +135,7 @@ class _PackedMixin:
 # --------------------------------------------------------------------------------------------
 # primitives
 # --------------------------------------------------------------------------------------------
-class _TriangleMultiplication(nn.Module, _PackedMixin):
+class _TriangleMultiplication(_PackedMixin, nn.Module):
     direction = "outgoing"
 
     def __init__(self, dim: int = 128, kernel_backend: str = "b200") -> None:
@@ -178,7 +179,7 @@ class _MHAParams(nn.Module):
         self.linear_g = LinearNoBias(c_in, c_hidden * no_heads)
 
 
-class _TriangleAttention(nn.Module, _PackedMixin):
+class _TriangleAttention(_PackedMixin, nn.Module):
     starting = True
 
     def __init__(self, c_in: int, no_heads: int, inf: float = 1e9, kernel_backend: str = "b200") -> None:
@@ -217,7 +218,7 @@ class TriangleAttentionEndingNode(_TriangleAttention):
     starting = False
 
 
-class Transition(nn.Module, _PackedMixin):
+class Transition(_PackedMixin, nn.Module):
     def __init__(self, channel: int, expansion_factor: int) -> None:
         super().__init__()
         self.model_dim = channel * expansion_factor
@@ -236,7 +237,7 @@ class Transition(nn.Module, _PackedMixin):
         return out.to(x.dtype)
 
 
-class AdaLN(nn.Module, _PackedMixin):
+class AdaLN(_PackedMixin, nn.Module):
     """Adaptive LayerNorm (model/primitives/normalization.py:94-125)."""
 
     def __init__(self, channel_a: int, channel_s: int):
@@ -360,7 +361,7 @@ class _StackPlan:
         return self.key == (device, precise) and self.state.current()
 
 
-class SelfAttentionPairBias(nn.Module, _PackedMixin):
+class SelfAttentionPairBias(_PackedMixin, nn.Module):
     """Pair-bias self-attention: the single-track form (``channel_s=None``, LayerNorm prologue) and the diffusion
     form (AdaLN prologue and the sigmoid(Linear(s)) output gate), model/layers/folding/attention_pair_bias.py:70-158."""
 
@@ -443,7 +444,7 @@ class SelfAttentionPairBias(nn.Module, _PackedMixin):
             return F.attention_pair_bias(an, pair_bias, mask, pk, out_dtype=a.dtype, resid=a if residual else None)
 
 
-class ConditionedTransitionBlock(nn.Module, _PackedMixin):
+class ConditionedTransitionBlock(_PackedMixin, nn.Module):
     """model/layers/folding/diffusion_transformer.py:45-81."""
 
     def __init__(self, channel_a: int, channel_s: int, expansion_factor: int = 2):
@@ -575,11 +576,11 @@ class CachedGlobalTransformerBlock(nn.Module):
 
 
 # the submodules that the native stack calls stand for (plans.StandsFor)
-_COND_TRANSITION = (ConditionedTransitionBlock, {"adaln": AdaLN})
-_TOKEN_BLOCK = (CachedGlobalTransformerBlock, {"attention": (SelfAttentionPairBias, {"adaln_a": AdaLN}), "transition": _COND_TRANSITION})
+_COND_TRANSITION = (ConditionedTransitionBlock, {"adaln*": AdaLN})
+_TOKEN_BLOCK = (CachedGlobalTransformerBlock, {"attention": (SelfAttentionPairBias, {"adaln_a*": AdaLN}), "transition": _COND_TRANSITION})
 
 
-class CachedGlobalTransformerStack(nn.Module, NativeCall):
+class CachedGlobalTransformerStack(NativeCall, nn.Module):
     """model/layers/folding/diffusion_transformer.py:260-339.  pair_bias (*, Nblock, H, L, L), as produced by
     DiffusionStack.get_pair_bias; it is converted to bf16 once per tensor and reused across sampler steps."""
 
@@ -589,10 +590,11 @@ class CachedGlobalTransformerStack(nn.Module, NativeCall):
         self.kernel_backend = kernel_backend
         self.blocks = nn.ModuleList(
             [CachedGlobalTransformerBlock(channel_a, channel_s, num_heads) for _ in range(num_blocks)])
-        self._bias_cache = None
-        self._bias_key = None
-        self._bias_src = None
         self._bank = _ConditioningBank()
+
+    # the converted pair bias of the present complex, known by its source's address: a copy has no claim to that
+    _bias_cache = _bias_key = _bias_src = None
+    _unshared = ("_plan", "_bias_cache", "_bias_key", "_bias_src")
 
     def _prepared_bias(self, pair_bias: torch.Tensor, precise: bool = False, per_block: bool = False):
         """(*, N, H, L, L) with the N blocks in front, in the compute dtype.  For the stack's call the rows lie at a pitch of a
@@ -754,7 +756,7 @@ def _index_share(lead: tuple, other_lead: tuple):
     return F._index_sharing(lead, other_lead)
 
 
-class CrossAttentionPairBias(nn.Module, _PackedMixin):
+class CrossAttentionPairBias(_PackedMixin, nn.Module):
     """Pair-bias cross attention of the atom windows (model/layers/folding/attention_pair_bias.py:161-260): AdaLN (or
     LayerNorm) prologues for the query and the key side, attention with `call_site="diffusion_local"`, and the
     sigmoid(Linear(s_q)) output gate."""
@@ -871,11 +873,11 @@ class LocalTransformerBlock(nn.Module):
         return out.view(shape)
 
 
-_ATOM_BLOCK = (LocalTransformerBlock, {"attention": (CrossAttentionPairBias, {"adaln_a_q": AdaLN, "adaln_a_k": AdaLN}),
+_ATOM_BLOCK = (LocalTransformerBlock, {"attention": (CrossAttentionPairBias, {"adaln_a_q*": AdaLN, "adaln_a_k*": AdaLN}),
                                        "transition": _COND_TRANSITION})
 
 
-class LocalTransformerStack(nn.Module, NativeCall):
+class LocalTransformerStack(NativeCall, nn.Module):
     """model/layers/folding/diffusion_transformer.py:419-512.  The whole stack works on the un-windowed atoms: the
     prologues, the projections, the output gate and the transition are row-wise, and under bfloat16 compute (head dim
     <= 32) the attention kernel walks the windows itself; the float32 path gathers the key side into windows.  The pair
@@ -891,10 +893,11 @@ class LocalTransformerStack(nn.Module, NativeCall):
             [LocalTransformerBlock(channel_a, channel_s, channel_z, num_heads) for _ in range(num_blocks)])
         self._bias_w = None
         self._bias_w_key = None
-        self._bias_all = None
-        self._bias_all_key = None
-        self._bias_all_src = None
         self._bank = _ConditioningBank()
+
+    # the window biases of the present complex, known by its pair tensor's address
+    _bias_all = _bias_all_key = _bias_all_src = None
+    _unshared = ("_plan", "_bias_all", "_bias_all_key", "_bias_all_src")
 
     def _stacked_bias_weights(self, device, dt):
         ws = [b.linear_z_to_bias.weight for b in self.blocks]
@@ -1269,7 +1272,7 @@ class _PairBlockPlan:
         return self.key == (device, dtype, precise) and self.state.current()
 
 
-class TriangularBlock(nn.Module, NativeCall):
+class TriangularBlock(NativeCall, nn.Module):
     """K-Fold trunk block: tri-mult out, tri-mult in, transition, residual adds fused into the kernels."""
 
     def __init__(self, channel_z: int = 256, dropout: float = 0.25, kernel_backend: str = "b200"):
@@ -1302,7 +1305,7 @@ class TriangularBlock(nn.Module, NativeCall):
         return self.transition_z(z, residual=True)
 
 
-class PairformerBlock(nn.Module, NativeCall):
+class PairformerBlock(NativeCall, nn.Module):
     """AF3-shaped Pairformer block assembled from the reference's modules: the pair track in the order of
     ``PairformerBlock.forward`` (tri-mult out/in, tri-att start/end, transition x4) and the single track of
     ``ConfidencePairSingleBlock.forward`` (pair bias from LN(z), single attention with pair bias, transition x4)."""

@@ -13,7 +13,7 @@ from itertools import chain
 import torch
 from torch.nn.modules import module as _nn_module
 
-__all__ = ["ParamState", "StandsFor", "NativeCall", "handed_out", "HandedOut"]
+__all__ = ["ParamState", "StandsFor", "NativeCall", "Unshared", "handed_out", "HandedOut"]
 
 _recording = threading.local()
 
@@ -65,7 +65,8 @@ class StandsFor:
 
     The native call reads their weights and never calls them.  That is the same thing only while they are what the framework
     made them: of exactly that class, without a `forward` of their own and without forward hooks, which would not fire.
-    Given as `module, class` or `module, (class, {child: ...})` pairs, children being looked at below a plain module only.
+    Given as `module, class` or `module, (class, {child: ...})` pairs, children being looked at below a plain module only; a child
+    whose name ends in `*` is read and not called without the native call either, so that its class is all that matters.
     `norms()`, asked when all are plain, lists the LayerNorms for which the call has one epsilon: they have to agree on it."""
 
     __slots__ = ("_submodules", "_classes", "_called", "_norms")
@@ -73,15 +74,16 @@ class StandsFor:
     def __init__(self, *pairs, norms):
         self._submodules, self._classes, self._called, todo = [], [], [], list(pairs)
         while todo:
-            m, cls = todo.pop()
+            m, cls, *read_only = todo.pop()
             children = {}
             if isinstance(cls, tuple):
                 cls, children = cls
             self._submodules.append(m)
             self._classes.append(cls)
             if type(m) is cls:
-                self._called.append(m.__dict__)
-                todo += [(m._modules.get(name), sub) for name, sub in children.items()]
+                if not any(read_only):
+                    self._called.append(m.__dict__)
+                todo += [(m._modules.get(name.rstrip("*")), sub, name[-1] == "*") for name, sub in children.items()]
         self._norms = norms() if self.plain() else []
 
     def plain(self) -> bool:
@@ -102,12 +104,23 @@ class StandsFor:
         return self.eps()
 
 
-class NativeCall:
+class Unshared:
+    """Mixin, before nn.Module, of a module that keeps things which are of use to it alone (addresses, views of its dictionaries):
+    `_unshared` names the attributes that a copy and a saved file go without.  The class has defaults for them."""
+
+    _unshared = ()
+
+    def __getstate__(self):
+        return {k: v for k, v in super().__getstate__().items() if k not in self._unshared}
+
+
+class NativeCall(Unshared):
     """Mixin of a block or stack that runs as one native call: `_plan_for(*key)` gives the plan of that call, or None where the
     submodules have to be called one by one.  The class provides `_stands_for()` and `_make_plan(*key)`; a plan has
     `fits(*key)` and `set_eps(eps)`, for an epsilon is no parameter and may be changed between calls."""
 
     _plan = None
+    _unshared = ("_plan",)
 
     def _plan_for(self, *key):
         plan = self._plan

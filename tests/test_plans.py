@@ -1,4 +1,7 @@
 """What a module keeps between calls: when its packed weights are stale, without a GPU."""
+import copy
+import io
+
 import pytest
 import torch
 from torch import nn
@@ -75,19 +78,20 @@ def test_submodules_that_are_hooked_or_replaced_are_called(name, path):
     sub = owner.get_submodule(path)
     parent, _, leaf = path.rpartition(".")
     parent = owner.get_submodule(parent)
+    read_only = path.endswith("adaln_a")      # its weights are read, it is not called in either case
     with torch.no_grad():
         plan = owner._plan_for(*key)
         assert plan is not None and owner._plan_for(*key) is plan
         for register in (sub.register_forward_hook, sub.register_forward_pre_hook):
             handle = register(lambda *a: None)
-            assert owner._plan_for(*key) is None
+            assert (owner._plan_for(*key) is None) is not read_only
             handle.remove()
             assert owner._plan_for(*key) is plan
         everywhere = nn.modules.module.register_module_forward_hook(lambda *a: None)
         assert owner._plan_for(*key) is None
         everywhere.remove()
         sub.forward = lambda *a, **k: a[0]
-        assert owner._plan_for(*key) is None
+        assert (owner._plan_for(*key) is None) is not read_only
         del sub.forward
         assert owner._plan_for(*key) is plan
         patched = type("Patched", (type(sub),), {"forward": lambda self, x, *a, **k: x})
@@ -136,3 +140,34 @@ def test_a_bias_for_blocks_called_one_by_one_is_converted_once(l, pitch):
     assert all(pb[i].is_contiguous() for i in range(3)) and stack._prepared_bias(bias, per_block=True) is pb
     assert torch.equal(pb.float(), bias.movedim(-4, 0).bfloat16().float())
     assert stack._prepared_bias(bias).stride(-2) % 8 == 0      # the stack's own form
+
+
+@pytest.mark.parametrize("name", sorted(_owners()))
+def test_a_module_that_has_run_can_be_copied_and_saved(name):
+    """What a module keeps for its native calls (addresses among it) stays with it: a copy, or what is loaded from a file, makes
+    its own, from its own weights."""
+    owner, key, _ = _owners()[name]
+    with torch.no_grad():
+        plan = owner._plan_for(*key)
+        buf = io.BytesIO()
+        torch.save(owner, buf)
+        buf.seek(0)
+        for other in (copy.deepcopy(owner), torch.load(buf, weights_only=False)):
+            made = other._plan_for(*key)
+            assert made is not None and made is not plan and owner._plan_for(*key) is plan
+            mine = {t.data_ptr() for t in plan.keep if t is not None}
+            assert not mine & {t.data_ptr() for t in made.keep if t is not None}
+            next(other.parameters()).zero_()
+            assert other._plan_for(*key) is not made and owner._plan_for(*key) is plan
+
+
+def test_a_copy_knows_no_complex_by_its_address(monkeypatch):
+    """The bias that a stack has converted is kept by the address of its source, which it holds; a copy must not keep the address
+    alone."""
+    monkeypatch.setattr(M.F, "window_bias", lambda z, lw, lb, w, eps: torch.randn(w.shape[0], *z.shape[:-1]))
+    token, atom = M.CachedGlobalTransformerStack(64, 32, 2, 2), M.LocalTransformerStack(64, 64, 16, 2, 2)
+    bias, z = torch.randn(1, 2, 2, 8, 8), torch.randn(1, 2, 32, 128, 16)
+    first, windows = token._prepared_bias(bias), atom._window_biases(z, torch.bfloat16)
+    t2, a2 = copy.deepcopy(token), copy.deepcopy(atom)
+    assert t2._bias_key is None and a2._bias_all_key is None
+    assert token._bias_src is bias and atom._window_biases(z, torch.bfloat16) is windows and first.shape == (2, 1, 2, 8, 8)
