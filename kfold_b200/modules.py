@@ -959,25 +959,24 @@ class LocalTransformerStack(NativeCall, nn.Module):
             raise ValueError(f"LocalTransformerStack: a {tuple(a.shape)}, z {tuple(z.shape)}, mask {tuple(mask.shape)}")
         h = self.num_heads
         s, _ = _shared_conditioning(a, s)
+        bias_all = self._window_biases(z, dt)                                        # (blocks*H, *z_lead, W, 32, 128)
+        z_lead = tuple(z.shape[:-3])                                                 # includes the window dim
+        # bf16 compute with head dim <= 32: the kernel walks the windows over the un-gathered atoms
+        native = (not precise and c // h <= 32 and c % h == 0
+                  and _index_share(lead, tuple(z.shape[:-4])) is not None and _index_share(lead, tuple(mask.shape[:-1])) is not None)
+        if native:
+            batch = _leading(lead)
+            bias_share = _index_share(lead, tuple(z.shape[:-4]))
+            mask2 = mask.to(torch.bool).reshape(-1, length)
+            # conditioning shared by the samples, window biases and mask shared inside each group: one native call
+            groups = _leading(tuple(s.shape[:-2]))
+            if (batch % groups == 0 and _index_share(lead, tuple(s.shape[:-2])) == batch // groups
+                    and (batch // groups) % bias_share == 0 and (batch // groups) % (batch // mask2.shape[0]) == 0):
+                plan = self._plan_for(a.device, False)
+                if plan is not None:
+                    return F.atom_stack(a, s, bias_all, mask2, plan, groups, bias_share, h, plan.hidden)
         with torch.autocast(a.device.type, enabled=False):
-            bias_all = self._window_biases(z, dt)                                        # (blocks*H, *z_lead, W, 32, 128)
-            z_lead = tuple(z.shape[:-3])                                                 # includes the window dim
-            # bf16 compute with head dim <= 32: the kernel walks the windows over the un-gathered atoms
-            native = (not precise and c // h <= 32 and c % h == 0
-                      and _index_share(lead, tuple(z.shape[:-4])) is not None and _index_share(lead, tuple(mask.shape[:-1])) is not None)
             if native:
-                batch = 1
-                for dd in lead:
-                    batch *= dd
-                bias_share = _index_share(lead, tuple(z.shape[:-4]))
-                mask2 = mask.to(torch.bool).reshape(-1, length)
-                # conditioning shared by the samples, window biases and mask shared inside each group: one native call
-                groups = _leading(tuple(s.shape[:-2]))
-                if (batch % groups == 0 and _index_share(lead, tuple(s.shape[:-2])) == batch // groups
-                        and (batch // groups) % bias_share == 0 and (batch // groups) % (batch // mask2.shape[0]) == 0):
-                    plan = self._plan_for(a.device, False)
-                    if plan is not None:
-                        return F.atom_stack(a, s, bias_all, mask2, plan, groups, bias_share, h, plan.hidden)
                 bias_all = bias_all.reshape(len(self.blocks), h, -1, WINDOW_Q, WINDOW_K)
             else:
                 to_qk = build_atom_to_qk_fn(length, a.device)
@@ -1066,14 +1065,12 @@ class AtomAttentionEncoder(nn.Module):
         precise = _is_precise(compute_dtype(q), "AtomAttentionEncoder")
         if self.use_structure:
             assert r_noisy is not None, "r_noisy must be provided if use_structure is True"
-            with torch.autocast(q.device.type, enabled=False):
-                q = F.coord_embed(q, r_noisy, self.linear_r_to_q.weight, mask=mask if mask_coords else None)
+            q = F.coord_embed(q, r_noisy, self.linear_r_to_q.weight, mask=mask if mask_coords else None)
         else:
             assert r_noisy is None, "r_noisy must be None if use_structure is False"
         q = self.transformer(q, c, p, mask)
-        with torch.autocast(q.device.type, enabled=False):
-            x = _project(q, self._proj.get(self.linear_q_to_a, q.device, precise), precise)
-            a = F.aggregate_atoms_to_tokens(x, token_index, mask, num_tokens, relu=True)
+        x = _project(q, self._proj.get(self.linear_q_to_a, q.device, precise), precise)
+        a = F.aggregate_atoms_to_tokens(x, token_index, mask, num_tokens, relu=True)
         return a, q, c, p
 
 
@@ -1100,13 +1097,11 @@ class AtomAttentionDecoder(nn.Module):
         `r_update * atom_mask` of DiffusionStack.step, fused into the projection)."""
         _check_inference(a)
         precise = _is_precise(compute_dtype(a), "AtomAttentionDecoder")
-        with torch.autocast(a.device.type, enabled=False):
-            a_to_q = _project(a, self._proj.get(self.linear_a_to_q, a.device, precise), precise)
-            q = F.broadcast_tokens_to_atoms(a_to_q, token_index, add=q_skip)
+        a_to_q = _project(a, self._proj.get(self.linear_a_to_q, a.device, precise), precise)
+        q = F.broadcast_tokens_to_atoms(a_to_q, token_index, add=q_skip)
         q = self.transformer(q, c_skip, p_skip, mask)
         ln = self.layernorm_q
-        with torch.autocast(a.device.type, enabled=False):
-            return F.ln_project(q, ln.weight, ln.bias, self.linear_q_to_r.weight, ln.eps, mask=mask if mask_out else None)
+        return F.ln_project(q, ln.weight, ln.bias, self.linear_q_to_r.weight, ln.eps, mask=mask if mask_out else None)
 
 
 class DiffusionStack(nn.Module):
@@ -1199,13 +1194,12 @@ class DiffusionStack(nn.Module):
             a, q_skip, c_skip, p_skip = self.atom_attention_encoder(q, c, p, token_index, atom_mask, token_mask.shape[-1],
                                                                     r_noisy=r_noisy, mask_coords=True)
         ln = self.layernorm_s
-        with torch.autocast(a.device.type, enabled=False):
-            # a.float() + linear_s_to_a(layernorm_s(s)): a float32 Linear in the reference whatever the autocast state
-            w_sa = self._proj.get(self.linear_s_to_a, a.device, True)
-            if s.shape[-3] == a.shape[-3]:
-                a = F.ln_linear_fp32(s.float(), ln.weight, ln.bias, w_sa, None, resid=a.float(), eps=ln.eps)
-            else:       # one conditioning row shared by the samples (the sampler's form): project once, add to every sample
-                a = a.float() + F.ln_linear_fp32(s.float(), ln.weight, ln.bias, w_sa, None, eps=ln.eps)
+        # a.float() + linear_s_to_a(layernorm_s(s)): a float32 Linear in the reference whatever the autocast state
+        w_sa = self._proj.get(self.linear_s_to_a, a.device, True)
+        if s.shape[-3] == a.shape[-3]:
+            a = F.ln_linear_fp32(s.float(), ln.weight, ln.bias, w_sa, None, resid=a.float(), eps=ln.eps)
+        else:       # one conditioning row shared by the samples (the sampler's form): project once, add to every sample
+            a = a.float() + F.ln_linear_fp32(s.float(), ln.weight, ln.bias, w_sa, None, eps=ln.eps)
         a = self.token_transformer(a, s, pair_bias.unsqueeze(-5), token_mask)
         a = self.layernorm_a(a)
         return self.atom_attention_decoder(a, q_skip, c_skip, p_skip, token_index, atom_mask, mask_out=True)

@@ -310,9 +310,10 @@ def test_a_capture_beside_a_full_cache():
     x = torch.randn(1 << 20, device=dev)
 
     def fn(t):
+        twice = t * 2
         scratch = torch.empty(big, dtype=torch.uint8, device=dev)      # freed to the capture stream's cache by the warm-up
         del scratch
-        return t * 2
+        return twice
 
     with torch.no_grad():
         try:
