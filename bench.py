@@ -73,10 +73,10 @@ def algorithmic_work(n: int | None = None, c: int = C_Z, h: int = 4, cs: int = C
     }
 
 
-# DRAM traffic of the triangle-attention kernel from its ncu capture at N=384 (dram__bytes_read.sum +
-# dram__bytes_write.sum of one launch: 144.9 MB + 23.9 MB); it grows with the number of pair positions.
-NCU_TRAFFIC = {"triatt_attention": {"n": 384, "bytes": 144.919040e6 + 23.904512e6,
-                                     "source": "ncu capture at N=384 scaled by pair positions (profiles/triatt_attention_n384_ncu.md)"}}
+# DRAM traffic of the triangle-attention kernel (attention_rows_kernel<3, 32>) from its ncu capture at N=768 (dram__bytes_read.sum +
+# dram__bytes_write.sum of one launch: 568.7 MB + 130.1 MB); it grows with the number of pair positions.
+NCU_TRAFFIC = {"triatt_attention": {"n": 768, "bytes": 568.657152e6 + 130.099712e6,
+                                     "source": "ncu capture at N=768 (profiles/attention_rows_ncu.md), scaled by pair positions at other sizes"}}
 
 
 def ncu_traffic(tag: str, n: int):
