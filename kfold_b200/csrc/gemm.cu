@@ -7,10 +7,11 @@
 
 #include "common.cuh"
 #include "gemm.cuh"
+#include "layernorm.cuh"
 
 namespace kfb {
 
-template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false>
+template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false>
 static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* tout,
                           const GemmParams& p, const char* tag) {
   using Cfg = GemmCfg<BN>;
@@ -19,7 +20,7 @@ static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUte
   KFB_CUDA(cudaGetDevice(&dev));
   cudaError_t attr_err = cudaSuccess;
   std::call_once(once[dev & 63], [&] {
-    attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP>, cudaFuncAttributeMaxDynamicSharedMemorySize,
+    attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                     Cfg::kSmemBytes);
   });
   KFB_CUDA(attr_err);
@@ -37,8 +38,8 @@ static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUte
   }
   {
     LaunchScope scope(stream, tag);
-    KFB_TRY(launch_kernel(stream, gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP>, grid,
-                          AUX ? kAuxThreads : kGemmThreads, Cfg::kSmemBytes, ta, tb, tout[0], tout[1], tout[2], q));
+    KFB_TRY(launch_kernel(stream, gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP, STATS>, grid,
+                          AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads, Cfg::kSmemBytes, ta, tb, tout[0], tout[1], tout[2], q));
   }
   return KFB_OK;
 }
@@ -47,7 +48,8 @@ template <int BN>
 static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* tout,
                      GemmParams p, const char* tag) {
   using Cfg = GemmCfg<BN>;
-  p.stages = Cfg::stages_for(p.aux ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes : Cfg::kStagingBytes);
+  p.stages = Cfg::stages_for(p.aux ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes + (p.stats_in_kernel ? kStatsBytes : 0)
+                                   : Cfg::kStagingBytes);
   if constexpr (BN == 32) {
     KFB_CHECK_ARG(!p.glu && !p.aux, "32-column tiles exist for the plain kernels only");
     if (p.precise) return launch_variant<32, false, false, true>(stream, ta, tb, tout, p, tag);
@@ -68,6 +70,9 @@ static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorM
   if (p.glu) {
     p.stages = Cfg::stages_for(Cfg::kGluStagingBytes);
     return launch_variant<BN, true, false, false>(stream, ta, tb, tout, p, tag);
+  }
+  if constexpr (BN == 64 || BN == 128) {
+    if (p.stats_in_kernel) return launch_variant<BN, false, true, false, false, true>(stream, ta, tb, tout, p, tag);
   }
   if constexpr (BN >= 64) {
     if (p.aux) return launch_variant<BN, false, true, false>(stream, ta, tb, tout, p, tag);
@@ -156,6 +161,15 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
     }
   }
   KFB_CHECK_ARG(bn == 32 || bn == 64 || bn == 128 || bn == 256, "unsupported BN %d", bn);
+  // LayerNorm statistics of K-outer rows: taken by the kernel itself where it has the warps for it, by a pass before it otherwise.  The
+  // statistics hold a stage of the ring a little longer, which costs little where a tile is few stages or comes from L2 (768 x 768 rows
+  // of 128 channels: pass + kernel 33 + 110 us, kernel alone 124; 400 x 400 of 256, 82 MB: 34 + 67, 87), and more than the pass where
+  // rows of four stages, read once for each of two column tiles, come from HBM (768 x 768 of 256, 302 MB: 58 + 215, 294).
+  p.stats_in_kernel = p.aux && bn <= 128 && a.s_k != 0 && p.row_stats != nullptr &&
+                      (p.k_extent <= 128 || static_cast<long long>(a.s_k) * p.k_extent * 2 <= (96ll << 20));
+  if (a.s_k != 0 && p.row_stats != nullptr && !p.stats_in_kernel)
+    KFB_TRY(launch_cm_stats(stream, static_cast<const __nv_bfloat16*>(a.ptr), p.row_stats, a.s_k, p.k_extent, a.s_k,
+                            p.stats_eps));
   if (p.precise) KFB_CHECK_ARG(p.k_extent % 48 == 0, "precise GEMM: K=%d is not six equal parts of whole 16-byte pieces", p.k_extent);
   if (p.glu) KFB_CHECK_ARG(p.n_cols % bn == 0, "GLU GEMM needs n_cols (%d) to be a multiple of the N tile (%d)", p.n_cols, bn);
   for (int i = 0; i < p.nseg; ++i) KFB_CHECK_ARG(p.seg[i].col_begin % 32 == 0, "segment start must be a multiple of 32");

@@ -65,8 +65,10 @@ struct GemmParams {
   int a_mn_major;                 // launcher: the A operand is stored K-outer ([k][row], rows contiguous) and read MN-major
   int k_inner;                    // launcher: != 0: both operands store K in pieces of k_inner elements (a multiple of the K
                                   // tile) that lie `s_k_hi` apart: K index = (k / k_inner, k % k_inner), five-dimensional maps
-  const float2* row_stats;        // optional LayerNorm fold: out = rstd[row] * (acc - mean[row] * col_s1[col]) + col_s0[col]
+  float2* row_stats;              // optional LayerNorm fold (K-outer A: scratch for them): out = rstd[row] * (acc - mean[row] * col_s1[col]) + col_s0[col]
   int stats_pitch;                //   rows of consecutive o lie stats_pitch entries apart (0: n_extent)
+  int stats_in_kernel;            //   launcher: the statistics are taken from the K-outer A tiles themselves (see STATS)
+  float stats_eps;                //   their epsilon
   const float* col_s1;            //   (mean, rstd) per flat row; col_s1 = sum_k W'[col][k], col_s0 = sum_k beta[k] W[col][k]
   const float* col_s0;            //   with W' = gamma * W the matrix actually multiplied (applied before gate / residual)
   int swap_col_begin;             // launcher (BN = 128, plain epilogue): tiles whose first column is >= this hold channel-major
@@ -99,6 +101,8 @@ static constexpr int kBK = 64;   // bf16 elements = 128 bytes = one swizzle span
 static constexpr int kEpiWarps = 8;  // two warps per TMEM lane quadrant, each taking every other 32-column chunk
 static constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 static constexpr int kAuxThreads = kGemmThreads + 32;  // the AUX variant's last warp hands finished tiles to the copy engine
+static constexpr int kStatsThreads = 64;               // the STATS variant's two warps after it: two rows of the tile per thread
+static constexpr int kStatsBytes = kBM * 8;            // (mean, rstd) of a tile's rows
 
 template <int BN>
 struct GemmCfg {
@@ -118,7 +122,7 @@ struct GemmCfg {
   // channel-major output tiles ([2 boxes of 64 positions][128 channels][128 bytes])
   static constexpr int kSwapStagingBytes = 1024 + 2 * kRowTileBytes;
   static constexpr int kBarrierBytes = 512;
-  static constexpr int kSmemBytes = 232448 - 1024;        // everything an SM offers one CTA
+  static constexpr int kSmemBytes = 232448;               // everything an SM offers one CTA
   // after the operand ring comes EITHER the channel-major staging slabs OR one or two buffers of prefetched
   // gate and / or residual tiles (128 rows x BN columns bf16 each); the launcher picks the ring depth accordingly
   static constexpr int kAuxTileBytes = kBM * BN * 2;
@@ -313,8 +317,11 @@ __device__ __forceinline__ void tile_advance(TileIdx& t, const GemmParams& p) {
 //         D[channel][position] = W[channel][:] . X[position][:], i.e. the 128 value rows and the 128 gate rows of the weight
 //         tile are the M operands of two N=128 MMAs and the 128 positions are the N operand.  A thread then holds
 //         consecutive positions of ONE channel and writes them with 32-byte stores: no transpose through shared memory.
-template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false>
-__global__ void __launch_bounds__(AUX ? kAuxThreads : kGemmThreads, 1)
+//   STATS (with AUX and a K-outer A operand): two more warps take the rows' LayerNorm statistics from the A tiles in shared memory while
+//         the tensor core multiplies them: a pass over A and a launch less (see the launcher for where and what it measured).  The
+//         sums run over the channels in order, as that pass does: the same bits.
+template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false>
+__global__ void __launch_bounds__(AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                  const __grid_constant__ CUtensorMap tm_out0, const __grid_constant__ CUtensorMap tm_out1,
                  const __grid_constant__ CUtensorMap tm_out2, const GemmParams p) {
@@ -324,6 +331,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   constexpr int OUT_BN_GLU = BN / 2;
   constexpr int ACC_COLS = PRECISE ? 2 * BN : BN;  // precise: main accumulator, then the correction accumulator
   static_assert(!PRECISE || BN <= 128, "the fp32-accurate variant needs four accumulators of BN columns");
+  static_assert(!STATS || AUX, "in-kernel statistics exist for the AUX variant");
   static_assert(!SWAP || (BN == 256 && GLU && !AUX && !PRECISE), "the swapped orientation exists for the BN = 256 GLU tile");
   constexpr bool kSplitGlu = GLU && !PRECISE && BN < 256;
   constexpr bool kXpose = BN <= 128 && !GLU && !AUX && !PRECISE;
@@ -335,8 +343,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   uint8_t* s_b = smem + kStages * Cfg::kAStage;
   uint8_t* s_stage_out = smem + kStages * Cfg::kStageBytes;  // [group of 4 epilogue warps][2][32 channels][128 rows] bf16 ...
   uint8_t* s_aux = s_stage_out;                               // ... or [buffers][gate, resid][BN / 64][128 x 64] bf16
+  float2* s_stats = reinterpret_cast<float2*>(s_aux + p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes);   // (STATS)
   uint64_t* bars = reinterpret_cast<uint64_t*>(
-      s_stage_out + (AUX ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes : (SWAP ? Cfg::kSwapStagingBytes : (GLU ? Cfg::kGluStagingBytes : Cfg::kStagingBytes))));
+      s_stage_out + (AUX ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes + (STATS ? kStatsBytes : 0) : (SWAP ? Cfg::kSwapStagingBytes : (GLU ? Cfg::kGluStagingBytes : Cfg::kStagingBytes))));
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + Cfg::kMaxStages;
   uint64_t* tmem_full = bars + 2 * Cfg::kMaxStages;
@@ -345,7 +354,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   uint64_t* aux_empty = aux_full + 2;    // [2]: the output tile has left, one arrival by the store warp
   uint64_t* cm_bar = aux_empty + 2;      // [2 groups][slab free, slab written], 128 arrivals each
   uint64_t* rm_bar = cm_bar + 4;         // [2 staging buffers]: row-major tile written, one arrival per epilogue thread
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(rm_bar + 2);
+  uint64_t* stats_bar = rm_bar + 2;      // STATS: [full: 2 warps, free: the epilogue warps]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stats_bar + 2);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -365,7 +375,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     ptx::prefetch_tmap(&tm_b);
     for (int s = 0; s < kStages; ++s) {
       ptx::mbar_init(&full_bar[s], 1);
-      ptx::mbar_init(&empty_bar[s], 1);
+      ptx::mbar_init(&empty_bar[s], STATS ? 1 + kStatsThreads / 32 : 1);
     }
     for (int a = 0; a < 2; ++a) {
       ptx::mbar_init(&tmem_full[a], 1);
@@ -375,6 +385,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     }
     for (int a = 0; a < 4; ++a) ptx::mbar_init(&cm_bar[a], 128);
     for (int a = 0; a < 2; ++a) ptx::mbar_init(&rm_bar[a], 32 * kEpiWarps);
+    ptx::mbar_init(&stats_bar[0], kStatsThreads / 32);
+    ptx::mbar_init(&stats_bar[1], kEpiWarps);
     ptx::fence_barrier_init();
   }
   if (warp == 1) {
@@ -605,6 +617,54 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       }
       ptx::tma_store_wait_all();
     }
+  } else if (STATS && warp > kGemmThreads / 32) {
+    // ------------------------------------------------------------ statistics of the A rows: thread t has rows 2 t and 2 t + 1 of the
+    // tile, i.e. one 4-byte cell of every k row of its 64-row box (neighbouring lanes, neighbouring cells: no bank conflicts)
+    const int t2 = (threadIdx.x - kAuxThreads) * 2;
+    uint32_t cell[8];             // offset of the cell in k rows 0..7 of a box (128-byte rows, the copy engine's 16-byte swizzle)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) cell[j] = (t2 >> 6) * (Cfg::kAStage / 2) + j * 128 + ((((t2 & 63) >> 3) ^ j) << 4) + (t2 & 7) * 2;
+    const float inv_c = 1.0f / static_cast<float>(p.k_extent);
+    int stage = 0;
+    uint32_t phase = 0, tile_iter = 0;
+    bool ok = true;
+    for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++tile_iter) {
+      // sums shifted by the first channel's value keep E[x^2] - E[x]^2 harmless
+      float x0 = 0.f, x1 = 0.f, s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
+      for (int kb = 0; kb < num_k; ++kb) {
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&full_bar[stage], phase, 114));
+        if (!ok) break;
+        const uint8_t* box = s_a + stage * Cfg::kAStage;
+        if (kb == 0) {
+          const uint32_t w = *reinterpret_cast<const uint32_t*>(box + cell[0]);
+          x0 = __uint_as_float(w << 16);
+          x1 = __uint_as_float(w & 0xffff0000u);
+        }
+#pragma unroll 2
+        for (int k8 = 0; k8 < kBK / 8; ++k8) {
+          uint32_t w[8];
+#pragma unroll
+          for (int j = 0; j < 8; ++j) w[j] = *reinterpret_cast<const uint32_t*>(box + k8 * 1024 + cell[j]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) {
+            const float d0 = __uint_as_float(w[j] << 16) - x0, d1 = __uint_as_float(w[j] & 0xffff0000u) - x1;
+            s0 += d0; q0 = fmaf(d0, d0, q0);
+            s1 += d1; q1 = fmaf(d1, d1, q1);
+          }
+        }
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&empty_bar[stage]);
+        if (++stage == kStages) { stage = 0; phase ^= 1; }
+      }
+      if (!ok) break;
+      ok = __all_sync(0xffffffffu, ptx::mbar_wait(&stats_bar[1], (tile_iter & 1) ^ 1, 115));   // the last tile's have been read
+      if (!ok) break;
+      const float m0 = s0 * inv_c, m1 = s1 * inv_c;
+      *reinterpret_cast<float4*>(s_stats + t2) = make_float4(x0 + m0, rsqrtf(fmaxf(q0 - s0 * m0, 0.f) * inv_c + p.stats_eps),
+                                                             x1 + m1, rsqrtf(fmaxf(q1 - s1 * m1, 0.f) * inv_c + p.stats_eps));
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(&stats_bar[0]);
+    }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..9)
     const int quad = warp & 3;  // TMEM lane quadrant this warp may read
@@ -673,7 +733,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       const uint32_t acc_phase = (tile_iter >> 1) & 1;
       float2 stats = make_float2(0.f, 1.f);     // this row's (mean, rstd), on its way while the tensor core works
       if constexpr (AUX) {
-        if (p.row_stats != nullptr && row_ok)
+        if (!STATS && p.row_stats != nullptr && row_ok)
           stats = p.row_stats[(static_cast<long long>(b) * p.o_extent + o) * (p.stats_pitch > 0 ? p.stats_pitch : p.n_extent) + n];
       }
       if constexpr (kXpose) {
@@ -685,6 +745,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       if (threadIdx.x == 64) KFB_GSTAMP(4 + tile_iter * 4 + 0);
       ptx::tc_fence_after_sync();
       if (AUX && !ptx::mbar_wait(&aux_full[aux_buf], aux_par, 107)) { ok = false; break; }
+      if constexpr (STATS) {
+        if (!ptx::mbar_wait(&stats_bar[0], tile_iter & 1, 116)) { ok = false; break; }
+        stats = s_stats[r];
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive(&stats_bar[1]);
+      }
       const uint32_t t_row = tmem_base + acc * ACC_COLS + (static_cast<uint32_t>(quad * 32) << 16);
 
       constexpr int out_bn = GLU ? OUT_BN_GLU : BN;
@@ -973,7 +1039,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 #pragma unroll
             for (int i = 0; i < 16; ++i) v[i] += __ldg(p.col_bias + out_col + i);
           }
-          if (p.row_stats != nullptr) {   // folded LayerNorm of the A rows (see GemmParams)
+          if (STATS || p.row_stats != nullptr) {   // folded LayerNorm of the A rows (see GemmParams)
             const float4* s1 = reinterpret_cast<const float4*>(p.col_s1 + out_col);
             const float4* s0 = reinterpret_cast<const float4*>(p.col_s0 + out_col);
 #pragma unroll

@@ -104,14 +104,64 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* __restric
   }
 }
 
+// Folded weights (see LnFold), kFoldRows rows per block of 256 threads: W' rounded to bf16, s1 of the rounded values.  The pair track's
+// LayerNorm kernels do it in blocks of their own before their rows: as a launch it was 3.3 us, whatever the size.
+constexpr int kFoldRows = 8;
+__device__ __forceinline__ void ln_fold_rows(const LnFold& f, int block) {
+  constexpr int kPer = kFoldRows / 2;                       // rows of each half of the block
+  const int half = threadIdx.x >> 7, tid = threadIdx.x & 127, w4 = tid >> 5;
+  const int n0 = block * kFoldRows + half * kPer;
+  float a1[kPer], a0[kPer];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    a1[j] = a0[j] = 0.f;
+    const long long row = static_cast<long long>(min(n0 + j, f.n - 1)) * f.k;
+    for (int i = tid; i < f.k; i += 128) {
+      const float wv = __bfloat162float(f.w[row + i]);
+      const __nv_bfloat16 wr = __float2bfloat16_rn(wv * (f.gamma != nullptr ? f.gamma[i] : 1.0f));
+      if (n0 + j < f.n) f.wf[row + i] = wr;
+      a1[j] += __bfloat162float(wr);
+      a0[j] += (f.beta != nullptr ? f.beta[i] : 0.0f) * wv;
+    }
+  }
+  __shared__ float red[2][kFoldRows][4];
+#pragma unroll
+  for (int j = 0; j < kPer; ++j) {
+    const float r1 = warp_sum(a1[j]), r0 = warp_sum(a0[j]);
+    if ((tid & 31) == 0) {
+      red[0][half * kPer + j][w4] = r1;
+      red[1][half * kPer + j][w4] = r0;
+    }
+  }
+  __syncthreads();
+  const int j = threadIdx.x % kFoldRows, n = block * kFoldRows + j;
+  if (threadIdx.x < 2 * kFoldRows && n < f.n) {
+    const float* r = red[threadIdx.x / kFoldRows][j];
+    (threadIdx.x < kFoldRows ? f.s1 : f.s0)[n] = (r[0] + r[1]) + (r[2] + r[3]);
+  }
+}
+__global__ void __launch_bounds__(256) ln_fold_weights_kernel(const LnFold f) {
+  grid_dependency_enter();
+  ln_fold_rows(f, blockIdx.x);
+}
+int launch_ln_fold_weights(cudaStream_t stream, const LnFold& f) {
+  KFB_CHECK_ARG(f.n > 0 && f.k > 0, "ln_fold_weights: n %d k %d", f.n, f.k);
+  LaunchScope scope(stream, "layernorm_fold_weights");
+  return launch_kernel(stream, ln_fold_weights_kernel, cdiv(f.n, kFoldRows), 256, 0, f);
+}
+
 // The pair track's shape: 128 bf16 channels, contiguous rows.  A row is 256 bytes = 16 lanes x 16 bytes, so a warp takes two
 // rows per step and two steps per iteration: four rows (1 KB) in flight per warp, 16-byte loads and stores, the statistics
 // reduced over the 16 lanes of a row.  Same arithmetic as layernorm_rows_kernel (two passes, fp32).
 __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                                                   const float* __restrict__ w, const float* __restrict__ b,
-                                                                  long long rows, float eps) {
+                                                                  long long rows, float eps, int fold_blocks, const LnFold fold) {
   constexpr int LANES = 16, STEPS = 2, C = LANES * 8, kRows = 32 / LANES;
   grid_dependency_enter();
+  if (static_cast<int>(blockIdx.x) < fold_blocks) {
+    ln_fold_rows(fold, blockIdx.x);
+    return;
+  }
   const int lane = threadIdx.x & 31;
   const int sub = lane % LANES;              // 16-byte chunk of the row
   const int half = lane / LANES;             // which of the step's rows
@@ -121,8 +171,8 @@ __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfl
     g[i] = w != nullptr ? w[sub * 8 + i] : 1.0f;
     o[i] = b != nullptr ? b[sub * 8 + i] : 0.0f;
   }
-  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
-  const long long warp_id = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const long long warps = static_cast<long long>(gridDim.x - fold_blocks) * (blockDim.x >> 5);
+  const long long warp_id = static_cast<long long>(blockIdx.x - fold_blocks) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   for (long long base = warp_id * (kRows * STEPS); base < rows; base += warps * (kRows * STEPS)) {
     uint4 raw[STEPS];
     bool live[STEPS];
@@ -176,9 +226,13 @@ __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfl
 constexpr int kC256Rows = 4;
 __global__ void __launch_bounds__(256) layernorm_c256_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
                                                                   const float* __restrict__ w, const float* __restrict__ b,
-                                                                  long long rows, float eps) {
+                                                                  long long rows, float eps, int fold_blocks, const LnFold fold) {
   constexpr int G = 4, C = 256;
   grid_dependency_enter();
+  if (static_cast<int>(blockIdx.x) < fold_blocks) {
+    ln_fold_rows(fold, blockIdx.x);
+    return;
+  }
   const int lane = threadIdx.x & 31;
   float2 ww[G], bb[G];
 #pragma unroll
@@ -186,8 +240,8 @@ __global__ void __launch_bounds__(256) layernorm_c256_bf16_kernel(const __nv_bfl
     ww[g] = w != nullptr ? *reinterpret_cast<const float2*>(w + (lane + 32 * g) * 2) : make_float2(1.f, 1.f);
     bb[g] = b != nullptr ? *reinterpret_cast<const float2*>(b + (lane + 32 * g) * 2) : make_float2(0.f, 0.f);
   }
-  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
-  const long long warp_id = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const long long warps = static_cast<long long>(gridDim.x - fold_blocks) * (blockDim.x >> 5);
+  const long long warp_id = static_cast<long long>(blockIdx.x - fold_blocks) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   for (long long base = warp_id * kC256Rows; base < rows; base += warps * kC256Rows) {
     float2 v[kC256Rows][G];
 #pragma unroll
@@ -264,7 +318,7 @@ static int dispatch_g(cudaStream_t stream, const void* x, void* y, const float* 
 }
 
 int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w, const float* b, long long rows, int c,
-                     long long xs, long long ys, float eps, int in_dtype, int out_dtype, RowPerm perm) {
+                     long long xs, long long ys, float eps, int in_dtype, int out_dtype, RowPerm perm, const LnFold* fold) {
   KFB_CHECK_ARG(rows >= 0 && c > 0 && c % 2 == 0, "layernorm: rows %lld, channels %d (must be even)", rows, c);
   KFB_CHECK_ARG(perm.rows == 0 || (perm.n % perm.rows == 0 && rows == static_cast<long long>(perm.rows) * perm.n),
                 "layernorm: exchange order needs a (%d, %d) shard, got %lld rows", perm.rows, perm.n, rows);
@@ -275,12 +329,15 @@ int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w
     long long blocks = (rows + 31) / 32;      // 8 warps x 4 rows per iteration
     const long long cap = static_cast<long long>(sm_count()) * 16;
     if (blocks > cap) blocks = cap;
+    const int fold_blocks = fold != nullptr ? cdiv(fold->n, kFoldRows) : 0;
     LaunchScope scope(stream, "layernorm_rows");
-    KFB_TRY(launch_kernel(stream, c == 128 ? layernorm_c128_bf16_kernel : layernorm_c256_bf16_kernel, static_cast<unsigned>(blocks),
-                          256, 0, static_cast<const __nv_bfloat16*>(x), static_cast<__nv_bfloat16*>(y), w, b, rows, eps));
+    KFB_TRY(launch_kernel(stream, c == 128 ? layernorm_c128_bf16_kernel : layernorm_c256_bf16_kernel,
+                          static_cast<unsigned>(blocks + fold_blocks), 256, 0, static_cast<const __nv_bfloat16*>(x),
+                          static_cast<__nv_bfloat16*>(y), w, b, rows, eps, fold_blocks, fold != nullptr ? *fold : LnFold{}));
     KFB_CUDA(cudaGetLastError());
     return KFB_OK;
   }
+  if (fold != nullptr) KFB_TRY(launch_ln_fold_weights(stream, *fold));
   if (in_dtype == KFB_BF16 && out_dtype == KFB_BF16)
     return dispatch_g<__nv_bfloat16, __nv_bfloat16>(stream, x, y, w, b, rows, c, xs, ys, eps, perm);
   if (in_dtype == KFB_FP32 && out_dtype == KFB_BF16)
@@ -812,7 +869,8 @@ __global__ void __launch_bounds__(kCmPos) layernorm_cm_kernel(const TI* __restri
 // LayerNorm folded into the GEMM that follows it.  For rows x (c channels) and a projection W,
 //   LN(x) W^T = rstd * (x W'^T - mean * s1) + s0,   W' = gamma * W,  s1[n] = sum_k W'[n][k],  s0[n] = sum_k beta[k] W[n][k],
 // so the GEMM can read the raw rows (here: channel-major, as the triangle contraction leaves them) and the epilogue
-// applies the per-row (mean, rstd) and the per-column s1, s0.  Two small kernels prepare those.
+// applies the per-row (mean, rstd) and the per-column s1, s0.  The projection's kernel takes the statistics itself where it has the
+// warps for it (gemm.cuh, STATS); cm_stats does where it has not.
 // ------------------------------------------------------------------------------------------------
 // (mean, rstd) over the channels of every position of a channel-major tensor t[c][npos]; two positions per thread
 __global__ void __launch_bounds__(256) cm_stats_kernel(const __nv_bfloat16* __restrict__ t, float2* __restrict__ stats,
@@ -908,40 +966,6 @@ int launch_cm_stats(cudaStream_t stream, const __nv_bfloat16* t, float2* stats, 
   const long long threads = npos / 2;
   KFB_TRY(launch_kernel(stream, cm_stats_kernel, static_cast<unsigned>((threads + 255) / 256), 256, 0, t, stats, npos, c,
       chan_stride, eps));
-  KFB_CUDA(cudaGetLastError());
-  return KFB_OK;
-}
-
-// W'[n][k] = bf16(gamma[k] W[n][k]); s1[n] = sum_k W'[n][k] (of the rounded values); s0[n] = sum_k beta[k] W[n][k]
-__global__ void __launch_bounds__(128) ln_fold_weights_kernel(const __nv_bfloat16* __restrict__ w, const float* __restrict__ gamma,
-                                                              const float* __restrict__ beta, __nv_bfloat16* __restrict__ wf,
-                                                              float* __restrict__ s1, float* __restrict__ s0, int k) {
-  grid_dependency_enter();
-  const int n = blockIdx.x;
-  float a1 = 0.f, a0 = 0.f;
-  for (int i = threadIdx.x; i < k; i += blockDim.x) {
-    const float wv = __bfloat162float(w[static_cast<long long>(n) * k + i]);
-    const __nv_bfloat16 f = __float2bfloat16_rn(wv * (gamma != nullptr ? gamma[i] : 1.0f));
-    wf[static_cast<long long>(n) * k + i] = f;
-    a1 += __bfloat162float(f);
-    a0 += (beta != nullptr ? beta[i] : 0.0f) * wv;
-  }
-  __shared__ float r1[4], r0[4];
-  a1 = warp_sum(a1);
-  a0 = warp_sum(a0);
-  if ((threadIdx.x & 31) == 0) { r1[threadIdx.x >> 5] = a1; r0[threadIdx.x >> 5] = a0; }
-  __syncthreads();
-  if (threadIdx.x == 0) {
-    s1[n] = (r1[0] + r1[1]) + (r1[2] + r1[3]);
-    s0[n] = (r0[0] + r0[1]) + (r0[2] + r0[3]);
-  }
-}
-
-int launch_ln_fold_weights(cudaStream_t stream, const __nv_bfloat16* w, const float* gamma, const float* beta, __nv_bfloat16* wf,
-                           float* s1, float* s0, int n, int k) {
-  KFB_CHECK_ARG(n > 0 && k > 0, "ln_fold_weights: n %d k %d", n, k);
-  LaunchScope scope(stream, "layernorm_fold_weights");
-  KFB_TRY(launch_kernel(stream, ln_fold_weights_kernel, n, 128, 0, w, gamma, beta, wf, s1, s0, k));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }

@@ -11,9 +11,22 @@ struct RowPerm {
   int n = 0;
 };
 
-// Row-wise LayerNorm, one warp per row, fp32 statistics.  in/out dtype KFB_BF16 or KFB_FP32.
+// Weights of a projection with the LayerNorm before it folded in (see layernorm.cu): wf[n][k] = bf16(gamma[k] w[n][k]),
+// s1[n] = sum_k wf[n][k], s0[n] = sum_k beta[k] w[n][k].
+struct LnFold {
+  const __nv_bfloat16* w;
+  const float *gamma, *beta;
+  __nv_bfloat16* wf;
+  float *s1, *s0;
+  int n, k;
+};
+int launch_ln_fold_weights(cudaStream_t stream, const LnFold& f);
+
+// Row-wise LayerNorm, one warp per row, fp32 statistics.  in/out dtype KFB_BF16 or KFB_FP32.  fold: weights to be folded along the
+// way, in the same launch where the kernel can.
 int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w, const float* b, long long rows, int c,
-                     long long xs, long long ys, float eps, int in_dtype, int out_dtype, RowPerm perm = RowPerm());
+                     long long xs, long long ys, float eps, int in_dtype, int out_dtype, RowPerm perm = RowPerm(),
+                     const LnFold* fold = nullptr);
 
 // fp32 -> bf16 (round to nearest), n elements.
 int launch_to_bf16(cudaStream_t stream, const float* x, __nv_bfloat16* y, long long n);
@@ -41,12 +54,9 @@ int launch_layernorm_cm(cudaStream_t stream, const void* t, __nv_bfloat16* y, co
 int launch_adaln(cudaStream_t stream, const void* a, void* y, const void* gv, long long rows, int c, int samples,
                  int l, float eps, int in_dtype, int out_dtype, long long gv_ld = 0);
 
-// LayerNorm folded into the following GEMM (see layernorm.cu): per-position (mean, rstd) of a channel-major tensor, and the
-// folded weights W' = gamma * W (bf16) with s1[n] = sum_k W'[n][k], s0[n] = sum_k beta[k] W[n][k].
+// LayerNorm folded into the following GEMM (see layernorm.cu): per-position (mean, rstd) of a channel-major tensor.
 int launch_cm_stats(cudaStream_t stream, const __nv_bfloat16* t, float2* stats, long long npos, int c, long long chan_stride,
                     float eps);
-int launch_ln_fold_weights(cudaStream_t stream, const __nv_bfloat16* w, const float* gamma, const float* beta, __nv_bfloat16* wf,
-                           float* s1, float* s0, int n, int k);
 
 // LayerNorm over c (16, 32 or 64) channels and projection to nh values per position: x [npos][c], w [nh][c] of `dtype`
 // (KFB_BF16 or KFB_FP32), y [nh][npos] of the same type.  normalise == 0: projection only.

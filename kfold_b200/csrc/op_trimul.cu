@@ -29,7 +29,8 @@ namespace {
 inline int pitch8(int n) { return (n + 7) / 8 * 8; }
 
 struct TrimulWs {
-  __nv_bfloat16 *xn, *ab, *gl, *t;
+  __nv_bfloat16 *xn, *ab, *gl, *t, *wf;
+  float* s;
 };
 size_t carve(TrimulWs& w, void* base, int batch, int n, int c) {
   Carver cv(base);
@@ -38,6 +39,8 @@ size_t carve(TrimulWs& w, void* base, int batch, int n, int c) {
   w.ab = cv.take<__nv_bfloat16>(pos_p * 2 * c);
   w.gl = cv.take<__nv_bfloat16>(pos * c);
   w.t = cv.take<__nv_bfloat16>(pos_p * c);
+  w.wf = cv.take<__nv_bfloat16>(static_cast<size_t>(c) * c);   // the output projection's weights with its LayerNorm folded in
+  w.s = cv.take<float>(2 * static_cast<size_t>(c));
   return cv.off;
 }
 
@@ -53,10 +56,11 @@ int check_shape(const char* what, int batch, int rows, int n, int c) {
 // parts > 1: only part `part` of the 2c operand channels (in packed order) is projected, into `ab` = that part's buffer.
 int project(cudaStream_t stream, int transposed_walk, const void* x, const unsigned char* mask, const float* ln_w,
             const float* ln_b, const void* w_in_packed, const void* w_gout, __nv_bfloat16* xn, __nv_bfloat16* ab,
-            __nv_bfloat16* gl, int batch, int rows, int n, int c, float eps, int dtype, int part = 0, int parts = 1) {
+            __nv_bfloat16* gl, int batch, int rows, int n, int c, float eps, int dtype, int part = 0, int parts = 1,
+            const LnFold* fold = nullptr) {
   const long long rn = static_cast<long long>(rows) * n;
   const long long pos = rn * batch;
-  if (x != nullptr) KFB_TRY(launch_layernorm(stream, x, xn, ln_w, ln_b, pos, c, c, c, eps, dtype, KFB_BF16));
+  if (x != nullptr) KFB_TRY(launch_layernorm(stream, x, xn, ln_w, ln_b, pos, c, c, c, eps, dtype, KFB_BF16, RowPerm(), fold));
   if (w_in_packed != nullptr) {
     // ab[ch][b][o][n_]: o = row of the shard, n_ = position inside the row (swapped for the transposed walk)
     GemmParams p = {};
@@ -107,13 +111,26 @@ int project(cudaStream_t stream, int transposed_walk, const void* x, const unsig
 
 // steps 4-6.  a: [c][batch][rows][np]; b: pieces of [c][batch][b_piece_rows][np], `b_piece_stride` elements apart; np = n rounded
 // up to the row pitch.  A ragged n costs nothing but tiles that end early: no padded copy of x, out or the mask is made.
+// folded: w_pout with the LayerNorm folded in, if an earlier launch of this call has done that.
 int finish(cudaStream_t stream, const __nv_bfloat16* a, const __nv_bfloat16* b, int b_piece_rows, long long b_piece_stride,
            const __nv_bfloat16* gl, const float* ln_out_w, const float* ln_out_b, const void* w_pout, __nv_bfloat16* t,
-           __nv_bfloat16* tn, void* out, const void* resid, int batch, int rows, int n, int c, float eps, int dtype) {
+           __nv_bfloat16* tn, void* out, const void* resid, int batch, int rows, int n, int c, float eps, int dtype,
+           const LnFold* folded = nullptr) {
   const long long rn = static_cast<long long>(rows) * n;
   const long long pos = rn * batch;
   const int np = pitch8(n);
   const long long rnp = static_cast<long long>(rows) * np, posp = rnp * batch;
+  // LayerNorm_out folded into the output projection: the GEMM reads t as it lies (channel-major, read MN-major), the
+  // epilogue applies the per-position statistics.  The scratch buffer tn holds the folded weights and the statistics.
+  const bool fold = (c % kBK == 0) && posp * static_cast<long long>(c) * 2 >= static_cast<long long>(c) * c * 2 + 256 + 2ll * c * 4 + 256 + posp * 8;
+  uint8_t* base = reinterpret_cast<uint8_t*>(tn);
+  float* s1 = reinterpret_cast<float*>(base + align_up(static_cast<size_t>(c) * c * 2, 256));
+  float2* stats = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(s1) + align_up(static_cast<size_t>(2) * c * 4, 256));
+  LnFold f = {static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, reinterpret_cast<__nv_bfloat16*>(base), s1, s1 + c, c, c};
+  if (folded != nullptr)
+    f = *folded;
+  else if (fold)
+    KFB_TRY(launch_ln_fold_weights(stream, f));
   if (a != nullptr) {
     // t[ch*B+b][i][j] = sum_k A[i][k] B[j][k]
     GemmParams p = {};
@@ -135,17 +152,7 @@ int finish(cudaStream_t stream, const __nv_bfloat16* a, const __nv_bfloat16* b, 
     }
     KFB_TRY(launch_gemm_bf16(stream, oa, ob, p, force_bn, "trimul_contraction"));
   }
-  // LayerNorm_out folded into the output projection: the GEMM reads t as it lies (channel-major, read MN-major), the
-  // epilogue applies the per-position statistics.  The scratch buffer tn holds the folded weights and the statistics.
-  const bool fold = (c % kBK == 0) && posp * static_cast<long long>(c) * 2 >= static_cast<long long>(c) * c * 2 + 256 + 2ll * c * 4 + 256 + posp * 8;
   if (fold) {
-    uint8_t* base = reinterpret_cast<uint8_t*>(tn);
-    __nv_bfloat16* wf = reinterpret_cast<__nv_bfloat16*>(base);
-    float* s1 = reinterpret_cast<float*>(base + align_up(static_cast<size_t>(c) * c * 2, 256));
-    float* s0 = s1 + c;
-    float2* stats = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(s1) + align_up(static_cast<size_t>(2) * c * 4, 256));
-    KFB_TRY(launch_ln_fold_weights(stream, static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, wf, s1, s0, c, c));
-    KFB_TRY(launch_cm_stats(stream, t, stats, posp, c, posp, eps));
     // flat rows when there is no pitch, row by row otherwise (t's rows are np apart, out's n)
     const bool flat = np == n;
     GemmParams p = {};
@@ -165,12 +172,13 @@ int finish(cudaStream_t stream, const __nv_bfloat16* a, const __nv_bfloat16* b, 
     p.stats_pitch = flat ? 0 : np;
     p.resid = resid;
     p.row_stats = stats;
-    p.col_s1 = s1;
-    p.col_s0 = s0;
+    p.stats_eps = eps;
+    p.col_s1 = f.s1;
+    p.col_s0 = f.s0;
     GemmOperandA oa = {t, 1, flat ? 0 : np, flat ? 0 : rnp};
     oa.s_k = posp;
-    GemmOperandB ob = {wf, c, 0};
-    p.b_static = 1;
+    GemmOperandB ob = {f.wf, c, 0};
+    p.b_static = folded != nullptr || a != nullptr;     // a launch lies between the one that folded the weights and this one
     KFB_TRY(launch_gemm_bf16(stream, oa, ob, p, 0, "trimul_out_proj"));
     return KFB_OK;
   }
@@ -345,9 +353,10 @@ KFB_API int kfb_trimul_fwd(int incoming, const void* x, const unsigned char* mas
   KFB_CHECK_ARG(workspace_bytes >= need, "trimul: workspace %zu < %zu bytes", workspace_bytes, need);
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "trimul: workspace must be 256-byte aligned");
   cudaStream_t stream = as_stream(stream_);
-  KFB_TRY(project(stream, incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, w.xn, w.ab, w.gl, batch, n, n, c, eps, dtype));
+  const LnFold fold = {static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, w.wf, w.s, w.s + c, c, c};
+  KFB_TRY(project(stream, incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, w.xn, w.ab, w.gl, batch, n, n, c, eps, dtype, 0, 1, &fold));
   return finish(stream, w.ab, w.ab + static_cast<long long>(c) * batch * n * pitch8(n), n, 0, w.gl, ln_out_w, ln_out_b, w_pout, w.t, w.xn, out,
-                resid, batch, n, n, c, eps, dtype);
+                resid, batch, n, n, c, eps, dtype, &fold);
 }
 
 KFB_API int kfb_trimul_project(const void* x, const unsigned char* mask, const float* ln_in_w, const float* ln_in_b,

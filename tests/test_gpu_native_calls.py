@@ -292,3 +292,18 @@ def test_a_block_with_a_mask_shared_by_its_complexes(dev):
         blk = M.PairformerBlock(128, 384)
     for got, ref in zip(blk(z, s, pm, m), blk(z, s, pm, m.expand(2, n))):
         _check(*err_stats(got.float(), ref.float()), "shared mask")
+
+
+@pytest.mark.parametrize("n,batch,c", [(24, 1, 64), (63, 2, 128), (65, 1, 256), (129, 1, 128), (200, 1, 256), (450, 1, 256)])
+def test_trimul_statistics_of_the_contraction(dev, n, batch, c):
+    """The output projection's LayerNorm statistics, taken by its kernel or (c = 256 beyond L2) by a pass: row counts around the tiles,
+    two, four and eight stages per tile, several column tiles."""
+    from kfold_b200 import functional as F
+    from kfold_b200 import packing
+    import synth
+    z, pm, _ = synth.pair_inputs(n, n, c, batch, pad_frac=0.1)
+    w = synth.trimul_weights(synth._Rng(n), c)
+    zb = z.bfloat16()
+    for direction in ("outgoing", "incoming"):
+        out = F.triangle_multiplication(zb.to(dev), pm.to(dev), packing.pack_trimul(w, dev), direction).float().cpu()
+        _check(*err_stats(out, _oracle_on(dev, O.triangle_multiplication, zb.float(), pm, w, direction)), f"trimul {direction} N={n} C={c}")
