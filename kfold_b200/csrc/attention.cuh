@@ -67,7 +67,8 @@ struct AttnParams {
 };
 
 int launch_attention(cudaStream_t stream, const AttnParams& p);
-int launch_attention_mask_rows(cudaStream_t stream, const AttnParams& p);
+// transposed_too: row_info[batch ..] gets the same of the mask with m_lo and m_k exchanged
+int launch_attention_mask_rows(cudaStream_t stream, const AttnParams& p, bool transposed_too = false);
 int launch_attention_rows(cudaStream_t stream, const AttnParams& p);   // (chosen by launch_attention)
 
 // fp32-accurate mode: q, g and k, v are columns of fp32 row-major buffers (row = batch * L + position, `ld` / `ld_kv`

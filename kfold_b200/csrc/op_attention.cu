@@ -187,30 +187,30 @@ size_t carve_apb_precise(ApbWsPrecise& w, void* base, int batch, int l, int c) {
 
 }  // namespace
 
-extern "C" {
+namespace kfb {
 
-KFB_API size_t kfb_triatt_workspace_bytes_precise(int batch, int n, int c, int heads) {
-  TriattWsPrecise w;
-  return carve_triatt_precise(w, nullptr, batch, n, c, heads);
+static void set_triatt_mask(AttnParams& p, const unsigned char* mask, int n, int ending) {
+  p.mask = mask;
+  p.mask_lo_extent = n;
+  p.m_hi = static_cast<long long>(n) * n;
+  p.m_lo = ending ? 1 : n;
+  p.m_k = ending ? n : 1;
 }
 
-KFB_API size_t kfb_apb_workspace_bytes_precise(int batch, int l, int c) {
-  ApbWsPrecise w;
-  return carve_apb_precise(w, nullptr, batch, l, c);
+bool triatt_scans_mask(int c, int heads, int n, int dtype) { return dtype != KFB_FP32_PRECISE && dpad_of(c / heads) == 32 && n >= 2; }
+
+int triatt_mask_rows(cudaStream_t stream, const unsigned char* mask, int2* rows, int batch, int n) {
+  AttnParams p = {};
+  p.batch = batch * n;
+  p.lk = n;
+  p.row_info = rows;
+  set_triatt_mask(p, mask, n, 0);
+  return launch_attention_mask_rows(stream, p, true);
 }
 
-KFB_API size_t kfb_pair_bias_workspace_bytes_precise(int batch, int n, int c) {
-  return align_up(static_cast<size_t>(batch) * n * n * 6 * c * sizeof(__nv_bfloat16), 256);
-}
-
-KFB_API size_t kfb_triatt_workspace_bytes(int batch, int n, int c, int heads) {
-  TriattWs w;
-  return carve_triatt(w, nullptr, batch, n, c, heads);
-}
-
-KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask, const float* ln_w, const float* ln_b,
-                           const void* w_proj_packed, const void* w_out, void* out, const void* resid, void* workspace,
-                           size_t workspace_bytes, int batch, int n, int c, int heads, float eps, int dtype, void* stream_) {
+int triatt_run(cudaStream_t stream, int ending, const void* x, const unsigned char* mask, const float* ln_w, const float* ln_b,
+               const void* w_proj_packed, const void* w_out, void* out, const void* resid, void* workspace, size_t workspace_bytes, int batch,
+               int n, int c, int heads, float eps, int dtype, int2* mask_rows) {
   KFB_CHECK_ARG(x && mask && w_proj_packed && w_out && out && workspace, "triatt: null pointer");
   KFB_CHECK_ARG(is_dtype(dtype), "triatt: bad dtype %d", dtype);
   KFB_CHECK_ARG(batch >= 1 && n >= 1, "triatt: batch %d N=%d", batch, n);
@@ -223,16 +223,15 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
     const size_t need_p = carve_triatt_precise(wp, workspace, batch, n, c, heads);
     KFB_CHECK_ARG(workspace_bytes >= need_p, "triatt: workspace %zu < %zu bytes", workspace_bytes, need_p);
     KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "triatt: workspace must be 256-byte aligned");
-    return triatt_precise(as_stream(stream_), ending, x, mask, ln_w, ln_b, w_proj_packed, w_out, out, resid, wp, batch, n, c,
+    return triatt_precise(stream, ending, x, mask, ln_w, ln_b, w_proj_packed, w_out, out, resid, wp, batch, n, c,
                           heads, eps);
   }
   const int dp = dpad_of(d), hdp = heads * dp;
-  const bool rows_kernel = dp == 32 && n >= 2;   // see attention_rows.cu
+  const bool rows_kernel = triatt_scans_mask(c, heads, n, dtype);
   TriattWs w;
   const size_t need = carve_triatt(w, workspace, batch, n, c, heads);
   KFB_CHECK_ARG(workspace_bytes >= need, "triatt: workspace %zu < %zu bytes", workspace_bytes, need);
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "triatt: workspace must be 256-byte aligned");
-  cudaStream_t stream = as_stream(stream_);
   const long long nn = static_cast<long long>(n) * n;
   const long long pos = nn * batch;
   const int np = pitch16(n);     // row pitch of V^T and the bias planes; everything else has the caller's n
@@ -287,12 +286,11 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
     p.g = w.qkg; p.ldg = 3 * hdp; p.g_col0 = 2 * hdp;
     p.vt = w.vt; p.ldv = np;
     p.bias = w.bias; p.ldb = np; p.bias_div = n;
-    p.mask = mask;
-    p.mask_lo_extent = n;
-    p.m_hi = nn;
-    p.m_lo = ending ? 1 : n;
-    p.m_k = ending ? n : 1;
-    if (rows_kernel) p.row_info = w.rows;
+    set_triatt_mask(p, mask, n, ending);
+    if (rows_kernel) {
+      p.row_info = mask_rows != nullptr ? mask_rows : w.rows;
+      p.row_info_ready = mask_rows != nullptr;
+    }
     p.out = w.og; p.ldo = c;
     p.tag = "triatt_attention";
     KFB_TRY(launch_attention(stream, p));
@@ -315,6 +313,36 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 0, "triatt_out_proj"));
   }
   return KFB_OK;
+}
+
+}  // namespace kfb
+
+extern "C" {
+
+KFB_API size_t kfb_triatt_workspace_bytes_precise(int batch, int n, int c, int heads) {
+  TriattWsPrecise w;
+  return carve_triatt_precise(w, nullptr, batch, n, c, heads);
+}
+
+KFB_API size_t kfb_apb_workspace_bytes_precise(int batch, int l, int c) {
+  ApbWsPrecise w;
+  return carve_apb_precise(w, nullptr, batch, l, c);
+}
+
+KFB_API size_t kfb_pair_bias_workspace_bytes_precise(int batch, int n, int c) {
+  return align_up(static_cast<size_t>(batch) * n * n * 6 * c * sizeof(__nv_bfloat16), 256);
+}
+
+KFB_API size_t kfb_triatt_workspace_bytes(int batch, int n, int c, int heads) {
+  TriattWs w;
+  return carve_triatt(w, nullptr, batch, n, c, heads);
+}
+
+KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask, const float* ln_w, const float* ln_b,
+                           const void* w_proj_packed, const void* w_out, void* out, const void* resid, void* workspace,
+                           size_t workspace_bytes, int batch, int n, int c, int heads, float eps, int dtype, void* stream) {
+  return triatt_run(as_stream(stream), ending, x, mask, ln_w, ln_b, w_proj_packed, w_out, out, resid, workspace, workspace_bytes, batch, n, c,
+                    heads, eps, dtype, nullptr);
 }
 
 // ------------------------------------------------------------------------------------------------

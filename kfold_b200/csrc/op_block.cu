@@ -23,6 +23,10 @@ size_t operator_bytes(const kfb_pair_block& k, int batch, int n, int precise) {
   return align_up(m, 256);
 }
 
+size_t mask_rows_bytes(const kfb_pair_block& k, int batch, int n) {
+  return k.has_attention ? align_up(sizeof(int2) * 2 * batch * n, 256) : 0;
+}
+
 int bias_pitch(int n, int precise) { return precise ? n : pitch16(n); }
 
 }  // namespace
@@ -30,7 +34,7 @@ int bias_pitch(int n, int precise) { return precise ? n : pitch16(n); }
 extern "C" {
 
 KFB_API size_t kfb_pair_block_workspace_bytes(const kfb_pair_block* blk, int batch, int n, int precise) {
-  size_t m = operator_bytes(*blk, batch, n, precise);
+  size_t m = operator_bytes(*blk, batch, n, precise) + mask_rows_bytes(*blk, batch, n);
   if (blk->has_single)
     m += align_up(static_cast<size_t>(batch) * blk->heads * n * bias_pitch(n, precise) * (precise ? 4 : 2), 256) +
          align_up(static_cast<size_t>(batch) * n * blk->c_s * (precise ? 4 : 2), 256);
@@ -60,16 +64,22 @@ KFB_API int kfb_pair_block_fwd(const kfb_pair_block* blk, const void* z, void* z
                            workspace, ob, batch, n, k.c, k.eps, z_dtype, stream));
     cur = z_out;
   }
+  // the mask scans of both directions in one launch, after the operators' scratch
+  int2* scans = nullptr;
+  if (k.has_attention && triatt_scans_mask(k.c, k.tri_heads, n, z_dtype)) {
+    scans = reinterpret_cast<int2*>(static_cast<uint8_t*>(workspace) + ob);
+    KFB_TRY(triatt_mask_rows(as_stream(stream), pair_mask, scans, batch, n));
+  }
   for (int dir = 0; k.has_attention && dir < 2; ++dir) {
     const kfb_triatt_weights& w = dir ? k.att_end : k.att_start;
-    KFB_TRY(kfb_triatt_fwd(dir, cur, pair_mask, w.ln_w, w.ln_b, w.w_proj, w.w_out, z_out, cur, workspace, ob, batch, n, k.c, k.tri_heads,
-                           k.eps, z_dtype, stream));
+    KFB_TRY(triatt_run(as_stream(stream), dir, cur, pair_mask, w.ln_w, w.ln_b, w.w_proj, w.w_out, z_out, cur, workspace, ob, batch, n, k.c,
+                       k.tri_heads, k.eps, z_dtype, scans != nullptr ? scans + static_cast<long long>(dir) * batch * n : nullptr));
   }
   KFB_TRY(kfb_transition_fwd(cur, k.trans_z.ln_w, k.trans_z.ln_b, k.trans_z.w_swiglu, k.trans_z.w_out, z_out, cur, workspace, ob, pos, k.c,
                              k.hidden_z, k.eps, z_dtype, stream));
   if (!k.has_single) return KFB_OK;
   // single track: its operands come after the operators' scratch
-  uint8_t* extra = static_cast<uint8_t*>(workspace) + ob;
+  uint8_t* extra = static_cast<uint8_t*>(workspace) + ob + mask_rows_bytes(k, batch, n);
   const int pitch = bias_pitch(n, precise);
   void* bias = extra;
   void* an = extra + align_up(static_cast<size_t>(batch) * k.heads * n * pitch * (precise ? 4 : 2), 256);

@@ -63,6 +63,15 @@ struct ApbArgs {
 };
 int apb_run(cudaStream_t stream, const ApbArgs& r);
 
+// kfb_triatt_fwd; mask_rows: what triatt_mask_rows wrote for this direction, or null (the operator scans the mask itself).
+int triatt_run(cudaStream_t stream, int ending, const void* x, const unsigned char* mask, const float* ln_w, const float* ln_b,
+               const void* w_proj_packed, const void* w_out, void* out, const void* resid, void* workspace, size_t workspace_bytes, int batch,
+               int n, int c, int heads, float eps, int dtype, int2* mask_rows);
+// Whether these sizes take the attention kernel that scans the mask, and the scan for both directions in one launch: batch * n entries
+// of the starting node, then those of the ending node.
+bool triatt_scans_mask(int c, int heads, int n, int dtype);
+int triatt_mask_rows(cudaStream_t stream, const unsigned char* mask, int2* rows, int batch, int n);
+
 // bf16 pair bias (kfb_pair_bias_fwd) with bias rows `pitch` elements apart (0: n).
 int pair_bias_run(const void* z, const float* ln_w, const float* ln_b, const void* w, void* bias_out, void* workspace, int batch,
                   int rows, int n, int c, int heads, int transposed, float eps, int dtype, cudaStream_t stream, int pitch);

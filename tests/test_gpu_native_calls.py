@@ -307,3 +307,21 @@ def test_trimul_statistics_of_the_contraction(dev, n, batch, c):
     for direction in ("outgoing", "incoming"):
         out = F.triangle_multiplication(zb.to(dev), pm.to(dev), packing.pack_trimul(w, dev), direction).float().cpu()
         _check(*err_stats(out, _oracle_on(dev, O.triangle_multiplication, zb.float(), pm, w, direction)), f"trimul {direction} N={n} C={c}")
+
+
+@pytest.mark.parametrize("n,batch", [(33, 2), (70, 1)])
+def test_block_with_a_mask_that_is_not_symmetric(dev, n, batch):
+    """Starting and ending node read the pair mask along its two directions; one launch scans both."""
+    from kfold_b200 import modules as M
+    import synth
+    z, pm, m = synth.pair_inputs(n, n, 128, batch)
+    s = synth.single_inputs(n, n, 384, batch)
+    pm = pm & (torch.arange(n)[:, None] + 7 > torch.arange(n) // 2) & (torch.arange(n) != 3)
+    w = synth.pairformer_block_weights(n)
+    blk = M.PairformerBlock().to(dev)
+    blk.load_state_dict(w, strict=True)
+    zb, sb = z.bfloat16(), s.bfloat16()
+    zo, so = blk(zb.to(dev), sb.to(dev), pm.to(dev), m.to(dev))
+    zr, sr = O.pairformer_block(zb.float(), sb.float(), pm, m, w)
+    _check(*err_stats(zo.float().cpu(), zr), "z")
+    _check(*err_stats(so.float().cpu(), sr), "s")
