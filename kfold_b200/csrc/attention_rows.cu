@@ -11,6 +11,13 @@
 //     behind the other groups' products on the one tensor core (910 -> 800);
 //   * R row groups (pair rows with the same bias tile) per CTA, four softmax warps each, that share nothing but the ring of operand
 //     tiles; one thread owns a query row and all 64 keys of a tile, so waits and arrivals come once per 64 keys;
+//   * the groups take turns: at most R - 1 of them do their exponentials at a time, while the other one waits, loads, stores and
+//     arrives.  Left alone, groups that are released by the same stage run in step (clock stamps, R = 3: all of them in 1 640 of a
+//     tile's 2 400 cycles of exponentials, at the MUFU's rate, then all of them in 760 cycles of round trips).  Both halves of a
+//     row's S are loaded before its turn, and one vote per tile decides about the stabiliser.  N = 251: 53.5 -> 48.6 us, 768: 660 ->
+//     655, 2048: 12.3 -> 12.0 ms; 5 x 768 samples of 48-wide heads: 42.5 -> 40.5 us.  (One group at a time: 765 us at N = 768, as one
+//     warp needs 14 cycles an exponential, not 8.  Loads ahead without turns: 700.  An eighth of the exponentials as polynomials on
+//     the FMA pipe: another 0.5 %; a quarter: slower.)
 //   * the stabiliser is zero unless a row needs another one: logits are in log2 units, and exp2(x) of a row whose first keys' sum
 //     lies in [2^-40, 2^100] and whose later sums stay below 2^100 neither overflows nor loses accuracy, so the common path
 //     subtracts nothing and keeps no maximum;
@@ -19,9 +26,9 @@
 //   * the key mask costs nothing where it masks nothing: a row's first masked and last valid key come from a scan kernel, the rank-1
 //     mask product is issued for the tiles that hold masked keys, and tiles after the last valid key are skipped.
 // N = 768 (4 heads): 1.15 -> 0.71 ms; N = 2048: 18.3 -> 11.9 ms (the exponentials alone: 0.40, 7.6).  The MUFU is busy 65 % of the
-// time; what is left are the conversions and sums between the exponentials and the latency of loads from and stores to tensor memory.
-// Warps: 4 g .. 4 g + 3 softmax and output of row group g (a warp reads the tensor-memory lanes warp % 4); then the TMA producer, the
-// mask warp, and one MMA-issuing warp per group.
+// time; without exponentials a tile still takes 660 of 790 cycles, and neither the bias nor the value products change that.
+// Warps: 4 g .. 4 g + 3 softmax and output of row group g (a warp reads the tensor-memory lanes warp % 4); then the TMA producer, which
+// also writes the mask operands, and one MMA-issuing warp per group.
 // Tensor memory per row group: two S tiles, 64 fp32 columns each, overwritten in place by their P (64 bf16 = 32 columns), and O, 32
 // fp32 columns.
 #include <cuda_bf16.h>
@@ -48,7 +55,7 @@ constexpr int kEyeBytes = (48 + 16 + 48) * 32; // a 16 x 16 identity (times a fa
 template <int R, int D>
 struct RowsCfg {
   static constexpr int kSoftWarps = 4 * R;
-  static constexpr int kThreads = 32 * (kSoftWarps + 2 + R);
+  static constexpr int kThreads = 32 * (kSoftWarps + 1 + R);
   static constexpr int kQBytes = kQ * D * 2, kKBytes = kT * D * 2, kVBytes = D * kT * 2;
   static constexpr int kStages = D == 64 ? 3 : (R == 3 ? 4 : 5);      // ring of tiles: bias, and K, V^T of all row groups
   static constexpr int kStageBytes = kBiasBytes + R * (kKBytes + kVBytes);
@@ -137,10 +144,12 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   uint64_t* m_full = p_ready + 2 * R;                 // [R][slots]: ring of mask operands
   uint64_t* m_empty = m_full + kMaskSlots * R;    // [R][slots]
   uint64_t* pv_done = m_empty + kMaskSlots * R;   // [R][2]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(pv_done + 2 * R);
+  uint64_t* turn = pv_done + 2 * R;               // [R][2 tiles][4]: a warp of the group has done a tile's exponentials
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(turn + 8 * R);
+  static_assert((2 * kStages + 4 + 6 * R + 2 * kMaskSlots * R + 8 * R) * 8 + 4 <= 512, "barriers");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  constexpr int kProducer = Cfg::kSoftWarps, kMasker = kProducer + 1, kMma = kProducer + 2;
+  constexpr int kProducer = Cfg::kSoftWarps, kMma = kProducer + 1;
   const AttnParams& a = p.a;
 
   if (threadIdx.x == 0) {
@@ -163,6 +172,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       ptx::mbar_init(&p_ready[2 * i + 1], 4);
       ptx::mbar_init(&pv_done[2 * i], 1);
       ptx::mbar_init(&pv_done[2 * i + 1], 1);
+      for (int w = 0; w < 8; ++w) ptx::mbar_init(&turn[8 * i + w], 1);
     }
     for (int i = 0; i < kMaskSlots * R; ++i) {
       ptx::mbar_init(&m_full[i], 1);
@@ -206,22 +216,34 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
   grid_dependency_enter();
 
   if (warp == kProducer) {
-    // ---------------------------------------------------------------- TMA producer
-    if (ptx::elect_one()) {
-      bool ok = true;
-      int st = 0;
-      uint32_t par = 0, k = 0;     // ring position; items so far
-      for (int item = blockIdx.x; ok && item < p.items; item += gridDim.x) {
-        const Item<R> it = load_item<R>(p, item);
-        if (it.tiles == 0) continue;
-        const uint32_t qbuf = k & 1;
-        if (!ptx::mbar_wait(&q_empty[qbuf], ((k >> 1) & 1) ^ 1, 301)) break;
+    // ---------------------------------------------------------------- TMA loads, and the mask operands of the tiles that hold masked
+    // or absent keys.  (One warp for both: a 17th would leave the softmax warps 96 registers, as one scheduler would hold five.  A
+    // tile's mask slot is free when the S before it has been computed, which is when the stage of the next tile is, too.)
+    bool ok = true;
+    int st = 0;
+    uint32_t par = 0, k = 0;        // ring position; items so far
+    uint32_t uses[R];               // mask ring position of each group
+#pragma unroll
+    for (int g = 0; g < R; ++g) uses[g] = 0;
+    for (int item = blockIdx.x; ok && item < p.items; item += gridDim.x) {
+      const Item<R> it = load_item<R>(p, item);
+      if (it.tiles == 0) continue;
+      const uint32_t qbuf = k & 1;
+      ok = __all_sync(0xffffffffu, ptx::mbar_wait(&q_empty[qbuf], ((k >> 1) & 1) ^ 1, 301));
+      if (!ok) break;
+      if (ptx::elect_one()) {
         ptx::mbar_expect_tx(&q_full[qbuf], R * kQBytes);
         for (int g = 0; g < R; ++g)   // (a row that does not exist reads another one or zeros: its results are dropped)
           ptx::tma_load_3d(s_q + (qbuf * R + g) * kQBytes, &tm_q, &q_full[qbuf], a.q_col0 + it.h * kD, it.qb * kQ, it.b0 + g);
-        const int bias_z = a.bias_head_major > 0 ? it.h * a.bias_head_major + it.bias_b : it.bias_b * a.heads + it.h;
-        for (int t = 0; t < it.tiles; ++t) {
-          if (!ptx::mbar_wait(&stage_empty[st], par ^ 1, 302)) { ok = false; break; }
+      }
+      const int bias_z = a.bias_head_major > 0 ? it.h * a.bias_head_major + it.bias_b : it.bias_b * a.heads + it.h;
+      int from = it.first[0];       // tiles before the first masked key of every row need no mask operand
+#pragma unroll
+      for (int g = 1; g < R; ++g) from = min(from, it.first[g]);
+      for (int t = 0; t < it.tiles; ++t) {
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&stage_empty[st], par ^ 1, 302));
+        if (!ok) break;
+        if (ptx::elect_one()) {
           uint8_t* dst = s_stage + st * kStageBytes;
           ptx::mbar_expect_tx(&stage_full[st], kStageBytes);
           for (int g = 0; g < R; ++g) {
@@ -230,10 +252,36 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
             ptx::tma_load_3d(kv + kKBytes, &tm_v, &stage_full[st], t * kT, it.h * kD, it.b0 + g);
           }
           ptx::tma_load_3d(dst, &tm_b, &stage_full[st], t * kT, it.qb * kQ, bias_z);
-          if (++st == kStages) { st = 0; par ^= 1u; }
         }
-        ++k;
+        if (++st == kStages) { st = 0; par ^= 1u; }
+        if (t * kT + kT <= from) continue;
+#pragma unroll
+        for (int g = 0; g < R; ++g) {
+          if (!ok || t * kT + kT <= it.first[g]) continue;
+          const int b = it.b0 + min(g, it.rows - 1);
+          const int b_hi = b / a.mask_lo_extent, b_lo = b - b_hi * a.mask_lo_extent;
+          const unsigned char* mrow = a.mask + static_cast<long long>(b_hi) * a.m_hi + static_cast<long long>(b_lo) * a.m_lo;
+          uint32_t v[2];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            const int key = t * kT + lane + 32 * i;
+            const float m = key >= a.lk ? kAbsent : (mrow[static_cast<long long>(key) * a.m_k] ? 0.f : kMasked);
+            v[i] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(m)));
+          }
+          const uint32_t slot = uses[g] % kMaskSlots, mpar = (uses[g] / kMaskSlots) & 1;
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&m_empty[g * kMaskSlots + slot], mpar ^ 1, 308));
+          if (!ok) continue;
+          uint8_t* dst = s_mask + (g * kMaskSlots + slot) * kMaskBytes;
+#pragma unroll
+          for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(dst + ptx::noswizzle_row_offset(lane + 32 * i)) = make_uint4(v[i], 0, 0, 0);
+          ptx::fence_proxy_async_smem();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive(&m_full[g * kMaskSlots + slot]);
+          ++uses[g];
+        }
+        if (!ok) break;
       }
+      ++k;
     }
   } else if (warp >= kMma) {
     // ---------------------------------------------------------------- MMA issue of row group g
@@ -328,44 +376,6 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
         }
       }
     }
-  } else if (warp == kMasker) {
-    // ---------------------------------------------------------------- mask operands of the tiles that hold masked or absent keys
-    bool ok = true;
-    uint32_t uses[R];               // ring position of each group
-#pragma unroll
-    for (int g = 0; g < R; ++g) uses[g] = 0;
-    for (int item = blockIdx.x; ok && item < p.items; item += gridDim.x) {
-      const Item<R> it = load_item<R>(p, item);
-      int from = it.first[0];       // tiles before the first masked key of every row need no operand
-#pragma unroll
-      for (int g = 1; g < R; ++g) from = min(from, it.first[g]);
-      for (int t = from / kT; ok && t < it.tiles; ++t) {
-#pragma unroll
-        for (int g = 0; g < R; ++g) {
-          if (!ok || t * kT + kT <= it.first[g]) continue;
-          const int b = it.b0 + min(g, it.rows - 1);
-          const int b_hi = b / a.mask_lo_extent, b_lo = b - b_hi * a.mask_lo_extent;
-          const unsigned char* mrow = a.mask + static_cast<long long>(b_hi) * a.m_hi + static_cast<long long>(b_lo) * a.m_lo;
-          uint32_t v[2];
-#pragma unroll
-          for (int i = 0; i < 2; ++i) {
-            const int key = t * kT + lane + 32 * i;
-            const float m = key >= a.lk ? kAbsent : (mrow[static_cast<long long>(key) * a.m_k] ? 0.f : kMasked);
-            v[i] = static_cast<uint32_t>(__bfloat16_as_ushort(__float2bfloat16_rn(m)));
-          }
-          const uint32_t slot = uses[g] % kMaskSlots, par = (uses[g] / kMaskSlots) & 1;
-          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&m_empty[g * kMaskSlots + slot], par ^ 1, 308));
-          if (!ok) continue;
-          uint8_t* dst = s_mask + (g * kMaskSlots + slot) * kMaskBytes;
-#pragma unroll
-          for (int i = 0; i < 2; ++i) *reinterpret_cast<uint4*>(dst + ptx::noswizzle_row_offset(lane + 32 * i)) = make_uint4(v[i], 0, 0, 0);
-          ptx::fence_proxy_async_smem();
-          __syncwarp();
-          if (lane == 0) ptx::mbar_arrive(&m_full[g * kMaskSlots + slot]);
-          ++uses[g];
-        }
-      }
-    }
   } else {
     // ---------------------------------------------------------------- softmax and output of row group g
     const int g = warp >> 2, quad = warp & 3;
@@ -377,67 +387,56 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
     float s_cur = 0.f, l_run = 0.f;   // the row's stabiliser and sum
     bool shifted = false;             // some lane of the warp has a stabiliser other than zero
 
-    // half `half` of tile t: S columns 32 half .. + 31 become P columns 16 half .. + 15
-    auto do_half = [&](auto half_c, int t, uint32_t tmem_s) {
-      constexpr int half = decltype(half_c)::value;
-      uint32_t x[32], out[16];
-      ptx::tmem_ld_32x32b_x32(tmem_s + half * 32, x);
-      ptx::tmem_ld_wait();
-      auto run = [&](auto sub) -> float {
-        float sum[4] = {0.f, 0.f, 0.f, 0.f};
+    // exponentials of 32 logits of the row, packed in pairs, and their sum
+    auto exps = [&](auto sub, const uint32_t (&x)[32], uint32_t (&out)[16]) -> float {
+      float sum[4] = {0.f, 0.f, 0.f, 0.f};
 #pragma unroll
-        for (int i = 0; i < 32; i += 2) {
-          float y0 = __uint_as_float(x[i]), y1 = __uint_as_float(x[i + 1]);
-          if constexpr (decltype(sub)::value) { y0 -= s_cur; y1 -= s_cur; }
-          const float p0 = ex2(y0), p1 = ex2(y1);
-          sum[i & 2] += p0;
-          sum[(i & 2) + 1] += p1;
-          out[i >> 1] = pack_bf16x2(p0, p1);
-        }
-        return (sum[0] + sum[1]) + (sum[2] + sum[3]);
-      };
-      float l = shifted ? run(std::true_type()) : run(std::false_type());
-      const bool fresh = half == 0 && t == 0;        // nothing of this row has been added yet
-      const bool mine = !(l < kHighSum) || (fresh && l < kLowSum);
-      if (__any_sync(0xffffffffu, mine)) {
-        // rare: move those rows' stabiliser to the maximum of these keys, and the accumulator, the first half's P and the sum with it
-        float mx = -INFINITY;
+      for (int i = 0; i < 32; i += 2) {
+        float y0 = __uint_as_float(x[i]), y1 = __uint_as_float(x[i + 1]);
+        if constexpr (decltype(sub)::value) { y0 -= s_cur; y1 -= s_cur; }
+        const float p0 = ex2(y0), p1 = ex2(y1);
+        sum[i & 2] += p0;
+        sum[(i & 2) + 1] += p1;
+        out[i >> 1] = pack_bf16x2(p0, p1);
+      }
+      return (sum[0] + sum[1]) + (sum[2] + sum[3]);
+    };
+    // rare: a tile whose sums ask for another stabiliser (S is still whole).  It moves to the row's maximum of this tile's keys, and
+    // the accumulator and the sum with it; writes P.
+    auto rescale = [&](int t, uint32_t tmem_s, bool mine) {
+      float mx = -INFINITY;
+      uint32_t x[32], out[16];
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {
         ptx::tmem_ld_32x32b_x32(tmem_s + half * 32, x);
         ptx::tmem_ld_wait();
 #pragma unroll
         for (int i = 0; i < 32; ++i) mx = fmaxf(mx, __uint_as_float(x[i]));
-        const float s_new = mine ? (fresh ? mx : fmaxf(mx, s_cur)) : s_cur;
-        const float alpha = ex2(s_cur - s_new);      // 1 for the rows whose stabiliser stays
-        if (t > 0) {
-          if (!__all_sync(0xffffffffu, ptx::mbar_wait(&pv_done[g * 2 + ((n - 1) & 1)], ((n - 1) >> 1) & 1, 310))) ok = false;
-          ptx::tc_fence_after_sync();
+      }
+      const float s_new = mine ? (t == 0 ? mx : fmaxf(mx, s_cur)) : s_cur;
+      const float alpha = ex2(s_cur - s_new);      // 1 for the rows whose stabiliser stays
+      if (t > 0) {
+        if (!__all_sync(0xffffffffu, ptx::mbar_wait(&pv_done[g * 2 + ((n - 1) & 1)], ((n - 1) >> 1) & 1, 310))) ok = false;
+        ptx::tc_fence_after_sync();
 #pragma unroll 1
-          for (int c = 0; c < kD / 16; ++c) {
-            uint32_t o16[16];
-            ptx::tmem_ld_32x32b_x16(tmem_o + c * 16, o16);
-            ptx::tmem_ld_wait();
-#pragma unroll
-            for (int i = 0; i < 16; ++i) o16[i] = __float_as_uint(__uint_as_float(o16[i]) * alpha);
-            ptx::tmem_st_32x32b_x16(tmem_o + c * 16, o16);
-          }
-        }
-        if (half == 1) {
-          uint32_t o16[16];
-          ptx::tmem_st_wait();
-          ptx::tmem_ld_32x32b_x16(tmem_s, o16);
+        for (int c = 0; c < kD / 16; ++c) {
+          ptx::tmem_ld_32x32b_x16(tmem_o + c * 16, out);
           ptx::tmem_ld_wait();
 #pragma unroll
-          for (int i = 0; i < 16; ++i)
-            o16[i] = pack_bf16x2(__uint_as_float(o16[i] << 16) * alpha, __uint_as_float(o16[i] & 0xffff0000u) * alpha);
-          ptx::tmem_st_32x32b_x16(tmem_s, o16);
+          for (int i = 0; i < 16; ++i) out[i] = __float_as_uint(__uint_as_float(out[i]) * alpha);
+          ptx::tmem_st_32x32b_x16(tmem_o + c * 16, out);
         }
-        if (!fresh) l_run *= alpha;
-        s_cur = s_new;
-        shifted = __any_sync(0xffffffffu, s_cur != 0.f);
-        l = run(std::true_type());
+        l_run *= alpha;
       }
-      l_run += l;
-      ptx::tmem_st_32x32b_x16(tmem_s + half * 16, out);
+      s_cur = s_new;
+      shifted = __any_sync(0xffffffffu, s_cur != 0.f);
+#pragma unroll 1
+      for (int half = 0; half < 2; ++half) {       // (P of the second half goes over S columns that the first has read)
+        ptx::tmem_ld_32x32b_x32(tmem_s + half * 32, x);
+        ptx::tmem_ld_wait();
+        l_run += exps(std::true_type(), x, out);
+        ptx::tmem_st_32x32b_x16(tmem_s + half * 16, out);
+      }
     };
 
     for (int item = blockIdx.x; ok && item < p.items; item += gridDim.x) {
@@ -445,15 +444,36 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
       s_cur = 0.f;
       l_run = 0.f;
       shifted = false;
+      // S columns 32 h .. 32 h + 31 become P columns 16 h .. 16 h + 15.
 #pragma unroll 1
       for (int t = 0; t < it.tiles; ++t) {
+        const uint32_t tmem_s = tmem_g + (n & 1) * kT;
         ok = __all_sync(0xffffffffu, ptx::mbar_wait(&s_full[g * 2 + (n & 1)], (n >> 1) & 1, 309));
         if (!ok) break;
-        const uint32_t tmem_s = tmem_g + (n & 1) * kT;
         ptx::tc_fence_after_sync();
-        do_half(std::integral_constant<int, 0>(), t, tmem_s);
-        do_half(std::integral_constant<int, 1>(), t, tmem_s);
-        if (!ok) break;
+        uint32_t xa[32], xb[32], oa[16], ob[16];
+        ptx::tmem_ld_32x32b_x32(tmem_s, xa);
+        ptx::tmem_ld_32x32b_x32(tmem_s + 32, xb);
+        ptx::tmem_ld_wait();
+        // the groups take turns (see above): in the order of tiles and groups, this one after the (R - 1)-th before it
+        if (g == R - 1 || n > 0) {
+          const uint32_t m = g == R - 1 ? n : n - 1;
+          ok = __all_sync(0xffffffffu, ptx::mbar_wait(&turn[((g + 1) % R * 2 + (m & 1)) * 4 + quad], (m >> 1) & 1, 311));
+          if (!ok) break;
+        }
+        const float l0 = shifted ? exps(std::true_type(), xa, oa) : exps(std::false_type(), xa, oa);
+        const float l1 = shifted ? exps(std::true_type(), xb, ob) : exps(std::false_type(), xb, ob);
+        if (lane == 0) ptx::mbar_arrive(&turn[(g * 2 + (n & 1)) * 4 + quad]);
+        const bool mine = !(l0 < kHighSum) || !(l1 < kHighSum) || (t == 0 && l0 + l1 < kLowSum);
+        if (__any_sync(0xffffffffu, mine)) {
+          rescale(t, tmem_s, mine);
+          if (!ok) break;
+        } else {
+          l_run += l0;
+          l_run += l1;
+          ptx::tmem_st_32x32b_x16(tmem_s, oa);
+          ptx::tmem_st_32x32b_x16(tmem_s + 16, ob);
+        }
         ptx::tmem_st_wait();
         ptx::tc_fence_before_sync();
         __syncwarp();
