@@ -62,21 +62,34 @@ int sm_count();  // multiprocessors of the current device (cached per device)
 // 310 -> 454 us; the bf16 LayerNorm of a 768-token pair tensor 152 -> 187 us).
 // Every kernel launched this way executes griddepcontrol.wait before it touches memory that the stream's earlier work wrote or
 // reads, and griddepcontrol.launch_dependents only after that wait: what lies two or more kernels back is then always complete.
+// cluster: CTAs per thread-block cluster (along x).
 template <typename... KArgs, typename... Args>
-inline int launch_kernel(cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
+inline int launch_kernel_clustered(cudaStream_t stream, void (*kernel)(KArgs...), unsigned cluster, dim3 grid, dim3 block, size_t smem,
+                                   Args&&... args) {
   cudaLaunchConfig_t cfg = {};
   cfg.gridDim = grid;
   cfg.blockDim = block;
   cfg.dynamicSmemBytes = smem;
   cfg.stream = stream;
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchAttribute attr[2];
   cfg.attrs = attr;
   const unsigned long long blocks = static_cast<unsigned long long>(grid.x) * grid.y * grid.z, sms = sm_count();
-  cfg.numAttrs = blocks <= sms || (blocks <= 4 * sms && (smem <= 4096 || smem > 114 * 1024)) ? 1 : 0;
+  if (blocks <= sms || (blocks <= 4 * sms && (smem <= 4096 || smem > 114 * 1024))) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[cfg.numAttrs++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[cfg.numAttrs].id = cudaLaunchAttributeClusterDimension;
+    attr[cfg.numAttrs].val.clusterDim.x = cluster;
+    attr[cfg.numAttrs].val.clusterDim.y = 1;
+    attr[cfg.numAttrs++].val.clusterDim.z = 1;
+  }
   KFB_CUDA(cudaLaunchKernelEx(&cfg, kernel, KArgs(args)...));
   return KFB_OK;
+}
+template <typename... KArgs, typename... Args>
+inline int launch_kernel(cudaStream_t stream, void (*kernel)(KArgs...), dim3 grid, dim3 block, size_t smem, Args&&... args) {
+  return launch_kernel_clustered(stream, kernel, 1, grid, block, smem, static_cast<Args&&>(args)...);
 }
 
 #ifdef __CUDACC__

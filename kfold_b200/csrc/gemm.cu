@@ -11,21 +11,38 @@
 
 namespace kfb {
 
-template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false>
+template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false, bool PAIR = false>
 static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* tout,
                           const GemmParams& p, const char* tag) {
-  using Cfg = GemmCfg<BN>;
+  using Cfg = GemmCfg<BN, PAIR>;
+  constexpr auto kernel = gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP, STATS, PAIR>;
+  constexpr int threads = AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads;
   static std::once_flag once[64];
+  static int resident[64];      // tiles in flight: CTAs, or pairs of them, that the device holds at once
   int dev = 0;
   KFB_CUDA(cudaGetDevice(&dev));
   cudaError_t attr_err = cudaSuccess;
   std::call_once(once[dev & 63], [&] {
-    attr_err = cudaFuncSetAttribute(gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP, STATS>, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                    Cfg::kSmemBytes);
+    attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
+    resident[dev & 63] = sm_count();
+    if (PAIR && attr_err == cudaSuccess) {     // (a multiprocessor without a neighbour to pair with stays idle)
+      cudaLaunchAttribute attr[1];
+      attr[0].id = cudaLaunchAttributeClusterDimension;
+      attr[0].val.clusterDim.x = 2;
+      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+      cudaLaunchConfig_t cfg = {};
+      cfg.gridDim = sm_count() / 2 * 2;
+      cfg.blockDim = threads;
+      cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+      cfg.attrs = attr;
+      cfg.numAttrs = 1;
+      attr_err = cudaOccupancyMaxActiveClusters(&resident[dev & 63], kernel, &cfg);
+    }
   });
   KFB_CUDA(attr_err);
+  KFB_CHECK_ARG(resident[dev & 63] > 0, "GEMM: the device holds no CTA pair");
   const int total = p.num_m_tiles * p.num_n_tiles;
-  const int grid = total < sm_count() ? total : sm_count();
+  const int grid = total < resident[dev & 63] ? total : resident[dev & 63];     // (pairs count as one)
   GemmParams q = p;
   {
     // the persistent loops step by the grid size: its digits in the (n tile, row block, outer, batch) index
@@ -38,10 +55,18 @@ static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUte
   }
   {
     LaunchScope scope(stream, tag);
-    KFB_TRY(launch_kernel(stream, gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP, STATS>, grid,
-                          AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads, Cfg::kSmemBytes, ta, tb, tout[0], tout[1], tout[2], q));
+    KFB_TRY(launch_kernel_clustered(stream, kernel, PAIR ? 2 : 1, PAIR ? 2 * grid : grid, threads, Cfg::kSmemBytes, ta, tb, tout[0], tout[1],
+                                    tout[2], q));
   }
   return KFB_OK;
+}
+
+static int launch_pair(cudaStream_t stream, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* tout, GemmParams p, const char* tag) {
+  using Cfg = GemmCfg<256, true>;
+  p.stages = Cfg::stages_for(p.aux ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes : p.glu ? Cfg::kGluStagingBytes : Cfg::kStagingBytes);
+  if (p.glu) return launch_variant<256, true, false, false, false, false, true>(stream, ta, tb, tout, p, tag);
+  if (p.aux) return launch_variant<256, false, true, false, false, false, true>(stream, ta, tb, tout, p, tag);
+  return launch_variant<256, false, false, false, false, false, true>(stream, ta, tb, tout, p, tag);
 }
 
 template <int BN>
@@ -101,6 +126,27 @@ static int narrow_tile(const GemmParams& p, int bn) {
   return pick;
 }
 
+// CTA pairs (PAIR in gemm.cuh) pay where the main loop is long enough to hide the epilogue of a tile twice as wide and the tiles are at
+// least a wave of pairs.  Measured, one CTA -> pair: triangle contraction at 768 tokens 108 -> 99 us (128 channels), 201 -> 180 (256);
+// SwiGLU of 256 channels at 768 x 768 rows 585 -> 472, its output projection (K = 1 024) 362 -> 318; token transformer, 5 x 768 rows of
+// 768: projection 35 -> 29, SwiGLU 24.5 -> 22.5.  The other side of the lines: SwiGLU of 128 channels (two K blocks) 106 -> 107; gate
+// projection of 256 (four, plain) 105 -> 109; conditioning table (six, plain) 100 -> 104; contraction at 333 tokens (three row blocks, a
+// quarter of the pairs' work padding) 49.7 -> 51.6; float32 output projections with gate and residual 22.4 -> 23.5.
+static bool pair_tile(const GemmParams& p, int bn) {
+  if (p.precise || bn < 128 || p.n_cols < 256 || p.glu == GLU_SIGMOID) return false;
+  const int num_k = cdiv(p.k_extent, kBK), pairs = cdiv(p.n_blocks, 2);
+  if (num_k < (p.glu ? 4 : 8) || (2 * pairs - p.n_blocks) * 8 > p.n_blocks) return false;
+  if (2ll * pairs * p.o_extent * p.batch * cdiv(p.n_cols, 256) < sm_count()) return false;
+  for (int i = 0; i < p.nseg; ++i) {
+    const EpiSeg& sg = p.seg[i];
+    const bool channel_major = sg.s_n == 1 && sg.s_col != 1;      // whole swapped tiles, behind the row-major segments
+    if (sg.col_begin % 256 != 0 || sg.out_fp32) return false;
+    if (channel_major && (p.glu || ((p.mask_segs >> i) & 1) || (i == 0 && (p.gate != nullptr || p.resid != nullptr)))) return false;
+    if (!channel_major && (sg.s_col != 1 || (i > 0 && p.seg[i - 1].s_n == 1 && p.seg[i - 1].s_col != 1))) return false;
+  }
+  return true;
+}
+
 static long long* g_trace_buf = nullptr;
 static char g_trace_tag[64] = "";
 void set_gemm_trace(long long* device_buffer, const char* tag) {
@@ -118,6 +164,8 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
   if (bn == 0) bn = p.n_cols >= 256 ? 256 : (p.n_cols > 64 ? 128 : 64);
   if (p.precise && bn > 128) bn = 128;  // the fp32-accurate variant keeps four accumulators in tensor memory
   if (a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0 && (p.precise ? !p.glu : p.glu != GLU_SIGMOID)) bn = narrow_tile(p, bn);
+  p.pair = pair_tile(p, bn) && a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0;
+  if (p.pair) bn = 256;
   // One row-major float32 segment with a gate and / or a residual (the output projections of the sampler's float32 activation
   // stream): 128-column tiles whose epilogue moves gate, residual and output through per-warp shared-memory tiles.
   p.xpose = 0;
@@ -135,6 +183,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
       if (bn > 128) bn = 128;
     }
   }
+  if (p.xpose) p.pair = 0;
   // Gate / residual prefetch and staged output: one row-major bf16 segment of whole 32-column chunks, aligned strides.  Two buffers
   // of 128-column tiles (each set is loaded while the one before is in the epilogue); with a long K and the residual only, one
   // buffer of 256-column tiles: its load hides behind the K loop, and A is read once.
@@ -160,6 +209,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
       }
     }
   }
+  if (bn != 256) p.pair = 0;
   KFB_CHECK_ARG(bn == 32 || bn == 64 || bn == 128 || bn == 256, "unsupported BN %d", bn);
   // LayerNorm statistics of K-outer rows: taken by the kernel itself where it has the warps for it, by a pass before it otherwise.  The
   // statistics hold a stage of the ring a little longer, which costs little where a tile is few stages or comes from L2 (768 x 768 rows
@@ -175,6 +225,10 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
   for (int i = 0; i < p.nseg; ++i) KFB_CHECK_ARG(p.seg[i].col_begin % 32 == 0, "segment start must be a multiple of 32");
   p.trace = (g_trace_buf != nullptr && strcmp(g_trace_tag, tag) == 0) ? g_trace_buf : nullptr;
   p.num_n_tiles = cdiv(p.n_cols, bn);
+  if (p.pair) {
+    p.n_blocks = cdiv(p.n_blocks, 2);
+    p.num_m_tiles = p.n_blocks * p.o_extent * p.batch;
+  }
 
   CUtensorMap ta, tb;
   p.a_mn_major = a.s_k != 0 ? 1 : 0;
@@ -231,7 +285,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
     const uint64_t dims[4] = {(uint64_t)p.k_extent, (uint64_t)inner, (uint64_t)(p.n_cols / inner),
                               (uint64_t)(p.b_batched ? p.batch : 1)};
     const uint64_t str[3] = {(uint64_t)b.s_col * 2, (uint64_t)b.s_col_hi * 2, (uint64_t)b.s_b * 2};
-    const uint32_t box[4] = {kBK, (uint32_t)(p.glu && bn < 256 ? bn / 2 : bn), 1, 1};
+    const uint32_t box[4] = {kBK, (uint32_t)(p.pair || (p.glu && bn < 256) ? bn / 2 : bn), 1, 1};
     KFB_TRY(make_tmap(&tb, b.ptr, 2, 4, dims, str, box, 128));
     }
   }
@@ -262,10 +316,10 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
   // trailing channel-major bf16 segments that start on a tile boundary are computed in the swapped orientation as well
   // (plain BN = 128 kernel): the threads then store runs of consecutive positions directly
   p.swap_col_begin = INT_MAX;
-  if (bn == 128 && !p.glu && !p.precise && !p.a_mn_major) {
+  if ((bn == 128 || p.pair) && !p.glu && !p.precise && !p.a_mn_major) {
     for (int i = p.nseg - 1; i >= 0; --i) {
       const EpiSeg& sg = p.seg[i];
-      const bool cm = sg.s_n == 1 && sg.s_col != 1 && !sg.out_fp32 && !sg.split && sg.col_begin % 128 == 0 &&
+      const bool cm = sg.s_n == 1 && sg.s_col != 1 && !sg.out_fp32 && !sg.split && sg.col_begin % bn == 0 &&
                       !((p.mask_segs >> i) & 1) && (i > 0 || (p.gate == nullptr && p.resid == nullptr));
       if (!cm) break;
       p.swap_col_begin = sg.col_begin;
@@ -299,7 +353,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
   // full tiles of one row-major bf16 segment of the plain BN = 128 kernel leave through shared memory and a TMA store
   p.rm_seg = -1;
   p.rm_slot = 0;
-  const bool rm_plain = bn == 128 && !p.glu;
+  const bool rm_plain = (bn == 128 || p.pair) && !p.glu;
   const bool rm_glu = bn == 256 && p.glu && !p.swap;      // the GLU kernel: 128 output columns per tile
   if ((rm_plain || rm_glu) && !p.precise && !p.aux && !p.a_mn_major && next_slot == 0) {
     for (int i = 0; i < p.nseg; ++i) {
@@ -318,6 +372,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
       break;
     }
   }
+  if (p.pair) return launch_pair(stream, ta, tb, tout, p, tag);
   switch (bn) {
     case 32: return launch_bn<32>(stream, ta, tb, tout, p, tag);
     case 64: return launch_bn<64>(stream, ta, tb, tout, p, tag);

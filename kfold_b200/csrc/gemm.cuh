@@ -71,6 +71,7 @@ struct GemmParams {
   float stats_eps;                //   their epsilon
   const float* col_s1;            //   (mean, rstd) per flat row; col_s1 = sum_k W'[col][k], col_s0 = sum_k beta[k] W[col][k]
   const float* col_s0;            //   with W' = gamma * W the matrix actually multiplied (applied before gate / residual)
+  int pair;                       // launcher: CTA pairs (see PAIR); n_blocks then counts the pairs' row blocks of 256
   int swap_col_begin;             // launcher (BN = 128, plain epilogue): tiles whose first column is >= this hold channel-major
                                   // segments only and are computed in the swapped orientation too (INT_MAX: none)
   int nseg;
@@ -104,10 +105,11 @@ static constexpr int kAuxThreads = kGemmThreads + 32;  // the AUX variant's last
 static constexpr int kStatsThreads = 64;               // the STATS variant's two warps after it: two rows of the tile per thread
 static constexpr int kStatsBytes = kBM * 8;            // (mean, rstd) of a tile's rows
 
-template <int BN>
+template <int BN, bool PAIR = false>
 struct GemmCfg {
   static constexpr int kAStage = kBM * kBK * 2;
-  static constexpr int kBStage = BN * kBK * 2;
+  static constexpr int kBRows = PAIR ? BN / 2 : BN;        // rows of the B tile that this CTA loads
+  static constexpr int kBStage = kBRows * kBK * 2;
   static constexpr int kStageBytes = kAStage + kBStage;
   static constexpr int kMaxStages = 8;
   // per group of 4 epilogue warps: 2 slabs of [32 channels][128 rows] bf16 -- or, in the BN = 128 kernel, two whole row-major
@@ -115,7 +117,7 @@ struct GemmCfg {
   static constexpr int kSlabBytes = (kEpiWarps / 4) * 2 * 32 * kBM * 2;
   static constexpr int kRowTileBytes = kBM * 128 * 2;
   static constexpr int kXposeBytes = kEpiWarps * 6144;     // per-warp tiles of the float32 gate / residual route
-  static constexpr int kStagingBytes = (BN == 128) ? 2 * kRowTileBytes : (BN < 128 ? kXposeBytes : kSlabBytes);
+  static constexpr int kStagingBytes = (BN == 128 || PAIR) ? 2 * kRowTileBytes : (BN < 128 ? kXposeBytes : kSlabBytes);
   // the GLU kernel at BN = 256 writes 128 output columns per tile: the same two row-major tile buffers
   static constexpr int kGluStagingBytes = (BN == 256) ? 2 * kRowTileBytes : kStagingBytes;
   // swapped-orientation GLU kernel (BN = 256): the tile's position mask (1 KB, two accumulators) and two whole
@@ -317,25 +319,33 @@ __device__ __forceinline__ void tile_advance(TileIdx& t, const GemmParams& p) {
 //         D[channel][position] = W[channel][:] . X[position][:], i.e. the 128 value rows and the 128 gate rows of the weight
 //         tile are the M operands of two N=128 MMAs and the 128 positions are the N operand.  A thread then holds
 //         consecutive positions of ONE channel and writes them with 32-byte stores: no transpose through shared memory.
+//   PAIR  (BN = 256) two CTAs on one tile of 256 x 256 (see ptx.cuh): each loads its own 128 rows of A and half of B, which the other's
+//         tensor core reads from it.  A K block moves 32 KB into an SM's shared memory and 32 KB out of it, not 48 and 48, at 128 B
+//         per cycle for both: 512 cycles, which is what its products take, instead of 768.  A channel-major tile is swapped by
+//         exchanging the operands, as in the plain 128-column kernel: each CTA then has 128 channels of all 256 positions.
 //   STATS (with AUX and a K-outer A operand): two more warps take the rows' LayerNorm statistics from the A tiles in shared memory while
 //         the tensor core multiplies them: a pass over A and a launch less (see the launcher for where and what it measured).  The
 //         sums run over the channels in order, as that pass does: the same bits.
-template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false>
+template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false, bool PAIR = false>
 __global__ void __launch_bounds__(AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                  const __grid_constant__ CUtensorMap tm_out0, const __grid_constant__ CUtensorMap tm_out1,
                  const __grid_constant__ CUtensorMap tm_out2, const GemmParams p) {
   // tm_out0 / tm_out1: TMA-store maps of channel-major segments, or (p.aux) the gate / residual load maps and, tm_out2, the output
-  using Cfg = GemmCfg<BN>;
+  using Cfg = GemmCfg<BN, PAIR>;
   const int kStages = p.stages;
   constexpr int OUT_BN_GLU = BN / 2;
   constexpr int ACC_COLS = PRECISE ? 2 * BN : BN;  // precise: main accumulator, then the correction accumulator
   static_assert(!PRECISE || BN <= 128, "the fp32-accurate variant needs four accumulators of BN columns");
+  static_assert(!PAIR || (BN == 256 && !PRECISE && !SWAP && !STATS), "CTA pairs exist for the plain, GLU and AUX kernels of 256 columns");
   static_assert(!STATS || AUX, "in-kernel statistics exist for the AUX variant");
   static_assert(!SWAP || (BN == 256 && GLU && !AUX && !PRECISE), "the swapped orientation exists for the BN = 256 GLU tile");
   constexpr bool kSplitGlu = GLU && !PRECISE && BN < 256;
   constexpr bool kXpose = BN <= 128 && !GLU && !AUX && !PRECISE;
-  constexpr bool kPlain128 = (BN == 128 && !GLU && !AUX && !PRECISE);  // the variant that may swap single tiles
+  constexpr bool kPlain128 = ((BN == 128 || PAIR) && !GLU && !AUX && !PRECISE);  // the variants that may swap single tiles
+  const int rank = PAIR ? static_cast<int>(ptx::cluster_ctarank()) : 0;
+  const int tile0 = PAIR ? blockIdx.x >> 1 : blockIdx.x, tile_step = PAIR ? gridDim.x >> 1 : gridDim.x;   // (a tile: of the pair)
+  auto row_block = [&](const TileIdx& t) { return PAIR ? 2 * t.nb + rank : t.nb; };                       // of this CTA's rows
 
   extern __shared__ uint8_t smem_raw[];
   uint8_t* smem = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));
@@ -379,7 +389,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     }
     for (int a = 0; a < 2; ++a) {
       ptx::mbar_init(&tmem_full[a], 1);
-      ptx::mbar_init(&tmem_empty[a], 32 * kEpiWarps);
+      ptx::mbar_init(&tmem_empty[a], PAIR ? 2 * kEpiWarps : 32 * kEpiWarps);
       ptx::mbar_init(&aux_full[a], 1);
       ptx::mbar_init(&aux_empty[a], 1);
     }
@@ -390,15 +400,25 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     ptx::fence_barrier_init();
   }
   if (warp == 1) {
-    ptx::tmem_alloc(tmem_slot, PRECISE ? 2 * Cfg::kTmemCols : Cfg::kTmemCols);
-    ptx::tmem_relinquish();
+    if constexpr (PAIR) {
+      ptx::tmem_alloc_pair(tmem_slot, Cfg::kTmemCols);
+      ptx::tmem_relinquish_pair();
+    } else {
+      ptx::tmem_alloc(tmem_slot, PRECISE ? 2 * Cfg::kTmemCols : Cfg::kTmemCols);
+      ptx::tmem_relinquish();
+    }
   }
   ptx::tc_fence_before_sync();
-  __syncthreads();
+  if constexpr (PAIR) {
+    __syncwarp();
+    ptx::cluster_sync();
+  } else {
+    __syncthreads();
+  }
   ptx::tc_fence_after_sync();
   const uint32_t tmem_base = *tmem_slot;
 
-  TileIdx first_tile = tile_decompose(static_cast<int>(blockIdx.x), p);   // (its divisions run before the wait, too)
+  TileIdx first_tile = tile_decompose(tile0, p);   // (its divisions run before the wait, too)
 
   // Everything above ran under the tail of the launch before this one (programmatic launch).  The producer also fetches the
   // weight half of the first tile's stages before it waits: for the few-row GEMMs of the samplers, whose time is the latency of
@@ -416,6 +436,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     const int b_col_hi = (n_tile * BN) / p.b_col_inner;
     b_ahead = num_k < kStages ? num_k : kStages;
     for (int kb = 0; kb < b_ahead; ++kb) {
+      if constexpr (PAIR) {
+        if (rank == 0) ptx::mbar_expect_tx(&full_bar[kb], 2 * Cfg::kStageBytes);     // (of both CTAs)
+        ptx::tma_load_4d_pair(s_b + kb * Cfg::kBStage, &tm_b, ptx::leader_addr(&full_bar[kb]), kb * kBK, n_tile * BN + rank * Cfg::kBRows, 0, 0);
+        continue;
+      }
       ptx::mbar_expect_tx(&full_bar[kb], Cfg::kStageBytes);
       if constexpr (kSplitGlu)
         load_glu_b(kb, n_tile, kb);
@@ -436,11 +461,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       int aux_buf = 0;
       uint32_t aux_par = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, tile_advance(first_tile, p)) {
-        const int n_tile = first_tile.n_tile, nb = first_tile.nb, o = first_tile.o, b = first_tile.b;
+      for (int tile = tile0; ok && tile < total_tiles; tile += tile_step, tile_advance(first_tile, p)) {
+        const int n_tile = first_tile.n_tile, nb = row_block(first_tile), o = first_tile.o, b = first_tile.b;
         const int bb = p.b_batched ? b : 0;
         // the next kernel's blocks may take this SM over as soon as this CTA is on its last tile
-        if (tile + static_cast<int>(gridDim.x) >= total_tiles) grid_dependency_launch();
+        if (tile + tile_step >= total_tiles) grid_dependency_launch();
         const int b_col_hi = (n_tile * BN) / p.b_col_inner;
         const int b_col_lo = n_tile * BN - b_col_hi * p.b_col_inner;
         // AUX: the gate / residual tiles of this output tile go out as soon as their buffer is free; operand tiles never wait for it
@@ -468,7 +493,15 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             --b_ahead;
           } else {
             if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1, 101)) { ok = false; break; }
-            ptx::mbar_expect_tx(&full_bar[stage], Cfg::kStageBytes);
+            if (rank == 0) ptx::mbar_expect_tx(&full_bar[stage], (PAIR ? 2 : 1) * Cfg::kStageBytes);
+          }
+          if constexpr (PAIR) {
+            const uint32_t bar = ptx::leader_addr(&full_bar[stage]);
+            ptx::tma_load_4d_pair(s_a + stage * Cfg::kAStage, &tm_a, bar, kb * kBK, nb * kBM, o, b);
+            if (!b_done)
+              ptx::tma_load_4d_pair(s_b + stage * Cfg::kBStage, &tm_b, bar, kb * kBK, n_tile * BN + rank * Cfg::kBRows, 0, bb);
+            if (++stage == kStages) { stage = 0; phase ^= 1; }
+            continue;
           }
           if constexpr (PRECISE) {
             ptx::tma_load_5d(s_a + stage * Cfg::kAStage, &tm_a, &full_bar[stage], kb_main * kBK, nb * kBM, o, part_a(part), b);
@@ -501,18 +534,24 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           if (!ptx::mbar_wait(&aux_empty[aux_buf], aux_par ^ 1, 106)) { ok = false; break; }
           load_aux();
         }
-        KFB_GSTAMP(4 + (tile / gridDim.x) * 4 + 3);
+        KFB_GSTAMP(4 + (tile / tile_step) * 4 + 3);
+      }
+      if constexpr (PAIR) {     // the last products' arrivals at this CTA's barriers, before it may exit
+        for (int i = 0; ok && i < kStages; ++i) {
+          ok = ptx::mbar_wait(&empty_bar[stage], phase ^ 1, 117);
+          if (++stage == kStages) { stage = 0; phase ^= 1; }
+        }
       }
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------ MMA issuer
-    if (ptx::elect_one()) {
-      constexpr uint32_t idesc = ptx::make_idesc(kBM, BN, /*bf16*/ 1);
+    if (rank == 0 && ptx::elect_one()) {
+      constexpr uint32_t idesc = ptx::make_idesc(PAIR ? 2 * kBM : kBM, BN, /*bf16*/ 1);
       uint32_t tile_iter = 0;
       int stage = 0;
       uint32_t phase = 0;
       bool ok = true;
-      for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++tile_iter) {
+      for (int tile = tile0; ok && tile < total_tiles; tile += tile_step, ++tile_iter) {
         const uint32_t acc = tile_iter & 1;
         const uint32_t acc_phase = (tile_iter >> 1) & 1;
         const int n_tile_mma = tile % p.num_n_tiles;
@@ -572,7 +611,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
               ptx::mma_f16_ss(d_acc, b_desc + k * 2, a_desc + k * 2, idesc_sw, (first && k == 0) ? 0u : 1u);
               ptx::mma_f16_ss(d_acc + 128, g_desc + k * 2, a_desc + k * 2, idesc_sw, (first && k == 0) ? 0u : 1u);
             }
-          } else if (p.a_mn_major) {
+          } else if (!PAIR && p.a_mn_major) {
             // A as [k][rows]: MN-major, 128-byte swizzled rows; 8 k-rows are 1024 bytes apart, the next 64 rows
             // (positions) half a stage further; a K=16 step advances by 16 k-rows = 2048 bytes
             const uint64_t am_desc = static_cast<uint64_t>((ptx::smem_u32(s_a + stage * Cfg::kAStage) & 0x3ffff) >> 4) |
@@ -586,13 +625,19 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             const bool sw = kPlain128 && n_tile_mma * BN >= p.swap_col_begin;
             const uint64_t m_desc = sw ? b_desc : a_desc, n_desc = sw ? a_desc : b_desc;
 #pragma unroll
-            for (int k = 0; k < kBK / 16; ++k)
-              ptx::mma_f16_ss(d_acc, m_desc + k * 2, n_desc + k * 2, idesc, (first && k == 0) ? 0u : 1u);
+            for (int k = 0; k < kBK / 16; ++k) {
+              if constexpr (PAIR) ptx::mma_f16_ss_pair(d_acc, m_desc + k * 2, n_desc + k * 2, idesc, (first && k == 0) ? 0u : 1u);
+              else ptx::mma_f16_ss(d_acc, m_desc + k * 2, n_desc + k * 2, idesc, (first && k == 0) ? 0u : 1u);
+            }
           }
-          ptx::tc_commit(&empty_bar[stage]);  // frees the smem stage once these MMAs have read it
+          if constexpr (PAIR) ptx::tc_commit_pair(&empty_bar[stage]);
+          else ptx::tc_commit(&empty_bar[stage]);  // frees the smem stage once these MMAs have read it
           if (++stage == kStages) { stage = 0; phase ^= 1; }
         }
-        if (ok) ptx::tc_commit(&tmem_full[acc]);
+        if (ok) {
+          if constexpr (PAIR) ptx::tc_commit_pair(&tmem_full[acc]);
+          else ptx::tc_commit(&tmem_full[acc]);
+        }
         KFB_GSTAMP(4 + tile_iter * 4 + 2);
       }
     }
@@ -603,13 +648,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       int buf = 0;
       uint32_t par = 0;
       TileIdx t = first_tile;
-      for (int tile = blockIdx.x; tile < total_tiles; tile += gridDim.x, tile_advance(t, p)) {
+      for (int tile = tile0; tile < total_tiles; tile += tile_step, tile_advance(t, p)) {
         if (!ptx::mbar_wait(&rm_bar[buf], par, 113)) break;
         const uint8_t* src = s_aux + buf * ((p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes) + (p.aux_resid ? p.aux_gate * Cfg::kAuxTileBytes : 0);
 #pragma unroll
         for (int hcol = 0; hcol < BN / 64; ++hcol)
-          if (t.n_tile * BN + hcol * 64 < p.n_cols)
-            ptx::tma_store_4d(&tm_out2, src + hcol * (kBM * 128), t.n_tile * BN + hcol * 64, t.nb * kBM, t.o, t.b);
+          if (t.n_tile * BN + hcol * 64 < p.n_cols && (!PAIR || row_block(t) * kBM < p.n_extent))
+            ptx::tma_store_4d(&tm_out2, src + hcol * (kBM * 128), t.n_tile * BN + hcol * 64, row_block(t) * kBM, t.o, t.b);
         ptx::tma_store_commit();
         ptx::tma_store_wait_read();
         ptx::mbar_arrive(&aux_empty[buf]);
@@ -628,7 +673,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     int stage = 0;
     uint32_t phase = 0, tile_iter = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++tile_iter) {
+    for (int tile = tile0; ok && tile < total_tiles; tile += tile_step, ++tile_iter) {
       // sums shifted by the first channel's value keep E[x^2] - E[x]^2 harmless
       float x0 = 0.f, x1 = 0.f, s0 = 0.f, s1 = 0.f, q0 = 0.f, q1 = 0.f;
       for (int kb = 0; kb < num_k; ++kb) {
@@ -681,7 +726,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     // comparison that consumes it happens one tile later
     auto load_mask = [&](int tile, const TileIdx& t) -> uint32_t {
       if (p.rowmask == nullptr || tile >= total_tiles) return 1u;
-      const int n = t.nb * kBM + r;
+      const int n = row_block(t) * kBM + r;
       if (n >= p.n_extent) return 1u;
       uint32_t raw;
       asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(raw)
@@ -718,16 +763,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       }
     };
     TileIdx tile_cur = first_tile;
-    uint32_t mask_next = load_mask(blockIdx.x, tile_cur);
-    for (int tile = blockIdx.x; ok && tile < total_tiles; tile += gridDim.x, ++tile_iter, tile_advance(tile_cur, p)) {
-      const int n_tile = tile_cur.n_tile, nb = tile_cur.nb, o = tile_cur.o, b = tile_cur.b;
+    uint32_t mask_next = load_mask(tile0, tile_cur);
+    for (int tile = tile0; ok && tile < total_tiles; tile += tile_step, ++tile_iter, tile_advance(tile_cur, p)) {
+      const int n_tile = tile_cur.n_tile, nb = row_block(tile_cur), o = tile_cur.o, b = tile_cur.b;
       const int n = nb * kBM + r;
       const bool row_ok = n < p.n_extent;
       const float mask_v = mask_next ? 1.0f : 0.0f;
       if (p.rowmask != nullptr) {   // the next tile's index only lives until its mask load is issued
         TileIdx peek = tile_cur;
         tile_advance(peek, p);
-        mask_next = load_mask(tile + gridDim.x, peek);
+        mask_next = load_mask(tile + tile_step, peek);
       }
       const uint32_t acc = tile_iter & 1;
       const uint32_t acc_phase = (tile_iter >> 1) & 1;
@@ -881,14 +926,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         if (p.nseg > 1 && out_col_tile >= p.seg[1].col_begin) si = 1;
         if (p.nseg > 2 && out_col_tile >= p.seg[2].col_begin) si = 2;
         const EpiSeg& sg = p.seg[si];
-        const int ch_local = out_col_tile + r - sg.col_begin;
+        // (a pair's tile: 256 channels, 128 in each CTA, and all 256 positions in both)
+        const int ch_local = out_col_tile + (PAIR ? rank * kBM : 0) + r - sg.col_begin;
+        const int pos0 = PAIR ? tile_cur.nb * 2 * kBM : nb * kBM;
         const bool lane_ok = ch_local < sg.ncols;
         const float scale_v = sg.scale != 0.f ? sg.scale : 1.f;
-        const float bias_v = (p.col_bias != nullptr && lane_ok) ? p.col_bias[out_col_tile + r] : 0.0f;
+        const float bias_v = (p.col_bias != nullptr && lane_ok) ? p.col_bias[sg.col_begin + ch_local] : 0.0f;
         __nv_bfloat16* drow = reinterpret_cast<__nv_bfloat16*>(sg.dst) + static_cast<long long>(lane_ok ? ch_local : 0) * sg.s_col +
                               static_cast<long long>(b) * sg.s_b + static_cast<long long>(o) * sg.s_o;
 #pragma unroll 1
-        for (int c = chunk_phase * 32; c < kBM; c += 32 * (kEpiWarps / 4)) {
+        for (int c = chunk_phase * 32; c < (PAIR ? 2 * kBM : kBM); c += 32 * (kEpiWarps / 4)) {
           uint32_t raw[32];
           ptx::tmem_ld_32x32b_x32(t_row + c, raw);
           ptx::tmem_ld_wait();
@@ -896,7 +943,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 #pragma unroll
           for (int i = 0; i < 32; i += 2)
             w[i >> 1] = pack_bf16x2(fmaf(__uint_as_float(raw[i]), scale_v, bias_v), fmaf(__uint_as_float(raw[i + 1]), scale_v, bias_v));
-          const int n0 = nb * kBM + c;
+          const int n0 = pos0 + c;
           if (lane_ok) {
             __nv_bfloat16* d = drow + n0;
             const int n_lim = sg.n_pad > 0 ? sg.n_pad : p.n_extent;
@@ -926,7 +973,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         if (p.nseg > 1 && out_col_tile >= p.seg[1].col_begin) si = 1;
         if (p.nseg > 2 && out_col_tile >= p.seg[2].col_begin) si = 2;
         const EpiSeg& sg = p.seg[si];
-        const bool plain = sg.vec && !sg.out_fp32 && sg.tma_slot < 0 && out_col_tile + BN <= sg.col_begin + sg.ncols &&
+        // (staged tiles of a pair may run over the end of the last segment: the copy engine clips them)
+        const bool whole = out_col_tile + BN <= sg.col_begin + sg.ncols ||
+                           (PAIR && si == p.rm_seg && si == p.nseg - 1 && p.col_bias == nullptr);
+        const bool plain = sg.vec && !sg.out_fp32 && sg.tma_slot < 0 && whole &&
                            (reinterpret_cast<uintptr_t>(p.col_bias) & 15) == 0 && p.row_stats == nullptr &&
                            !((p.mask_segs >> si) & 1) &&
                            (si != 0 || (p.gate == nullptr && p.resid == nullptr));
@@ -962,7 +1012,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
               w0[i] = pack_bf16x2(__uint_as_float(r0[2 * i]), __uint_as_float(r0[2 * i + 1]));
               w1[i] = pack_bf16x2(__uint_as_float(r1[2 * i]), __uint_as_float(r1[2 * i + 1]));
             }
-            if constexpr (BN == 128) {
+            if constexpr (BN == 128 || PAIR) {
               if (si == p.rm_seg) {
                 // Through shared memory: a thread's 32-byte stores to 32 different rows cost one memory request per
                 // sector; the copy engine writes whole rows of the tile instead.  Two buffers alternate; a buffer is
@@ -971,7 +1021,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 uint8_t* buf = s_stage_out + (rm_use & 1) * Cfg::kRowTileBytes;
                 uint8_t* row0 = buf + r * 128;                              // columns 0..63 of this row
                 uint8_t* row1 = buf + Cfg::kRowTileBytes / 2 + r * 128;     // columns 64..127
-                const int piece = (c >> 3);                                 // first 16-byte piece: 0 or 4
+                const int piece = (c & 127) >> 3;                           // first 16-byte piece: 0 or 4
 #pragma unroll
                 for (int q4 = 0; q4 < 4; ++q4) {
                   const int phys = ((piece + q4) ^ (r & 7)) << 4;
@@ -985,9 +1035,11 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
                 if (!ptx::mbar_wait(&rm_bar[rm_use & 1], (rm_use >> 1) & 1, 110)) { ok = false; break; }
                 if (issuer) {
                   const CUtensorMap* tm = p.rm_slot == 0 ? &tm_out0 : &tm_out1;
-                  const int col0 = out_col_tile - sg.col_begin;
-                  ptx::tma_store_4d(tm, buf, col0, nb * kBM, o, b);
-                  if (col0 + 64 < sg.ncols) ptx::tma_store_4d(tm, buf + Cfg::kRowTileBytes / 2, col0 + 64, nb * kBM, o, b);
+                  const int col0 = out_col_tile - sg.col_begin + (PAIR ? c : 0);     // (the issuer's c: 0, then 128)
+                  if (!PAIR || (nb * kBM < p.n_extent && col0 < sg.ncols)) {
+                    ptx::tma_store_4d(tm, buf, col0, nb * kBM, o, b);
+                    if (col0 + 64 < sg.ncols) ptx::tma_store_4d(tm, buf + Cfg::kRowTileBytes / 2, col0 + 64, nb * kBM, o, b);
+                  }
                   ptx::tma_store_commit();
                 }
                 ++rm_use;
@@ -1446,8 +1498,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           } else if (issuer) {
             const uint8_t* buf = s_stage_out + (rm_use & 1) * Cfg::kRowTileBytes;
             const int col0 = out_col_tile - p.seg[0].col_begin;
-            ptx::tma_store_4d(&tm_out0, buf, col0, nb * kBM, o, b);
-            ptx::tma_store_4d(&tm_out0, buf + Cfg::kRowTileBytes / 2, col0 + 64, nb * kBM, o, b);
+            if (!PAIR || nb * kBM < p.n_extent) {
+              ptx::tma_store_4d(&tm_out0, buf, col0, nb * kBM, o, b);
+              ptx::tma_store_4d(&tm_out0, buf + Cfg::kRowTileBytes / 2, col0 + 64, nb * kBM, o, b);
+            }
             ptx::tma_store_commit();
           }
           ++rm_use;
@@ -1456,19 +1510,30 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       }
       if (!ok) break;
       ptx::tc_fence_before_sync();
-      ptx::mbar_arrive(&tmem_empty[acc]);
+      if constexpr (PAIR) {
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster(ptx::leader_addr(&tmem_empty[acc]));
+      } else {
+        ptx::mbar_arrive(&tmem_empty[acc]);
+      }
       if (threadIdx.x == 64) KFB_GSTAMP(4 + tile_iter * 4 + 1);
     }
     if (quad == 0 && lane == 0) ptx::tma_store_wait_all();
   }
 
   ptx::tc_fence_before_sync();
-  __syncthreads();
+  if constexpr (PAIR) {   // neither CTA leaves while the other may still read its operands or reach its barriers
+    __syncwarp();
+    ptx::cluster_sync();
+  } else {
+    __syncthreads();
+  }
   if (threadIdx.x == 0) KFB_GSTAMP(1);
 #undef KFB_GSTAMP
   if (warp == 1) {
     ptx::tc_fence_after_sync();
-    ptx::tmem_dealloc(tmem_base, PRECISE ? 2 * Cfg::kTmemCols : Cfg::kTmemCols);
+    if constexpr (PAIR) ptx::tmem_dealloc_pair(tmem_base, Cfg::kTmemCols);
+    else ptx::tmem_dealloc(tmem_base, PRECISE ? 2 * Cfg::kTmemCols : Cfg::kTmemCols);
   }
 }
 
@@ -1496,6 +1561,8 @@ struct GemmOperandB {  // B[(b), col, k]; optionally col = hi * col_inner + lo w
 // `tag` names the launch in the profile report (a string literal).
 // A segment whose rows are contiguous along n (s_n == 1) and whose other strides and base are 16-byte
 // aligned can go through the TMA-store path; the launcher decides and fills `tma_slot`.
+// force_bn: N tile the operands or segments ask for, 0: the launcher's choice.  A forced 128 may still become the 256 of a CTA pair where
+// the channel-major segments start at multiples of 256.
 int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOperandB& b, GemmParams p, int force_bn = 0,
                      const char* tag = "gemm");
 

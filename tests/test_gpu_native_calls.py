@@ -81,7 +81,8 @@ def test_token_stack_ragged(dev, l, groups, samples, own_s, precise):
         _compare(out.float().cpu(), ref, precise, f"token stack L={l}")
 
 
-@pytest.mark.parametrize("l,groups,samples,c,heads", [(65, 4, 3, 768, 16), (130, 2, 5, 768, 16), (257, 1, 4, 768, 16), (200, 3, 4, 512, 8)])
+@pytest.mark.parametrize("l,groups,samples,c,heads", [(65, 4, 3, 768, 16), (130, 2, 5, 768, 16), (257, 1, 4, 768, 16), (200, 3, 4, 512, 8),
+                                                         (1100, 1, 2, 768, 16)])
 def test_token_stack_shared_bias(dev, l, groups, samples, c, heads):
     """Head dims 48 and 64, enough samples per complex for the attention that adds one bias tile to several of them: odd sample
     counts, ragged tokens, scattered masks, heads whose bias lies far above and below zero."""
@@ -325,3 +326,32 @@ def test_block_with_a_mask_that_is_not_symmetric(dev, n, batch):
     zr, sr = O.pairformer_block(zb.float(), sb.float(), pm, m, w)
     _check(*err_stats(zo.float().cpu(), zr), "z")
     _check(*err_stats(so.float().cpu(), sr), "s")
+
+
+@pytest.mark.parametrize("b,m,n,k", [(1, 19000, 512, 520), (1, 9601, 1024, 600), (3, 6500, 776, 712), (20, 1100, 520, 520), (40, 200, 512, 640)])
+def test_gemm_of_cta_pairs(dev, b, m, n, k):
+    """Tiles of two CTAs: even and odd counts of row blocks, rows, columns and K that end inside a tile, one and several waves."""
+    from kfold_b200 import _lib as L
+    g = torch.Generator(device=dev).manual_seed(m)
+    a = torch.randn(b, m, k, generator=g, device=dev).bfloat16()
+    w = torch.randn(b, n, k, generator=g, device=dev).bfloat16()
+    d = torch.full((b, m, n), float("nan"), device=dev, dtype=torch.bfloat16)
+    L.check(L.lib().kfb_gemm_bf16(L.ptr(a), L.ptr(w), L.ptr(d), None, b, m, n, k, k, k, n, m * k, n * k, m * n, 0, L.stream_ptr()))
+    prev = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = False
+    ref = torch.matmul(a.float(), w.float().transpose(1, 2))
+    torch.backends.cuda.matmul.allow_tf32 = prev
+    # identical bf16 operands and float32 sums on both sides; the result is off by half a unit in its last place, 2^-9 of itself
+    assert ((d.float() - ref).abs() <= 1e-4 * k ** 0.5 + 2.0 ** -8 * ref.abs()).all()
+
+
+@pytest.mark.parametrize("rows", [9473, 9601, 19200])
+def test_transition_of_cta_pairs(dev, rows):
+    """Gated tiles and tiles with a prefetched residual, at 75, 76 and 150 row blocks."""
+    from kfold_b200 import functional as F
+    from kfold_b200 import packing
+    import synth
+    w = synth.transition_weights(synth._Rng(rows), 256, 4)
+    x = torch.randn(1, rows, 256, generator=torch.Generator().manual_seed(rows)).bfloat16()
+    out = F.transition(x.to(dev), packing.pack_transition(w, dev), residual=True).float().cpu()
+    _check(*err_stats(out, x.float() + _oracle_on(dev, O.transition, x.float(), w)), f"transition rows={rows}")
