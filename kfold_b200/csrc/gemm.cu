@@ -11,12 +11,12 @@
 
 namespace kfb {
 
-template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false, bool PAIR = false>
+template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false, bool PAIR = false, bool TWIN = false>
 static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* tout,
                           const GemmParams& p, const char* tag) {
   using Cfg = GemmCfg<BN, PAIR>;
-  constexpr auto kernel = gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP, STATS, PAIR>;
-  constexpr int threads = AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads;
+  constexpr auto kernel = gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP, STATS, PAIR, TWIN>;
+  constexpr int threads = TWIN ? kTwinThreads : AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads;
   static std::once_flag once[64];
   static int resident[64];      // tiles in flight: CTAs, or pairs of them, that the device holds at once
   int dev = 0;
@@ -64,6 +64,9 @@ static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUte
 static int launch_pair(cudaStream_t stream, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* tout, GemmParams p, const char* tag) {
   using Cfg = GemmCfg<256, true>;
   p.stages = Cfg::stages_for(p.aux ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes : p.glu ? Cfg::kGluStagingBytes : Cfg::kStagingBytes);
+  if (p.twin)
+    return p.glu ? launch_variant<256, true, false, false, false, false, true, true>(stream, ta, tb, tout, p, tag)
+                 : launch_variant<256, false, false, false, false, false, true, true>(stream, ta, tb, tout, p, tag);
   if (p.glu) return launch_variant<256, true, false, false, false, false, true>(stream, ta, tb, tout, p, tag);
   if (p.aux) return launch_variant<256, false, true, false, false, false, true>(stream, ta, tb, tout, p, tag);
   return launch_variant<256, false, false, false, false, false, true>(stream, ta, tb, tout, p, tag);
@@ -89,11 +92,15 @@ static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorM
   if constexpr (BN == 256) {
     if (p.glu && p.swap) {
       p.stages = Cfg::stages_for(Cfg::kSwapStagingBytes);
+      if (p.twin) return launch_variant<BN, true, false, false, true, false, false, true>(stream, ta, tb, tout, p, tag);
       return launch_variant<BN, true, false, false, true>(stream, ta, tb, tout, p, tag);
     }
   }
   if (p.glu) {
     p.stages = Cfg::stages_for(Cfg::kGluStagingBytes);
+    if constexpr (BN == 256) {
+      if (p.twin) return launch_variant<BN, true, false, false, false, false, false, true>(stream, ta, tb, tout, p, tag);
+    }
     return launch_variant<BN, true, false, false>(stream, ta, tb, tout, p, tag);
   }
   if constexpr (BN == 64 || BN == 128) {
@@ -101,6 +108,9 @@ static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorM
   }
   if constexpr (BN >= 64) {
     if (p.aux) return launch_variant<BN, false, true, false>(stream, ta, tb, tout, p, tag);
+  }
+  if constexpr (BN == 128) {
+    if (p.twin) return launch_variant<BN, false, false, false, false, false, false, true>(stream, ta, tb, tout, p, tag);
   }
   return launch_variant<BN, false, false, false>(stream, ta, tb, tout, p, tag);
   }
@@ -128,14 +138,14 @@ static int narrow_tile(const GemmParams& p, int bn) {
 
 // CTA pairs (PAIR in gemm.cuh) pay where the main loop is long enough to hide the epilogue of a tile twice as wide and the tiles are at
 // least a wave of pairs.  Measured, one CTA -> pair: triangle contraction at 768 tokens 108 -> 99 us (128 channels), 201 -> 180 (256);
-// SwiGLU of 256 channels at 768 x 768 rows 585 -> 472, its output projection (K = 1 024) 362 -> 318; token transformer, 5 x 768 rows of
-// 768: projection 35 -> 29, SwiGLU 24.5 -> 22.5.  The other side of the lines: SwiGLU of 128 channels (two K blocks) 106 -> 107; gate
+// at 400 tokens (seven K blocks) 71 -> 62; SwiGLU of 256 channels at 768 x 768 rows 585 -> 472, its output projection (K = 1 024) 362 ->
+// 318; token transformer, 5 x 768 rows of 768: projection 35 -> 29, SwiGLU 24.5 -> 22.5.  The other side of the lines: SwiGLU of 128 channels (two K blocks) 106 -> 107; gate
 // projection of 256 (four, plain) 105 -> 109; conditioning table (six, plain) 100 -> 104; contraction at 333 tokens (three row blocks, a
 // quarter of the pairs' work padding) 49.7 -> 51.6; float32 output projections with gate and residual 22.4 -> 23.5.
 static bool pair_tile(const GemmParams& p, int bn) {
   if (p.precise || bn < 128 || p.n_cols < 256 || p.glu == GLU_SIGMOID) return false;
   const int num_k = cdiv(p.k_extent, kBK), pairs = cdiv(p.n_blocks, 2);
-  if (num_k < (p.glu ? 4 : 8) || (2 * pairs - p.n_blocks) * 8 > p.n_blocks) return false;
+  if (num_k < (p.glu ? 4 : 7) || (2 * pairs - p.n_blocks) * 8 > p.n_blocks) return false;
   if (2ll * pairs * p.o_extent * p.batch * cdiv(p.n_cols, 256) < sm_count()) return false;
   for (int i = 0; i < p.nseg; ++i) {
     const EpiSeg& sg = p.seg[i];
@@ -370,6 +380,24 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
       KFB_TRY(make_tmap(&tout[0], sg.dst, 2, 4, dims, str, box, 128));
       p.rm_seg = i;
       break;
+    }
+  }
+  // two epilogue groups: every tile staged or swapped, nothing else to do to it, and more than one tile for each CTA (with one, the
+  // second group has nothing to do)
+  p.twin = 0;
+  {
+    const EpiSeg& s0 = p.seg[0];
+    const bool bare = p.gate == nullptr && p.resid == nullptr && p.row_stats == nullptr;
+    const bool whole_columns = s0.ncols % (p.glu ? 128 : bn) == 0 || (p.nseg == 1 && p.col_bias == nullptr && !p.glu);
+    const long long tiles = static_cast<long long>(p.num_m_tiles) * p.num_n_tiles * (p.pair ? 2 : 1);
+    if (bare && !p.precise && !p.aux && !p.a_mn_major && tiles > sm_count()) {
+      if (p.swap)
+        p.twin = p.swap_staged;
+      else if (p.glu)
+        p.twin = p.rm_seg == 0 && p.nseg == 1 && p.col_bias == nullptr && whole_columns && (p.mask_segs & 1) == 0;
+      else
+        p.twin = p.rm_seg == 0 && whole_columns && s0.col_begin == 0 && s0.scale == 0.f && (reinterpret_cast<uintptr_t>(p.col_bias) & 15) == 0 &&
+                 (p.nseg == 1 || p.seg[1].col_begin >= p.swap_col_begin);
     }
   }
   if (p.pair) return launch_pair(stream, ta, tb, tout, p, tag);

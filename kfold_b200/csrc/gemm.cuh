@@ -71,6 +71,7 @@ struct GemmParams {
   float stats_eps;                //   their epsilon
   const float* col_s1;            //   (mean, rstd) per flat row; col_s1 = sum_k W'[col][k], col_s0 = sum_k beta[k] W[col][k]
   const float* col_s0;            //   with W' = gamma * W the matrix actually multiplied (applied before gate / residual)
+  int twin;                       // launcher: two epilogue groups (see TWIN)
   int pair;                       // launcher: CTA pairs (see PAIR); n_blocks then counts the pairs' row blocks of 256
   int swap_col_begin;             // launcher (BN = 128, plain epilogue): tiles whose first column is >= this hold channel-major
                                   // segments only and are computed in the swapped orientation too (INT_MAX: none)
@@ -104,6 +105,7 @@ static constexpr int kGemmThreads = 64 + 32 * kEpiWarps;
 static constexpr int kAuxThreads = kGemmThreads + 32;  // the AUX variant's last warp hands finished tiles to the copy engine
 static constexpr int kStatsThreads = 64;               // the STATS variant's two warps after it: two rows of the tile per thread
 static constexpr int kStatsBytes = kBM * 8;            // (mean, rstd) of a tile's rows
+static constexpr int kTwinThreads = 64 + 2 * 32 * kEpiWarps + 64;   // the TWIN variant: two epilogue groups, a store warp for each
 
 template <int BN, bool PAIR = false>
 struct GemmCfg {
@@ -280,6 +282,53 @@ __device__ __forceinline__ void epi_store_chunk(const EpiSeg& sg, long long row_
   }
 }
 
+// A tile of channel-major segments, computed swapped: the lane is output column (channel) out_col_tile + lane_col, the tile's columns are
+// its 128 positions from pos0 on (a pair's tile: 256 channels, 128 in each CTA, and all 256 positions in both).  The launcher guarantees
+// that the tile lies inside one segment.  A warp takes every other 32 positions.
+template <bool PAIR>
+__device__ __forceinline__ void epi_swapped_tile(const GemmParams& p, uint32_t t_row, int out_col_tile, int lane_col, int pos0, int chunk_phase,
+                                                 int o, int b) {
+  int si = 0;
+  if (p.nseg > 1 && out_col_tile >= p.seg[1].col_begin) si = 1;
+  if (p.nseg > 2 && out_col_tile >= p.seg[2].col_begin) si = 2;
+  const EpiSeg& sg = p.seg[si];
+  const int ch_local = out_col_tile + lane_col - sg.col_begin;
+  const bool lane_ok = ch_local < sg.ncols;
+  const float scale_v = sg.scale != 0.f ? sg.scale : 1.f;
+  const float bias_v = (p.col_bias != nullptr && lane_ok) ? p.col_bias[out_col_tile + lane_col] : 0.0f;
+  __nv_bfloat16* drow = reinterpret_cast<__nv_bfloat16*>(sg.dst) + static_cast<long long>(lane_ok ? ch_local : 0) * sg.s_col +
+                        static_cast<long long>(b) * sg.s_b + static_cast<long long>(o) * sg.s_o;
+#pragma unroll 1
+  for (int c = chunk_phase * 32; c < (PAIR ? 256 : 128); c += 64) {
+    uint32_t raw[32];
+    ptx::tmem_ld_32x32b_x32(t_row + c, raw);
+    ptx::tmem_ld_wait();
+    uint32_t w[16];
+#pragma unroll
+    for (int i = 0; i < 32; i += 2)
+      w[i >> 1] = pack_bf16x2(fmaf(__uint_as_float(raw[i]), scale_v, bias_v), fmaf(__uint_as_float(raw[i + 1]), scale_v, bias_v));
+    const int n0 = pos0 + c;
+    if (lane_ok) {
+      __nv_bfloat16* d = drow + n0;
+      const int n_lim = sg.n_pad > 0 ? sg.n_pad : p.n_extent;
+      if (n0 + 32 <= n_lim && (reinterpret_cast<uintptr_t>(d) & 31) == 0) {
+        st_global_v8(d, w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7]);
+        st_global_v8(d + 16, w[8], w[9], w[10], w[11], w[12], w[13], w[14], w[15]);
+      } else if ((n_lim & 7) == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+          if (n0 + 8 * i < n_lim)
+            *reinterpret_cast<uint4*>(d + 8 * i) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
+      } else {
+#pragma unroll
+        for (int i = 0; i < 32; ++i)
+          if (n0 + i < p.n_extent)
+            d[i] = __ushort_as_bfloat16(static_cast<unsigned short>((i & 1) ? (w[i >> 1] >> 16) : (w[i >> 1] & 0xffffu)));
+      }
+    }
+  }
+}
+
 // A tile index as (n tile, row block, outer, batch).  The persistent loops step by the grid size; stepping the mixed-radix
 // digits with carries replaces five integer divisions per tile and role (which cost the epilogue warps about 800 cycles
 // of every 4500-cycle tile).
@@ -323,11 +372,16 @@ __device__ __forceinline__ void tile_advance(TileIdx& t, const GemmParams& p) {
 //         tensor core reads from it.  A K block moves 32 KB into an SM's shared memory and 32 KB out of it, not 48 and 48, at 128 B
 //         per cycle for both: 512 cycles, which is what its products take, instead of 768.  A channel-major tile is swapped by
 //         exchanging the operands, as in the plain 128-column kernel: each CTA then has 128 channels of all 256 positions.
+//   TWIN  two groups of eight epilogue warps take the tiles in turn, one accumulator each, and two more warps send what they stage: the
+//         launches whose every tile is staged or swapped, so that the epilogue is small enough for 20 warps' registers.  With one group
+//         a tile's chain of latencies (accumulator seen, tensor memory read, staged, all warps at the barrier, sent, next tile's index)
+//         was the time of the short-K projections: 3 350 cycles a SwiGLU tile, of which 1 890 arithmetic.  768 x 768 rows of 128 channels:
+//         SwiGLU 193 -> 172 us, attention projection 177 -> 168, gated input projection 112 -> 110; of 256: SwiGLU 469 -> 449.
 //   STATS (with AUX and a K-outer A operand): two more warps take the rows' LayerNorm statistics from the A tiles in shared memory while
 //         the tensor core multiplies them: a pass over A and a launch less (see the launcher for where and what it measured).  The
 //         sums run over the channels in order, as that pass does: the same bits.
-template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false, bool PAIR = false>
-__global__ void __launch_bounds__(AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads, 1)
+template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false, bool PAIR = false, bool TWIN = false>
+__global__ void __launch_bounds__(TWIN ? kTwinThreads : AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads, 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                  const __grid_constant__ CUtensorMap tm_out0, const __grid_constant__ CUtensorMap tm_out1,
                  const __grid_constant__ CUtensorMap tm_out2, const GemmParams p) {
@@ -337,6 +391,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   constexpr int OUT_BN_GLU = BN / 2;
   constexpr int ACC_COLS = PRECISE ? 2 * BN : BN;  // precise: main accumulator, then the correction accumulator
   static_assert(!PRECISE || BN <= 128, "the fp32-accurate variant needs four accumulators of BN columns");
+  static_assert(!TWIN || (BN >= 128 && !AUX && !PRECISE), "two epilogue groups exist for the staged kernels");
   static_assert(!PAIR || (BN == 256 && !PRECISE && !SWAP && !STATS), "CTA pairs exist for the plain, GLU and AUX kernels of 256 columns");
   static_assert(!STATS || AUX, "in-kernel statistics exist for the AUX variant");
   static_assert(!SWAP || (BN == 256 && GLU && !AUX && !PRECISE), "the swapped orientation exists for the BN = 256 GLU tile");
@@ -365,7 +420,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   uint64_t* cm_bar = aux_empty + 2;      // [2 groups][slab free, slab written], 128 arrivals each
   uint64_t* rm_bar = cm_bar + 4;         // [2 staging buffers]: row-major tile written, one arrival per epilogue thread
   uint64_t* stats_bar = rm_bar + 2;      // STATS: [full: 2 warps, free: the epilogue warps]
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(stats_bar + 2);
+  uint64_t* box_bar = stats_bar + 2;     // TWIN: [2 groups][2 boxes][full: a group's warps, free: its store warp]
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(box_bar + 8);
 
   const int warp = threadIdx.x >> 5;
   const int lane = threadIdx.x & 31;
@@ -397,6 +453,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     for (int a = 0; a < 2; ++a) ptx::mbar_init(&rm_bar[a], 32 * kEpiWarps);
     ptx::mbar_init(&stats_bar[0], kStatsThreads / 32);
     ptx::mbar_init(&stats_bar[1], kEpiWarps);
+    for (int a = 0; a < 8; ++a) ptx::mbar_init(&box_bar[a], (a & 1) ? 1 : kEpiWarps);
     ptx::fence_barrier_init();
   }
   if (warp == 1) {
@@ -710,6 +767,174 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       __syncwarp();
       if (lane == 0) ptx::mbar_arrive(&stats_bar[0]);
     }
+  } else if (TWIN && warp >= 2 + 2 * kEpiWarps) {
+    // ------------------------------------------------------------ store warp of an epilogue group: boxes of 64 columns (swapped: 64
+    // positions) x 128 rows leave as they are filled
+    if (ptx::elect_one()) {
+      const int group = warp - (2 + 2 * kEpiWarps);
+      constexpr int kBoxes = (GLU ? OUT_BN_GLU : BN) / 64;
+      const EpiSeg& sg = p.seg[0];
+      uint32_t use = 0;
+      TileIdx t = first_tile;
+      if (group == 1) tile_advance(t, p);
+      bool ok = true;
+      for (int tile = tile0 + group * tile_step; ok && tile < total_tiles; tile += 2 * tile_step, tile_advance(t, p), tile_advance(t, p)) {
+        const int out_col_tile = t.n_tile * (GLU ? OUT_BN_GLU : BN), row0 = row_block(t) * kBM;
+        if (kPlain128 && out_col_tile >= p.swap_col_begin) continue;
+        for (int i = 0; i < kBoxes; ++i, ++use) {
+          uint64_t* bar = box_bar + group * 4 + (use & 1) * 2;
+          if (!ptx::mbar_wait(bar, (use >> 1) & 1, 118)) { ok = false; break; }
+          const uint8_t* box = s_stage_out + (SWAP ? 1024 : 0) + (group * 2 + (use & 1)) * (Cfg::kRowTileBytes / 2);
+          if constexpr (SWAP) {
+            if (row0 + 64 * i < p.n_extent) ptx::tma_store_4d(&tm_out0, box, row0 + 64 * i, t.o, out_col_tile, t.b);
+          } else {
+            if (row0 < p.n_extent && out_col_tile + 64 * i < sg.ncols)
+              ptx::tma_store_4d(&tm_out0, box, out_col_tile + 64 * i, row0, t.o, t.b);
+          }
+          ptx::tma_store_commit();
+          ptx::tma_store_wait_read();
+          ptx::mbar_arrive(bar + 1);
+        }
+      }
+      ptx::tma_store_wait_all();
+    }
+  } else if constexpr (TWIN) {
+    // ------------------------------------------------------------ the two epilogue groups: tiles of one accumulator each
+    const int group = (warp - 2) >> 3, quad = warp & 3, chunk_phase = ((warp - 2) >> 2) & 1;
+    const int r = quad * 32 + lane;
+    uint32_t iter = 0, use = 0;       // tiles and boxes of this group so far
+    TileIdx t = first_tile;
+    if (group == 1) tile_advance(t, p);
+    // every lane of the warp goes on, or none (what follows needs them all)
+    auto wait_warp = [&](uint64_t* bar, uint32_t parity, int code) { return __all_sync(0xffffffffu, ptx::mbar_wait(bar, parity, code)) != 0; };
+    // (the row's mask byte a tile ahead, as in the single group below)
+    auto load_mask = [&](int tile, const TileIdx& at) -> uint32_t {
+      const int n = row_block(at) * kBM + r;
+      if (p.rowmask == nullptr || tile >= total_tiles || n >= p.n_extent) return 1u;
+      uint32_t raw;
+      asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(raw)
+                   : "l"(p.rowmask + static_cast<long long>(at.b) * p.m_b + static_cast<long long>(at.o) * p.m_o + static_cast<long long>(n) * p.m_n));
+      return raw;
+    };
+    uint8_t* box_row = nullptr;       // this lane's row of the box
+    uint64_t* box_full = nullptr;
+    auto box_begin = [&]() -> bool {
+      box_full = box_bar + group * 4 + (use & 1) * 2;
+      box_row = s_stage_out + (SWAP ? 1024 : 0) + (group * 2 + (use & 1)) * (Cfg::kRowTileBytes / 2) + r * 128;
+      return use < 2 || wait_warp(box_full + 1, ((use >> 1) - 1) & 1, 119);
+    };
+    auto box_put = [&](int piece, uint32_t w0, uint32_t w1, uint32_t w2, uint32_t w3) {   // 16 bytes: eight of the box's 64 columns
+      *reinterpret_cast<uint4*>(box_row + ((piece ^ (r & 7)) << 4)) = make_uint4(w0, w1, w2, w3);
+    };
+    auto box_end = [&]() {
+      ptx::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive(box_full);
+      ++use;
+    };
+    bool ok = true;
+    uint32_t mask_next = 1u;
+    if constexpr (SWAP) mask_next = load_mask(tile0 + group * tile_step, t);
+    for (int tile = tile0 + group * tile_step; ok && tile < total_tiles; tile += 2 * tile_step, ++iter) {
+      const int nb = row_block(t), o = t.o, b = t.b, pair_nb = t.nb;
+      const int out_col_tile = t.n_tile * (GLU ? OUT_BN_GLU : BN);
+      const float mask_v = mask_next ? 1.0f : 0.0f;
+      tile_advance(t, p);
+      tile_advance(t, p);
+      if constexpr (SWAP) mask_next = load_mask(tile + 2 * tile_step, t);
+      ok = wait_warp(&tmem_full[group], iter & 1, 104);
+      if (!ok) break;
+      ptx::tc_fence_after_sync();
+      const uint32_t t_row = tmem_base + group * ACC_COLS + (static_cast<uint32_t>(quad * 32) << 16);
+      if constexpr (GLU) {
+        const float* s_maskf = reinterpret_cast<const float*>(s_stage_out) + group * kBM;
+        if constexpr (SWAP) {
+          // lanes are channels, columns the tile's 128 positions; their mask goes through shared memory
+          if (chunk_phase == 0) {
+            reinterpret_cast<float*>(s_stage_out)[group * kBM + r] = mask_v;
+            ptx::mbar_arrive(&cm_bar[group]);
+          }
+          ok = wait_warp(&cm_bar[group], iter & 1, 108);
+          if (!ok) break;
+        }
+        const bool swiglu = p.glu != GLU_SIGMOID;
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int c0 = i * 64 + chunk_phase * 32;
+          uint32_t va[16], ga[16], vb[16], gb[16];
+          ptx::tmem_ld_32x32b_x16(t_row + c0, va);
+          ptx::tmem_ld_32x32b_x16(t_row + 128 + c0, ga);
+          ok = box_begin();
+          if (!ok) break;
+          ptx::tmem_ld_wait();
+          ptx::tmem_ld_32x32b_x16(t_row + c0 + 16, vb);
+          ptx::tmem_ld_32x32b_x16(t_row + 128 + c0 + 16, gb);
+          auto finish = [&](int h, const uint32_t (&vv)[16], const uint32_t (&gg)[16]) {
+            uint32_t w[8];
+#pragma unroll
+            for (int j = 0; j < 16; j += 2) {
+              const float a0 = __uint_as_float(vv[j]), a1 = __uint_as_float(vv[j + 1]);
+              const float g0 = __uint_as_float(gg[j]), g1 = __uint_as_float(gg[j + 1]);
+              float x0, x1;
+              if constexpr (SWAP) {
+                const float2 m = *reinterpret_cast<const float2*>(s_maskf + c0 + h * 16 + j);
+                x0 = glu_half(a0, g0) * m.x;
+                x1 = glu_half(a1, g1) * m.y;
+              } else {
+                x0 = swiglu ? glu_half(a0, a0) * g0 : glu_half(a0, g0);
+                x1 = swiglu ? glu_half(a1, a1) * g1 : glu_half(a1, g1);
+              }
+              w[j >> 1] = pack_bf16x2(x0, x1);
+            }
+            box_put(chunk_phase * 4 + h * 2, w[0], w[1], w[2], w[3]);
+            box_put(chunk_phase * 4 + h * 2 + 1, w[4], w[5], w[6], w[7]);
+          };
+          finish(0, va, ga);
+          ptx::tmem_ld_wait();
+          finish(1, vb, gb);
+          box_end();
+        }
+      } else if (out_col_tile < p.swap_col_begin) {
+#pragma unroll 1
+        for (int i = 0; i < BN / 64; ++i) {
+          const int c0 = i * 64 + chunk_phase * 32;
+          uint32_t x[32];
+          ptx::tmem_ld_32x32b_x32(t_row + c0, x);
+          ok = box_begin();
+          if (!ok) break;
+          ptx::tmem_ld_wait();
+          if (p.col_bias != nullptr) {   // per output column, the same for every row: uniform 16-byte loads
+            const float4* bias = reinterpret_cast<const float4*>(p.col_bias + out_col_tile + c0);
+#pragma unroll
+            for (int q4 = 0; q4 < 8; ++q4) {
+              const float4 u = __ldg(bias + q4);
+              x[4 * q4] = __float_as_uint(__uint_as_float(x[4 * q4]) + u.x);
+              x[4 * q4 + 1] = __float_as_uint(__uint_as_float(x[4 * q4 + 1]) + u.y);
+              x[4 * q4 + 2] = __float_as_uint(__uint_as_float(x[4 * q4 + 2]) + u.z);
+              x[4 * q4 + 3] = __float_as_uint(__uint_as_float(x[4 * q4 + 3]) + u.w);
+            }
+          }
+#pragma unroll
+          for (int q4 = 0; q4 < 4; ++q4) {
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) w[j] = pack_bf16x2(__uint_as_float(x[q4 * 8 + 2 * j]), __uint_as_float(x[q4 * 8 + 2 * j + 1]));
+            box_put(chunk_phase * 4 + q4, w[0], w[1], w[2], w[3]);
+          }
+          box_end();
+        }
+      } else {
+        epi_swapped_tile<PAIR>(p, t_row, out_col_tile, PAIR ? rank * kBM + r : r, PAIR ? pair_nb * 2 * kBM : nb * kBM, chunk_phase, o, b);
+      }
+      if (!ok) break;
+      ptx::tc_fence_before_sync();
+      if constexpr (PAIR) {
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster(ptx::leader_addr(&tmem_empty[group]));
+      } else {
+        ptx::mbar_arrive(&tmem_empty[group]);
+      }
+    }
   } else {
     // ------------------------------------------------------------ epilogue (warps 2..9)
     const int quad = warp & 3;  // TMEM lane quadrant this warp may read
@@ -920,49 +1145,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           ++rm_use;
         }
       } else if (kPlain128 && out_col_tile >= p.swap_col_begin) {
-        // a tile of channel-major segments, computed swapped: this lane is output column (channel) out_col_tile + r, the
-        // tile's columns are its 128 positions.  The launcher guarantees that the tile lies inside one segment.
-        int si = 0;
-        if (p.nseg > 1 && out_col_tile >= p.seg[1].col_begin) si = 1;
-        if (p.nseg > 2 && out_col_tile >= p.seg[2].col_begin) si = 2;
-        const EpiSeg& sg = p.seg[si];
-        // (a pair's tile: 256 channels, 128 in each CTA, and all 256 positions in both)
-        const int ch_local = out_col_tile + (PAIR ? rank * kBM : 0) + r - sg.col_begin;
-        const int pos0 = PAIR ? tile_cur.nb * 2 * kBM : nb * kBM;
-        const bool lane_ok = ch_local < sg.ncols;
-        const float scale_v = sg.scale != 0.f ? sg.scale : 1.f;
-        const float bias_v = (p.col_bias != nullptr && lane_ok) ? p.col_bias[sg.col_begin + ch_local] : 0.0f;
-        __nv_bfloat16* drow = reinterpret_cast<__nv_bfloat16*>(sg.dst) + static_cast<long long>(lane_ok ? ch_local : 0) * sg.s_col +
-                              static_cast<long long>(b) * sg.s_b + static_cast<long long>(o) * sg.s_o;
-#pragma unroll 1
-        for (int c = chunk_phase * 32; c < (PAIR ? 2 * kBM : kBM); c += 32 * (kEpiWarps / 4)) {
-          uint32_t raw[32];
-          ptx::tmem_ld_32x32b_x32(t_row + c, raw);
-          ptx::tmem_ld_wait();
-          uint32_t w[16];
-#pragma unroll
-          for (int i = 0; i < 32; i += 2)
-            w[i >> 1] = pack_bf16x2(fmaf(__uint_as_float(raw[i]), scale_v, bias_v), fmaf(__uint_as_float(raw[i + 1]), scale_v, bias_v));
-          const int n0 = pos0 + c;
-          if (lane_ok) {
-            __nv_bfloat16* d = drow + n0;
-            const int n_lim = sg.n_pad > 0 ? sg.n_pad : p.n_extent;
-            if (n0 + 32 <= n_lim && (reinterpret_cast<uintptr_t>(d) & 31) == 0) {
-              st_global_v8(d, w[0], w[1], w[2], w[3], w[4], w[5], w[6], w[7]);
-              st_global_v8(d + 16, w[8], w[9], w[10], w[11], w[12], w[13], w[14], w[15]);
-            } else if ((n_lim & 7) == 0 && (reinterpret_cast<uintptr_t>(d) & 15) == 0) {
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                if (n0 + 8 * i < n_lim)
-                  *reinterpret_cast<uint4*>(d + 8 * i) = make_uint4(w[4 * i], w[4 * i + 1], w[4 * i + 2], w[4 * i + 3]);
-            } else {
-#pragma unroll
-              for (int i = 0; i < 32; ++i)
-                if (n0 + i < p.n_extent)
-                  d[i] = __ushort_as_bfloat16(static_cast<unsigned short>((i & 1) ? (w[i >> 1] >> 16) : (w[i >> 1] & 0xffffu)));
-            }
-          }
-        }
+        epi_swapped_tile<PAIR>(p, t_row, out_col_tile, PAIR ? rank * kBM + r : r, PAIR ? tile_cur.nb * 2 * kBM : nb * kBM, chunk_phase, o, b);
       } else {
       // Fast path of the plain kernel: a tile that lies inside one row-major bf16 segment and needs nothing but the
       // conversion and a column bias (the q / k / g columns of the attention projections, plain projections): none of the
