@@ -174,12 +174,19 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
   if (bn == 0) bn = p.n_cols >= 256 ? 256 : (p.n_cols > 64 ? 128 : 64);
   if (p.precise && bn > 128) bn = 128;  // the fp32-accurate variant keeps four accumulators in tensor memory
   if (a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0 && (p.precise ? !p.glu : p.glu != GLU_SIGMOID)) bn = narrow_tile(p, bn);
-  p.pair = pair_tile(p, bn) && a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0;
+  // K shared by a cluster where rows are few (the gate / residual epilogue of 128 float32 columns takes the other kernel 8 000 cycles)
+  const bool plain_operands = a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0;
+  SplitPlan plan = {0, 0};
+  if (force_bn == 0 && static_cast<long long>(p.num_m_tiles) * cdiv(p.n_cols, bn) <= sm_count())
+    plan = split_plan(p, plain_operands, split_cycles(p.precise, bn, cdiv(p.precise ? p.k_extent / 6 : p.k_extent, kBK)) +
+                                             ((p.gate != nullptr || p.resid != nullptr) && !p.precise ? 50.0 : 12.0) * bn);
+  if (plan.bn != 0) bn = plan.bn;
+  p.pair = plan.bn == 0 && pair_tile(p, bn) && a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0;
   if (p.pair) bn = 256;
   // One row-major float32 segment with a gate and / or a residual (the output projections of the sampler's float32 activation
   // stream): 128-column tiles whose epilogue moves gate, residual and output through per-warp shared-memory tiles.
   p.xpose = 0;
-  if (!p.precise && !p.glu && force_bn == 0 && p.nseg == 1 && a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0 &&
+  if (plan.bn == 0 && !p.precise && !p.glu && force_bn == 0 && p.nseg == 1 && a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0 &&
       (p.gate != nullptr || p.resid != nullptr) && p.resid_scale == nullptr) {
     const EpiSeg& sg = p.seg[0];
     const bool seg_ok = sg.out_fp32 && sg.vec && sg.s_col == 1 && sg.col_begin == 0 && !sg.split && sg.ncols % 32 == 0 &&
@@ -199,7 +206,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
   // buffer of 256-column tiles: its load hides behind the K loop, and A is read once.
   p.aux = p.aux_gate = p.aux_resid = 0;
   p.aux_bufs = 2;
-  if (!p.precise && !p.xpose && !p.glu && p.nseg == 1 && p.seg[0].vec && !p.seg[0].out_fp32 && p.seg[0].s_col == 1 &&
+  if (plan.bn == 0 && !p.precise && !p.xpose && !p.glu && p.nseg == 1 && p.seg[0].vec && !p.seg[0].out_fp32 && p.seg[0].s_col == 1 &&
       p.seg[0].col_begin == 0 && p.seg[0].ncols == p.n_cols && (p.gate != nullptr || p.resid != nullptr) && bn >= 64 && p.n_cols % 32 == 0) {
     const EpiSeg& sg = p.seg[0];
     const bool ok_o = (reinterpret_cast<uintptr_t>(sg.dst) & 15) == 0 && sg.s_n % 8 == 0 && sg.s_o % 8 == 0 && (sg.s_o != 0 || p.o_extent == 1) &&
@@ -299,6 +306,7 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
     KFB_TRY(make_tmap(&tb, b.ptr, 2, 4, dims, str, box, 128));
     }
   }
+  if (plan.bn != 0) return launch_gemm_split(stream, ta, tb, p, plan, tag);
   // channel-major bf16 segments that satisfy the TMA alignment rules are stored through shared memory
   CUtensorMap tout[3];
   tout[0] = tout[1] = tout[2] = ta;  // placeholders (never dereferenced unless a segment selects them)

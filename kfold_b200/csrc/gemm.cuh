@@ -1749,6 +1749,20 @@ struct GemmOperandB {  // B[(b), col, k]; optionally col = hi * col_inner + lo w
 int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOperandB& b, GemmParams p, int force_bn = 0,
                      const char* tag = "gemm");
 
+// GEMMs of few rows whose K a cluster of CTAs shares (gemm_split.cu): tile width and CTAs per tile, bn = 0 where the other kernel is the
+// better one.  plain_operands: neither operand is split or K-outer; other_cycles: that kernel's modelled time.
+struct SplitPlan {
+  int bn, split;
+};
+SplitPlan split_plan(const GemmParams& p, bool plain_operands, double other_cycles);
+int launch_gemm_split(cudaStream_t stream, const CUtensorMap& ta, const CUtensorMap& tb, const GemmParams& p, const SplitPlan& plan, const char* tag);
+// Cycles of a tile's main loop: the larger of its copies (64 B per cycle) and of the multiplying thread's turn per K block (waits,
+// products, commits: clock stamps).
+inline double split_cycles(bool precise, int bn, int k_blocks) {
+  const double copies = (precise ? 3 : 1) * (16384.0 + 128.0 * bn) / 64.0, turn = precise ? 1430.0 : 400.0;
+  return k_blocks * (copies > turn ? copies : turn);
+}
+
 // Debugging aid: launches whose tag equals `tag` store per-tile clock stamps of CTA 0 into `device_buffer`
 // (>= 512 long longs); nullptr switches it off.
 void set_gemm_trace(long long* device_buffer, const char* tag);

@@ -355,3 +355,18 @@ def test_transition_of_cta_pairs(dev, rows):
     x = torch.randn(1, rows, 256, generator=torch.Generator().manual_seed(rows)).bfloat16()
     out = F.transition(x.to(dev), packing.pack_transition(w, dev), residual=True).float().cpu()
     _check(*err_stats(out, x.float() + _oracle_on(dev, O.transition, x.float(), w)), f"transition rows={rows}")
+
+
+@pytest.mark.parametrize("m,n,k", [(1, 384, 1536), (64, 32, 520), (96, 768, 768), (130, 772, 1096), (300, 1024, 2048)])
+def test_gemm_with_k_shared_by_a_cluster(dev, m, n, k):
+    """Few rows, float32 results: rows, columns and K that end inside a tile, shares of K of unequal length, one to three row blocks."""
+    from kfold_b200 import _lib as L
+    g = torch.Generator(device=dev).manual_seed(m)
+    a = torch.randn(m, k, generator=g, device=dev).bfloat16()
+    w = torch.randn(n, k, generator=g, device=dev).bfloat16()
+    bias = torch.randn(n, generator=g, device=dev)
+    d = torch.full((m, n), float("nan"), device=dev)
+    L.check(L.lib().kfb_gemm_bf16(L.ptr(a), L.ptr(w), L.ptr(d), L.ptr(bias), 1, m, n, k, k, k, n, 0, 0, 0, 1, L.stream_ptr()))
+    ref = a.double() @ w.double().T + bias.double()
+    # products of bf16 numbers are exact; each of the K / 16 steps cuts the running sum, at most 6 sqrt(K) here, to 24 bits
+    assert (d - ref).abs().max() <= k / 16 * 2.0 ** -23 * 6 * k ** 0.5
