@@ -632,15 +632,15 @@ __device__ __forceinline__ void load8(const float* p, float (&f)[8]) {
   f[0] = lo.x; f[1] = lo.y; f[2] = lo.z; f[3] = lo.w; f[4] = hi.x; f[5] = hi.y; f[6] = hi.z; f[7] = hi.w;
 }
 template <typename TI, int CH, int LANES>
-__global__ void __launch_bounds__(256) adaln_vec_kernel(const TI* __restrict__ a, __nv_bfloat16* __restrict__ y,
+__global__ void __launch_bounds__(256) adaln_vec_kernel(const TI* a /*no __restrict__: its loads must stay behind the wait*/, __nv_bfloat16* y,
                                                         const __nv_bfloat16* __restrict__ gv, long long gv_ld, long long rows,
-                                                        int samples, int l, float eps) {
-  grid_dependency_enter();
+                                                        int samples, int l, float eps, int gv_static) {
   constexpr int c = 8 * LANES * CH;
   constexpr int kRowsPerWarp = 32 / LANES;
   const int lane = threadIdx.x & 31;
   const int sub = lane % LANES;
   const long long warps_per_grid = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  bool waited = false;
   for (long long base = (static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5)) * kRowsPerWarp; base < rows;
        base += warps_per_grid * kRowsPerWarp) {
     const long long row = base + lane / LANES;
@@ -651,13 +651,19 @@ __global__ void __launch_bounds__(256) adaln_vec_kernel(const TI* __restrict__ a
     const __nv_bfloat16* gr = gv + srow * gv_ld;
     uint4 gt[CH], sh[CH];
     float v[CH][8];
+    // the conditioning rows of a stack's tables are there long before the rows to be normalised: fetched under the launch before
+    // this one, which is writing those
+    if (!gv_static && !waited) grid_dependency_enter();
 #pragma unroll
     for (int k = 0; k < CH; ++k) {
       const int ch = (sub + LANES * k) * 8;
-      load8(xr + ch, v[k]);
       gt[k] = *reinterpret_cast<const uint4*>(gr + ch);
       sh[k] = *reinterpret_cast<const uint4*>(gr + c + ch);
     }
+    if (gv_static && !waited) grid_dependency_enter();
+    waited = true;
+#pragma unroll
+    for (int k = 0; k < CH; ++k) load8(xr + (sub + LANES * k) * 8, v[k]);
     float s = 0.f;
 #pragma unroll
     for (int k = 0; k < CH; ++k)
@@ -702,7 +708,7 @@ __global__ void __launch_bounds__(256) adaln_vec_kernel(const TI* __restrict__ a
 
 template <typename TI, int CH, int LANES>
 static int launch_adaln_vec(cudaStream_t stream, const void* a, void* y, const void* gv, long long gv_ld, long long rows, int samples,
-                            int l, float eps) {
+                            int l, float eps, int gv_static) {
   const long long rows_per_block = 8 * (32 / LANES);
   long long blocks = (rows + rows_per_block - 1) / rows_per_block;
   const long long cap = static_cast<long long>(sm_count()) * 16;
@@ -710,7 +716,7 @@ static int launch_adaln_vec(cudaStream_t stream, const void* a, void* y, const v
   LaunchScope scope(stream, "adaln_rows");
   KFB_TRY(launch_kernel(stream, adaln_vec_kernel<TI, CH, LANES>, static_cast<unsigned>(blocks), 256, 0,
       static_cast<const TI*>(a), static_cast<__nv_bfloat16*>(y), static_cast<const __nv_bfloat16*>(gv), gv_ld, rows,
-      samples, l, eps));
+      samples, l, eps, gv_static));
   KFB_CUDA(cudaGetLastError());
   return KFB_OK;
 }
@@ -742,7 +748,7 @@ static int adaln_dispatch(cudaStream_t stream, const void* a, void* y, const voi
 }
 
 int launch_adaln(cudaStream_t stream, const void* a, void* y, const void* gv, long long rows, int c, int samples,
-                 int l, float eps, int in_dtype, int out_dtype, long long gv_ld) {
+                 int l, float eps, int in_dtype, int out_dtype, long long gv_ld, int gv_static) {
   if (gv_ld <= 0) gv_ld = 2ll * c;
   KFB_CHECK_ARG(gv_ld >= 2ll * c && gv_ld % 2 == 0 && (reinterpret_cast<uintptr_t>(gv) & 7) == 0,
                 "adaln: gate/shift row stride %lld (at least 2c, even) or misaligned pointer", gv_ld);
@@ -753,8 +759,8 @@ int launch_adaln(cudaStream_t stream, const void* a, void* y, const void* gv, lo
   if ((in_dtype == KFB_BF16 || in_dtype == KFB_FP32) && out_dtype == KFB_BF16 && gv_ld % 8 == 0 &&
       ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(gv)) & 15) == 0) {
 #define KFB_ADALN_VEC(CH, LANES)                                                                                          \
-  return in_dtype == KFB_BF16 ? launch_adaln_vec<__nv_bfloat16, CH, LANES>(stream, a, y, gv, gv_ld, rows, samples, l, eps) \
-                              : launch_adaln_vec<float, CH, LANES>(stream, a, y, gv, gv_ld, rows, samples, l, eps)
+  return in_dtype == KFB_BF16 ? launch_adaln_vec<__nv_bfloat16, CH, LANES>(stream, a, y, gv, gv_ld, rows, samples, l, eps, gv_static) \
+                              : launch_adaln_vec<float, CH, LANES>(stream, a, y, gv, gv_ld, rows, samples, l, eps, gv_static)
     switch (c) {
       case 128: KFB_ADALN_VEC(1, 16);
       case 256: KFB_ADALN_VEC(1, 32);

@@ -153,7 +153,7 @@ KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, con
   for (int i = 0; i < n_blocks; ++i) {
     const kfb_token_block& w = blocks[i];
     KFB_TRY(launch_adaln(stream, cur, an, column(t.gs, 4ll * c * i, precise), rows, c, share, l, eps, ada_dtype,
-                         precise ? KFB_FP32_PRECISE : KFB_BF16, t.gs_cols));
+                         precise ? KFB_FP32_PRECISE : KFB_BF16, t.gs_cols, 1));
     ApbArgs r;
     r.x = an;
     r.x_is_split = precise;
@@ -169,7 +169,7 @@ KFB_API int kfb_token_stack_fwd(const kfb_token_block* blocks, int n_blocks, con
     KFB_TRY(apb_run(stream, r));
     cur = out;                                      // from here on the stream is updated in place
     KFB_TRY(launch_adaln(stream, cur, an, column(t.gs, 4ll * c * i + 2ll * c, precise), rows, c, share, l, eps, ada_dtype,
-                         precise ? KFB_FP32_PRECISE : KFB_BF16, t.gs_cols));
+                         precise ? KFB_FP32_PRECISE : KFB_BF16, t.gs_cols, 1));
     KFB_TRY(cond_transition_run(stream, an, precise, 1, w.w_swiglu, w.w_tout, column(t.og, 2ll * c * i + c, precise), t.og_cols, out, cur, op_ws,
                                 op_bytes, rows, c, hidden, share, l, op_dtype));
   }
@@ -212,8 +212,8 @@ KFB_API int kfb_atom_stack_fwd(const kfb_atom_block* blocks, int n_blocks, const
   for (int i = 0; i < n_blocks; ++i) {
     const kfb_atom_block& w = blocks[i];
     const long long g0 = 6ll * c * i;
-    KFB_TRY(launch_adaln(stream, cur, xq, column(t.gs, g0, 0), rows, c, samples, l, eps, act_dtype, KFB_BF16, t.gs_cols));
-    KFB_TRY(launch_adaln(stream, cur, xk, column(t.gs, g0 + 2ll * c, 0), rows, c, samples, l, eps, act_dtype, KFB_BF16, t.gs_cols));
+    KFB_TRY(launch_adaln(stream, cur, xq, column(t.gs, g0, 0), rows, c, samples, l, eps, act_dtype, KFB_BF16, t.gs_cols, 1));
+    KFB_TRY(launch_adaln(stream, cur, xk, column(t.gs, g0 + 2ll * c, 0), rows, c, samples, l, eps, act_dtype, KFB_BF16, t.gs_cols, 1));
     // the output gate is shared by the samples: query row r reads gate row r % (l) of its group
     for (int g = 0; g < groups; ++g) {
       const size_t row0 = static_cast<size_t>(g) * samples * l, e = act_dtype == KFB_FP32 ? 4 : 2;
@@ -226,7 +226,7 @@ KFB_API int kfb_atom_stack_fwd(const kfb_atom_block* blocks, int n_blocks, const
                                  samples, l, c, heads, bias_share, mask_share, static_cast<int>(bias_windows), act_dtype, stream_));
     }
     cur = out;
-    KFB_TRY(launch_adaln(stream, cur, xq, column(t.gs, g0 + 4ll * c, 0), rows, c, samples, l, eps, act_dtype, KFB_BF16, t.gs_cols));
+    KFB_TRY(launch_adaln(stream, cur, xq, column(t.gs, g0 + 4ll * c, 0), rows, c, samples, l, eps, act_dtype, KFB_BF16, t.gs_cols, 1));
     KFB_TRY(cond_transition_run(stream, xq, 0, 1, w.w_swiglu, w.w_tout, column(t.og, 2ll * c * i + c, 0), t.og_cols, out, cur, op_ws, op_bytes,
                                 rows, c, hidden, samples, l, act_dtype));
   }
