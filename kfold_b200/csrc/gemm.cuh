@@ -72,6 +72,7 @@ struct GemmParams {
   const float* col_s1;            //   (mean, rstd) per flat row; col_s1 = sum_k W'[col][k], col_s0 = sum_k beta[k] W[col][k]
   const float* col_s0;            //   with W' = gamma * W the matrix actually multiplied (applied before gate / residual)
   int twin;                       // launcher: two epilogue groups (see TWIN)
+  int glu_tiles;                  // launcher (swapped GLU kernel): column tiles before the plain ones of a GemmExtra
   int pair;                       // launcher: CTA pairs (see PAIR); n_blocks then counts the pairs' row blocks of 256
   int swap_col_begin;             // launcher (BN = 128, plain epilogue): tiles whose first column is >= this hold channel-major
                                   // segments only and are computed in the swapped orientation too (INT_MAX: none)
@@ -377,6 +378,8 @@ __device__ __forceinline__ void tile_advance(TileIdx& t, const GemmParams& p) {
 //         a tile's chain of latencies (accumulator seen, tensor memory read, staged, all warps at the barrier, sent, next tile's index)
 //         was the time of the short-K projections: 3 350 cycles a SwiGLU tile, of which 1 890 arithmetic.  768 x 768 rows of 128 channels:
 //         SwiGLU 193 -> 172 us, attention projection 177 -> 168, gated input projection 112 -> 110; of 256: SwiGLU 469 -> 449.
+//         The swapped GLU kernel of this form also takes plain column tiles from a second matrix of 128-row blocks (GemmExtra): maps
+//         tm_out1 (the matrix) and tm_out2 (its row-major output).
 //   STATS (with AUX and a K-outer A operand): two more warps take the rows' LayerNorm statistics from the A tiles in shared memory while
 //         the tensor core multiplies them: a pass over A and a launch less (see the launcher for where and what it measured).  The
 //         sums run over the channels in order, as that pass does: the same bits.
@@ -488,7 +491,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     ptx::tma_load_4d(s_b + stage * Cfg::kBStage, &tm_b, &full_bar[stage], kb * kBK, row, 0, 0);
     ptx::tma_load_4d(s_b + stage * Cfg::kBStage + Cfg::kBStage / 2, &tm_b, &full_bar[stage], kb * kBK, row + 128, 0, 0);
   };
-  if (warp == 0 && p.b_static && !p.k_inner && ptx::elect_one()) {
+  constexpr bool kExtra = SWAP && TWIN;
+  constexpr int kExtraStage = Cfg::kAStage + 128 * kBK * 2;      // bytes of a stage of a plain tile
+  if (warp == 0 && p.b_static && !p.k_inner && !(kExtra && first_tile.n_tile >= p.glu_tiles) && ptx::elect_one()) {
     const int n_tile = first_tile.n_tile;
     const int b_col_hi = (n_tile * BN) / p.b_col_inner;
     b_ahead = num_k < kStages ? num_k : kStages;
@@ -550,7 +555,17 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             --b_ahead;
           } else {
             if (!ptx::mbar_wait(&empty_bar[stage], phase ^ 1, 101)) { ok = false; break; }
-            if (rank == 0) ptx::mbar_expect_tx(&full_bar[stage], (PAIR ? 2 : 1) * Cfg::kStageBytes);
+            if constexpr (kExtra) {
+              ptx::mbar_expect_tx(&full_bar[stage], n_tile >= p.glu_tiles ? kExtraStage : Cfg::kStageBytes);
+              if (n_tile >= p.glu_tiles) {
+                ptx::tma_load_4d(s_a + stage * Cfg::kAStage, &tm_a, &full_bar[stage], kb * kBK, nb * kBM, o, b);
+                ptx::tma_load_4d(s_b + stage * Cfg::kBStage, &tm_out1, &full_bar[stage], kb * kBK, (n_tile - p.glu_tiles) * 128, 0, 0);
+                if (++stage == kStages) { stage = 0; phase ^= 1; }
+                continue;
+              }
+            } else if (rank == 0) {
+              ptx::mbar_expect_tx(&full_bar[stage], (PAIR ? 2 : 1) * Cfg::kStageBytes);
+            }
           }
           if constexpr (PAIR) {
             const uint32_t bar = ptx::leader_addr(&full_bar[stage]);
@@ -663,6 +678,10 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             // value rows (first 128 rows of the weight stage) -> columns 0..127, gate rows -> columns 128..255
             constexpr uint32_t idesc_sw = ptx::make_idesc(kBM, 128, /*bf16*/ 1);
             const uint64_t g_desc = b_desc + ((128 * 128) >> 4);
+            if (kExtra && n_tile_mma >= p.glu_tiles) {
+#pragma unroll
+              for (int k = 0; k < kBK / 16; ++k) ptx::mma_f16_ss(d_acc, a_desc + k * 2, b_desc + k * 2, idesc_sw, (first && k == 0) ? 0u : 1u);
+            } else
 #pragma unroll
             for (int k = 0; k < kBK / 16; ++k) {
               ptx::mma_f16_ss(d_acc, b_desc + k * 2, a_desc + k * 2, idesc_sw, (first && k == 0) ? 0u : 1u);
@@ -785,7 +804,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           uint64_t* bar = box_bar + group * 4 + (use & 1) * 2;
           if (!ptx::mbar_wait(bar, (use >> 1) & 1, 118)) { ok = false; break; }
           const uint8_t* box = s_stage_out + (SWAP ? 1024 : 0) + (group * 2 + (use & 1)) * (Cfg::kRowTileBytes / 2);
-          if constexpr (SWAP) {
+          if (kExtra && t.n_tile >= p.glu_tiles) {
+            if (row0 < p.n_extent) ptx::tma_store_4d(&tm_out2, box, (t.n_tile - p.glu_tiles) * 128 + 64 * i, row0, t.o, t.b);
+          } else if constexpr (SWAP) {
             if (row0 + 64 * i < p.n_extent) ptx::tma_store_4d(&tm_out0, box, row0 + 64 * i, t.o, out_col_tile, t.b);
           } else {
             if (row0 < p.n_extent && out_col_tile + 64 * i < sg.ncols)
@@ -802,7 +823,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     // ------------------------------------------------------------ the two epilogue groups: tiles of one accumulator each
     const int group = (warp - 2) >> 3, quad = warp & 3, chunk_phase = ((warp - 2) >> 2) & 1;
     const int r = quad * 32 + lane;
-    uint32_t iter = 0, use = 0;       // tiles and boxes of this group so far
+    uint32_t iter = 0, use = 0, masks = 0;       // tiles, boxes and position masks of this group so far
     TileIdx t = first_tile;
     if (group == 1) tile_advance(t, p);
     // every lane of the warp goes on, or none (what follows needs them all)
@@ -837,6 +858,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     if constexpr (SWAP) mask_next = load_mask(tile0 + group * tile_step, t);
     for (int tile = tile0 + group * tile_step; ok && tile < total_tiles; tile += 2 * tile_step, ++iter) {
       const int nb = row_block(t), o = t.o, b = t.b, pair_nb = t.nb;
+      const bool plain = !GLU || (kExtra && t.n_tile >= p.glu_tiles);
       const int out_col_tile = t.n_tile * (GLU ? OUT_BN_GLU : BN);
       const float mask_v = mask_next ? 1.0f : 0.0f;
       tile_advance(t, p);
@@ -846,7 +868,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       if (!ok) break;
       ptx::tc_fence_after_sync();
       const uint32_t t_row = tmem_base + group * ACC_COLS + (static_cast<uint32_t>(quad * 32) << 16);
-      if constexpr (GLU) {
+      if (GLU && !plain) {
         const float* s_maskf = reinterpret_cast<const float*>(s_stage_out) + group * kBM;
         if constexpr (SWAP) {
           // lanes are channels, columns the tile's 128 positions; their mask goes through shared memory
@@ -854,8 +876,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             reinterpret_cast<float*>(s_stage_out)[group * kBM + r] = mask_v;
             ptx::mbar_arrive(&cm_bar[group]);
           }
-          ok = wait_warp(&cm_bar[group], iter & 1, 108);
+          ok = wait_warp(&cm_bar[group], masks & 1, 108);
           if (!ok) break;
+          ++masks;
         }
         const bool swiglu = p.glu != GLU_SIGMOID;
 #pragma unroll
@@ -894,16 +917,16 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           finish(1, vb, gb);
           box_end();
         }
-      } else if (out_col_tile < p.swap_col_begin) {
+      } else if (GLU || out_col_tile < p.swap_col_begin) {
 #pragma unroll 1
-        for (int i = 0; i < BN / 64; ++i) {
+        for (int i = 0; i < (GLU ? 128 : BN) / 64; ++i) {
           const int c0 = i * 64 + chunk_phase * 32;
           uint32_t x[32];
           ptx::tmem_ld_32x32b_x32(t_row + c0, x);
           ok = box_begin();
           if (!ok) break;
           ptx::tmem_ld_wait();
-          if (p.col_bias != nullptr) {   // per output column, the same for every row: uniform 16-byte loads
+          if (!GLU && p.col_bias != nullptr) {   // per output column, the same for every row: uniform 16-byte loads
             const float4* bias = reinterpret_cast<const float4*>(p.col_bias + out_col_tile + c0);
 #pragma unroll
             for (int q4 = 0; q4 < 8; ++q4) {
@@ -923,7 +946,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           }
           box_end();
         }
-      } else {
+      } else if constexpr (!GLU) {
         epi_swapped_tile<PAIR>(p, t_row, out_col_tile, PAIR ? rank * kBM + r : r, PAIR ? pair_nb * 2 * kBM : nb * kBM, chunk_phase, o, b);
       }
       if (!ok) break;
@@ -1740,6 +1763,18 @@ struct GemmOperandB {  // B[(b), col, k]; optionally col = hi * col_inner + lo w
   long long s_k_hi = 0;
 };
 
+// A second matrix for the rows of a swapped GLU GEMM (the triangle multiplication's gate logits beside its operands): `cols` more columns
+// (a multiple of 128), dst[(b, o, n)][col] = sum_k A w[col][k] in bf16, row-major with the given strides.  taken: whether the
+// launch did it; otherwise the caller launches a GEMM of its own.
+struct GemmExtra {
+  const void* w;
+  long long w_ld;
+  int cols;
+  void* dst;
+  long long s_n, s_o, s_b;
+  bool taken;
+};
+
 // Fills the tile bookkeeping of `p`, builds the tensor maps and launches on `stream`.
 // `tag` names the launch in the profile report (a string literal).
 // A segment whose rows are contiguous along n (s_n == 1) and whose other strides and base are 16-byte
@@ -1747,7 +1782,7 @@ struct GemmOperandB {  // B[(b), col, k]; optionally col = hi * col_inner + lo w
 // force_bn: N tile the operands or segments ask for, 0: the launcher's choice.  A forced 128 may still become the 256 of a CTA pair where
 // the channel-major segments start at multiples of 256.
 int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOperandB& b, GemmParams p, int force_bn = 0,
-                     const char* tag = "gemm");
+                     const char* tag = "gemm", GemmExtra* extra = nullptr);
 
 // GEMMs of few rows whose K a cluster of CTAs shares (gemm_split.cu): tile width and CTAs per tile, bn = 0 where the other kernel is the
 // better one.  plain_operands: neither operand is split or K-outer; other_cycles: that kernel's modelled time.

@@ -5,7 +5,7 @@
 //   2. input projection + gate + mask    ab[ch] = (xn Wp^T) * sigmoid(xn Wg^T) * m  [tcgen05 GEMM, GLU epilogue,
 //                                        stored CHANNEL-major so each channel is      channel-major TMA store]
 //                                        a dense rows x N matrix
-//   3. output gate logits                gl = xn Wg_out^T                            [tcgen05 GEMM]
+//   3. output gate logits                gl = xn Wg_out^T          [tcgen05 GEMM; C <= 128: columns of step 2]
 //   phase "finish"
 //   4. triangle contraction              t[ch] = A_ch * B_ch^T, batch over channels   [tcgen05 batched GEMM]
 //   5. LayerNorm_out, channel-major in   t -> tn (bf16, position-major)             [HBM bound]
@@ -61,6 +61,7 @@ int project(cudaStream_t stream, int transposed_walk, const void* x, const unsig
   const long long rn = static_cast<long long>(rows) * n;
   const long long pos = rn * batch;
   if (x != nullptr) KFB_TRY(launch_layernorm(stream, x, xn, ln_w, ln_b, pos, c, c, c, eps, dtype, KFB_BF16, RowPerm(), fold));
+  bool gate_done = false;
   if (w_in_packed != nullptr) {
     // ab[ch][b][o][n_]: o = row of the shard, n_ = position inside the row (swapped for the transposed walk)
     GemmParams p = {};
@@ -90,9 +91,12 @@ int project(cudaStream_t stream, int transposed_walk, const void* x, const unsig
                       transposed_walk ? c : static_cast<long long>(n) * c, rn * c};
     GemmOperandB b = {static_cast<const __nv_bfloat16*>(w_in_packed) + static_cast<long long>(part) * (4 * c / parts) * c, c, 0};
     p.b_static = x != nullptr;
-    KFB_TRY(launch_gemm_bf16(stream, a, b, p, 256, "trimul_in_proj"));
+    // the gate logits of the same rows in the same launch, if it takes them
+    GemmExtra gate = {w_gout, c, c, gl, a.s_n, a.s_o, rn * c, false};
+    KFB_TRY(launch_gemm_bf16(stream, a, b, p, 256, "trimul_in_proj", w_gout != nullptr ? &gate : nullptr));
+    gate_done = gate.taken;
   }
-  if (w_gout != nullptr) {
+  if (w_gout != nullptr && !gate_done) {
     GemmParams p = {};
     p.n_extent = static_cast<int>(pos);
     p.o_extent = 1;
