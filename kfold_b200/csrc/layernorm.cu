@@ -350,6 +350,130 @@ int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w
   return KFB_ERR_INVALID_ARGUMENT;
 }
 
+// LayerNorm and projection to at most 16 heads.  What bounds it: the rows, read once; written normalised and read again by a GEMM of 16
+// columns they had moved three times.  A warp takes 16 rows: four lanes share a row (a lane has 8 channels of every 32, 16-byte loads),
+// the statistics take two shuffles, and the normalised bf16 pairs are already the A fragments of 16 x 8 x 16 products -- a product does
+// not care which channel is called k, so the weights' fragments follow the lanes' channels.  (Sixteen columns are too few for a tile of
+// the tensor memory kernels to be anything but latency; the products are 5 % of the time here.)
+// 768 x 768 rows of 128 channels, between CUDA events: LayerNorm 56 + GEMM 44 us -> 54 in one launch; 400 x 400 of 256: 45 + 28 -> 43.
+// (The unpacked rows live in registers, 128 and 254 of them; held to 64 or 80 they spill: 72 us.)
+template <int C>
+__global__ void __launch_bounds__(256) ln_heads_kernel(const __nv_bfloat16* __restrict__ z, const float* __restrict__ ln_w,
+                                                       const float* __restrict__ ln_b, const __nv_bfloat16* __restrict__ w, const HeadsOut out,
+                                                       int rows, int o_extent, int n_extent, int heads, float eps) {
+  constexpr int Q = C / 32, kWLd = C + 8;       // (rows of the weights 16 bytes off: eight of them cover the banks)
+  __shared__ __align__(16) __nv_bfloat16 s_w[16 * kWLd];
+  __shared__ __align__(16) float s_g[C], s_b[C];
+  grid_dependency_enter();
+  for (int i = threadIdx.x; i < 16 * (C / 8); i += 256) {
+    const int h = i / (C / 8), ch = (i % (C / 8)) * 8;
+    *reinterpret_cast<uint4*>(s_w + h * kWLd + ch) = h < heads ? *reinterpret_cast<const uint4*>(w + h * C + ch) : make_uint4(0, 0, 0, 0);
+  }
+  for (int i = threadIdx.x; i < C; i += 256) {
+    s_g[i] = ln_w != nullptr ? ln_w[i] : 1.0f;
+    s_b[i] = ln_b != nullptr ? ln_b[i] : 0.0f;
+  }
+  __syncthreads();
+  const int lane = threadIdx.x & 31, g = lane >> 2, t = lane & 3;
+  const int warps = gridDim.x * 8;
+  for (int base = (blockIdx.x * 8 + (threadIdx.x >> 5)) * 16; base < rows; base += warps * 16) {
+    uint4 raw[2][Q];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const __nv_bfloat16* zr = z + static_cast<long long>(min(base + g + 8 * r, rows - 1)) * C + t * 8;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) raw[r][q] = *reinterpret_cast<const uint4*>(zr + q * 32);
+    }
+    float mean[2], rstd[2];
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      float s = 0.f;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const uint32_t u[4] = {raw[r][q].x, raw[r][q].y, raw[r][q].z, raw[r][q].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) s += __uint_as_float(u[i] << 16) + __uint_as_float(u[i] & 0xffff0000u);
+      }
+      s += __shfl_xor_sync(0xffffffffu, s, 1);
+      s += __shfl_xor_sync(0xffffffffu, s, 2);
+      mean[r] = s * (1.0f / C);
+      float v = 0.f;
+#pragma unroll
+      for (int q = 0; q < Q; ++q) {
+        const uint32_t u[4] = {raw[r][q].x, raw[r][q].y, raw[r][q].z, raw[r][q].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const float d0 = __uint_as_float(u[i] << 16) - mean[r], d1 = __uint_as_float(u[i] & 0xffff0000u) - mean[r];
+          v = fmaf(d0, d0, v);
+          v = fmaf(d1, d1, v);
+        }
+      }
+      v += __shfl_xor_sync(0xffffffffu, v, 1);
+      v += __shfl_xor_sync(0xffffffffu, v, 2);
+      rstd[r] = rsqrtf(v * (1.0f / C) + eps);
+    }
+    float acc[2][4] = {};       // [heads 0-7, 8-15][row g: heads 2t, 2t + 1; row g + 8: the same]
+#pragma unroll
+    for (int q = 0; q < Q; ++q) {
+      const int ch = q * 32 + t * 8;
+      uint32_t a[2][4];         // the rows' normalised pairs
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float2 gg = *reinterpret_cast<const float2*>(s_g + ch + 2 * i), bb = *reinterpret_cast<const float2*>(s_b + ch + 2 * i);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const uint32_t u = i == 0 ? raw[r][q].x : i == 1 ? raw[r][q].y : i == 2 ? raw[r][q].z : raw[r][q].w;
+          const __nv_bfloat162 pr = __floats2bfloat162_rn(fmaf((__uint_as_float(u << 16) - mean[r]) * rstd[r], gg.x, bb.x),
+                                                          fmaf((__uint_as_float(u & 0xffff0000u) - mean[r]) * rstd[r], gg.y, bb.y));
+          a[r][i] = *reinterpret_cast<const uint32_t*>(&pr);
+        }
+      }
+#pragma unroll
+      for (int h8 = 0; h8 < 2; ++h8) {
+        const uint4 wv = *reinterpret_cast<const uint4*>(s_w + (h8 * 8 + g) * kWLd + ch);
+        const uint32_t wb[4] = {wv.x, wv.y, wv.z, wv.w};
+#pragma unroll
+        for (int k = 0; k < 4; k += 2)
+          asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0, %1, %2, %3}, {%4, %5, %6, %7}, {%8, %9}, {%0, %1, %2, %3};"
+              : "+f"(acc[h8][0]), "+f"(acc[h8][1]), "+f"(acc[h8][2]), "+f"(acc[h8][3])
+              : "r"(a[0][k]), "r"(a[1][k]), "r"(a[0][k + 1]), "r"(a[1][k + 1]), "r"(wb[k]), "r"(wb[k + 1]));
+      }
+    }
+#pragma unroll
+    for (int r = 0; r < 2; ++r) {
+      const int row = base + g + 8 * r;
+      if (row >= rows) break;
+      const int n = row % n_extent, rest = row / n_extent;
+      __nv_bfloat16* dst = out.out + static_cast<long long>(rest / o_extent) * out.s_b + static_cast<long long>(rest % o_extent) * out.s_o +
+                           static_cast<long long>(n) * out.s_n;
+#pragma unroll
+      for (int h8 = 0; h8 < 2; ++h8)
+#pragma unroll
+        for (int i = 0; i < 2; ++i) {
+          const int h = h8 * 8 + 2 * t + i;
+          if (h < heads) dst[h * out.s_h] = __float2bfloat16_rn(acc[h8][2 * r + i]);
+        }
+    }
+  }
+}
+
+bool ln_heads_ok(const void* z, const void* w, int c, int heads, long long rows) {
+  return (c == 128 || c == 256) && heads <= 16 && rows > 0 && rows < (1ll << 31) - 64 &&
+         ((reinterpret_cast<uintptr_t>(z) | reinterpret_cast<uintptr_t>(w)) & 15) == 0;
+}
+int launch_ln_heads(cudaStream_t stream, const void* z, const float* ln_w, const float* ln_b, const void* w, const HeadsOut& o, int batch,
+                    int o_extent, int n_extent, int c, int heads, float eps) {
+  const long long rows = static_cast<long long>(batch) * o_extent * n_extent;
+  KFB_CHECK_ARG(ln_heads_ok(z, w, c, heads, rows), "ln_heads: c %d heads %d rows %lld", c, heads, rows);
+  long long blocks = (rows + 127) / 128;
+  const long long cap = static_cast<long long>(sm_count()) * 8;
+  if (blocks > cap) blocks = cap;
+  LaunchScope scope(stream, "pair_bias_proj");
+  return launch_kernel(stream, c == 128 ? ln_heads_kernel<128> : ln_heads_kernel<256>, static_cast<unsigned>(blocks), 256, 0,
+                       static_cast<const __nv_bfloat16*>(z), ln_w, ln_b, static_cast<const __nv_bfloat16*>(w), o, static_cast<int>(rows), o_extent,
+                       n_extent, heads, eps);
+}
+
 // fp32 -> bf16 conversion, eight elements per thread (HBM-bound; the conditioning rows of a stack: one small launch).
 __global__ void __launch_bounds__(256) to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
   grid_dependency_enter();

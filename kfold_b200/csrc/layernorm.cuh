@@ -28,6 +28,16 @@ int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w
                      long long xs, long long ys, float eps, int in_dtype, int out_dtype, RowPerm perm = RowPerm(),
                      const LnFold* fold = nullptr);
 
+// LayerNorm of bf16 rows (128 or 256 channels, contiguous, 16-byte aligned) and projection to heads <= 16 values in one pass: the pair
+// bias.  w [heads][c] bf16; row (b, o, n) of batch x o_extent x n_extent, head h -> out + b s_b + o s_o + n s_n + h s_h (elements).
+struct HeadsOut {
+  __nv_bfloat16* out;
+  long long s_b, s_o, s_n, s_h;
+};
+bool ln_heads_ok(const void* z, const void* w, int c, int heads, long long rows);
+int launch_ln_heads(cudaStream_t stream, const void* z, const float* ln_w, const float* ln_b, const void* w, const HeadsOut& o, int batch,
+                    int o_extent, int n_extent, int c, int heads, float eps);
+
 // fp32 -> bf16 (round to nearest), n elements.
 int launch_to_bf16(cudaStream_t stream, const float* x, __nv_bfloat16* y, long long n);
 

@@ -498,6 +498,12 @@ int pair_bias_run(const void* z, const float* ln_w, const float* ln_b, const voi
                           int dtype, cudaStream_t stream, int pitch) {
   if (pitch == 0) pitch = n;     // row pitch of the bias planes (untransposed)
   const long long rn = static_cast<long long>(rows) * n;
+  if (dtype == KFB_BF16 && ln_heads_ok(z, w, c, heads, rn * batch)) {
+    HeadsOut o = {static_cast<__nv_bfloat16*>(bias_out), 0, transposed ? 1ll : pitch, transposed ? static_cast<long long>(rows) : 1ll,
+                  static_cast<long long>(rows) * pitch};
+    o.s_b = o.s_h * heads;
+    return launch_ln_heads(stream, z, ln_w, ln_b, w, o, batch, rows, n, c, heads, eps);
+  }
   __nv_bfloat16* zn = static_cast<__nv_bfloat16*>(workspace);
   KFB_TRY(launch_layernorm(stream, z, zn, ln_w, ln_b, rn * batch, c, c, c, eps, dtype, KFB_BF16));
   GemmParams p = {};

@@ -370,3 +370,22 @@ def test_gemm_with_k_shared_by_a_cluster(dev, m, n, k):
     ref = a.double() @ w.double().T + bias.double()
     # products of bf16 numbers are exact; each of the K / 16 steps cuts the running sum, at most 6 sqrt(K) here, to 24 bits
     assert (d - ref).abs().max() <= k / 16 * 2.0 ** -23 * 6 * k ** 0.5
+
+
+@pytest.mark.parametrize("n,batch,c,heads", [(8, 1, 128, 16), (24, 2, 256, 16), (40, 1, 128, 6), (136, 2, 128, 16)])
+@pytest.mark.parametrize("transposed", [0, 1])
+def test_pair_bias_in_one_pass(dev, n, batch, c, heads, transposed):
+    """Rows that end inside a warp's sixteen, fewer heads than a fragment holds, both orders of the two positions."""
+    from kfold_b200 import _lib as L
+    g = torch.Generator(device=dev).manual_seed(n)
+    z = torch.randn(batch, n, n, c, generator=g, device=dev).bfloat16()
+    w = (torch.randn(heads, c, generator=g, device=dev) * c ** -0.5).bfloat16()
+    lw, lb = 1 + 0.1 * torch.randn(c, generator=g, device=dev), 0.1 * torch.randn(c, generator=g, device=dev)
+    out = torch.full((batch, heads, n, n), float("nan"), device=dev, dtype=torch.bfloat16)
+    ws = torch.empty(L.lib().kfb_pair_bias_workspace_bytes(batch, n, c), dtype=torch.uint8, device=dev)
+    L.check(L.lib().kfb_pair_bias_fwd(L.ptr(z), L.ptr(lw), L.ptr(lb), L.ptr(w), L.ptr(out), L.ptr(ws), ws.numel(), batch, n, c, heads, transposed,
+                                      1e-5, 0, L.stream_ptr()))
+    ref = torch.einsum("bijc,hc->bhij", torch.nn.functional.layer_norm(z.double(), (c,), lw.double(), lb.double(), 1e-5), w.double())
+    ref = ref.transpose(-1, -2) if transposed else ref
+    # operands and result are rounded to bf16, 2^-9 of themselves each: the sum's error stays within six sigma of c independent roundings
+    assert (out.double() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max() + 6 * 2.0 ** -9
