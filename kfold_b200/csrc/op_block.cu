@@ -11,7 +11,7 @@ size_t max_of(size_t a, size_t b) { return a > b ? a : b; }
 
 size_t operator_bytes(const kfb_pair_block& k, int batch, int n, int precise) {
   const long long pos = static_cast<long long>(batch) * n * n, rows = static_cast<long long>(batch) * n;
-  size_t m = precise ? kfb_trimul_workspace_bytes_precise(batch, n, k.c) : kfb_trimul_workspace_bytes(batch, n, k.c);
+  size_t m = precise ? kfb_trimul_workspace_bytes_precise(batch, n, k.c) : kfb_trimul_workspace_bytes(batch, n, k.c) + trimul_fold_bytes(k.c);
   if (k.has_attention)
     m = max_of(m, precise ? kfb_triatt_workspace_bytes_precise(batch, n, k.c, k.tri_heads) : kfb_triatt_workspace_bytes(batch, n, k.c, k.tri_heads));
   m = max_of(m, precise ? kfb_transition_workspace_bytes_precise(pos, k.c, k.hidden_z) : kfb_transition_workspace_bytes(pos, k.c, k.hidden_z));

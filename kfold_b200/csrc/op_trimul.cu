@@ -29,8 +29,7 @@ namespace {
 inline int pitch8(int n) { return (n + 7) / 8 * 8; }
 
 struct TrimulWs {
-  __nv_bfloat16 *xn, *ab, *gl, *t, *wf;
-  float* s;
+  __nv_bfloat16 *xn, *ab, *gl, *t;
 };
 size_t carve(TrimulWs& w, void* base, int batch, int n, int c) {
   Carver cv(base);
@@ -39,10 +38,16 @@ size_t carve(TrimulWs& w, void* base, int batch, int n, int c) {
   w.ab = cv.take<__nv_bfloat16>(pos_p * 2 * c);
   w.gl = cv.take<__nv_bfloat16>(pos * c);
   w.t = cv.take<__nv_bfloat16>(pos_p * c);
-  w.wf = cv.take<__nv_bfloat16>(static_cast<size_t>(c) * c);   // the output projection's weights with its LayerNorm folded in
-  w.s = cv.take<float>(2 * static_cast<size_t>(c));
   return cv.off;
 }
+
+}  // namespace
+
+namespace kfb {
+size_t trimul_fold_bytes(int c) { return align_up(static_cast<size_t>(c) * c * sizeof(__nv_bfloat16), 256) + align_up(2 * static_cast<size_t>(c) * sizeof(float), 256); }
+}  // namespace kfb
+
+namespace {
 
 int check_shape(const char* what, int batch, int rows, int n, int c) {
   KFB_CHECK_ARG(batch >= 1 && n >= 8 && n % 8 == 0, "%s: N=%d must be a positive multiple of 8 (pad in the caller)", what, n);
@@ -357,10 +362,17 @@ KFB_API int kfb_trimul_fwd(int incoming, const void* x, const unsigned char* mas
   KFB_CHECK_ARG(workspace_bytes >= need, "trimul: workspace %zu < %zu bytes", workspace_bytes, need);
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "trimul: workspace must be 256-byte aligned");
   cudaStream_t stream = as_stream(stream_);
-  const LnFold fold = {static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, w.wf, w.s, w.s + c, c, c};
-  KFB_TRY(project(stream, incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, w.xn, w.ab, w.gl, batch, n, n, c, eps, dtype, 0, 1, &fold));
+  // The output projection's weights with its LayerNorm folded in: by the first launch into what lies behind the workspace, where the
+  // caller gave that much more (the pair blocks do), otherwise by a launch of their own into the normalised rows once those are used.
+  const bool early = workspace_bytes >= need + trimul_fold_bytes(c);
+  Carver behind(static_cast<uint8_t*>(workspace) + need);
+  __nv_bfloat16* wf = behind.take<__nv_bfloat16>(static_cast<size_t>(c) * c);
+  float* sums = behind.take<float>(2 * static_cast<size_t>(c));
+  const LnFold fold = {static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, wf, sums, sums + c, c, c};
+  KFB_TRY(project(stream, incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, w.xn, w.ab, w.gl, batch, n, n, c, eps, dtype, 0, 1,
+                  early ? &fold : nullptr));
   return finish(stream, w.ab, w.ab + static_cast<long long>(c) * batch * n * pitch8(n), n, 0, w.gl, ln_out_w, ln_out_b, w_pout, w.t, w.xn, out,
-                resid, batch, n, n, c, eps, dtype, &fold);
+                resid, batch, n, n, c, eps, dtype, early ? &fold : nullptr);
 }
 
 KFB_API int kfb_trimul_project(const void* x, const unsigned char* mask, const float* ln_in_w, const float* ln_in_b,

@@ -67,6 +67,8 @@ int apb_run(cudaStream_t stream, const ApbArgs& r);
 int triatt_run(cudaStream_t stream, int ending, const void* x, const unsigned char* mask, const float* ln_w, const float* ln_b,
                const void* w_proj_packed, const void* w_out, void* out, const void* resid, void* workspace, size_t workspace_bytes, int batch,
                int n, int c, int heads, float eps, int dtype, int2* mask_rows);
+// What kfb_trimul_fwd can use behind its workspace (bf16): room for the output projection's folded weights.
+size_t trimul_fold_bytes(int c);
 // Whether these sizes take the attention kernel that scans the mask, and the scan for both directions in one launch: batch * n entries
 // of the starting node, then those of the ending node.
 bool triatt_scans_mask(int c, int heads, int n, int dtype);
