@@ -77,7 +77,7 @@ static int launch_bn(cudaStream_t stream, const CUtensorMap& ta, const CUtensorM
                      GemmParams p, const char* tag) {
   using Cfg = GemmCfg<BN>;
   p.stages = Cfg::stages_for(p.aux ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes + (p.stats_in_kernel ? kStatsBytes : 0)
-                                   : Cfg::kStagingBytes);
+                                   : p.xpose ? Cfg::kXposeStagingBytes : Cfg::kStagingBytes);
   if constexpr (BN == 32) {
     KFB_CHECK_ARG(!p.glu && !p.aux, "32-column tiles exist for the plain kernels only");
     if (p.precise) return launch_variant<32, false, false, true>(stream, ta, tb, tout, p, tag);

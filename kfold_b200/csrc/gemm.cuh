@@ -119,7 +119,8 @@ struct GemmCfg {
   // output tiles (two 64-column boxes of [128 rows][128 bytes] each) on their way to a TMA store
   static constexpr int kSlabBytes = (kEpiWarps / 4) * 2 * 32 * kBM * 2;
   static constexpr int kRowTileBytes = kBM * 128 * 2;
-  static constexpr int kXposeBytes = kEpiWarps * 6144;     // per-warp tiles of the float32 gate / residual route
+  static constexpr int kXposeBytes = kEpiWarps * 6144;     // per-warp tiles of the float32 gate / residual route,
+  static constexpr int kXposeStagingBytes = (BN == 128 ? 2 : 1) * kXposeBytes;   // one for each 32-column chunk of a warp
   static constexpr int kStagingBytes = (BN == 128 || PAIR) ? 2 * kRowTileBytes : (BN < 128 ? kXposeBytes : kSlabBytes);
   // the GLU kernel at BN = 256 writes 128 output columns per tile: the same two row-major tile buffers
   static constexpr int kGluStagingBytes = (BN == 256) ? 2 * kRowTileBytes : kStagingBytes;
@@ -413,7 +414,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
   uint8_t* s_aux = s_stage_out;                               // ... or [buffers][gate, resid][BN / 64][128 x 64] bf16
   float2* s_stats = reinterpret_cast<float2*>(s_aux + p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes);   // (STATS)
   uint64_t* bars = reinterpret_cast<uint64_t*>(
-      s_stage_out + (AUX ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes + (STATS ? kStatsBytes : 0) : (SWAP ? Cfg::kSwapStagingBytes : (GLU ? Cfg::kGluStagingBytes : Cfg::kStagingBytes))));
+      s_stage_out + (AUX ? p.aux_bufs * (p.aux_gate + p.aux_resid) * Cfg::kAuxTileBytes + (STATS ? kStatsBytes : 0)
+                         : (SWAP ? Cfg::kSwapStagingBytes
+                                 : (GLU ? Cfg::kGluStagingBytes : kXpose && p.xpose ? Cfg::kXposeStagingBytes : Cfg::kStagingBytes))));
   uint64_t* full_bar = bars;
   uint64_t* empty_bar = bars + Cfg::kMaxStages;
   uint64_t* tmem_full = bars + 2 * Cfg::kMaxStages;
@@ -984,9 +987,12 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
     };
     // Float32 route (GemmParams::xpose): this warp's shared-memory tile, and the lane-contiguous asynchronous copies that bring
     // the gate logits (32 rows x 64 bytes) and the residual (32 rows x 128 bytes) of one 32-column chunk into it.
-    uint8_t* xp_res = s_stage_out + (warp - 2) * 6144;
-    uint8_t* xp_gate = xp_res + 4096;
+    uint8_t *xp_res = s_stage_out + (warp - 2) * 6144, *xp_gate = xp_res + 4096;
     int xp_nb = 0, xp_o = 0, xp_b = 0;
+    auto xp_chunk = [&](int i) {
+      xp_res = s_stage_out + (i * kEpiWarps + warp - 2) * 6144;
+      xp_gate = xp_res + 4096;
+    };
     auto xp_fetch = [&](int out_col) {
       const EpiSeg& s0 = p.seg[0];
       const int n_first = xp_nb * kBM + quad * 32;
@@ -1032,7 +1038,13 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       if constexpr (kXpose) {
         const int out_col = n_tile * BN + chunk_phase * 32;
         xp_nb = nb; xp_o = o; xp_b = b;
-        if (p.xpose && chunk_phase * 32 < BN && out_col + 32 <= p.seg[0].ncols) xp_fetch(out_col);
+        // (both chunks of the warp, a group of copies each: fetched after the first, the second's trip to memory had shown in the epilogue)
+#pragma unroll
+        for (int i = 0; i < (BN == 128 ? 2 : 1); ++i) {
+          xp_chunk(i);
+          if (p.xpose && chunk_phase * 32 < BN && out_col + i * 64 + 32 <= p.seg[0].ncols) xp_fetch(out_col + i * 64);
+          ptx::cp_async_commit();
+        }
       }
       if (!ptx::mbar_wait(&tmem_full[acc], acc_phase, 104)) { ok = false; break; }
       if (threadIdx.x == 64) KFB_GSTAMP(4 + tile_iter * 4 + 0);
@@ -1429,7 +1441,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         bool xp = false;
         if constexpr (kXpose) {
           xp = p.xpose != 0 && out_col + 32 <= p.seg[0].ncols;   // uniform across the warp
-          if (xp && c != chunk_phase * 32) xp_fetch(out_col);     // (the first chunk's copies went out before the accumulator was ready)
+          xp_chunk(c >> 6);
         }
         float v[32];
         if (GLU && !PRECISE) {
@@ -1555,7 +1567,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
         if constexpr (kXpose) {
           if (xp) {
             const int rl = lane;   // this thread's row within the warp's 32
-            ptx::cp_async_wait_all();
+            if (BN == 128 && c < 64) ptx::cp_async_wait_le1();
+            else ptx::cp_async_wait_all();
             __syncwarp();
             if (p.gate != nullptr) {
               const uint8_t* grow = xp_gate + rl * 64;
