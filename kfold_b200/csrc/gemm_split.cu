@@ -241,8 +241,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   }
   ptx::tc_fence_before_sync();
   __syncwarp();
-  if (split > 1) ptx::cluster_sync();
-  else __syncthreads();
+  ptx::cluster_sync();
   if (warp == 1) {
     ptx::tc_fence_after_sync();
     ptx::tmem_dealloc(tmem, kTmemCols);
@@ -254,7 +253,7 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       float4 acc = make_float4(0.f, 0.f, 0.f, 0.f);
 #pragma unroll 4
       for (int s = 0; s < split; ++s) {
-        const float4 v = ld_cluster(cluster_addr(s_part + it.off, split > 1 ? s : ptx::cluster_ctarank()));
+        const float4 v = ld_cluster(cluster_addr(s_part + it.off, s));
         acc.x += v.x; acc.y += v.y; acc.z += v.z; acc.w += v.w;
       }
       if (!it.live) continue;
@@ -276,23 +275,19 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       *reinterpret_cast<float4*>(reinterpret_cast<float*>(sg.dst) + it.at) = acc;
     }
   }
-  if (split > 1) {     // nobody leaves while a partial tile is still being read
-    __syncwarp();
-    ptx::cluster_sync();
-  }
+  __syncwarp();
+  ptx::cluster_sync();     // nobody leaves while a partial tile is still being read
 }
 
 template <int BN, bool PRECISE>
 struct SplitLauncher {
   // clusters of `split` CTAs that the device holds at once (0: the size cannot be launched)
-  static int resident(int split) {
+  static int resident(int dev, int split) {
     static std::once_flag once[64];
     static int held[64][kMaxSplit + 1];
-    int dev = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess) return 0;
     std::call_once(once[dev & 63], [&] {
       if (cudaFuncSetAttribute(gemm_split_kernel<BN, PRECISE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg<BN>::kSmem) != cudaSuccess) return;
-      for (int s = 1; s <= kMaxSplit; ++s) {
+      for (int s = 2; s <= kMaxSplit; ++s) {
         cudaLaunchAttribute attr[1];
         attr[0].id = cudaLaunchAttributeClusterDimension;
         attr[0].val.clusterDim.x = s;
@@ -317,9 +312,9 @@ struct SplitLauncher {
 };
 
 template <bool PRECISE>
-int resident(int bn, int split) {
-  return bn == 32 ? SplitLauncher<32, PRECISE>::resident(split) : bn == 64 ? SplitLauncher<64, PRECISE>::resident(split)
-                                                                             : SplitLauncher<128, PRECISE>::resident(split);
+int resident(int dev, int bn, int split) {
+  return bn == 32 ? SplitLauncher<32, PRECISE>::resident(dev, split) : bn == 64 ? SplitLauncher<64, PRECISE>::resident(dev, split)
+                                                                                  : SplitLauncher<128, PRECISE>::resident(dev, split);
 }
 
 }  // namespace
@@ -336,15 +331,20 @@ SplitPlan split_plan(const GemmParams& p, bool plain_operands, double other_cycl
                   (p.gate == nullptr || (p.g_col == 1 && p.g_n % 4 == 0 && p.g_o % 4 == 0 && p.g_b % 4 == 0 &&
                                          (reinterpret_cast<uintptr_t>(p.gate) & (p.precise ? 15 : 7)) == 0));
   if (!ok) return best;
-  const int blocks = cdiv(p.precise ? p.k_extent / 6 : p.k_extent, kBK);
+  const int blocks = cdiv(p.precise ? p.k_extent / 6 : p.k_extent, kBK), sms = sm_count();
   double least = 0.8 * other_cycles;
+  // (cheapest first: the two K blocks of a least share and what comes beside them do not fit)
+  if (blocks < 2 || least < split_cycles(p.precise, 32, 1) + 2500.0) return best;
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) return best;
   for (int bn = 32; bn <= 128; bn *= 2) {
-    const long long tiles = static_cast<long long>(p.num_m_tiles) * cdiv(p.n_cols, bn);
+    const int tiles = p.num_m_tiles * cdiv(p.n_cols, bn);
     for (int s : {2, 3, 4, 6, 8}) {
-      if (s > blocks || tiles * s > sm_count()) continue;
+      if (s > blocks || static_cast<long long>(tiles) * s > sms) break;
       // beside the main loop: barriers and launch, element groups one after the other, partial tiles of the others at 16 B per cycle
       const double t = split_cycles(p.precise, bn, cdiv(blocks, s)) + 2000.0 + 500.0 * cdiv(bn, 8 * s) + 32.0 * bn * (s - 1) / s;
-      if (t < least && tiles <= (p.precise ? resident<true>(bn, s) : resident<false>(bn, s))) {
+      // (a cluster's CTAs share a GPC: 24 clusters of six need not all fit, though 144 CTAs do)
+      if (t < least && tiles <= (p.precise ? resident<true>(dev, bn, s) : resident<false>(dev, bn, s))) {
         least = t;
         best = {bn, s};
       }
