@@ -64,8 +64,8 @@ def algorithmic_work(n: int | None = None, c: int = C_Z, h: int = 4, cs: int = C
         "layernorm_rows": ("hbm", 2.0 * p * c * 2),
         "layernorm_cm": ("hbm", 2.0 * p * c * 2),
         "layernorm_cm_stats": ("hbm", 1.0 * p * c * 2 + p * 8),   # read t, write (mean, rstd) per position
-        "trimul_in_proj": ("hbm", 3.0 * p * c * 2),            # read x~, write a and b
-        "trimul_gate_proj": ("hbm", 2.0 * p * c * 2),          # read x~, write the gate logits
+        "trimul_in_proj": ("hbm", (4.0 if c <= 128 else 3.0) * p * c * 2),   # read x~, write a and b (c <= 128: and the gate logits)
+        "trimul_gate_proj": ("hbm", 2.0 * p * c * 2),          # read x~, write the gate logits (c > 128)
         "trimul_out_proj": ("hbm", 4.0 * p * c * 2),           # read LN(t), gate logits, residual; write out
         "triatt_proj": ("hbm", 5.0 * p * c * 2 + p * h * 2),   # read x~; write q, k, g, v^T and the bias
         "triatt_out_proj": ("hbm", 3.0 * p * c * 2),           # read gated o, residual; write out
