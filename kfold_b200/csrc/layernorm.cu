@@ -680,8 +680,7 @@ __global__ void __launch_bounds__(256) layernorm_cm_split_kernel(const float* __
 // ------------------------------------------------------------------------------------------------
 // SPLIT: the result as a bf16 triple split (an A operand's row of six times c, see part_a) for the fp32-accurate projections.
 template <typename TI, typename TO, typename TG, int G, bool SPLIT>
-__global__ void __launch_bounds__(256) adaln_rows_kernel(const TI* __restrict__ a, TO* __restrict__ y,
-                                                         const TG* __restrict__ gv, long long gv_ld, long long rows, int c,
+__global__ void __launch_bounds__(256) adaln_rows_kernel(const TI* a, TO* y, const TG* gv, long long gv_ld, long long rows, int c,
                                                          int samples, int l, float eps) {
   grid_dependency_enter();
   const int lane = threadIdx.x & 31;
@@ -740,6 +739,8 @@ __global__ void __launch_bounds__(256) adaln_rows_kernel(const TI* __restrict__ 
 // 0.5 + 0.5 tanh(g / 2) on the MUFU (one op instead of an exponential and a reciprocal; relative error 5e-4, below the
 // bf16 rounding of the result).  LANES = 32: one row per warp; LANES = 16 (CH = 1, c = 128: the atom transformer):
 // two rows per warp.
+// Nothing here is __restrict__: behind a wait the compiler moved loads of `a` through such a pointer ahead of it, and `gv` stands behind
+// the wait as well where the launch before may be the one that writes it (an AdaLN by itself: its gate / shift projection).
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -756,9 +757,8 @@ __device__ __forceinline__ void load8(const float* p, float (&f)[8]) {
   f[0] = lo.x; f[1] = lo.y; f[2] = lo.z; f[3] = lo.w; f[4] = hi.x; f[5] = hi.y; f[6] = hi.z; f[7] = hi.w;
 }
 template <typename TI, int CH, int LANES>
-__global__ void __launch_bounds__(256) adaln_vec_kernel(const TI* a /*no __restrict__: its loads must stay behind the wait*/, __nv_bfloat16* y,
-                                                        const __nv_bfloat16* __restrict__ gv, long long gv_ld, long long rows,
-                                                        int samples, int l, float eps, int gv_static) {
+__global__ void __launch_bounds__(256) adaln_vec_kernel(const TI* a, __nv_bfloat16* y, const __nv_bfloat16* gv, long long gv_ld,
+                                                        long long rows, int samples, int l, float eps, int gv_static) {
   constexpr int c = 8 * LANES * CH;
   constexpr int kRowsPerWarp = 32 / LANES;
   const int lane = threadIdx.x & 31;

@@ -59,8 +59,9 @@ int launch_layernorm_cm(cudaStream_t stream, const void* t, __nv_bfloat16* y, co
 // Adaptive LayerNorm: y[r] = sigmoid(g[s(r)]) * LN(a[r]) + v[s(r)], LN without affine, fp32 statistics.
 // a, y: `rows` rows of c channels; gv: rows_s rows of [2c] (gate logits | shift), bf16.  Row r of a uses row
 // (r / (samples * l)) * l + r % l of gv: the conditioning is shared by the `samples` diffusion samples.
-// gv_static: a launch of this library lies between the last write of gv and this call.  gv_ld: elements between consecutive gv rows (0 = 2c), for rows that are slices of a wider table.  in_dtype KFB_FP32_PRECISE: a
-// and gv fp32, y fp32 rows, or (out_dtype KFB_FP32_PRECISE) bf16 triple-split rows of 6c.
+// gv_static: a launch of this library lies between the last write of gv and this call.  gv_ld: elements between consecutive gv rows
+// (0 = 2c), for rows that are slices of a wider table.  in_dtype KFB_FP32_PRECISE: a and gv fp32, y fp32 rows, or (out_dtype
+// KFB_FP32_PRECISE) bf16 triple-split rows of 6c.
 int launch_adaln(cudaStream_t stream, const void* a, void* y, const void* gv, long long rows, int c, int samples,
                  int l, float eps, int in_dtype, int out_dtype, long long gv_ld = 0, int gv_static = 0);
 

@@ -389,3 +389,31 @@ def test_pair_bias_in_one_pass(dev, n, batch, c, heads, transposed):
     ref = ref.transpose(-1, -2) if transposed else ref
     # operands and result are rounded to bf16, 2^-9 of themselves each: the sum's error stays within six sigma of c independent roundings
     assert (out.double() - ref).abs().max() <= 2.0 ** -8 * ref.abs().max() + 6 * 2.0 ** -9
+
+
+@pytest.mark.parametrize("l,samples,c", [(96, 1, 768), (301, 2, 1024), (700, 3, 768), (1000, 4, 128), (64, 3, 256), (130, 1, 384)])
+def test_adaln_behind_its_projection_in_a_captured_graph(dev, l, samples, c):
+    """A replay has the projection of the gate / shift rows and the AdaLN that reads them back to back; every replay gets another
+    conditioning, so that rows read too early are the last replay's.  One and several rows per warp, up to 592 blocks and more, and
+    the kernel for other widths."""
+    from kfold_b200 import modules as M
+    from kfold_b200.graphs import GraphedCall
+    g = torch.Generator().manual_seed(l)
+    mod = M.AdaLN(c, 384)
+    w = {k: torch.randn(p.shape, generator=g) * (p.shape[-1] ** -0.5 if p.dim() == 2 else 0.1) + (1.0 if k == "layernorm_s.weight" else 0.0)
+         for k, p in mod.state_dict().items()}
+    mod.load_state_dict(w, strict=True)
+    mod = mod.to(dev)
+
+    def three(a_, s_):
+        with torch.autocast("cuda", dtype=torch.bfloat16):
+            return tuple(mod(a_, s_[i]) for i in range(3))
+
+    a = torch.randn(1, samples, l, c, generator=g)
+    graphed = GraphedCall(three, a.to(dev), torch.zeros(3, 1, 1, l, 384, device=dev))
+    for _ in range(3):
+        s = torch.randn(3, 1, 1, l, 384, generator=g)
+        outs = graphed(a.to(dev), s.to(dev))
+        for i in range(3):
+            ref = _oracle_on(dev, O.adaln, a, s[i].expand(1, samples, l, 384).contiguous(), w)
+            _check(*err_stats(outs[i].float().cpu(), ref), f"AdaLN L={l} x {samples}, C={c}")
