@@ -24,8 +24,7 @@ __device__ __forceinline__ float warp_sum(float v) {
 // code 900 in the device status word instead of reading out of bounds.
 static constexpr int kBadIndexCode = 900;
 template <typename TX, typename TO>
-__global__ void __launch_bounds__(256) tokens_to_atoms_kernel(const TX* __restrict__ x, const long long* __restrict__ index,
-                                                              const TO* __restrict__ addend, TO* __restrict__ out, long long rows,
+__global__ void __launch_bounds__(256) tokens_to_atoms_kernel(const TX* x, const long long* index, const TO* addend, TO* out, long long rows,
                                                               int n_atom, int n_token, int d, int index_div) {
   grid_dependency_enter();
   const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
@@ -41,22 +40,42 @@ __global__ void __launch_bounds__(256) tokens_to_atoms_kernel(const TX* __restri
   if constexpr (sizeof(TX) == sizeof(TO)) {
     constexpr int kVec = 16 / sizeof(TX);
     if (addend == nullptr && d % kVec == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0) {
-      for (int i = lane * kVec; i < d; i += 32 * kVec)
-        *reinterpret_cast<uint4*>(dst + i) = ok ? *reinterpret_cast<const uint4*>(src + i) : make_uint4(0, 0, 0, 0);
+      for (int i0 = lane * kVec; i0 < d; i0 += 4 * 32 * kVec) {       // (four loads before the first store)
+        uint4 piece[4];
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u * 32 * kVec;
+          piece[u] = ok && i < d ? *reinterpret_cast<const uint4*>(src + i) : make_uint4(0, 0, 0, 0);
+        }
+#pragma unroll
+        for (int u = 0; u < 4; ++u) {
+          const int i = i0 + u * 32 * kVec;
+          if (i < d) *reinterpret_cast<uint4*>(dst + i) = piece[u];
+        }
+      }
       return;
     }
   }
   const TO* add = addend == nullptr ? nullptr : addend + row * d;
-  for (int i = lane; i < d; i += 32) st_f(dst + i, (ok ? ld_f(src + i) : 0.f) + (add != nullptr ? ld_f(add + i) : 0.f));
+  for (int i0 = lane; i0 < d; i0 += 128) {
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = min(i0 + 32 * u, d - 1);
+      v[u] = (ok ? ld_f(src + i) : 0.f) + (add != nullptr ? ld_f(add + i) : 0.f);
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + 32 * u < d) st_f(dst + i0 + 32 * u, v[u]);
+  }
 }
 
 // out[row][:] = q[qrow][:] + sum_k w[:, k] r[row][k], fp32 out: the coordinate embedding added to the atom features
 // (row r of out uses row (r / (samples * l)) * l + r % l of q and of the optional atom mask: the samples share them).
 // One warp per row.
 template <typename TQ>
-__global__ void __launch_bounds__(256) coord_embed_kernel(const TQ* __restrict__ q, const float* __restrict__ r,
-                                                          const float* __restrict__ w, const unsigned char* __restrict__ mask,
-                                                          float* __restrict__ out, long long rows, int c, int kc, int samples, int l) {
+__global__ void __launch_bounds__(256) coord_embed_kernel(const TQ* q, const float* r, const float* w, const unsigned char* mask, float* out,
+                                                          long long rows, int c, int kc, int samples, int l) {
   grid_dependency_enter();
   const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -65,20 +84,26 @@ __global__ void __launch_bounds__(256) coord_embed_kernel(const TQ* __restrict__
   float rv[8] = {0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f, 0.f};
   const bool keep = mask == nullptr || mask[qrow] != 0;   // coordinates of padding atoms count as zero
   for (int k = 0; k < kc; ++k) rv[k] = keep ? r[row * kc + k] : 0.f;
-  for (int i = lane; i < c; i += 32) {
-    float acc = 0.f;
-    for (int k = 0; k < kc; ++k) acc = fmaf(rv[k], w[i * kc + k], acc);   // same order as a dot product over k
-    out[row * c + i] = ld_f(q + qrow * c + i) + acc;
+  for (int i0 = lane; i0 < c; i0 += 128) {
+    float v[4];
+#pragma unroll
+    for (int u = 0; u < 4; ++u) {
+      const int i = min(i0 + 32 * u, c - 1);
+      float acc = 0.f;
+      for (int k = 0; k < kc; ++k) acc = fmaf(rv[k], w[i * kc + k], acc);   // same order as a dot product over k
+      v[u] = ld_f(q + qrow * c + i) + acc;
+    }
+#pragma unroll
+    for (int u = 0; u < 4; ++u)
+      if (i0 + 32 * u < c) out[row * c + i0 + 32 * u] = v[u];
   }
 }
 
 // out[row][j] = sum_i LayerNorm(x[row])[i] w[j][i], j < n_out <= 8, everything fp32 after the load: the projection of the
 // atom features to coordinate updates.  One warp per row; the row is re-read from L1 for the three passes.
 template <typename T>
-__global__ void __launch_bounds__(256) ln_project_kernel(const T* __restrict__ x, const float* __restrict__ ln_w,
-                                                         const float* __restrict__ ln_b, const float* __restrict__ w,
-                                                         const unsigned char* __restrict__ mask, float* __restrict__ out,
-                                                         long long rows, int c, int n_out, float eps, int samples, int l) {
+__global__ void __launch_bounds__(256) ln_project_kernel(const T* x, const float* ln_w, const float* ln_b, const float* w,
+                                                         const unsigned char* mask, float* out, long long rows, int c, int n_out, float eps, int samples, int l) {
   grid_dependency_enter();
   const long long row = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   if (row >= rows) return;
@@ -116,13 +141,13 @@ __global__ void __launch_bounds__(256) ln_project_kernel(const T* __restrict__ x
 // Per (index row, token): the first and last valid atom that maps to the token (first > last: none).  The mean below
 // then scans only that range; it still tests every atom in it, so unsorted indices stay correct, and for the usual
 // sorted atom order the range is just the token's own atoms.
-__global__ void __launch_bounds__(256) token_range_init_kernel(int2* __restrict__ range, long long n) {
+__global__ void __launch_bounds__(256) token_range_init_kernel(int2* range, long long n) {
   grid_dependency_enter();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i < n) range[i] = make_int2(0x7fffffff, -1);
 }
-__global__ void __launch_bounds__(256) token_range_kernel(const long long* __restrict__ index, const unsigned char* __restrict__ mask,
-                                                          int2* __restrict__ range, long long total, int n_atom, int n_token) {
+__global__ void __launch_bounds__(256) token_range_kernel(const long long* index, const unsigned char* mask, int2* range, long long total,
+                                                          int n_atom, int n_token) {
   grid_dependency_enter();
   const long long i = static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x;
   if (i >= total) return;
@@ -161,10 +186,9 @@ __device__ __forceinline__ void ld_vec(const __nv_bfloat16* p, float (&v)[VEC]) 
 // scheduling.  Latency-bound (a token has about eight atoms): rows are loaded four at a time, and the channels are spread over
 // warps, where one warp walked 768 channels in three passes, a row at a time (55 us for 96 tokens).
 template <typename T, int VEC>
-__global__ void __launch_bounds__(256) atoms_to_tokens_kernel(const T* __restrict__ x, const long long* __restrict__ index,
-                                                              const unsigned char* __restrict__ mask, T* __restrict__ out,
+__global__ void __launch_bounds__(256) atoms_to_tokens_kernel(const T* x, const long long* index, const unsigned char* mask, T* out,
                                                               long long rows, int n_atom, int n_token, int d, int index_div,
-                                                              int relu, const int2* __restrict__ range, int pieces) {
+                                                              int relu, const int2* range, int pieces) {
   grid_dependency_enter();
   const long long item = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   const long long row = item / pieces;

@@ -110,7 +110,7 @@ __device__ __forceinline__ Item<R> load_item(const RowsParams& p, int item) {
   bool empty = false;     // a row without valid keys: its result is the uniform average over all keys
 #pragma unroll
   for (int g = 0; g < R; ++g) {
-    const int2 r = __ldg(p.rows + it.b0 + min(g, it.rows - 1));
+    const int2 r = p.rows[it.b0 + min(g, it.rows - 1)];
     it.first[g] = r.y;
     most = max(most, r.x);
     empty = empty || r.x == 0;
@@ -561,7 +561,7 @@ attention_rows_kernel(const __grid_constant__ CUtensorMap tm_q, const __grid_con
 // rows), 13.8 us for 768 x 768 keys between CUDA events (about 4 of them the events'), twice a block; now 10.4, once.
 constexpr int kMaskWarps = 32;
 // blockIdx.y == 1: the same of the transposed mask (the ending node's), behind the first result.
-__global__ void __launch_bounds__(32 * kMaskWarps) mask_rows_kernel(AttnParams a, int2* __restrict__ rows) {
+__global__ void __launch_bounds__(32 * kMaskWarps) mask_rows_kernel(AttnParams a, int2* rows) {
   grid_dependency_enter();
   if (blockIdx.y == 1) {
     const long long m_lo = a.m_lo;

@@ -62,6 +62,10 @@ int sm_count();  // multiprocessors of the current device (cached per device)
 // 310 -> 454 us; the bf16 LayerNorm of a 768-token pair tensor 152 -> 187 us).
 // Every kernel launched this way executes griddepcontrol.wait before it touches memory that the stream's earlier work wrote or
 // reads, and griddepcontrol.launch_dependents only after that wait: what lies two or more kernels back is then always complete.
+// Such a kernel has no __restrict__ pointer and reads nothing through __ldg or ld.global.nc: both promise that nobody else writes the
+// data while the kernel lives, which the launch before it does until the wait, and the compiler may then move the loads ahead of the
+// wait (it did: the rows of adaln_vec_kernel).  What the promise gave, loads that overtake earlier stores, is written out where it
+// matters: a row's loads stand before its first store.
 // cluster: CTAs per thread-block cluster (along x).
 template <typename... KArgs, typename... Args>
 inline int launch_kernel_clustered(cudaStream_t stream, void (*kernel)(KArgs...), unsigned cluster, dim3 grid, dim3 block, size_t smem,

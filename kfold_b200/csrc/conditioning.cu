@@ -9,8 +9,7 @@ namespace {
 
 // out[row][j] = cos(2 pi t[row] w[j] + b[j]): the random Fourier features of the noise level.  The argument is
 // reduced exactly by cospif (cos(pi x) with x = 2 t w + b / pi), so large |t w| loses nothing to range reduction.
-__global__ void __launch_bounds__(256) fourier_embed_kernel(const float* __restrict__ t, const float* __restrict__ w,
-                                                            const float* __restrict__ b, float* __restrict__ out, int rows, int dim) {
+__global__ void __launch_bounds__(256) fourier_embed_kernel(const float* t, const float* w, const float* b, float* out, int rows, int dim) {
   grid_dependency_enter();
   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
   if (idx >= rows * dim) return;
@@ -20,8 +19,8 @@ __global__ void __launch_bounds__(256) fourier_embed_kernel(const float* __restr
 }
 
 // out[g][n][l][:] = s[g][l][:] + f[g][n][:]   (token conditioning plus the per-sample noise embedding), fp32
-__global__ void __launch_bounds__(256) broadcast_add_kernel(const float* __restrict__ s, const float* __restrict__ f,
-                                                            float* __restrict__ out, long long total, int samples, int l, int c) {
+__global__ void __launch_bounds__(256) broadcast_add_kernel(const float* s, const float* f, float* out, long long total, int samples, int l,
+                                                            int c) {
   grid_dependency_enter();
   const long long idx = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   if (idx >= total) return;

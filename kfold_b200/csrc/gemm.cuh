@@ -836,7 +836,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       const int n = row_block(at) * kBM + r;
       if (p.rowmask == nullptr || tile >= total_tiles || n >= p.n_extent) return 1u;
       uint32_t raw;
-      asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(raw)
+      asm volatile("ld.global.u8 %0, [%1];" : "=r"(raw)
                    : "l"(p.rowmask + static_cast<long long>(at.b) * p.m_b + static_cast<long long>(at.o) * p.m_o + static_cast<long long>(n) * p.m_n));
       return raw;
     };
@@ -933,7 +933,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
             const float4* bias = reinterpret_cast<const float4*>(p.col_bias + out_col_tile + c0);
 #pragma unroll
             for (int q4 = 0; q4 < 8; ++q4) {
-              const float4 u = __ldg(bias + q4);
+              const float4 u = bias[q4];
               x[4 * q4] = __float_as_uint(__uint_as_float(x[4 * q4]) + u.x);
               x[4 * q4 + 1] = __float_as_uint(__uint_as_float(x[4 * q4 + 1]) + u.y);
               x[4 * q4 + 2] = __float_as_uint(__uint_as_float(x[4 * q4 + 2]) + u.z);
@@ -980,7 +980,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       const int n = row_block(t) * kBM + r;
       if (n >= p.n_extent) return 1u;
       uint32_t raw;
-      asm volatile("ld.global.nc.u8 %0, [%1];" : "=r"(raw)
+      asm volatile("ld.global.u8 %0, [%1];" : "=r"(raw)
                    : "l"(p.rowmask + static_cast<long long>(t.b) * p.m_b + static_cast<long long>(t.o) * p.m_o +
                          static_cast<long long>(n) * p.m_n));
       return raw;
@@ -1213,7 +1213,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
               const float4* b1 = reinterpret_cast<const float4*>(p.col_bias + out_col_tile + c + 64);
 #pragma unroll
               for (int q4 = 0; q4 < 8; ++q4) {
-                const float4 u0 = __ldg(b0 + q4), u1 = __ldg(b1 + q4);
+                const float4 u0 = b0[q4], u1 = b1[q4];
                 r0[4 * q4] = __float_as_uint(__uint_as_float(r0[4 * q4]) + u0.x);
                 r0[4 * q4 + 1] = __float_as_uint(__uint_as_float(r0[4 * q4 + 1]) + u0.y);
                 r0[4 * q4 + 2] = __float_as_uint(__uint_as_float(r0[4 * q4 + 2]) + u0.z);
@@ -1307,14 +1307,14 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           for (int i = 0; i < 16; ++i) v[i] = __uint_as_float(vv[i]);
           if (p.col_bias != nullptr) {
 #pragma unroll
-            for (int i = 0; i < 16; ++i) v[i] += __ldg(p.col_bias + out_col + i);
+            for (int i = 0; i < 16; ++i) v[i] += p.col_bias[out_col + i];
           }
           if (STATS || p.row_stats != nullptr) {   // folded LayerNorm of the A rows (see GemmParams)
             const float4* s1 = reinterpret_cast<const float4*>(p.col_s1 + out_col);
             const float4* s0 = reinterpret_cast<const float4*>(p.col_s0 + out_col);
 #pragma unroll
             for (int q = 0; q < 4; ++q) {
-              const float4 a1 = __ldg(s1 + q), a0 = __ldg(s0 + q);
+              const float4 a1 = s1[q], a0 = s0[q];
               v[4 * q] = fmaf(stats.y, fmaf(-stats.x, a1.x, v[4 * q]), a0.x);
               v[4 * q + 1] = fmaf(stats.y, fmaf(-stats.x, a1.y, v[4 * q + 1]), a0.y);
               v[4 * q + 2] = fmaf(stats.y, fmaf(-stats.x, a1.z, v[4 * q + 2]), a0.z);
@@ -1345,9 +1345,9 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
               if (p.resid_scale != nullptr) {
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
-                  v[h * 8 + j * 2] = fmaf(__uint_as_float(w[j] << 16), __ldg(p.resid_scale + out_col + h * 8 + j * 2), v[h * 8 + j * 2]);
+                  v[h * 8 + j * 2] = fmaf(__uint_as_float(w[j] << 16), p.resid_scale[out_col + h * 8 + j * 2], v[h * 8 + j * 2]);
                   v[h * 8 + j * 2 + 1] =
-                      fmaf(__uint_as_float(w[j] & 0xffff0000u), __ldg(p.resid_scale + out_col + h * 8 + j * 2 + 1), v[h * 8 + j * 2 + 1]);
+                      fmaf(__uint_as_float(w[j] & 0xffff0000u), p.resid_scale[out_col + h * 8 + j * 2 + 1], v[h * 8 + j * 2 + 1]);
                 }
               } else {
 #pragma unroll
@@ -1518,7 +1518,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           const float4* s0 = reinterpret_cast<const float4*>(p.col_s0 + out_col);
 #pragma unroll
           for (int q = 0; q < 8; ++q) {
-            const float4 a1 = __ldg(s1 + q), a0 = __ldg(s0 + q);
+            const float4 a1 = s1[q], a0 = s0[q];
             v[4 * q] = fmaf(st.y, fmaf(-st.x, a1.x, v[4 * q]), a0.x);
             v[4 * q + 1] = fmaf(st.y, fmaf(-st.x, a1.y, v[4 * q + 1]), a0.y);
             v[4 * q + 2] = fmaf(st.y, fmaf(-st.x, a1.z, v[4 * q + 2]), a0.z);
@@ -1650,7 +1650,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 #pragma unroll
               for (int q = 0; q < 8; ++q) {
                 const float4 f = rs[q];
-                const float4 sc = p.resid_scale != nullptr ? __ldg(reinterpret_cast<const float4*>(p.resid_scale + out_col + q * 4))
+                const float4 sc = p.resid_scale != nullptr ? *reinterpret_cast<const float4*>(p.resid_scale + out_col + q * 4)
                                                            : make_float4(1.f, 1.f, 1.f, 1.f);
                 v[q * 4] = fmaf(f.x, sc.x, v[q * 4]); v[q * 4 + 1] = fmaf(f.y, sc.y, v[q * 4 + 1]);
                 v[q * 4 + 2] = fmaf(f.z, sc.z, v[q * 4 + 2]); v[q * 4 + 3] = fmaf(f.w, sc.w, v[q * 4 + 3]);
@@ -1664,8 +1664,8 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
 #pragma unroll
                 for (int j = 0; j < 4; ++j) {
                   const float2 f = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&w[j]));
-                  const float sx = p.resid_scale != nullptr ? __ldg(p.resid_scale + out_col + q * 8 + j * 2) : 1.0f;
-                  const float sy = p.resid_scale != nullptr ? __ldg(p.resid_scale + out_col + q * 8 + j * 2 + 1) : 1.0f;
+                  const float sx = p.resid_scale != nullptr ? p.resid_scale[out_col + q * 8 + j * 2] : 1.0f;
+                  const float sy = p.resid_scale != nullptr ? p.resid_scale[out_col + q * 8 + j * 2 + 1] : 1.0f;
                   v[q * 8 + j * 2] = fmaf(f.x, sx, v[q * 8 + j * 2]);
                   v[q * 8 + j * 2 + 1] = fmaf(f.y, sy, v[q * 8 + j * 2 + 1]);
                 }

@@ -262,8 +262,8 @@ gemm_split_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
       else if (j == 1) e = pre[1];
       else e = fetch(it);
       if (p.col_bias != nullptr) {
-        acc.x += __ldg(p.col_bias + it.col); acc.y += __ldg(p.col_bias + it.col + 1);
-        acc.z += __ldg(p.col_bias + it.col + 2); acc.w += __ldg(p.col_bias + it.col + 3);
+        acc.x += p.col_bias[it.col]; acc.y += p.col_bias[it.col + 1];
+        acc.z += p.col_bias[it.col + 2]; acc.w += p.col_bias[it.col + 3];
       }
       if (p.gate != nullptr) {
         acc.x *= PRECISE ? sigmoidf_exact(e.gate.x) : sigmoidf_fast(e.gate.x);

@@ -45,10 +45,8 @@ __device__ __forceinline__ float warp_sum(float v) {
 
 // One warp per row; lane l holds channel pairs (l + 32 g) * 2, g < G.
 template <typename TI, typename TO, int G, bool PERM>
-__global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* __restrict__ x, TO* __restrict__ y,
-                                                             const float* __restrict__ w, const float* __restrict__ b,
-                                                             long long rows, int c, long long xs, long long ys, float eps,
-                                                             RowPerm perm) {
+__global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* x, TO* y, const float* w, const float* b, long long rows, int c,
+                                                             long long xs, long long ys, float eps, RowPerm perm) {
   grid_dependency_enter();
   const int lane = threadIdx.x & 31;
   const long long warps_per_grid = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
@@ -83,23 +81,21 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* __restric
       orow = (static_cast<long long>(q) * perm.rows + i) * perm.rows + (rest - q * perm.rows);
     }
     TO* yr = y + orow * ys;
+    // (scale and offset of the whole row before its first store: behind one, a load waits for it)
 #pragma unroll
     for (int g = 0; g < G; ++g) {
       const int ch = (lane + 32 * g) * 2;
       if (ch < c) {
-        float a0 = v[g].x * rstd, a1 = v[g].y * rstd;
-        if (w != nullptr) {
-          const float2 ww = *reinterpret_cast<const float2*>(w + ch);
-          a0 *= ww.x;
-          a1 *= ww.y;
-        }
-        if (b != nullptr) {
-          const float2 bb = *reinterpret_cast<const float2*>(b + ch);
-          a0 += bb.x;
-          a1 += bb.y;
-        }
-        store2<TO>(yr + ch, a0, a1);
+        const float2 ww = w != nullptr ? *reinterpret_cast<const float2*>(w + ch) : make_float2(1.f, 1.f);
+        const float2 bb = b != nullptr ? *reinterpret_cast<const float2*>(b + ch) : make_float2(0.f, 0.f);
+        v[g].x = fmaf(v[g].x * rstd, ww.x, bb.x);
+        v[g].y = fmaf(v[g].y * rstd, ww.y, bb.y);
       }
+    }
+#pragma unroll
+    for (int g = 0; g < G; ++g) {
+      const int ch = (lane + 32 * g) * 2;
+      if (ch < c) store2<TO>(yr + ch, v[g].x, v[g].y);
     }
   }
 }
@@ -153,8 +149,7 @@ int launch_ln_fold_weights(cudaStream_t stream, const LnFold& f) {
 // The pair track's shape: 128 bf16 channels, contiguous rows.  A row is 256 bytes = 16 lanes x 16 bytes, so a warp takes two
 // rows per step and two steps per iteration: four rows (1 KB) in flight per warp, 16-byte loads and stores, the statistics
 // reduced over the 16 lanes of a row.  Same arithmetic as layernorm_rows_kernel (two passes, fp32).
-__global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
-                                                                  const float* __restrict__ w, const float* __restrict__ b,
+__global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const float* w, const float* b,
                                                                   long long rows, float eps, int fold_blocks, const LnFold fold) {
   constexpr int LANES = 16, STEPS = 2, C = LANES * 8, kRows = 32 / LANES;
   grid_dependency_enter();
@@ -224,8 +219,7 @@ __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfl
 // rows; this one 130 (92 at the memory's rate; 16-byte accesses gave 96, but another order of summation: a last-bit difference that
 // four blocks of bf16 rounding turn into 0.8 % of the result).
 constexpr int kC256Rows = 4;
-__global__ void __launch_bounds__(256) layernorm_c256_bf16_kernel(const __nv_bfloat16* __restrict__ x, __nv_bfloat16* __restrict__ y,
-                                                                  const float* __restrict__ w, const float* __restrict__ b,
+__global__ void __launch_bounds__(256) layernorm_c256_bf16_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const float* w, const float* b,
                                                                   long long rows, float eps, int fold_blocks, const LnFold fold) {
   constexpr int G = 4, C = 256;
   grid_dependency_enter();
@@ -268,12 +262,7 @@ __global__ void __launch_bounds__(256) layernorm_c256_bf16_kernel(const __nv_bfl
       __nv_bfloat16* yr = y + (base + r) * C;
 #pragma unroll
       for (int g = 0; g < G; ++g) {
-        float a0 = v[r][g].x * rstd, a1 = v[r][g].y * rstd;
-        a0 *= ww[g].x;
-        a1 *= ww[g].y;
-        a0 += bb[g].x;
-        a1 += bb[g].y;
-        store2<__nv_bfloat16>(yr + (lane + 32 * g) * 2, a0, a1);
+        store2<__nv_bfloat16>(yr + (lane + 32 * g) * 2, fmaf(v[r][g].x * rstd, ww[g].x, bb[g].x), fmaf(v[r][g].y * rstd, ww[g].y, bb[g].y));
       }
     }
   }
@@ -358,9 +347,9 @@ int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w
 // 768 x 768 rows of 128 channels, between CUDA events: LayerNorm 56 + GEMM 44 us -> 54 in one launch; 400 x 400 of 256: 45 + 28 -> 43.
 // (The unpacked rows live in registers, 128 and 254 of them; held to 64 or 80 they spill: 72 us.)
 template <int C>
-__global__ void __launch_bounds__(256) ln_heads_kernel(const __nv_bfloat16* __restrict__ z, const float* __restrict__ ln_w,
-                                                       const float* __restrict__ ln_b, const __nv_bfloat16* __restrict__ w, const HeadsOut out,
-                                                       int rows, int o_extent, int n_extent, int heads, float eps) {
+__global__ void __launch_bounds__(256) ln_heads_kernel(const __nv_bfloat16* z, const float* ln_w, const float* ln_b,
+                                                       const __nv_bfloat16* w, const HeadsOut out, int rows, int o_extent, int n_extent,
+                                                       int heads, float eps) {
   constexpr int Q = C / 32, kWLd = C + 8;       // (rows of the weights 16 bytes off: eight of them cover the banks)
   __shared__ __align__(16) __nv_bfloat16 s_w[16 * kWLd];
   __shared__ __align__(16) float s_g[C], s_b[C];
@@ -475,7 +464,7 @@ int launch_ln_heads(cudaStream_t stream, const void* z, const float* ln_w, const
 }
 
 // fp32 -> bf16 conversion, eight elements per thread (HBM-bound; the conditioning rows of a stack: one small launch).
-__global__ void __launch_bounds__(256) to_bf16_kernel(const float* __restrict__ x, __nv_bfloat16* __restrict__ y, long long n) {
+__global__ void __launch_bounds__(256) to_bf16_kernel(const float* x, __nv_bfloat16* y, long long n) {
   grid_dependency_enter();
   const long long i = (static_cast<long long>(blockIdx.x) * 256 + threadIdx.x) * 8;
   if (i + 8 <= n) {
@@ -514,8 +503,7 @@ __device__ __forceinline__ void split3_store(__nv_bfloat16* y6, int c, int ch, f
 // HBM-bound; 25 600 rows of 128 float32 channels 13 -> 6 us against the form below, which reads a row three times, channel by
 // channel, and remains for rows that are not whole aligned pieces of four.
 template <typename TI, int G>
-__global__ void __launch_bounds__(256) layernorm_split_vec_kernel(const TI* __restrict__ x, __nv_bfloat16* __restrict__ y6,
-                                                                  const float* __restrict__ w, const float* __restrict__ b,
+__global__ void __launch_bounds__(256) layernorm_split_vec_kernel(const TI* x, __nv_bfloat16* y6, const float* w, const float* b,
                                                                   long long rows, int c, long long xs, float eps, int normalise) {
   grid_dependency_enter();
   const int lane = threadIdx.x & 31;
@@ -549,17 +537,21 @@ __global__ void __launch_bounds__(256) layernorm_split_vec_kernel(const TI* __re
     }
     __nv_bfloat16* yr = y6 + row * 6 * c;
 #pragma unroll
+    for (int g = 0; g < G; ++g) {      // (before the row's first store, as above)
+      const int ch = (lane + 32 * g) * 4;
+#pragma unroll
+      for (int i = 0; i < 4; ++i)
+        v[g][i] = fmaf((v[g][i] - mean) * rstd, w != nullptr && ch < c ? w[ch + i] : 1.f, b != nullptr && ch < c ? b[ch + i] : 0.f);
+    }
+#pragma unroll
     for (int g = 0; g < G; ++g) {
       const int ch = (lane + 32 * g) * 4;
       if (ch >= c) continue;
       uint16_t parts[3][4];
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
-        float o = (v[g][i] - mean) * rstd;
-        if (w != nullptr) o *= w[ch + i];
-        if (b != nullptr) o += b[ch + i];
         __nv_bfloat16 x0, x1, x2;
-        split3(o, x0, x1, x2);
+        split3(v[g][i], x0, x1, x2);
         parts[0][i] = __bfloat16_as_ushort(x0);
         parts[1][i] = __bfloat16_as_ushort(x1);
         parts[2][i] = __bfloat16_as_ushort(x2);
@@ -573,8 +565,7 @@ __global__ void __launch_bounds__(256) layernorm_split_vec_kernel(const TI* __re
 }
 
 template <typename TI>
-__global__ void __launch_bounds__(256) layernorm_split_kernel(const TI* __restrict__ x, __nv_bfloat16* __restrict__ y6,
-                                                              const float* __restrict__ w, const float* __restrict__ b,
+__global__ void __launch_bounds__(256) layernorm_split_kernel(const TI* x, __nv_bfloat16* y6, const float* w, const float* b,
                                                               long long rows, int c, long long xs, float eps, int normalise) {
   grid_dependency_enter();
   const int lane = threadIdx.x & 31;
@@ -595,11 +586,16 @@ __global__ void __launch_bounds__(256) layernorm_split_kernel(const TI* __restri
       rstd = 1.0f / sqrtf(warp_sum(q) / static_cast<float>(c) + eps);
     }
     __nv_bfloat16* yr = y6 + row * 6 * c;
-    for (int ch = lane; ch < c; ch += 32) {
-      float v = (load1(xr + ch) - mean) * rstd;
-      if (w != nullptr) v *= w[ch];
-      if (b != nullptr) v += b[ch];
-      split3_store(yr, c, ch, v);
+    for (int c0 = lane; c0 < c; c0 += 128) {
+      float v[4];
+#pragma unroll
+      for (int k = 0; k < 4; ++k) {
+        const int ch = min(c0 + 32 * k, c - 1);
+        v[k] = fmaf((load1(xr + ch) - mean) * rstd, w != nullptr ? w[ch] : 1.f, b != nullptr ? b[ch] : 0.f);
+      }
+#pragma unroll
+      for (int k = 0; k < 4; ++k)
+        if (c0 + 32 * k < c) split3_store(yr, c, c0 + 32 * k, v[k]);
     }
   }
 }
@@ -639,8 +635,7 @@ int launch_layernorm_split(cudaStream_t stream, const __nv_bfloat16* x, __nv_bfl
 // that loads and all six stores are whole sectors.  (One thread per position, two-byte stores 6 C apart, took 300 us for 160 x 160
 // positions of 128 channels; the 4 + 12 bytes per element take 8 at the memory's rate.)
 constexpr int kCmSplitPos = 32;
-__global__ void __launch_bounds__(256) layernorm_cm_split_kernel(const float* __restrict__ t, __nv_bfloat16* __restrict__ y6,
-                                                                 const float* __restrict__ w, const float* __restrict__ b,
+__global__ void __launch_bounds__(256) layernorm_cm_split_kernel(const float* t, __nv_bfloat16* y6, const float* w, const float* b,
                                                                  long long npos, int c, long long chan_stride,
                                                                  long long batch_stride, float eps, int blocks_per_batch) {
   grid_dependency_enter();
@@ -653,6 +648,13 @@ __global__ void __launch_bounds__(256) layernorm_cm_split_kernel(const float* __
   const bool in = p0 + lane < npos;
 #pragma unroll 8
   for (int ch = warp; ch < c; ch += 8) slab[ch * (kCmSplitPos + 1) + lane] = in ? tb[ch * chan_stride] : 0.f;
+  float gamma[8], beta[8];        // of the lane's channels (at most 256 in all)
+#pragma unroll
+  for (int k = 0; k < 8; ++k) {
+    const int ch = lane + 32 * k;
+    gamma[k] = w != nullptr && ch < c ? w[ch] : 1.f;
+    beta[k] = b != nullptr && ch < c ? b[ch] : 0.f;
+  }
   __syncthreads();
   for (int pp = warp; pp < kCmSplitPos && p0 + pp < npos; pp += 8) {
     const float* col = slab + pp;
@@ -666,11 +668,10 @@ __global__ void __launch_bounds__(256) layernorm_cm_split_kernel(const float* __
     }
     const float rstd = 1.0f / sqrtf(warp_sum(q) / static_cast<float>(c) + eps);
     __nv_bfloat16* yr = y6 + (static_cast<long long>(batch) * npos + p0 + pp) * 6 * c;
-    for (int ch = lane; ch < c; ch += 32) {
-      float v = (col[ch * (kCmSplitPos + 1)] - mean) * rstd;
-      if (w != nullptr) v *= w[ch];
-      if (b != nullptr) v += b[ch];
-      split3_store(yr, c, ch, v);
+#pragma unroll
+    for (int k = 0; k < 8; ++k) {
+      const int ch = lane + 32 * k;
+      if (ch < c) split3_store(yr, c, ch, fmaf((col[ch * (kCmSplitPos + 1)] - mean) * rstd, gamma[k], beta[k]));
     }
   }
 }
@@ -739,8 +740,7 @@ __global__ void __launch_bounds__(256) adaln_rows_kernel(const TI* a, TO* y, con
 // 0.5 + 0.5 tanh(g / 2) on the MUFU (one op instead of an exponential and a reciprocal; relative error 5e-4, below the
 // bf16 rounding of the result).  LANES = 32: one row per warp; LANES = 16 (CH = 1, c = 128: the atom transformer):
 // two rows per warp.
-// Nothing here is __restrict__: behind a wait the compiler moved loads of `a` through such a pointer ahead of it, and `gv` stands behind
-// the wait as well where the launch before may be the one that writes it (an AdaLN by itself: its gate / shift projection).
+// `gv` stands behind the wait where the launch before may be the one that writes it (an AdaLN by itself: its gate / shift projection).
 __device__ __forceinline__ void unpack8(const uint4& u, float (&f)[8]) {
   const uint32_t w[4] = {u.x, u.y, u.z, u.w};
 #pragma unroll
@@ -924,10 +924,8 @@ __device__ __forceinline__ uint32_t cm_pack(float lo, float hi) {
 }
 
 template <typename TI>
-__global__ void __launch_bounds__(kCmPos) layernorm_cm_kernel(const TI* __restrict__ t, __nv_bfloat16* __restrict__ y,
-                                                              const float* __restrict__ w, const float* __restrict__ b,
-                                                              long long npos, int c, long long chan_stride,
-                                                              long long batch_stride, float eps, int blocks_per_batch) {
+__global__ void __launch_bounds__(kCmPos) layernorm_cm_kernel(const TI* t, __nv_bfloat16* y, const float* w, const float* b, long long npos, int c,
+                                                              long long chan_stride, long long batch_stride, float eps, int blocks_per_batch) {
   grid_dependency_enter();
   extern __shared__ __align__(16) unsigned char slab_raw[];
   __nv_bfloat16* slab = reinterpret_cast<__nv_bfloat16*>(slab_raw);  // [c][128]
@@ -1003,8 +1001,8 @@ __global__ void __launch_bounds__(kCmPos) layernorm_cm_kernel(const TI* __restri
 // warps for it (gemm.cuh, STATS); cm_stats does where it has not.
 // ------------------------------------------------------------------------------------------------
 // (mean, rstd) over the channels of every position of a channel-major tensor t[c][npos]; two positions per thread
-__global__ void __launch_bounds__(256) cm_stats_kernel(const __nv_bfloat16* __restrict__ t, float2* __restrict__ stats,
-                                                       long long npos, int c, long long chan_stride, float eps) {
+__global__ void __launch_bounds__(256) cm_stats_kernel(const __nv_bfloat16* t, float2* stats, long long npos, int c, long long chan_stride,
+                                                       float eps) {
   grid_dependency_enter();
   const long long p2 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 2;
   if (p2 >= npos) return;
@@ -1041,8 +1039,8 @@ __global__ void __launch_bounds__(256) cm_stats_kernel(const __nv_bfloat16* __re
 
 // The same with four positions per thread (8-byte loads): half as many CTAs, all resident at once for a 768 x 768 pair
 // tensor, and twice the bytes in flight per thread.  npos and the channel stride multiples of 4, t 8-byte aligned.
-__global__ void __launch_bounds__(128) cm_stats4_kernel(const __nv_bfloat16* __restrict__ t, float2* __restrict__ stats,
-                                                        long long npos, int c, long long chan_stride, float eps) {
+__global__ void __launch_bounds__(128) cm_stats4_kernel(const __nv_bfloat16* t, float2* stats, long long npos, int c, long long chan_stride,
+                                                        float eps) {
   grid_dependency_enter();
   const long long p4 = (static_cast<long long>(blockIdx.x) * blockDim.x + threadIdx.x) * 4;
   if (p4 >= npos) return;
@@ -1111,9 +1109,8 @@ template <> __device__ __forceinline__ float from_float<float>(float v) { return
 // positions contiguous).  bf16 mode rounds the normalised value to bf16 as the reference's LayerNorm does and
 // accumulates in fp32; fp32 mode keeps everything in fp32.
 template <int C, typename T>
-__global__ void __launch_bounds__(256) window_bias_kernel(const T* __restrict__ x, const float* __restrict__ ln_w,
-                                                          const float* __restrict__ ln_b, const T* __restrict__ w,
-                                                          T* __restrict__ y, long long npos, int nh, float eps, int normalise) {
+__global__ void __launch_bounds__(256) window_bias_kernel(const T* x, const float* ln_w, const float* ln_b, const T* w, T* y, long long npos,
+                                                          int nh, float eps, int normalise) {
   grid_dependency_enter();
   extern __shared__ float s_w[];  // [nh][C] fp32, then gamma[C], beta[C]
   float* s_g = s_w + nh * C;
