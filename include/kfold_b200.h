@@ -13,7 +13,8 @@
  *   - returns an `int` status (KFB_OK = 0); never throws, exits or synchronises
  *     the device (except kfb_device_status, which is a deliberate sync);
  *   - allocates nothing: every temporary lives in a caller-provided workspace
- *     whose size the matching `*_workspace_bytes` function reports;
+ *     whose size the matching `*_workspace_bytes` function reports; a larger
+ *     one is taken too, and what lies past that size is left alone;
  *   - launches on the stream passed in; safe to call from several host threads
  *     on different streams;
  *   - `dtype` is KFB_BF16 or KFB_FP32 and describes activations in and out;

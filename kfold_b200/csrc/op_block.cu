@@ -57,11 +57,13 @@ KFB_API int kfb_pair_block_fwd(const kfb_pair_block* blk, const void* z, void* z
   KFB_CHECK_ARG(workspace_bytes >= need, "pair_block: workspace %zu < %zu bytes", workspace_bytes, need);
   const size_t ob = operator_bytes(k, batch, n, precise);
   const long long pos = static_cast<long long>(batch) * n * n, rows = static_cast<long long>(batch) * n;
+  // (inside the operators' scratch, behind what the triangle multiplication takes of it)
+  void* fold_room = precise ? nullptr : static_cast<uint8_t*>(workspace) + kfb_trimul_workspace_bytes(batch, n, k.c);
   const void* cur = z;
   for (int dir = 0; dir < 2; ++dir) {
     const kfb_trimul_weights& w = dir ? k.mul_in : k.mul_out;
-    KFB_TRY(kfb_trimul_fwd(dir, cur, pair_mask, w.ln_in_w, w.ln_in_b, w.w_in, w.w_gout, w.ln_out_w, w.ln_out_b, w.w_pout, z_out, cur,
-                           workspace, ob, batch, n, k.c, k.eps, z_dtype, stream));
+    KFB_TRY(trimul_run(as_stream(stream), dir, cur, pair_mask, w.ln_in_w, w.ln_in_b, w.w_in, w.w_gout, w.ln_out_w, w.ln_out_b, w.w_pout, z_out,
+                       cur, workspace, ob, batch, n, k.c, k.eps, z_dtype, fold_room));
     cur = z_out;
   }
   // the mask scans of both directions in one launch, after the operators' scratch

@@ -327,6 +327,41 @@ int trimul_precise(cudaStream_t stream, int incoming, const void* x, const unsig
 
 }  // namespace
 
+namespace kfb {
+int trimul_run(cudaStream_t stream, int incoming, const void* x, const unsigned char* mask, const float* ln_in_w, const float* ln_in_b,
+               const void* w_in_packed, const void* w_gout, const float* ln_out_w, const float* ln_out_b, const void* w_pout, void* out,
+               const void* resid, void* workspace, size_t workspace_bytes, int batch, int n, int c, float eps, int dtype, void* fold_room) {
+  KFB_CHECK_ARG(x && mask && w_in_packed && w_gout && w_pout && out && workspace, "trimul: null pointer");
+  KFB_CHECK_ARG(is_dtype(dtype), "trimul: bad dtype %d", dtype);
+  // any N on the bf16 path (except tensors too small for the folded LayerNorm's scratch), multiples of 8 otherwise
+  const bool ragged_ok = dtype != KFB_FP32_PRECISE && n >= 24;
+  KFB_TRY(check_shape("trimul", batch, ragged_ok ? pitch8(n) : n, ragged_ok ? pitch8(n) : n, c));
+  if (dtype == KFB_FP32_PRECISE) {
+    KFB_CHECK_ARG(c <= 256, "trimul: the fp32-accurate mode supports at most 256 channels");
+    TrimulWsPrecise wp;
+    const size_t need_p = carve_precise(wp, workspace, batch, n, c);
+    KFB_CHECK_ARG(workspace_bytes >= need_p, "trimul: workspace %zu < %zu bytes", workspace_bytes, need_p);
+    KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "trimul: workspace must be 256-byte aligned");
+    return trimul_precise(stream, incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, ln_out_w, ln_out_b, w_pout, out, resid, wp,
+                          batch, n, c, eps);
+  }
+  TrimulWs w;
+  const size_t need = carve(w, workspace, batch, n, c);
+  KFB_CHECK_ARG(workspace_bytes >= need, "trimul: workspace %zu < %zu bytes", workspace_bytes, need);
+  KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "trimul: workspace must be 256-byte aligned");
+  // The output projection's weights with its LayerNorm folded in: by the first launch where the caller has room for them, otherwise by a
+  // launch of their own into the normalised rows once those are used (3 us, whatever the size).
+  Carver room(fold_room);
+  __nv_bfloat16* wf = room.take<__nv_bfloat16>(static_cast<size_t>(c) * c);
+  float* sums = room.take<float>(2 * static_cast<size_t>(c));
+  const LnFold fold = {static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, wf, sums, sums + c, c, c};
+  const LnFold* early = fold_room != nullptr ? &fold : nullptr;
+  KFB_TRY(project(stream, incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, w.xn, w.ab, w.gl, batch, n, n, c, eps, dtype, 0, 1, early));
+  return finish(stream, w.ab, w.ab + static_cast<long long>(c) * batch * n * pitch8(n), n, 0, w.gl, ln_out_w, ln_out_b, w_pout, w.t, w.xn, out,
+                resid, batch, n, n, c, eps, dtype, early);
+}
+}  // namespace kfb
+
 extern "C" {
 
 KFB_API size_t kfb_trimul_workspace_bytes_precise(int batch, int n, int c) {
@@ -342,37 +377,9 @@ KFB_API size_t kfb_trimul_workspace_bytes(int batch, int n, int c) {
 KFB_API int kfb_trimul_fwd(int incoming, const void* x, const unsigned char* mask, const float* ln_in_w, const float* ln_in_b,
                            const void* w_in_packed, const void* w_gout, const float* ln_out_w, const float* ln_out_b,
                            const void* w_pout, void* out, const void* resid, void* workspace, size_t workspace_bytes,
-                           int batch, int n, int c, float eps, int dtype, void* stream_) {
-  KFB_CHECK_ARG(x && mask && w_in_packed && w_gout && w_pout && out && workspace, "trimul: null pointer");
-  KFB_CHECK_ARG(is_dtype(dtype), "trimul: bad dtype %d", dtype);
-  // any N on the bf16 path (except tensors too small for the folded LayerNorm's scratch), multiples of 8 otherwise
-  const bool ragged_ok = dtype != KFB_FP32_PRECISE && n >= 24;
-  KFB_TRY(check_shape("trimul", batch, ragged_ok ? pitch8(n) : n, ragged_ok ? pitch8(n) : n, c));
-  if (dtype == KFB_FP32_PRECISE) {
-    KFB_CHECK_ARG(c <= 256, "trimul: the fp32-accurate mode supports at most 256 channels");
-    TrimulWsPrecise wp;
-    const size_t need_p = carve_precise(wp, workspace, batch, n, c);
-    KFB_CHECK_ARG(workspace_bytes >= need_p, "trimul: workspace %zu < %zu bytes", workspace_bytes, need_p);
-    KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "trimul: workspace must be 256-byte aligned");
-    return trimul_precise(as_stream(stream_), incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, ln_out_w, ln_out_b,
-                          w_pout, out, resid, wp, batch, n, c, eps);
-  }
-  TrimulWs w;
-  const size_t need = carve(w, workspace, batch, n, c);
-  KFB_CHECK_ARG(workspace_bytes >= need, "trimul: workspace %zu < %zu bytes", workspace_bytes, need);
-  KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "trimul: workspace must be 256-byte aligned");
-  cudaStream_t stream = as_stream(stream_);
-  // The output projection's weights with its LayerNorm folded in: by the first launch into what lies behind the workspace, where the
-  // caller gave that much more (the pair blocks do), otherwise by a launch of their own into the normalised rows once those are used.
-  const bool early = workspace_bytes >= need + trimul_fold_bytes(c);
-  Carver behind(static_cast<uint8_t*>(workspace) + need);
-  __nv_bfloat16* wf = behind.take<__nv_bfloat16>(static_cast<size_t>(c) * c);
-  float* sums = behind.take<float>(2 * static_cast<size_t>(c));
-  const LnFold fold = {static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, wf, sums, sums + c, c, c};
-  KFB_TRY(project(stream, incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, w.xn, w.ab, w.gl, batch, n, n, c, eps, dtype, 0, 1,
-                  early ? &fold : nullptr));
-  return finish(stream, w.ab, w.ab + static_cast<long long>(c) * batch * n * pitch8(n), n, 0, w.gl, ln_out_w, ln_out_b, w_pout, w.t, w.xn, out,
-                resid, batch, n, n, c, eps, dtype, early ? &fold : nullptr);
+                           int batch, int n, int c, float eps, int dtype, void* stream) {
+  return trimul_run(as_stream(stream), incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, ln_out_w, ln_out_b, w_pout, out, resid,
+                    workspace, workspace_bytes, batch, n, c, eps, dtype, nullptr);
 }
 
 KFB_API int kfb_trimul_project(const void* x, const unsigned char* mask, const float* ln_in_w, const float* ln_in_b,

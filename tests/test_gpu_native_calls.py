@@ -417,3 +417,33 @@ def test_adaln_behind_its_projection_in_a_captured_graph(dev, l, samples, c):
         for i in range(3):
             ref = _oracle_on(dev, O.adaln, a, s[i].expand(1, samples, l, 384).contiguous(), w)
             _check(*err_stats(outs[i].float().cpu(), ref), f"AdaLN L={l} x {samples}, C={c}")
+
+
+@pytest.mark.parametrize("n,batch,c", [(24, 1, 64), (65, 2, 128), (40, 1, 256)])
+def test_nothing_is_written_past_the_reported_workspace(dev, monkeypatch, n, batch, c):
+    """A caller may pass an arena whose tail holds something else: the triangle multiplication by itself, and in a block, whose workspace
+    has room for its folded weights, leave that tail as it was and give the same result."""
+    from kfold_b200 import functional as F
+    from kfold_b200 import modules as M
+    from kfold_b200 import packing
+    import synth
+    arenas = []
+
+    def arena(device, nbytes, most_kept=None):
+        arenas.append((torch.full((nbytes + tail,), 0xAB, dtype=torch.uint8, device=device), nbytes))
+        return arenas[-1][0]
+
+    monkeypatch.setattr(F, "_workspace", arena)
+    z, pm, _ = synth.pair_inputs(n, n, c, batch)
+    z, pm = z.bfloat16().to(dev), pm.to(dev)
+    pk = packing.pack_trimul(synth.trimul_weights(synth._Rng(n), c), dev)
+    torch.manual_seed(n)
+    block = M.TriangularBlock(c).to(dev)
+    for call in (lambda: F.triangle_multiplication(z, pm, pk, "outgoing"), lambda: F.triangle_multiplication(z, pm, pk, "incoming"),
+                 lambda: block(z, pm)):
+        results = []
+        for tail in (0, 1 << 20):
+            results.append(call())
+            ws, nbytes = arenas[-1]
+            assert (ws[nbytes:] == 0xAB).all()
+        assert torch.equal(*results)
