@@ -11,20 +11,19 @@
 
 namespace kfb {
 
-template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false, bool PAIR = false, bool TWIN = false>
-static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* tout,
-                          const GemmParams& p, const char* tag) {
-  using Cfg = GemmCfg<BN, PAIR>;
+// Tiles in flight: CTAs, or pairs of them, that the current device holds at once (0: it holds no pair).  Once per device and kernel, whose
+// shared memory it also allows.
+template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP, bool STATS, bool PAIR, bool TWIN>
+static int tiles_held(int* held) {
   constexpr auto kernel = gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP, STATS, PAIR, TWIN>;
-  constexpr int threads = TWIN ? kTwinThreads : AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads;
   static std::once_flag once[64];
-  static int resident[64];      // tiles in flight: CTAs, or pairs of them, that the device holds at once
+  static int resident[64];
   int dev = 0;
   KFB_CUDA(cudaGetDevice(&dev));
   cudaError_t attr_err = cudaSuccess;
   std::call_once(once[dev & 63], [&] {
-    attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmemBytes);
-    resident[dev & 63] = sm_count();
+    attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN, PAIR>::kSmemBytes);
+    resident[dev & 63] = attr_err == cudaSuccess ? sm_count() : 0;
     if (PAIR && attr_err == cudaSuccess) {     // (a multiprocessor without a neighbour to pair with stays idle)
       cudaLaunchAttribute attr[1];
       attr[0].id = cudaLaunchAttributeClusterDimension;
@@ -32,17 +31,29 @@ static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUte
       attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
       cudaLaunchConfig_t cfg = {};
       cfg.gridDim = sm_count() / 2 * 2;
-      cfg.blockDim = threads;
-      cfg.dynamicSmemBytes = Cfg::kSmemBytes;
+      cfg.blockDim = gemm_threads<AUX, STATS, TWIN>();
+      cfg.dynamicSmemBytes = GemmCfg<BN, PAIR>::kSmemBytes;
       cfg.attrs = attr;
       cfg.numAttrs = 1;
       attr_err = cudaOccupancyMaxActiveClusters(&resident[dev & 63], kernel, &cfg);
     }
   });
   KFB_CUDA(attr_err);
-  KFB_CHECK_ARG(resident[dev & 63] > 0, "GEMM: the device holds no CTA pair");
+  *held = resident[dev & 63];
+  return KFB_OK;
+}
+
+template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false, bool PAIR = false, bool TWIN = false>
+static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUtensorMap& tb, const CUtensorMap* tout,
+                          const GemmParams& p, const char* tag) {
+  using Cfg = GemmCfg<BN, PAIR>;
+  constexpr auto kernel = gemm_bf16_kernel<BN, GLU, AUX, PRECISE, SWAP, STATS, PAIR, TWIN>;
+  constexpr int threads = gemm_threads<AUX, STATS, TWIN>();
+  int held = 0;
+  KFB_TRY((tiles_held<BN, GLU, AUX, PRECISE, SWAP, STATS, PAIR, TWIN>(&held)));
+  KFB_CHECK_ARG(held > 0, "GEMM: the device holds no tile of this kernel");
   const int total = p.num_m_tiles * p.num_n_tiles;
-  const int grid = total < resident[dev & 63] ? total : resident[dev & 63];     // (pairs count as one)
+  const int grid = total < held ? total : held;     // (pairs count as one)
   GemmParams q = p;
   {
     // the persistent loops step by the grid size: its digits in the (n tile, row block, outer, batch) index
@@ -154,7 +165,12 @@ static bool pair_tile(const GemmParams& p, int bn) {
     if (channel_major && (p.glu || ((p.mask_segs >> i) & 1) || (i == 0 && (p.gate != nullptr || p.resid != nullptr)))) return false;
     if (!channel_major && (sg.s_col != 1 || (i > 0 && p.seg[i - 1].s_n == 1 && p.seg[i - 1].s_col != 1))) return false;
   }
-  return true;
+  // (a device, or the part of one that this process may use, without two free multiprocessors in a cluster's reach; every pair kernel
+  // takes a multiprocessor's whole shared memory, so that one of them answers for all)
+  int held = 0;
+  const bool known = tiles_held<256, true, false, false, false, false, true, true>(&held) == KFB_OK;
+  if (!known) cudaGetLastError();
+  return known && held > 0;
 }
 
 static long long* g_trace_buf = nullptr;

@@ -107,6 +107,8 @@ static constexpr int kAuxThreads = kGemmThreads + 32;  // the AUX variant's last
 static constexpr int kStatsThreads = 64;               // the STATS variant's two warps after it: two rows of the tile per thread
 static constexpr int kStatsBytes = kBM * 8;            // (mean, rstd) of a tile's rows
 static constexpr int kTwinThreads = 64 + 2 * 32 * kEpiWarps + 64;   // the TWIN variant: two epilogue groups, a store warp for each
+template <bool AUX, bool STATS, bool TWIN>
+constexpr int gemm_threads() { return TWIN ? kTwinThreads : AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads; }
 
 template <int BN, bool PAIR = false>
 struct GemmCfg {
@@ -385,7 +387,7 @@ __device__ __forceinline__ void tile_advance(TileIdx& t, const GemmParams& p) {
 //         the tensor core multiplies them: a pass over A and a launch less (see the launcher for where and what it measured).  The
 //         sums run over the channels in order, as that pass does: the same bits.
 template <int BN, bool GLU, bool AUX, bool PRECISE, bool SWAP = false, bool STATS = false, bool PAIR = false, bool TWIN = false>
-__global__ void __launch_bounds__(TWIN ? kTwinThreads : AUX ? kAuxThreads + (STATS ? kStatsThreads : 0) : kGemmThreads, 1)
+__global__ void __launch_bounds__(gemm_threads<AUX, STATS, TWIN>(), 1)
 gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant__ CUtensorMap tm_b,
                  const __grid_constant__ CUtensorMap tm_out0, const __grid_constant__ CUtensorMap tm_out1,
                  const __grid_constant__ CUtensorMap tm_out2, const GemmParams p) {
