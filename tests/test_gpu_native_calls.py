@@ -357,6 +357,40 @@ def test_transition_of_cta_pairs(dev, rows):
     _check(*err_stats(out, x.float() + _oracle_on(dev, O.transition, x.float(), w)), f"transition rows={rows}")
 
 
+@pytest.mark.parametrize("m,n,k,ldd,shift,bias", [(9472, 512, 520, 512, 0, None), (9601, 776, 712, 776, 0, 0), (9601, 776, 712, 777, 0, None),
+                                                  (9473, 520, 456, 528, 4, None), (9600, 512, 448, 512, 0, 1)],
+                         ids=["one wave", "ragged columns with bias", "odd pitch", "destination off by 8 bytes", "bias off by 4 bytes"])
+def test_gemm_of_cta_pairs_with_one_epilogue_group(dev, m, n, k, ldd, shift, bias):
+    """Tiles of two CTAs that one group of warps takes: exactly one wave of them, or columns that the copy engine cannot store.  Nothing
+    is written between the rows."""
+    from kfold_b200 import _lib as L
+    g = torch.Generator(device=dev).manual_seed(m + n)
+    a = torch.randn(m, k, generator=g, device=dev).bfloat16()
+    w = torch.randn(n, k, generator=g, device=dev).bfloat16()
+    col_bias = None if bias is None else torch.randn(n + 4, generator=g, device=dev)[bias:bias + n]
+    buf = torch.full((m * ldd + 16,), 7.0, device=dev, dtype=torch.bfloat16)
+    d = buf[shift:shift + m * ldd].view(m, ldd)
+    L.check(L.lib().kfb_gemm_bf16(L.ptr(a), L.ptr(w), L.ptr(d), L.ptr(col_bias), 1, m, n, k, k, k, ldd, 0, 0, 0, 0, L.stream_ptr()))
+    prev = torch.backends.cuda.matmul.allow_tf32
+    torch.backends.cuda.matmul.allow_tf32 = False
+    ref = torch.matmul(a.float(), w.float().T) + (0.0 if col_bias is None else col_bias)
+    torch.backends.cuda.matmul.allow_tf32 = prev
+    # (the bound of the test above)
+    assert ((d[:, :n].float() - ref).abs() <= 1e-4 * k ** 0.5 + 2.0 ** -8 * ref.abs()).all()
+    assert (d[:, n:] == 7.0).all() and (buf[:shift] == 7.0).all() and (buf[shift + m * ldd:] == 7.0).all()
+
+
+def test_gated_tiles_of_cta_pairs_in_one_wave(dev):
+    """37 row blocks of pairs x 2 gated tiles: one for each pair that 148 multiprocessors hold."""
+    from kfold_b200 import functional as F
+    from kfold_b200 import packing
+    import synth
+    w = synth.transition_weights(synth._Rng(3), 256, 1)
+    x = torch.randn(1, 9472, 256, generator=torch.Generator().manual_seed(3)).bfloat16()
+    out = F.transition(x.to(dev), packing.pack_transition(w, dev)).float().cpu()
+    _check(*err_stats(out, _oracle_on(dev, O.transition, x.float(), w)), "transition in one wave of pairs")
+
+
 @pytest.mark.parametrize("m,n,k", [(1, 384, 1536), (64, 32, 520), (96, 768, 768), (130, 772, 1096), (300, 1024, 2048)])
 def test_gemm_with_k_shared_by_a_cluster(dev, m, n, k):
     """Few rows, float32 results: rows, columns and K that end inside a tile, shares of K of unequal length, one to three row blocks."""
