@@ -298,10 +298,15 @@ KFB_API int kfb_atoms_to_tokens(const void* x, const long long* token_index, con
                   "atoms_to_tokens: workspace too small or misaligned");
     range = static_cast<int2*>(workspace);
     const long long nr = static_cast<long long>(batch / index_div) * n_token, na = static_cast<long long>(batch / index_div) * n_atom;
-    LaunchScope scope_r(stream, "atoms_to_tokens_ranges");
-    KFB_TRY(launch_kernel(stream, token_range_init_kernel, static_cast<unsigned>((nr + 255) / 256), 256, 0, range, nr));
-    KFB_TRY(launch_kernel(stream, token_range_kernel, static_cast<unsigned>((na + 255) / 256), 256, 0, token_index, mask,
-        range, na, n_atom, n_token));
+    {
+      LaunchScope scope(stream, "atoms_to_tokens_ranges");
+      KFB_TRY(launch_kernel(stream, token_range_init_kernel, static_cast<unsigned>((nr + 255) / 256), 256, 0, range, nr));
+    }
+    {
+      LaunchScope scope(stream, "atoms_to_tokens_ranges");
+      KFB_TRY(launch_kernel(stream, token_range_kernel, static_cast<unsigned>((na + 255) / 256), 256, 0, token_index, mask, range, na, n_atom,
+                            n_token));
+    }
     KFB_CUDA(cudaGetLastError());
   }
   LaunchScope scope(stream, "atoms_to_tokens");

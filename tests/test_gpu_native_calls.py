@@ -167,16 +167,45 @@ def test_layernorm_bf16_rows(dev, c, rows):
 @pytest.mark.parametrize("d", [6, 130, 132, 768])
 def test_atoms_to_tokens_widths(dev, d):
     """The masked mean at widths that end inside a warp's channels and that are not whole vectors, with tokens of 0 to 40 atoms."""
+    from kfold_b200 import _lib as L
     from kfold_b200 import functional as F
     g = torch.Generator().manual_seed(d)
     index = torch.cat([torch.zeros(40, dtype=torch.long), torch.randint(2, 30, (160,), generator=g)]).sort().values.view(1, 200)
     mask = torch.rand(1, 200, generator=g) < 0.8
     x = torch.randn(1, 3, 200, d, generator=g)
+    launches = L.launch_count()
     out = F.aggregate_atoms_to_tokens(x.to(dev), index.to(dev), mask.to(dev), 31).cpu()
+    assert L.launch_count() - launches == 3      # two for the tokens' ranges of atoms
     for t in range(31):
         rows = x[:, :, (index[0] == t) & mask[0]]
         ref = rows.mean(2) if rows.shape[2] else torch.zeros(1, 3, d)
         assert torch.allclose(out[:, :, t], ref, atol=1e-5), t
+
+
+@pytest.mark.parametrize("d", [6, 130, 520, 1100])
+@pytest.mark.parametrize("x_dtype,add_dtype", [(torch.bfloat16, None), (torch.float32, None), (torch.bfloat16, torch.float32), (torch.float32, torch.float32)])
+def test_tokens_to_atoms_widths(dev, d, x_dtype, add_dtype):
+    """Rows that are no, one and several groups of four pieces, copied and with something added: exact, the sum of two rounded numbers."""
+    from kfold_b200 import functional as F
+    g = torch.Generator().manual_seed(d)
+    index = torch.randint(0, 9, (1, 65), generator=g)
+    x = torch.randn(1, 2, 9, d, generator=g).to(x_dtype)
+    add = None if add_dtype is None else torch.randn(1, 2, 65, d, generator=g).to(add_dtype)
+    out = F.broadcast_tokens_to_atoms(x.to(dev), index.to(dev), None if add is None else add.to(dev)).cpu()
+    ref = x[:, :, index[0]]
+    assert torch.equal(out, ref if add is None else (ref.float() + add.float()).to(out.dtype))
+
+
+@pytest.mark.parametrize("c", [6, 128, 130, 300])
+def test_coord_embed_widths(dev, c):
+    from kfold_b200 import functional as F
+    g = torch.Generator().manual_seed(c)
+    q, r, w = torch.randn(1, 37, c, generator=g), torch.randn(1, 3, 37, 6, generator=g), torch.randn(c, 6, generator=g)
+    mask = torch.rand(1, 37, generator=g) < 0.8
+    out = F.coord_embed(q.to(dev), r.to(dev), w.to(dev), mask.to(dev)).cpu()
+    q, r, w = q.double().unsqueeze(1), r.double() * mask[:, None, :, None], w.double()
+    # seven float32 roundings of partial sums that the magnitudes' sum bounds
+    assert ((out - (q + r @ w.T)).abs() <= 7 * 2.0 ** -24 * (q.abs() + r.abs() @ w.abs().T)).all()
 
 
 @pytest.mark.parametrize("bf16", [False, True])
