@@ -74,8 +74,8 @@ def algorithmic_work(n: int | None = None, c: int = C_Z, h: int = 4, cs: int = C
 
 
 # DRAM traffic of the triangle-attention kernel (attention_rows_kernel<3, 32>) from its ncu capture at N=768 (dram__bytes_read.sum +
-# dram__bytes_write.sum of one launch: 568.7 MB + 130.1 MB); it grows with the number of pair positions.
-NCU_TRAFFIC = {"triatt_attention": {"n": 768, "bytes": 568.657152e6 + 130.099712e6,
+# dram__bytes_write.sum of one launch: 568.5 MB + 128.9 MB); it grows with the number of pair positions.
+NCU_TRAFFIC = {"triatt_attention": {"n": 768, "bytes": 568.472320e6 + 128.862720e6,
                                      "source": "ncu capture at N=768 (profiles/attention_rows_ncu.md), scaled by pair positions at other sizes"}}
 
 

@@ -25,8 +25,9 @@
 //     previous one;
 //   * the key mask costs nothing where it masks nothing: a row's first masked and last valid key come from a scan kernel, the rank-1
 //     mask product is issued for the tiles that hold masked keys, and tiles after the last valid key are skipped.
-// N = 768 (4 heads): 1.15 -> 0.71 ms; N = 2048: 18.3 -> 11.9 ms (the exponentials alone: 0.40, 7.6).  The MUFU is busy 65 % of the
-// time; without exponentials a tile still takes 660 of 790 cycles, and neither the bias nor the value products change that.
+// N = 768 (4 heads): 1.15 -> 0.69 ms; N = 2048: 18.3 -> 11.4 ms (the exponentials alone: 0.40, 7.6), 790 cycles a tile.  The MUFU is
+// busy 59 % of a launch at N = 768 (ncu); without exponentials a tile still takes 660 cycles, and neither the bias nor the value
+// products change that.
 // Warps: 4 g .. 4 g + 3 softmax and output of row group g (a warp reads the tensor-memory lanes warp % 4); then the TMA producer, which
 // also writes the mask operands, and one MMA-issuing warp per group.
 // Tensor memory per row group: two S tiles, 64 fp32 columns each, overwritten in place by their P (64 bf16 = 32 columns), and O, 32
