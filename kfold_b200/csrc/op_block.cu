@@ -77,8 +77,8 @@ KFB_API int kfb_pair_block_fwd(const kfb_pair_block* blk, const void* z, void* z
     KFB_TRY(triatt_run(as_stream(stream), dir, cur, pair_mask, w.ln_w, w.ln_b, w.w_proj, w.w_out, z_out, cur, workspace, ob, batch, n, k.c,
                        k.tri_heads, k.eps, z_dtype, scans != nullptr ? scans + static_cast<long long>(dir) * batch * n : nullptr));
   }
-  KFB_TRY(kfb_transition_fwd(cur, k.trans_z.ln_w, k.trans_z.ln_b, k.trans_z.w_swiglu, k.trans_z.w_out, z_out, cur, workspace, ob, pos, k.c,
-                             k.hidden_z, k.eps, z_dtype, stream));
+  KFB_TRY(transition_run(as_stream(stream), cur, k.trans_z.ln_w, k.trans_z.ln_b, k.trans_z.w_swiglu, k.trans_z.w_out, z_out, cur, workspace, ob,
+                         pos, k.c, k.hidden_z, k.eps, z_dtype, 1));
   if (!k.has_single) return KFB_OK;
   // single track: its operands come after the operators' scratch
   uint8_t* extra = static_cast<uint8_t*>(workspace) + ob + mask_rows_bytes(k, batch, n);
@@ -102,8 +102,8 @@ KFB_API int kfb_pair_block_fwd(const kfb_pair_block* blk, const void* z, void* z
   r.workspace = workspace; r.workspace_bytes = ob;
   r.batch = batch; r.l = n; r.c = k.c_s; r.heads = k.heads; r.out_dtype = s_dtype;
   KFB_TRY(apb_run(as_stream(stream), r));
-  return kfb_transition_fwd(s_out, k.trans_s.ln_w, k.trans_s.ln_b, k.trans_s.w_swiglu, k.trans_s.w_out, s_out, s_out, workspace, ob, rows, k.c_s,
-                            k.hidden_s, k.eps, s_dtype, stream);
+  return transition_run(as_stream(stream), s_out, k.trans_s.ln_w, k.trans_s.ln_b, k.trans_s.w_swiglu, k.trans_s.w_out, s_out, s_out, workspace, ob,
+                        rows, k.c_s, k.hidden_s, k.eps, s_dtype, 1);
 }
 
 }  // extern "C"

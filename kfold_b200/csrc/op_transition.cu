@@ -3,6 +3,7 @@
 //   2. GEMM xn [Wa ; Wb]^T with the SwiGLU epilogue  h = silu(u_a) * u_b  (bf16)     [tcgen05]
 //   3. GEMM h W_out^T (+ optional residual)                                          [tcgen05]
 #include "ops_common.cuh"
+#include "transition_pair.cuh"
 
 using namespace kfb;
 
@@ -77,7 +78,16 @@ static int transition_precise(cudaStream_t stream, const void* x, const float* l
 
 KFB_API int kfb_transition_fwd(const void* x, const float* ln_w, const float* ln_b, const void* w_swiglu_packed,
                                const void* w_out, void* out, const void* resid, void* workspace, size_t workspace_bytes,
-                               long long rows, int c, int hidden, float eps, int dtype, void* stream_) {
+                               long long rows, int c, int hidden, float eps, int dtype, void* stream) {
+  return transition_run(as_stream(stream), x, ln_w, ln_b, w_swiglu_packed, w_out, out, resid, workspace, workspace_bytes, rows, c, hidden, eps,
+                        dtype, 0);
+}
+
+}  // extern "C"
+
+int kfb::transition_run(cudaStream_t stream, const void* x, const float* ln_w, const float* ln_b, const void* w_swiglu_packed,
+                        const void* w_out, void* out, const void* resid, void* workspace, size_t workspace_bytes, long long rows, int c,
+                        int hidden, float eps, int dtype, int w_static) {
   KFB_CHECK_ARG(x && w_swiglu_packed && w_out && out && workspace, "transition: null pointer");
   KFB_CHECK_ARG(is_dtype(dtype), "transition: bad dtype %d", dtype);
   KFB_CHECK_ARG(rows >= 1 && rows < (1ll << 31), "transition: rows %lld", rows);
@@ -85,14 +95,15 @@ KFB_API int kfb_transition_fwd(const void* x, const float* ln_w, const float* ln
   if (dtype == KFB_FP32_PRECISE) {
     KFB_CHECK_ARG(workspace_bytes >= kfb_transition_workspace_bytes_precise(rows, c, hidden), "transition: workspace too small");
     KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "transition: workspace must be 256-byte aligned");
-    return transition_precise(as_stream(stream_), x, ln_w, ln_b, w_swiglu_packed, w_out, out, resid, workspace, rows, c, hidden,
+    return transition_precise(stream, x, ln_w, ln_b, w_swiglu_packed, w_out, out, resid, workspace, rows, c, hidden,
                               eps);
   }
   TransWs w;
   const size_t need = carve(w, workspace, rows, c, hidden);
   KFB_CHECK_ARG(workspace_bytes >= need, "transition: workspace %zu < %zu bytes", workspace_bytes, need);
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "transition: workspace must be 256-byte aligned");
-  cudaStream_t stream = as_stream(stream_);
+  if (transition_pair_ok(x, w_swiglu_packed, w_out, out, resid, rows, c, hidden, dtype))
+    return launch_transition_pair(stream, x, ln_w, ln_b, w_swiglu_packed, w_out, out, resid, rows, c, hidden, eps, w_static);
   KFB_TRY(launch_layernorm(stream, x, w.xn, ln_w, ln_b, rows, c, c, c, eps, dtype, KFB_BF16));
   {
     GemmParams p = {};
@@ -126,8 +137,6 @@ KFB_API int kfb_transition_fwd(const void* x, const float* ln_w, const float* ln
   }
   return KFB_OK;
 }
-
-}  // extern "C"
 
 // ------------------------------------------------------------------------------------------------
 // Transition without a caller-provided workspace.

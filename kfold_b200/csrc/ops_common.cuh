@@ -73,6 +73,10 @@ size_t trimul_fold_bytes(int c);
 int trimul_run(cudaStream_t stream, int incoming, const void* x, const unsigned char* mask, const float* ln_in_w, const float* ln_in_b,
                const void* w_in_packed, const void* w_gout, const float* ln_out_w, const float* ln_out_b, const void* w_pout, void* out,
                const void* resid, void* workspace, size_t workspace_bytes, int batch, int n, int c, float eps, int dtype, void* fold_room);
+// kfb_transition_fwd; w_static as in ApbArgs.
+int transition_run(cudaStream_t stream, const void* x, const float* ln_w, const float* ln_b, const void* w_swiglu_packed, const void* w_out,
+                   void* out, const void* resid, void* workspace, size_t workspace_bytes, long long rows, int c, int hidden, float eps, int dtype,
+                   int w_static);
 // Whether these sizes take the attention kernel that scans the mask, and the scan for both directions in one launch: batch * n entries
 // of the starting node, then those of the ending node.
 bool triatt_scans_mask(int c, int heads, int n, int dtype);

@@ -1,0 +1,552 @@
+// The pair track's transition in one kernel: LayerNorm, both gated projections, SwiGLU, output projection, residual.  bf16 rows of 128
+// or 256 channels.
+//
+// What bounds it.  As three launches (LayerNorm, SwiGLU GEMM, output GEMM) it moved the normalised rows and four times as many hidden
+// activations through HBM: 1.5 GB for 768 x 768 rows of 128 channels, where reading and writing z is 0.3.  Here the hidden activations
+// never leave the SM, and the time is the tensor core's: 6 144 cycles per 128 rows of 128 channels, 24 576 of 256.
+//
+// Split.  A CTA pair (cta_group::2) takes 256 rows, 128 in each CTA, and walks the hidden channels in chunks of 64:
+//   S = LN(z) . [W_a; W_b]^T     256 x 128 (CTA 0 loads the chunk's 64 value rows, CTA 1 its 64 gate rows), K = C
+//   h = silu(S_a) S_b            softmax-style in place: a thread owns a row, h goes over S in tensor memory as bf16
+//   O += h . W_out^T             A from tensor memory, 256 x C, K = 64
+// With single CTAs each would load all of the weights: operand traffic, 128 bytes a cycle through a shared memory, is what the products
+// compete with (a chunk of 128 channels reads 56 KB of operands and is filled with 24 KB in 768 cycles of products; h in shared memory
+// would add 32).
+//   * S has three buffers of 128 columns (C = 128) or two (C = 256), which with O fill the tensor memory.  The tensor core runs ahead by
+//     all of them and executes in order, so a buffer needs no barrier of its own: its next S is issued behind the product that read its h.
+//   * Two groups of four SwiGLU warps take the chunks in turn.
+//   * Four more warps normalise the next tile's rows in place in shared memory (two buffers) while this one is multiplied, and turn the
+//     finished tile around: the residual comes back (from L2) into the tile's own buffer, which the products have left, is added, and the
+//     buffer leaves as it is.
+// The arithmetic and its order are those of layernorm_c128_bf16_kernel / layernorm_c256_bf16_kernel and of the GEMMs this replaces: the
+// same bits (four blocks of bf16 rounding turn a last bit into up to 1 % of the confidence head's result).
+#include <cuda_bf16.h>
+
+#include <mutex>
+
+#include "gemm.cuh"   // glu_half, pack_bf16x2
+#include "ptx.cuh"
+#include "transition_pair.cuh"
+
+namespace kfb {
+namespace {
+
+constexpr int kRows = 128;                 // rows of a CTA
+constexpr int kChunk = 64;                 // hidden channels of a chunk
+constexpr int kBox = kRows * 128;          // [128 rows][64 bf16], 128-byte swizzle
+constexpr int kSlot = 16384;               // unit of the weight ring: 128 columns of K of S's 64 weight rows, or a chunk's K of O's C / 2
+constexpr int kThreads = 512;              // producer, MMA, 2 idle (a warp reads the tensor-memory lanes warp % 4), 4 rows, 2 x 4 SwiGLU
+constexpr int kRowWarp = 4, kGluWarp = 8;
+
+template <int C>
+struct Cfg {
+  static constexpr int kABytes = (C / 64) * kBox;
+  static constexpr int kSlots = C == 128 ? 8 : 6;
+  static constexpr int kS = C == 128 ? 3 : 2;         // S buffers
+  static constexpr int kUnits = C / 128;              // ring units of a chunk's S
+  static constexpr int kOutUnit = (C / 2) * 128;      // bytes of a chunk's unit of W_out in a CTA
+  static constexpr int kSmem = 2 * kABytes + kSlots * kSlot + 512 + 1024;
+  static_assert(kSmem <= 232448, "shared memory");
+};
+
+struct PairTransParams {
+  const float *ln_w, *ln_b;
+  int rows, tiles, chunks, has_resid, w_static;
+  float eps;
+};
+
+template <int C>
+__global__ void __launch_bounds__(kThreads, 1)
+transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_constant__ CUtensorMap tm_w1, const __grid_constant__ CUtensorMap tm_w2,
+                       const __grid_constant__ CUtensorMap tm_r, const __grid_constant__ CUtensorMap tm_out, const PairTransParams p) {
+  using K = Cfg<C>;
+  constexpr int kLag = K::kS - 1;
+  extern __shared__ uint8_t smem_raw[];
+  uint8_t* s_a = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));   // [2][C / 64] boxes
+  uint8_t* s_w = s_a + 2 * K::kABytes;
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_w + K::kSlots * kSlot);
+  uint64_t* full = bars;                     // [slots], in the leader: both CTAs' copies
+  uint64_t* empty = full + K::kSlots;        // [slots]
+  uint64_t* s_full = empty + K::kSlots;      // [kS]
+  uint64_t* h_ready = s_full + K::kS;        // [kS], in the leader: 4 warps of each CTA
+  uint64_t* rows_in = h_ready + K::kS;       // [2] a tile's rows, or its residual, have arrived
+  uint64_t* a_ready = rows_in + 2;           // [2], in the leader: normalised rows
+  uint64_t* a_done = a_ready + 2;            // [2] every S of the tile
+  uint64_t* o_full = a_done + 2;
+  uint64_t* o_empty = o_full + 1;            // in the leader
+  uint64_t* out_done = o_empty + 1;          // the row warps have written the output tile
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(out_done + 1);
+  static_assert((2 * 8 + 2 * 3 + 9) * 8 + 4 <= 512, "barriers");
+
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int rank = static_cast<int>(ptx::cluster_ctarank());
+  const int tile0 = blockIdx.x >> 1, tile_step = gridDim.x >> 1;
+  const int my_tiles = (p.tiles - tile0 + tile_step - 1) / tile_step;      // (the grid has no pair without a tile)
+  const int total = my_tiles * p.chunks;
+
+  if (threadIdx.x == 0) {
+    ptx::prefetch_tmap(&tm_x);
+    ptx::prefetch_tmap(&tm_w1);
+    ptx::prefetch_tmap(&tm_w2);
+    ptx::prefetch_tmap(&tm_out);
+    for (int i = 0; i < K::kSlots; ++i) {
+      ptx::mbar_init(&full[i], 1);
+      ptx::mbar_init(&empty[i], 1);
+    }
+    for (int i = 0; i < K::kS; ++i) {
+      ptx::mbar_init(&s_full[i], 1);
+      ptx::mbar_init(&h_ready[i], 8);
+    }
+    for (int i = 0; i < 2; ++i) {
+      ptx::mbar_init(&rows_in[i], 1);
+      ptx::mbar_init(&a_ready[i], 8);
+      ptx::mbar_init(&a_done[i], 1);
+    }
+    ptx::mbar_init(o_full, 1);
+    ptx::mbar_init(o_empty, 8);
+    ptx::mbar_init(out_done, 4);
+    ptx::fence_barrier_init();
+  }
+  if (warp == 1) {
+    ptx::tmem_alloc_pair(tmem_slot, 512);
+    ptx::tmem_relinquish_pair();
+  }
+  ptx::tc_fence_before_sync();
+  __syncwarp();
+  ptx::cluster_sync();
+  ptx::tc_fence_after_sync();
+  const uint32_t tmem_base = *tmem_slot;
+  const uint32_t tmem_s = tmem_base + C;      // O lies before the S buffers
+
+  if (warp == 0) {
+    // ---------------------------------------------------------------- weights, in the order of the products.  Where they were written
+    // before the launch before this one, the first of them come while that one drains.
+    if (ptx::elect_one()) {
+      if (!p.w_static) grid_dependency_wait();
+      const int last = max((my_tiles - 1) * p.chunks, 2);      // the last tile, and a few chunks on their way
+      int slot = 0;
+      uint32_t par = 0;
+      bool ok = true;
+      auto unit = [&](const CUtensorMap* map, int bytes, int boxes, int col, int row) {
+        ok = ptx::mbar_wait(&empty[slot], par ^ 1, 401);
+        if (!ok) return;
+        if (rank == 0) ptx::mbar_expect_tx(&full[slot], 2 * bytes);
+        const uint32_t bar = ptx::leader_addr(&full[slot]);
+        for (int i = 0; i < boxes; ++i) ptx::tma_load_4d_pair(s_w + slot * kSlot + i * (bytes / boxes), map, bar, col + 64 * i, row, 0, 0);
+        if (++slot == K::kSlots) { slot = 0; par ^= 1u; }
+      };
+      int c1 = 0, c2 = 0;                     // chunk of the next S and of the next product with h
+      for (int i = 0; ok && i < total + kLag; ++i) {
+        if (i == last) {
+          grid_dependency_wait();             // (a kernel lets the next one start after its own wait)
+          grid_dependency_launch();
+        }
+        if (i < total) {
+          const int row = (c1 >> 1) * 256 + 128 * rank + (c1 & 1) * kChunk;
+          for (int u = 0; ok && u < K::kUnits; ++u) unit(&tm_w1, kSlot, 2, u * 128, row);
+          if (++c1 == p.chunks) c1 = 0;
+        }
+        if (ok && i >= kLag) {
+          unit(&tm_w2, K::kOutUnit, 1, c2 * kChunk, rank * (C / 2));
+          if (++c2 == p.chunks) c2 = 0;
+        }
+      }
+      // the last products' arrivals at this CTA's barriers, before it may exit
+      for (int i = 0; ok && i < K::kSlots; ++i) {
+        ok = ptx::mbar_wait(&empty[slot], par ^ 1, 402);
+        if (++slot == K::kSlots) { slot = 0; par ^= 1u; }
+      }
+    }
+  } else if (warp == 1) {
+    // ---------------------------------------------------------------- MMA issue
+    if (rank == 0 && ptx::elect_one()) {
+      constexpr uint32_t idesc_s = ptx::make_idesc(2 * kRows, 2 * kChunk, 1);
+      constexpr uint32_t idesc_o = ptx::make_idesc(2 * kRows, C, 1);
+      const uint64_t a_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_a));
+      const uint64_t w_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_w));
+      int slot = 0, c1 = 0, c2 = 0, s1 = 0, s2 = 0;
+      uint32_t par = 0, t1 = 0, t2 = 0, h_par = 0;    // t1, t2: tiles begun by S and by O
+      bool ok = true;
+      auto slot_wait = [&]() -> uint64_t {
+        ok = ptx::mbar_wait(&full[slot], par, 403);
+        ptx::tc_fence_after_sync();
+        return w_desc + static_cast<uint64_t>(slot * (kSlot >> 4));
+      };
+      auto slot_done = [&]() {
+        ptx::tc_commit_pair(&empty[slot]);
+        if (++slot == K::kSlots) { slot = 0; par ^= 1u; }
+      };
+      for (int i = 0; ok && i < total + kLag; ++i) {
+        if (i < total) {
+          if (c1 == 0 && !ptx::mbar_wait_cluster(&a_ready[t1 & 1], (t1 >> 1) & 1, 404)) break;
+          const uint64_t ad = a_desc + (t1 & 1) * (K::kABytes >> 4);
+          const uint32_t d = tmem_s + s1 * 128;
+#pragma unroll
+          for (int u = 0; u < K::kUnits; ++u) {
+            const uint64_t wd = slot_wait();
+            if (!ok) break;
+#pragma unroll
+            for (int k = 0; k < 8; ++k)
+              ptx::mma_f16_ss_pair(d, ad + (2 * u + k / 4) * (kBox >> 4) + (k & 3) * 2, wd + (k / 4) * (kSlot >> 5) + (k & 3) * 2, idesc_s,
+                                   (u > 0 || k > 0) ? 1u : 0u);
+            slot_done();
+          }
+          if (!ok) break;
+          ptx::tc_commit_pair(&s_full[s1]);
+          if (++s1 == K::kS) s1 = 0;
+          if (++c1 == p.chunks) {
+            ptx::tc_commit_pair(&a_done[t1 & 1]);
+            c1 = 0;
+            ++t1;
+          }
+        }
+        if (i >= kLag) {
+          if (c2 == 0 && !ptx::mbar_wait(o_empty, (t2 & 1) ^ 1, 405)) break;
+          if (!ptx::mbar_wait(&h_ready[s2], h_par, 406)) break;
+          const uint64_t wd = slot_wait();
+          if (!ok) break;
+#pragma unroll
+          for (int k = 0; k < kChunk / 16; ++k)
+            ptx::mma_f16_ts_pair(tmem_base, tmem_s + s2 * 128 + k * 8, wd + k * 2, idesc_o, (c2 > 0 || k > 0) ? 1u : 0u);
+          slot_done();
+          if (++s2 == K::kS) { s2 = 0; h_par ^= 1u; }
+          if (++c2 == p.chunks) {
+            ptx::tc_commit_pair(o_full);
+            c2 = 0;
+            ++t2;
+          }
+        }
+      }
+    }
+  } else if (warp >= kGluWarp) {
+    // ---------------------------------------------------------------- SwiGLU: chunks of one parity (a tile has an even number of them)
+    const int group = (warp - kGluWarp) >> 2, quad = warp & 3;
+    const uint32_t t_row = tmem_s + (static_cast<uint32_t>(quad * 32) << 16);
+    int s = group;
+    uint32_t par = 0;
+    for (int i = group; i < total; i += 2) {
+      const uint32_t t = t_row + s * 128;
+      if (!__all_sync(0xffffffffu, ptx::mbar_wait(&s_full[s], par, 407))) break;
+      ptx::tc_fence_after_sync();
+      // pieces of 16 channels; the next one's trip under the arithmetic of this one.  h (8 columns a piece) goes over values that have
+      // been read
+      uint32_t va[16], ga[16], vb[16], gb[16];
+      auto load = [&](int c, uint32_t (&v)[16], uint32_t (&g)[16]) {
+        ptx::tmem_ld_32x32b_x16(t + c, v);
+        ptx::tmem_ld_32x32b_x16(t + kChunk + c, g);
+      };
+      auto finish = [&](int c, const uint32_t (&v)[16], const uint32_t (&g)[16]) {
+        uint32_t w[8];
+#pragma unroll
+        for (int j = 0; j < 16; j += 2) {
+          const float a0 = __uint_as_float(v[j]), a1 = __uint_as_float(v[j + 1]);
+          w[j >> 1] = pack_bf16x2(glu_half(a0, a0) * __uint_as_float(g[j]), glu_half(a1, a1) * __uint_as_float(g[j + 1]));
+        }
+        ptx::tmem_st_32x32b_x8(t + c / 2, w);
+      };
+      load(0, va, ga);
+      ptx::tmem_ld_wait();
+      load(16, vb, gb);
+      finish(0, va, ga);
+      ptx::tmem_ld_wait();
+      load(32, va, ga);
+      finish(16, vb, gb);
+      ptx::tmem_ld_wait();
+      load(48, vb, gb);
+      finish(32, va, ga);
+      ptx::tmem_ld_wait();
+      finish(48, vb, gb);
+      ptx::tmem_st_wait();
+      ptx::tc_fence_before_sync();
+      __syncwarp();
+      if (lane == 0) ptx::mbar_arrive_cluster(ptx::leader_addr(&h_ready[s]));
+      s += 2;
+      if (s >= K::kS) { s -= K::kS; par ^= 1u; }
+    }
+  } else if (warp >= kRowWarp) {
+    // ---------------------------------------------------------------- rows: LayerNorm of the next tile, residual and output of the last
+    const int quad = warp & 3;
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
+    const bool issuer = quad == 0 && ptx::elect_one();
+    constexpr int kPer = C == 128 ? 8 : 4;       // channel pairs or channels of a lane, see below
+    grid_dependency_wait();
+    float lw[8], lb[8];
+#pragma unroll
+    for (int i = 0; i < 8; ++i) {
+      const int ch = C == 128 ? (lane & 15) * 8 + i : (lane + 32 * (i >> 1)) * 2 + (i & 1);
+      lw[i] = p.ln_w != nullptr ? p.ln_w[ch] : 1.0f;
+      lb[i] = p.ln_b != nullptr ? p.ln_b[ch] : 0.0f;
+    }
+    auto row0_of = [&](int it) { return (2 * (tile0 + it * tile_step) + rank) * kRows; };
+    auto fetch = [&](const CUtensorMap* map, int it) {      // a tile's rows into its buffer
+      uint8_t* dst = s_a + (it & 1) * K::kABytes;
+      ptx::mbar_expect_tx(&rows_in[it & 1], K::kABytes);
+#pragma unroll
+      for (int kb = 0; kb < C / 64; ++kb) ptx::tma_load_4d(dst + kb * kBox, map, &rows_in[it & 1], kb * 64, row0_of(it), 0, 0);
+    };
+    uint32_t in_par = 0;        // bit b: phase of rows_in[b]
+    bool ok = true;
+    auto wait_rows = [&](int b) -> bool {
+      const bool r = __all_sync(0xffffffffu, ptx::mbar_wait(&rows_in[b], (in_par >> b) & 1, 408)) != 0;
+      in_par ^= 1u << b;
+      return r;
+    };
+    if (issuer) {
+      fetch(&tm_x, 0);
+      if (my_tiles > 1) fetch(&tm_x, 1);
+    }
+    for (int it = 0; it <= my_tiles; ++it) {
+      if (it < my_tiles) {
+        // LayerNorm in place.  Lanes, expressions and their order: those of the LayerNorm kernels.
+        ok = wait_rows(it & 1);
+        if (!ok) break;
+        uint8_t* a = s_a + (it & 1) * K::kABytes;
+        if constexpr (C == 128) {
+          const int sub = lane & 15, half = lane >> 4;
+          constexpr int kSteps = 4;        // of two rows each in flight
+#pragma unroll 1
+          for (int base = quad * 32; base < quad * 32 + 32; base += 2 * kSteps) {
+            float v[kSteps][8], sum[kSteps], sq[kSteps];
+            uint4* cell[kSteps];
+#pragma unroll
+            for (int s = 0; s < kSteps; ++s) {
+              const int r = base + 2 * s + half;
+              cell[s] = reinterpret_cast<uint4*>(a + (sub >> 3) * kBox + r * 128 + (((sub & 7) ^ (r & 7)) << 4));
+              const uint4 raw = *cell[s];
+              const uint32_t wv[4] = {raw.x, raw.y, raw.z, raw.w};
+              sum[s] = 0.f;
+#pragma unroll
+              for (int i = 0; i < 4; ++i) {
+                v[s][2 * i] = __uint_as_float(wv[i] << 16);
+                v[s][2 * i + 1] = __uint_as_float(wv[i] & 0xffff0000u);
+                sum[s] += v[s][2 * i] + v[s][2 * i + 1];
+              }
+            }
+#pragma unroll
+            for (int m = 8; m > 0; m >>= 1)
+#pragma unroll
+              for (int s = 0; s < kSteps; ++s) sum[s] += __shfl_xor_sync(0xffffffffu, sum[s], m);
+#pragma unroll
+            for (int s = 0; s < kSteps; ++s) {
+              const float mean = sum[s] * (1.0f / C);
+              sq[s] = 0.f;
+#pragma unroll
+              for (int i = 0; i < 8; ++i) {
+                v[s][i] -= mean;
+                sq[s] = fmaf(v[s][i], v[s][i], sq[s]);
+              }
+            }
+#pragma unroll
+            for (int m = 8; m > 0; m >>= 1)
+#pragma unroll
+              for (int s = 0; s < kSteps; ++s) sq[s] += __shfl_xor_sync(0xffffffffu, sq[s], m);
+#pragma unroll
+            for (int s = 0; s < kSteps; ++s) {
+              const float rstd = rsqrtf(sq[s] * (1.0f / C) + p.eps);
+              uint32_t ov[4];
+#pragma unroll
+              for (int i = 0; i < 4; ++i)
+                ov[i] = pack_bf16x2(fmaf(v[s][2 * i] * rstd, lw[2 * i], lb[2 * i]), fmaf(v[s][2 * i + 1] * rstd, lw[2 * i + 1], lb[2 * i + 1]));
+              *cell[s] = make_uint4(ov[0], ov[1], ov[2], ov[3]);
+            }
+          }
+        } else {
+          constexpr int kStep = 4;         // rows in flight
+#pragma unroll 1
+          for (int base = quad * 32; base < quad * 32 + 32; base += kStep) {
+            float2 v[kStep][kPer];
+            float s[kStep], q[kStep];
+            uint32_t* cell[kStep];
+#pragma unroll
+            for (int r = 0; r < kStep; ++r) {
+              cell[r] = reinterpret_cast<uint32_t*>(a + (base + r) * 128 + (((lane >> 2) ^ ((base + r) & 7)) << 4) + (lane & 3) * 4);
+              s[r] = 0.f;
+#pragma unroll
+              for (int g = 0; g < kPer; ++g) {
+                const uint32_t u = cell[r][g * (kBox / 4)];
+                v[r][g] = make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
+                s[r] += v[r][g].x + v[r][g].y;
+              }
+            }
+#pragma unroll
+            for (int m = 16; m > 0; m >>= 1)
+#pragma unroll
+              for (int r = 0; r < kStep; ++r) s[r] += __shfl_xor_sync(0xffffffffu, s[r], m);
+#pragma unroll
+            for (int r = 0; r < kStep; ++r) {
+              const float mean = s[r] / static_cast<float>(C);
+              q[r] = 0.f;
+#pragma unroll
+              for (int g = 0; g < kPer; ++g) {
+                v[r][g].x -= mean;
+                v[r][g].y -= mean;
+                q[r] += v[r][g].x * v[r][g].x + v[r][g].y * v[r][g].y;
+              }
+            }
+#pragma unroll
+            for (int m = 16; m > 0; m >>= 1)
+#pragma unroll
+              for (int r = 0; r < kStep; ++r) q[r] += __shfl_xor_sync(0xffffffffu, q[r], m);
+#pragma unroll
+            for (int r = 0; r < kStep; ++r) {
+              const float rstd = rsqrtf(q[r] / static_cast<float>(C) + p.eps);
+#pragma unroll
+              for (int g = 0; g < kPer; ++g)
+                cell[r][g * (kBox / 4)] = pack_bf16x2(fmaf(v[r][g].x * rstd, lw[2 * g], lb[2 * g]), fmaf(v[r][g].y * rstd, lw[2 * g + 1], lb[2 * g + 1]));
+            }
+          }
+        }
+        ptx::fence_proxy_async_smem();
+        __syncwarp();
+        if (lane == 0) ptx::mbar_arrive_cluster_release(ptx::leader_addr(&a_ready[it & 1]));
+      }
+      if (it == 0) continue;
+      // output of the tile before: its buffer takes the residual once its last S has read the rows
+      const int done = it - 1, b = done & 1;
+      uint8_t* a = s_a + b * K::kABytes;
+      ok = __all_sync(0xffffffffu, ptx::mbar_wait(&a_done[b], (done >> 1) & 1, 409)) != 0;
+      if (!ok) break;
+      if (p.has_resid) {
+        if (issuer) fetch(&tm_r, done);
+        ok = wait_rows(b);
+        if (!ok) break;
+      }
+      ok = __all_sync(0xffffffffu, ptx::mbar_wait(o_full, done & 1, 410)) != 0;
+      if (!ok) break;
+      ptx::tc_fence_after_sync();
+      {
+        const int r = quad * 32 + lane;
+        uint32_t x[2][32];
+        ptx::tmem_ld_32x32b_x32(t_row, x[0]);
+#pragma unroll
+        for (int c = 0; c < C / 32; ++c) {
+          ptx::tmem_ld_wait();
+          if (c + 1 < C / 32) ptx::tmem_ld_32x32b_x32(t_row + 32 * (c + 1), x[(c + 1) & 1]);
+          uint8_t* row = a + (c >> 1) * kBox + r * 128;
+#pragma unroll
+          for (int i = 0; i < 4; ++i) {
+            uint4* cell = reinterpret_cast<uint4*>(row + ((((c & 1) * 4 + i) ^ (r & 7)) << 4));
+            const uint4 u = p.has_resid ? *cell : make_uint4(0, 0, 0, 0);
+            const uint32_t rw[4] = {u.x, u.y, u.z, u.w};
+            uint32_t w[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j)
+              w[j] = pack_bf16x2(__uint_as_float(x[c & 1][8 * i + 2 * j]) + __uint_as_float(rw[j] << 16),
+                                 __uint_as_float(x[c & 1][8 * i + 2 * j + 1]) + __uint_as_float(rw[j] & 0xffff0000u));
+            *cell = make_uint4(w[0], w[1], w[2], w[3]);
+          }
+        }
+      }
+      ptx::tc_fence_before_sync();
+      ptx::fence_proxy_async_smem();
+      __syncwarp();
+      if (lane == 0) {
+        ptx::mbar_arrive_cluster(ptx::leader_addr(o_empty));
+        ptx::mbar_arrive(out_done);
+      }
+      if (quad == 0) {
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(out_done, done & 1, 411)) != 0;
+        if (!ok) break;
+        if (issuer) {
+          if (row0_of(done) < p.rows) {
+#pragma unroll
+            for (int kb = 0; kb < C / 64; ++kb) ptx::tma_store_4d(&tm_out, a + kb * kBox, kb * 64, row0_of(done), 0, 0);
+            ptx::tma_store_commit();
+            ptx::tma_store_wait_read();
+          }
+          if (done + 2 < my_tiles) fetch(&tm_x, done + 2);
+        }
+        __syncwarp();
+      }
+    }
+    if (issuer) ptx::tma_store_wait_all();
+  }
+
+  ptx::tc_fence_before_sync();
+  __syncwarp();
+  ptx::cluster_sync();      // neither CTA leaves while the other may still read its operands or reach its barriers
+  if (warp == 1) {
+    ptx::tc_fence_after_sync();
+    ptx::tmem_dealloc_pair(tmem_base, 512);
+  }
+}
+
+// Pairs of CTAs that the current device holds at once (0: none), once per device.
+template <int C>
+int pairs_held(int* held) {
+  static std::once_flag once[64];
+  static int resident[64];
+  int dev = 0;
+  KFB_CUDA(cudaGetDevice(&dev));
+  cudaError_t err = cudaSuccess;
+  std::call_once(once[dev & 63], [&] {
+    err = cudaFuncSetAttribute(transition_pair_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<C>::kSmem);
+    if (err != cudaSuccess) return;
+    cudaLaunchAttribute attr[1];
+    attr[0].id = cudaLaunchAttributeClusterDimension;
+    attr[0].val.clusterDim.x = 2;
+    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = sm_count() / 2 * 2;
+    cfg.blockDim = kThreads;
+    cfg.dynamicSmemBytes = Cfg<C>::kSmem;
+    cfg.attrs = attr;
+    cfg.numAttrs = 1;
+    err = cudaOccupancyMaxActiveClusters(&resident[dev & 63], transition_pair_kernel<C>, &cfg);
+  });
+  KFB_CUDA(err);
+  *held = resident[dev & 63];
+  return KFB_OK;
+}
+
+template <int C>
+int launch(cudaStream_t stream, const void* x, const float* ln_w, const float* ln_b, const void* w_swiglu, const void* w_out, void* out,
+           const void* resid, long long rows, int hidden, float eps, int w_static) {
+  auto rows_map = [&](CUtensorMap* m, const void* ptr, long long n, int c, uint32_t box_rows) {
+    const uint64_t dims[4] = {(uint64_t)c, (uint64_t)n, 1, 1};
+    const uint64_t str[3] = {(uint64_t)c * 2, (uint64_t)c * 2 * n, (uint64_t)c * 2 * n};
+    const uint32_t box[4] = {64, box_rows, 1, 1};
+    return make_tmap(m, ptr, 2, 4, dims, str, box, 128);
+  };
+  CUtensorMap tx, t1, t2, tr, to;
+  KFB_TRY(rows_map(&tx, x, rows, C, kRows));
+  KFB_TRY(rows_map(&t1, w_swiglu, 2ll * hidden, C, kChunk));
+  KFB_TRY(rows_map(&t2, w_out, C, hidden, C / 2));
+  KFB_TRY(rows_map(&tr, resid != nullptr ? resid : x, rows, C, kRows));
+  KFB_TRY(rows_map(&to, out, rows, C, kRows));
+  int held = 0;
+  KFB_TRY(pairs_held<C>(&held));
+  PairTransParams p;
+  p.ln_w = ln_w;
+  p.ln_b = ln_b;
+  p.rows = static_cast<int>(rows);
+  p.tiles = static_cast<int>((rows + 2 * kRows - 1) / (2 * kRows));
+  p.chunks = hidden / kChunk;
+  p.has_resid = resid != nullptr;
+  p.w_static = w_static;
+  p.eps = eps;
+  LaunchScope scope(stream, "transition_pair");
+  return launch_kernel_clustered(stream, transition_pair_kernel<C>, 2, 2 * (p.tiles < held ? p.tiles : held), kThreads, Cfg<C>::kSmem, tx, t1, t2,
+                                 tr, to, p);
+}
+
+}  // namespace
+
+bool transition_pair_ok(const void* x, const void* w_swiglu, const void* w_out, const void* out, const void* resid, long long rows, int c,
+                        int hidden, int dtype) {
+  const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w_swiglu) | reinterpret_cast<uintptr_t>(w_out) |
+                        reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(resid);
+  if (dtype != KFB_BF16 || (c != 128 && c != 256) || hidden % 128 != 0 || (all & 15) != 0 || rows > (1ll << 30)) return false;
+  int held = 0;
+  const bool known = (c == 128 ? pairs_held<128>(&held) : pairs_held<256>(&held)) == KFB_OK;
+  if (!known) cudaGetLastError();
+  return known && held > 0;
+}
+
+int launch_transition_pair(cudaStream_t stream, const void* x, const float* ln_w, const float* ln_b, const void* w_swiglu, const void* w_out,
+                           void* out, const void* resid, long long rows, int c, int hidden, float eps, int w_static) {
+  return c == 128 ? launch<128>(stream, x, ln_w, ln_b, w_swiglu, w_out, out, resid, rows, hidden, eps, w_static)
+                  : launch<256>(stream, x, ln_w, ln_b, w_swiglu, w_out, out, resid, rows, hidden, eps, w_static);
+}
+
+}  // namespace kfb
