@@ -58,15 +58,13 @@ def algorithmic_work(n: int | None = None, c: int = C_Z, h: int = 4, cs: int = C
         "apb_out_proj": ("tensor", 2.0 * n * cs * cs),
         # HBM-bound kernels: bytes per launch (every tensor read or written once, bf16).  The K = c projections do
         # 8 tensor-core instructions per 128-row tile: their time is the traffic of the tensors around them.
-        # (8 launches per block share this tag: 6 over the pair tensor and 2 over the single track; the figures of the
-        # pair-sized ones are reported)
-        "layernorm_rows": ("hbm", 2.0 * p * c * 2),
+        # (the pair tensor is normalised inside the kernels that multiply its rows: this tag is the single track's)
+        "layernorm_rows": ("hbm", 2.0 * n * cs * 2),
         "layernorm_cm": ("hbm", 2.0 * p * c * 2),
         "layernorm_cm_stats": ("hbm", 1.0 * p * c * 2 + p * 8),   # read t, write (mean, rstd) per position
-        "trimul_in_proj": ("hbm", (4.0 if c <= 128 else 3.0) * p * c * 2),   # read x~, write a and b (c <= 128: and the gate logits)
-        "trimul_gate_proj": ("hbm", 2.0 * p * c * 2),          # read x~, write the gate logits (c > 128)
+        "trimul_project": ("hbm", 4.0 * p * c * 2),            # read x, write a, b and the gate logits
         "trimul_out_proj": ("hbm", 4.0 * p * c * 2),           # read LN(t), gate logits, residual; write out
-        "triatt_proj": ("hbm", 5.0 * p * c * 2 + p * h * 2),   # read x~; write q, k, g, v^T and the bias
+        "triatt_project": ("hbm", 5.0 * p * c * 2 + p * h * 2),   # read x; write q, k, g, v^T and the bias
         "triatt_out_proj": ("hbm", 3.0 * p * c * 2),           # read gated o, residual; write out
         "pair_bias_proj": ("hbm", p * c * 2 + p * hs * 2),
     }

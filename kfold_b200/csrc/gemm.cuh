@@ -1543,7 +1543,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
           uint64_t* bar_free = &cm_bar[grp * 2];
           uint64_t* bar_done = &cm_bar[grp * 2 + 1];
           const uint32_t par = staging_use & 1;
-          if (issuer) ptx::tma_store_wait_read_le1();  // the store that last read this slab (two uses ago) is done
+          if (issuer) ptx::tma_store_wait_read_le<1>();  // the store that last read this slab (two uses ago) is done
           ptx::mbar_arrive(bar_free);
           if (!ptx::mbar_wait(bar_free, par, 108)) { ok = false; break; }
           // packed conversions (two values per instruction), then the halves go to their channels' rows

@@ -100,8 +100,8 @@ __global__ void __launch_bounds__(256) layernorm_rows_kernel(const TI* x, TO* y,
   }
 }
 
-// Folded weights (see LnFold), kFoldRows rows per block of 256 threads: W' rounded to bf16, s1 of the rounded values.  The pair track's
-// LayerNorm kernels do it in blocks of their own before their rows: as a launch it was 3.3 us, whatever the size.
+// Folded weights (see LnFold), kFoldRows rows per block of 256 threads: W' rounded to bf16, s1 of the rounded values.  (A launch of 3.3 us,
+// whatever the size; pair_project_kernel does the same beside its projections.)
 constexpr int kFoldRows = 8;
 __device__ __forceinline__ void ln_fold_rows(const LnFold& f, int block) {
   constexpr int kPer = kFoldRows / 2;                       // rows of each half of the block
@@ -150,13 +150,9 @@ int launch_ln_fold_weights(cudaStream_t stream, const LnFold& f) {
 // rows per step and two steps per iteration: four rows (1 KB) in flight per warp, 16-byte loads and stores, the statistics
 // reduced over the 16 lanes of a row.  Same arithmetic as layernorm_rows_kernel (two passes, fp32).
 __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const float* w, const float* b,
-                                                                  long long rows, float eps, int fold_blocks, const LnFold fold) {
+                                                                  long long rows, float eps) {
   constexpr int LANES = 16, STEPS = 2, C = LANES * 8, kRows = 32 / LANES;
   grid_dependency_enter();
-  if (static_cast<int>(blockIdx.x) < fold_blocks) {
-    ln_fold_rows(fold, blockIdx.x);
-    return;
-  }
   const int lane = threadIdx.x & 31;
   const int sub = lane % LANES;              // 16-byte chunk of the row
   const int half = lane / LANES;             // which of the step's rows
@@ -166,8 +162,8 @@ __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfl
     g[i] = w != nullptr ? w[sub * 8 + i] : 1.0f;
     o[i] = b != nullptr ? b[sub * 8 + i] : 0.0f;
   }
-  const long long warps = static_cast<long long>(gridDim.x - fold_blocks) * (blockDim.x >> 5);
-  const long long warp_id = static_cast<long long>(blockIdx.x - fold_blocks) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  const long long warp_id = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   for (long long base = warp_id * (kRows * STEPS); base < rows; base += warps * (kRows * STEPS)) {
     uint4 raw[STEPS];
     bool live[STEPS];
@@ -220,13 +216,9 @@ __global__ void __launch_bounds__(256) layernorm_c128_bf16_kernel(const __nv_bfl
 // four blocks of bf16 rounding turn into 0.8 % of the result).
 constexpr int kC256Rows = 4;
 __global__ void __launch_bounds__(256) layernorm_c256_bf16_kernel(const __nv_bfloat16* x, __nv_bfloat16* y, const float* w, const float* b,
-                                                                  long long rows, float eps, int fold_blocks, const LnFold fold) {
+                                                                  long long rows, float eps) {
   constexpr int G = 4, C = 256;
   grid_dependency_enter();
-  if (static_cast<int>(blockIdx.x) < fold_blocks) {
-    ln_fold_rows(fold, blockIdx.x);
-    return;
-  }
   const int lane = threadIdx.x & 31;
   float2 ww[G], bb[G];
 #pragma unroll
@@ -234,8 +226,8 @@ __global__ void __launch_bounds__(256) layernorm_c256_bf16_kernel(const __nv_bfl
     ww[g] = w != nullptr ? *reinterpret_cast<const float2*>(w + (lane + 32 * g) * 2) : make_float2(1.f, 1.f);
     bb[g] = b != nullptr ? *reinterpret_cast<const float2*>(b + (lane + 32 * g) * 2) : make_float2(0.f, 0.f);
   }
-  const long long warps = static_cast<long long>(gridDim.x - fold_blocks) * (blockDim.x >> 5);
-  const long long warp_id = static_cast<long long>(blockIdx.x - fold_blocks) * (blockDim.x >> 5) + (threadIdx.x >> 5);
+  const long long warps = static_cast<long long>(gridDim.x) * (blockDim.x >> 5);
+  const long long warp_id = static_cast<long long>(blockIdx.x) * (blockDim.x >> 5) + (threadIdx.x >> 5);
   for (long long base = warp_id * kC256Rows; base < rows; base += warps * kC256Rows) {
     float2 v[kC256Rows][G];
 #pragma unroll
@@ -307,7 +299,7 @@ static int dispatch_g(cudaStream_t stream, const void* x, void* y, const float* 
 }
 
 int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w, const float* b, long long rows, int c,
-                     long long xs, long long ys, float eps, int in_dtype, int out_dtype, RowPerm perm, const LnFold* fold) {
+                     long long xs, long long ys, float eps, int in_dtype, int out_dtype, RowPerm perm) {
   KFB_CHECK_ARG(rows >= 0 && c > 0 && c % 2 == 0, "layernorm: rows %lld, channels %d (must be even)", rows, c);
   KFB_CHECK_ARG(perm.rows == 0 || (perm.n % perm.rows == 0 && rows == static_cast<long long>(perm.rows) * perm.n),
                 "layernorm: exchange order needs a (%d, %d) shard, got %lld rows", perm.rows, perm.n, rows);
@@ -318,15 +310,13 @@ int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w
     long long blocks = (rows + 31) / 32;      // 8 warps x 4 rows per iteration
     const long long cap = static_cast<long long>(sm_count()) * 16;
     if (blocks > cap) blocks = cap;
-    const int fold_blocks = fold != nullptr ? cdiv(fold->n, kFoldRows) : 0;
     LaunchScope scope(stream, "layernorm_rows");
     KFB_TRY(launch_kernel(stream, c == 128 ? layernorm_c128_bf16_kernel : layernorm_c256_bf16_kernel,
-                          static_cast<unsigned>(blocks + fold_blocks), 256, 0, static_cast<const __nv_bfloat16*>(x),
-                          static_cast<__nv_bfloat16*>(y), w, b, rows, eps, fold_blocks, fold != nullptr ? *fold : LnFold{}));
+                          static_cast<unsigned>(blocks), 256, 0, static_cast<const __nv_bfloat16*>(x),
+                          static_cast<__nv_bfloat16*>(y), w, b, rows, eps));
     KFB_CUDA(cudaGetLastError());
     return KFB_OK;
   }
-  if (fold != nullptr) KFB_TRY(launch_ln_fold_weights(stream, *fold));
   if (in_dtype == KFB_BF16 && out_dtype == KFB_BF16)
     return dispatch_g<__nv_bfloat16, __nv_bfloat16>(stream, x, y, w, b, rows, c, xs, ys, eps, perm);
   if (in_dtype == KFB_FP32 && out_dtype == KFB_BF16)

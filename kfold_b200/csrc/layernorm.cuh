@@ -22,11 +22,9 @@ struct LnFold {
 };
 int launch_ln_fold_weights(cudaStream_t stream, const LnFold& f);
 
-// Row-wise LayerNorm, one warp per row, fp32 statistics.  in/out dtype KFB_BF16 or KFB_FP32.  fold: weights to be folded along the
-// way, in the same launch where the kernel can.
+// Row-wise LayerNorm, one warp per row, fp32 statistics.  in/out dtype KFB_BF16 or KFB_FP32.
 int launch_layernorm(cudaStream_t stream, const void* x, void* y, const float* w, const float* b, long long rows, int c,
-                     long long xs, long long ys, float eps, int in_dtype, int out_dtype, RowPerm perm = RowPerm(),
-                     const LnFold* fold = nullptr);
+                     long long xs, long long ys, float eps, int in_dtype, int out_dtype, RowPerm perm = RowPerm());
 
 // LayerNorm of bf16 rows (128 or 256 channels, contiguous, 16-byte aligned) and projection to heads <= 16 values in one pass: the pair
 // bias.  w [heads][c] bf16; row (b, o, n) of batch x o_extent x n_extent, head h -> out + b s_b + o s_o + n s_n + h s_h (elements).

@@ -9,11 +9,13 @@
 //        triangle bias channel-major [h][j][k]               (channel-major segment)
 //   3. flash attention with the bias tile streamed through shared memory, output gated by sigmoid(g)
 //   4. output projection GEMM (+ optional residual)
+// bf16 tensors of 128 channels take steps 1 and 2 in one kernel (pair_project.cu).
 // The ending node is the starting node on the transposed pair tensor: step 2 walks xn with its two
 // position strides swapped (a tensor-map change, no data movement), the key mask is read transposed,
 // and step 4 scatters its rows back to the untransposed positions.
 #include "attention.cuh"
 #include "ops_common.cuh"
+#include "pair_project.cuh"
 
 using namespace kfb;
 
@@ -210,7 +212,7 @@ int triatt_mask_rows(cudaStream_t stream, const unsigned char* mask, int2* rows,
 
 int triatt_run(cudaStream_t stream, int ending, const void* x, const unsigned char* mask, const float* ln_w, const float* ln_b,
                const void* w_proj_packed, const void* w_out, void* out, const void* resid, void* workspace, size_t workspace_bytes, int batch,
-               int n, int c, int heads, float eps, int dtype, int2* mask_rows) {
+               int n, int c, int heads, float eps, int dtype, int2* mask_rows, int w_static) {
   KFB_CHECK_ARG(x && mask && w_proj_packed && w_out && out && workspace, "triatt: null pointer");
   KFB_CHECK_ARG(is_dtype(dtype), "triatt: bad dtype %d", dtype);
   KFB_CHECK_ARG(batch >= 1 && n >= 1, "triatt: batch %d N=%d", batch, n);
@@ -236,9 +238,14 @@ int triatt_run(cudaStream_t stream, int ending, const void* x, const unsigned ch
   const long long pos = nn * batch;
   const int np = pitch16(n);     // row pitch of V^T and the bias planes; everything else has the caller's n
 
-  KFB_TRY(launch_layernorm(stream, x, w.xn, ln_w, ln_b, pos, c, c, c, eps, dtype, KFB_BF16));
-  // projection: rows walked as (b, o, n); for the ending node (o, n) = (second, first) pair index
-  {
+  // rows walked as (b, o, n); for the ending node (o, n) = (second, first) pair index
+  const long long s_n = ending ? static_cast<long long>(n) * c : c, s_o = ending ? c : static_cast<long long>(n) * c;
+  const float bias_scale = rows_kernel ? 1.4426950408889634f : 1.0f;   // the kernel that scans the mask has its bias in log2 units, as q is
+  const PairRows r = {x, ln_w, ln_b, s_n, s_o, nn * c, batch, n, c, eps, w_static};
+  if (triatt_pair_project_ok(r, w_proj_packed, heads, hdp, w.qkg, w.vt, w.bias, dtype)) {
+    KFB_TRY(launch_triatt_pair_project(stream, r, w_proj_packed, heads, w.qkg, w.vt, w.bias, np, bias_scale));
+  } else {
+    KFB_TRY(launch_layernorm(stream, x, w.xn, ln_w, ln_b, pos, c, c, c, eps, dtype, KFB_BF16));
     GemmParams p = {};
     p.n_extent = n;
     p.o_extent = n;
@@ -261,14 +268,14 @@ int triatt_run(cudaStream_t stream, int ending, const void* x, const unsigned ch
     sb = {};
     sb.col_begin = 4 * hdp;
     sb.ncols = heads;
-    if (rows_kernel) sb.scale = 1.4426950408889634f;   // its bias is in log2 units, as q is
+    sb.scale = bias_scale;
     sb.dst = w.bias;
     sb.s_col = static_cast<long long>(np) * n;
     sb.s_n = 1;
     sb.n_pad = np;
     sb.s_o = np;
     sb.s_b = static_cast<long long>(heads) * np * n;
-    GemmOperandA a = {w.xn, ending ? static_cast<long long>(n) * c : c, ending ? c : static_cast<long long>(n) * c, nn * c};
+    GemmOperandA a = {w.xn, s_n, s_o, nn * c};
     GemmOperandB b = {w_proj_packed, c, 0};
     p.b_static = 1;
     KFB_TRY(launch_gemm_bf16(stream, a, b, p, 128, "triatt_proj"));
@@ -342,7 +349,7 @@ KFB_API int kfb_triatt_fwd(int ending, const void* x, const unsigned char* mask,
                            const void* w_proj_packed, const void* w_out, void* out, const void* resid, void* workspace,
                            size_t workspace_bytes, int batch, int n, int c, int heads, float eps, int dtype, void* stream) {
   return triatt_run(as_stream(stream), ending, x, mask, ln_w, ln_b, w_proj_packed, w_out, out, resid, workspace, workspace_bytes, batch, n, c,
-                    heads, eps, dtype, nullptr);
+                    heads, eps, dtype, nullptr, 0);
 }
 
 // ------------------------------------------------------------------------------------------------

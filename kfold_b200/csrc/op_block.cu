@@ -63,7 +63,7 @@ KFB_API int kfb_pair_block_fwd(const kfb_pair_block* blk, const void* z, void* z
   for (int dir = 0; dir < 2; ++dir) {
     const kfb_trimul_weights& w = dir ? k.mul_in : k.mul_out;
     KFB_TRY(trimul_run(as_stream(stream), dir, cur, pair_mask, w.ln_in_w, w.ln_in_b, w.w_in, w.w_gout, w.ln_out_w, w.ln_out_b, w.w_pout, z_out,
-                       cur, workspace, ob, batch, n, k.c, k.eps, z_dtype, fold_room));
+                       cur, workspace, ob, batch, n, k.c, k.eps, z_dtype, fold_room, dir));
     cur = z_out;
   }
   // the mask scans of both directions in one launch, after the operators' scratch
@@ -75,7 +75,7 @@ KFB_API int kfb_pair_block_fwd(const kfb_pair_block* blk, const void* z, void* z
   for (int dir = 0; k.has_attention && dir < 2; ++dir) {
     const kfb_triatt_weights& w = dir ? k.att_end : k.att_start;
     KFB_TRY(triatt_run(as_stream(stream), dir, cur, pair_mask, w.ln_w, w.ln_b, w.w_proj, w.w_out, z_out, cur, workspace, ob, batch, n, k.c,
-                       k.tri_heads, k.eps, z_dtype, scans != nullptr ? scans + static_cast<long long>(dir) * batch * n : nullptr));
+                       k.tri_heads, k.eps, z_dtype, scans != nullptr ? scans + static_cast<long long>(dir) * batch * n : nullptr, 1));
   }
   KFB_TRY(transition_run(as_stream(stream), cur, k.trans_z.ln_w, k.trans_z.ln_b, k.trans_z.w_swiglu, k.trans_z.w_out, z_out, cur, workspace, ob,
                          pos, k.c, k.hidden_z, k.eps, z_dtype, 1));

@@ -10,6 +10,7 @@
 //   4. triangle contraction              t[ch] = A_ch * B_ch^T, batch over channels   [tcgen05 batched GEMM]
 //   5. LayerNorm_out, channel-major in   t -> tn (bf16, position-major)             [HBM bound]
 //   6. output projection * sigmoid(gl)   out = (tn Wp_out^T) * sigmoid(gl) (+ resid) [tcgen05 GEMM, gated epilogue]
+// bf16 tensors of 128 and 256 channels take steps 1 to 3 in one kernel (pair_project.cu).
 //
 // The incoming direction needs t[i,j] = sum_k a[k,i] b[k,j].  Instead of a second, MN-major contraction
 // kernel, step 2 walks the pair tensor transposed (the TMA map of xn swaps its two position strides) so that
@@ -19,6 +20,7 @@
 // all-gathers the b operand (every rank needs all rows j of b), and "finish" takes the gathered operand in the
 // layout the collective leaves it in: rank after rank, each piece [channel][rows][n].
 #include "ops_common.cuh"
+#include "pair_project.cuh"
 
 using namespace kfb;
 
@@ -49,6 +51,18 @@ size_t trimul_fold_bytes(int c) { return align_up(static_cast<size_t>(c) * c * s
 
 namespace {
 
+// LayerNorm_out's folded weights at `room` (trimul_fold_bytes(c) bytes; null: nowhere).
+LnFold fold_into(void* room, const void* w_pout, const float* ln_out_w, const float* ln_out_b, int c) {
+  Carver cv(room);
+  __nv_bfloat16* wf = cv.take<__nv_bfloat16>(static_cast<size_t>(c) * c);
+  float* sums = cv.take<float>(2 * static_cast<size_t>(c));
+  return {static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, wf, sums, sums + c, c, c};
+}
+// Whether the scratch of posp normalised rows has room for them and the rows' statistics.
+bool folds(long long posp, int c) {
+  return c % kBK == 0 && posp * static_cast<long long>(c) * 2 >= static_cast<long long>(c) * c * 2 + 256 + 2ll * c * 4 + 256 + posp * 8;
+}
+
 int check_shape(const char* what, int batch, int rows, int n, int c) {
   KFB_CHECK_ARG(batch >= 1 && n >= 8 && n % 8 == 0, "%s: N=%d must be a positive multiple of 8 (pad in the caller)", what, n);
   KFB_CHECK_ARG(rows >= 1 && rows <= n, "%s: rows=%d out of range for N=%d", what, rows, n);
@@ -61,11 +75,10 @@ int check_shape(const char* what, int batch, int rows, int n, int c) {
 // parts > 1: only part `part` of the 2c operand channels (in packed order) is projected, into `ab` = that part's buffer.
 int project(cudaStream_t stream, int transposed_walk, const void* x, const unsigned char* mask, const float* ln_w,
             const float* ln_b, const void* w_in_packed, const void* w_gout, __nv_bfloat16* xn, __nv_bfloat16* ab,
-            __nv_bfloat16* gl, int batch, int rows, int n, int c, float eps, int dtype, int part = 0, int parts = 1,
-            const LnFold* fold = nullptr) {
+            __nv_bfloat16* gl, int batch, int rows, int n, int c, float eps, int dtype, int part = 0, int parts = 1) {
   const long long rn = static_cast<long long>(rows) * n;
   const long long pos = rn * batch;
-  if (x != nullptr) KFB_TRY(launch_layernorm(stream, x, xn, ln_w, ln_b, pos, c, c, c, eps, dtype, KFB_BF16, RowPerm(), fold));
+  if (x != nullptr) KFB_TRY(launch_layernorm(stream, x, xn, ln_w, ln_b, pos, c, c, c, eps, dtype, KFB_BF16));
   bool gate_done = false;
   if (w_in_packed != nullptr) {
     // ab[ch][b][o][n_]: o = row of the shard, n_ = position inside the row (swapped for the transposed walk)
@@ -131,11 +144,9 @@ int finish(cudaStream_t stream, const __nv_bfloat16* a, const __nv_bfloat16* b, 
   const long long rnp = static_cast<long long>(rows) * np, posp = rnp * batch;
   // LayerNorm_out folded into the output projection: the GEMM reads t as it lies (channel-major, read MN-major), the
   // epilogue applies the per-position statistics.  The scratch buffer tn holds the folded weights and the statistics.
-  const bool fold = (c % kBK == 0) && posp * static_cast<long long>(c) * 2 >= static_cast<long long>(c) * c * 2 + 256 + 2ll * c * 4 + 256 + posp * 8;
-  uint8_t* base = reinterpret_cast<uint8_t*>(tn);
-  float* s1 = reinterpret_cast<float*>(base + align_up(static_cast<size_t>(c) * c * 2, 256));
-  float2* stats = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(s1) + align_up(static_cast<size_t>(2) * c * 4, 256));
-  LnFold f = {static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, reinterpret_cast<__nv_bfloat16*>(base), s1, s1 + c, c, c};
+  const bool fold = folds(posp, c);
+  float2* stats = reinterpret_cast<float2*>(reinterpret_cast<uint8_t*>(tn) + trimul_fold_bytes(c));
+  LnFold f = fold_into(tn, w_pout, ln_out_w, ln_out_b, c);
   if (folded != nullptr)
     f = *folded;
   else if (fold)
@@ -330,7 +341,8 @@ int trimul_precise(cudaStream_t stream, int incoming, const void* x, const unsig
 namespace kfb {
 int trimul_run(cudaStream_t stream, int incoming, const void* x, const unsigned char* mask, const float* ln_in_w, const float* ln_in_b,
                const void* w_in_packed, const void* w_gout, const float* ln_out_w, const float* ln_out_b, const void* w_pout, void* out,
-               const void* resid, void* workspace, size_t workspace_bytes, int batch, int n, int c, float eps, int dtype, void* fold_room) {
+               const void* resid, void* workspace, size_t workspace_bytes, int batch, int n, int c, float eps, int dtype, void* fold_room,
+               int w_static) {
   KFB_CHECK_ARG(x && mask && w_in_packed && w_gout && w_pout && out && workspace, "trimul: null pointer");
   KFB_CHECK_ARG(is_dtype(dtype), "trimul: bad dtype %d", dtype);
   // any N on the bf16 path (except tensors too small for the folded LayerNorm's scratch), multiples of 8 otherwise
@@ -349,16 +361,18 @@ int trimul_run(cudaStream_t stream, int incoming, const void* x, const unsigned 
   const size_t need = carve(w, workspace, batch, n, c);
   KFB_CHECK_ARG(workspace_bytes >= need, "trimul: workspace %zu < %zu bytes", workspace_bytes, need);
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "trimul: workspace must be 256-byte aligned");
-  // The output projection's weights with its LayerNorm folded in: by the first launch where the caller has room for them, otherwise by a
-  // launch of their own into the normalised rows once those are used (3 us, whatever the size).
-  Carver room(fold_room);
-  __nv_bfloat16* wf = room.take<__nv_bfloat16>(static_cast<size_t>(c) * c);
-  float* sums = room.take<float>(2 * static_cast<size_t>(c));
-  const LnFold fold = {static_cast<const __nv_bfloat16*>(w_pout), ln_out_w, ln_out_b, wf, sums, sums + c, c, c};
-  const LnFold* early = fold_room != nullptr ? &fold : nullptr;
-  KFB_TRY(project(stream, incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, w.xn, w.ab, w.gl, batch, n, n, c, eps, dtype, 0, 1, early));
-  return finish(stream, w.ab, w.ab + static_cast<long long>(c) * batch * n * pitch8(n), n, 0, w.gl, ln_out_w, ln_out_b, w_pout, w.t, w.xn, out,
-                resid, batch, n, n, c, eps, dtype, early);
+  const long long nn = static_cast<long long>(n) * n, plane = nn / n * pitch8(n);
+  PairRows r = {x, ln_in_w, ln_in_b, incoming ? static_cast<long long>(n) * c : c, incoming ? c : static_cast<long long>(n) * c, nn * c, batch, n, c,
+                eps, w_static};
+  if (trimul_pair_project_ok(r, w_in_packed, w_gout, w.ab, w.gl, dtype) && folds(batch * plane, c)) {
+    // steps 1-3, and the folded weights of step 6, in one launch
+    const LnFold fold = fold_into(fold_room != nullptr ? fold_room : w.xn, w_pout, ln_out_w, ln_out_b, c);
+    KFB_TRY(launch_trimul_pair_project(stream, r, w_in_packed, w_gout, w.ab, pitch8(n), w.gl, mask, incoming ? n : 1, incoming ? 1 : n, nn, &fold));
+    return finish(stream, w.ab, w.ab + c * batch * plane, n, 0, w.gl, ln_out_w, ln_out_b, w_pout, w.t, w.xn, out, resid, batch, n, n, c, eps, dtype,
+                  &fold);
+  }
+  KFB_TRY(project(stream, incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, w.xn, w.ab, w.gl, batch, n, n, c, eps, dtype));
+  return finish(stream, w.ab, w.ab + c * batch * plane, n, 0, w.gl, ln_out_w, ln_out_b, w_pout, w.t, w.xn, out, resid, batch, n, n, c, eps, dtype);
 }
 }  // namespace kfb
 
@@ -379,7 +393,7 @@ KFB_API int kfb_trimul_fwd(int incoming, const void* x, const unsigned char* mas
                            const void* w_pout, void* out, const void* resid, void* workspace, size_t workspace_bytes,
                            int batch, int n, int c, float eps, int dtype, void* stream) {
   return trimul_run(as_stream(stream), incoming, x, mask, ln_in_w, ln_in_b, w_in_packed, w_gout, ln_out_w, ln_out_b, w_pout, out, resid,
-                    workspace, workspace_bytes, batch, n, c, eps, dtype, nullptr);
+                    workspace, workspace_bytes, batch, n, c, eps, dtype, nullptr, 0);
 }
 
 KFB_API int kfb_trimul_project(const void* x, const unsigned char* mask, const float* ln_in_w, const float* ln_in_b,

@@ -79,6 +79,18 @@ __device__ __forceinline__ bool mbar_try_wait(uint64_t* bar, uint32_t parity) {
       : "memory");
   return ok != 0;
 }
+// ... that sees what the other CTA of a pair released.
+__device__ __forceinline__ bool mbar_try_wait_cluster(uint64_t* bar, uint32_t parity) {
+  uint32_t ok;
+  asm volatile(
+      "{\n\t.reg .pred p;\n\t"
+      "mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], %2;\n\t"
+      "selp.u32 %0, 1, 0, p;\n\t}"
+      : "=r"(ok)
+      : "r"(smem_u32(bar)), "r"(parity)
+      : "memory");
+  return ok != 0;
+}
 // One look, no suspension.
 __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
   uint32_t ok;
@@ -95,20 +107,24 @@ __device__ __forceinline__ bool mbar_test(uint64_t* bar, uint32_t parity) {
 // flip within the time limit, or when another thread of the grid already failed.
 // The clock is first read after 256 looks: reading it at once would hold up a
 // waiter whose barrier flips a moment after the first look.
+__device__ __forceinline__ bool spin_on(uint32_t& spins, unsigned long long& t0, int code) {   // (one more look, or give up)
+  if ((++spins & 0xff) == 0) {
+    if (*reinterpret_cast<volatile int*>(&g_status) != 0) return false;
+    const unsigned long long now = globaltimer();
+    if (t0 == 0) t0 = now;
+    if (now - t0 > kWaitTimeoutNs) {
+      atomicCAS(&g_status, 0, code);
+      return false;
+    }
+  }
+  return true;
+}
+template <bool kCluster = false>
 __device__ __forceinline__ bool mbar_wait(uint64_t* bar, uint32_t parity, int code) {
   unsigned long long t0 = 0;
   uint32_t spins = 0;
-  while (!mbar_try_wait(bar, parity)) {
-    if ((++spins & 0xff) == 0) {
-      if (*reinterpret_cast<volatile int*>(&g_status) != 0) return false;
-      const unsigned long long now = globaltimer();
-      if (t0 == 0) t0 = now;
-      if (now - t0 > kWaitTimeoutNs) {
-        atomicCAS(&g_status, 0, code);
-        return false;
-      }
-    }
-  }
+  while (!(kCluster ? mbar_try_wait_cluster(bar, parity) : mbar_try_wait(bar, parity)))
+    if (!spin_on(spins, t0, code)) return false;
   return true;
 }
 
@@ -161,8 +177,9 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 __device__ __forceinline__ void tma_store_commit() { asm volatile("cp.async.bulk.commit_group;" ::: "memory"); }
 // Wait until the shared-memory source of every committed store has been read.
 __device__ __forceinline__ void tma_store_wait_read() { asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory"); }
-// ... of every committed store except the most recent one.
-__device__ __forceinline__ void tma_store_wait_read_le1() { asm volatile("cp.async.bulk.wait_group.read 1;" ::: "memory"); }
+// ... of every committed store except the most recent N.
+template <int N>
+__device__ __forceinline__ void tma_store_wait_read_le() { asm volatile("cp.async.bulk.wait_group.read %0;" ::"n"(N) : "memory"); }
 __device__ __forceinline__ void tma_store_wait_all() { asm volatile("cp.async.bulk.wait_group 0;" ::: "memory"); }
 
 // ---------------------------------------------------------------- tcgen05 / TMEM
@@ -274,6 +291,24 @@ __device__ __forceinline__ void tmem_ld_32x32b_x16(uint32_t taddr, uint32_t (&r)
       : "memory");
 }
 
+// 16 lanes x 16 consecutive columns as fragments of 8 x 8 blocks: of columns 8 i .. 8 i + 7, thread t holds columns 2 (t % 4) and the one
+// after of lane t / 4 (r[4 i], r[4 i + 1]) and of lane t / 4 + 8 (r[4 i + 2], r[4 i + 3]).
+__device__ __forceinline__ void tmem_ld_16x256b_x2(uint32_t taddr, uint32_t (&r)[8]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x2.b32 {%0, %1, %2, %3, %4, %5, %6, %7}, [%8];"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7])
+               : "r"(taddr)
+               : "memory");
+}
+__device__ __forceinline__ void tmem_ld_16x256b_x1(uint32_t taddr, uint32_t (&r)[4]) {
+  asm volatile("tcgen05.ld.sync.aligned.16x256b.x1.b32 {%0, %1, %2, %3}, [%4];" : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"(taddr) : "memory");
+}
+// Four such 8 x 8 blocks of 16-bit values (two columns of a lane in a register) into shared memory transposed: thread t gives the address
+// of the 16 bytes that receive column t % 8 of block t / 8.
+__device__ __forceinline__ void stmatrix_x4_trans(uint32_t smem_addr, uint32_t r0, uint32_t r1, uint32_t r2, uint32_t r3) {
+  asm volatile("stmatrix.sync.aligned.m8n8.x4.trans.shared.b16 [%0], {%1, %2, %3, %4};" ::"r"(smem_addr), "r"(r0), "r"(r1), "r"(r2), "r"(r3)
+               : "memory");
+}
+
 // 32 lanes x 8 consecutive 32-bit columns from registers into tensor memory.
 __device__ __forceinline__ void tmem_st_32x32b_x8(uint32_t taddr, const uint32_t (&r)[8]) {
   asm volatile("tcgen05.st.sync.aligned.32x32b.x8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"r"(taddr), "r"(r[0]),
@@ -347,10 +382,10 @@ __device__ __forceinline__ void mma_f16_ts_pair(uint32_t d_tmem, uint32_t a_tmem
 __device__ __forceinline__ void mbar_arrive_cluster_release(uint32_t cluster_addr) {
   asm volatile("mbarrier.arrive.release.cluster.shared::cluster.b64 _, [%0];" ::"r"(cluster_addr) : "memory");
 }
+// (The acquire belongs to the looks themselves: a fence.acq_rel.cluster behind them held the MMA thread up for 2 600 to 5 300 cycles a tile
+// of the pair kernels, clock stamps.)
 __device__ __forceinline__ bool mbar_wait_cluster(uint64_t* bar, uint32_t parity, int code) {
-  if (!mbar_wait(bar, parity, code)) return false;
-  asm volatile("fence.acq_rel.cluster;" ::: "memory");
-  return true;
+  return mbar_wait<true>(bar, parity, code);
 }
 // Arrive on the barrier at this offset in both CTAs once every product issued so far has completed.
 __device__ __forceinline__ void tc_commit_pair(uint64_t* bar) {

@@ -19,21 +19,22 @@
 //     finished tile around: the residual comes back (from L2) into the tile's own buffer, which the products have left, is added, and the
 //     buffer leaves as it is.
 // The arithmetic and its order are those of layernorm_c128_bf16_kernel / layernorm_c256_bf16_kernel and of the GEMMs this replaces: the
-// same bits (four blocks of bf16 rounding turn a last bit into up to 1 % of the confidence head's result).
+// same bits.
 #include <cuda_bf16.h>
 
 #include <mutex>
 
 #include "gemm.cuh"   // glu_half, pack_bf16x2
+#include "pair_rows.cuh"
 #include "ptx.cuh"
 #include "transition_pair.cuh"
 
 namespace kfb {
 namespace {
 
-constexpr int kRows = 128;                 // rows of a CTA
+constexpr int kRows = kRowTile;            // rows of a CTA
 constexpr int kChunk = 64;                 // hidden channels of a chunk
-constexpr int kBox = kRows * 128;          // [128 rows][64 bf16], 128-byte swizzle
+constexpr int kBox = kRowBox;              // [128 rows][64 bf16], 128-byte swizzle
 constexpr int kSlot = 16384;               // unit of the weight ring: 128 columns of K of S's 64 weight rows, or a chunk's K of O's C / 2
 constexpr int kThreads = 512;              // producer, MMA, 2 idle (a warp reads the tensor-memory lanes warp % 4), 4 rows, 2 x 4 SwiGLU
 constexpr int kRowWarp = 4, kGluWarp = 8;
@@ -268,15 +269,9 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     const int quad = warp & 3;
     const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
     const bool issuer = quad == 0 && ptx::elect_one();
-    constexpr int kPer = C == 128 ? 8 : 4;       // channel pairs or channels of a lane, see below
     grid_dependency_wait();
     float lw[8], lb[8];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {
-      const int ch = C == 128 ? (lane & 15) * 8 + i : (lane + 32 * (i >> 1)) * 2 + (i & 1);
-      lw[i] = p.ln_w != nullptr ? p.ln_w[ch] : 1.0f;
-      lb[i] = p.ln_b != nullptr ? p.ln_b[ch] : 0.0f;
-    }
+    rows_affine<C>(p.ln_w, p.ln_b, lane, lw, lb);
     auto row0_of = [&](int it) { return (2 * (tile0 + it * tile_step) + rank) * kRows; };
     auto fetch = [&](const CUtensorMap* map, int it) {      // a tile's rows into its buffer
       uint8_t* dst = s_a + (it & 1) * K::kABytes;
@@ -297,105 +292,10 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     }
     for (int it = 0; it <= my_tiles; ++it) {
       if (it < my_tiles) {
-        // LayerNorm in place.  Lanes, expressions and their order: those of the LayerNorm kernels.
         ok = wait_rows(it & 1);
         if (!ok) break;
         uint8_t* a = s_a + (it & 1) * K::kABytes;
-        if constexpr (C == 128) {
-          const int sub = lane & 15, half = lane >> 4;
-          constexpr int kSteps = 4;        // of two rows each in flight
-#pragma unroll 1
-          for (int base = quad * 32; base < quad * 32 + 32; base += 2 * kSteps) {
-            float v[kSteps][8], sum[kSteps], sq[kSteps];
-            uint4* cell[kSteps];
-#pragma unroll
-            for (int s = 0; s < kSteps; ++s) {
-              const int r = base + 2 * s + half;
-              cell[s] = reinterpret_cast<uint4*>(a + (sub >> 3) * kBox + r * 128 + (((sub & 7) ^ (r & 7)) << 4));
-              const uint4 raw = *cell[s];
-              const uint32_t wv[4] = {raw.x, raw.y, raw.z, raw.w};
-              sum[s] = 0.f;
-#pragma unroll
-              for (int i = 0; i < 4; ++i) {
-                v[s][2 * i] = __uint_as_float(wv[i] << 16);
-                v[s][2 * i + 1] = __uint_as_float(wv[i] & 0xffff0000u);
-                sum[s] += v[s][2 * i] + v[s][2 * i + 1];
-              }
-            }
-#pragma unroll
-            for (int m = 8; m > 0; m >>= 1)
-#pragma unroll
-              for (int s = 0; s < kSteps; ++s) sum[s] += __shfl_xor_sync(0xffffffffu, sum[s], m);
-#pragma unroll
-            for (int s = 0; s < kSteps; ++s) {
-              const float mean = sum[s] * (1.0f / C);
-              sq[s] = 0.f;
-#pragma unroll
-              for (int i = 0; i < 8; ++i) {
-                v[s][i] -= mean;
-                sq[s] = fmaf(v[s][i], v[s][i], sq[s]);
-              }
-            }
-#pragma unroll
-            for (int m = 8; m > 0; m >>= 1)
-#pragma unroll
-              for (int s = 0; s < kSteps; ++s) sq[s] += __shfl_xor_sync(0xffffffffu, sq[s], m);
-#pragma unroll
-            for (int s = 0; s < kSteps; ++s) {
-              const float rstd = rsqrtf(sq[s] * (1.0f / C) + p.eps);
-              uint32_t ov[4];
-#pragma unroll
-              for (int i = 0; i < 4; ++i)
-                ov[i] = pack_bf16x2(fmaf(v[s][2 * i] * rstd, lw[2 * i], lb[2 * i]), fmaf(v[s][2 * i + 1] * rstd, lw[2 * i + 1], lb[2 * i + 1]));
-              *cell[s] = make_uint4(ov[0], ov[1], ov[2], ov[3]);
-            }
-          }
-        } else {
-          constexpr int kStep = 4;         // rows in flight
-#pragma unroll 1
-          for (int base = quad * 32; base < quad * 32 + 32; base += kStep) {
-            float2 v[kStep][kPer];
-            float s[kStep], q[kStep];
-            uint32_t* cell[kStep];
-#pragma unroll
-            for (int r = 0; r < kStep; ++r) {
-              cell[r] = reinterpret_cast<uint32_t*>(a + (base + r) * 128 + (((lane >> 2) ^ ((base + r) & 7)) << 4) + (lane & 3) * 4);
-              s[r] = 0.f;
-#pragma unroll
-              for (int g = 0; g < kPer; ++g) {
-                const uint32_t u = cell[r][g * (kBox / 4)];
-                v[r][g] = make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
-                s[r] += v[r][g].x + v[r][g].y;
-              }
-            }
-#pragma unroll
-            for (int m = 16; m > 0; m >>= 1)
-#pragma unroll
-              for (int r = 0; r < kStep; ++r) s[r] += __shfl_xor_sync(0xffffffffu, s[r], m);
-#pragma unroll
-            for (int r = 0; r < kStep; ++r) {
-              const float mean = s[r] / static_cast<float>(C);
-              q[r] = 0.f;
-#pragma unroll
-              for (int g = 0; g < kPer; ++g) {
-                v[r][g].x -= mean;
-                v[r][g].y -= mean;
-                q[r] += v[r][g].x * v[r][g].x + v[r][g].y * v[r][g].y;
-              }
-            }
-#pragma unroll
-            for (int m = 16; m > 0; m >>= 1)
-#pragma unroll
-              for (int r = 0; r < kStep; ++r) q[r] += __shfl_xor_sync(0xffffffffu, q[r], m);
-#pragma unroll
-            for (int r = 0; r < kStep; ++r) {
-              const float rstd = rsqrtf(q[r] / static_cast<float>(C) + p.eps);
-#pragma unroll
-              for (int g = 0; g < kPer; ++g)
-                cell[r][g * (kBox / 4)] = pack_bf16x2(fmaf(v[r][g].x * rstd, lw[2 * g], lb[2 * g]), fmaf(v[r][g].y * rstd, lw[2 * g + 1], lb[2 * g + 1]));
-            }
-          }
-        }
+        rows_layernorm<C>(a, quad * 32, 32, lane, lw, lb, p.eps);
         ptx::fence_proxy_async_smem();
         __syncwarp();
         if (lane == 0) ptx::mbar_arrive_cluster_release(ptx::leader_addr(&a_ready[it & 1]));
