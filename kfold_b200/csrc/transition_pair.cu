@@ -12,14 +12,20 @@
 // With single CTAs each would load all of the weights: operand traffic, 128 bytes a cycle through a shared memory, is what the products
 // compete with (a chunk of 128 channels reads 56 KB of operands and is filled with 24 KB in 768 cycles of products; h in shared memory
 // would add 32).
-//   * S has three buffers of 128 columns (C = 128) or two (C = 256), which with O fill the tensor memory.  The tensor core runs ahead by
-//     all of them and executes in order, so a buffer needs no barrier of its own: its next S is issued behind the product that read its h.
-//   * Two groups of four SwiGLU warps take the chunks in turn.
-//   * Four more warps normalise the next tile's rows in place in shared memory (two buffers) while this one is multiplied, and turn the
-//     finished tile around: the residual comes back (from L2) into the tile's own buffer, which the products have left, is added, and the
-//     buffer leaves as it is.
+//   * S has three buffers of 128 columns (C = 128) or two (C = 256), which with O fill the tensor memory.  S and O have a thread each that
+//     issues them.  The tensor core works in the order of issue: a buffer's next S needs no more than that the product with its h has been
+//     issued, not that it is done (which took the chain another 500 cycles a turn).
+//   * Two groups of four SwiGLU warps take the chunks in turn.  (All eight on one chunk: the special-function unit, 512 cycles a chunk, then
+//     waits out every chunk's latencies: 191 -> 197 us.)
+//   * Eight more warps normalise the next tile's rows in place in shared memory while this one is multiplied, and turn the finished tile
+//     around: the residual comes back (from L2) into the tile's own buffer, which the products have left, is added, and the buffer leaves
+//     as it is.  A thread of its own sees to what a buffer receives and sends.
 // The arithmetic and its order are those of layernorm_c128_bf16_kernel / layernorm_c256_bf16_kernel and of the GEMMs this replaces: the
 // same bits.
+//
+// Measured (events): 589 824 rows of 128 channels 376 us as three launches, 255 with one issuing thread and four row warps, 187 now (62 %
+// more than the products alone: the chain S - h - O through three S buffers); of 256 channels 955, 637, 633 (1 466 TFLOP/s, at the power
+// limit); 63 001 rows: 53, 42, 34 and 112, 89, 86.
 #include <cuda_bf16.h>
 
 #include <mutex>
@@ -35,18 +41,19 @@ namespace {
 constexpr int kRows = kRowTile;            // rows of a CTA
 constexpr int kChunk = 64;                 // hidden channels of a chunk
 constexpr int kBox = kRowBox;              // [128 rows][64 bf16], 128-byte swizzle
-constexpr int kSlot = 16384;               // unit of the weight ring: 128 columns of K of S's 64 weight rows, or a chunk's K of O's C / 2
-constexpr int kThreads = 512;              // producer, MMA, 2 idle (a warp reads the tensor-memory lanes warp % 4), 4 rows, 2 x 4 SwiGLU
-constexpr int kRowWarp = 4, kGluWarp = 8;
+constexpr int kSlot = 16384;               // unit of the ring of S's weights: 128 columns of K of a CTA's 64 rows
+constexpr int kRowWarp = 4, kRowWarps = 8, kGluWarp = kRowWarp + kRowWarps;
+constexpr int kThreads = 32 * (kGluWarp + 8);   // weights, S, rows in and out, O, 8 rows, 2 x 4 SwiGLU (a warp reads the tensor-memory lanes warp % 4)
 
 template <int C>
 struct Cfg {
   static constexpr int kABytes = (C / 64) * kBox;
-  static constexpr int kSlots = C == 128 ? 8 : 6;
+  static constexpr int kA = C == 128 ? 3 : 2;         // tiles of rows: multiplied and finished, normalised, on their way
+  static constexpr int kSlots = C == 128 ? 6 : 4;
   static constexpr int kS = C == 128 ? 3 : 2;         // S buffers
   static constexpr int kUnits = C / 128;              // ring units of a chunk's S
-  static constexpr int kOutUnit = (C / 2) * 128;      // bytes of a chunk's unit of W_out in a CTA
-  static constexpr int kSmem = 2 * kABytes + kSlots * kSlot + 512 + 1024;
+  static constexpr int kOutUnit = (C / 2) * 128;      // bytes of a chunk's W_out in a CTA; as many of them as S buffers
+  static constexpr int kSmem = kA * kABytes + kSlots * kSlot + kS * kOutUnit + 512 + 1024;
   static_assert(kSmem <= 232448, "shared memory");
 };
 
@@ -63,21 +70,27 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   using K = Cfg<C>;
   constexpr int kLag = K::kS - 1;
   extern __shared__ uint8_t smem_raw[];
-  uint8_t* s_a = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));   // [2][C / 64] boxes
-  uint8_t* s_w = s_a + 2 * K::kABytes;
-  uint64_t* bars = reinterpret_cast<uint64_t*>(s_w + K::kSlots * kSlot);
+  uint8_t* s_a = reinterpret_cast<uint8_t*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) & ~uintptr_t(1023));   // [kA][C / 64] boxes
+  uint8_t* s_w = s_a + K::kA * K::kABytes;
+  uint8_t* s_v = s_w + K::kSlots * kSlot;    // [kS] W_out
+  uint64_t* bars = reinterpret_cast<uint64_t*>(s_v + K::kS * K::kOutUnit);
   uint64_t* full = bars;                     // [slots], in the leader: both CTAs' copies
   uint64_t* empty = full + K::kSlots;        // [slots]
-  uint64_t* s_full = empty + K::kSlots;      // [kS]
+  uint64_t* v_full = empty + K::kSlots;      // [kS], in the leader
+  uint64_t* v_free = v_full + K::kS;         // [kS] the product has read it
+  uint64_t* o_sent = v_free + K::kS;         // [kS], in the leader: the product with the h of S buffer i % kS has been issued
+  uint64_t* s_full = o_sent + K::kS;         // [kS]
   uint64_t* h_ready = s_full + K::kS;        // [kS], in the leader: 4 warps of each CTA
-  uint64_t* rows_in = h_ready + K::kS;       // [2] a tile's rows, or its residual, have arrived
-  uint64_t* a_ready = rows_in + 2;           // [2], in the leader: normalised rows
-  uint64_t* a_done = a_ready + 2;            // [2] every S of the tile
-  uint64_t* o_full = a_done + 2;
-  uint64_t* o_empty = o_full + 1;            // in the leader
-  uint64_t* out_done = o_empty + 1;          // the row warps have written the output tile
-  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(out_done + 1);
-  static_assert((2 * 8 + 2 * 3 + 9) * 8 + 4 <= 512, "barriers");
+  uint64_t* rows_in = h_ready + K::kS;       // [kA] a tile's rows have arrived
+  uint64_t* resid_in = rows_in + K::kA;      // [kA] a tile's residual has, in their place
+  uint64_t* a_norm = resid_in + K::kA;       // [kA] this CTA's rows are normalised: the row warps
+  uint64_t* a_peer = a_norm + K::kA;         // [kA], in the leader: and the other CTA's
+  uint64_t* a_done = a_peer + K::kA;         // [kA] every S of the tile
+  uint64_t* out_done = a_done + K::kA;       // [kA] the row warps have written the output tile
+  uint64_t* o_full = out_done + K::kA;
+  uint64_t* o_empty = o_full + 1;            // in the leader: the row warps of both CTAs
+  uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_empty + 1);
+  static_assert((2 * 6 + 5 * 3 + 6 * 3 + 2) * 8 + 4 <= 512, "barriers");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(ptx::cluster_ctarank());
@@ -95,17 +108,22 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
       ptx::mbar_init(&empty[i], 1);
     }
     for (int i = 0; i < K::kS; ++i) {
+      ptx::mbar_init(&v_full[i], 1);
+      ptx::mbar_init(&v_free[i], 1);
+      ptx::mbar_init(&o_sent[i], 1);
       ptx::mbar_init(&s_full[i], 1);
       ptx::mbar_init(&h_ready[i], 8);
     }
-    for (int i = 0; i < 2; ++i) {
+    for (int i = 0; i < K::kA; ++i) {
       ptx::mbar_init(&rows_in[i], 1);
-      ptx::mbar_init(&a_ready[i], 8);
+      ptx::mbar_init(&resid_in[i], 1);
+      ptx::mbar_init(&a_norm[i], kRowWarps);
+      ptx::mbar_init(&a_peer[i], 1);
       ptx::mbar_init(&a_done[i], 1);
+      ptx::mbar_init(&out_done[i], kRowWarps);
     }
     ptx::mbar_init(o_full, 1);
-    ptx::mbar_init(o_empty, 8);
-    ptx::mbar_init(out_done, 4);
+    ptx::mbar_init(o_empty, 2 * kRowWarps);
     ptx::fence_barrier_init();
   }
   if (warp == 1) {
@@ -125,17 +143,9 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     if (ptx::elect_one()) {
       if (!p.w_static) grid_dependency_wait();
       const int last = max((my_tiles - 1) * p.chunks, 2);      // the last tile, and a few chunks on their way
-      int slot = 0;
-      uint32_t par = 0;
+      int slot = 0, v = 0;
+      uint32_t par = 0, v_par = 0;
       bool ok = true;
-      auto unit = [&](const CUtensorMap* map, int bytes, int boxes, int col, int row) {
-        ok = ptx::mbar_wait(&empty[slot], par ^ 1, 401);
-        if (!ok) return;
-        if (rank == 0) ptx::mbar_expect_tx(&full[slot], 2 * bytes);
-        const uint32_t bar = ptx::leader_addr(&full[slot]);
-        for (int i = 0; i < boxes; ++i) ptx::tma_load_4d_pair(s_w + slot * kSlot + i * (bytes / boxes), map, bar, col + 64 * i, row, 0, 0);
-        if (++slot == K::kSlots) { slot = 0; par ^= 1u; }
-      };
       int c1 = 0, c2 = 0;                     // chunk of the next S and of the next product with h
       for (int i = 0; ok && i < total + kLag; ++i) {
         if (i == last) {
@@ -144,11 +154,23 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
         }
         if (i < total) {
           const int row = (c1 >> 1) * 256 + 128 * rank + (c1 & 1) * kChunk;
-          for (int u = 0; ok && u < K::kUnits; ++u) unit(&tm_w1, kSlot, 2, u * 128, row);
+          for (int u = 0; u < K::kUnits; ++u) {
+            ok = ptx::mbar_wait(&empty[slot], par ^ 1, 401);
+            if (!ok) break;
+            if (rank == 0) ptx::mbar_expect_tx(&full[slot], 2 * kSlot);
+            const uint32_t bar = ptx::leader_addr(&full[slot]);
+#pragma unroll
+            for (int k = 0; k < 2; ++k) ptx::tma_load_4d_pair(s_w + slot * kSlot + k * (kSlot / 2), &tm_w1, bar, u * 128 + 64 * k, row, 0, 0);
+            if (++slot == K::kSlots) { slot = 0; par ^= 1u; }
+          }
           if (++c1 == p.chunks) c1 = 0;
         }
         if (ok && i >= kLag) {
-          unit(&tm_w2, K::kOutUnit, 1, c2 * kChunk, rank * (C / 2));
+          ok = ptx::mbar_wait(&v_free[v], v_par ^ 1, 415);
+          if (!ok) break;
+          if (rank == 0) ptx::mbar_expect_tx(&v_full[v], 2 * K::kOutUnit);
+          ptx::tma_load_4d_pair(s_v + v * K::kOutUnit, &tm_w2, ptx::leader_addr(&v_full[v]), c2 * kChunk, rank * (C / 2), 0, 0);
+          if (++v == K::kS) { v = 0; v_par ^= 1u; }
           if (++c2 == p.chunks) c2 = 0;
         }
       }
@@ -157,66 +179,86 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
         ok = ptx::mbar_wait(&empty[slot], par ^ 1, 402);
         if (++slot == K::kSlots) { slot = 0; par ^= 1u; }
       }
+      for (int i = 0; ok && i < K::kS; ++i) {
+        ok = ptx::mbar_wait(&v_free[v], v_par ^ 1, 416);
+        if (++v == K::kS) { v = 0; v_par ^= 1u; }
+      }
     }
   } else if (warp == 1) {
-    // ---------------------------------------------------------------- MMA issue
-    if (rank == 0 && ptx::elect_one()) {
-      constexpr uint32_t idesc_s = ptx::make_idesc(2 * kRows, 2 * kChunk, 1);
-      constexpr uint32_t idesc_o = ptx::make_idesc(2 * kRows, C, 1);
+    if (rank == 1) {
+      // -------------------------------------------------------------- word to the leader that this CTA's rows are normalised (a thread of its
+      // own: the release to the other CTA costs the thread that gives it some 1 500 cycles)
+      if (ptx::elect_one()) {
+        int ab = 0;
+        uint32_t a_par = 0;
+        for (int it = 0; it < my_tiles; ++it) {
+          if (!ptx::mbar_wait(&a_norm[ab], a_par, 412)) break;
+          ptx::mbar_arrive_cluster_release(ptx::leader_addr(&a_peer[ab]));
+          if (++ab == K::kA) { ab = 0; a_par ^= 1u; }
+        }
+      }
+      // -------------------------------------------------------------- S
+    } else if (ptx::elect_one()) {
+      constexpr uint32_t idesc = ptx::make_idesc(2 * kRows, 2 * kChunk, 1);
       const uint64_t a_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_a));
       const uint64_t w_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_w));
-      int slot = 0, c1 = 0, c2 = 0, s1 = 0, s2 = 0;
-      uint32_t par = 0, t1 = 0, t2 = 0, h_par = 0;    // t1, t2: tiles begun by S and by O
+      int slot = 0, s1 = 0, ab = 0;
+      uint32_t par = 0, s_par = 1, a_par = 0;      // s_par: phase of o_sent that the buffer's next S stands behind (the first kS: none)
       bool ok = true;
-      auto slot_wait = [&]() -> uint64_t {
-        ok = ptx::mbar_wait(&full[slot], par, 403);
-        ptx::tc_fence_after_sync();
-        return w_desc + static_cast<uint64_t>(slot * (kSlot >> 4));
-      };
-      auto slot_done = [&]() {
-        ptx::tc_commit_pair(&empty[slot]);
-        if (++slot == K::kSlots) { slot = 0; par ^= 1u; }
-      };
-      for (int i = 0; ok && i < total + kLag; ++i) {
-        if (i < total) {
-          if (c1 == 0 && !ptx::mbar_wait_cluster(&a_ready[t1 & 1], (t1 >> 1) & 1, 404)) break;
-          const uint64_t ad = a_desc + (t1 & 1) * (K::kABytes >> 4);
+      for (int it = 0; ok && it < my_tiles; ++it) {
+        ok = ptx::mbar_wait(&a_norm[ab], a_par, 404) && ptx::mbar_wait_cluster(&a_peer[ab], a_par, 413);
+        const uint64_t ad = a_desc + ab * (K::kABytes >> 4);
+        for (int c = 0; ok && c < p.chunks; ++c) {
+          ok = ptx::mbar_wait(&o_sent[s1], s_par, 417);
+          if (!ok) break;
+          ptx::tc_fence_after_sync();
           const uint32_t d = tmem_s + s1 * 128;
 #pragma unroll
           for (int u = 0; u < K::kUnits; ++u) {
-            const uint64_t wd = slot_wait();
+            ok = ptx::mbar_wait(&full[slot], par, 403);
             if (!ok) break;
+            ptx::tc_fence_after_sync();
+            const uint64_t wd = w_desc + static_cast<uint64_t>(slot * (kSlot >> 4));
 #pragma unroll
             for (int k = 0; k < 8; ++k)
-              ptx::mma_f16_ss_pair(d, ad + (2 * u + k / 4) * (kBox >> 4) + (k & 3) * 2, wd + (k / 4) * (kSlot >> 5) + (k & 3) * 2, idesc_s,
+              ptx::mma_f16_ss_pair(d, ad + (2 * u + k / 4) * (kBox >> 4) + (k & 3) * 2, wd + (k / 4) * (kSlot >> 5) + (k & 3) * 2, idesc,
                                    (u > 0 || k > 0) ? 1u : 0u);
-            slot_done();
+            ptx::tc_commit_pair(&empty[slot]);
+            if (++slot == K::kSlots) { slot = 0; par ^= 1u; }
           }
           if (!ok) break;
           ptx::tc_commit_pair(&s_full[s1]);
-          if (++s1 == K::kS) s1 = 0;
-          if (++c1 == p.chunks) {
-            ptx::tc_commit_pair(&a_done[t1 & 1]);
-            c1 = 0;
-            ++t1;
-          }
+          if (++s1 == K::kS) { s1 = 0; s_par ^= 1u; }
         }
-        if (i >= kLag) {
-          if (c2 == 0 && !ptx::mbar_wait(o_empty, (t2 & 1) ^ 1, 405)) break;
-          if (!ptx::mbar_wait(&h_ready[s2], h_par, 406)) break;
-          const uint64_t wd = slot_wait();
+        if (ok) ptx::tc_commit_pair(&a_done[ab]);
+        if (++ab == K::kA) { ab = 0; a_par ^= 1u; }
+      }
+    }
+  } else if (warp == 3) {
+    // ---------------------------------------------------------------- O.  (By a thread of its own: one for both products took 1 370 cycles a
+    // chunk for its waits and commits, of which the products are 768 at 128 channels.)
+    if (rank == 0 && ptx::elect_one()) {
+      constexpr uint32_t idesc = ptx::make_idesc(2 * kRows, C, 1);
+      const uint64_t v_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_v));
+      int s2 = 0;
+      uint32_t par = 0;
+      bool ok = true;
+      for (int it = 0; ok && it < my_tiles; ++it) {
+        ok = ptx::mbar_wait(o_empty, (it & 1) ^ 1, 405);
+        for (int c = 0; ok && c < p.chunks; ++c) {
+          ok = ptx::mbar_wait(&v_full[s2], par, 418) && ptx::mbar_wait(&h_ready[s2], par, 406);
           if (!ok) break;
+          ptx::tc_fence_after_sync();
 #pragma unroll
           for (int k = 0; k < kChunk / 16; ++k)
-            ptx::mma_f16_ts_pair(tmem_base, tmem_s + s2 * 128 + k * 8, wd + k * 2, idesc_o, (c2 > 0 || k > 0) ? 1u : 0u);
-          slot_done();
-          if (++s2 == K::kS) { s2 = 0; h_par ^= 1u; }
-          if (++c2 == p.chunks) {
-            ptx::tc_commit_pair(o_full);
-            c2 = 0;
-            ++t2;
-          }
+            ptx::mma_f16_ts_pair(tmem_base, tmem_s + s2 * 128 + k * 8, v_desc + static_cast<uint64_t>(s2 * (K::kOutUnit >> 4)) + k * 2, idesc,
+                                 (c > 0 || k > 0) ? 1u : 0u);
+          ptx::tc_commit_pair(&v_free[s2]);
+          ptx::tc_fence_before_sync();
+          ptx::mbar_arrive(&o_sent[s2]);
+          if (++s2 == K::kS) { s2 = 0; par ^= 1u; }
         }
+        if (ok) ptx::tc_commit_pair(o_full);
       }
     }
   } else if (warp >= kGluWarp) {
@@ -266,100 +308,95 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     }
   } else if (warp >= kRowWarp) {
     // ---------------------------------------------------------------- rows: LayerNorm of the next tile, residual and output of the last
-    const int quad = warp & 3;
-    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16);
-    const bool issuer = quad == 0 && ptx::elect_one();
+    const int part = warp - kRowWarp, quad = warp & 3;
+    constexpr int kHalf = C / 2;                 // output columns of a warp: two warps share a quadrant's rows
+    const int col0 = part / 4 * kHalf;
+    const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + col0;
     grid_dependency_wait();
     float lw[8], lb[8];
     rows_affine<C>(p.ln_w, p.ln_b, lane, lw, lb);
-    auto row0_of = [&](int it) { return (2 * (tile0 + it * tile_step) + rank) * kRows; };
-    auto fetch = [&](const CUtensorMap* map, int it) {      // a tile's rows into its buffer
-      uint8_t* dst = s_a + (it & 1) * K::kABytes;
-      ptx::mbar_expect_tx(&rows_in[it & 1], K::kABytes);
-#pragma unroll
-      for (int kb = 0; kb < C / 64; ++kb) ptx::tma_load_4d(dst + kb * kBox, map, &rows_in[it & 1], kb * 64, row0_of(it), 0, 0);
-    };
-    uint32_t in_par = 0;        // bit b: phase of rows_in[b]
     bool ok = true;
-    auto wait_rows = [&](int b) -> bool {
-      const bool r = __all_sync(0xffffffffu, ptx::mbar_wait(&rows_in[b], (in_par >> b) & 1, 408)) != 0;
-      in_par ^= 1u << b;
-      return r;
-    };
-    if (issuer) {
-      fetch(&tm_x, 0);
-      if (my_tiles > 1) fetch(&tm_x, 1);
-    }
+    int ab = 0, ob = 0;                          // buffers of the next tile and of the last, and their phases
+    uint32_t a_par = 0, o_par = 0;
     for (int it = 0; it <= my_tiles; ++it) {
       if (it < my_tiles) {
-        ok = wait_rows(it & 1);
+        ok = __all_sync(0xffffffffu, ptx::mbar_wait(&rows_in[ab], a_par, 408)) != 0;
         if (!ok) break;
-        uint8_t* a = s_a + (it & 1) * K::kABytes;
-        rows_layernorm<C>(a, quad * 32, 32, lane, lw, lb, p.eps);
+        rows_layernorm<C>(s_a + ab * K::kABytes, part * (kRows / kRowWarps), kRows / kRowWarps, lane, lw, lb, p.eps);
         ptx::fence_proxy_async_smem();
         __syncwarp();
-        if (lane == 0) ptx::mbar_arrive_cluster_release(ptx::leader_addr(&a_ready[it & 1]));
+        if (lane == 0) ptx::mbar_arrive(&a_norm[ab]);
+        if (++ab == K::kA) { ab = 0; a_par ^= 1u; }
       }
       if (it == 0) continue;
-      // output of the tile before: its buffer takes the residual once its last S has read the rows
-      const int done = it - 1, b = done & 1;
-      uint8_t* a = s_a + b * K::kABytes;
-      ok = __all_sync(0xffffffffu, ptx::mbar_wait(&a_done[b], (done >> 1) & 1, 409)) != 0;
+      // output of the tile before, over its rows (every S has read them) and, where there is one, the residual that has come in their place
+      uint8_t* a = s_a + ob * K::kABytes;
+      ok = __all_sync(0xffffffffu, ptx::mbar_wait(p.has_resid ? &resid_in[ob] : &a_done[ob], o_par, 409)) != 0;
       if (!ok) break;
-      if (p.has_resid) {
-        if (issuer) fetch(&tm_r, done);
-        ok = wait_rows(b);
-        if (!ok) break;
-      }
-      ok = __all_sync(0xffffffffu, ptx::mbar_wait(o_full, done & 1, 410)) != 0;
+      ok = __all_sync(0xffffffffu, ptx::mbar_wait(o_full, (it - 1) & 1, 410)) != 0;
       if (!ok) break;
       ptx::tc_fence_after_sync();
-      {
-        const int r = quad * 32 + lane;
+      const int r = quad * 32 + lane;
+#pragma unroll 1
+      for (int c = 0; c < kHalf; c += 64) {
         uint32_t x[2][32];
-        ptx::tmem_ld_32x32b_x32(t_row, x[0]);
+        ptx::tmem_ld_32x32b_x32(t_row + c, x[0]);
+        ptx::tmem_ld_32x32b_x32(t_row + c + 32, x[1]);
+        ptx::tmem_ld_wait();
+        if (c + 64 == kHalf) {
+          ptx::tc_fence_before_sync();
+          __syncwarp();
+          if (lane == 0) ptx::mbar_arrive_cluster(ptx::leader_addr(o_empty));
+        }
+        uint8_t* row = a + (col0 + c) / 64 * kBox + r * 128;
 #pragma unroll
-        for (int c = 0; c < C / 32; ++c) {
-          ptx::tmem_ld_wait();
-          if (c + 1 < C / 32) ptx::tmem_ld_32x32b_x32(t_row + 32 * (c + 1), x[(c + 1) & 1]);
-          uint8_t* row = a + (c >> 1) * kBox + r * 128;
+        for (int i = 0; i < 8; ++i) {
+          uint4* cell = reinterpret_cast<uint4*>(row + ((i ^ (r & 7)) << 4));
+          const uint4 u = p.has_resid ? *cell : make_uint4(0, 0, 0, 0);
+          const uint32_t rw[4] = {u.x, u.y, u.z, u.w};
+          uint32_t w[4];
 #pragma unroll
-          for (int i = 0; i < 4; ++i) {
-            uint4* cell = reinterpret_cast<uint4*>(row + ((((c & 1) * 4 + i) ^ (r & 7)) << 4));
-            const uint4 u = p.has_resid ? *cell : make_uint4(0, 0, 0, 0);
-            const uint32_t rw[4] = {u.x, u.y, u.z, u.w};
-            uint32_t w[4];
-#pragma unroll
-            for (int j = 0; j < 4; ++j)
-              w[j] = pack_bf16x2(__uint_as_float(x[c & 1][8 * i + 2 * j]) + __uint_as_float(rw[j] << 16),
-                                 __uint_as_float(x[c & 1][8 * i + 2 * j + 1]) + __uint_as_float(rw[j] & 0xffff0000u));
-            *cell = make_uint4(w[0], w[1], w[2], w[3]);
-          }
+          for (int j = 0; j < 4; ++j)
+            w[j] = pack_bf16x2(__uint_as_float(x[i >> 2][8 * (i & 3) + 2 * j]) + __uint_as_float(rw[j] << 16),
+                               __uint_as_float(x[i >> 2][8 * (i & 3) + 2 * j + 1]) + __uint_as_float(rw[j] & 0xffff0000u));
+          *cell = make_uint4(w[0], w[1], w[2], w[3]);
         }
       }
-      ptx::tc_fence_before_sync();
       ptx::fence_proxy_async_smem();
       __syncwarp();
-      if (lane == 0) {
-        ptx::mbar_arrive_cluster(ptx::leader_addr(o_empty));
-        ptx::mbar_arrive(out_done);
-      }
-      if (quad == 0) {
-        ok = __all_sync(0xffffffffu, ptx::mbar_wait(out_done, done & 1, 411)) != 0;
-        if (!ok) break;
-        if (issuer) {
-          if (row0_of(done) < p.rows) {
-#pragma unroll
-            for (int kb = 0; kb < C / 64; ++kb) ptx::tma_store_4d(&tm_out, a + kb * kBox, kb * 64, row0_of(done), 0, 0);
-            ptx::tma_store_commit();
-            ptx::tma_store_wait_read();
-          }
-          if (done + 2 < my_tiles) fetch(&tm_x, done + 2);
-        }
-        __syncwarp();
-      }
+      if (lane == 0) ptx::mbar_arrive(&out_done[ob]);
+      if (++ob == K::kA) { ob = 0; o_par ^= 1u; }
     }
-    if (issuer) ptx::tma_store_wait_all();
+  } else if (warp == 2) {
+    // ---------------------------------------------------------------- a buffer's course: rows in, residual in once every S has read them, output out
+    if (ptx::elect_one()) {
+      grid_dependency_wait();
+      auto row0_of = [&](int it) { return (2 * (tile0 + it * tile_step) + rank) * kRows; };
+      auto fetch = [&](const CUtensorMap* map, uint64_t* bar, int it, int b) {
+        ptx::mbar_expect_tx(bar, K::kABytes);
+#pragma unroll
+        for (int kb = 0; kb < C / 64; ++kb) ptx::tma_load_4d(s_a + b * K::kABytes + kb * kBox, map, bar, kb * 64, row0_of(it), 0, 0);
+      };
+      for (int it = 0; it < K::kA && it < my_tiles; ++it) fetch(&tm_x, &rows_in[it], it, it);
+      int b = 0;
+      uint32_t b_par = 0;
+      for (int it = 0; it < my_tiles; ++it) {
+        if (!ptx::mbar_wait(&a_done[b], b_par, 414)) break;
+        if (p.has_resid) fetch(&tm_r, &resid_in[b], it, b);
+        if (!ptx::mbar_wait(&out_done[b], b_par, 411)) break;
+        if (row0_of(it) < p.rows) {
+#pragma unroll
+          for (int kb = 0; kb < C / 64; ++kb) ptx::tma_store_4d(&tm_out, s_a + b * K::kABytes + kb * kBox, kb * 64, row0_of(it), 0, 0);
+          ptx::tma_store_commit();
+        }
+        if (it + K::kA < my_tiles) {
+          ptx::tma_store_wait_read();
+          fetch(&tm_x, &rows_in[b], it + K::kA, b);
+        }
+        if (++b == K::kA) { b = 0; b_par ^= 1u; }
+      }
+      ptx::tma_store_wait_all();
+    }
   }
 
   ptx::tc_fence_before_sync();
