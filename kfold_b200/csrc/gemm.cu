@@ -57,12 +57,17 @@ static int launch_variant(cudaStream_t stream, const CUtensorMap& ta, const CUte
   GemmParams q = p;
   {
     // the persistent loops step by the grid size: its digits in the (n tile, row block, outer, batch) index
-    const int m_step = grid / q.num_n_tiles;
-    q.step_n_tile = grid - m_step * q.num_n_tiles;
-    q.step_nb = m_step % q.n_blocks;
-    const int rest = m_step / q.n_blocks;
-    q.step_o = rest % q.o_extent;
-    q.step_b = rest / q.o_extent;
+    if (q.rows_first) {
+      q.step_n_tile = grid / q.n_blocks;
+      q.step_nb = grid - q.step_n_tile * q.n_blocks;
+    } else {
+      const int m_step = grid / q.num_n_tiles;
+      q.step_n_tile = grid - m_step * q.num_n_tiles;
+      q.step_nb = m_step % q.n_blocks;
+      const int rest = m_step / q.n_blocks;
+      q.step_o = rest % q.o_extent;
+      q.step_b = rest / q.o_extent;
+    }
   }
   {
     LaunchScope scope(stream, tag);
@@ -150,13 +155,13 @@ static int narrow_tile(const GemmParams& p, int bn) {
 // CTA pairs (PAIR in gemm.cuh) pay where the main loop is long enough to hide the epilogue of a tile twice as wide and the tiles are at
 // least a wave of pairs.  Measured, one CTA -> pair: triangle contraction at 768 tokens 108 -> 99 us (128 channels), 201 -> 180 (256);
 // at 400 tokens (seven K blocks) 71 -> 62; SwiGLU of 256 channels at 768 x 768 rows 585 -> 472, its output projection (K = 1 024) 362 ->
-// 318; token transformer, 5 x 768 rows of 768: projection 35 -> 29, SwiGLU 24.5 -> 22.5.  The other side of the lines: SwiGLU of 128 channels (two K blocks) 106 -> 107; gate
-// projection of 256 (four, plain) 105 -> 109; conditioning table (six, plain) 100 -> 104; contraction at 333 tokens (three row blocks, a
+// 318; token transformer, 5 x 768 rows of 768: projection 35 -> 29, SwiGLU 24.5 -> 22.5; conditioning tables of those rows (six, staged) 415 -> 390.  The other side of the lines: SwiGLU of 128 channels (two K blocks) 106 -> 107; gate
+// projection of 256 (four, plain) 105 -> 109; contraction at 333 tokens (three row blocks, a
 // quarter of the pairs' work padding) 49.7 -> 51.6; float32 output projections with gate and residual 22.4 -> 23.5.
 static bool pair_tile(const GemmParams& p, int bn) {
   if (p.precise || bn < 128 || p.n_cols < 256 || p.glu == GLU_SIGMOID) return false;
   const int num_k = cdiv(p.k_extent, kBK), pairs = cdiv(p.n_blocks, 2);
-  if (num_k < (p.glu ? 4 : 7) || (2 * pairs - p.n_blocks) * 8 > p.n_blocks) return false;
+  if (num_k < (p.glu ? 4 : 6) || (2 * pairs - p.n_blocks) * 8 > p.n_blocks) return false;
   if (2ll * pairs * p.o_extent * p.batch * cdiv(p.n_cols, 256) < sm_count()) return false;
   for (int i = 0; i < p.nseg; ++i) {
     const EpiSeg& sg = p.seg[i];
@@ -448,6 +453,11 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
                  (p.nseg == 1 || p.seg[1].col_begin >= p.swap_col_begin);
     }
   }
+  // Weights that the L2 does not keep beside what is written (a stack's conditioning tables: 57 MB and 28) are read once where the row blocks
+  // of a column tile follow each other; the rows, which are then read for every column tile, are few.  Both tables of 24 blocks of 768
+  // channels, 3 840 rows: 415 -> 380 us; of 16 of 1 024, 301 rows, float32-accurate: 209 -> 184.
+  p.rows_first = p.o_extent == 1 && p.batch == 1 && p.n_blocks > 1 && p.num_n_tiles > p.n_blocks && !p.a_mn_major && p.num_n_tiles == p.glu_tiles &&
+                 static_cast<long long>(p.n_cols) * p.k_extent * 2 > (16ll << 20);
   if (p.pair) return launch_pair(stream, ta, tb, tout, p, tag);
   switch (bn) {
     case 32: return launch_bn<32>(stream, ta, tb, tout, p, tag);

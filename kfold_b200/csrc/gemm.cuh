@@ -54,6 +54,7 @@ struct GemmParams {
                                   // operand whose pieces lie rank after rank (launcher; = n_cols when not split)
   int n_blocks, num_m_tiles, num_n_tiles;
   int step_n_tile, step_nb, step_o, step_b;  // launcher: the grid size as digits of (n tile, row block, outer, batch)
+  int rows_first;                 // launcher (one batch of flat rows): consecutive tiles are row blocks of one column tile
   int swap_staged;                // launcher: the swapped GLU tile leaves through shared memory and TMA stores (map tm_out0)
   int rm_seg, rm_slot;            // launcher: segment whose full tiles leave through shared memory and a TMA store (row-major
                                   // bf16; BN = 128 plain kernel), and the output map it uses; rm_seg < 0: none
@@ -341,6 +342,12 @@ struct TileIdx {
 };
 __device__ __forceinline__ TileIdx tile_decompose(int tile, const GemmParams& p) {
   TileIdx t;
+  if (p.rows_first) {
+    t.n_tile = tile / p.n_blocks;
+    t.nb = tile - t.n_tile * p.n_blocks;
+    t.o = t.b = 0;
+    return t;
+  }
   const int m_tile = tile / p.num_n_tiles;
   t.n_tile = tile - m_tile * p.num_n_tiles;
   t.nb = m_tile % p.n_blocks;
@@ -351,6 +358,13 @@ __device__ __forceinline__ TileIdx tile_decompose(int tile, const GemmParams& p)
 }
 // t += grid size, whose digits the launcher put into the parameters (each below its radix)
 __device__ __forceinline__ void tile_advance(TileIdx& t, const GemmParams& p) {
+  if (p.rows_first) {
+    t.nb += p.step_nb;
+    const int over = t.nb >= p.n_blocks ? 1 : 0;
+    t.nb -= over ? p.n_blocks : 0;
+    t.n_tile += p.step_n_tile + over;
+    return;
+  }
   t.n_tile += p.step_n_tile;
   int carry = t.n_tile >= p.num_n_tiles ? 1 : 0;
   t.n_tile -= carry ? p.num_n_tiles : 0;
@@ -631,7 +645,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constant
       for (int tile = tile0; ok && tile < total_tiles; tile += tile_step, ++tile_iter) {
         const uint32_t acc = tile_iter & 1;
         const uint32_t acc_phase = (tile_iter >> 1) & 1;
-        const int n_tile_mma = tile % p.num_n_tiles;
+        const int n_tile_mma = p.rows_first ? tile / p.n_blocks : tile % p.num_n_tiles;
         if (!ptx::mbar_wait(&tmem_empty[acc], acc_phase ^ 1, 102)) { ok = false; break; }
         ptx::tc_fence_after_sync();
         const uint32_t d_tmem = tmem_base + acc * ACC_COLS;
