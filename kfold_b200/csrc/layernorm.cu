@@ -760,7 +760,8 @@ __global__ void __launch_bounds__(256) adaln_vec_kernel(const TI* a, __nv_bfloat
     const long long row = base + lane / LANES;
     const bool live = row < rows;
     const long long rr = live ? row : 0;
-    const long long srow = (rr / (static_cast<long long>(samples) * l)) * l + rr % l;
+    const unsigned r32 = static_cast<unsigned>(rr);     // (the launcher sends 2^31 rows and more elsewhere; a 64-bit division is 400 cycles)
+    const long long srow = static_cast<long long>(r32 / (static_cast<unsigned>(samples) * static_cast<unsigned>(l))) * l + r32 % static_cast<unsigned>(l);
     const TI* xr = a + rr * c;
     const __nv_bfloat16* gr = gv + srow * gv_ld;
     uint4 gt[CH], sh[CH];
@@ -870,7 +871,7 @@ int launch_adaln(cudaStream_t stream, const void* a, void* y, const void* gv, lo
                 samples, l);
   KFB_CHECK_ARG(rows % (static_cast<long long>(samples) * l) == 0, "adaln: rows %lld is not a multiple of samples*l", rows);
   if (rows == 0) return KFB_OK;
-  if ((in_dtype == KFB_BF16 || in_dtype == KFB_FP32) && out_dtype == KFB_BF16 && gv_ld % 8 == 0 &&
+  if ((in_dtype == KFB_BF16 || in_dtype == KFB_FP32) && out_dtype == KFB_BF16 && gv_ld % 8 == 0 && rows < (1ll << 31) &&
       ((reinterpret_cast<uintptr_t>(a) | reinterpret_cast<uintptr_t>(y) | reinterpret_cast<uintptr_t>(gv)) & 15) == 0) {
 #define KFB_ADALN_VEC(CH, LANES)                                                                                          \
   return in_dtype == KFB_BF16 ? launch_adaln_vec<__nv_bfloat16, CH, LANES>(stream, a, y, gv, gv_ld, rows, samples, l, eps, gv_static) \

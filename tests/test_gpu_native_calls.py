@@ -510,3 +510,32 @@ def test_nothing_is_written_past_the_reported_workspace(dev, monkeypatch, n, bat
             ws, nbytes = arenas[-1]
             assert (ws[nbytes:] == 0xAB).all()
         assert torch.equal(*results)
+
+
+@pytest.mark.parametrize("rows", [1, 23, 9472, 20001])
+@pytest.mark.parametrize("bf16", [False, True])
+def test_atom_rows_of_128_channels(dev, rows, bf16):
+    """The coordinate embedding and the projection to updates at 128 channels: one row, rows that leave a pair's second empty, as many as
+    warps, more than go round once; masked atoms; three samples that share features and mask."""
+    from kfold_b200 import _lib as L
+    lib, samples = L.lib(), 3
+    g = torch.Generator(device=dev).manual_seed(rows)
+    rnd = lambda *shape: torch.randn(shape, generator=g, device=dev)
+    dt, code = (torch.bfloat16, L.KFB_BF16) if bf16 else (torch.float32, L.KFB_FP32)
+    mask = torch.rand(rows, generator=g, device=dev) < 0.8
+    q, r, w = rnd(rows, 128).to(dt), rnd(samples, rows, 3), rnd(128, 3)
+    out = torch.full((samples * rows * 128 + 8,), 7.0, device=dev)
+    L.check(lib.kfb_coord_embed(L.ptr(q), L.ptr(r), L.ptr(w), L.ptr(mask), L.ptr(out), samples * rows, 128, 3, samples, rows, code, L.stream_ptr()))
+    rm = r.double() * mask[:, None]
+    ref = q.double() + rm @ w.double().T
+    assert ((out[:-8].view(samples, rows, 128) - ref).abs() <= 4 * 2.0 ** -24 * (q.double().abs() + rm.abs() @ w.double().abs().T)).all()
+    assert (out[-8:] == 7.0).all()
+    x, lw, lb, wo = (rnd(samples * rows, 128) * 2 + 0.5).to(dt), rnd(128), rnd(128), rnd(3, 128)
+    upd = torch.full((samples * rows * 3 + 8,), 7.0, device=dev)
+    L.check(lib.kfb_ln_project(L.ptr(x), L.ptr(lw), L.ptr(lb), L.ptr(wo), L.ptr(mask), L.ptr(upd), samples * rows, 128, 3, 1e-5, samples, rows, code,
+                               L.stream_ptr()))
+    xn = torch.nn.functional.layer_norm(x.double(), (128,), lw.double(), lb.double(), 1e-5)
+    ref = (xn @ wo.double().T).view(samples, rows, 3) * mask[:, None]
+    # 128 products and a normalisation in float32
+    assert ((upd[:-8].view(samples, rows, 3) - ref).abs() <= 2e-6 * (xn.abs() @ wo.double().abs().T).view(samples, rows, 3)).all()
+    assert (upd[-8:] == 7.0).all()
