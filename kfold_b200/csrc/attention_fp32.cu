@@ -47,24 +47,25 @@ __device__ __forceinline__ float2 halves_of(uint64_t v) {
   return f;
 }
 
-template <int D, int QPT, int kWarps>
+template <int D, int QPT, int LPR, int kWarps>
 struct F32Cfg {
-  static constexpr int kQ = 32 * QPT;
-  static constexpr int kRing = kWarps * 2 * 2 * kKeys * D;             // floats: [warp][slot][K | V][key][D]
+  static constexpr int kQ = 32 / LPR * QPT;
+  static constexpr int kPitch = LPR == 2 ? D + 4 : D;                  // a row's halves 4 banks apart
+  static constexpr int kRing = kWarps * 2 * 2 * kKeys * kPitch;        // floats: [warp][slot][K | V][key][kPitch]
   static constexpr int kMerge = (kWarps / 2) * kQ * (D + 1);           // the same memory after the loop
   static constexpr int kMain = kRing > kMerge ? kRing : kMerge;
   static constexpr int kBias = kWarps * kQ * (kKeys + 1);
   static constexpr int kSmem = (kMain + kBias + 2 * kWarps * kQ) * 4;
 };
 
-template <int D, int QPT, int kWarps>
-__global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnFp32Params p) {
-  using Cfg = F32Cfg<D, QPT, kWarps>;
-  constexpr int kQ = Cfg::kQ;
+template <int D, int QPT, int LPR, int kWarps>
+__global__ void __launch_bounds__(kWarps * 32, LPR == 2 ? 2 : 1) attention_fp32_kernel(const AttnFp32Params p) {
+  using Cfg = F32Cfg<D, QPT, LPR, kWarps>;
+  constexpr int kQ = Cfg::kQ, kPitch = Cfg::kPitch, kL = 32 / LPR, DL = D / LPR;    // rows side by side in a warp, channels of a lane
   grid_dependency_enter();
   extern __shared__ __align__(16) float smem[];
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  float* ring = smem + warp * (4 * kKeys * D);
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31, lrow = lane % kL, part = lane / kL;
+  float* ring = smem + warp * (4 * kKeys * kPitch);
   float* s_bias = smem + Cfg::kMain + warp * kQ * (kKeys + 1);
   float* s_m = smem + Cfg::kMain + Cfg::kBias;      // [warp][query]
   float* s_l = s_m + kWarps * kQ;
@@ -80,40 +81,42 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
   const float* k_base = p.k + static_cast<long long>(b) * p.lk * ld_kv + p.k_col0 + h * D;
   const float* v_base = p.v + static_cast<long long>(b) * p.lk * ld_kv + p.v_col0 + h * D;
 
-  uint64_t q[QPT][D / 2], acc2[QPT][D / 2];      // pairs of neighbouring channels
+  uint64_t q[QPT][DL / 2], acc2[QPT][DL / 2];      // pairs of neighbouring channels
   float m_run[QPT], l_run[QPT];
 #pragma unroll
   for (int i = 0; i < QPT; ++i) {
-    const long long row = static_cast<long long>(b) * p.lq + min(q0 + i * 32 + lane, p.lq - 1);
-    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(p.q + row * p.ld + p.q_col0 + h * D);
+    const long long row = static_cast<long long>(b) * p.lq + min(q0 + i * kL + lrow, p.lq - 1);
+    const ulonglong2* src = reinterpret_cast<const ulonglong2*>(p.q + row * p.ld + p.q_col0 + h * D + part * DL);
 #pragma unroll
-    for (int d = 0; d < D / 4; ++d) {
+    for (int d = 0; d < DL / 4; ++d) {
       const ulonglong2 f = src[d];
       q[i][2 * d] = f.x;
       q[i][2 * d + 1] = f.y;
     }
 #pragma unroll
-    for (int d = 0; d < D / 2; ++d) acc2[i][d] = 0;
+    for (int d = 0; d < DL / 2; ++d) acc2[i][d] = 0;
     m_run[i] = -INFINITY;
     l_run[i] = 0.f;
   }
 
   const int groups = (p.lk + kKeys - 1) / kKeys;
   // bias and mask of a group are fetched a step ahead: lane = (row of four, key), which reads whole sectors
-  float bias_r[8 * QPT], mask_r = 0.f;
+  constexpr int kFetch = kQ / 4;
+  float bias_r[kFetch], mask_r = 0.f;
   auto fetch = [&](int g, int slot) {
-    float* dst = ring + slot * (2 * kKeys * D);
+    float* dst = ring + slot * (2 * kKeys * kPitch);
 #pragma unroll
     for (int idx = lane; idx < kKeys * D / 4; idx += 32) {
       const int kk = idx / (D / 4), c = idx - kk * (D / 4);
       const long long off = static_cast<long long>(min(g * kKeys + kk, p.lk - 1)) * ld_kv + c * 4;
-      cp_async16(dst + idx * 4, k_base + off);
-      cp_async16(dst + kKeys * D + idx * 4, v_base + off);
+      const int at = kk * kPitch + c * 4 + (LPR == 2 && c >= DL / 4 ? 4 : 0);
+      cp_async16(dst + at, k_base + off);
+      cp_async16(dst + kKeys * kPitch + at, v_base + off);
     }
     const int key = g * kKeys + (lane & 7);
     mask_r = key < p.lk ? ((mrow == nullptr || mrow[static_cast<long long>(key) * p.m_k]) ? 0.f : -1e9f) : -INFINITY;
 #pragma unroll
-    for (int i = 0; i < 8 * QPT; ++i) {
+    for (int i = 0; i < kFetch; ++i) {
       const int row = min(q0 + i * 4 + (lane >> 3), p.lq - 1);
       bias_r[i] = key < p.lk ? bias_base[static_cast<long long>(row) * p.ldb + key] : 0.f;
     }
@@ -124,23 +127,23 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
   for (int g = warp; g < groups; g += kWarps, slot ^= 1) {
     const float mask_v = mask_r;
 #pragma unroll
-    for (int i = 0; i < 8 * QPT; ++i) s_bias[(i * 4 + (lane >> 3)) * (kKeys + 1) + (lane & 7)] = bias_r[i];
+    for (int i = 0; i < kFetch; ++i) s_bias[(i * 4 + (lane >> 3)) * (kKeys + 1) + (lane & 7)] = bias_r[i];
     if (g + kWarps < groups) fetch(g + kWarps, slot ^ 1);
     asm volatile("cp.async.commit_group;" ::: "memory");
     asm volatile("cp.async.wait_group 1;" ::: "memory");
     __syncwarp();
-    const ulonglong2* sk = reinterpret_cast<const ulonglong2*>(ring + slot * (2 * kKeys * D));
-    const ulonglong2* sv = sk + kKeys * D / 4;
+    const ulonglong2* sk = reinterpret_cast<const ulonglong2*>(ring + slot * (2 * kKeys * kPitch) + part * (DL + 4));
+    const ulonglong2* sv = sk + kKeys * kPitch / 4;
     uint64_t s2[QPT][kKeys];
 #pragma unroll
     for (int i = 0; i < QPT; ++i)
 #pragma unroll
       for (int kk = 0; kk < kKeys; ++kk) s2[i][kk] = 0;
 #pragma unroll
-    for (int d = 0; d < D / 4; ++d)
+    for (int d = 0; d < DL / 4; ++d)
 #pragma unroll
       for (int kk = 0; kk < kKeys; ++kk) {
-        const ulonglong2 f = sk[kk * (D / 4) + d];
+        const ulonglong2 f = sk[kk * (kPitch / 4) + d];
 #pragma unroll
         for (int i = 0; i < QPT; ++i) {
           s2[i][kk] = fma2(q[i][2 * d], f.x, s2[i][kk]);
@@ -155,7 +158,9 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
       for (int kk = 0; kk < kKeys; ++kk) {
         // same order of additions as the reference: (q k + mask) + bias
         const float2 f = halves_of(s2[i][kk]);
-        s[i][kk] = ((f.x + f.y) + __shfl_sync(0xffffffffu, mask_v, kk)) + s_bias[(i * 32 + lane) * (kKeys + 1) + kk];
+        float qk = f.x + f.y;
+        if constexpr (LPR == 2) qk += __shfl_xor_sync(0xffffffffu, qk, kL);
+        s[i][kk] = (qk + __shfl_sync(0xffffffffu, mask_v, kk)) + s_bias[(i * kL + lrow) * (kKeys + 1) + kk];
         mx = fmaxf(mx, s[i][kk]);
       }
       const float m_new = fmaxf(m_run[i], mx);
@@ -163,7 +168,7 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
       const uint64_t a2 = pair_of(alpha, alpha);
       l_run[i] *= alpha;
 #pragma unroll
-      for (int d = 0; d < D / 2; ++d) acc2[i][d] = mul2(acc2[i][d], a2);
+      for (int d = 0; d < DL / 2; ++d) acc2[i][d] = mul2(acc2[i][d], a2);
 #pragma unroll
       for (int kk = 0; kk < kKeys; ++kk) {
         s[i][kk] = expf(s[i][kk] - m_new);
@@ -177,8 +182,8 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
 #pragma unroll
       for (int i = 0; i < QPT; ++i) p2[i] = pair_of(s[i][kk], s[i][kk]);
 #pragma unroll
-      for (int d = 0; d < D / 4; ++d) {
-        const ulonglong2 f = sv[kk * (D / 4) + d];
+      for (int d = 0; d < DL / 4; ++d) {
+        const ulonglong2 f = sv[kk * (kPitch / 4) + d];
 #pragma unroll
         for (int i = 0; i < QPT; ++i) {
           acc2[i][2 * d] = fma2(p2[i], f.x, acc2[i][2 * d]);
@@ -189,11 +194,11 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
     __syncwarp();   // the slot and the bias tile may be written again
   }
 
-  float acc[QPT][D];
+  float acc[QPT][DL];
 #pragma unroll
   for (int i = 0; i < QPT; ++i)
 #pragma unroll
-    for (int d = 0; d < D / 2; ++d) {
+    for (int d = 0; d < DL / 2; ++d) {
       const float2 f = halves_of(acc2[i][d]);
       acc[i][2 * d] = f.x;
       acc[i][2 * d + 1] = f.y;
@@ -202,8 +207,8 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
   // merge the warps' softmax states; a warp without keys has m = -inf, l = 0
 #pragma unroll
   for (int i = 0; i < QPT; ++i) {
-    s_m[warp * kQ + i * 32 + lane] = m_run[i];
-    s_l[warp * kQ + i * 32 + lane] = l_run[i];
+    s_m[warp * kQ + i * kL + lrow] = m_run[i];
+    s_l[warp * kQ + i * kL + lrow] = l_run[i];
   }
   __syncthreads();
   float inv_l[QPT];
@@ -211,13 +216,13 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
   for (int i = 0; i < QPT; ++i) {
     float m = -INFINITY, l = 0.f;
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) m = fmaxf(m, s_m[w * kQ + i * 32 + lane]);
+    for (int w = 0; w < kWarps; ++w) m = fmaxf(m, s_m[w * kQ + i * kL + lrow]);
 #pragma unroll
-    for (int w = 0; w < kWarps; ++w) l += s_l[w * kQ + i * 32 + lane] * expf(s_m[w * kQ + i * 32 + lane] - m);
+    for (int w = 0; w < kWarps; ++w) l += s_l[w * kQ + i * kL + lrow] * expf(s_m[w * kQ + i * kL + lrow] - m);
     inv_l[i] = 1.0f / l;
     const float scale = expf(m_run[i] - m);
 #pragma unroll
-    for (int d = 0; d < D; ++d) acc[i][d] *= scale;
+    for (int d = 0; d < DL; ++d) acc[i][d] *= scale;
   }
 #pragma unroll 1
   for (int half = kWarps / 2; half >= 1; half >>= 1) {
@@ -225,14 +230,14 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
 #pragma unroll
       for (int i = 0; i < QPT; ++i)
 #pragma unroll
-        for (int d = 0; d < D; ++d) smem[((warp - half) * kQ + i * 32 + lane) * (D + 1) + d] = acc[i][d];
+        for (int d = 0; d < DL; ++d) smem[((warp - half) * kQ + i * kL + lrow) * (D + 1) + part * DL + d] = acc[i][d];
     }
     __syncthreads();
     if (warp < half) {
 #pragma unroll
       for (int i = 0; i < QPT; ++i)
 #pragma unroll
-        for (int d = 0; d < D; ++d) acc[i][d] += smem[(warp * kQ + i * 32 + lane) * (D + 1) + d];
+        for (int d = 0; d < DL; ++d) acc[i][d] += smem[(warp * kQ + i * kL + lrow) * (D + 1) + part * DL + d];
     }
     __syncthreads();
   }
@@ -240,7 +245,7 @@ __global__ void __launch_bounds__(kWarps * 32) attention_fp32_kernel(const AttnF
 #pragma unroll
     for (int i = 0; i < QPT; ++i)
 #pragma unroll
-      for (int d = 0; d < D; ++d) smem[(i * 32 + lane) * (D + 1) + d] = acc[i][d] * inv_l[i];
+      for (int d = 0; d < DL; ++d) smem[(i * kL + lrow) * (D + 1) + part * DL + d] = acc[i][d] * inv_l[i];
   }
   __syncthreads();
   const int hd = p.heads * D;
@@ -505,20 +510,20 @@ bool takes_rows(const AttnFp32Params& p) {
          p.q_col0 % 4 == 0 && p.k_col0 % 4 == 0 && p.v_col0 % 4 == 0 && (p.g == nullptr || p.g_col0 % 4 == 0) && (p.heads * p.d) % 8 == 0;
 }
 
-template <int D, int QPT, int kWarps>
+template <int D, int QPT, int LPR, int kWarps>
 int launch(cudaStream_t stream, const AttnFp32Params& p) {
-  using Cfg = F32Cfg<D, QPT, kWarps>;
+  using Cfg = F32Cfg<D, QPT, LPR, kWarps>;
   static std::once_flag once[64];
   int dev = 0;
   KFB_CUDA(cudaGetDevice(&dev));
   cudaError_t attr_err = cudaSuccess;
   std::call_once(once[dev & 63], [&] {
-    attr_err = cudaFuncSetAttribute(attention_fp32_kernel<D, QPT, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
+    attr_err = cudaFuncSetAttribute(attention_fp32_kernel<D, QPT, LPR, kWarps>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg::kSmem);
   });
   KFB_CUDA(attr_err);
   LaunchScope scope(stream, p.tag ? p.tag : "attention_fp32");
   const dim3 grid(cdiv(p.lq, Cfg::kQ), p.heads, p.batch);
-  KFB_TRY(launch_kernel(stream, attention_fp32_kernel<D, QPT, kWarps>, grid, kWarps * 32, Cfg::kSmem, p));
+  KFB_TRY(launch_kernel(stream, attention_fp32_kernel<D, QPT, LPR, kWarps>, grid, kWarps * 32, Cfg::kSmem, p));
   return KFB_OK;
 }
 
@@ -539,11 +544,11 @@ int launch_attention_fp32(cudaStream_t stream, const AttnFp32Params& p) {
     }
   }
   switch (p.d) {
-    case 16: return two ? launch<16, 2, 4>(stream, p) : launch<16, 1, 8>(stream, p);
-    case 24: return two ? launch<24, 2, 4>(stream, p) : launch<24, 1, 8>(stream, p);
-    case 32: return two ? launch<32, 2, 4>(stream, p) : launch<32, 1, 8>(stream, p);
-    case 48: return launch<48, 1, 8>(stream, p);
-    case 64: return launch<64, 1, 8>(stream, p);
+    case 16: return two ? launch<16, 2, 1, 4>(stream, p) : launch<16, 1, 2, 8>(stream, p);
+    case 24: return two ? launch<24, 2, 1, 4>(stream, p) : launch<24, 1, 2, 8>(stream, p);
+    case 32: return two ? launch<32, 2, 1, 4>(stream, p) : launch<32, 1, 2, 8>(stream, p);
+    case 48: return launch<48, 1, 2, 8>(stream, p);
+    case 64: return launch<64, 1, 2, 8>(stream, p);
     default:
       set_error("attention_fp32: head dim %d not supported (16, 24, 32, 48, 64)", p.d);
       return KFB_ERR_UNSUPPORTED;
