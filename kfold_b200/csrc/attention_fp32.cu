@@ -25,27 +25,8 @@ __device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ptx::smem_u32(smem)), "l"(gmem) : "memory");
 }
 
-// Two float32 operations in one issue slot: the same IEEE results, pair by pair.
-__device__ __forceinline__ uint64_t fma2(uint64_t a, uint64_t b, uint64_t c) {
-  uint64_t d;
-  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(d) : "l"(a), "l"(b), "l"(c));
-  return d;
-}
-__device__ __forceinline__ uint64_t mul2(uint64_t a, uint64_t b) {
-  uint64_t d;
-  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(d) : "l"(a), "l"(b));
-  return d;
-}
-__device__ __forceinline__ uint64_t pair_of(float lo, float hi) {
-  uint64_t d;
-  asm("mov.b64 %0, {%1, %2};" : "=l"(d) : "f"(lo), "f"(hi));
-  return d;
-}
-__device__ __forceinline__ float2 halves_of(uint64_t v) {
-  float2 f;
-  asm("mov.b64 {%0, %1}, %2;" : "=f"(f.x), "=f"(f.y) : "l"(v));
-  return f;
-}
+using ptx::fma2;
+using ptx::mul2;
 
 template <int D, int QPT, int LPR, int kWarps>
 struct F32Cfg {
@@ -157,7 +138,7 @@ __global__ void __launch_bounds__(kWarps * 32, LPR == 2 ? 2 : 1) attention_fp32_
 #pragma unroll
       for (int kk = 0; kk < kKeys; ++kk) {
         // same order of additions as the reference: (q k + mask) + bias
-        const float2 f = halves_of(s2[i][kk]);
+        const float2 f = ptx::unpack2(s2[i][kk]);
         float qk = f.x + f.y;
         if constexpr (LPR == 2) qk += __shfl_xor_sync(0xffffffffu, qk, kL);
         s[i][kk] = (qk + __shfl_sync(0xffffffffu, mask_v, kk)) + s_bias[(i * kL + lrow) * (kKeys + 1) + kk];
@@ -165,7 +146,7 @@ __global__ void __launch_bounds__(kWarps * 32, LPR == 2 ? 2 : 1) attention_fp32_
       }
       const float m_new = fmaxf(m_run[i], mx);
       const float alpha = expf(m_run[i] - m_new);
-      const uint64_t a2 = pair_of(alpha, alpha);
+      const uint64_t a2 = ptx::pack2(alpha, alpha);
       l_run[i] *= alpha;
 #pragma unroll
       for (int d = 0; d < DL / 2; ++d) acc2[i][d] = mul2(acc2[i][d], a2);
@@ -180,7 +161,7 @@ __global__ void __launch_bounds__(kWarps * 32, LPR == 2 ? 2 : 1) attention_fp32_
     for (int kk = 0; kk < kKeys; ++kk) {
       uint64_t p2[QPT];
 #pragma unroll
-      for (int i = 0; i < QPT; ++i) p2[i] = pair_of(s[i][kk], s[i][kk]);
+      for (int i = 0; i < QPT; ++i) p2[i] = ptx::pack2(s[i][kk], s[i][kk]);
 #pragma unroll
       for (int d = 0; d < DL / 4; ++d) {
         const ulonglong2 f = sv[kk * (kPitch / 4) + d];
@@ -199,7 +180,7 @@ __global__ void __launch_bounds__(kWarps * 32, LPR == 2 ? 2 : 1) attention_fp32_
   for (int i = 0; i < QPT; ++i)
 #pragma unroll
     for (int d = 0; d < DL / 2; ++d) {
-      const float2 f = halves_of(acc2[i][d]);
+      const float2 f = ptx::unpack2(acc2[i][d]);
       acc[i][2 * d] = f.x;
       acc[i][2 * d + 1] = f.y;
     }
@@ -398,7 +379,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attention_fp32_rows_kernel(cons
         m_new[i] = m_run[i];
 #pragma unroll
         for (int kk = 0; kk < kKeys; ++kk) {
-          const float2 f = halves_of(s2[i][kk]);
+          const float2 f = ptx::unpack2(s2[i][kk]);
           // same order of additions as the reference: (q k + mask) + bias
           s[i][kk] = ((f.x + f.y) + mask[kk]) + bv[kk];
           m_new[i] = fmaxf(m_new[i], s[i][kk]);
@@ -408,7 +389,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attention_fp32_rows_kernel(cons
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const float alpha = expf(m_run[i] - m_new[i]);
-          const uint64_t a2 = pair_of(alpha, alpha);
+          const uint64_t a2 = ptx::pack2(alpha, alpha);
           l_run[i] *= alpha;
 #pragma unroll
           for (int d = 0; d < D / 2; ++d) acc[i][d] = mul2(acc[i][d], a2);
@@ -424,7 +405,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attention_fp32_rows_kernel(cons
         }
 #pragma unroll
       for (int kk = 0; kk < kKeys; ++kk) {
-        const uint64_t p0 = pair_of(s[0][kk], s[0][kk]), p1 = pair_of(s[1][kk], s[1][kk]);
+        const uint64_t p0 = ptx::pack2(s[0][kk], s[0][kk]), p1 = ptx::pack2(s[1][kk], s[1][kk]);
 #pragma unroll
         for (int d = 0; d < D / 4; ++d) {
           const ulonglong2 f = sv[kk * (D / 4) + d];
@@ -450,7 +431,7 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attention_fp32_rows_kernel(cons
       float o[8];
 #pragma unroll
       for (int d = 0; d < 4; ++d) {
-        const float2 f = halves_of(acc[i][d0 / 2 + d]);
+        const float2 f = ptx::unpack2(acc[i][d0 / 2 + d]);
         o[2 * d] = f.x * inv_l;
         o[2 * d + 1] = f.y * inv_l;
       }

@@ -153,6 +153,12 @@ __device__ __forceinline__ float tanh_fast(float x) {
 }
 __device__ __forceinline__ float glu_half(float v_half, float g_half) { return fmaf(v_half, tanh_fast(g_half), v_half); }
 
+// ... of two neighbouring channels
+__device__ __forceinline__ uint64_t glu_half2(uint32_t v0, uint32_t v1, uint32_t g0, uint32_t g1) {
+  const uint64_t v = ptx::pack2(v0, v1);
+  return ptx::fma2(v, ptx::pack2(tanh_fast(__uint_as_float(g0)), tanh_fast(__uint_as_float(g1))), v);
+}
+
 // sigmoid(x) = 0.5 tanh(x / 2) + 0.5: one MUFU op instead of an exp2 and a reciprocal
 __device__ __forceinline__ float sigmoidf_fast(float x) {
   float t;
@@ -163,6 +169,11 @@ __device__ __forceinline__ float sigmoidf_fast(float x) {
 __device__ __forceinline__ uint32_t pack_bf16x2(float lo, float hi) {
   __nv_bfloat162 v = __floats2bfloat162_rn(lo, hi);
   return *reinterpret_cast<uint32_t*>(&v);
+}
+
+__device__ __forceinline__ uint32_t pack_bf16x2(uint64_t pair) {
+  const float2 f = ptx::unpack2(pair);
+  return pack_bf16x2(f.x, f.y);
 }
 
 __device__ __forceinline__ float sigmoidf_exact(float x) { return 1.0f / (1.0f + __expf(-x)); }

@@ -289,7 +289,7 @@ pair_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
     // ---------------------------------------------------------------- rows: normalised in place
     const int part = warp - kRowWarp;
     grid_dependency_wait();
-    float lw[8], lb[8];
+    uint64_t lw[4], lb[4];
     rows_affine<C>(p.ln_w, p.ln_b, lane, lw, lb);
     int ab = 0;
     uint32_t a_par = 0;
@@ -377,8 +377,7 @@ pair_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
 #pragma unroll
             for (int j = 0; j < 4; ++j) {
               const float m = keep[(i & 1) * 2 + (j & 1)];
-              w[j] = pack_bf16x2(glu_half(__uint_as_float(v[2 * j]), __uint_as_float(g[2 * j])) * m,
-                                 glu_half(__uint_as_float(v[2 * j + 1]), __uint_as_float(g[2 * j + 1])) * m);
+              w[j] = pack_bf16x2(ptx::mul2(glu_half2(v[2 * j], v[2 * j + 1], g[2 * j], g[2 * j + 1]), ptx::pack2(m, m)));
             }
             put(i, w);
           };

@@ -3,34 +3,36 @@
 #include <cuda_bf16.h>
 
 #include "gemm.cuh"   // pack_bf16x2
+#include "ptx.cuh"
 
 namespace kfb {
 
 static constexpr int kRowTile = 128;              // rows of a CTA's tile
 static constexpr int kRowBox = kRowTile * 128;    // [128 rows][64 bf16], 128-byte swizzle: the tile is C / 64 of them
 
-// A lane's eight channels' scale and offset (1 and 0 where there are none).
+// A lane's eight channels' scale and offset in pairs (1 and 0 where there are none).
 template <int C>
-__device__ __forceinline__ void rows_affine(const float* ln_w, const float* ln_b, int lane, float (&lw)[8], float (&lb)[8]) {
+__device__ __forceinline__ void rows_affine(const float* ln_w, const float* ln_b, int lane, uint64_t (&lw)[4], uint64_t (&lb)[4]) {
 #pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int ch = C == 128 ? (lane & 15) * 8 + i : (lane + 32 * (i >> 1)) * 2 + (i & 1);
-    lw[i] = ln_w != nullptr ? ln_w[ch] : 1.0f;
-    lb[i] = ln_b != nullptr ? ln_b[ch] : 0.0f;
+  for (int i = 0; i < 4; ++i) {
+    const int ch = C == 128 ? (lane & 15) * 8 + 2 * i : (lane + 32 * i) * 2;
+    lw[i] = ln_w != nullptr ? ptx::pack2(ln_w[ch], ln_w[ch + 1]) : ptx::pack2(1.0f, 1.0f);
+    lb[i] = ln_b != nullptr ? ptx::pack2(ln_b[ch], ln_b[ch + 1]) : ptx::pack2(0.0f, 0.0f);
   }
 }
 
 // Rows first .. first + rows - 1 (a multiple of eight) in place, by one warp.  Lanes, expressions and their order are those of layernorm_c128_bf16_kernel and
 // layernorm_c256_bf16_kernel: the same bits (four blocks of bf16 rounding turn a last bit into up to 1 % of the confidence head's result).
 template <int C>
-__device__ __forceinline__ void rows_layernorm(uint8_t* a, int first, int rows, int lane, const float (&lw)[8], const float (&lb)[8], float eps) {
-  constexpr int kPer = C == 128 ? 8 : 4;       // channels, or channel pairs, of a lane
+__device__ __forceinline__ void rows_layernorm(uint8_t* a, int first, int rows, int lane, const uint64_t (&lw)[4], const uint64_t (&lb)[4],
+                                               float eps) {
   if constexpr (C == 128) {
     const int sub = lane & 15, half = lane >> 4;
     constexpr int kSteps = 4;        // of two rows each in flight
 #pragma unroll 1
     for (int base = first; base < first + rows; base += 2 * kSteps) {
-      float v[kSteps][8], sum[kSteps], sq[kSteps];
+      uint64_t v[kSteps][4];
+      float sum[kSteps], sq[kSteps];
       uint4* cell[kSteps];
 #pragma unroll
       for (int s = 0; s < kSteps; ++s) {
@@ -41,9 +43,8 @@ __device__ __forceinline__ void rows_layernorm(uint8_t* a, int first, int rows, 
         sum[s] = 0.f;
 #pragma unroll
         for (int i = 0; i < 4; ++i) {
-          v[s][2 * i] = __uint_as_float(wv[i] << 16);
-          v[s][2 * i + 1] = __uint_as_float(wv[i] & 0xffff0000u);
-          sum[s] += v[s][2 * i] + v[s][2 * i + 1];
+          v[s][i] = ptx::pack2(wv[i] << 16, wv[i] & 0xffff0000u);
+          sum[s] += __uint_as_float(wv[i] << 16) + __uint_as_float(wv[i] & 0xffff0000u);
         }
       }
 #pragma unroll
@@ -55,9 +56,11 @@ __device__ __forceinline__ void rows_layernorm(uint8_t* a, int first, int rows, 
         const float mean = sum[s] * (1.0f / C);
         sq[s] = 0.f;
 #pragma unroll
-        for (int i = 0; i < 8; ++i) {
-          v[s][i] -= mean;
-          sq[s] = fmaf(v[s][i], v[s][i], sq[s]);
+        for (int i = 0; i < 4; ++i) {
+          v[s][i] = ptx::add2(v[s][i], ptx::pack2(-mean, -mean));
+          const float2 d = ptx::unpack2(v[s][i]);
+          sq[s] = fmaf(d.x, d.x, sq[s]);
+          sq[s] = fmaf(d.y, d.y, sq[s]);
         }
       }
 #pragma unroll
@@ -69,8 +72,10 @@ __device__ __forceinline__ void rows_layernorm(uint8_t* a, int first, int rows, 
         const float rstd = rsqrtf(sq[s] * (1.0f / C) + eps);
         uint32_t ov[4];
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
-          ov[i] = pack_bf16x2(fmaf(v[s][2 * i] * rstd, lw[2 * i], lb[2 * i]), fmaf(v[s][2 * i + 1] * rstd, lw[2 * i + 1], lb[2 * i + 1]));
+        for (int i = 0; i < 4; ++i) {
+          const float2 y = ptx::unpack2(ptx::fma2(ptx::mul2(v[s][i], ptx::pack2(rstd, rstd)), lw[i], lb[i]));
+          ov[i] = pack_bf16x2(y.x, y.y);
+        }
         *cell[s] = make_uint4(ov[0], ov[1], ov[2], ov[3]);
       }
     }
@@ -78,7 +83,7 @@ __device__ __forceinline__ void rows_layernorm(uint8_t* a, int first, int rows, 
     constexpr int kStep = 4;         // rows in flight
 #pragma unroll 1
     for (int base = first; base < first + rows; base += kStep) {
-      float2 v[kStep][kPer];
+      uint64_t v[kStep][4];
       float s[kStep], q[kStep];
       uint32_t* cell[kStep];
 #pragma unroll
@@ -86,10 +91,10 @@ __device__ __forceinline__ void rows_layernorm(uint8_t* a, int first, int rows, 
         cell[r] = reinterpret_cast<uint32_t*>(a + (base + r) * 128 + (((lane >> 2) ^ ((base + r) & 7)) << 4) + (lane & 3) * 4);
         s[r] = 0.f;
 #pragma unroll
-        for (int g = 0; g < kPer; ++g) {
+        for (int g = 0; g < 4; ++g) {
           const uint32_t u = cell[r][g * (kRowBox / 4)];
-          v[r][g] = make_float2(__uint_as_float(u << 16), __uint_as_float(u & 0xffff0000u));
-          s[r] += v[r][g].x + v[r][g].y;
+          v[r][g] = ptx::pack2(u << 16, u & 0xffff0000u);
+          s[r] += __uint_as_float(u << 16) + __uint_as_float(u & 0xffff0000u);
         }
       }
 #pragma unroll
@@ -101,10 +106,10 @@ __device__ __forceinline__ void rows_layernorm(uint8_t* a, int first, int rows, 
         const float mean = s[r] / static_cast<float>(C);
         q[r] = 0.f;
 #pragma unroll
-        for (int g = 0; g < kPer; ++g) {
-          v[r][g].x -= mean;
-          v[r][g].y -= mean;
-          q[r] += v[r][g].x * v[r][g].x + v[r][g].y * v[r][g].y;
+        for (int g = 0; g < 4; ++g) {
+          v[r][g] = ptx::add2(v[r][g], ptx::pack2(-mean, -mean));
+          const float2 d = ptx::unpack2(v[r][g]);
+          q[r] += d.x * d.x + d.y * d.y;
         }
       }
 #pragma unroll
@@ -115,8 +120,10 @@ __device__ __forceinline__ void rows_layernorm(uint8_t* a, int first, int rows, 
       for (int r = 0; r < kStep; ++r) {
         const float rstd = rsqrtf(q[r] / static_cast<float>(C) + eps);
 #pragma unroll
-        for (int g = 0; g < kPer; ++g)
-          cell[r][g * (kRowBox / 4)] = pack_bf16x2(fmaf(v[r][g].x * rstd, lw[2 * g], lb[2 * g]), fmaf(v[r][g].y * rstd, lw[2 * g + 1], lb[2 * g + 1]));
+        for (int g = 0; g < 4; ++g) {
+          const float2 y = ptx::unpack2(ptx::fma2(ptx::mul2(v[r][g], ptx::pack2(rstd, rstd)), lw[g], lb[g]));
+          cell[r][g * (kRowBox / 4)] = pack_bf16x2(y.x, y.y);
+        }
       }
     }
   }

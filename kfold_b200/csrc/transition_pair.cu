@@ -282,8 +282,7 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
         uint32_t w[8];
 #pragma unroll
         for (int j = 0; j < 16; j += 2) {
-          const float a0 = __uint_as_float(v[j]), a1 = __uint_as_float(v[j + 1]);
-          w[j >> 1] = pack_bf16x2(glu_half(a0, a0) * __uint_as_float(g[j]), glu_half(a1, a1) * __uint_as_float(g[j + 1]));
+          w[j >> 1] = pack_bf16x2(ptx::mul2(glu_half2(v[j], v[j + 1], v[j], v[j + 1]), ptx::pack2(g[j], g[j + 1])));
         }
         ptx::tmem_st_32x32b_x8(t + c / 2, w);
       };
@@ -313,7 +312,7 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     const int col0 = part / 4 * kHalf;
     const uint32_t t_row = tmem_base + (static_cast<uint32_t>(quad * 32) << 16) + col0;
     grid_dependency_wait();
-    float lw[8], lb[8];
+    uint64_t lw[4], lb[4];
     rows_affine<C>(p.ln_w, p.ln_b, lane, lw, lb);
     bool ok = true;
     int ab = 0, ob = 0;                          // buffers of the next tile and of the last, and their phases
