@@ -62,6 +62,10 @@ int launch_layernorm_cm(cudaStream_t stream, const void* t, __nv_bfloat16* y, co
 // KFB_FP32_PRECISE) bf16 triple-split rows of 6c.
 int launch_adaln(cudaStream_t stream, const void* a, void* y, const void* gv, long long rows, int c, int samples,
                  int l, float eps, int in_dtype, int out_dtype, long long gv_ld = 0, int gv_static = 0);
+// ... of bf16 or fp32 rows with two sets of gates and shifts (bf16, rows gv_ld apart in either) into two bf16 tensors; one launch where the
+// kernel takes the shape.
+int launch_adaln_two(cudaStream_t stream, const void* a, void* y, void* y2, const void* gv, const void* gv2, long long rows, int c, int samples, int l,
+                     float eps, int in_dtype, long long gv_ld, int gv_static);
 
 // LayerNorm folded into the following GEMM (see layernorm.cu): per-position (mean, rstd) of a channel-major tensor.
 int launch_cm_stats(cudaStream_t stream, const __nv_bfloat16* t, float2* stats, long long npos, int c, long long chan_stride,

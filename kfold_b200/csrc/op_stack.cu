@@ -212,8 +212,7 @@ KFB_API int kfb_atom_stack_fwd(const kfb_atom_block* blocks, int n_blocks, const
   for (int i = 0; i < n_blocks; ++i) {
     const kfb_atom_block& w = blocks[i];
     const long long g0 = 6ll * c * i;
-    KFB_TRY(launch_adaln(stream, cur, xq, column(t.gs, g0, 0), rows, c, samples, l, eps, act_dtype, KFB_BF16, t.gs_cols, 1));
-    KFB_TRY(launch_adaln(stream, cur, xk, column(t.gs, g0 + 2ll * c, 0), rows, c, samples, l, eps, act_dtype, KFB_BF16, t.gs_cols, 1));
+    KFB_TRY(launch_adaln_two(stream, cur, xq, xk, column(t.gs, g0, 0), column(t.gs, g0 + 2ll * c, 0), rows, c, samples, l, eps, act_dtype, t.gs_cols, 1));
     // the output gate is shared by the samples: query row r reads gate row r % (l) of its group
     for (int g = 0; g < groups; ++g) {
       const size_t row0 = static_cast<size_t>(g) * samples * l, e = act_dtype == KFB_FP32 ? 4 : 2;
