@@ -309,22 +309,24 @@ class _ConditioningBank:
         fix = packing.split3_weights if precise else (lambda t: t.to(torch.bfloat16).contiguous())
         return fix(torch.cat(w1)), torch.cat(b1).contiguous(), fix(torch.cat(w2)), torch.cat(b2).contiguous()
 
-    def _pack(self, adalns, gates, device):
+    def _pack(self, adalns, gates, device, precise: bool = False):
         params = [p for m in adalns for p in (m.layernorm_s.weight, m.linear_g.weight, m.linear_g.bias, m.linear_bias.weight)]
         params += [p for g in gates for p in (g.weight, g.bias)]
-        key = (device,) + tuple(v for p in params for v in (p.data_ptr(), None if torch.is_inference(p) else p._version))
+        key = (device, precise) + tuple(v for p in params for v in (p.data_ptr(), None if torch.is_inference(p) else p._version))
         if self._key != key:
-            self._packed = self.pack(adalns, gates, device)
+            self._packed = self.pack(adalns, gates, device, precise)
             self._key = key
         return handed_out(self._packed)
 
-    def tables(self, s: torch.Tensor, adalns, gates):
-        """-> (gate_shift, out_gate): lists of views, one per AdaLN (..., L, 2 c_a) and one per gate (..., L, c_a)."""
+    def tables(self, s: torch.Tensor, adalns, gates, precise: bool = False):
+        """-> (gate_shift, out_gate): lists of views, one per AdaLN (..., L, 2 c_a) and one per gate (..., L, c_a); bf16, or
+        float32 when ``precise``."""
         eps = adalns[0].layernorm_s.eps
-        w1, b1, w2, b2 = self._pack(adalns, gates, s.device)
-        sn = F.layer_norm(s, None, None, eps, out_dtype=torch.bfloat16)
-        t1 = F.linear(sn, w1, b1)
-        t2 = F.linear(s, w2, b2)
+        w1, b1, w2, b2 = self._pack(adalns, gates, s.device, precise)
+        s = s.float() if precise else s
+        sn = F.layer_norm(s, None, None, eps, out_dtype=torch.float32 if precise else torch.bfloat16)
+        linear = F.linear_fp32 if precise else F.linear
+        t1, t2 = linear(sn, w1, b1), linear(s, w2, b2)
         gs, off = [], 0
         for m in adalns:
             gs.append(t1[..., off: off + 2 * m.channel_a])
@@ -471,11 +473,11 @@ class ConditionedTransitionBlock(_PackedMixin, nn.Module):
         pk = self._packed_transition(a.device, precise)
         with torch.autocast(a.device.type, enabled=False):
             s, share = _shared_conditioning(a, s)
-            if precise:
+            if cond is not None:
+                an, gate = F.adaln(a.float() if precise else a, cond[0], share), cond[1]
+            elif precise:
                 an = F.adaln(a.float(), self.adaln.gate_shift(s, True), share)
                 gate = F.linear_fp32(s.float(), pk["w_g"], pk["b_g"])
-            elif cond is not None:
-                an, gate = F.adaln(a, cond[0], share), cond[1]
             else:
                 an = F.adaln(a, self.adaln.gate_shift(s), share)
                 gate = F.linear(s, pk["w_g"], pk["b_g"])
@@ -798,9 +800,9 @@ class CrossAttentionPairBias(_PackedMixin, nn.Module):
         if self.use_single_conditioning:
             assert s is not None
             s, share = _shared_conditioning(a, s)
-            if cond is not None and not precise:
-                return F.adaln(a, cond[0], share), F.adaln(a, cond[1], share), cond[2]
             af = a.float() if precise else a
+            if cond is not None:
+                return F.adaln(af, cond[0], share), F.adaln(af, cond[1], share), cond[2]
             xq = F.adaln(af, self.adaln_a_q.gate_shift(s, precise), share)
             xk = F.adaln(af, self.adaln_a_k.gate_shift(s, precise), share)
             w_ada, b_ada = self._ada_out(a.device, precise)
@@ -989,10 +991,12 @@ class LocalTransformerStack(NativeCall, nn.Module):
                 bias_all = bias_all.reshape(len(self.blocks), h, -1, WINDOW_Q, WINDOW_K)
                 batch = mask_k.shape[0]
             conds = [None] * len(self.blocks)
-            if (not precise and all(b.attention.use_single_conditioning for b in self.blocks)
-                    and len({m.layernorm_s.eps for m in self._adalns()}) == 1):
-                # the conditioning projections of all blocks: one LayerNorm of s and two GEMMs
-                gs, og = self._bank.tables(s, self._adalns(), self._gates())
+            if (all(b.attention.use_single_conditioning for b in self.blocks)
+                    and len({m.layernorm_s.eps for m in self._adalns()}) == 1
+                    and not (precise and any(type(m) is not AdaLN for m in self._adalns()))):
+                # the conditioning projections of all blocks: one LayerNorm of s and two GEMMs (float32, 2 400 atoms, two stacks of
+                # three blocks: 78 launches of a step become 12)
+                gs, og = self._bank.tables(s, self._adalns(), self._gates(), precise)
                 conds = [((gs[3 * i], gs[3 * i + 1], og[2 * i]), (gs[3 * i + 2], og[2 * i + 1])) for i in range(len(self.blocks))]
             for i, blk in enumerate(self.blocks):
                 att = blk.attention
