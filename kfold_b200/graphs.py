@@ -1,7 +1,7 @@
 """CUDA-graph replay of a fixed-shape call.
 
 The sampler of K-Fold calls its token transformer 200 times per prediction with tensors of the same shape
-(src/kfold/model/modules/ecsi.py:468-560).  One step of the network is about 246 kernel launches of a few microseconds
+(src/kfold/model/modules/ecsi.py:468-560).  One step of the network is about 240 kernel launches of a few microseconds
 each, so for small complexes it is bound by the host that issues them; captured once into a CUDA graph and replayed it is not
 (bench.py --sampler-step prints both).  The library is capturable as it is: it allocates nothing, never synchronises, and
 every temporary of the Python layer comes from torch's caching allocator, which gives a capture its own pool.
