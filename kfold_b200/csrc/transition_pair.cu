@@ -23,8 +23,8 @@
 // The arithmetic and its order are those of layernorm_c128_bf16_kernel / layernorm_c256_bf16_kernel and of the GEMMs this replaces: the
 // same bits.
 //
-// Measured (events): 589 824 rows of 128 channels 376 us as three launches, 255 with one issuing thread and four row warps, 187 now (62 %
-// more than the products alone: the chain S - h - O through three S buffers); of 256 channels 955, 637, 633 (1 466 TFLOP/s, at the power
+// Measured (events): 589 824 rows of 128 channels 376 us as three launches, 255 with one issuing thread and four row warps, 187 now (its
+// products: 141 at the measured burst rate; the chain S - h - O through three S buffers is the rest); of 256 channels 955, 637, 633 (1 466 TFLOP/s, at the power
 // limit); 63 001 rows: 53, 42, 34 and 112, 89, 86.
 #include <cuda_bf16.h>
 
