@@ -254,6 +254,9 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
     }
   }
   if (bn != 256) p.pair = 0;
+  // few rows with statistics to take: twice the tiles, half the epilogue (pair block of 64 tokens, two of them: 142.5 -> 138.9 us;
+  // 251 tokens, which have the tiles: as they were)
+  if (p.aux && bn == 128 && a.s_k != 0 && p.row_stats != nullptr && static_cast<long long>(p.num_m_tiles) * cdiv(p.n_cols, 64) <= sm_count()) bn = 64;
   KFB_CHECK_ARG(bn == 32 || bn == 64 || bn == 128 || bn == 256, "unsupported BN %d", bn);
   // LayerNorm statistics of K-outer rows: taken by the kernel itself where it has the warps for it, by a pass before it otherwise.  The
   // statistics hold a stage of the ring a little longer, which costs little where a tile is few stages or comes from L2 (768 x 768 rows
