@@ -13,19 +13,19 @@
 // compete with (a chunk of 128 channels reads 56 KB of operands and is filled with 24 KB in 768 cycles of products; h in shared memory
 // would add 32).
 //   * S has three buffers of 128 columns (C = 128) or two (C = 256), which with O fill the tensor memory.  S and O have a thread each that
-//     issues them.  The tensor core works in the order of issue: a buffer's next S needs no more than that the product with its h has been
-//     issued, not that it is done (which took the chain another 500 cycles a turn).
+//     issues them.  A buffer's next S waits until the product that reads its h is done: tcgen05.mma promises an order only to products of the
+//     same accumulator and shape, which these two have not.
 //   * Two groups of four SwiGLU warps take the chunks in turn.  (All eight on one chunk: the special-function unit, 512 cycles a chunk, then
-//     waits out every chunk's latencies: 191 -> 197 us.)
+//     waits out every chunk's latencies: 6 us more.)
 //   * Eight more warps normalise the next tile's rows in place in shared memory while this one is multiplied, and turn the finished tile
 //     around: the residual comes back (from L2) into the tile's own buffer, which the products have left, is added, and the buffer leaves
 //     as it is.  A thread of its own sees to what a buffer receives and sends.
 // The arithmetic and its order are those of layernorm_c128_bf16_kernel / layernorm_c256_bf16_kernel and of the GEMMs this replaces: the
 // same bits.
 //
-// Measured (events): 589 824 rows of 128 channels 376 us as three launches, 255 with one issuing thread and four row warps, 187 now (its
-// products: 141 at the measured burst rate; the chain S - h - O through three S buffers is the rest); of 256 channels 955, 637, 633 (1 466 TFLOP/s, at the power
-// limit); 63 001 rows: 53, 42, 34 and 112, 89, 86.
+// Measured (graph replays, three launches -> this): 589 824 rows of 128 channels 380 -> 191 us (its products: 141 at the measured burst rate; the
+// chain S - h - O through three S buffers is the rest), of 256 channels 976 -> 800 (at the power limit); 63 001 rows: 51 -> 28 and 111 -> 84.
+// With the next S behind the issue of the product before it they were 187, 749, 28 and 79.
 #include <cuda_bf16.h>
 
 #include <mutex>
@@ -77,9 +77,8 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   uint64_t* full = bars;                     // [slots], in the leader: both CTAs' copies
   uint64_t* empty = full + K::kSlots;        // [slots]
   uint64_t* v_full = empty + K::kSlots;      // [kS], in the leader
-  uint64_t* v_free = v_full + K::kS;         // [kS] the product has read it
-  uint64_t* o_sent = v_free + K::kS;         // [kS], in the leader: the product with the h of S buffer i % kS has been issued
-  uint64_t* s_full = o_sent + K::kS;         // [kS]
+  uint64_t* v_free = v_full + K::kS;         // [kS] the product has read it, and the h of the S buffer of the same number
+  uint64_t* s_full = v_free + K::kS;         // [kS]
   uint64_t* h_ready = s_full + K::kS;        // [kS], in the leader: 4 warps of each CTA
   uint64_t* rows_in = h_ready + K::kS;       // [kA] a tile's rows have arrived
   uint64_t* resid_in = rows_in + K::kA;      // [kA] a tile's residual has, in their place
@@ -90,7 +89,7 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   uint64_t* o_full = out_done + K::kA;
   uint64_t* o_empty = o_full + 1;            // in the leader: the row warps of both CTAs
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_empty + 1);
-  static_assert((2 * 6 + 5 * 3 + 6 * 3 + 2) * 8 + 4 <= 512, "barriers");
+  static_assert((2 * 6 + 4 * 3 + 6 * 3 + 2) * 8 + 4 <= 512, "barriers");
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int rank = static_cast<int>(ptx::cluster_ctarank());
@@ -110,7 +109,6 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
     for (int i = 0; i < K::kS; ++i) {
       ptx::mbar_init(&v_full[i], 1);
       ptx::mbar_init(&v_free[i], 1);
-      ptx::mbar_init(&o_sent[i], 1);
       ptx::mbar_init(&s_full[i], 1);
       ptx::mbar_init(&h_ready[i], 8);
     }
@@ -203,13 +201,13 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
       const uint64_t a_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_a));
       const uint64_t w_desc = ptx::make_kmajor_desc<128>(ptx::smem_u32(s_w));
       int slot = 0, s1 = 0, ab = 0;
-      uint32_t par = 0, s_par = 1, a_par = 0;      // s_par: phase of o_sent that the buffer's next S stands behind (the first kS: none)
+      uint32_t par = 0, s_par = 1, a_par = 0;      // s_par: phase of v_free that the buffer's next S waits for (the first kS: none)
       bool ok = true;
       for (int it = 0; ok && it < my_tiles; ++it) {
         ok = ptx::mbar_wait(&a_norm[ab], a_par, 404) && ptx::mbar_wait_cluster(&a_peer[ab], a_par, 413);
         const uint64_t ad = a_desc + ab * (K::kABytes >> 4);
         for (int c = 0; ok && c < p.chunks; ++c) {
-          ok = ptx::mbar_wait(&o_sent[s1], s_par, 417);
+          ok = ptx::mbar_wait(&v_free[s1], s_par, 417);
           if (!ok) break;
           ptx::tc_fence_after_sync();
           const uint32_t d = tmem_s + s1 * 128;
@@ -254,8 +252,6 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
             ptx::mma_f16_ts_pair(tmem_base, tmem_s + s2 * 128 + k * 8, v_desc + static_cast<uint64_t>(s2 * (K::kOutUnit >> 4)) + k * 2, idesc,
                                  (c > 0 || k > 0) ? 1u : 0u);
           ptx::tc_commit_pair(&v_free[s2]);
-          ptx::tc_fence_before_sync();
-          ptx::mbar_arrive(&o_sent[s2]);
           if (++s2 == K::kS) { s2 = 0; par ^= 1u; }
         }
         if (ok) ptx::tc_commit_pair(o_full);
