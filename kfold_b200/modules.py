@@ -897,6 +897,8 @@ class LocalTransformerStack(NativeCall, nn.Module):
         self._bias_w_key = None
         self._bank = _ConditioningBank()
 
+    table_limit = 1 << 30        # bytes of the float32 conditioning tables of all blocks
+
     # the window biases of the present complex, known by its pair tensor's address
     _bias_all = _bias_all_key = _bias_all_src = None
     _unshared = ("_plan", "_bias_all", "_bias_all_key", "_bias_all_src")
@@ -991,11 +993,12 @@ class LocalTransformerStack(NativeCall, nn.Module):
                 bias_all = bias_all.reshape(len(self.blocks), h, -1, WINDOW_Q, WINDOW_K)
                 batch = mask_k.shape[0]
             conds = [None] * len(self.blocks)
+            # the conditioning projections of all blocks: one LayerNorm of s and two GEMMs (float32, 2 400 atoms, two stacks of three blocks: 78
+            # launches of a step become 12); block by block where their float32 tables, 12 KB an atom, would be gigabytes
+            table_bytes = 4 * 8 * c * len(self.blocks) * (s.numel() // s.shape[-1])
             if (all(b.attention.use_single_conditioning for b in self.blocks)
                     and len({m.layernorm_s.eps for m in self._adalns()}) == 1
-                    and not (precise and any(type(m) is not AdaLN for m in self._adalns()))):
-                # the conditioning projections of all blocks: one LayerNorm of s and two GEMMs (float32, 2 400 atoms, two stacks of
-                # three blocks: 78 launches of a step become 12)
+                    and not (precise and (table_bytes > self.table_limit or any(type(m) is not AdaLN for m in self._adalns())))):
                 gs, og = self._bank.tables(s, self._adalns(), self._gates(), precise)
                 conds = [((gs[3 * i], gs[3 * i + 1], og[2 * i]), (gs[3 * i + 2], og[2 * i + 1])) for i in range(len(self.blocks))]
             for i, blk in enumerate(self.blocks):
