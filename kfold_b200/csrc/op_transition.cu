@@ -102,7 +102,10 @@ int kfb::transition_run(cudaStream_t stream, const void* x, const float* ln_w, c
   const size_t need = carve(w, workspace, rows, c, hidden);
   KFB_CHECK_ARG(workspace_bytes >= need, "transition: workspace %zu < %zu bytes", workspace_bytes, need);
   KFB_CHECK_ARG((reinterpret_cast<uintptr_t>(workspace) & 255) == 0, "transition: workspace must be 256-byte aligned");
-  if (transition_pair_ok(x, w_swiglu_packed, w_out, out, resid, rows, c, hidden, dtype))
+  // In a block the faster form.  A call of its own is one launch wherever the kernel takes the operands: with few rows its time is the host's,
+  // which needs some 3 us for each.
+  if (transition_pair_ok(x, w_swiglu_packed, w_out, out, resid, rows, c, hidden, dtype) &&
+      (!w_static || transition_pair_is_faster(rows, c, hidden)))
     return launch_transition_pair(stream, x, ln_w, ln_b, w_swiglu_packed, w_out, out, resid, rows, c, hidden, eps, w_static);
   KFB_TRY(launch_layernorm(stream, x, w.xn, ln_w, ln_b, rows, c, c, c, eps, dtype, KFB_BF16));
   {

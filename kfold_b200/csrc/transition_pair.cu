@@ -462,19 +462,6 @@ int launch(cudaStream_t stream, const void* x, const float* ln_w, const float* l
                                  tr, to, p);
 }
 
-// Few rows: a pair walks all hidden channels of its 256 rows, 1.0 us a chunk at 256 channels and 0.52 at 128, however few tiles there are,
-// where the three launches (the same bits) spread the hidden channels over the chip.  us for either, fitted to graph replays of 1 to 40 000
-// rows with 128 to 2 048 hidden channels.  Three launches / this, 256 channels and 1 024 hidden: 4 096 rows 19.9 / 25.4, 6 400 23.8 / 25.6,
-// 9 216 25.6 / 25.8, 10 500 30.8 / 27.1; 512 hidden: 4 096 16.6 / 17.6, 5 000 17.8 / 17.5; 128 channels and 512 hidden: 256 rows 12.2 / 10.7.
-// (Beyond 64 rows for each multiprocessor the three launches take a second round: a fifth more.)
-bool pair_is_faster(long long rows, int c, int hidden, int held) {
-  const double chunks = hidden / kChunk;
-  const long long tiles = (rows + 2 * kRows - 1) / (2 * kRows), rounds = (tiles + held - 1) / held;
-  const double pair = c == 128 ? 6.9 + 0.52 * chunks * rounds : 9.2 + chunks * rounds;
-  const double three = (c == 128 ? 10.3 + 0.22 * chunks : 11.3 + 0.24 * chunks) + 1e-3 * rows * (0.4 + 0.05 * chunks);
-  return pair <= (rows > 64ll * sm_count() ? 1.2 : 1.0) * three;
-}
-
 }  // namespace
 
 bool transition_pair_ok(const void* x, const void* w_swiglu, const void* w_out, const void* out, const void* resid, long long rows, int c,
@@ -485,7 +472,22 @@ bool transition_pair_ok(const void* x, const void* w_swiglu, const void* w_out, 
   int held = 0;
   const bool known = (c == 128 ? pairs_held<128>(&held) : pairs_held<256>(&held)) == KFB_OK;
   if (!known) cudaGetLastError();
-  return known && held > 0 && pair_is_faster(rows, c, hidden, held);
+  return known && held > 0;
+}
+
+// Few rows: a pair walks all hidden channels of its 256 rows, 1.0 us a chunk at 256 channels and 0.52 at 128, however few tiles there are,
+// where the three launches (the same bits) spread the hidden channels over the chip.  us for either, fitted to graph replays of 1 to 40 000
+// rows with 128 to 2 048 hidden channels.  Three launches / this, 256 channels and 1 024 hidden: 4 096 rows 19.9 / 25.4, 6 400 23.8 / 25.6,
+// 9 216 25.6 / 25.8, 10 500 30.8 / 27.1; 512 hidden: 4 096 16.6 / 17.6, 5 000 17.8 / 17.5; 128 channels and 512 hidden: 256 rows 12.2 / 10.7.
+// (Beyond 64 rows for each multiprocessor the three launches take a second round: a fifth more.)
+bool transition_pair_is_faster(long long rows, int c, int hidden) {
+  int held = 1;
+  if ((c == 128 ? pairs_held<128>(&held) : pairs_held<256>(&held)) != KFB_OK || held < 1) return false;
+  const double chunks = hidden / kChunk;
+  const long long tiles = (rows + 2 * kRows - 1) / (2 * kRows), rounds = (tiles + held - 1) / held;
+  const double pair = c == 128 ? 6.9 + 0.52 * chunks * rounds : 9.2 + chunks * rounds;
+  const double three = (c == 128 ? 10.3 + 0.22 * chunks : 11.3 + 0.24 * chunks) + 1e-3 * rows * (0.4 + 0.05 * chunks);
+  return pair <= (rows > 64ll * sm_count() ? 1.2 : 1.0) * three;
 }
 
 int launch_transition_pair(cudaStream_t stream, const void* x, const float* ln_w, const float* ln_b, const void* w_swiglu, const void* w_out,

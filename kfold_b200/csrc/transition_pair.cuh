@@ -8,6 +8,8 @@ namespace kfb {
 // blocks of 128, a device that holds CTA pairs.
 bool transition_pair_ok(const void* x, const void* w_swiglu, const void* w_out, const void* out, const void* resid, long long rows, int c,
                         int hidden, int dtype);
+// Whether it then takes less of the GPU's time than the three launches.
+bool transition_pair_is_faster(long long rows, int c, int hidden);
 // out may be x, and so may resid.  w_static: the weights were written before the launch before this one.
 int launch_transition_pair(cudaStream_t stream, const void* x, const float* ln_w, const float* ln_b, const void* w_swiglu, const void* w_out,
                            void* out, const void* resid, long long rows, int c, int hidden, float eps, int w_static);

@@ -35,12 +35,9 @@ def _call(x, out, resid, pk):
     return L.launch_count() - before
 
 
-@pytest.mark.parametrize("c,factor,rows,launches", [
-    (128, 4, 1, 1), (128, 4, 127, 1), (128, 4, 128, 1), (128, 4, 129, 1), (128, 1, 256, 1), (128, 1, 57001, 1), (128, 4, 37889, 1),
-    (256, 1, 2303, 1), (256, 1, 2304, 1), (256, 1, 2305, 1), (256, 1, 57001, 1), (256, 2, 18944, 1), (256, 4, 10497, 1),
-    # few rows and many hidden channels, where one pair's walk over them all is slower than three launches
-    (256, 4, 1, 3), (256, 4, 255, 3), (256, 4, 257, 3), (256, 4, 4096, 3), (256, 8, 19200, 3), (128, 8, 64, 3)])
-def test_one_launch(dev, c, factor, rows, launches):
+@pytest.mark.parametrize("c,factor,rows", [(128, 4, 1), (128, 4, 127), (128, 4, 128), (128, 4, 129), (128, 1, 256), (128, 1, 57001), (128, 4, 37889),
+                                           (256, 4, 1), (256, 4, 255), (256, 4, 257), (256, 1, 57001), (256, 2, 18944)])
+def test_one_launch(dev, c, factor, rows):
     from kfold_b200 import packing
     import synth
     w = synth.transition_weights(synth._Rng(c + rows), c, factor)
@@ -52,11 +49,11 @@ def test_one_launch(dev, c, factor, rows, launches):
     for resid in (None, xd, other):
         buf = torch.full((rows * c + 16,), 7.0, device=dev, dtype=torch.bfloat16)
         out = buf[:rows * c].view(rows, c)
-        assert _call(xd, out, resid, pk) == launches
+        assert _call(xd, out, resid, pk) == 1
         _check(*err_stats(out.float().cpu(), ref if resid is None else ref + resid.float().cpu()), f"transition c={c} rows={rows}")
         assert (buf[rows * c:] == 7.0).all()
         off = torch.empty(rows * c + 8, device=dev, dtype=torch.bfloat16)[4:4 + rows * c].view(rows, c)
         assert _call(xd, off, resid, pk) == 3
         assert torch.equal(off, out)
-    assert _call(xd, xd, xd, pk) == launches        # in place
+    assert _call(xd, xd, xd, pk) == 1        # in place
     _check(*err_stats(xd.float().cpu(), ref + x.float()), f"transition in place c={c} rows={rows}")
