@@ -199,14 +199,15 @@ int launch_gemm_bf16(cudaStream_t stream, const GemmOperandA& a, const GemmOpera
   // K shared by a cluster where rows are few (the gate / residual epilogue of 128 float32 columns takes the other kernel 8 000 cycles)
   const bool plain_operands = a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0;
   SplitPlan plan = {0, 0};
-  ResidPlan onto = {0, 0.0};
-  if (force_bn == 0) onto = resid_plan(p, a, b);
   if (force_bn == 0 && static_cast<long long>(p.num_m_tiles) * cdiv(p.n_cols, bn) <= sm_count())
-    plan = split_plan(p, plain_operands,
-                      onto.bn != 0 ? onto.cycles
-                                   : split_cycles(p.precise, bn, cdiv(p.precise ? p.k_extent / 6 : p.k_extent, kBK)) +
-                                         ((p.gate != nullptr || p.resid != nullptr) && !p.precise ? 50.0 : 12.0) * bn);
-  if (plan.bn == 0 && onto.bn != 0) return launch_gemm_resid(stream, a, b, p, onto.bn, tag);
+    plan = split_plan(p, plain_operands, split_cycles(p.precise, bn, cdiv(p.precise ? p.k_extent / 6 : p.k_extent, kBK)) +
+                                             ((p.gate != nullptr || p.resid != nullptr) && !p.precise ? 50.0 : 12.0) * bn);
+  // One wave of pairs onto a residual stream otherwise: the bits of the plain tiles.  (It has no say in whether K is shared, which they and
+  // the sum's order hang on.)
+  if (plan.bn == 0 && force_bn == 0) {
+    const int onto = resid_tile(p, a, b);
+    if (onto != 0) return launch_gemm_resid(stream, a, b, p, onto, tag);
+  }
   if (plan.bn != 0) bn = plan.bn;
   p.pair = plan.bn == 0 && pair_tile(p, bn) && a.s_k == 0 && a.k_inner == 0 && b.col_inner == 0;
   if (p.pair) bn = 256;

@@ -1838,13 +1838,8 @@ inline double split_cycles(bool precise, int bn, int k_blocks) {
   return k_blocks * (copies > turn ? copies : turn);
 }
 
-// GEMMs onto a float32 residual stream, one tile for each CTA pair of one wave (gemm_resid.cu): columns of a tile and modelled cycles, bn = 0
-// where it does not take them.
-struct ResidPlan {
-  int bn;
-  double cycles;
-};
-ResidPlan resid_plan(const GemmParams& p, const GemmOperandA& a, const GemmOperandB& b);
+// GEMMs onto a float32 residual stream, one tile for each CTA pair of one wave (gemm_resid.cu): columns of a tile, 0 where it does not take them.
+int resid_tile(const GemmParams& p, const GemmOperandA& a, const GemmOperandB& b);
 int launch_gemm_resid(cudaStream_t stream, const GemmOperandA& a, const GemmOperandB& b, const GemmParams& p, int bn, const char* tag);
 
 // Debugging aid: launches whose tag equals `tag` store per-tile clock stamps of CTA 0 into `device_buffer`

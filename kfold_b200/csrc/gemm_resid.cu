@@ -10,8 +10,7 @@
 // registers of the epilogue warps while K goes by.  What is left for the end is one multiply-add per value in place, and every warp sends its
 // own 32 x 32 pieces.
 // Between events (4 us of them the events'), K = 2 x width: 5 x 768 rows of 768 24.9 -> 18.8 us, of 1 024 30.9 -> 24.9; 5 x 384 rows 17.2 ->
-// 15.8 and 20.8 -> 17.1; 2 x 301 of 1 024 16.7 -> 14.7; fewer rows, where a cluster shares K (gemm_split.cu) or the times are those of the
-// launch, within 0.3 us.
+// 15.8 and 20.8 -> 17.1; 2 x 301 of 1 024 16.7 -> 14.7.  Where a cluster shares K (gemm_split.cu) it is left out.
 #include <mutex>
 
 #include "common.cuh"
@@ -325,9 +324,13 @@ int launch(cudaStream_t stream, const GemmOperandA& a, const GemmOperandB& b, co
 
 }  // namespace
 
-// One wave only: with more, the persistent kernel's epilogues run under the next tile's products.
-ResidPlan resid_plan(const GemmParams& p, const GemmOperandA& a, const GemmOperandB& b) {
-  ResidPlan best = {0, 0.0};
+// One wave only: with more, the persistent kernel's epilogues run under the next tile's products.  Of one wave it is the faster of the two
+// everywhere (graph replays of SwiGLU and this, K = one and two widths, us, plain tiles / this; the same bits): 128 columns, 64 rows
+// 7.6 / 6.5, 3 008 9.3 / 7.6, 15 040 13.5 / 11.3; 768 columns, 1 row 12.5 / 10.5, 129 12.6 / 11.4, 385 13.5 / 11.7, 1 024 14.3 / 13.4,
+// 3 840 25.1 / 20.7; K = 1 536 385 16.3 / 13.8, 768 17.6 / 15.1; 1 024 columns, 301 15.3 / 13.5, 3 840 30.0 / 27.5.
+int resid_tile(const GemmParams& p, const GemmOperandA& a, const GemmOperandB& b) {
+  int best = 0;
+  double least = 0.0;
   const EpiSeg& sg = p.seg[0];
   auto extent_ok = [](long long stride, int extent, int unit) { return stride % unit == 0 && (stride != 0 || extent == 1); };
   const bool ok =
@@ -348,7 +351,10 @@ ResidPlan resid_plan(const GemmParams& p, const GemmOperandA& a, const GemmOpera
     if (turn < 2.0 * bn) turn = 2.0 * bn;
     if (turn < 400.0) turn = 400.0;
     const double t = blocks * turn + 2500.0 + 6.0 * bn;
-    if ((best.bn == 0 || t < best.cycles) && row_tiles(p) * (p.n_cols / bn) <= held_of(bn)) best = {bn, t};
+    if ((best == 0 || t < least) && row_tiles(p) * (p.n_cols / bn) <= held_of(bn)) {
+      best = bn;
+      least = t;
+    }
   }
   return best;
 }
