@@ -241,42 +241,48 @@ gemm_resid_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
   }
 }
 
-// Pairs of CTAs that the current device holds at once (0: none), once per device.
+constexpr int kWidths[] = {64, 96, 128, 192, 256};
+constexpr int kNumWidths = sizeof(kWidths) / sizeof(kWidths[0]);
+
 template <int BN>
-int pairs_held() {
+int query_pairs() {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = 2;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = sm_count() / 2 * 2;
+  cfg.blockDim = kThreads;
+  cfg.dynamicSmemBytes = Cfg<BN>::kSmem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int held = 0;
+  if (cudaFuncSetAttribute(gemm_resid_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem) != cudaSuccess ||
+      cudaOccupancyMaxActiveClusters(&held, gemm_resid_kernel<BN>, &cfg) != cudaSuccess) {
+    cudaGetLastError();      // (this failure's: an error that the caller has pending is the caller's)
+    return 0;
+  }
+  return held;
+}
+
+// Pairs of CTAs of each width that the current device holds at once (0: none), asked once per device; null without a device.
+const int* pairs_held() {
   static std::once_flag once[64];
-  static int resident[64];
+  static int held[64][kNumWidths];
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess) {
     cudaGetLastError();
-    return 0;
+    return nullptr;
   }
+  int* const of = held[dev & 63];
   std::call_once(once[dev & 63], [&] {
-    if (cudaFuncSetAttribute(gemm_resid_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem) != cudaSuccess) return;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = sm_count() / 2 * 2;
-    cfg.blockDim = kThreads;
-    cfg.dynamicSmemBytes = Cfg<BN>::kSmem;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    if (cudaOccupancyMaxActiveClusters(&resident[dev & 63], gemm_resid_kernel<BN>, &cfg) != cudaSuccess) resident[dev & 63] = 0;
+    of[0] = query_pairs<64>();
+    of[1] = query_pairs<96>();
+    of[2] = query_pairs<128>();
+    of[3] = query_pairs<192>();
+    of[4] = query_pairs<256>();
   });
-  cudaGetLastError();
-  return resident[dev & 63];
-}
-
-int held_of(int bn) {
-  switch (bn) {
-    case 64: return pairs_held<64>();
-    case 96: return pairs_held<96>();
-    case 128: return pairs_held<128>();
-    case 192: return pairs_held<192>();
-    default: return pairs_held<256>();
-  }
+  return of;
 }
 
 int row_tiles(const GemmParams& p) { return cdiv(p.batch * p.o_extent * cdiv(p.n_extent, kRun), 4); }
@@ -343,15 +349,18 @@ int resid_tile(const GemmParams& p, const GemmOperandA& a, const GemmOperandB& b
       (p.gate == nullptr || (p.g_col == 1 && p.g_n % 8 == 0 && p.g_o % 8 == 0 && p.g_b % 8 == 0)) &&
       static_cast<long long>(p.batch) * p.o_extent * cdiv(p.n_extent, kRun) <= 4096;
   if (!ok) return best;
-  const int blocks = cdiv(p.k_extent, kBK);
-  for (int bn : {64, 96, 128, 192, 256}) {
+  const int* const held = pairs_held();
+  if (held == nullptr) return best;
+  const int blocks = cdiv(p.k_extent, kBK), tiles = row_tiles(p);
+  for (int i = 0; i < kNumWidths; ++i) {
+    const int bn = kWidths[i];
     if (p.n_cols % bn != 0) continue;
     // a K block: its copies at 64 B per cycle, its products, the issuing thread's turn; beside it launch, fill and the epilogue
     double turn = 256.0 + bn;
     if (turn < 2.0 * bn) turn = 2.0 * bn;
     if (turn < 400.0) turn = 400.0;
     const double t = blocks * turn + 2500.0 + 6.0 * bn;
-    if ((best == 0 || t < least) && row_tiles(p) * (p.n_cols / bn) <= held_of(bn)) {
+    if ((best == 0 || t < least) && tiles * (p.n_cols / bn) <= held[i]) {
       best = bn;
       least = t;
     }
