@@ -58,6 +58,8 @@ template <int VEC>
 __device__ __forceinline__ void st_vec(__nv_bfloat16* p, const float (&v)[VEC]) {
   if constexpr (VEC == 8)
     *reinterpret_cast<uint4*>(p) = make_uint4(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]), pack_bf16x2(v[4], v[5]), pack_bf16x2(v[6], v[7]));
+  else if constexpr (VEC == 4)
+    *reinterpret_cast<uint2*>(p) = make_uint2(pack_bf16x2(v[0], v[1]), pack_bf16x2(v[2], v[3]));
   else
     *p = __float2bfloat16_rn(v[0]);
 }
@@ -316,7 +318,7 @@ __global__ void __launch_bounds__(256) token_range_kernel(const long long* index
 template <typename T, int VEC>
 __global__ void __launch_bounds__(256) atoms_to_tokens_kernel(const T* x, const long long* index, const unsigned char* mask, T* out,
                                                               long long rows, int n_atom, int n_token, int d, int index_div,
-                                                              int relu, const int2* range, int pieces) {
+                                                              int relu, const int2* range, int pieces, int out_vec) {
   grid_dependency_enter();
   const long long item = static_cast<long long>(blockIdx.x) * 8 + (threadIdx.x >> 5);
   const long long row = item / pieces;
@@ -368,7 +370,12 @@ __global__ void __launch_bounds__(256) atoms_to_tokens_kernel(const T* x, const 
   for (int i = 0; i < VEC; ++i)
     // the reference divides the sum by the count (scatter_reduce "mean"): a division, not a multiplication
     acc[i] = count > 0 ? acc[i] / static_cast<float>(count) : 0.f;
-  st_vec<VEC>(out + row * d + col, acc);
+  if (out_vec) {
+    st_vec<VEC>(out + row * d + col, acc);
+  } else {
+#pragma unroll
+    for (int i = 0; i < VEC; ++i) st_f(out + row * d + col + i, acc[i]);
+  }
 }
 
 }  // namespace
@@ -439,18 +446,23 @@ KFB_API int kfb_atoms_to_tokens(const void* x, const long long* token_index, con
     KFB_CUDA(cudaGetLastError());
   }
   LaunchScope scope(stream, "atoms_to_tokens");
-  const int vec16 = dtype == KFB_BF16 ? 8 : 4;       // elements of 16 bytes
-  const bool vec = d % vec16 == 0 && ((reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(out)) & 15) == 0;
-  const int pieces = cdiv(d, vec ? 32 * vec16 : 32);
+  // 16-byte pieces of bf16 where a row then needs fewer warps, 8-byte ones where its channels are whole fours; results by themselves where
+  // they start between pieces.  5 x 768 tokens of eight atoms, us by pieces of 16 / 8 bytes: 768 channels 17.2 / 21.3, 136 9.4 / 10.7, 128
+  // 9.4 / 6.7; single channels / 8 bytes: 124 12.8 / 6.6, 260 22.1 / 13.6.
+  const bool x_ok = (reinterpret_cast<uintptr_t>(x) & 15) == 0;
+  const int vec = x_ok && dtype == KFB_BF16 && d % 8 == 0 && d > 128 ? 8 : x_ok && d % 4 == 0 ? 4 : 1;
+  const int out_vec = (reinterpret_cast<uintptr_t>(out) & (vec * (dtype == KFB_BF16 ? 2 : 4) - 1)) == 0;
+  const int pieces = cdiv(d, 32 * vec);
   const unsigned blocks = static_cast<unsigned>((rows * pieces + 7) / 8);
   auto launch = [&](auto kernel, auto* xt, auto* ot) {
-    return launch_kernel(stream, kernel, blocks, 256, 0, xt, token_index, mask, ot, rows, n_atom, n_token, d, index_div, relu, range, pieces);
+    return launch_kernel(stream, kernel, blocks, 256, 0, xt, token_index, mask, ot, rows, n_atom, n_token, d, index_div, relu, range, pieces, out_vec);
   };
   if (dtype == KFB_BF16) {
     using T = __nv_bfloat16;
-    KFB_TRY(launch(vec ? atoms_to_tokens_kernel<T, 8> : atoms_to_tokens_kernel<T, 1>, static_cast<const T*>(x), static_cast<T*>(out)));
+    KFB_TRY(launch(vec == 8 ? atoms_to_tokens_kernel<T, 8> : vec == 4 ? atoms_to_tokens_kernel<T, 4> : atoms_to_tokens_kernel<T, 1>,
+                   static_cast<const T*>(x), static_cast<T*>(out)));
   } else {
-    KFB_TRY(launch(vec ? atoms_to_tokens_kernel<float, 4> : atoms_to_tokens_kernel<float, 1>, static_cast<const float*>(x),
+    KFB_TRY(launch(vec == 4 ? atoms_to_tokens_kernel<float, 4> : atoms_to_tokens_kernel<float, 1>, static_cast<const float*>(x),
                    static_cast<float*>(out)));
   }
   KFB_CUDA(cudaGetLastError());
