@@ -4,12 +4,12 @@
 // additive pair bias, masked keys get -1e9 (finite, as the reference does), optional sigmoid gate, and the result is written as the
 // bf16 triple split (an A operand's row, see part_a) that the fp32-accurate output projection consumes.
 //
-// A block takes 32 or 64 queries of one head and splits the keys over its eight or four warps, eight keys at a time; a lane owns one
-// or two query rows, and the warps' (maximum, sum, accumulator) are merged at the end.  The single-track problems (a few hundred queries,
-// one batch entry, 16 heads) have too few rows to fill the chip with one thread per row and all keys each: 301 queries x 16 heads x 48
-// took 250 us that way.  A warp stages its own keys in a two-slot ring with cp.async, so nothing but the merge waits for another
-// warp; K and V are read as broadcast 16-byte pieces, which bounds the loop (one load feeds four multiply-adds per query row: two
-// rows per lane where there are enough blocks without it).
+// Few rows (attention_fp32_kernel): a block takes 16 queries of one head, two lanes a row, and splits the keys over its eight warps, eight keys
+// at a time; where there are enough blocks without it, 64 queries, two rows a lane, over four warps.  The warps' (maximum, sum, accumulator)
+// are merged at the end.  The single-track problems (a few hundred queries, one batch entry, 16 heads) have too few rows to fill the chip
+// with one thread per row and all keys each: 301 queries x 16 heads x 48 took 250 us that way.  A warp stages its own keys in a two-slot ring
+// with cp.async, so nothing but the merge waits for another warp; K and V are read as broadcast 16-byte pieces, which bounds the loop.
+// Many rows: attention_fp32_rows_kernel below.
 #include "attention.cuh"
 #include "gemm.cuh"  // part_a
 #include "ptx.cuh"
@@ -256,7 +256,10 @@ __global__ void __launch_bounds__(kWarps * 32, LPR == 2 ? 2 : 1) attention_fp32_
 // (two rows a lane), and all keys go by in tiles of 32 that its warps share: one broadcast load of 16 bytes feeds eight multiply-adds of a
 // row pair, issued two at a time (fma.rn.f32x2: the same IEEE operations, sums over even and over odd channels added at the end).  The bias
 // comes with the keys by cp.async, 36 floats a row so that a lane's 16-byte pieces of its own row meet no bank conflict.
-// Measured (events, 4 heads of 32): 96 x 96 rows 53 -> 37 us, 128 x 128 82 -> 50, 160 x 160 149 -> 105, 200 x 200 298 -> 182, 256 x 256 460 -> 255.
+// Sums over keys are of eight by themselves, then added to the row's: in one accumulator for all keys the operator's error against 64 bits
+// was 5.6e-7 at 160 tokens and 6.4e-7 at 400 (root mean square of the result), with the split keys above 5.1e-7 and 5.2e-7, and is 5.05e-7 and
+// 5.15e-7 so, for 1 to 4 % of the time.
+// Measured (events, 4 heads of 32): 96 x 96 rows 54 -> 39 us, 128 x 128 82 -> 52, 160 x 160 150 -> 107, 200 x 200 298 -> 185, 256 x 256 461 -> 261.
 constexpr int kTile = 32, kBiasPitch = 36, kRowsWarp = 64;
 
 __device__ __forceinline__ void cp_async4(void* smem, const void* gmem) {
@@ -396,23 +399,35 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attention_fp32_rows_kernel(cons
           m_run[i] = m_new[i];
         }
       }
+      // eight keys by themselves: 512 are 64 + 8 roundings of a sum, not 512
+      uint64_t p2[2][kKeys];
 #pragma unroll
-      for (int i = 0; i < 2; ++i)
+      for (int i = 0; i < 2; ++i) {
+        float sum = 0.f;
 #pragma unroll
         for (int kk = 0; kk < kKeys; ++kk) {
           s[i][kk] = expf(s[i][kk] - m_run[i]);
-          l_run[i] += s[i][kk];
+          sum += s[i][kk];
+          p2[i][kk] = ptx::pack2(s[i][kk], s[i][kk]);
+        }
+        l_run[i] += sum;
+      }
+#pragma unroll
+      for (int d = 0; d < D / 4; ++d) {
+        uint64_t t[2][2];
+#pragma unroll
+        for (int kk = 0; kk < kKeys; ++kk) {
+          const ulonglong2 f = sv[kk * (D / 4) + d];
+#pragma unroll
+          for (int i = 0; i < 2; ++i) {
+            t[i][0] = kk == 0 ? mul2(p2[i][kk], f.x) : fma2(p2[i][kk], f.x, t[i][0]);
+            t[i][1] = kk == 0 ? mul2(p2[i][kk], f.y) : fma2(p2[i][kk], f.y, t[i][1]);
+          }
         }
 #pragma unroll
-      for (int kk = 0; kk < kKeys; ++kk) {
-        const uint64_t p0 = ptx::pack2(s[0][kk], s[0][kk]), p1 = ptx::pack2(s[1][kk], s[1][kk]);
-#pragma unroll
-        for (int d = 0; d < D / 4; ++d) {
-          const ulonglong2 f = sv[kk * (D / 4) + d];
-          acc[0][2 * d] = fma2(p0, f.x, acc[0][2 * d]);
-          acc[0][2 * d + 1] = fma2(p0, f.y, acc[0][2 * d + 1]);
-          acc[1][2 * d] = fma2(p1, f.x, acc[1][2 * d]);
-          acc[1][2 * d + 1] = fma2(p1, f.y, acc[1][2 * d + 1]);
+        for (int i = 0; i < 2; ++i) {
+          acc[i][2 * d] = ptx::add2(acc[i][2 * d], t[i][0]);
+          acc[i][2 * d + 1] = ptx::add2(acc[i][2 * d + 1], t[i][1]);
         }
       }
     }
@@ -475,14 +490,14 @@ int launch_rows(cudaStream_t stream, const AttnFp32Params& p, int bias_vec) {
 template <int D>
 int launch_rows(cudaStream_t stream, const AttnFp32Params& p) {
   const int bias_vec = (reinterpret_cast<uintptr_t>(p.bias) & 15) == 0 && p.ldb % 4 == 0 && (p.bias_hs > 0 ? p.bias_hs : p.lq * p.ldb) % 4 == 0;
-  // two warps share a tile's copies; one where the second would have nothing to do in every other block (160 rows: 117 us with two, 105 with
-  // one; 128: 50, 60; four: 80 and 118)
+  // two warps share a tile's copies; one where the second would have nothing to do in every other block (with one accumulator, 160 rows: 117 us
+  // with two, 105 with one; 128: 50, 60; four: 80 and 118)
   const int tiles = cdiv(p.lq, kRowsWarp);
   return tiles == 1 || tiles == 3 ? launch_rows<D, 1>(stream, p, bias_vec) : launch_rows<D, 2>(stream, p, bias_vec);
 }
 
-// The operands' rows by 16 bytes, and a block for every multiprocessor at least: below that (single-track problems) the keys of a row have to
-// be split to fill the chip, and a warp of fewer than 48 rows wastes more than the split costs.
+// The operands' rows by 16 bytes, and two (entry, head) problems for every multiprocessor at least: below that (single-track problems) the keys
+// of a row have to be split to fill the chip, and a warp of fewer than 48 rows wastes more than the split costs.
 bool takes_rows(const AttnFp32Params& p) {
   const long long ld_kv = p.ld_kv > 0 ? p.ld_kv : p.ld;
   const uintptr_t all = reinterpret_cast<uintptr_t>(p.q) | reinterpret_cast<uintptr_t>(p.k) | reinterpret_cast<uintptr_t>(p.v) |
