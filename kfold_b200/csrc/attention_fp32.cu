@@ -21,10 +21,6 @@ namespace {
 
 constexpr int kKeys = 8;    // keys per warp and step
 
-__device__ __forceinline__ void cp_async16(void* smem, const void* gmem) {
-  asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(ptx::smem_u32(smem)), "l"(gmem) : "memory");
-}
-
 using ptx::fma2;
 using ptx::mul2;
 
@@ -91,8 +87,8 @@ __global__ void __launch_bounds__(kWarps * 32, LPR == 2 ? 2 : 1) attention_fp32_
       const int kk = idx / (D / 4), c = idx - kk * (D / 4);
       const long long off = static_cast<long long>(min(g * kKeys + kk, p.lk - 1)) * ld_kv + c * 4;
       const int at = kk * kPitch + c * 4 + (LPR == 2 && c >= DL / 4 ? 4 : 0);
-      cp_async16(dst + at, k_base + off);
-      cp_async16(dst + kKeys * kPitch + at, v_base + off);
+      ptx::cp_async_16(dst + at, k_base + off);
+      ptx::cp_async_16(dst + kKeys * kPitch + at, v_base + off);
     }
     const int key = g * kKeys + (lane & 7);
     mask_r = key < p.lk ? ((mrow == nullptr || mrow[static_cast<long long>(key) * p.m_k]) ? 0.f : -1e9f) : -INFINITY;
@@ -296,14 +292,14 @@ __global__ void __launch_bounds__(W * 32, 8 / W) attention_fp32_rows_kernel(cons
     for (int idx = threadIdx.x; idx < kTile * D / 4; idx += threads) {
       const int kk = idx / (D / 4), c = idx - kk * (D / 4);
       const long long off = static_cast<long long>(min(k0 + kk, p.lk - 1)) * ld_kv + c * 4;
-      cp_async16(kv + idx * 4, k_base + off);
-      cp_async16(kv + kTile * D + idx * 4, v_base + off);
+      ptx::cp_async_16(kv + idx * 4, k_base + off);
+      ptx::cp_async_16(kv + kTile * D + idx * 4, v_base + off);
     }
     float* bias = s_bias + slot * rows * kBiasPitch;
     if (bias_vec && k0 + kTile <= p.lk) {
       for (int idx = threadIdx.x; idx < rows * (kTile / 4); idx += threads) {
         const int row = idx >> 3, c = idx & 7;
-        if (q0 + row < p.lq) cp_async16(bias + row * kBiasPitch + c * 4, bias_base + static_cast<long long>(q0 + row) * p.ldb + k0 + c * 4);
+        if (q0 + row < p.lq) ptx::cp_async_16(bias + row * kBiasPitch + c * 4, bias_base + static_cast<long long>(q0 + row) * p.ldb + k0 + c * 4);
       }
     } else {
       for (int idx = threadIdx.x; idx < rows * kTile; idx += threads) {

@@ -96,6 +96,29 @@ inline int launch_kernel(cudaStream_t stream, void (*kernel)(KArgs...), dim3 gri
   return launch_kernel_clustered(stream, kernel, 1, grid, block, smem, static_cast<Args&&>(args)...);
 }
 
+// Clusters of `cluster` CTAs of a kernel that the current device holds at once, after it has been allowed its shared memory; 0 where the device,
+// or the part of one that this process may use, holds none or does not say.  (Only a failure of the question itself is cleared: an error that
+// the caller has pending is the caller's.)  A call of some us: whoever asks keeps the answer for each device.
+template <typename... KArgs>
+inline int clusters_held(void (*kernel)(KArgs...), unsigned cluster, int threads, size_t smem) {
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster;
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = sm_count() / static_cast<int>(cluster) * static_cast<int>(cluster);
+  cfg.blockDim = threads;
+  cfg.dynamicSmemBytes = smem;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+  int held = 0;
+  if (cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, static_cast<int>(smem)) == cudaSuccess &&
+      cudaOccupancyMaxActiveClusters(&held, kernel, &cfg) == cudaSuccess)
+    return held;
+  cudaGetLastError();
+  return 0;
+}
+
 #ifdef __CUDACC__
 // (see launch_kernel)
 __device__ __forceinline__ void grid_dependency_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }

@@ -22,21 +22,12 @@ static int tiles_held(int* held) {
   KFB_CUDA(cudaGetDevice(&dev));
   cudaError_t attr_err = cudaSuccess;
   std::call_once(once[dev & 63], [&] {
+    if (PAIR) {     // (a multiprocessor without a neighbour to pair with stays idle)
+      resident[dev & 63] = clusters_held(kernel, 2, gemm_threads<AUX, STATS, TWIN>(), GemmCfg<BN, PAIR>::kSmemBytes);
+      return;
+    }
     attr_err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, GemmCfg<BN, PAIR>::kSmemBytes);
     resident[dev & 63] = attr_err == cudaSuccess ? sm_count() : 0;
-    if (PAIR && attr_err == cudaSuccess) {     // (a multiprocessor without a neighbour to pair with stays idle)
-      cudaLaunchAttribute attr[1];
-      attr[0].id = cudaLaunchAttributeClusterDimension;
-      attr[0].val.clusterDim.x = 2;
-      attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-      cudaLaunchConfig_t cfg = {};
-      cfg.gridDim = sm_count() / 2 * 2;
-      cfg.blockDim = gemm_threads<AUX, STATS, TWIN>();
-      cfg.dynamicSmemBytes = GemmCfg<BN, PAIR>::kSmemBytes;
-      cfg.attrs = attr;
-      cfg.numAttrs = 1;
-      attr_err = cudaOccupancyMaxActiveClusters(&resident[dev & 63], kernel, &cfg);
-    }
   });
   KFB_CUDA(attr_err);
   *held = resident[dev & 63];

@@ -244,27 +244,6 @@ gemm_resid_kernel(const __grid_constant__ CUtensorMap tm_a, const __grid_constan
 constexpr int kWidths[] = {64, 96, 128, 192, 256};
 constexpr int kNumWidths = sizeof(kWidths) / sizeof(kWidths[0]);
 
-template <int BN>
-int query_pairs() {
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = 2;
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = sm_count() / 2 * 2;
-  cfg.blockDim = kThreads;
-  cfg.dynamicSmemBytes = Cfg<BN>::kSmem;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  int held = 0;
-  if (cudaFuncSetAttribute(gemm_resid_kernel<BN>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<BN>::kSmem) != cudaSuccess ||
-      cudaOccupancyMaxActiveClusters(&held, gemm_resid_kernel<BN>, &cfg) != cudaSuccess) {
-    cudaGetLastError();      // (this failure's: an error that the caller has pending is the caller's)
-    return 0;
-  }
-  return held;
-}
-
 // Pairs of CTAs of each width that the current device holds at once (0: none), asked once per device; null without a device.
 const int* pairs_held() {
   static std::once_flag once[64];
@@ -276,11 +255,11 @@ const int* pairs_held() {
   }
   int* const of = held[dev & 63];
   std::call_once(once[dev & 63], [&] {
-    of[0] = query_pairs<64>();
-    of[1] = query_pairs<96>();
-    of[2] = query_pairs<128>();
-    of[3] = query_pairs<192>();
-    of[4] = query_pairs<256>();
+    of[0] = clusters_held(gemm_resid_kernel<64>, 2, kThreads, Cfg<64>::kSmem);
+    of[1] = clusters_held(gemm_resid_kernel<96>, 2, kThreads, Cfg<96>::kSmem);
+    of[2] = clusters_held(gemm_resid_kernel<128>, 2, kThreads, Cfg<128>::kSmem);
+    of[3] = clusters_held(gemm_resid_kernel<192>, 2, kThreads, Cfg<192>::kSmem);
+    of[4] = clusters_held(gemm_resid_kernel<256>, 2, kThreads, Cfg<256>::kSmem);
   });
   return of;
 }

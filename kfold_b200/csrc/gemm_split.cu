@@ -286,21 +286,7 @@ struct SplitLauncher {
     static std::once_flag once[64];
     static int held[64][kMaxSplit + 1];
     std::call_once(once[dev & 63], [&] {
-      if (cudaFuncSetAttribute(gemm_split_kernel<BN, PRECISE>, cudaFuncAttributeMaxDynamicSharedMemorySize, SplitCfg<BN>::kSmem) != cudaSuccess) return;
-      for (int s = 2; s <= kMaxSplit; ++s) {
-        cudaLaunchAttribute attr[1];
-        attr[0].id = cudaLaunchAttributeClusterDimension;
-        attr[0].val.clusterDim.x = s;
-        attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-        cudaLaunchConfig_t cfg = {};
-        cfg.gridDim = sm_count() / s * s;
-        cfg.blockDim = kSplitThreads;
-        cfg.dynamicSmemBytes = SplitCfg<BN>::kSmem;
-        cfg.attrs = attr;
-        cfg.numAttrs = 1;
-        if (cudaOccupancyMaxActiveClusters(&held[dev & 63][s], gemm_split_kernel<BN, PRECISE>, &cfg) != cudaSuccess) held[dev & 63][s] = 0;
-      }
-      cudaGetLastError();
+      for (int s = 2; s <= kMaxSplit; ++s) held[dev & 63][s] = clusters_held(gemm_split_kernel<BN, PRECISE>, s, kSplitThreads, SplitCfg<BN>::kSmem);
     });
     return split <= kMaxSplit ? held[dev & 63][split] : 0;
   }

@@ -564,41 +564,18 @@ pair_project_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_const
   }
 }
 
-// Pairs of CTAs that the current device holds at once (0: none), once per device.
+// Pairs of CTAs that the current device holds at once (0: none), asked once per device.
 template <int C, bool ATT>
-int pairs_held(int* held) {
+int pairs_held() {
   static std::once_flag once[64];
-  static int resident[64];
+  static int held[64];
   int dev = 0;
-  KFB_CUDA(cudaGetDevice(&dev));
-  cudaError_t err = cudaSuccess;
-  std::call_once(once[dev & 63], [&] {
-    constexpr auto kernel = pair_project_kernel<C, ATT>;
-    err = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<C, ATT>::kSmem);
-    if (err != cudaSuccess) return;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = sm_count() / 2 * 2;
-    cfg.blockDim = kThreads;
-    cfg.dynamicSmemBytes = Cfg<C, ATT>::kSmem;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    err = cudaOccupancyMaxActiveClusters(&resident[dev & 63], kernel, &cfg);
-  });
-  KFB_CUDA(err);
-  *held = resident[dev & 63];
-  return KFB_OK;
-}
-
-template <int C, bool ATT>
-bool holds_pairs() {
-  int held = 0;
-  const bool known = pairs_held<C, ATT>(&held) == KFB_OK;
-  if (!known) cudaGetLastError();
-  return known && held > 0;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  std::call_once(once[dev & 63], [&] { held[dev & 63] = clusters_held(pair_project_kernel<C, ATT>, 2, kThreads, Cfg<C, ATT>::kSmem); });
+  return held[dev & 63];
 }
 
 bool rows_ok(const PairRows& r, int dtype) {
@@ -627,8 +604,8 @@ int launch(cudaStream_t stream, const PairRows& r, const void* w, const void* w_
   const long long w_rows = (K::kUnits - 1) * kUnit;
   KFB_TRY(map4(&tw, w, C, w_rows, 1, 1, C, C * w_rows, C * w_rows, 64, kUnit / 2, 1));
   KFB_TRY(map4(&tl, w_last, C, K::kLastN, 1, 1, C, C * K::kLastN, C * K::kLastN, 64, K::kLastN / 2, 1));
-  int held = 0;
-  KFB_TRY((pairs_held<C, ATT>(&held)));
+  const int held = pairs_held<C, ATT>();
+  KFB_CHECK_ARG(held > 0, "%s: the device holds no pair of this kernel", tag);
   p.ln_w = r.ln_w;
   p.ln_b = r.ln_b;
   p.eps = r.eps;
@@ -653,7 +630,7 @@ int launch(cudaStream_t stream, const PairRows& r, const void* w, const void* w_
 bool trimul_pair_project_ok(const PairRows& r, const void* w_in, const void* w_gout, const void* ab, const void* gl, int dtype) {
   const uintptr_t all = reinterpret_cast<uintptr_t>(w_in) | reinterpret_cast<uintptr_t>(w_gout) | reinterpret_cast<uintptr_t>(ab) |
                         reinterpret_cast<uintptr_t>(gl);
-  return (all & 15) == 0 && rows_ok(r, dtype) && (r.c == 128 ? holds_pairs<128, false>() : r.c == 256 && holds_pairs<256, false>());
+  return (all & 15) == 0 && rows_ok(r, dtype) && (r.c == 128 ? pairs_held<128, false>() > 0 : r.c == 256 && pairs_held<256, false>() > 0);
 }
 
 int launch_trimul_pair_project(cudaStream_t stream, const PairRows& r, const void* w_in, const void* w_gout, __nv_bfloat16* ab, int pitch,
@@ -677,7 +654,7 @@ int launch_trimul_pair_project(cudaStream_t stream, const PairRows& r, const voi
 bool triatt_pair_project_ok(const PairRows& r, const void* w, int heads, int hdp, const void* qkg, const void* vt, const void* bias, int dtype) {
   const uintptr_t all = reinterpret_cast<uintptr_t>(w) | reinterpret_cast<uintptr_t>(qkg) | reinterpret_cast<uintptr_t>(vt) |
                         reinterpret_cast<uintptr_t>(bias);
-  return r.c == 128 && hdp == 128 && heads <= 8 && (all & 15) == 0 && rows_ok(r, dtype) && row_tiles(r) >= 16 && holds_pairs<128, true>();
+  return r.c == 128 && hdp == 128 && heads <= 8 && (all & 15) == 0 && rows_ok(r, dtype) && row_tiles(r) >= 16 && pairs_held<128, true>() > 0;
 }
 
 int launch_triatt_pair_project(cudaStream_t stream, const PairRows& r, const void* w, int heads, __nv_bfloat16* qkg, __nv_bfloat16* vt,

@@ -403,33 +403,20 @@ transition_pair_kernel(const __grid_constant__ CUtensorMap tm_x, const __grid_co
   }
 }
 
-// Pairs of CTAs that the current device holds at once (0: none), once per device.
+// Pairs of CTAs that the current device holds at once (0: none), asked once per device.
 template <int C>
-int pairs_held(int* held) {
+int pairs_held() {
   static std::once_flag once[64];
-  static int resident[64];
+  static int held[64];
   int dev = 0;
-  KFB_CUDA(cudaGetDevice(&dev));
-  cudaError_t err = cudaSuccess;
-  std::call_once(once[dev & 63], [&] {
-    err = cudaFuncSetAttribute(transition_pair_kernel<C>, cudaFuncAttributeMaxDynamicSharedMemorySize, Cfg<C>::kSmem);
-    if (err != cudaSuccess) return;
-    cudaLaunchAttribute attr[1];
-    attr[0].id = cudaLaunchAttributeClusterDimension;
-    attr[0].val.clusterDim.x = 2;
-    attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-    cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = sm_count() / 2 * 2;
-    cfg.blockDim = kThreads;
-    cfg.dynamicSmemBytes = Cfg<C>::kSmem;
-    cfg.attrs = attr;
-    cfg.numAttrs = 1;
-    err = cudaOccupancyMaxActiveClusters(&resident[dev & 63], transition_pair_kernel<C>, &cfg);
-  });
-  KFB_CUDA(err);
-  *held = resident[dev & 63];
-  return KFB_OK;
+  if (cudaGetDevice(&dev) != cudaSuccess) {
+    cudaGetLastError();
+    return 0;
+  }
+  std::call_once(once[dev & 63], [&] { held[dev & 63] = clusters_held(transition_pair_kernel<C>, 2, kThreads, Cfg<C>::kSmem); });
+  return held[dev & 63];
 }
+int pairs_held(int c) { return c == 128 ? pairs_held<128>() : pairs_held<256>(); }
 
 template <int C>
 int launch(cudaStream_t stream, const void* x, const float* ln_w, const float* ln_b, const void* w_swiglu, const void* w_out, void* out,
@@ -446,8 +433,8 @@ int launch(cudaStream_t stream, const void* x, const float* ln_w, const float* l
   KFB_TRY(rows_map(&t2, w_out, C, hidden, C / 2));
   KFB_TRY(rows_map(&tr, resid != nullptr ? resid : x, rows, C, kRows));
   KFB_TRY(rows_map(&to, out, rows, C, kRows));
-  int held = 0;
-  KFB_TRY(pairs_held<C>(&held));
+  const int held = pairs_held<C>();
+  KFB_CHECK_ARG(held > 0, "transition: the device holds no pair of this kernel");
   PairTransParams p;
   p.ln_w = ln_w;
   p.ln_b = ln_b;
@@ -469,10 +456,7 @@ bool transition_pair_ok(const void* x, const void* w_swiglu, const void* w_out, 
   const uintptr_t all = reinterpret_cast<uintptr_t>(x) | reinterpret_cast<uintptr_t>(w_swiglu) | reinterpret_cast<uintptr_t>(w_out) |
                         reinterpret_cast<uintptr_t>(out) | reinterpret_cast<uintptr_t>(resid);
   if (dtype != KFB_BF16 || (c != 128 && c != 256) || hidden % 128 != 0 || (all & 15) != 0 || rows > (1ll << 30)) return false;
-  int held = 0;
-  const bool known = (c == 128 ? pairs_held<128>(&held) : pairs_held<256>(&held)) == KFB_OK;
-  if (!known) cudaGetLastError();
-  return known && held > 0;
+  return pairs_held(c) > 0;
 }
 
 // Few rows: a pair walks all hidden channels of its 256 rows, 1.0 us a chunk at 256 channels and 0.52 at 128, however few tiles there are,
@@ -481,8 +465,8 @@ bool transition_pair_ok(const void* x, const void* w_swiglu, const void* w_out, 
 // 9 216 25.6 / 25.8, 10 500 30.8 / 27.1; 512 hidden: 4 096 16.6 / 17.6, 5 000 17.8 / 17.5; 128 channels and 512 hidden: 256 rows 12.2 / 10.7.
 // (Beyond 64 rows for each multiprocessor the three launches take a second round: a fifth more.)
 bool transition_pair_is_faster(long long rows, int c, int hidden) {
-  int held = 1;
-  if ((c == 128 ? pairs_held<128>(&held) : pairs_held<256>(&held)) != KFB_OK || held < 1) return false;
+  const int held = pairs_held(c);
+  if (held < 1) return false;
   const double chunks = hidden / kChunk;
   const long long tiles = (rows + 2 * kRows - 1) / (2 * kRows), rounds = (tiles + held - 1) / held;
   const double pair = c == 128 ? 6.9 + 0.52 * chunks * rounds : 9.2 + chunks * rounds;
