@@ -146,9 +146,10 @@ static int narrow_tile(const GemmParams& p, int bn) {
 // CTA pairs (PAIR in gemm.cuh) pay where the main loop is long enough to hide the epilogue of a tile twice as wide and the tiles are at
 // least a wave of pairs.  Measured, one CTA -> pair: triangle contraction at 768 tokens 108 -> 99 us (128 channels), 201 -> 180 (256);
 // at 400 tokens (seven K blocks) 71 -> 62; SwiGLU of 256 channels at 768 x 768 rows 585 -> 472, its output projection (K = 1 024) 362 ->
-// 318; token transformer, 5 x 768 rows of 768: projection 35 -> 29, SwiGLU 24.5 -> 22.5; conditioning tables of those rows (six, staged) 415 -> 390.  The other side of the lines: SwiGLU of 128 channels (two K blocks) 106 -> 107; gate
-// projection of 256 (four, plain) 105 -> 109; contraction at 333 tokens (three row blocks, a
-// quarter of the pairs' work padding) 49.7 -> 51.6; float32 output projections with gate and residual 22.4 -> 23.5.
+// 318; token transformer, 5 x 768 rows of 768: projection 35 -> 29, SwiGLU 24.5 -> 22.5; conditioning tables of those rows (six, staged)
+// 415 -> 390.  The other side of the lines: SwiGLU of 128 channels (two K blocks) 106 -> 107; gate projection of 256 (four, plain) 105 -> 109;
+// contraction at 333 tokens (three row blocks, a quarter of the pairs' work padding) 49.7 -> 51.6; float32 output projections with gate and
+// residual 22.4 -> 23.5.
 static bool pair_tile(const GemmParams& p, int bn) {
   if (p.precise || bn < 128 || p.n_cols < 256 || p.glu == GLU_SIGMOID) return false;
   const int num_k = cdiv(p.k_extent, kBK), pairs = cdiv(p.n_blocks, 2);

@@ -747,8 +747,7 @@ __device__ __forceinline__ void load8(const float* p, float (&f)[8]) {
   f[0] = lo.x; f[1] = lo.y; f[2] = lo.z; f[3] = lo.w; f[4] = hi.x; f[5] = hi.y; f[6] = hi.z; f[7] = hi.w;
 }
 // OUTS = 2: a second set of gates and shifts (`gv2`, rows as far apart) from the same statistics into `y2`: the queries' and the keys' AdaLN of
-// an atom block in one launch (66 launches a step become 60: 705 -> 672 us of
-// AdaLN between events, 5 x 768 tokens).
+// an atom block in one launch (66 launches a step become 60; 5 x 768 tokens: 705 -> 672 us of AdaLN between events).
 template <typename TI, int CH, int LANES, int OUTS>
 __global__ void __launch_bounds__(256) adaln_vec_kernel(const TI* a, __nv_bfloat16* y, __nv_bfloat16* y2, const __nv_bfloat16* gv,
                                                         const __nv_bfloat16* gv2, long long gv_ld, long long rows, int samples, int l, float eps,

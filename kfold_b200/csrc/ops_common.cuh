@@ -69,8 +69,7 @@ int triatt_run(cudaStream_t stream, int ending, const void* x, const unsigned ch
                const void* w_proj_packed, const void* w_out, void* out, const void* resid, void* workspace, size_t workspace_bytes, int batch,
                int n, int c, int heads, float eps, int dtype, int2* mask_rows, int w_static);
 // kfb_trimul_fwd; fold_room: trimul_fold_bytes(c) bytes (256-byte aligned) beside the workspace for the output projection's folded
-// weights, which then cost no launch, or null.  (bf16 path; the fp32-accurate one folds nothing.)  w_static
-// as in ApbArgs.
+// weights, which then cost no launch, or null.  (bf16 path; the fp32-accurate one folds nothing.)  w_static as in ApbArgs.
 size_t trimul_fold_bytes(int c);
 int trimul_run(cudaStream_t stream, int incoming, const void* x, const unsigned char* mask, const float* ln_in_w, const float* ln_in_b,
                const void* w_in_packed, const void* w_gout, const float* ln_out_w, const float* ln_out_b, const void* w_pout, void* out,

@@ -18,8 +18,9 @@
 // Few rows: with fewer tiles than pairs / units, a pair takes one unit of a tile (and normalises the rows for it alone).
 // The arithmetic is that of the LayerNorm kernels and of the GEMMs: the same bits.
 //
-// Measured (events, LayerNorm and projections as two or three launches -> this): 768 x 768 rows, triangle multiplication of 128 channels 202 ->
-// 133 us (604 MB: 4.5 TB/s), of 256 600 -> 336, triangle attention's 220 -> 141; 251 x 251: 33 -> 29.5, 97 -> 55 and 29 -> 30.5.
+// Measured (events inside the operators, LayerNorm and projections as two or three launches -> this): 768 x 768 rows, triangle multiplication
+// of 128 channels 206 -> 139 us (604 MB: 4.4 TB/s), of 256 544 -> 331, triangle attention's 224 -> 151; 251 x 251: 41 -> 30.5, 88 -> 55 and
+// 43 -> 31.6; 64 x 64: 21 -> 16.6, 35 -> 25.8 and 21 -> 18.2.
 #include <cuda_bf16.h>
 
 #include <mutex>
